@@ -3,19 +3,28 @@
 //
 // Replaces the eager chain of the reference's `genstep` (fp32 cast, topk, sort, softmax, cumsum, scatter,
 // Categorical, gather, mask compare: nn/real_llm_generate.py:26-141, utils/logits_warper.py) — about 1 ms per decode
-// step at [128, 32000] — with radix selection in shared memory:
-//   * the row is staged once in shared memory as fp32 (V * 4 bytes <= 200 KB);
-//   * top-k threshold = k-th largest key by a 4 x 8-bit radix descent over per-warp histograms;
+// step at [128, 32000].  The row is staged once in shared memory as fp32 (V * 4 bytes <= 200 KB).
+//
+// Nothing here is bound by bytes (8 MB at [128, 32000]): a row's time is the chain of block-wide steps.  A radix descent over the whole row
+// (4 digits each for top-k and top-p) spends them on shared atomics that pile up on the few bins logits fall in: 89 us at
+// [128, 32000], top-k 50, top-p 0.9.  For top_k <= 512 the row is therefore cut down first: the k-th largest of the 1024 per-thread maxima is
+// a lower bound of the k-th largest logit (those are k elements at least as large), and only a few hundred elements reach it.  They
+// are compacted in index order; the exact k-th largest among them comes from a bitwise search that counts with the block barrier itself, the
+// top-p threshold from every kept element summing the mass of the strictly larger ones, the draw from one block scan: 25 us.
+// A larger top_k, and a row with more than 1536 candidates or 1024 kept elements (ties), takes the radix descent:
+//   * top-k threshold = k-th largest key by a 4 x 8-bit descent over a shared histogram;
 //   * top-p threshold = the same descent with probability mass instead of counts (keep x iff the mass of strictly
-//     larger logits is < top_p * total);
-//   * the sample is drawn by inverse CDF in index order over the kept set with a block scan (counter-based RNG).
-// Ties at a threshold are all kept (same rule as `logits < kth` in the PyTorch reference).
+//     larger logits is < top_p * total).
+// The sample is drawn by inverse CDF in index order over the kept set (counter-based RNG).  Ties at a threshold are all kept (same
+// rule as `logits < kth` in the PyTorch reference).
 #include "common.cuh"
 
 namespace {
 
 constexpr int kThreads = 1024;
 constexpr int kWarps = kThreads / 32;
+constexpr int kFastTopK = 512;      // the thread maxima bound the k-th logit tightly only while k is well below their number
+constexpr int kMaxCand = 1536, kMaxKept = kThreads;   // with 51200 staged logits the block's shared memory is nearly full
 
 RB_DEVICE uint32_t f2key(float x) {  // order-preserving float -> uint
   const uint32_t u = __float_as_uint(x);
@@ -49,14 +58,91 @@ struct SampleParams {
   const int64_t* seed_ptr;   // device-resident seed (a replayed graph must not repeat the random stream of the previous call)
 };
 
+struct SampleShared {
+  float red[32];
+  uint32_t redu[32];
+  uint32_t u[4];
+  float f[4];
+  union {
+    struct { uint32_t hist[256]; float histm[256]; };                     // radix descent
+    struct { float cand[kMaxCand]; int cand_idx[kMaxCand]; };             // candidates in index order: value and index
+  };
+  float kept[kMaxKept];           // elements of the top-k set: value, index, exp(value - max)
+  int kept_idx[kMaxKept];
+  float kept_e[kMaxKept];
+};
+
+// Inclusive prefix over the block of `v`, and the block's total; `red` holds one entry per warp.  Two barriers.
+template <typename V> RB_DEVICE V block_inclusive(V v, V* red, V& total) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  V incl = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const V x = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += x;
+  }
+  __syncthreads();               // protect `red` from a previous use
+  if (lane == 31) red[warp] = incl;
+  __syncthreads();
+  V w = red[lane];
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const V x = __shfl_up_sync(0xffffffffu, w, o);
+    if (lane >= o) w += x;
+  }
+  total = __shfl_sync(0xffffffffu, w, 31);
+  const V base = __shfl_sync(0xffffffffu, w, warp == 0 ? 0 : warp - 1);
+  return (warp == 0 ? V(0) : base) + incl;
+}
+
+// The k-th largest of the block's keys, kPer of them per thread (a thread without one passes 0: it is never counted, and k never exceeds
+// the number of real keys).  One counting barrier per bit and key.
+template <int kPer> RB_DEVICE uint32_t kth_largest(const uint32_t (&key)[kPer], int k) {
+  uint32_t prefix = 0;
+#pragma unroll 1
+  for (int bit = 31; bit >= 0; --bit) {
+    const uint32_t c = prefix | (1u << bit);
+    int n = 0;
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) n += __syncthreads_count(key[i] >= c);
+    if (n >= k) prefix = c;
+  }
+  return prefix;
+}
+
+// Largest bin b such that the sum of the bins above it is below `want` and including it reaches it (0 if none does), and that sum above
+// it plus `above`: one warp, eight bins a lane, from the top.
+template <typename V> RB_DEVICE void find_bin(const V* bins, V above, V want, uint32_t* out_bin, V* out_above) {
+  const int lane = threadIdx.x & 31;
+  V mine[8], sum = 0;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) { mine[i] = bins[255 - (lane * 8 + i)]; sum += mine[i]; }
+  V incl = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const V x = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += x;
+  }
+  V cum = above + incl - sum;
+  int bin = -1;
+  V at = 0;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    if (bin < 0 && cum + mine[i] >= want) { bin = 255 - (lane * 8 + i); at = cum; }
+    cum += mine[i];
+  }
+  const unsigned hit = __ballot_sync(0xffffffffu, bin >= 0);
+  const int w = hit ? __ffs(hit) - 1 : 31;
+  const V all = __shfl_sync(0xffffffffu, cum - mine[7], 31);       // nothing reaches `want`: bin 0, everything above it
+  const int b = __shfl_sync(0xffffffffu, bin, w);
+  const V a = __shfl_sync(0xffffffffu, at, w);
+  if (lane == 0) { *out_bin = hit ? (uint32_t)b : 0u; *out_above = hit ? a : all; }
+}
+
 template <typename T>
 __global__ void __launch_bounds__(kThreads, 1) sample_kernel(SampleParams p) {
   extern __shared__ float srow[];                       // [V] scaled logits
-  __shared__ uint32_t hist[256];
-  __shared__ float histm[256];
-  __shared__ float red[32];
-  __shared__ uint32_t sh_u[4];
-  __shared__ float sh_f[4];
+  __shared__ SampleShared sh;
   const int row = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const T* src = reinterpret_cast<const T*>(p.logits) + (int64_t)row * p.row_stride;
   const int V = p.V;
@@ -74,169 +160,236 @@ __global__ void __launch_bounds__(kThreads, 1) sample_kernel(SampleParams p) {
 
   // ---- stage + max
   float mx = -INFINITY;
-  for (int j = tid; j < V; j += kThreads) {
-    float x = rb::to_f(src[j]) * p.inv_temp;
+  uint32_t kmax = 0;
+  auto put = [&](int j, float raw) {
+    float x = raw * p.inv_temp;
     if (p.suppress_eos && j == p.eos_id) x = -INFINITY;
-    srow[j] = x;
     mx = fmaxf(mx, x);
+    kmax = max(kmax, f2key(x));
+    return x;
+  };
+  constexpr int VEC = 16 / sizeof(T);
+  if (p.row_stride % VEC == 0 && (reinterpret_cast<uintptr_t>(p.logits) & 15) == 0) {
+    const int nvec = V / VEC;
+    for (int i = tid; i < nvec; i += kThreads) {
+      const rb::Pack<T, VEC> v = reinterpret_cast<const rb::Pack<T, VEC>*>(src)[i];
+#pragma unroll
+      for (int q = 0; q < VEC / 4; ++q)
+        reinterpret_cast<float4*>(srow)[i * (VEC / 4) + q] =
+            make_float4(put(i * VEC + 4 * q, rb::to_f(v.v[4 * q])), put(i * VEC + 4 * q + 1, rb::to_f(v.v[4 * q + 1])),
+                        put(i * VEC + 4 * q + 2, rb::to_f(v.v[4 * q + 2])), put(i * VEC + 4 * q + 3, rb::to_f(v.v[4 * q + 3])));
+    }
+    for (int j = nvec * VEC + tid; j < V; j += kThreads) srow[j] = put(j, rb::to_f(src[j]));
+  } else {
+    for (int j = tid; j < V; j += kThreads) srow[j] = put(j, rb::to_f(src[j]));
   }
-  mx = rb::block_reduce<true>(mx, red);
+  mx = rb::block_reduce<true>(mx, sh.red);
 
   int64_t chosen = 0;
   float chosen_lp = 0.f;
   uint32_t keep_key = 0;  // keep elements with key >= keep_key
+  // every warp owns a range of whole 32-element groups: (warp, group, lane) is index order
+  const int span = ((V + 31) / 32 + kWarps - 1) / kWarps * 32, w0 = min(V, warp * span), w1 = min(V, w0 + span);
 
   if (p.greedy) {
     // argmax (lowest index among ties)
     int best = V;
     for (int j = tid; j < V; j += kThreads) if (srow[j] == mx) best = min(best, j);
     __syncthreads();
-    // block min via shuffles + smem
     for (int o = 16; o > 0; o >>= 1) best = min(best, __shfl_xor_sync(0xffffffffu, best, o));
-    if (lane == 0) sh_u[0] = 0xffffffffu;
+    if (lane == 0) sh.u[0] = 0xffffffffu;
     __syncthreads();
-    if (lane == 0) atomicMin(&sh_u[0], (uint32_t)best);
+    if (lane == 0) atomicMin(&sh.u[0], (uint32_t)best);
     __syncthreads();
-    chosen = sh_u[0];
+    chosen = sh.u[0];
     float s = 0.f;
     for (int j = tid; j < V; j += kThreads) s += __expf(srow[j] - mx);
-    s = rb::block_reduce<false>(s, red);
+    s = rb::block_reduce<false>(s, sh.red);
     chosen_lp = -__logf(s);
     keep_key = 0;
   } else {
-    // ---- top-k: k-th largest key by radix descent
-    uint32_t prefix = 0, maskbits = 0;
-    if (p.top_k < V) {
-      uint32_t remaining = (uint32_t)p.top_k;
-      for (int pass = 0; pass < 4; ++pass) {
-        const int shift = 24 - 8 * pass;
-        for (int b = tid; b < 256; b += kThreads) hist[b] = 0;
-        __syncthreads();
-        for (int j = tid; j < V; j += kThreads) {
-          const uint32_t k = f2key(srow[j]);
-          if ((k & maskbits) == prefix) atomicAdd(&hist[(k >> shift) & 255u], 1u);
-        }
-        __syncthreads();
-        if (tid == 0) {
-          uint32_t cum = 0;
-          int b = 255;
-          for (; b > 0; --b) {
-            if (cum + hist[b] >= remaining) break;
-            cum += hist[b];
-          }
-          sh_u[0] = (uint32_t)b;
-          sh_u[1] = remaining - cum;
-        }
-        __syncthreads();
-        prefix |= sh_u[0] << shift;
-        maskbits |= 255u << shift;
-        remaining = sh_u[1];
-        __syncthreads();
-      }
-      keep_key = prefix;
-    }
-    // ---- softmax mass of the top-k set
-    float tot = 0.f;
-    for (int j = tid; j < V; j += kThreads) {
-      const float x = srow[j];
-      if (f2key(x) >= keep_key) tot += __expf(x - mx);
-    }
-    tot = rb::block_reduce<false>(tot, red);
-    // ---- top-p: weighted radix descent inside the top-k set
-    if (p.top_p < 1.f) {
-      const float P = p.top_p * tot;
-      float above = 0.f;
-      prefix = 0; maskbits = 0;
-      for (int pass = 0; pass < 4; ++pass) {
-        const int shift = 24 - 8 * pass;
-        for (int b = tid; b < 256; b += kThreads) histm[b] = 0.f;
-        __syncthreads();
-        for (int j = tid; j < V; j += kThreads) {
-          const float x = srow[j];
-          const uint32_t k = f2key(x);
-          if (k >= keep_key && (k & maskbits) == prefix) atomicAdd(&histm[(k >> shift) & 255u], __expf(x - mx));
-        }
-        __syncthreads();
-        if (tid == 0) {
-          float cum = above;
-          int b = 255;
-          for (; b > 0; --b) {
-            if (cum + histm[b] >= P) break;
-            cum += histm[b];
-          }
-          sh_u[0] = (uint32_t)b;
-          sh_f[0] = cum;
-        }
-        __syncthreads();
-        prefix |= sh_u[0] << shift;
-        maskbits |= 255u << shift;
-        above = sh_f[0];
-        __syncthreads();
-      }
-      keep_key = max(keep_key, prefix);
-    }
-    // ---- kept mass, then inverse-CDF sample in index order
-    const int per = (V + kThreads - 1) / kThreads;
-    const int j0 = tid * per, j1 = min(V, j0 + per);
-    float local = 0.f;
-    for (int j = j0; j < j1; ++j) {
-      const float x = srow[j];
-      if (f2key(x) >= keep_key) local += __expf(x - mx);
-    }
-    // block exclusive scan of `local`
-    float incl = local;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const float v = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += v;
-    }
-    __syncthreads();
-    if (lane == 31) red[warp] = incl;
-    __syncthreads();
-    if (warp == 0) {
-      float w = lane < kWarps ? red[lane] : 0.f;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const float v = __shfl_up_sync(0xffffffffu, w, o);
-        if (lane >= o) w += v;
-      }
-      red[lane] = w;  // inclusive warp totals
-    }
-    __syncthreads();
-    const float warp_base = warp == 0 ? 0.f : red[warp - 1];
-    const float kept = red[kWarps - 1];
-    const float excl = warp_base + incl - local;
     const uint32_t r = mix32((uint32_t)p.seed ^ mix32((uint32_t)(p.seed >> 32) + 0x9e3779b9u * (uint32_t)row) ^ mix32(p.step * 0x85ebca6bu + 1u));
     const float u = ((r >> 8) + 0.5f) * (1.0f / 16777216.0f);
-    const float target = u * kept;
-    if (tid == 0) sh_u[2] = 0xffffffffu;
-    __syncthreads();
-    if (local > 0.f && target >= excl && target < excl + local) {
-      float c = excl;
-      int pick = -1;
-      for (int j = j0; j < j1; ++j) {
-        const float x = srow[j];
-        if (f2key(x) >= keep_key) {
-          c += __expf(x - mx);
-          pick = j;
-          if (target < c) break;
+    bool done = false;
+    if (p.top_k < V && p.top_k <= kFastTopK) {
+      // ---- candidates: elements that reach the k-th largest thread maximum, in index order
+      const uint32_t mine[1] = {kmax};
+      const uint32_t t0 = kth_largest(mine, p.top_k);
+      uint32_t n_w = 0;
+      for (int j = w0 + lane; j - lane < w1; j += 32) n_w += __popc(__ballot_sync(0xffffffffu, j < w1 && f2key(srow[j]) >= t0));
+      __syncthreads();
+      if (lane == 0) sh.redu[warp] = n_w;
+      __syncthreads();
+      uint32_t base = 0, n_cand = 0;
+      for (int w = 0; w < kWarps; ++w) { const uint32_t c = sh.redu[w]; base += w < warp ? c : 0u; n_cand += c; }
+      if (n_cand <= kMaxCand) {
+        for (int j = w0 + lane; j - lane < w1; j += 32) {
+          const float x = j < w1 ? srow[j] : 0.f;
+          const bool in = j < w1 && f2key(x) >= t0;
+          const unsigned b = __ballot_sync(0xffffffffu, in);
+          if (in) {
+            const uint32_t at = base + __popc(b & ((1u << lane) - 1u));
+            sh.cand[at] = x;
+            sh.cand_idx[at] = j;
+          }
+          base += __popc(b);
+        }
+        __syncthreads();
+        // ---- the exact k-th largest (two candidates a thread, consecutive ones), then the top-k set in index order
+        const int c0 = 2 * tid;
+        uint32_t key[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) key[i] = c0 + i < (int)n_cand ? f2key(sh.cand[c0 + i]) : 0u;
+        keep_key = kth_largest(key, p.top_k);
+        uint32_t n_kept;
+        const bool in0 = c0 < (int)n_cand && key[0] >= keep_key, in1 = c0 + 1 < (int)n_cand && key[1] >= keep_key;
+        uint32_t at = block_inclusive((uint32_t)in0 + (uint32_t)in1, sh.redu, n_kept) - in0 - in1;
+        if (n_kept <= kMaxKept) {
+#pragma unroll
+          for (int i = 0; i < 2; ++i)
+            if (i == 0 ? in0 : in1) {
+              sh.kept[at] = sh.cand[c0 + i];
+              sh.kept_idx[at] = sh.cand_idx[c0 + i];
+              sh.kept_e[at] = __expf(sh.cand[c0 + i] - mx);
+              ++at;
+            }
+          __syncthreads();
+          const bool have = tid < (int)n_kept;
+          const float x = have ? sh.kept[tid] : 0.f;
+          float e = have ? sh.kept_e[tid] : 0.f;
+          if (p.top_p < 1.f) {
+            const float P = p.top_p * rb::block_reduce<false>(e, sh.red);
+            const uint32_t k = f2key(x);
+            float larger = 0.f;
+            if (have)
+              for (int j = 0; j < (int)n_kept; ++j) larger += f2key(sh.kept[j]) > k ? sh.kept_e[j] : 0.f;
+            const bool in = have && larger < P;
+            // the smallest kept key (a key is kept together with all larger ones)
+            uint32_t lowest = in ? k : 0xffffffffu;
+            for (int o = 16; o > 0; o >>= 1) lowest = min(lowest, __shfl_xor_sync(0xffffffffu, lowest, o));
+            __syncthreads();
+            if (lane == 0) sh.redu[warp] = lowest;
+            __syncthreads();
+            lowest = sh.redu[lane];
+            for (int o = 16; o > 0; o >>= 1) lowest = min(lowest, __shfl_xor_sync(0xffffffffu, lowest, o));
+            if (lowest != 0xffffffffu) keep_key = max(keep_key, lowest);
+            if (!(have && k >= keep_key)) e = 0.f;
+          }
+          // ---- inverse CDF over the kept elements
+          float kept;
+          const float incl = block_inclusive(e, sh.red, kept);
+          const float target = u * kept;
+          if (tid == 0) { sh.u[2] = 0xffffffffu; sh.u[3] = 0; }
+          __syncthreads();
+          if (e > 0.f && target < incl) atomicMin(&sh.u[2], (uint32_t)tid);
+          if (have && f2key(x) >= keep_key) atomicMax(&sh.u[3], (uint32_t)tid);       // rounding at the very end of the CDF: the last kept one
+          __syncthreads();
+          const uint32_t pick = sh.u[2] == 0xffffffffu ? sh.u[3] : sh.u[2];
+          chosen = sh.kept_idx[pick];
+          chosen_lp = sh.kept[pick] - mx - __logf(kept);
+          done = true;
         }
       }
-      atomicMin(&sh_u[2], (uint32_t)pick);
     }
-    __syncthreads();
-    if (sh_u[2] == 0xffffffffu) {  // rounding at the very end of the CDF: take the last kept element
-      int last = -1;
-      for (int j = j1 - 1; j >= j0; --j) if (f2key(srow[j]) >= keep_key) { last = j; break; }
-      if (tid == 0) sh_u[3] = 0;
+    if (!done) {
+      // ---- top-k: k-th largest key by radix descent
+      uint32_t prefix = 0, maskbits = 0;
+      keep_key = 0;
+      if (p.top_k < V) {
+        uint32_t remaining = (uint32_t)p.top_k;
+        for (int pass = 0; pass < 4; ++pass) {
+          const int shift = 24 - 8 * pass;
+          __syncthreads();
+          if (tid < 256) sh.hist[tid] = 0;
+          __syncthreads();
+          for (int j = tid; j < V; j += kThreads) {
+            const uint32_t k = f2key(srow[j]);
+            if ((k & maskbits) == prefix) atomicAdd(&sh.hist[(k >> shift) & 255u], 1u);
+          }
+          __syncthreads();
+          if (warp == 0) find_bin<uint32_t>(sh.hist, 0u, remaining, &sh.u[0], &sh.u[1]);
+          __syncthreads();
+          prefix |= sh.u[0] << shift;
+          maskbits |= 255u << shift;
+          remaining -= sh.u[1];
+        }
+        keep_key = prefix;
+      }
+      // ---- softmax mass of the top-k set
+      float tot = 0.f;
+      for (int j = tid; j < V; j += kThreads) {
+        const float x = srow[j];
+        if (f2key(x) >= keep_key) tot += __expf(x - mx);
+      }
+      tot = rb::block_reduce<false>(tot, sh.red);
+      // ---- top-p: weighted radix descent inside the top-k set
+      if (p.top_p < 1.f) {
+        const float P = p.top_p * tot;
+        float above = 0.f;
+        prefix = 0; maskbits = 0;
+        for (int pass = 0; pass < 4; ++pass) {
+          const int shift = 24 - 8 * pass;
+          __syncthreads();
+          if (tid < 256) sh.histm[tid] = 0.f;
+          __syncthreads();
+          for (int j = tid; j < V; j += kThreads) {
+            const float x = srow[j];
+            const uint32_t k = f2key(x);
+            if (k >= keep_key && (k & maskbits) == prefix) atomicAdd(&sh.histm[(k >> shift) & 255u], __expf(x - mx));
+          }
+          __syncthreads();
+          if (warp == 0) find_bin<float>(sh.histm, above, P, &sh.u[0], &sh.f[0]);
+          __syncthreads();
+          prefix |= sh.u[0] << shift;
+          maskbits |= 255u << shift;
+          above = sh.f[0];
+        }
+        keep_key = max(keep_key, prefix);
+      }
+      // ---- kept mass per warp range, then inverse-CDF sample in index order: the range that holds the target is searched by its warp
+      float local = 0.f;
+      for (int j = w0 + lane; j < w1; j += 32) {
+        const float x = srow[j];
+        if (f2key(x) >= keep_key) local += __expf(x - mx);
+      }
+      local = rb::warp_sum(local);
       __syncthreads();
-      if (last >= 0) atomicMax(&sh_u[3], (uint32_t)last);
+      if (lane == 0) sh.red[warp] = local;
+      if (tid == 0) { sh.u[2] = 0xffffffffu; sh.u[3] = 0; }
       __syncthreads();
-      chosen = sh_u[3];
-    } else {
-      chosen = sh_u[2];
+      float before = 0.f, kept = 0.f;
+      for (int w = 0; w < kWarps; ++w) { if (w == warp) before = kept; kept += sh.red[w]; }
+      const float target = u * kept;
+      if (local > 0.f) {
+        const bool here = target >= before && target < before + local;
+        float c = before;
+        int pick = -1, last = -1;
+        for (int j0 = w0; j0 < w1; j0 += 32) {
+          const int j = j0 + lane;
+          const bool in = j < w1 && f2key(srow[j]) >= keep_key;
+          const unsigned b = __ballot_sync(0xffffffffu, in);
+          if (b) last = j0 + 31 - __clz(b);
+          if (here && pick < 0 && b) {
+            float incl = in ? __expf(srow[j] - mx) : 0.f;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+              const float x = __shfl_up_sync(0xffffffffu, incl, o);
+              if (lane >= o) incl += x;
+            }
+            const unsigned hit = __ballot_sync(0xffffffffu, in && target < c + incl);
+            if (hit) pick = j0 + __ffs(hit) - 1;
+            c += __shfl_sync(0xffffffffu, incl, 31);
+          }
+        }
+        if (lane == 0) {
+          if (here) atomicMin(&sh.u[2], (uint32_t)(pick >= 0 ? pick : last));
+          atomicMax(&sh.u[3], (uint32_t)last);      // rounding at the very end of the CDF: the last kept element
+        }
+      }
+      __syncthreads();
+      chosen = sh.u[2] == 0xffffffffu ? sh.u[3] : sh.u[2];
+      chosen_lp = srow[chosen] - mx - __logf(kept);
     }
-    chosen_lp = srow[chosen] - mx - __logf(kept);
   }
 
   const bool live = p.unfinished == nullptr || p.unfinished[row];
@@ -254,16 +407,25 @@ __global__ void __launch_bounds__(kThreads, 1) sample_kernel(SampleParams p) {
     }
   }
   if (p.mask_bits != nullptr) {
+    // 32 elements a ballot, 1024 a warp and round: lane i ends up with the i-th word of the round
     uint8_t* mrow = p.mask_bits + (int64_t)row * p.mask_stride;
     const int nbytes = (V + 7) / 8;
-    for (int b = tid; b < nbytes; b += kThreads) {
-      uint32_t bits = 0;
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int j = b * 8 + i;
-        if (j < V && f2key(srow[j]) < keep_key) bits |= 1u << i;
+    const bool words = (reinterpret_cast<uintptr_t>(mrow) & 3) == 0;
+    for (int j0 = warp * 1024; j0 < V; j0 += kThreads * 32) {
+      uint32_t word = 0;
+#pragma unroll 8
+      for (int i = 0; i < 32; ++i) {
+        const int j = j0 + i * 32 + lane;
+        const unsigned b = __ballot_sync(0xffffffffu, j < V && f2key(srow[j]) < keep_key);
+        if (lane == i) word = b;
       }
-      mrow[b] = (uint8_t)bits;
+      const int byte = j0 / 8 + lane * 4;
+      if (words && byte + 4 <= nbytes) {
+        *reinterpret_cast<uint32_t*>(mrow + byte) = word;
+      } else {
+        for (int i = 0; i < 4; ++i)
+          if (byte + i < nbytes) mrow[byte + i] = (uint8_t)(word >> (8 * i));
+      }
     }
   }
 }

@@ -109,3 +109,32 @@ def test_in_graph_sampling_matches_eager_decode_loop(greedy, monkeypatch):
         torch.testing.assert_close(a.logprobs[i, :n], lp_ref, atol=0.08, rtol=0.05)  # bf16 decode vs packed forward
         assert (a.tokens[i, :min(n, 6) - 1] != 2).all()          # EOS suppressed before min_new_tokens
         assert (a.tokens[i, n:] == 0).all() and (a.logprobs[i, n:] == 0).all()  # padding after EOS
+
+
+@pytest.mark.parametrize("V,top_k,top_p", [(97, 96, 0.5), (2048, 256, 0.9), (4099, 1, 1.0), (32000, 512, 0.95), (32003, 513, 0.8), (50257, 50, 0.9),
+                                           (51200, 200, 1.0), (8192, 8192, 0.7)])
+@pytest.mark.parametrize("ties", [False, True])
+def test_sample_thresholds_at_the_edges_of_the_candidate_path(V, top_k, top_p, ties):
+    """Kept set, draw and log-prob against float64 at both sides of the top_k limit, with unaligned rows and with tie groups that overflow
+    the candidate list.  The mask may differ only where the mass above an element is within fp32 rounding of top_p (1e-5 of the total)."""
+    torch.manual_seed(V + top_k)
+    B = 6
+    x = torch.randn(B, V, device=DEV) * 2.0
+    if ties:
+        x = (x * 2).round() / 2                      # a few dozen values: tie groups of hundreds to thousands of elements
+    tok, lp, mb = lib().sample(x, None, top_k, top_p, 1.0, -1, False, False, 0, 77, 3, True)
+    xd = x.double()
+    kth = torch.topk(xd, min(top_k, V), -1).values[:, -1:]
+    p = torch.softmax(xd.masked_fill(xd < kth, float("-inf")), -1)
+    srt, idx = torch.sort(xd, -1, descending=True)
+    before = p.gather(1, idx).cumsum(-1) - p.gather(1, idx)
+    first = torch.searchsorted(-srt, -srt)           # equal logits share the mass above the first of them
+    above = torch.zeros_like(p).scatter_(1, idx, before.gather(1, first))
+    keep = (p > 0) & ((above < top_p) if top_p < 1 else torch.ones_like(above, dtype=torch.bool))
+    removed = OF.unpack_mask_bits(mb, V)
+    sure = (above - top_p).abs() > 1e-5
+    assert torch.equal(removed[sure | (p == 0)], ~keep[sure | (p == 0)])
+    rows = torch.arange(B, device=DEV)
+    assert not removed[rows, tok].any()
+    ref = torch.log_softmax(xd.masked_fill(removed, float("-inf")), -1)[rows, tok]
+    torch.testing.assert_close(lp.double(), ref, atol=2e-5, rtol=1e-5)
