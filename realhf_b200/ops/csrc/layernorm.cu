@@ -4,7 +4,7 @@
 // Replaces `F.layer_norm` (reference: torch.nn.LayerNorm in modules/mlp.py:56-62).
 //
 // STATUS: compiled for sm_100a, not yet run on hardware: opt-in (`REAL_LAYERNORM=native`), test gated by REAL_TEST_EXPERIMENTAL=1.
-#include "common.cuh"
+#include "colsum.cuh"
 
 namespace {
 
@@ -139,15 +139,6 @@ __global__ void __launch_bounds__(2 * kLnThreads) layernorm_bwd_kernel(const T* 
   }
 }
 
-template <typename T>
-__global__ void ln_colsum_kernel(const float* __restrict__ partial, T* __restrict__ out, int n_part, int H) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= H) return;
-  float acc = 0.f;
-  for (int p = 0; p < n_part; ++p) acc += partial[(int64_t)p * H + c];
-  out[c] = rb::from_f<T>(acc);
-}
-
 }  // namespace
 
 extern "C" {
@@ -182,8 +173,8 @@ int rb_layernorm_bwd(const void* x, const void* w, const void* dy, const float* 
 #define RB_L(T)                                                                                      \
   { const int nv = RB_CEIL_DIV(H, 2 * kLnThreads * 8);                                                \
     if (nv <= 1) { RB_L2(T, 1) } else if (nv <= 2) { RB_L2(T, 2) } else { RB_L2(T, 4) }              \
-    ln_colsum_kernel<T><<<RB_CEIL_DIV(H, 256), 256, 0, s>>>(dw_partial, (T*)dw, grid, H);           \
-    if (db) ln_colsum_kernel<T><<<RB_CEIL_DIV(H, 256), 256, 0, s>>>(db_partial, (T*)db, grid, H); }
+    rb::launch_colsum<T>(dw_partial, dw, grid, H, s);                                                 \
+    if (db) rb::launch_colsum<T>(db_partial, db, grid, H, s); }
   if (dt == 0) { RB_L(float) } else if (dt == 1) { RB_L(__nv_bfloat16) } else if (dt == 2) { RB_L(__half) } else return -1;
 #undef RB_L
 #undef RB_L2

@@ -3,9 +3,9 @@
 // Forward: one CTA (128 threads) per token row; the row stays in registers between the
 // sum-of-squares pass and the scale pass, so HBM traffic is exactly read-x (+read-residual) and
 // write-y (+write-residual).  Backward: persistent CTAs walk rows, produce dx and keep the weight
-// gradient in registers; per-CTA partials are reduced by a second tiny kernel.
+// gradient in registers; per-CTA partials are reduced by a second tiny kernel (colsum.cuh).
 // Replaces the eager fp32-upcast RMSNorm of the reference (modules/mlp.py:425-467).
-#include "common.cuh"
+#include "colsum.cuh"
 
 namespace {
 
@@ -65,84 +65,145 @@ __global__ void __launch_bounds__(kThreads) rmsnorm_fwd_kernel(const T* __restri
   }
 }
 
-// dx = rstd * (g - xhat * mean(g*xhat)),  g = dy * (w + off);  dw += dy * xhat
-template <typename T, int kMaxVec>
-__global__ void __launch_bounds__(2 * kThreads) rmsnorm_bwd_kernel(const T* __restrict__ x, const T* __restrict__ w,
-                                                               const T* __restrict__ dy, const float* __restrict__ rstd,
-                                                               T* __restrict__ dx, float* __restrict__ dw_partial,
-                                                               int64_t T_rows, int H, float w_offset,
-                                                               const T* __restrict__ dres) {
-  __shared__ float red[32];
-  constexpr int V = 8;
-  const int nvec = H / V;
-  float dw[kMaxVec][V];
-  float wv[kMaxVec][V];
+// dx = rstd * (g - xhat * mean(g*xhat)) (+ dres),  g = dy * (w + off);  dw += dy * xhat
+//
+// Bound by HBM: x, dy (and the gradient arriving on the residual stream, `dres`) in, dx out.  A row is one reduction deep, so a CTA that
+// loads, reduces and stores row after row leaves the memory idle for most of each row (20480 x 4096 bf16 with dres: 220 us, 3.0 TB/s; with
+// one row prefetched into registers 192 us).  Every thread therefore keeps the pieces of kStages rows in flight with cp.async, into
+// shared memory only it reads back (no barrier, no wait on another thread), and the reduction takes one barrier (two alternating sets of
+// warp sums).  ~190 KB of rows are in flight per SM at every width.
+template <typename T, int TB, int NV> struct RmsBwd {
+  static constexpr int kPieces = 8 * sizeof(T) / 16;                 // 16-byte pieces of a thread's 8 elements
+  static constexpr int kStageBytes = 3 * NV * TB * 8 * (int)sizeof(T);
+  static constexpr int kStages = kStageBytes > 48 * 1024 ? 2 : 4;
+  static constexpr int kSmem = kStages * kStageBytes;
+  static constexpr int kFit = 200 * 1024 / kSmem, kCtas = kFit > 4 ? 4 : kFit;   // 4: the partial sums have 4 rows per SM
+};
+
+RB_DEVICE void cp_async16(uint32_t dst, const void* src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory"); }
+RB_DEVICE void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> RB_DEVICE void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+template <typename T, int TB, int NV>
+__global__ void __launch_bounds__(TB, RmsBwd<T, TB, NV>::kCtas)
+    rmsnorm_bwd_kernel(const T* __restrict__ x, const T* __restrict__ w, const T* __restrict__ dy, const float* __restrict__ rstd, T* __restrict__ dx,
+                       float* __restrict__ dw_partial, int64_t T_rows, int H, float w_offset, const T* __restrict__ dres) {
+  using C = RmsBwd<T, TB, NV>;
+  constexpr int V = 8, kWarps = TB / 32, P = C::kPieces;
+  using Vec = rb::Pack<T, V>;
+  extern __shared__ uint4 ring[];       // [kStages][3 operands][NV][P][TB]
+  __shared__ float red[2][kWarps];
+  const int nvec = H / V, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const float inv_h = 1.f / (float)H;
+  float dw[NV][V];
+  Vec wv[NV];
 #pragma unroll
-  for (int it = 0; it < kMaxVec; ++it) {
-    const int i = threadIdx.x + it * 2 * kThreads;
+  for (int it = 0; it < NV; ++it) {
+    const int i = threadIdx.x + it * TB;
 #pragma unroll
     for (int k = 0; k < V; ++k) dw[it][k] = 0.f;
-    if (i < nvec) {
-      rb::Pack<T, V> ww = reinterpret_cast<const rb::Pack<T, V>*>(w)[i];
-#pragma unroll
-      for (int k = 0; k < V; ++k) wv[it][k] = rb::to_f(ww.v[k]) + w_offset;
-    }
+    if (i < nvec) wv[it] = reinterpret_cast<const Vec*>(w)[i];
   }
-  for (int64_t row = blockIdx.x; row < T_rows; row += gridDim.x) {
-    const float rs = rstd[row];
-    float xh[kMaxVec][V], g[kMaxVec][V];
+  auto slot = [&](int st, int op, int it, int q) { return ring + (((st * 3 + op) * NV + it) * P + q) * TB + threadIdx.x; };
+  auto fetch = [&](int64_t row, int st) {
+    if (row < T_rows) {
+#pragma unroll
+      for (int it = 0; it < NV; ++it) {
+        const int i = threadIdx.x + it * TB;
+        if (i < nvec) {
+#pragma unroll
+          for (int q = 0; q < P; ++q) {
+            const int64_t at = (row * H + (int64_t)i * V) + q * (V / P);
+            cp_async16((uint32_t)__cvta_generic_to_shared(slot(st, 0, it, q)), x + at);
+            cp_async16((uint32_t)__cvta_generic_to_shared(slot(st, 1, it, q)), dy + at);
+            if (dres != nullptr) cp_async16((uint32_t)__cvta_generic_to_shared(slot(st, 2, it, q)), dres + at);
+          }
+        }
+      }
+    }
+    cp_async_commit();                  // (an empty group past the end keeps the count)
+  };
+  auto take = [&](int st, int op, int it) {
+    Vec v;
+#pragma unroll
+    for (int q = 0; q < P; ++q) reinterpret_cast<uint4*>(&v)[q] = *slot(st, op, it, q);
+    return v;
+  };
+#pragma unroll
+  for (int st = 0; st < C::kStages; ++st) fetch(blockIdx.x + (int64_t)st * gridDim.x, st);
+  int par = 0, st = 0;
+  float rs_next = blockIdx.x < T_rows ? rstd[blockIdx.x] : 0.f;
+  for (int64_t row = blockIdx.x; row < T_rows; row += gridDim.x, par ^= 1) {
+    const float rs = rs_next;
+    if (row + gridDim.x < T_rows) rs_next = rstd[row + gridDim.x];
+    cp_async_wait<C::kStages - 1>();
+    Vec a[NV], d[NV], e[NV];
     float dot = 0.f;
 #pragma unroll
-    for (int it = 0; it < kMaxVec; ++it) {
-      const int i = threadIdx.x + it * 2 * kThreads;
-      if (i < nvec) {
-        rb::Pack<T, V> a = reinterpret_cast<const rb::Pack<T, V>*>(x + row * H)[i];
-        rb::Pack<T, V> d = reinterpret_cast<const rb::Pack<T, V>*>(dy + row * H)[i];
+    for (int it = 0; it < NV; ++it) {
+      if (threadIdx.x + it * TB < nvec) {
+        a[it] = take(st, 0, it);
+        d[it] = take(st, 1, it);
+        if (dres != nullptr) e[it] = take(st, 2, it);
 #pragma unroll
         for (int k = 0; k < V; ++k) {
-          xh[it][k] = rb::to_f(a.v[k]) * rs;
-          const float dyk = rb::to_f(d.v[k]);
-          g[it][k] = dyk * wv[it][k];
-          dw[it][k] = fmaf(dyk, xh[it][k], dw[it][k]);
-          dot = fmaf(g[it][k], xh[it][k], dot);
+          const float xh = rb::to_f(a[it].v[k]) * rs, dyk = rb::to_f(d[it].v[k]);
+          dw[it][k] = fmaf(dyk, xh, dw[it][k]);
+          dot = fmaf(dyk * (rb::to_f(wv[it].v[k]) + w_offset), xh, dot);
         }
       }
     }
-    dot = rb::block_reduce<false>(dot, red) / (float)H;
+    dot = rb::warp_sum(dot);
+    if (lane == 0) red[par][warp] = dot;
+    __syncthreads();     // (the other set is rewritten only behind the next row's barrier)
+    fetch(row + (int64_t)C::kStages * gridDim.x, st);
+    st = st + 1 == C::kStages ? 0 : st + 1;
+    dot = 0.f;
 #pragma unroll
-    for (int it = 0; it < kMaxVec; ++it) {
-      const int i = threadIdx.x + it * 2 * kThreads;
+    for (int k = 0; k < kWarps; ++k) dot += red[par][k];
+    dot *= inv_h;
+#pragma unroll
+    for (int it = 0; it < NV; ++it) {
+      const int i = threadIdx.x + it * TB;
       if (i < nvec) {
-        rb::Pack<T, V> o;
-        if (dres != nullptr) {  // fused residual add in training: the gradient arriving on the residual stream joins here
-          rb::Pack<T, V> e = reinterpret_cast<const rb::Pack<T, V>*>(dres + row * H)[i];
+        Vec o;
 #pragma unroll
-          for (int k = 0; k < V; ++k) o.v[k] = rb::from_f<T>(rs * (g[it][k] - xh[it][k] * dot) + rb::to_f(e.v[k]));
-        } else {
-#pragma unroll
-          for (int k = 0; k < V; ++k) o.v[k] = rb::from_f<T>(rs * (g[it][k] - xh[it][k] * dot));
+        for (int k = 0; k < V; ++k) {
+          const float xh = rb::to_f(a[it].v[k]) * rs, g = rb::to_f(d[it].v[k]) * (rb::to_f(wv[it].v[k]) + w_offset);
+          float v = rs * (g - xh * dot);
+          if (dres != nullptr) v += rb::to_f(e[it].v[k]);
+          o.v[k] = rb::from_f<T>(v);
         }
-        reinterpret_cast<rb::Pack<T, V>*>(dx + row * H)[i] = o;
+        reinterpret_cast<Vec*>(dx + row * H)[i] = o;
       }
     }
   }
 #pragma unroll
-  for (int it = 0; it < kMaxVec; ++it) {
-    const int i = threadIdx.x + it * 2 * kThreads;
+  for (int it = 0; it < NV; ++it) {
+    const int i = threadIdx.x + it * TB;
     if (i < nvec) {
 #pragma unroll
-      for (int k = 0; k < V; ++k) dw_partial[(int64_t)blockIdx.x * H + i * V + k] = dw[it][k];
+      for (int k = 0; k < V; k += 4)
+        *reinterpret_cast<float4*>(dw_partial + (int64_t)blockIdx.x * H + i * V + k) = make_float4(dw[it][k], dw[it][k + 1], dw[it][k + 2], dw[it][k + 3]);
     }
   }
 }
 
-template <typename T>
-__global__ void colsum_kernel(const float* __restrict__ partial, T* __restrict__ out, int n_part, int H) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= H) return;
-  float acc = 0.f;
-  for (int p = 0; p < n_part; ++p) acc += partial[(int64_t)p * H + c];
-  out[c] = rb::from_f<T>(acc);
+template <typename T, int TB, int NV>
+int launch_rmsnorm_bwd(const void* x, const void* w, const void* dy, const float* rstd, void* dx, float* dw_partial, void* dw, int64_t rows, int H,
+                       float w_offset, const void* dres, cudaStream_t s) {
+  using C = RmsBwd<T, TB, NV>;
+  auto kern = rmsnorm_bwd_kernel<T, TB, NV>;
+  static bool attr_set = false;
+  if (!attr_set) {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmem) != cudaSuccess) return -2;
+    attr_set = true;
+  }
+  const int64_t ctas = (int64_t)rb::kNumSMs * C::kCtas;
+  const int grid = (int)(rows < ctas ? rows : ctas);
+  kern<<<grid, TB, C::kSmem, s>>>((const T*)x, (const T*)w, (const T*)dy, rstd, (T*)dx, dw_partial, rows, H, w_offset, (const T*)dres);
+  rb::launch_colsum<T>(dw_partial, dw, grid, H, s);
+  return 0;
 }
 
 }  // namespace
@@ -174,18 +235,13 @@ int rb_rmsnorm_bwd(const void* x, const void* w, const void* dy, const float* rs
                    void* dw, int64_t rows, int H, float w_offset, int dt, const void* dres, cudaStream_t s) {
   if (rows == 0) return 0;
   if (H % 8 != 0 || H > kThreads * 8 * 8) return -1;
-  const int grid = (int)(rows < rb::kNumSMs * 4 ? rows : rb::kNumSMs * 4);
-#define RB_L2(T, NV)                                                                                               \
-  rmsnorm_bwd_kernel<T, NV><<<grid, 2 * kThreads, 0, s>>>((const T*)x, (const T*)w, (const T*)dy, rstd, (T*)dx,        \
-                                                          dw_partial, rows, H, w_offset, (const T*)dres);
-#define RB_L(T)                                                            \
-  { const int nv = RB_CEIL_DIV(H, 2 * kThreads * 8);                        \
-    if (nv <= 1) { RB_L2(T, 1) } else if (nv <= 2) { RB_L2(T, 2) } else { RB_L2(T, 4) }                            \
-    colsum_kernel<T><<<RB_CEIL_DIV(H, 256), 256, 0, s>>>(dw_partial, (T*)dw, grid, H); }
+  // 128 threads up to 1024 columns (a thread's 8 columns once), 256 beyond
+#define RB_L2(T, TB, NV) return launch_rmsnorm_bwd<T, TB, NV>(x, w, dy, rstd, dx, dw_partial, dw, rows, H, w_offset, dres, s)
+#define RB_L(T)                                                                                                       \
+  { if (H <= 1024) RB_L2(T, 128, 1); if (H <= 2048) RB_L2(T, 256, 1); if (H <= 4096) RB_L2(T, 256, 2); RB_L2(T, 256, 4); }
   if (dt == 0) { RB_L(float) } else if (dt == 1) { RB_L(__nv_bfloat16) } else if (dt == 2) { RB_L(__half) } else return -1;
 #undef RB_L
 #undef RB_L2
-  return 0;
 }
 
 }  // extern "C"

@@ -3,6 +3,7 @@ import pytest
 import torch
 
 from realhf_b200.ops import functional as OF
+from realhf_b200.ops import lib
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
@@ -279,3 +280,25 @@ def test_layernorm_native_matches_reference(H, dtype, monkeypatch):
     torch.testing.assert_close(x.grad.float(), xr.grad, **tol)
     torch.testing.assert_close(w.grad.float(), wr.grad, atol=tol["atol"] * 20, rtol=tol["rtol"])
     torch.testing.assert_close(b.grad.float(), br.grad, atol=tol["atol"] * 20, rtol=tol["rtol"])
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("rows,H", [(1, 8), (3, 1024), (593, 1032), (1500, 2048), (149, 2056), (2400, 4096), (37, 4104), (700, 8192)])
+@pytest.mark.parametrize("with_dres", [False, True])
+def test_rmsnorm_bwd_row_rings(dtype, rows, H, with_dres):
+    """The backward kernel against float64 where its rings of rows wrap, end early or stay empty, at the edges of its widths.  dx is one rounding of a
+    sum of three terms (each rounded in fp32), dw an fp32 sum over the rows rounded once."""
+    torch.manual_seed(rows + H)
+    x, dy, dres = (torch.randn(rows, H, device=DEV).to(dtype) for _ in range(3))
+    w = (1 + 0.1 * torch.randn(H, device=DEV)).to(dtype)
+    y, rstd = lib().rmsnorm_fwd(x, None, w, 1e-5, 0.5)[:2]
+    dx, dw = lib().rmsnorm_bwd(x, w, dy, rstd, 0.5, dres if with_dres else None)
+    xd, wd = x.double(), w.double() + 0.5
+    r = torch.rsqrt(xd.pow(2).mean(-1, keepdim=True) + 1e-5)
+    xh, g = xd * r, dy.double() * wd
+    rdx = r * (g - xh * (g * xh).mean(-1, keepdim=True)) + (dres.double() if with_dres else 0.0)
+    rdw = (dy.double() * xh).sum(0)
+    eps = {torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11, torch.float32: 2.0 ** -20}[dtype]
+    mag = r * (g.abs() + xh.abs() * (g * xh).abs().mean(-1, keepdim=True)) + (dres.double().abs() if with_dres else 0.0)
+    assert ((dx.double() - rdx).abs() <= eps * rdx.abs() + 2.0 ** -20 * mag + 1e-7).all()
+    assert ((dw.double() - rdw).abs() <= eps * rdw.abs() + 2.0 ** -20 * (dy.double() * xh).abs().sum(0) + 1e-7).all()
