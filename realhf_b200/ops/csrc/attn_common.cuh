@@ -1,0 +1,73 @@
+// Pieces shared by the tcgen05 attention kernels: parameters, bounded waits, packing, the soft cap.
+#pragma once
+#include "gemm_common.cuh"
+
+namespace rb {
+
+struct AttnParams {
+  const int* cu_seqlens;  // [B + 1]
+  void* out;              // [T, nq, D]
+  float* lse;             // [nq, T]
+  int64_t out_ld;         // elements between consecutive tokens of `out`
+  int T, nq, nkv;
+  float scale;
+  int causal;
+  int window;             // > 0 (with causal): a query at position i sees keys (i - window, i]
+  // forms with a sink only
+  int keep;               // with a window: keys [0, keep) stay visible to every later query
+  const void* temp;       // [nq] per-head factor on the scaled score, or null
+  const void* sink;       // [nq] per-head sink logit, or null
+  const void* gate;       // gate logits, element (t, h) at gate[t * gate_ld + h], or null
+  int64_t gate_ld;
+  float slope_base;       // < 0: no distance term
+  int vshare = 1;         // consecutive key heads that read one value head (V has nkv / vshare heads)
+  int gate_mode = 1;      // gate logits: 1 one per head, 2 one per output element (element (t, h, c) at gate[t * gate_ld + h * D + c])
+  int chunk = 0;          // > 0 (window 0): a query sees the keys of its own chunk
+  float softcap = 0.f;    // > 0: capped scores
+  const float* bias = nullptr;   // [nq, bias_ld], the first n_bias columns are used; distances beyond read the last one
+  int n_bias = 0, bias_ld = 0;
+  int B = 0, pair_heads = 0, n_head_units = 0;   // set by the launch: sequences, tile pairs over heads, work units per row block
+};
+
+}  // namespace rb
+
+namespace {
+
+using rb::AttnParams;
+
+constexpr int kMaxSmem = 227 * 1024;
+
+// Every wait is bounded: a wait that runs out sets the CTA's `dead` flag (all later waits of the CTA then return at once), and the
+// kernel ends normally after a pause that lets its own copies land; `rb_attn_wait_error` tells the host.
+constexpr int kWaitPolls = 1 << 20;
+
+RB_DEVICE void bounded_wait(uint32_t bar, uint32_t parity, volatile uint32_t* dead) {
+  for (int i = 0; !ptx::mbar_try_wait(bar, parity); ++i)
+    if (i >= kWaitPolls || *dead) { *dead = 1; return; }
+}
+
+RB_DEVICE void st_shared_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+RB_DEVICE uint4 ld_shared_v4(uint32_t addr) {
+  uint4 v;
+  asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
+  return v;
+}
+template <typename T> RB_DEVICE uint32_t pack2(float lo, float hi);
+template <> RB_DEVICE uint32_t pack2<__nv_bfloat16>(float lo, float hi) {
+  __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+  return *reinterpret_cast<uint32_t*>(&v);
+}
+template <> RB_DEVICE uint32_t pack2<__half>(float lo, float hi) {
+  __half2 v = __floats2half2_rn(lo, hi);
+  return *reinterpret_cast<uint32_t*>(&v);
+}
+
+// cap * tanh(s * scale / cap) + add in the log2 domain, tanh(x) = 1 - 2 / (1 + 2^(2 x log2 e)): c = 2 log2 e * scale / cap,
+// k = cap log2 e, k_add = k + add.  Absolute error a few ulp of k; saturates to +-k.
+RB_DEVICE float soft_cap2(float s, float c, float k, float k_add) {
+  return fmaf(-2.f * k, __fdividef(1.f, 1.f + exp2f(fminf(s * c, 80.f))), k_add);
+}
+
+}  // namespace

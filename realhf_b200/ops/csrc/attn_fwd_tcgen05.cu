@@ -2,181 +2,116 @@
 //
 //   O[t, h, :] = softmax(scale * Q[t, h, :] K[seq(t), kv(h), :]^T  (+ causal mask)) V        bf16 / fp16, fp32 softmax
 //
-// Optional sliding window (causal only): query i sees keys (i - window, i].  Key tiles that lie wholly below the window of the
-// CTA's first query row are never loaded (all three roles walk the same tile range [tile0, tile0 + n_kv)); inside the
-// remaining tiles the lower edge is a per-row column mask like the diagonal.
+// Optional sliding window (causal only): query i sees keys (i - window, i].  Reference: flash-attn's `flash_attn_varlen_func` called
+// from `impl/model/modules/attn.py:240-262`.
 //
-// Reference: flash-attn's `flash_attn_varlen_func` called from `impl/model/modules/attn.py:240-262`.  One CTA owns a
-// 128-row query tile of one (sequence, head) and walks the key / value tiles of that sequence (up to the diagonal).
+// What bounds it: per 128 x 128 tile the two products take 1024 tensor-pipe cycles at D = 128 and the 16384 exponentials as many cycles
+// of the special-function unit, so the tensor pipe is only busy while some other tile's softmax runs beside it.  A work item is therefore
+// a PAIR of 128-row query tiles over one K / V stream, each with softmax threads of its own: two query heads of one key head at the same
+// rows (grouped heads, even group: both walk the same tiles), else two neighbouring query tiles of a head (counted from the end of
+// the sequence, so that a left-over single tile is the shortest one).  Sharing the stream also halves the L2 traffic per product: one
+// tile each would ask for 64 B per cycle and SM, more than L2 gives.  With one tile per CTA and four softmax warps the tensor pipe was
+// active 19% of the time: 32 x 640 tokens x 32 heads took 527 us (now 294), 8 x 1500..4096 x 32 / 8 heads 2396 us (now 1023).
 //
-// CTA = 6 warps.  warp 0: TMA producer (Q once, then K_j / V_j into two-stage rings; K and V have their own barriers so a K
-// stage is recycled as soon as S_j = Q K_j^T retired, before P_j V_j even started).  warp 1: MMA issuer + TMEM allocator.
-// warps 2-5: softmax, one thread per query row (thread <-> TMEM lane), no cross-thread reductions.
+// CTA = 12 warps, one CTA per SM.  Warps 0-3 / 4-7: softmax of tile 0 / 1 (thread = query row = TMEM lane).  Warp 8: MMA issue and TMEM
+// allocation.  Warp 9: TMA producer and scheduler (10, 11: idle, they complete the warpgroup whose registers go to the softmax).  The
+// grid holds one CTA per work item (a bound: sequence lengths are on the device); a running CTA takes the items of CTAs that have
+// not started (`clusterlaunchcontrol.try_cancel`), so barriers, TMEM and descriptors are set up once per SM, the next item's Q / K / V
+// load while the last one's softmax and output run, and ragged batches balance themselves.
 //
-// Tensor memory (512 columns): S double buffer [0,128) [128,256) and a double buffer for the per-tile product
-// T_j = P_j V_j at [256,256+D) [384,384+D).  The running output stays in registers: O <- O * alpha_j + T_j with
-// alpha_j = exp2((m_{j-1} - m_j) * scale * log2 e); accumulating per tile in TMEM and folding in registers costs one
-// tcgen05.ld of T_j but no TMEM read-modify-write of O when the row maximum moves.  Issue order on the tensor pipe is
-// S_0, S_1, PV_0, S_2, PV_1, ...: S_{j+1} is in flight while the softmax warps work on S_j, and the fold of T_{j-1} happens
-// after P_j has been handed to the MMA warp, so it overlaps PV_j.
+// Tensor memory (512 columns): S_t at 128 t, O_t at 256 + 128 t.  P_t (16 bit) overwrites the front of S_t and is the TMEM A operand of
+// P V, so it never travels through shared memory; S_t of the next tile is issued behind that product on the in-order tensor pipe.  O
+// accumulates in TMEM over the whole stream.  The row maximum that weights are taken against only moves when a tile's maximum exceeds it
+// by more than 2^8 (then the warp scales O once the product in flight has retired): weights, sum and output carry the same factor, so the
+// result is the softmax of the same scores, and fp32 / bf16 / fp16 all have room for 2^8.  V_j is the MN-major B operand.
+// Issue order: S_0, S_1, then per key tile PV_0, S_0', PV_1, S_1'.
 //
-// P_j is written by the softmax threads as bf16 straight into the canonical K-major SWIZZLE_128B layout (the same bytes a
-// TMA load of a [128 x 64] box would produce), fenced into the async proxy and consumed as the A operand of PV_j; V_j is
-// the MN-major B operand (keys are the K dimension, head-dim contiguous), exactly the wgrad operand form of the GEMM.
+// Outputs: O [T, nq, DV] through a per-warp staging buffer (whole 128-byte lines), LSE [nq, T] (natural log, scale applied).
 //
-// Outputs: O [T, nq, D] and LSE [nq, T] (natural log, scale applied) in the layout flash-attn's backward consumes.
-//
-// kSink variant (`WindowAttentionConfig`, inference only, no LSE): score = s * scale * temp_h - slope_h * (i - j) with
-// slope_h = 2^(-slope_base (h + 1) / nq) (formed per element in the log2 domain with one extra FMA in each pass), a sliding
-// window that also keeps the first `keep` keys (the key tiles of [0, keep) that lie below the window's first tile are walked
-// first by all three roles), a per-head sink logit that starts the running maximum with denominator 1, and the row's output
-// times sigmoid(gate logit of its head, or of the output element).  `chunk` > 0 replaces the window: a query sees the keys of its own
-// chunk of positions up to itself (the tiles below the first row's chunk are not walked, a later row's chunk start is its lower
-// mask edge).  kSimple: no distance term, no temperature, no kept first keys and a positive scale: the row maximum is taken over the raw
-// products and scaled once, a weight costs one FMA and one exp2, the mask one comparison.  kCap (kSimple only): score = softcap *
-// tanh(s * scale / softcap); the cap is monotone, so the raw maximum is capped once, and only the pass that forms the weights
-// evaluates tanh per element.  kBias: score = s * scale * temp_h + bias_h(i - j), a learned number per head and distance.  The head's
-// table (times log2 e) is staged in shared memory with 127 entries in front (distances of masked columns) and its last value
-// repeated behind: a row's column c then reads entry (distance of the row's first column) - c, i.e. one base address per row and tile
-// and an immediate offset per column, and the 32 rows of a warp read 32 consecutive entries.  Tiles beyond the table start in its
-// constant tail.  kShared: the values are the keys.  Only K tiles travel; the MN-major operand of P V is the K tile read in the other
-// major-ness (its 64-wide chunks of the head lie kBKV rows apart), so a stage is recycled after P V instead of after S, and the
-// shared memory that V would take holds two more stages.  Query / key size kD and value size kDV may differ.
-#include "gemm_common.cuh"
+// Modes (`WindowAttentionConfig`, inference only, no LSE): kGeneral: score = s * scale * temp_h - slope_h * (i - j) with slope_h =
+// 2^(-slope_base (h + 1) / nq) (log2 domain, two FMAs per score), a sliding window that also keeps the first `keep` keys (their
+// tiles below the window's first tile are walked first).  kSimple: no distance term, temperature or kept keys and a positive scale: the
+// maximum is taken over the raw products.  kCap: kSimple with score = softcap * tanh(s * scale / softcap); the cap is monotone, so the
+// raw maximum is capped once.  All three: a per-head sink logit starts the running maximum with denominator 1; the output is
+// multiplied by sigmoid(gate logit of its head, or of the output element); `chunk` > 0 replaces the window: a query sees the keys of its own
+// chunk of positions up to itself.  (32 x 1024 tokens, 16 / 4 heads, window 512 + 64 kept: 1382 us with one tile per CTA, now 316.)
+// Learned distance biases and shared keys / values run in attn_fwd_bias.cu.
+#include "attn_common.cuh"
 
 namespace {
 
-constexpr int kBQ = 128;   // query rows per CTA (= UMMA M)
-constexpr int kBKV = 128;  // keys per tile (= UMMA N of S, K of PV)
-constexpr int kAttnThreads = 192;
+constexpr int kTile = 128;          // query rows of a tile (= UMMA M) and keys of a tile (= UMMA N of S, K of P V)
+constexpr int kFwdThreads = 384;    // three warpgroups: 168 registers a thread at launch, 64512 in all
+constexpr int kSoftmaxRegs = 208, kOtherRegs = 80;   // 2 x 128 x 208 + 128 x 80 = 63488: a softmax thread holds a whole score row
+constexpr int kStages = 4;          // K and V tiles share one ring: two key tiles in flight
+constexpr float kLazy = 8.f;        // log2 of how far weights may exceed 1 before the maximum moves
 
-struct AttnParams {
-  const int* cu_seqlens;  // [B + 1]
-  void* out;              // [T, nq, D]
-  float* lse;             // [nq, T]
-  int64_t out_ld;         // elements between consecutive tokens of `out`
-  int T, nq, nkv;
-  float scale;
-  int causal;
-  int window;             // > 0 (with causal): a query at position i sees keys (i - window, i]
-  // kSink variant only
-  int keep;               // with a window: keys [0, keep) stay visible to every later query
-  const void* temp;       // [nq] per-head factor on the scaled score, or null
-  const void* sink;       // [nq] per-head sink logit, or null
-  const void* gate;       // gate logits, element (t, h) at gate[t * gate_ld + h], or null
-  int64_t gate_ld;
-  float slope_base;       // < 0: no distance term
-  int vshare = 1;         // consecutive key heads that read one value head (V has nkv / vshare heads)
-  int gate_mode = 1;      // gate logits: 1 one per head, 2 one per output element (element (t, h, c) at gate[t * gate_ld + h * D + c])
-  int chunk = 0;          // > 0 (window 0): a query sees the keys of its own chunk
-  float softcap = 0.f;    // kCap variant
-  const float* bias = nullptr;   // kBias variant: [nq, bias_ld], the first n_bias columns are used; distances beyond read the last one
-  int n_bias = 0, bias_ld = 0;
+enum Mode { kPlain = 0, kSimple = 1, kCap = 2, kGeneral = 3 };
+
+template <int kD, int kDV> struct FCfg {
+  static constexpr int kQBytes = kTile * kD * 2, kKBytes = kTile * kD * 2, kVBytes = kTile * kDV * 2;
+  static constexpr int kStageBytes = kKBytes > kVBytes ? kKBytes : kVBytes;
+  static constexpr int kKV = 2 * kQBytes, kOut = kKV + kStages * kStageBytes, kBars = kOut + 8 * 4096;
+  static constexpr int kSmemBytes = kBars + 1024 /*align*/ + 512 /*barriers, items*/;
 };
 
-template <int kD, int kDV, bool kShared> struct ACfg {
-  static constexpr int kDBlocks = kD / 64, kDVBlocks = kDV / 64;   // 64-element (128 B) column blocks of Q / K and of V
-  static constexpr int kQBytes = kBQ * kD * 2;
-  static constexpr int kKBytes = kBKV * kD * 2, kVBytes = kBKV * kDV * 2;   // one K / V stage
-  static constexpr int kKStages = kShared ? 4 : 2;
-  static constexpr int kPBytes = kBQ * kBKV * 2;
-  static constexpr int kBars = kQBytes + kKStages * kKBytes + (kShared ? 0 : 2 * kVBytes) + kPBytes;   // offset of the barriers
-  static constexpr int kSmemBytes = kBars + 1024 /*align*/ + 256 /*barriers*/;
-};
-constexpr int kBiasFront = kBKV - 1, kBiasPad = 2 * kBKV + kBKV;   // table entries in front / in all beyond n_bias
-constexpr int kMaxSmem = 227 * 1024;
+enum FBar { Q_FULL = 0, Q_EMPTY = 2, KV_FULL = 4, KV_EMPTY = 8, S_FULL = 12, P_FULL = 14, O_FULL = 16, O_EMPTY = 18, IT_FULL = 20, IT_EMPTY = 22,
+            CLC_FULL = 24, F_NUM_BARS = 25 };
 
-enum Bar { Q_FULL = 0, K_FULL = 1, K_EMPTY = 3, V_FULL = 5, V_EMPTY = 7, S_FULL = 9, S_EMPTY = 11, P_FULL = 13, P_EMPTY = 14,
-           O_FULL = 15, O_EMPTY = 17, NUM_BARS = 19 };
-
-// Every wait is bounded: a wait that runs out sets the CTA's `dead` flag (all later waits of the CTA then return at once), and the
-// kernel ends normally after a pause that lets its own copies land; `rb_attn_wait_error` tells the host.
 __device__ int g_wait_error = 0;
-constexpr int kWaitPolls = 1 << 20;
 
-RB_DEVICE void bounded_wait(uint32_t bar, uint32_t parity, volatile uint32_t* dead) {
-  for (int i = 0; !ptx::mbar_try_wait(bar, parity); ++i)
-    if (i >= kWaitPolls || *dead) { *dead = 1; return; }
-}
+// One work item: sequence (first token, length), heads and query tiles of the two tiles (tile 1 < 0: absent); L < 0 ends the CTA's loop.
+struct Item { int tok0, L, head0, head1, qt0, qt1; };
 
-RB_DEVICE void st_shared_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
-  asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
-}
-template <typename T> RB_DEVICE uint32_t pack2(float lo, float hi);
-template <> RB_DEVICE uint32_t pack2<__nv_bfloat16>(float lo, float hi) {
-  __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
-  return *reinterpret_cast<uint32_t*>(&v);
-}
-template <> RB_DEVICE uint32_t pack2<__half>(float lo, float hi) {
-  __half2 v = __floats2half2_rn(lo, hi);
-  return *reinterpret_cast<uint32_t*>(&v);
-}
+// The key tiles of an item: the kept first tiles [0, nk), then [lo, end); a tile takes part in key tile j when j < its end and j is at or
+// behind its first tile or among the kept ones.  (Plain numbers, no arrays: indexing them by a run-time tile would go through memory.)
+struct Walk {
+  int first0, end0, first1, end1, keep_tiles, nk, lo, n;
+  RB_DEVICE Walk(const Item& it, const AttnParams& p) {
+    const int win = (p.causal && p.window > 0) ? p.window : 0;
+    keep_tiles = win > 0 ? RB_CEIL_DIV(p.keep, kTile) : 0;
+    auto first = [&](int qt) { const int q0 = qt * kTile; return p.chunk > 0 ? (q0 / p.chunk * p.chunk) / kTile : win > 0 ? max(0, q0 - win + 1) / kTile : 0; };
+    auto end = [&](int qt) { return qt < 0 ? 0 : RB_CEIL_DIV(p.causal ? min(it.L, qt * kTile + kTile) : it.L, kTile); };
+    first0 = first(it.qt0);
+    end0 = end(it.qt0);
+    end1 = end(it.qt1);
+    first1 = it.qt1 < 0 ? first0 : first(it.qt1);
+    lo = min(first0, first1);
+    nk = min(keep_tiles, lo);
+    n = nk + max(end0, end1) - lo;
+  }
+  RB_DEVICE int tile(int k) const { return k < nk ? k : lo + k - nk; }
+  RB_DEVICE bool takes(int t, int j) const { return j < (t ? end1 : end0) && (j >= (t ? first1 : first0) || j < keep_tiles); }
+};
 
-// cap * tanh(s * scale / cap) + add in the log2 domain, tanh(x) = 1 - 2 / (1 + 2^(2 x log2 e)): c = 2 log2 e * scale / cap,
-// k = cap log2 e, k_add = k + add.  Absolute error a few ulp of k; saturates to +-k.
-RB_DEVICE float soft_cap2(float s, float c, float k, float k_add) {
-  return fmaf(-2.f * k, __fdividef(1.f, 1.f + exp2f(fminf(s * c, 80.f))), k_add);
-}
-
-template <int kD, int kDV, typename T, int kFmt, bool kSink = false, bool kCap = false, bool kSimple = false, bool kBias = false, bool kShared = false>
-__global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q,
-                                                                   const __grid_constant__ CUtensorMap tma_k,
-                                                                   const __grid_constant__ CUtensorMap tma_v, AttnParams p) {
-  static_assert(!kShared || kD == kDV, "shared keys and values have one size");
-  static_assert(!kBias || (kSink && !kSimple && !kCap), "kBias is a form of kSink");
-  constexpr bool kOneMask = kSimple || kBias;      // no kept first keys: visible columns are one range
-  using C = ACfg<kD, kDV, kShared>;
-  const int seq = blockIdx.z, head = blockIdx.y;
-  const int qt = gridDim.x - 1 - blockIdx.x;  // long (late) query tiles first: they walk the most key tiles
-  const int tok0 = p.cu_seqlens[seq];
-  const int L = p.cu_seqlens[seq + 1] - tok0;
-  const int q0 = qt * kBQ;
-  if (q0 >= L) return;  // uniform for the CTA, before any barrier / TMEM allocation
-  const int hk = head / (p.nq / p.nkv);
-  const int kv_len = p.causal ? min(L, q0 + kBQ) : L;
-  const int win = (p.causal && p.window > 0) ? p.window : 0;
-  const int chunk = kSink ? p.chunk : 0;
-  // first key tile any row of this CTA can see
-  const int tile0 = (kSink && chunk > 0) ? (q0 / chunk * chunk) / kBKV : win > 0 ? max(0, q0 - win + 1) / kBKV : 0;
-  // kSink: the tiles of the kept first keys that lie wholly below tile0 come first in every role's walk
-  const int n_keep = (kSink && !kOneMask && win > 0) ? min(RB_CEIL_DIV(p.keep, kBKV), tile0) : 0;
-  const int n_kv = n_keep + RB_CEIL_DIV(kv_len, kBKV) - tile0;    // >= 1: the diagonal tile is always visible
-  auto tile_of = [&](int j) { return j < n_keep ? j : tile0 + j - n_keep; };
-
+template <int kD, int kDV, typename T, int kFmt, int kMode>
+__global__ void __launch_bounds__(kFwdThreads, 1) attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant__ CUtensorMap tma_k,
+                                                                  const __grid_constant__ CUtensorMap tma_v, const __grid_constant__ AttnParams p) {
+  using C = FCfg<kD, kDV>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  const uint32_t sQ = ptx::smem_u32(smem);
-  const uint32_t sK = sQ + C::kQBytes;
-  const uint32_t sV = sK + C::kKStages * C::kKBytes;
-  const uint32_t sP = sV + (kShared ? 0 : 2 * C::kVBytes);
+  const uint32_t sQ = ptx::smem_u32(smem), sKV = sQ + C::kKV;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::kBars);
-  float* tab = reinterpret_cast<float*>(smem + C::kBars + 256);      // kBias
-  uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(bars + NUM_BARS);
+  Item* items = reinterpret_cast<Item*>(smem + C::kBars + 256);                // two slots of 24 bytes
+  const uint32_t clc = sQ + C::kBars + 256 + 64;                               // 16 bytes
+  uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(smem + C::kBars + 256 + 80);
   volatile uint32_t* dead = tmem_ptr + 1;
   auto bar = [&](int i) { return ptx::smem_u32(&bars[i]); };
-  // stage and barriers of key tile j (kShared: four stages, the last two on V's barriers)
-  auto k_stage = [](int j) { return kShared ? j & 3 : j & 1; };
-  auto k_par = [](int j) { return (uint32_t)(kShared ? j >> 2 : j >> 1) & 1u; };
-  auto k_full = [](int st) { return st < 2 ? K_FULL + st : V_FULL + st - 2; };
-  auto k_empty = [](int st) { return st < 2 ? K_EMPTY + st : V_EMPTY + st - 2; };
-  if constexpr (kBias) {
-    for (int i = threadIdx.x; i < p.n_bias + kBiasPad; i += kAttnThreads)
-      tab[i] = p.bias[(int64_t)head * p.bias_ld + min(max(i - kBiasFront, 0), p.n_bias - 1)] * 1.4426950408889634f;
-  }
-
+  auto wait = [&](int i, uint32_t parity) { bounded_wait(bar(i), parity, dead); };
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (warp == 0 && lane == 0) {
+
+  if (warp == 9 && lane == 0) {
     *dead = 0;
     ptx::prefetch_tensormap(&tma_q);
     ptx::prefetch_tensormap(&tma_k);
     ptx::prefetch_tensormap(&tma_v);
-    for (int i = 0; i < NUM_BARS; ++i) {
-      const bool softmax_side = (i == S_EMPTY || i == S_EMPTY + 1 || i == P_FULL || i == O_EMPTY || i == O_EMPTY + 1);
-      ptx::mbar_init(bar(i), softmax_side ? 4 : 1);  // one arrival per softmax warp
+    for (int i = 0; i < F_NUM_BARS; ++i) {
+      const bool softmax_side = (i >= P_FULL && i < P_FULL + 2) || (i >= O_EMPTY && i < O_EMPTY + 2);
+      ptx::mbar_init(bar(i), softmax_side ? 4 : (i >= IT_EMPTY && i < IT_EMPTY + 2) ? 9 : 1);   // items: the MMA thread and 8 softmax warps
     }
     ptx::fence_barrier_init();
   }
-  if (warp == 1) {
+  if (warp == 8) {
     ptx::tmem_alloc(ptx::smem_u32(tmem_ptr), 512);
     ptx::tmem_relinquish();
   }
@@ -185,246 +120,357 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
   ptx::tc_fence_after();
   const uint32_t tmem_base = *tmem_ptr;
 
-  auto wait = [&](uint32_t b, uint32_t parity) { bounded_wait(b, parity, dead); };
-
-  if (warp == 0) {
-    // ===================================================== TMA producer
-    if (lane == 0) {
-      ptx::mbar_arrive_expect_tx(bar(Q_FULL), C::kQBytes);
-#pragma unroll
-      for (int kb = 0; kb < C::kDBlocks; ++kb)
-        ptx::tma_load_2d(sQ + kb * (kBQ * 128), &tma_q, bar(Q_FULL), head * kD + kb * 64, tok0 + q0);
-      for (int j = 0; j < n_kv; ++j) {
-        const int row = tok0 + tile_of(j) * kBKV;
-        const int ks = k_stage(j);
-        wait(bar(k_empty(ks)), k_par(j) ^ 1);
-        ptx::mbar_arrive_expect_tx(bar(k_full(ks)), C::kKBytes);
-#pragma unroll
-        for (int kb = 0; kb < C::kDBlocks; ++kb)
-          ptx::tma_load_2d(sK + ks * C::kKBytes + kb * (kBKV * 128), &tma_k, bar(k_full(ks)), hk * kD + kb * 64, row);
-        if constexpr (kShared) continue;
-        const int st = j & 1;
-        const uint32_t par = (uint32_t)(j >> 1) & 1u;
-        wait(bar(V_EMPTY + st), par ^ 1);
-        ptx::mbar_arrive_expect_tx(bar(V_FULL + st), C::kVBytes);
-        // V is the MN-major B operand of P V: it is staged as two 64-key halves, each [d chunk][64 keys][128 B], i.e. exactly
-        // the stage format (and the 8 KB chunk stride) of the GEMM's MN-major operands
-#pragma unroll
-        for (int half = 0; half < kBKV / 64; ++half)
-#pragma unroll
-          for (int kb = 0; kb < C::kDVBlocks; ++kb)
-            ptx::tma_load_2d(sV + st * C::kVBytes + half * (64 * kDV * 2) + kb * (64 * 128), &tma_v, bar(V_FULL + st),
-                             (hk / p.vshare) * kDV + kb * 64, row + half * 64);
-      }
-    }
-  } else if (warp == 1) {
-    // ===================================================== MMA issuer
-    if (lane == 0) {
-      constexpr uint32_t idesc_s = ptx::make_idesc_f16(kFmt, kBQ, kBKV, 0, 0);  // Q, K both K-major (head-dim contiguous)
-      constexpr uint32_t idesc_o = ptx::make_idesc_f16(kFmt, kBQ, kDV, 0, 1);    // P K-major, V MN-major
-      auto issue_s = [&](int j) {
-        const int st = j & 1, ks = k_stage(j);
-        const uint32_t par = (uint32_t)(j >> 1) & 1u;
-        wait(bar(k_full(ks)), k_par(j));
-        wait(bar(S_EMPTY + st), par ^ 1);
-        ptx::tc_fence_after();
-#pragma unroll
-        for (int kk = 0; kk < kD / 16; ++kk) {
-          const uint32_t off = (kk >> 2) * (kBQ * 128) + (kk & 3) * 32;
-          ptx::tc_mma_f16(tmem_base + st * 128, ptx::make_smem_desc_sw128(sQ + off, 16, 1024),
-                          ptx::make_smem_desc_sw128(sK + ks * C::kKBytes + off, 16, 1024), idesc_s, kk != 0 ? 1u : 0u);
+  if (warp >= 8) {
+    ptx::reg_dec<kOtherRegs>();
+    if (warp == 9) {
+      // ===================================================== scheduler + TMA producer
+      auto request = [&] {
+        if (lane == 0) {
+          ptx::mbar_arrive_expect_tx(bar(CLC_FULL), 16);
+          ptx::clc_try_cancel(clc, bar(CLC_FULL));
         }
-        if constexpr (!kShared) ptx::tc_commit(bar(k_empty(ks)));  // K stage reusable once S_j retired
-        ptx::tc_commit(bar(S_FULL + st));
+        __syncwarp();
       };
-      wait(bar(Q_FULL), 0);
-      issue_s(0);
-      for (int j = 0; j < n_kv; ++j) {
-        if (j + 1 < n_kv) issue_s(j + 1);
-        const int st = j & 1;
-        const uint32_t par = (uint32_t)(j >> 1) & 1u;
-        wait(bar(P_FULL), (uint32_t)j & 1u);
-        if constexpr (!kShared) wait(bar(V_FULL + st), par);   // (kShared: the tile arrived before S_j was issued)
-        wait(bar(O_EMPTY + st), par ^ 1);
-        ptx::tc_fence_after();
+      int unit_base = 0, s0 = 0;    // work units in front of sequence block [s0, s0 + 32): item numbers mostly grow, so the search goes on from here
+      auto find = [&](int idx, Item& it) {
+        const int unit = idx / p.n_head_units, hu = idx - unit * p.n_head_units;
+        if (unit < unit_base) { unit_base = 0; s0 = 0; }
+        for (; s0 < p.B; s0 += 32) {
+          const int s = s0 + lane;
+          const int a = s < p.B ? p.cu_seqlens[s] : 0;
+          const int L = s < p.B ? max(p.cu_seqlens[s + 1] - a, 0) : 0;
+          const int c = p.pair_heads ? RB_CEIL_DIV(L, kTile) : RB_CEIL_DIV(L, 2 * kTile);
+          int incl = c;
 #pragma unroll
-        for (int kk = 0; kk < kBKV / 16; ++kk) {
-          // A: 16 keys = 32 B inside the 128 B row of key block kk/4; B: 16 key rows = 2048 B down every 64-wide d chunk of
-          // key half kk/4 (kShared: of the whole K tile, whose chunks hold all kBKV keys)
-          const uint32_t b_off = kShared ? sK + k_stage(j) * C::kKBytes + kk * 2048 : sV + st * C::kVBytes + (kk >> 2) * (64 * kDV * 2) + (kk & 3) * 2048;
-          ptx::tc_mma_f16(tmem_base + 256 + st * 128,
-                          ptx::make_smem_desc_sw128(sP + (kk >> 2) * (kBQ * 128) + (kk & 3) * 32, 16, 1024),
-                          ptx::make_smem_desc_sw128(b_off, (kShared ? kBKV : 64) * 128, 1024), idesc_o, kk != 0 ? 1u : 0u);
+          for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += v;
+          }
+          const unsigned hit = __ballot_sync(0xffffffffu, unit_base + incl > unit);
+          if (hit != 0) {
+            const int w = __ffs(hit) - 1;
+            it.tok0 = __shfl_sync(0xffffffffu, a, w);
+            it.L = __shfl_sync(0xffffffffu, L, w);
+            const int r = unit - unit_base - __shfl_sync(0xffffffffu, incl - c, w);   // r-th unit of the sequence, longest first
+            const int last = RB_CEIL_DIV(it.L, kTile) - 1;
+            it.head0 = p.pair_heads ? 2 * hu : hu;
+            it.head1 = p.pair_heads ? 2 * hu + 1 : hu;
+            it.qt0 = p.pair_heads ? last - r : last - 2 * r;
+            it.qt1 = p.pair_heads ? last - r : last - 2 * r - 1;
+            return true;
+          }
+          unit_base += __shfl_sync(0xffffffffu, incl, 31);
         }
-        ptx::tc_commit(bar(kShared ? k_empty(k_stage(j)) : V_EMPTY + st));
-        ptx::tc_commit(bar(P_EMPTY));
-        ptx::tc_commit(bar(O_FULL + st));
+        unit_base = 0;
+        s0 = 0;
+        return false;
+      };
+
+      int idx = blockIdx.x, n_pub = 0;
+      uint32_t kvc = 0, qc0 = 0, qc1 = 0, n_req = 0;
+      request();
+      auto publish = [&](const Item& it) {
+        const int slot = n_pub & 1;
+        wait(IT_EMPTY + slot, ((uint32_t)(n_pub >> 1) & 1u) ^ 1u);
+        if (lane == 0) {
+          items[slot] = it;
+          ptx::mbar_arrive(bar(IT_FULL + slot));
+        }
+        ++n_pub;
+      };
+      while (true) {
+        Item it{0, 0, 0, 0, 0, 0};
+        if (find(idx, it)) {
+          publish(it);
+          if (lane == 0) {
+            const Walk w(it, p);
+            const int hk = it.head0 / (p.nq / p.nkv);
+            auto load_q = [&](int t, int head, int qt, uint32_t& count) {
+              if (qt < 0) return;
+              wait(Q_EMPTY + t, (count & 1u) ^ 1u);
+              ++count;
+              ptx::mbar_arrive_expect_tx(bar(Q_FULL + t), C::kQBytes);
+#pragma unroll
+              for (int kb = 0; kb < kD / 64; ++kb)
+                ptx::tma_load_2d(sQ + t * C::kQBytes + kb * (kTile * 128), &tma_q, bar(Q_FULL + t), head * kD + kb * 64, it.tok0 + qt * kTile);
+            };
+            auto load_kv = [&](bool is_v, int j) {
+              const int st = kvc & (kStages - 1);
+              wait(KV_EMPTY + st, ((kvc / kStages) & 1u) ^ 1u);
+              ++kvc;
+              ptx::mbar_arrive_expect_tx(bar(KV_FULL + st), is_v ? C::kVBytes : C::kKBytes);
+              const int col = is_v ? (hk / p.vshare) * kDV : hk * kD, blocks = is_v ? kDV / 64 : kD / 64;
+              for (int kb = 0; kb < blocks; ++kb)
+                ptx::tma_load_2d(sKV + st * C::kStageBytes + kb * (kTile * 128), is_v ? &tma_v : &tma_k, bar(KV_FULL + st), col + kb * 64,
+                                 it.tok0 + j * kTile);
+            };
+            load_q(0, it.head0, it.qt0, qc0);
+            load_kv(false, w.tile(0));
+            load_q(1, it.head1, it.qt1, qc1);
+            load_kv(true, w.tile(0));
+            for (int k = 1; k < w.n; ++k) {
+              load_kv(false, w.tile(k));
+              load_kv(true, w.tile(k));
+            }
+          }
+          __syncwarp();
+        }
+        wait(CLC_FULL, n_req & 1u);
+        ++n_req;
+        if (*dead) break;
+        int x;
+        const bool got = ptx::clc_query(clc, x);
+        __syncwarp();
+        if (!got) break;
+        idx = x;
+        ptx::fence_proxy_async();   // the response was read before it is overwritten
+        request();
       }
+      publish(Item{0, -1, 0, 0, -1, -1});
+    } else if (warp == 8) {
+      // ===================================================== MMA issuer
+      if (lane == 0) {
+        constexpr uint32_t idesc_s = ptx::make_idesc_f16(kFmt, kTile, kTile, 0, 0);   // Q, K both K-major (head-dim contiguous)
+        constexpr uint32_t idesc_o = ptx::make_idesc_f16(kFmt, kTile, kDV, 0, 1);     // P (TMEM), V MN-major
+        uint32_t kvc = 0, qc[2] = {0, 0}, pc[2] = {0, 0}, oc[2] = {0, 0};
+        for (int n_it = 0;; ++n_it) {
+          const int slot = n_it & 1;
+          wait(IT_FULL + slot, (uint32_t)(n_it >> 1) & 1u);
+          const Item it = items[slot];
+          ptx::mbar_arrive(bar(IT_EMPTY + slot));
+          if (it.L < 0 || *dead) break;
+          const Walk w(it, p);
+          bool s_open[2] = {false, false}, o_open[2] = {false, false};
+          auto issue_s = [&](int t, int j, int st) {
+            if (!s_open[t]) { wait(Q_FULL + t, qc[t] & 1u); ++qc[t]; s_open[t] = true; }
+            ptx::tc_fence_after();
+#pragma unroll
+            for (int kk = 0; kk < kD / 16; ++kk) {
+              const uint32_t off = (kk >> 2) * (kTile * 128) + (kk & 3) * 32;
+              ptx::tc_mma_f16(tmem_base + t * 128, ptx::make_smem_desc_sw128(sQ + t * C::kQBytes + off, 16, 1024),
+                              ptx::make_smem_desc_sw128(sKV + st * C::kStageBytes + off, 16, 1024), idesc_s, kk != 0 ? 1u : 0u);
+            }
+            ptx::tc_commit(bar(S_FULL + t));
+            if (j == (t ? w.end1 : w.end0) - 1) ptx::tc_commit(bar(Q_EMPTY + t));
+          };
+          auto issue_pv = [&](int t, int st) {
+            wait(P_FULL + t, pc[t] & 1u);
+            ++pc[t];
+            if (!o_open[t]) { wait(O_EMPTY + t, (oc[t] & 1u) ^ 1u); ++oc[t]; }
+            ptx::tc_fence_after();
+#pragma unroll
+            for (int kk = 0; kk < kTile / 16; ++kk)      // A: 16 keys = 8 TMEM columns; B: 16 key rows = 2048 B down every 64-wide chunk of DV
+              ptx::tc_mma_f16_ts(tmem_base + 256 + t * 128, tmem_base + t * 128 + kk * 8,
+                                 ptx::make_smem_desc_sw128(sKV + st * C::kStageBytes + kk * 2048, kTile * 128, 1024), idesc_o,
+                                 (o_open[t] || kk != 0) ? 1u : 0u);
+            o_open[t] = true;
+            ptx::tc_commit(bar(O_FULL + t));
+          };
+          auto open_kv = [&](uint32_t c) { wait(KV_FULL + (c & (kStages - 1)), (c / kStages) & 1u); return (int)(c & (kStages - 1)); };
+          int st = open_kv(kvc);
+#pragma unroll
+          for (int t = 0; t < 2; ++t)
+            if (w.takes(t, w.tile(0))) issue_s(t, w.tile(0), st);
+          ptx::tc_commit(bar(KV_EMPTY + st));
+          for (int k = 0; k < w.n; ++k) {
+            const int j = w.tile(k), jn = w.tile(k + 1);
+            const bool more = k + 1 < w.n;
+            const int sv = open_kv(kvc + 2 * k + 1);
+            int sk = -1;
+#pragma unroll
+            for (int t = 0; t < 2; ++t) {
+              if (w.takes(t, j)) issue_pv(t, sv);
+              if (t == 1) ptx::tc_commit(bar(KV_EMPTY + sv));
+              if (more) {
+                if (sk < 0) sk = open_kv(kvc + 2 * k + 2);
+                if (w.takes(t, jn)) issue_s(t, jn, sk);
+              }
+            }
+            if (more) ptx::tc_commit(bar(KV_EMPTY + sk));
+          }
+          kvc += 2 * w.n;
+        }
+      }
+      __syncwarp();
     }
   } else {
-    // ===================================================== softmax + output (4 warps; thread = query row = TMEM lane)
-    const int quad = warp & 3;
+    ptx::reg_inc<kSoftmaxRegs>();
+    // ===================================================== softmax + output (4 warps per tile; thread = query row = TMEM lane)
+    const int t = warp >> 2, quad = warp & 3;
     const int row = quad * 32 + lane;
-    const int q_pos = q0 + row;
     const uint32_t lane_addr = tmem_base + ((uint32_t)(quad * 32) << 16);
-    const float sl2 = p.scale * 1.4426950408889634f;
-    const uint32_t p_row = sP + (uint32_t)(row >> 3) * 1024u + (uint32_t)(row & 7) * 128u;
-    const uint32_t sw = (uint32_t)(row & 7);
-    float m_run = -INFINITY, l_run = 0.f, alpha_prev = 0.f;
-    const int row_lo = (kSink && chunk > 0) ? q_pos / chunk * chunk : win > 0 ? q_pos - win + 1 : 0;   // first visible key of the row
-    const int last_lo = (kSink && chunk > 0) ? (q0 + kBQ - 1) / chunk * chunk : q0 + kBQ - win;      // of the tile's last row
-    const bool bounded = win > 0 || (kSink && chunk > 0);
-    const float cap_c = kCap ? 2.f * 1.4426950408889634f * p.scale / p.softcap : 0.f, cap_k = kCap ? p.softcap * 1.4426950408889634f : 0.f;
-    // kSink: scores live in the log2 domain, t = s * c2 - slope2 * (q_pos - key_pos); the sink starts the maximum
-    float c2 = 0.f, slope2 = 0.f;
-    if constexpr (kSink) {
-      c2 = sl2 * (p.temp ? rb::to_f(reinterpret_cast<const T*>(p.temp)[head]) : 1.f);
-      if constexpr (!kSimple && !kBias) slope2 = p.slope_base >= 0.f ? exp2f(-p.slope_base * (float)(head + 1) / (float)p.nq) * 1.4426950408889634f : 0.f;
-      if (p.sink) { m_run = rb::to_f(reinterpret_cast<const T*>(p.sink)[head]) * 1.4426950408889634f; l_run = 1.f; }
-    }
-    float O[kDV];
-#pragma unroll
-    for (int i = 0; i < kDV; ++i) O[i] = 0.f;
-
-    auto fold = [&](int t, float a) {  // O <- O * a + T_t
-      const int b = t & 1;
-      wait(bar(O_FULL + b), (uint32_t)(t >> 1) & 1u);
-      ptx::tc_fence_after();
-#pragma unroll
-      for (int c = 0; c < kDV / 32; ++c) {
-        uint32_t r[32];
-        ptx::tc_ld_32x32(lane_addr + 256 + b * 128 + c * 32, r);
-        ptx::tc_wait_ld();
-#pragma unroll
-        for (int i = 0; i < 32; ++i) O[c * 32 + i] = fmaf(O[c * 32 + i], a, __uint_as_float(r[i]));
-      }
-      ptx::tc_fence_before();
+    const uint32_t tS = lane_addr + t * 128, tO = lane_addr + 256 + t * 128;
+    const uint32_t stage = sQ + C::kOut + warp * 4096;
+    const float cap_c = kMode == kCap ? 2.f * 1.4426950408889634f * p.scale / p.softcap : 0.f, cap_k = kMode == kCap ? p.softcap * 1.4426950408889634f : 0.f;
+    const int win = (p.causal && p.window > 0) ? p.window : 0;
+    const bool bounded = win > 0 || p.chunk > 0;
+    uint32_t sc = 0, vc = 0;      // S tiles / P V products of this tile so far
+    for (int n_it = 0;; ++n_it) {
+      const int slot = n_it & 1;
+      wait(IT_FULL + slot, (uint32_t)(n_it >> 1) & 1u);
+      const Item it = items[slot];
       __syncwarp();
-      if (lane == 0) ptx::mbar_arrive(bar(O_EMPTY + b));
-    };
+      if (lane == 0) ptx::mbar_arrive(bar(IT_EMPTY + slot));
+      if (it.L < 0 || *dead) break;
+      const int qt = t ? it.qt1 : it.qt0;
+      if (qt < 0) continue;
+      const int head = t ? it.head1 : it.head0, L = it.L, q0 = qt * kTile, q_pos = q0 + row;
+      // scores live in the log2 domain: weight = exp2(s * c2 [+ distance term] - m_run)
+      float c2 = p.scale * 1.4426950408889634f, slope2 = 0.f, m_run = -INFINITY, l_run = 0.f;
+      if constexpr (kMode != kPlain) {
+        if (p.temp) c2 *= rb::to_f(reinterpret_cast<const T*>(p.temp)[head]);
+        if (kMode == kGeneral && p.slope_base >= 0.f) slope2 = exp2f(-p.slope_base * (float)(head + 1) / (float)p.nq) * 1.4426950408889634f;
+        if (p.sink) { m_run = rb::to_f(reinterpret_cast<const T*>(p.sink)[head]) * 1.4426950408889634f; l_run = 1.f; }
+      }
+      const int row_lo = p.chunk > 0 ? q_pos / p.chunk * p.chunk : win > 0 ? q_pos - win + 1 : 0;                 // first visible key of the row
+      const int last_lo = p.chunk > 0 ? (q0 + kTile - 1) / p.chunk * p.chunk : q0 + kTile - win;                  // of the tile's last row
+      // this tile's key tiles, in the order of the item's walk
+      const int first_tile = p.chunk > 0 ? (q0 / p.chunk * p.chunk) / kTile : win > 0 ? max(0, q0 - win + 1) / kTile : 0;
+      const int n_keep = win > 0 ? min(RB_CEIL_DIV(p.keep, kTile), first_tile) : 0;
+      const int n_tiles = n_keep + RB_CEIL_DIV(p.causal ? min(L, q0 + kTile) : L, kTile) - first_tile;
+      bool first = true;
 
-    for (int j = 0; j < n_kv; ++j) {
-      const int b = j & 1;
-      const int kv0 = tile_of(j) * kBKV;
-      wait(bar(S_FULL + b), (uint32_t)(j >> 1) & 1u);
-      ptx::tc_fence_after();
-      // only the last tile of the sequence, the diagonal tile and the tiles the window's lower edge crosses need per-element
-      // masks (uniform over the CTA)
-      const bool need_mask = (kv0 + kBKV > L) || (p.causal && kv0 + kBKV - 1 > q0) || (bounded && last_lo > kv0);
-      const int lim = (p.causal ? min(L, q_pos + 1) : L) - kv0;  // local key columns [lo, lim) are visible to this row
-      const int lo = bounded ? row_lo - kv0 : 0;
-      const int kept = kSink && !kOneMask ? p.keep - kv0 : 0;                 // kSink: local columns below `kept` stay visible under `lo`
-      const uint32_t n_vis = (uint32_t)max(lim - lo, 0);
-      auto hidden = [&](int col) {
-        if constexpr (kOneMask) return (uint32_t)(col - lo) >= n_vis;
-        return col >= lim || (col < lo && (!kSink || col >= kept));
-      };
-      const float base = kSink && !kBias ? slope2 * (float)(kv0 - q_pos) : 0.f;
-      // kBias: entry of the row's column 0 (q0 - kv0 >= 0: the diagonal tile is the last one); beyond the table its constant tail
-      const float* brow = kBias ? tab + min(q0 - kv0, p.n_bias - 1 + kBiasFront) + row + kBiasFront : nullptr;
-      float mx = -INFINITY;
+      for (int k = 0; k < n_tiles; ++k) {
+        const int kv0 = (k < n_keep ? k : first_tile + k - n_keep) * kTile;
+        wait(S_FULL + t, sc & 1u);
+        ++sc;
+        ptx::tc_fence_after();
+        uint32_t r[128];
 #pragma unroll
-      for (int c = 0; c < kBKV / 32; ++c) {
-        uint32_t r[32];
-        ptx::tc_ld_32x32(lane_addr + b * 128 + c * 32, r);
+        for (int c = 0; c < 4; ++c) ptx::tc_ld_32x32(tS + c * 32, r + c * 32);
         ptx::tc_wait_ld();
+        float s[128];
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          float s = __uint_as_float(r[i]);
-          if constexpr (kBias) s = fmaf(s, c2, brow[-(c * 32 + i)]);
-          else if constexpr (kSink && !kSimple) s = fmaf(s, c2, fmaf(slope2, (float)(c * 32 + i), base));
-          if (need_mask && hidden(c * 32 + i)) s = -INFINITY;
-          mx = fmaxf(mx, s);
+        for (int i = 0; i < 128; ++i) s[i] = __uint_as_float(r[i]);
+        if constexpr (kMode == kGeneral) {
+          const float base = slope2 * (float)(kv0 - q_pos);
+#pragma unroll
+          for (int i = 0; i < 128; ++i) s[i] = fmaf(s[i], c2, fmaf(slope2, (float)i, base));
         }
-      }
-      if constexpr (kSimple) {
-        if (mx != -INFINITY) mx = kCap ? soft_cap2(mx, cap_c, cap_k, cap_k) : mx * c2;
-      }
-      const float m_new = fmaxf(m_run, mx);
-      const float m_eff = (m_new == -INFINITY) ? 0.f : m_new;  // fully masked so far: keep exp2 arguments finite
-      const float alpha = kSink ? exp2f(m_run - m_eff) : exp2f((m_run - m_eff) * sl2);
-      const float neg_m = kSink ? -m_eff : -m_eff * sl2;
-      if (j > 0) wait(bar(P_EMPTY), (uint32_t)(j - 1) & 1u);  // PV_{j-1} finished reading the P buffer
-      float sum = 0.f;
+        // only the last tile of the sequence, the diagonal tile and the tiles the window's lower edge crosses need per-element masks
+        if ((kv0 + kTile > L) || (p.causal && kv0 + kTile - 1 > q0) || (bounded && last_lo > kv0)) {
+          const int lim = (p.causal ? min(L, q_pos + 1) : L) - kv0;   // local key columns [lo, lim) are visible to this row
+          const int lo = bounded ? row_lo - kv0 : 0;
+          if constexpr (kMode == kGeneral) {
+            const int kept = p.keep - kv0;                            // columns below `kept` stay visible under `lo`
 #pragma unroll
-      for (int c = 0; c < kBKV / 32; ++c) {
-        uint32_t r[32];
-        ptx::tc_ld_32x32(lane_addr + b * 128 + c * 32, r);
-        ptx::tc_wait_ld();
-        uint32_t w[16];
-#pragma unroll
-        for (int i = 0; i < 32; i += 2) {
-          float e0, e1;
-          if constexpr (kCap) {
-            e0 = exp2f(soft_cap2(__uint_as_float(r[i]), cap_c, cap_k, cap_k + neg_m));
-            e1 = exp2f(soft_cap2(__uint_as_float(r[i + 1]), cap_c, cap_k, cap_k + neg_m));
-          } else if constexpr (kBias) {
-            e0 = exp2f(fmaf(__uint_as_float(r[i]), c2, brow[-(c * 32 + i)]) + neg_m);
-            e1 = exp2f(fmaf(__uint_as_float(r[i + 1]), c2, brow[-(c * 32 + i + 1)]) + neg_m);
-          } else if constexpr (kSimple) {
-            e0 = exp2f(fmaf(__uint_as_float(r[i]), c2, neg_m));
-            e1 = exp2f(fmaf(__uint_as_float(r[i + 1]), c2, neg_m));
-          } else if constexpr (kSink) {
-            e0 = exp2f(fmaf(__uint_as_float(r[i]), c2, fmaf(slope2, (float)(c * 32 + i), base)) + neg_m);
-            e1 = exp2f(fmaf(__uint_as_float(r[i + 1]), c2, fmaf(slope2, (float)(c * 32 + i + 1), base)) + neg_m);
+            for (int i = 0; i < 128; ++i)
+              if (i >= lim || (i < lo && i >= kept)) s[i] = -INFINITY;
           } else {
-            e0 = exp2f(fmaf(__uint_as_float(r[i]), sl2, neg_m));
-            e1 = exp2f(fmaf(__uint_as_float(r[i + 1]), sl2, neg_m));
-          }
-          if (need_mask) {
-            if (hidden(c * 32 + i)) e0 = 0.f;
-            if (hidden(c * 32 + i + 1)) e1 = 0.f;
-          }
-          sum += e0 + e1;
-          w[i >> 1] = pack2<T>(e0, e1);
-        }
+            const uint32_t n_vis = (uint32_t)max(lim - lo, 0);
 #pragma unroll
-        for (int t = 0; t < 4; ++t) {
-          const uint32_t piece = (uint32_t)(c * 4 + t);  // 16-byte piece (8 keys) of this row: key block piece/8, slot piece%8
-          st_shared_v4(p_row + (piece >> 3) * (kBQ * 128) + (((piece & 7) ^ sw) << 4), w[4 * t], w[4 * t + 1], w[4 * t + 2],
-                       w[4 * t + 3]);
+            for (int i = 0; i < 128; ++i)
+              if ((uint32_t)(i - lo) >= n_vis) s[i] = -INFINITY;
+          }
         }
+        float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+        for (int i = 0; i < 128; i += 8)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) mx4[e] = fmaxf(mx4[e], fmaxf(s[i + 2 * e], s[i + 2 * e + 1]));
+        float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
+        if (kMode != kGeneral && mx != -INFINITY) mx = kMode == kCap ? soft_cap2(mx, cap_c, cap_k, cap_k) : mx * c2;
+        if (first) {
+          const float m_new = fmaxf(m_run, mx);
+          if (m_new != -INFINITY) l_run *= exp2f(m_run - m_new);
+          m_run = m_new;
+        } else if (__any_sync(0xffffffffu, mx > m_run + kLazy)) {
+          const float m_new = mx > m_run + kLazy ? mx : m_run;
+          const float a = m_new == m_run ? 1.f : exp2f(m_run - m_new);
+          wait(O_FULL + t, (vc - 1) & 1u);          // the product in flight has retired, and the next one waits for this tile's P
+          ptx::tc_fence_after();
+#pragma unroll
+          for (int c = 0; c < kDV / 32; ++c) {
+            uint32_t o[32];
+            ptx::tc_ld_32x32(tO + c * 32, o);
+            ptx::tc_wait_ld();
+#pragma unroll
+            for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * a);
+            ptx::tc_st_32x32(tO + c * 32, o);
+          }
+          l_run *= a;
+          m_run = m_new;
+        }
+        first = false;
+        const float neg_m = m_run == -INFINITY ? 0.f : -m_run;      // fully masked so far: keep exp2 arguments finite
+        float sum4[4] = {0.f, 0.f, 0.f, 0.f};
+        uint32_t pw[64];
+#pragma unroll
+        for (int i = 0; i < 128; i += 2) {
+          float e0, e1;
+          if constexpr (kMode == kCap) {
+            e0 = s[i] == -INFINITY ? 0.f : exp2f(soft_cap2(s[i], cap_c, cap_k, cap_k + neg_m));
+            e1 = s[i + 1] == -INFINITY ? 0.f : exp2f(soft_cap2(s[i + 1], cap_c, cap_k, cap_k + neg_m));
+          } else if constexpr (kMode == kGeneral) {
+            e0 = exp2f(s[i] + neg_m);
+            e1 = exp2f(s[i + 1] + neg_m);
+          } else {
+            e0 = exp2f(fmaf(s[i], c2, neg_m));
+            e1 = exp2f(fmaf(s[i + 1], c2, neg_m));
+          }
+          sum4[(i >> 1) & 3] += e0 + e1;
+          pw[i >> 1] = pack2<T>(e0, e1);
+          if (i == 62) ptx::tc_st_32x32(tS, pw);
+        }
+        ptx::tc_st_32x32(tS + 32, pw + 32);
+        l_run += (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
+        ptx::tc_wait_st();
+        ptx::tc_fence_before();
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive(bar(P_FULL + t));
+        ++vc;
       }
-      ptx::tc_fence_before();     // our tcgen05.ld of S_j are complete (wait::ld) before the MMA warp may overwrite the buffer
-      ptx::fence_proxy_async();   // P_j (generic-proxy stores) visible to the tensor core's async-proxy reads
-      __syncwarp();
-      if (lane == 0) {
-        ptx::mbar_arrive(bar(S_EMPTY + b));
-        ptx::mbar_arrive(bar(P_FULL));
-      }
-      l_run = fmaf(l_run, alpha, sum);
-      m_run = m_new;
-      if (j > 0) fold(j - 1, alpha_prev);
-      alpha_prev = alpha;
-    }
-    fold(n_kv - 1, alpha_prev);
 
-    if (q_pos < L) {
+      // ---- output: O / l (times the gate), 64 columns at a time through the warp's staging rows
       float inv = 1.f / l_run;
-      if constexpr (kSink) {
-        if (p.gate && p.gate_mode == 1)
-          inv *= 1.f / (1.f + __expf(-rb::to_f(reinterpret_cast<const T*>(p.gate)[(int64_t)(tok0 + q_pos) * p.gate_ld + head])));
-        if (p.gate && p.gate_mode == 2) {          // (rows of the gate are 16-byte aligned: checked by the host)
-          const T* gr = reinterpret_cast<const T*>(p.gate) + (int64_t)(tok0 + q_pos) * p.gate_ld + (int64_t)head * kDV;
+      if constexpr (kMode != kPlain) {
+        if (p.gate && p.gate_mode == 1 && q_pos < L)
+          inv *= 1.f / (1.f + __expf(-rb::to_f(reinterpret_cast<const T*>(p.gate)[(int64_t)(it.tok0 + q_pos) * p.gate_ld + head])));
+      }
+      wait(O_FULL + t, (vc - 1) & 1u);
+      ptx::tc_fence_after();
 #pragma unroll
-          for (int i = 0; i < kDV; i += 8) {
-            const rb::Pack<T, 8> gv = *reinterpret_cast<const rb::Pack<T, 8>*>(gr + i);
+      for (int half = 0; half < kDV / 64; ++half) {
+        uint32_t o[64];
+        ptx::tc_ld_32x32(tO + half * 64, o);
+        ptx::tc_ld_32x32(tO + half * 64 + 32, o + 32);
+        ptx::tc_wait_ld();
+        if (half == kDV / 64 - 1) {
+          ptx::tc_fence_before();
+          __syncwarp();
+          if (lane == 0) ptx::mbar_arrive(bar(O_EMPTY + t));
+        }
+        float of[64];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) O[i + j] *= __fdividef(1.f, 1.f + __expf(-rb::to_f(gv.v[j])));
+        for (int i = 0; i < 64; ++i) of[i] = __uint_as_float(o[i]);
+        if constexpr (kMode != kPlain) {
+          if (p.gate && p.gate_mode == 2 && q_pos < L) {          // (rows of the gate are 16-byte aligned: checked by the host)
+            const T* gr = reinterpret_cast<const T*>(p.gate) + (int64_t)(it.tok0 + q_pos) * p.gate_ld + (int64_t)head * kDV + half * 64;
+#pragma unroll
+            for (int i = 0; i < 64; i += 8) {
+              const rb::Pack<T, 8> gv = *reinterpret_cast<const rb::Pack<T, 8>*>(gr + i);
+#pragma unroll
+              for (int e = 0; e < 8; ++e) of[i + e] *= __fdividef(1.f, 1.f + __expf(-rb::to_f(gv.v[e])));
+            }
           }
         }
-      }
-      T* dst = reinterpret_cast<T*>(p.out) + (int64_t)(tok0 + q_pos) * p.out_ld + (int64_t)head * kDV;
 #pragma unroll
-      for (int i = 0; i < kDV; i += 8) {
-        uint4 v;
-        v.x = pack2<T>(O[i] * inv, O[i + 1] * inv);
-        v.y = pack2<T>(O[i + 2] * inv, O[i + 3] * inv);
-        v.z = pack2<T>(O[i + 4] * inv, O[i + 5] * inv);
-        v.w = pack2<T>(O[i + 6] * inv, O[i + 7] * inv);
-        *reinterpret_cast<uint4*>(dst + i) = v;
+        for (int c = 0; c < 8; ++c)
+          st_shared_v4(stage + lane * 128 + ((c ^ (lane & 7)) << 4), pack2<T>(of[8 * c] * inv, of[8 * c + 1] * inv), pack2<T>(of[8 * c + 2] * inv, of[8 * c + 3] * inv),
+                       pack2<T>(of[8 * c + 4] * inv, of[8 * c + 5] * inv), pack2<T>(of[8 * c + 6] * inv, of[8 * c + 7] * inv));
+        __syncwarp();
+        T* dst = reinterpret_cast<T*>(p.out) + (int64_t)head * kDV + half * 64 + (lane & 7) * 8;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int rr = i * 4 + (lane >> 3), pos = q0 + quad * 32 + rr;
+          const uint4 v = ld_shared_v4(stage + rr * 128 + (((lane & 7) ^ (rr & 7)) << 4));
+          if (pos < L) *reinterpret_cast<uint4*>(dst + (int64_t)(it.tok0 + pos) * p.out_ld) = v;
+        }
+        __syncwarp();
       }
-      if constexpr (!kSink) p.lse[(int64_t)head * p.T + tok0 + q_pos] = m_run * p.scale + __logf(l_run);
+      if constexpr (kMode == kPlain) {
+        if (q_pos < L) p.lse[(int64_t)head * p.T + it.tok0 + q_pos] = m_run * 0.6931471805599453f + __logf(l_run);
+      }
     }
   }
 
@@ -435,37 +481,46 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
     for (int i = 0; i < 1000; ++i) __nanosleep(1000);
     __syncthreads();
   }
-  if (warp == 1) {
+  if (warp == 8) {
     ptx::tc_fence_after();
     ptx::tmem_dealloc(tmem_base, 512);
   }
 }
 
-template <int kD, int kDV, typename T, int kFmt, bool kSink = false, bool kCap = false, bool kSimple = false, bool kBias = false, bool kShared = false>
-int launch_attn_fwd(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const AttnParams& p, int B,
-                    int max_seqlen, cudaStream_t s) {
-  using C = ACfg<kD, kDV, kShared>;
-  auto kern = attn_fwd_kernel<kD, kDV, T, kFmt, kSink, kCap, kSimple, kBias, kShared>;
-  const int smem = C::kSmemBytes + (kBias ? (p.n_bias + kBiasPad) * 4 : 0);
-  if (smem > kMaxSmem) return -32;
+template <int kD, int kDV, typename T, int kFmt, int kMode>
+int launch_attn_fwd(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, AttnParams p, int B, cudaStream_t s) {
+  using C = FCfg<kD, kDV>;
+  static_assert(C::kSmemBytes <= kMaxSmem, "shared memory");
+  auto kern = attn_fwd_kernel<kD, kDV, T, kFmt, kMode>;
   static bool attr_set = false;
   if (!attr_set) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kBias ? kMaxSmem : C::kSmemBytes) != cudaSuccess) return -30;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes) != cudaSuccess) return -30;
     attr_set = true;
   }
-  dim3 grid(RB_CEIL_DIV(max_seqlen, kBQ), p.nq, B);
-  kern<<<grid, kAttnThreads, smem, s>>>(mq, mk, mv, p);
+  p.B = B;
+  p.pair_heads = (p.nq / p.nkv) % 2 == 0;
+  p.n_head_units = p.pair_heads ? p.nq / 2 : p.nq;
+  // the sequences' lengths are on the device: sum of ceil(L / rows) is at most (T + (rows - 1) B) / rows
+  const int64_t rows = p.pair_heads ? kTile : 2 * kTile;
+  const int64_t n = (p.T + (rows - 1) * B) / rows * p.n_head_units;
+  if (n <= 0 || n > 0x7fffffff) return -33;
+  kern<<<dim3((unsigned)n), kFwdThreads, C::kSmemBytes, s>>>(mq, mk, mv, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -31;
 }
 
 }  // namespace
 
-// 1 if a bounded wait of the kernel ran out since the last call (synchronises; for diagnostics)
+extern "C" int rb_attn_bias_wait_error();
+extern "C" int rb_attn_fwd_bias(const CUtensorMap* mq, const CUtensorMap* mk, const CUtensorMap* mv, const AttnParams* p, int B, int hd, int max_seqlen,
+                                int kv_shared, int bf, cudaStream_t s);
+
+// 1 if a bounded wait of the kernels ran out since the last call (synchronises; for diagnostics)
 extern "C" int rb_attn_wait_error() {
   int v = 0, zero = 0;
   if (cudaMemcpyFromSymbol(&v, g_wait_error, sizeof(int)) != cudaSuccess) return -1;
   if (v != 0) cudaMemcpyToSymbol(g_wait_error, &zero, sizeof(int));
-  return v;
+  const int b = rb_attn_bias_wait_error();
+  return b != 0 ? b : v;
 }
 
 // q / k / v: [T, heads, hd] views (unit stride over hd, `heads * hd` contiguous columns, row pitch *_ld elements) -- e.g. the
@@ -482,17 +537,15 @@ extern "C" int rb_attn_fwd_window(const void* q, const void* k, const void* v, v
   if (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)out) & 15) return -5;
   CUtensorMap mq, mk, mv;
   const int bf = dt == 1;
-  if (!make_tmap(&mq, q, bf, T, (uint64_t)nq * hd, q_ld, 64, kBQ)) return -10;
-  if (!make_tmap(&mk, k, bf, T, (uint64_t)nkv * hd, k_ld, 64, kBKV)) return -11;
-  if (!make_tmap(&mv, v, bf, T, (uint64_t)nkv * hd, v_ld, 64, 64)) return -12;  // 64-key halves, see the producer
+  if (!make_tmap(&mq, q, bf, T, (uint64_t)nq * hd, q_ld, 64, kTile)) return -10;
+  if (!make_tmap(&mk, k, bf, T, (uint64_t)nkv * hd, k_ld, 64, kTile)) return -11;
+  if (!make_tmap(&mv, v, bf, T, (uint64_t)nkv * hd, v_ld, 64, kTile)) return -12;
   if (window > 0 && !causal) return -6;
   AttnParams p{cu_seqlens, out, lse, out_ld, T, nq, nkv, scale, causal, window, 0, nullptr, nullptr, nullptr, 0, -1.f};
   if (hd == 128) {
-    return bf ? launch_attn_fwd<128, 128, __nv_bfloat16, 1>(mq, mk, mv, p, B, max_seqlen, s)
-              : launch_attn_fwd<128, 128, __half, 0>(mq, mk, mv, p, B, max_seqlen, s);
+    return bf ? launch_attn_fwd<128, 128, __nv_bfloat16, 1, kPlain>(mq, mk, mv, p, B, s) : launch_attn_fwd<128, 128, __half, 0, kPlain>(mq, mk, mv, p, B, s);
   }
-  return bf ? launch_attn_fwd<64, 64, __nv_bfloat16, 1>(mq, mk, mv, p, B, max_seqlen, s)
-            : launch_attn_fwd<64, 64, __half, 0>(mq, mk, mv, p, B, max_seqlen, s);
+  return bf ? launch_attn_fwd<64, 64, __nv_bfloat16, 1, kPlain>(mq, mk, mv, p, B, s) : launch_attn_fwd<64, 64, __half, 0, kPlain>(mq, mk, mv, p, B, s);
 }
 
 extern "C" int rb_attn_fwd(const void* q, const void* k, const void* v, void* out, float* lse, const int* cu_seqlens,
@@ -501,7 +554,7 @@ extern "C" int rb_attn_fwd(const void* q, const void* k, const void* v, void* ou
   return rb_attn_fwd_window(q, k, v, out, lse, cu_seqlens, q_ld, k_ld, v_ld, out_ld, T, B, nq, nkv, hd, max_seqlen, scale, causal, 0, dt, s);
 }
 
-// Window attention with a sink on the tensor cores (see the kSink notes at the top): q / k [T, heads, hd], v [T, heads, vd] as for
+// Window attention with a sink on the tensor cores (see the modes at the top): q / k [T, heads, hd], v [T, heads, vd] as for
 // rb_attn_fwd (head sizes of 64 or 128), temp / sink [nq] in the operand type or null, gate logits at gate[t * gate_ld + h] (gate_mode
 // 1) or gate[t * gate_ld + h * vd + c] (gate_mode 2) or null, window <= 0 = every earlier key, keep = first keys that stay visible,
 // chunk > 0 = chunked instead of windowed, softcap > 0 = capped scores (kSimple cases only), slope_base < 0 = no distance term, bias
@@ -526,26 +579,25 @@ extern "C" int rb_attn_fwd_sink(const void* q, const void* k, const void* v, voi
   if (hd != vd && (!simple || softcap > 0.f)) return -9;
   CUtensorMap mq, mk, mv;
   const int bf = dt == 1;
-  if (!make_tmap(&mq, q, bf, T, (uint64_t)nq * hd, q_ld, 64, kBQ)) return -10;
-  if (!make_tmap(&mk, k, bf, T, (uint64_t)nkv * hd, k_ld, 64, kBKV)) return -11;
-  if (!make_tmap(&mv, v, bf, T, (uint64_t)(nkv / vshare) * vd, v_ld, 64, 64)) return -12;
+  if (!make_tmap(&mq, q, bf, T, (uint64_t)nq * hd, q_ld, 64, kTile)) return -10;
+  if (!make_tmap(&mk, k, bf, T, (uint64_t)nkv * hd, k_ld, 64, kTile)) return -11;
+  if (!make_tmap(&mv, v, bf, T, (uint64_t)(nkv / vshare) * vd, v_ld, 64, bias != nullptr ? 64 : kTile)) return -12;
   AttnParams p{cu_seqlens, out, nullptr, out_ld, T, nq, nkv, scale, 1, window > 0 ? window : 0, window > 0 ? keep : 0, temp, sink, gate, gate_ld,
                slope_base, vshare, gate_mode, chunk, softcap, bias, window > 0 && n_bias > window ? window : n_bias, n_bias};
-#define RB_GO2(HD, VD, ...)                                                                                               \
-  return bf ? launch_attn_fwd<HD, VD, __nv_bfloat16, 1, true, __VA_ARGS__>(mq, mk, mv, p, B, max_seqlen, s)              \
-            : launch_attn_fwd<HD, VD, __half, 0, true, __VA_ARGS__>(mq, mk, mv, p, B, max_seqlen, s)
-#define RB_GO(...)                                 \
-  if (hd == 128) { RB_GO2(128, 128, __VA_ARGS__); } \
-  RB_GO2(64, 64, __VA_ARGS__)
+  if (bias != nullptr) return rb_attn_fwd_bias(&mq, &mk, &mv, &p, B, hd, max_seqlen, kv_shared, bf, s);
+#define RB_GO2(HD, VD, M)                                                                   \
+  return bf ? launch_attn_fwd<HD, VD, __nv_bfloat16, 1, M>(mq, mk, mv, p, B, s)            \
+            : launch_attn_fwd<HD, VD, __half, 0, M>(mq, mk, mv, p, B, s)
+#define RB_GO(M)                           \
+  if (hd == 128) { RB_GO2(128, 128, M); } \
+  RB_GO2(64, 64, M)
   if (hd != vd) {
-    if (hd == 128) { RB_GO2(128, 64, false, true); }
-    RB_GO2(64, 128, false, true);
+    if (hd == 128) { RB_GO2(128, 64, kSimple); }
+    RB_GO2(64, 128, kSimple);
   }
-  if (bias != nullptr && kv_shared) { RB_GO(false, false, true, true); }
-  if (bias != nullptr) { RB_GO(false, false, true); }
-  if (softcap > 0.f) { RB_GO(true, true); }
-  if (simple) { RB_GO(false, true); }
-  RB_GO(false, false);
+  if (softcap > 0.f) { RB_GO(kCap); }
+  if (simple) { RB_GO(kSimple); }
+  RB_GO(kGeneral);
 #undef RB_GO
 #undef RB_GO2
 }

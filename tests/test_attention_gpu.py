@@ -4,6 +4,7 @@ import torch
 
 from realhf_b200.ops import attention as A
 from realhf_b200.ops import functional as OF
+from realhf_b200.ops import lib
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
@@ -136,3 +137,52 @@ def test_attn_bwd_tcgen05_matches_autograd_of_the_reference(hd, nq, nkv, causal)
     lib().attn_bwd(dout, q, k, v, ref.detach().to(torch.bfloat16), lse, dq, dk, dv, cu, max(lens), scale, causal)
     assert torch.isfinite(dqkv.float()).all()
     torch.testing.assert_close(dqkv.float(), x.grad, atol=6e-2, rtol=6e-2)
+
+
+def _attention_f64(q, k, v, lens, scale, causal, window):
+    """(out, sum of weights * |v|, lse) in float64."""
+    out, mag, lse = torch.zeros(q.shape, dtype=torch.float64, device=DEV), torch.zeros(q.shape, dtype=torch.float64, device=DEV), []
+    a = 0
+    for n in lens:
+        qq, kk, vv = (t[a:a + n].double().transpose(0, 1) for t in (q, k, v))
+        kk, vv = (t.repeat_interleave(q.shape[1] // k.shape[1], 0) for t in (kk, vv))
+        i = torch.arange(n, device=DEV)
+        ok = torch.ones(n, n, dtype=torch.bool, device=DEV)
+        if causal:
+            ok = i[None] <= i[:, None]
+            if window:
+                ok = ok & (i[None] > i[:, None] - window)
+        s = (qq @ kk.transpose(1, 2) * scale).masked_fill(~ok, float("-inf"))
+        p = torch.softmax(s, -1)
+        out[a:a + n], mag[a:a + n] = (p @ vv).transpose(0, 1), (p @ vv.abs()).transpose(0, 1)
+        lse.append(torch.logsumexp(s, -1))
+        a += n
+    return out, mag, torch.cat(lse, 1)
+
+
+@pytest.mark.parametrize("heads", [(1, 1, 128), (4, 2, 64), (3, 1, 128), (6, 3, 128), (2, 2, 64), (8, 1, 128)])
+@pytest.mark.parametrize("lens", [[1], [127, 128, 129, 255, 256, 257], [0, 5, 0, 640, 1], [33] * 70 + [1100], [1536, 385]])
+@pytest.mark.parametrize("form", ["causal", "full", "window", "growing"])
+def test_attn_fwd_tile_pairs(heads, lens, form):
+    """Tile pairs over heads (even groups) and over rows (odd groups), left-over tiles, empty sequences, more than 32 sequences, windows, and scores
+    whose maximum grows by far more than the lazy step from tile to tile.  Bound: the weights and the result are rounded to 16 bits once each,
+    2^-9 of the weighted sum of |v| and 2^-9 of the result, doubled for the exponentials and the stale maximum's factor."""
+    nq, nkv, hd = heads
+    dt = torch.float16 if form == "window" else torch.bfloat16
+    torch.manual_seed(len(lens) + nq)
+    T = sum(lens)
+    qkv = torch.randn(T, (nq + 2 * nkv) * hd, device=DEV)
+    if form == "growing":                    # queries and keys share a direction that grows with the position: row maxima climb by hundreds
+        pos = torch.cat([torch.arange(n, device=DEV) for n in lens]).float()
+        qkv[:, 0:nq * hd:hd] = 8.0
+        qkv[:, nq * hd:(nq + nkv) * hd:hd] = pos[:, None] / 8
+    qkv = qkv.to(dt)
+    q, k, v = (t.view(T, -1, hd) for t in qkv.split([nq * hd, nkv * hd, nkv * hd], 1))
+    cu = torch.tensor([0] + list(torch.tensor(lens).cumsum(0)), dtype=torch.int32, device=DEV)
+    window = 150 if form == "window" else 0
+    out, lse = lib().attn_fwd_window(q, k, v, cu, max(lens), hd ** -0.5, form != "full", window)
+    assert lib().attn_wait_error() == 0
+    ref, mag, rlse = _attention_f64(q, k, v, lens, hd ** -0.5, form != "full", window)
+    eps = 2.0 ** (-8 if dt == torch.bfloat16 else -11)
+    assert ((out.double() - ref).abs() <= eps * ref.abs() + eps * mag + 1e-6).all()
+    torch.testing.assert_close(lse.double(), rlse, atol=2e-5, rtol=2e-6)
