@@ -11,7 +11,7 @@
 // rows (grouped heads, even group: both walk the same tiles), else two neighbouring query tiles of a head (counted from the end of
 // the sequence, so that a left-over single tile is the shortest one).  Sharing the stream also halves the L2 traffic per product: one
 // tile each would ask for 64 B per cycle and SM, more than L2 gives.  With one tile per CTA and four softmax warps the tensor pipe was
-// active 19% of the time: 32 x 640 tokens x 32 heads took 527 us (now 294), 8 x 1500..4096 x 32 / 8 heads 2396 us (now 1023).
+// active 19% of the time: 32 x 640 tokens x 32 heads took 527 us (now 221), 8 x 1500..4096 x 32 / 8 heads 2396 us (now 751).
 //
 // CTA = 12 warps, one CTA per SM.  Warps 0-3 / 4-7: softmax of tile 0 / 1 (thread = query row = TMEM lane).  Warp 8: MMA issue and TMEM
 // allocation.  Warp 9: TMA producer and scheduler (10, 11: idle, they complete the warpgroup whose registers go to the softmax).  The
@@ -24,7 +24,9 @@
 // accumulates in TMEM over the whole stream.  The row maximum that weights are taken against only moves when a tile's maximum exceeds it
 // by more than 2^8 (then the warp scales O once the product in flight has retired): weights, sum and output carry the same factor, so the
 // result is the softmax of the same scores, and fp32 / bf16 / fp16 all have room for 2^8.  V_j is the MN-major B operand.
-// Issue order: S_0, S_1, then per key tile PV_0, S_0', PV_1, S_1'.
+// Issue order: S_0, S_1, then per key tile PV_0, S_0', PV_1, S_1'.  The issuing warp runs converged and elects a lane for the MMAs alone: issued from
+// `if (lane == 0)` with descriptors built there, eight MMAs took 820-960 cycles of one thread, whatever their size (294 -> 242 us converged, 231 us with the
+// descriptors built in front of the elected branch; two scores per instruction in the softmax: 221 us).
 //
 // Outputs: O [T, nq, DV] through a per-warp staging buffer (whole 128-byte lines), LSE [nq, T] (natural log, scale applied).
 //
@@ -34,7 +36,7 @@
 // maximum is taken over the raw products.  kCap: kSimple with score = softcap * tanh(s * scale / softcap); the cap is monotone, so the
 // raw maximum is capped once.  All three: a per-head sink logit starts the running maximum with denominator 1; the output is
 // multiplied by sigmoid(gate logit of its head, or of the output element); `chunk` > 0 replaces the window: a query sees the keys of its own
-// chunk of positions up to itself.  (32 x 1024 tokens, 16 / 4 heads, window 512 + 64 kept: 1382 us with one tile per CTA, now 316.)
+// chunk of positions up to itself.  (32 x 1024 tokens, 16 / 4 heads, window 512 + 64 kept: 1382 us with one tile per CTA, now 259.)
 // Learned distance biases and shared keys / values run in attn_fwd_bias.cu.
 #include "attn_common.cuh"
 
@@ -59,6 +61,16 @@ enum FBar { Q_FULL = 0, Q_EMPTY = 2, KV_FULL = 4, KV_EMPTY = 8, S_FULL = 12, P_F
             CLC_FULL = 24, F_NUM_BARS = 25 };
 
 __device__ int g_wait_error = 0;
+
+// (x0, x1) <- (x0, x1) * m + a and (s0, s1) <- (s0, s1) + (a0, a1), one instruction each
+RB_DEVICE void fma_pair(float& x0, float& x1, float m, float a) {
+  asm("{\n\t.reg .b64 x, m, a;\n\tmov.b64 x, {%0, %1};\n\tmov.b64 m, {%2, %2};\n\tmov.b64 a, {%3, %3};\n\tfma.rn.f32x2 x, x, m, a;\n\tmov.b64 {%0, %1}, x;\n\t}"
+      : "+f"(x0), "+f"(x1) : "f"(m), "f"(a));
+}
+RB_DEVICE void add_pair(float& s0, float& s1, float a0, float a1) {
+  asm("{\n\t.reg .b64 s, a;\n\tmov.b64 s, {%0, %1};\n\tmov.b64 a, {%2, %3};\n\tadd.rn.f32x2 s, s, a;\n\tmov.b64 {%0, %1}, s;\n\t}"
+      : "+f"(s0), "+f"(s1) : "f"(a0), "f"(a1));
+}
 
 // One work item: sequence (first token, length), heads and query tiles of the two tiles (tile 1 < 0: absent); L < 0 ends the CTA's loop.
 struct Item { int tok0, L, head0, head1, qt0, qt1; };
@@ -228,70 +240,83 @@ __global__ void __launch_bounds__(kFwdThreads, 1) attn_fwd_kernel(const __grid_c
       }
       publish(Item{0, -1, 0, 0, -1, -1});
     } else if (warp == 8) {
-      // ===================================================== MMA issuer
-      if (lane == 0) {
-        constexpr uint32_t idesc_s = ptx::make_idesc_f16(kFmt, kTile, kTile, 0, 0);   // Q, K both K-major (head-dim contiguous)
-        constexpr uint32_t idesc_o = ptx::make_idesc_f16(kFmt, kTile, kDV, 0, 1);     // P (TMEM), V MN-major
-        uint32_t kvc = 0, qc[2] = {0, 0}, pc[2] = {0, 0}, oc[2] = {0, 0};
-        for (int n_it = 0;; ++n_it) {
-          const int slot = n_it & 1;
-          wait(IT_FULL + slot, (uint32_t)(n_it >> 1) & 1u);
-          const Item it = items[slot];
-          ptx::mbar_arrive(bar(IT_EMPTY + slot));
-          if (it.L < 0 || *dead) break;
-          const Walk w(it, p);
-          bool s_open[2] = {false, false}, o_open[2] = {false, false};
-          auto issue_s = [&](int t, int j, int st) {
-            if (!s_open[t]) { wait(Q_FULL + t, qc[t] & 1u); ++qc[t]; s_open[t] = true; }
-            ptx::tc_fence_after();
+      // ===================================================== MMA issuer: the whole warp runs the loop, one elected lane issues
+      constexpr uint32_t idesc_s = ptx::make_idesc_f16(kFmt, kTile, kTile, 0, 0);   // Q, K both K-major (head-dim contiguous)
+      constexpr uint32_t idesc_o = ptx::make_idesc_f16(kFmt, kTile, kDV, 0, 1);     // P (TMEM), V MN-major
+      const uint32_t tm = (uint32_t)ptx::uniform((int)tmem_base);
+      uint32_t kvc = 0, qc[2] = {0, 0}, pc[2] = {0, 0}, oc[2] = {0, 0};
+      for (int n_it = 0;; ++n_it) {
+        const int slot = n_it & 1;
+        wait(IT_FULL + slot, (uint32_t)(n_it >> 1) & 1u);
+        Item it = items[slot];
+        it.L = ptx::uniform(it.L);
+        it.qt0 = ptx::uniform(it.qt0);
+        it.qt1 = ptx::uniform(it.qt1);
+        if (lane == 0) ptx::mbar_arrive(bar(IT_EMPTY + slot));
+        __syncwarp();
+        if (it.L < 0 || ptx::uniform((int)*dead)) break;
+        const Walk w(it, p);
+        bool s_open[2] = {false, false}, o_open[2] = {false, false};
+        auto issue_s = [&](int t, int j, int st) {
+          if (!s_open[t]) { wait(Q_FULL + t, qc[t] & 1u); ++qc[t]; s_open[t] = true; }
+          ptx::tc_fence_after();
+          const uint64_t a = ptx::make_smem_desc_sw128(sQ + t * C::kQBytes, 16, 1024), b = ptx::make_smem_desc_sw128(sKV + st * C::kStageBytes, 16, 1024);
+          if (ptx::elect_one()) {
 #pragma unroll
             for (int kk = 0; kk < kD / 16; ++kk) {
               const uint32_t off = (kk >> 2) * (kTile * 128) + (kk & 3) * 32;
-              ptx::tc_mma_f16(tmem_base + t * 128, ptx::make_smem_desc_sw128(sQ + t * C::kQBytes + off, 16, 1024),
-                              ptx::make_smem_desc_sw128(sKV + st * C::kStageBytes + off, 16, 1024), idesc_s, kk != 0 ? 1u : 0u);
+              ptx::tc_mma_f16(tm + t * 128, a + (off >> 4), b + (off >> 4), idesc_s,
+                              kk != 0 ? 1u : 0u);
             }
             ptx::tc_commit(bar(S_FULL + t));
             if (j == (t ? w.end1 : w.end0) - 1) ptx::tc_commit(bar(Q_EMPTY + t));
-          };
-          auto issue_pv = [&](int t, int st) {
-            wait(P_FULL + t, pc[t] & 1u);
-            ++pc[t];
-            if (!o_open[t]) { wait(O_EMPTY + t, (oc[t] & 1u) ^ 1u); ++oc[t]; }
-            ptx::tc_fence_after();
+          }
+          __syncwarp();
+        };
+        auto issue_pv = [&](int t, int st) {
+          wait(P_FULL + t, pc[t] & 1u);
+          ++pc[t];
+          if (!o_open[t]) { wait(O_EMPTY + t, (oc[t] & 1u) ^ 1u); ++oc[t]; }
+          ptx::tc_fence_after();
+          const uint64_t b = ptx::make_smem_desc_sw128(sKV + st * C::kStageBytes, kTile * 128, 1024);
+          if (ptx::elect_one()) {
 #pragma unroll
             for (int kk = 0; kk < kTile / 16; ++kk)      // A: 16 keys = 8 TMEM columns; B: 16 key rows = 2048 B down every 64-wide chunk of DV
-              ptx::tc_mma_f16_ts(tmem_base + 256 + t * 128, tmem_base + t * 128 + kk * 8,
-                                 ptx::make_smem_desc_sw128(sKV + st * C::kStageBytes + kk * 2048, kTile * 128, 1024), idesc_o,
+              ptx::tc_mma_f16_ts(tm + 256 + t * 128, tm + t * 128 + kk * 8, b + kk * 128, idesc_o,
                                  (o_open[t] || kk != 0) ? 1u : 0u);
-            o_open[t] = true;
             ptx::tc_commit(bar(O_FULL + t));
-          };
-          auto open_kv = [&](uint32_t c) { wait(KV_FULL + (c & (kStages - 1)), (c / kStages) & 1u); return (int)(c & (kStages - 1)); };
-          int st = open_kv(kvc);
-#pragma unroll
-          for (int t = 0; t < 2; ++t)
-            if (w.takes(t, w.tile(0))) issue_s(t, w.tile(0), st);
-          ptx::tc_commit(bar(KV_EMPTY + st));
-          for (int k = 0; k < w.n; ++k) {
-            const int j = w.tile(k), jn = w.tile(k + 1);
-            const bool more = k + 1 < w.n;
-            const int sv = open_kv(kvc + 2 * k + 1);
-            int sk = -1;
-#pragma unroll
-            for (int t = 0; t < 2; ++t) {
-              if (w.takes(t, j)) issue_pv(t, sv);
-              if (t == 1) ptx::tc_commit(bar(KV_EMPTY + sv));
-              if (more) {
-                if (sk < 0) sk = open_kv(kvc + 2 * k + 2);
-                if (w.takes(t, jn)) issue_s(t, jn, sk);
-              }
-            }
-            if (more) ptx::tc_commit(bar(KV_EMPTY + sk));
           }
-          kvc += 2 * w.n;
+          __syncwarp();
+          o_open[t] = true;
+        };
+        auto open_kv = [&](uint32_t c) { wait(KV_FULL + (c & (kStages - 1)), (c / kStages) & 1u); return (int)(c & (kStages - 1)); };
+        auto free_kv = [&](int st) {
+          if (ptx::elect_one()) ptx::tc_commit(bar(KV_EMPTY + st));
+          __syncwarp();
+        };
+        int st = open_kv(kvc);
+#pragma unroll
+        for (int t = 0; t < 2; ++t)
+          if (w.takes(t, w.tile(0))) issue_s(t, w.tile(0), st);
+        free_kv(st);
+        for (int k = 0; k < w.n; ++k) {
+          const int j = w.tile(k), jn = w.tile(k + 1);
+          const bool more = k + 1 < w.n;
+          const int sv = open_kv(kvc + 2 * k + 1);
+          int sk = -1;
+#pragma unroll
+          for (int t = 0; t < 2; ++t) {
+            if (w.takes(t, j)) issue_pv(t, sv);
+            if (t == 1) free_kv(sv);
+            if (more) {
+              if (sk < 0) sk = open_kv(kvc + 2 * k + 2);
+              if (w.takes(t, jn)) issue_s(t, jn, sk);
+            }
+          }
+          if (more) free_kv(sk);
         }
+        kvc += 2 * w.n;
       }
-      __syncwarp();
     }
   } else {
     ptx::reg_inc<kSoftmaxRegs>();
@@ -405,10 +430,12 @@ __global__ void __launch_bounds__(kFwdThreads, 1) attn_fwd_kernel(const __grid_c
             e0 = exp2f(s[i] + neg_m);
             e1 = exp2f(s[i + 1] + neg_m);
           } else {
-            e0 = exp2f(fmaf(s[i], c2, neg_m));
-            e1 = exp2f(fmaf(s[i + 1], c2, neg_m));
+            float x0 = s[i], x1 = s[i + 1];
+            fma_pair(x0, x1, c2, neg_m);
+            e0 = exp2f(x0);
+            e1 = exp2f(x1);
           }
-          sum4[(i >> 1) & 3] += e0 + e1;
+          add_pair(sum4[i & 2], sum4[(i & 2) + 1], e0, e1);
           pw[i >> 1] = pack2<T>(e0, e1);
           if (i == 62) ptx::tc_st_32x32(tS, pw);
         }

@@ -10,6 +10,18 @@ namespace ptx {
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
+// ------------------------------------------------------------------ warp-uniform issue
+// tcgen05.mma / commit take their operands from uniform registers.  Inside `if (lane == 0)` the compiler cannot use the uniform datapath and
+// moves every operand across (~100 cycles per MMA, whatever its size); in code that all 32 lanes run with values the compiler knows to be
+// uniform, `elect_one()` around the instruction alone leaves the descriptors in uniform registers.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t ok;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok));
+  return ok != 0;
+}
+// a value all lanes hold, as one the compiler knows to be uniform
+__device__ __forceinline__ int uniform(int v) { return __reduce_max_sync(0xffffffffu, v); }
+
 // ------------------------------------------------------------------ mbarrier
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
@@ -132,6 +144,14 @@ __device__ __forceinline__ void tc_ld_32x32(uint32_t taddr, uint32_t* r) {
       : "memory");
 }
 
+// the same with 16 columns
+__device__ __forceinline__ void tc_ld_32x16(uint32_t taddr, uint32_t* r) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]),
+                 "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+               : "r"(taddr)
+               : "memory");
+}
 __device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 // thread i of the warp writes 32 consecutive 32-bit columns of row (lane_base + i)
 __device__ __forceinline__ void tc_st_32x32(uint32_t taddr, const uint32_t* r) {
@@ -142,6 +162,14 @@ __device__ __forceinline__ void tc_st_32x32(uint32_t taddr, const uint32_t* r) {
       "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]),
       "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31]), "r"(taddr)
       : "memory");
+}
+
+// the same with 16 columns
+__device__ __forceinline__ void tc_st_32x16(uint32_t taddr, const uint32_t* r) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15};" ::"r"(r[0]), "r"(r[1]), "r"(r[2]),
+               "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]),
+               "r"(r[15]), "r"(taddr)
+               : "memory");
 }
 
 // ------------------------------------------------------------------ register split (executed by every warp of a warpgroup)
