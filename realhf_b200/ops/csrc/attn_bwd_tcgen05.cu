@@ -5,29 +5,35 @@
 //
 //   pass "dKV" (CTA = 128 keys of one kv head): resident K_j, V_j; streams Q_t, dO_t over all q blocks at / below the
 //       diagonal and over the q heads of the GQA group.  Transposed orientation -- tensor-memory lanes are KEYS:
-//         S^T = K_j Q_t^T      dP^T = V_j dO_t^T                         (two M=128, N=64, K=D MMAs per step)
+//         S^T = K_j Q_t^T      dP^T = V_j dO_t^T                         (two M=128, N=64, K=D products per step)
 //         P^T = exp2(S^T * scale*log2e - lse_q * log2e)                  (softmax statistics vary along columns)
 //         dS^T = P^T o (dP^T - delta_q) * scale
-//         dV_j += P^T dO_t     dK_j += dS^T Q_t                          (two M=128, N=D, K=64 MMAs per step)
+//         dV_j += P^T dO_t     dK_j += dS^T Q_t                          (two M=128, N=D, K=64 products per step)
 //   pass "dQ" (CTA = 128 query rows of one q head): resident Q_i, dO_i; streams K_t, V_t up to the diagonal:
 //         S = Q_i K_t^T        dP = dO_i V_t^T      dS = P o (dP - delta) * scale      dQ_i += dS K_t
 //
 // The streamed tiles are used twice with two different descriptors over the same bytes: as the K-major B operand of the
-// S-type MMAs (rows = N) and as the MN-major B operand of the accumulating MMAs (rows = K), exactly the two operand forms of
-// the GEMM kernel (forward / wgrad).  P^T, dS^T (or dS) are written by the softmax threads as bf16 in the K-major
-// SWIZZLE_128B layout and consumed as A operands.  S / dP tensor-memory buffers and the P-type shared buffers are double
-// buffered: the tensor pipe runs the S-type MMAs of step t+1 while the threads work on step t.
-// Recomputing S and dP in both passes costs 7 instead of 5 MMAs per block pair; in exchange the result is deterministic,
+// S-type products (rows = N) and as the MN-major B operand of the accumulating products (rows = K), exactly the two operand forms of
+// the GEMM kernel (forward / wgrad).  P^T and dS^T (or dS) overwrite the front of the S / dP columns they came from, as 16-bit TMEM A operands
+// of the accumulating products: they never travel through shared memory, and since the tensor pipe runs in issue order no buffer needs an
+// "empty" barrier.  S / dP are double buffered: the pipe runs the S-type products of step t+1 while the threads work on step t.
+// Recomputing S and dP in both passes costs 7 instead of 5 products per block pair; in exchange the result is deterministic,
 // there is no fp32 dQ scratch tensor to zero / convert, and dK / dV of a GQA group are reduced inside one CTA.
 //
+// What bounds it: a step is 1024 (dKV) or 768 (dQ) tensor-pipe cycles at D = 128, and its 8192 elements take the CUDA cores about as long when
+// eight warps share them (a warp has 32 rows and 32 of the 64 columns).  Four warps, P through shared memory, the streamed rows' statistics
+// fetched from global memory inside every step and MMAs issued from a divergent branch kept the tensor pipe 19% busy (32 x 640 tokens x 32
+// heads: dKV 613, dQ 506 us, now 412, 388; 8 x 1500..4096, 32 / 8 heads: 2473, 2109 us, now 1777, 1662).
+//
 // delta[h, t] = sum_d dO[t, h, d] * O[t, h, d] comes from a small pre-pass; LSE is the forward's ([nq, T], natural log).
-#include "gemm_common.cuh"
+#include "attn_common.cuh"
 
 namespace {
 
 constexpr int kR = 128;   // resident rows per CTA (= UMMA M)
-constexpr int kX = 64;    // streamed rows per step (= UMMA N of the S-type MMAs, K of the accumulating MMAs)
-constexpr int kBwdThreads = 192;
+constexpr int kX = 64;    // streamed rows per step (= UMMA N of the S-type products, K of the accumulating ones)
+constexpr int kXStages = 4;
+constexpr int kBwdThreads = 320;   // warp 0: TMA, warp 1: MMA, warps 2-9: elements (two per TMEM quadrant, one per column half)
 
 struct BwdParams {
   const int* cu_seqlens;
@@ -41,31 +47,21 @@ struct BwdParams {
   int causal;
 };
 
-template <int kD, bool kDKV> struct BCfg {
+template <int kD> struct BCfg {
   static constexpr int kDBlocks = kD / 64;
   static constexpr int kRBytes = kR * kD * 2;     // one resident tile
   static constexpr int kXBytes = kX * kD * 2;     // one streamed tile
-  static constexpr int kPBytes = kR * kX * 2;     // one P-type buffer [128 x 64] bf16 = one 16 KB swizzle block
-  static constexpr int kPBufs = kDKV ? 2 : 1;     // P^T and dS^T, or dS only
-  static constexpr int kSmemData = 2 * kRBytes + 4 * kXBytes + 2 * kPBufs * kPBytes;
-  static constexpr int kSmemBytes = kSmemData + 1024 /*align*/ + 256 /*barriers*/ + (kDKV ? 2 * 2 * kX * 4 : 0) /*stats*/;
+  static constexpr int kBars = 2 * kRBytes + kXStages * 2 * kXBytes;
+  static constexpr int kStats = kBars + 256;      // [2 buffers][lse | delta][64]
+  static constexpr int kSmemBytes = kStats + 2 * 2 * kX * 4 + 1024 /*align*/;
 };
 
-enum BBar { R_FULL = 0, X_FULL = 1, X_EMPTY = 3, S_FULL = 5, S_EMPTY = 7, P_FULL = 9, P_EMPTY = 11, ACC_FULL = 13, B_NUM_BARS = 14 };
+enum BBar { R_FULL = 0, X_FULL = 1, X_EMPTY = X_FULL + kXStages, S_FULL = X_EMPTY + kXStages, P_FULL = S_FULL + 2, ACC_FULL = P_FULL + 2,
+            B_NUM_BARS = ACC_FULL + 1 };
 
-RB_DEVICE void st_shared_v4b(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
-  asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
-}
-template <typename T> RB_DEVICE uint32_t pack2b(float lo, float hi);
-template <> RB_DEVICE uint32_t pack2b<__nv_bfloat16>(float lo, float hi) {
-  __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
-  return *reinterpret_cast<uint32_t*>(&v);
-}
-template <> RB_DEVICE uint32_t pack2b<__half>(float lo, float hi) {
-  __half2 v = __floats2half2_rn(lo, hi);
-  return *reinterpret_cast<uint32_t*>(&v);
-}
-RB_DEVICE void softmax_bar_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
+__device__ int g_wait_error = 0;
+
+RB_DEVICE void element_bar_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
 
 // tma_r1 / tma_r2: resident operands (box 64 cols x 128 rows); tma_x1 / tma_x2: streamed operands (box 64 x 64).
 //   kDKV: r1 = K, r2 = V (kv-head columns), x1 = Q, x2 = dO (q-head columns).   !kDKV: r1 = Q, r2 = dO, x1 = K, x2 = V.
@@ -73,8 +69,8 @@ template <int kD, typename T, int kFmt, bool kDKV>
 __global__ void __launch_bounds__(kBwdThreads, 1) attn_bwd_kernel(const __grid_constant__ CUtensorMap tma_r1,
                                                                   const __grid_constant__ CUtensorMap tma_r2,
                                                                   const __grid_constant__ CUtensorMap tma_x1,
-                                                                  const __grid_constant__ CUtensorMap tma_x2, BwdParams p) {
-  using C = BCfg<kD, kDKV>;
+                                                                  const __grid_constant__ CUtensorMap tma_x2, const __grid_constant__ BwdParams p) {
+  using C = BCfg<kD>;
   const int seq = blockIdx.z, head = blockIdx.y;  // kDKV: kv head; else q head
   const int tile = kDKV ? (int)blockIdx.x : (int)(gridDim.x - 1 - blockIdx.x);  // heaviest tiles first in both passes
   const int tok0 = p.cu_seqlens[seq];
@@ -93,25 +89,24 @@ __global__ void __launch_bounds__(kBwdThreads, 1) attn_bwd_kernel(const __grid_c
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   const uint32_t sR1 = ptx::smem_u32(smem);
   const uint32_t sR2 = sR1 + C::kRBytes;
-  const uint32_t sXr = sR2 + C::kRBytes;            // stage b: X1 at sXr + b * 2 * kXBytes, X2 right after it
-  const uint32_t sP = sXr + 4 * C::kXBytes;         // buffer b: sP + b * kPBufs * kPBytes (+ kPBytes for the second one)
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::kSmemData);
+  const uint32_t sX = sR2 + C::kRBytes;            // stage s: X1 at sX + s * 2 * kXBytes, X2 right after it
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::kBars);
   uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(bars + B_NUM_BARS);
-  float* stats = reinterpret_cast<float*>(smem + C::kSmemData + 256);  // dKV only: [2 buffers][lse | delta][64]
+  volatile uint32_t* dead = tmem_ptr + 1;
+  float* stats = reinterpret_cast<float*>(smem + C::kStats);
   auto bar = [&](int i) { return ptx::smem_u32(&bars[i]); };
+  auto wait = [&](int i, uint32_t parity) { bounded_wait(bar(i), parity, dead); };
   // TMEM columns: S buffers [0,64) [64,128); dP buffers [128,192) [192,256); accumulators at 256 (dV / dQ) and 384 (dK)
   constexpr uint32_t kTmS = 0, kTmDP = 128, kTmAcc1 = 256, kTmAcc2 = 384;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (warp == 0 && lane == 0) {
+    *dead = 0;
     ptx::prefetch_tensormap(&tma_r1);
     ptx::prefetch_tensormap(&tma_r2);
     ptx::prefetch_tensormap(&tma_x1);
     ptx::prefetch_tensormap(&tma_x2);
-    for (int i = 0; i < B_NUM_BARS; ++i) {
-      const bool thread_side = (i == S_EMPTY || i == S_EMPTY + 1 || i == P_FULL || i == P_FULL + 1);
-      ptx::mbar_init(bar(i), thread_side ? 4 : 1);
-    }
+    for (int i = 0; i < B_NUM_BARS; ++i) ptx::mbar_init(bar(i), (i == P_FULL || i == P_FULL + 1) ? 8 : 1);   // one arrival per element warp
     ptx::fence_barrier_init();
   }
   if (warp == 1) {
@@ -126,98 +121,95 @@ __global__ void __launch_bounds__(kBwdThreads, 1) attn_bwd_kernel(const __grid_c
   // step t -> (q head, streamed block)
   auto step_head = [&](int t) { return kDKV ? head * G + t / nblk : head; };
   auto step_blk = [&](int t) { return blk0 + (kDKV ? t % nblk : t); };
-  const int r_head = head;                                   // column block of the resident tiles
-  const int x_kv_head = kDKV ? head : head / G;              // dQ pass streams the kv head of this q head
 
   if (warp == 0) {
     // ===================================================== TMA producer
     if (lane == 0) {
+      const int x_kv_head = kDKV ? head : head / G;            // dQ pass streams the kv head of this q head
       ptx::mbar_arrive_expect_tx(bar(R_FULL), 2 * C::kRBytes);
 #pragma unroll
       for (int kb = 0; kb < C::kDBlocks; ++kb) {
-        ptx::tma_load_2d(sR1 + kb * (kR * 128), &tma_r1, bar(R_FULL), r_head * kD + kb * 64, tok0 + r0);
-        ptx::tma_load_2d(sR2 + kb * (kR * 128), &tma_r2, bar(R_FULL), r_head * kD + kb * 64, tok0 + r0);
+        ptx::tma_load_2d(sR1 + kb * (kR * 128), &tma_r1, bar(R_FULL), head * kD + kb * 64, tok0 + r0);
+        ptx::tma_load_2d(sR2 + kb * (kR * 128), &tma_r2, bar(R_FULL), head * kD + kb * 64, tok0 + r0);
       }
       for (int t = 0; t < n_steps; ++t) {
-        const int b = t & 1;
-        const uint32_t par = (uint32_t)(t >> 1) & 1u;
+        const int st = t % kXStages;
         const int row = tok0 + step_blk(t) * kX;
         const int col = (kDKV ? step_head(t) : x_kv_head) * kD;
-        ptx::mbar_wait(bar(X_EMPTY + b), par ^ 1);
-        ptx::mbar_arrive_expect_tx(bar(X_FULL + b), 2 * C::kXBytes);
-        const uint32_t x1 = sXr + b * 2 * C::kXBytes, x2 = x1 + C::kXBytes;
+        wait(X_EMPTY + st, ((uint32_t)(t / kXStages) & 1u) ^ 1u);
+        ptx::mbar_arrive_expect_tx(bar(X_FULL + st), 2 * C::kXBytes);
+        const uint32_t x1 = sX + st * 2 * C::kXBytes, x2 = x1 + C::kXBytes;
 #pragma unroll
         for (int kb = 0; kb < C::kDBlocks; ++kb) {
-          ptx::tma_load_2d(x1 + kb * (kX * 128), &tma_x1, bar(X_FULL + b), col + kb * 64, row);
-          ptx::tma_load_2d(x2 + kb * (kX * 128), &tma_x2, bar(X_FULL + b), col + kb * 64, row);
+          ptx::tma_load_2d(x1 + kb * (kX * 128), &tma_x1, bar(X_FULL + st), col + kb * 64, row);
+          ptx::tma_load_2d(x2 + kb * (kX * 128), &tma_x2, bar(X_FULL + st), col + kb * 64, row);
         }
       }
     }
+    __syncwarp();
   } else if (warp == 1) {
-    // ===================================================== MMA issuer
-    if (lane == 0) {
-      constexpr uint32_t idesc_s = ptx::make_idesc_f16(kFmt, kR, kX, 0, 0);   // resident x streamed^T, both K-major
-      constexpr uint32_t idesc_a = ptx::make_idesc_f16(kFmt, kR, kD, 0, 1);   // P-type (K-major) x streamed (MN-major)
-      auto issue_sdp = [&](int t) {
-        const int b = t & 1;
-        const uint32_t par = (uint32_t)(t >> 1) & 1u;
-        ptx::mbar_wait(bar(X_FULL + b), par);
-        ptx::mbar_wait(bar(S_EMPTY + b), par ^ 1);
-        ptx::tc_fence_after();
-        const uint32_t x1 = sXr + b * 2 * C::kXBytes, x2 = x1 + C::kXBytes;
+    // ===================================================== MMA issuer: the whole warp runs the loop, one elected lane issues
+    constexpr uint32_t idesc_s = ptx::make_idesc_f16(kFmt, kR, kX, 0, 0);   // resident x streamed^T, both K-major
+    constexpr uint32_t idesc_a = ptx::make_idesc_f16(kFmt, kR, kD, 0, 1);   // P-type (TMEM) x streamed (MN-major)
+    const uint32_t tm = (uint32_t)ptx::uniform((int)tmem_base);
+    const int n = ptx::uniform(n_steps);
+    const uint64_t r1 = ptx::make_smem_desc_sw128(sR1, 16, 1024), r2 = ptx::make_smem_desc_sw128(sR2, 16, 1024);
+    auto issue_sdp = [&](int t) {
+      const int st = t % kXStages;
+      wait(X_FULL + st, (uint32_t)(t / kXStages) & 1u);
+      ptx::tc_fence_after();
+      const uint32_t d = tm + (t & 1) * 64;
+      const uint64_t x1 = ptx::make_smem_desc_sw128(sX + st * 2 * C::kXBytes, 16, 1024);
+      const uint64_t x2 = ptx::make_smem_desc_sw128(sX + st * 2 * C::kXBytes + C::kXBytes, 16, 1024);
+      if (ptx::elect_one()) {
 #pragma unroll
-        for (int kk = 0; kk < kD / 16; ++kk) {
-          const uint32_t ro = (kk >> 2) * (kR * 128) + (kk & 3) * 32, xo = (kk >> 2) * (kX * 128) + (kk & 3) * 32;
-          ptx::tc_mma_f16(tmem_base + kTmS + b * 64, ptx::make_smem_desc_sw128(sR1 + ro, 16, 1024),
-                          ptx::make_smem_desc_sw128(x1 + xo, 16, 1024), idesc_s, kk != 0 ? 1u : 0u);
-        }
+        for (int kk = 0; kk < kD / 16; ++kk)
+          ptx::tc_mma_f16(d + kTmS, r1 + (((kk >> 2) * (kR * 128) + (kk & 3) * 32) >> 4), x1 + (((kk >> 2) * (kX * 128) + (kk & 3) * 32) >> 4), idesc_s,
+                          kk != 0 ? 1u : 0u);
 #pragma unroll
-        for (int kk = 0; kk < kD / 16; ++kk) {
-          const uint32_t ro = (kk >> 2) * (kR * 128) + (kk & 3) * 32, xo = (kk >> 2) * (kX * 128) + (kk & 3) * 32;
-          ptx::tc_mma_f16(tmem_base + kTmDP + b * 64, ptx::make_smem_desc_sw128(sR2 + ro, 16, 1024),
-                          ptx::make_smem_desc_sw128(x2 + xo, 16, 1024), idesc_s, kk != 0 ? 1u : 0u);
-        }
-        ptx::tc_commit(bar(S_FULL + b));
-      };
-      ptx::mbar_wait(bar(R_FULL), 0);
-      issue_sdp(0);
-      for (int t = 0; t < n_steps; ++t) {
-        if (t + 1 < n_steps) issue_sdp(t + 1);
-        const int b = t & 1;
-        const uint32_t par = (uint32_t)(t >> 1) & 1u;
-        ptx::mbar_wait(bar(P_FULL + b), par);
-        ptx::tc_fence_after();
-        const uint32_t x1 = sXr + b * 2 * C::kXBytes, x2 = x1 + C::kXBytes;
-        const uint32_t pb = sP + b * C::kPBufs * C::kPBytes;
+        for (int kk = 0; kk < kD / 16; ++kk)
+          ptx::tc_mma_f16(d + kTmDP, r2 + (((kk >> 2) * (kR * 128) + (kk & 3) * 32) >> 4), x2 + (((kk >> 2) * (kX * 128) + (kk & 3) * 32) >> 4), idesc_s,
+                          kk != 0 ? 1u : 0u);
+        ptx::tc_commit(bar(S_FULL + (t & 1)));
+      }
+      __syncwarp();
+    };
+    wait(R_FULL, 0);
+    issue_sdp(0);
+    for (int t = 0; t < n; ++t) {
+      if (t + 1 < n) issue_sdp(t + 1);       // its S / dP columns: the products that read P of step t-1 there are ahead in the pipe
+      const int st = t % kXStages;
+      wait(P_FULL + (t & 1), (uint32_t)(t >> 1) & 1u);
+      ptx::tc_fence_after();
+      const uint32_t a = tm + (t & 1) * 64;
+      const uint64_t x1 = ptx::make_smem_desc_sw128(sX + st * 2 * C::kXBytes, kX * 128, 1024);
+      const uint64_t x2 = ptx::make_smem_desc_sw128(sX + st * 2 * C::kXBytes + C::kXBytes, kX * 128, 1024);
+      const uint32_t keep = t != 0 ? 1u : 0u;
+      if (ptx::elect_one()) {
 #pragma unroll
         for (int kk = 0; kk < kX / 16; ++kk) {
-          const uint32_t acc = (t | kk) != 0 ? 1u : 0u;
-          // A: 16 streamed rows = 32 B inside the 128 B row of the P-type buffer; B: 16 rows = 2048 B down every 64-wide chunk
+          // A: 16 streamed rows = 8 columns, the two halves of a row 32 columns apart; B: 16 rows = 2048 B down every 64-wide chunk
+          const uint32_t ao = (kk >> 1) * 32 + (kk & 1) * 8;
           if constexpr (kDKV) {
-            ptx::tc_mma_f16(tmem_base + kTmAcc1, ptx::make_smem_desc_sw128(pb + kk * 32, 16, 1024),
-                            ptx::make_smem_desc_sw128(x2 + kk * 2048, kX * 128, 1024), idesc_a, acc);  // dV += P^T dO
-            ptx::tc_mma_f16(tmem_base + kTmAcc2, ptx::make_smem_desc_sw128(pb + C::kPBytes + kk * 32, 16, 1024),
-                            ptx::make_smem_desc_sw128(x1 + kk * 2048, kX * 128, 1024), idesc_a, acc);  // dK += dS^T Q
+            ptx::tc_mma_f16_ts(tm + kTmAcc1, a + kTmS + ao, x2 + kk * 128, idesc_a, kk != 0 ? 1u : keep);    // dV += P^T dO
+            ptx::tc_mma_f16_ts(tm + kTmAcc2, a + kTmDP + ao, x1 + kk * 128, idesc_a, kk != 0 ? 1u : keep);   // dK += dS^T Q
           } else {
-            ptx::tc_mma_f16(tmem_base + kTmAcc1, ptx::make_smem_desc_sw128(pb + kk * 32, 16, 1024),
-                            ptx::make_smem_desc_sw128(x1 + kk * 2048, kX * 128, 1024), idesc_a, acc);  // dQ += dS K
+            ptx::tc_mma_f16_ts(tm + kTmAcc1, a + kTmDP + ao, x1 + kk * 128, idesc_a, kk != 0 ? 1u : keep);   // dQ += dS K
           }
         }
-        ptx::tc_commit(bar(X_EMPTY + b));
-        ptx::tc_commit(bar(P_EMPTY + b));
+        ptx::tc_commit(bar(X_EMPTY + st));
+        if (t == n - 1) ptx::tc_commit(bar(ACC_FULL));
       }
-      ptx::tc_commit(bar(ACC_FULL));
+      __syncwarp();
     }
   } else {
-    // ===================================================== softmax-gradient threads (thread = resident row = TMEM lane)
-    const int quad = warp & 3;
-    const int row = quad * 32 + lane;
-    const int tid = row;  // 0..127 among these four warps (warps 2,3,4,5 own quadrants 2,3,0,1)
+    // ===================================================== element threads (thread = resident row = TMEM lane, and one half of the columns)
+    const int quad = warp & 3, half = (warp - 2) >> 2;
+    const int row = quad * 32 + lane, tid = threadIdx.x - 64;
     const int r_pos = r0 + row;  // key (dKV) / query (dQ) position of this thread inside the sequence
+    const int rw = r0 + quad * 32;
     const uint32_t lane_addr = tmem_base + ((uint32_t)(quad * 32) << 16);
     const float sl2 = p.scale * 1.4426950408889634f;
-    const uint32_t p_row_off = (uint32_t)(row >> 3) * 1024u + (uint32_t)(row & 7) * 128u;
-    const uint32_t sw = (uint32_t)(row & 7);
     float lse_r = INFINITY, delta_r = 0.f;  // dQ pass: per-row statistics in registers
     if constexpr (!kDKV) {
       if (r_pos < L) {
@@ -225,134 +217,163 @@ __global__ void __launch_bounds__(kBwdThreads, 1) attn_bwd_kernel(const __grid_c
         delta_r = p.delta[(int64_t)head * p.T + tok0 + r_pos];
       }
     }
+    // dKV: statistics of a step's 64 streamed queries, [lse * log2e | delta], fetched a step ahead by the first 128 threads; rows past the end of
+    // the sequence get lse = +inf, which zeroes their probabilities
+    auto fetch_stat = [&](int t) {
+      float v = tid < 64 ? INFINITY : 0.f;
+      const int qpos = step_blk(t) * kX + (tid & 63);
+      if (tid < 128 && qpos < L) {
+        const int64_t idx = (int64_t)step_head(t) * p.T + tok0 + qpos;
+        v = tid < 64 ? p.lse[idx] * 1.4426950408889634f : p.delta[idx];
+      }
+      return v;
+    };
+    float stat = kDKV ? fetch_stat(0) : 0.f;
 
     for (int t = 0; t < n_steps; ++t) {
       const int b = t & 1;
-      const uint32_t par = (uint32_t)(t >> 1) & 1u;
-      const int x0 = step_blk(t) * kX;  // first streamed position (query for dKV, key for dQ)
+      const int x0 = step_blk(t) * kX + half * 32;  // first streamed position of this warp's columns (query for dKV, key for dQ)
       if constexpr (kDKV) {
-        // statistics of the 64 streamed queries, shared by all 128 threads: [lse * log2e | delta]; rows past the end of the
-        // sequence get lse = +inf, which zeroes their probabilities
-        const int h = step_head(t);
-        const int c = tid & 63, qpos = x0 + c;
-        float v = tid < 64 ? INFINITY : 0.f;
-        if (qpos < L) {
-          const int64_t idx = (int64_t)h * p.T + tok0 + qpos;
-          v = tid < 64 ? p.lse[idx] * 1.4426950408889634f : p.delta[idx];
-        }
-        stats[b * 128 + tid] = v;
-        softmax_bar_sync();
+        if (tid < 128) stats[b * 128 + tid] = stat;
+        if (t + 1 < n_steps) stat = fetch_stat(t + 1);
+        element_bar_sync();
       }
-      ptx::mbar_wait(bar(S_FULL + b), par);
+      wait(S_FULL + b, (uint32_t)(t >> 1) & 1u);
       ptx::tc_fence_after();
-      ptx::mbar_wait(bar(P_EMPTY + b), par ^ 1);  // the accumulating MMAs of step t-2 are done with these shared buffers
-      bool need_mask;
-      if constexpr (kDKV) need_mask = p.causal && (r0 + kR - 1 > x0);                    // some key > some query
-      else need_mask = (x0 + kX > L) || (p.causal && x0 + kX - 1 > r0);                   // key past the end / above the diagonal
-      const uint32_t pb = sP + b * C::kPBufs * C::kPBytes + p_row_off;
+      const uint32_t tS = lane_addr + kTmS + b * 64 + half * 32, tDP = lane_addr + kTmDP + b * 64 + half * 32;
+      bool need_mask, none;         // some / all elements of the warp's block are hidden (uniform)
+      if constexpr (kDKV) {
+        need_mask = p.causal && rw + 31 > x0;                        // some key > some query
+        none = x0 >= L || (p.causal && rw > x0 + 31);
+      } else {
+        need_mask = x0 + 32 > L || (p.causal && x0 + 31 > rw);        // key past the end / above the diagonal
+        none = x0 >= L || (p.causal && x0 > rw + 31);
+      }
+      uint32_t wp[16], wd[16];
+      if (none) {
 #pragma unroll
-      for (int c = 0; c < kX / 32; ++c) {
+        for (int i = 0; i < 16; ++i) wp[i] = wd[i] = 0u;
+      } else {
         uint32_t rs[32], rd[32];
-        ptx::tc_ld_32x32(lane_addr + kTmS + b * 64 + c * 32, rs);
-        ptx::tc_ld_32x32(lane_addr + kTmDP + b * 64 + c * 32, rd);
+        ptx::tc_ld_32x32(tS, rs);
+        ptx::tc_ld_32x32(tDP, rd);
         ptx::tc_wait_ld();
-        uint32_t wp[16], wd[16];
+        float lse4[4], del4[4];
 #pragma unroll
         for (int i = 0; i < 32; i += 2) {
+          if constexpr (kDKV) {
+            if (i % 4 == 0) {
+              *reinterpret_cast<float4*>(lse4) = *reinterpret_cast<const float4*>(stats + b * 128 + half * 32 + i);
+              *reinterpret_cast<float4*>(del4) = *reinterpret_cast<const float4*>(stats + b * 128 + 64 + half * 32 + i);
+            }
+          }
           float pr[2], ds[2];
 #pragma unroll
           for (int e = 0; e < 2; ++e) {
-            const int col = c * 32 + i + e;
-            const float lse_c = kDKV ? stats[b * 128 + col] : lse_r;
-            const float del_c = kDKV ? stats[b * 128 + 64 + col] : delta_r;
+            const float lse_c = kDKV ? lse4[(i + e) & 3] : lse_r, del_c = kDKV ? del4[(i + e) & 3] : delta_r;
             float pv = exp2f(fmaf(__uint_as_float(rs[i + e]), sl2, -lse_c));
             if (need_mask) {
-              const int xpos = x0 + col;
+              const int xpos = x0 + i + e;
               const bool vis = kDKV ? (r_pos <= xpos) : (xpos < L && (!p.causal || xpos <= r_pos));
               if (!vis) pv = 0.f;
             }
             pr[e] = pv;
             ds[e] = pv * (__uint_as_float(rd[i + e]) - del_c) * p.scale;
           }
-          wp[i >> 1] = pack2b<T>(pr[0], pr[1]);
-          wd[i >> 1] = pack2b<T>(ds[0], ds[1]);
-        }
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const uint32_t off = (((uint32_t)(c * 4 + q)) ^ sw) << 4;  // 16-byte piece (8 streamed positions) of this row
-          if constexpr (kDKV) {
-            st_shared_v4b(pb + off, wp[4 * q], wp[4 * q + 1], wp[4 * q + 2], wp[4 * q + 3]);
-            st_shared_v4b(pb + C::kPBytes + off, wd[4 * q], wd[4 * q + 1], wd[4 * q + 2], wd[4 * q + 3]);
-          } else {
-            st_shared_v4b(pb + off, wd[4 * q], wd[4 * q + 1], wd[4 * q + 2], wd[4 * q + 3]);
-          }
+          wp[i >> 1] = pack2<T>(pr[0], pr[1]);
+          wd[i >> 1] = pack2<T>(ds[0], ds[1]);
         }
       }
+      if constexpr (kDKV) ptx::tc_st_32x16(tS, wp);
+      ptx::tc_st_32x16(tDP, wd);
+      ptx::tc_wait_st();
       ptx::tc_fence_before();
-      ptx::fence_proxy_async();
       __syncwarp();
-      if (lane == 0) {
-        ptx::mbar_arrive(bar(S_EMPTY + b));
-        ptx::mbar_arrive(bar(P_FULL + b));
-      }
+      if (lane == 0) ptx::mbar_arrive(bar(P_FULL + b));
     }
 
-    // ---- accumulators -> global
-    ptx::mbar_wait(bar(ACC_FULL), 0);
+    // ---- accumulators -> global, 64 columns at a time through the warp's staging rows (the streamed ring is done with): dKV: the first four
+    // warps store dV, the others dK; dQ: each half of the warps one 64-column block
+    wait(ACC_FULL, 0);
     ptx::tc_fence_after();
-    // tcgen05.ld is warp-collective: every lane executes the loads, only the stores are predicated on the row being real
-    const bool row_ok = r_pos < L;
+    const uint32_t stage = sX + (warp - 2) * 4096;
 #pragma unroll
-    for (int which = 0; which < (kDKV ? 2 : 1); ++which) {
-      T* dst = reinterpret_cast<T*>(which == 0 ? p.out1 : p.out2) + (int64_t)(tok0 + r_pos) * (which == 0 ? p.ld1 : p.ld2) +
-               (int64_t)head * kD;  // dKV: kv head; dQ: q head
+    for (int blk = 0; blk < C::kDBlocks; ++blk) {
+      if (!kDKV && blk != half) continue;
+      const bool second = kDKV && half == 1;
+      const int64_t ld = second ? p.ld2 : p.ld1;
+      T* dst = reinterpret_cast<T*>(second ? p.out2 : p.out1) + (int64_t)head * kD + blk * 64 + (lane & 7) * 8;
+      uint32_t o[64];
+      ptx::tc_ld_32x32(lane_addr + (second ? kTmAcc2 : kTmAcc1) + blk * 64, o);
+      ptx::tc_ld_32x32(lane_addr + (second ? kTmAcc2 : kTmAcc1) + blk * 64 + 32, o + 32);
+      ptx::tc_wait_ld();
 #pragma unroll
-      for (int c = 0; c < kD / 32; ++c) {
-        uint32_t r[32];
-        ptx::tc_ld_32x32(lane_addr + (which == 0 ? kTmAcc1 : kTmAcc2) + c * 32, r);
-        ptx::tc_wait_ld();
-        if (row_ok) {
+      for (int c = 0; c < 8; ++c) {
+        uint32_t v[4];
 #pragma unroll
-          for (int i = 0; i < 32; i += 8) {
-            uint4 v;
-            v.x = pack2b<T>(__uint_as_float(r[i]), __uint_as_float(r[i + 1]));
-            v.y = pack2b<T>(__uint_as_float(r[i + 2]), __uint_as_float(r[i + 3]));
-            v.z = pack2b<T>(__uint_as_float(r[i + 4]), __uint_as_float(r[i + 5]));
-            v.w = pack2b<T>(__uint_as_float(r[i + 6]), __uint_as_float(r[i + 7]));
-            *reinterpret_cast<uint4*>(dst + c * 32 + i) = v;
-          }
-        }
+        for (int e = 0; e < 4; ++e) v[e] = pack2<T>(__uint_as_float(o[8 * c + 2 * e]), __uint_as_float(o[8 * c + 2 * e + 1]));
+        st_shared_v4(stage + lane * 128 + ((c ^ (lane & 7)) << 4), v[0], v[1], v[2], v[3]);
       }
+      __syncwarp();
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int rr = i * 4 + (lane >> 3), pos = rw + rr;
+        const uint4 v = ld_shared_v4(stage + rr * 128 + (((lane & 7) ^ (rr & 7)) << 4));
+        if (pos < L) *reinterpret_cast<uint4*>(dst + (int64_t)(tok0 + pos) * ld) = v;
+      }
+      __syncwarp();
     }
   }
 
   ptx::tc_fence_before();
   __syncthreads();
+  if (*dead) {
+    if (threadIdx.x == 0) g_wait_error = 1;
+    for (int i = 0; i < 1000; ++i) __nanosleep(1000);
+    __syncthreads();
+  }
   if (warp == 1) {
     ptx::tc_fence_after();
     ptx::tmem_dealloc(tmem_base, 512);
   }
 }
 
-// delta[h, t] = sum_d dO[t, h, d] * O[t, h, d]; one warp per (t, h)
-template <typename T>
-__global__ void attn_delta_kernel(const T* __restrict__ out, const T* __restrict__ dout, float* __restrict__ delta, int64_t o_ld,
-                                  int64_t do_ld, int Tn, int nq, int D) {
-  const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (w >= Tn * nq) return;
-  const int t = w / nq, h = w - t * nq;
-  const T* o = out + (int64_t)t * o_ld + (int64_t)h * D;
-  const T* g = dout + (int64_t)t * do_ld + (int64_t)h * D;
-  float acc = 0.f;
-  for (int i = lane * 2; i < D; i += 64) acc += rb::to_f(o[i]) * rb::to_f(g[i]) + rb::to_f(o[i + 1]) * rb::to_f(g[i + 1]);
-  acc = rb::warp_sum(acc);
-  if (lane == 0) delta[(int64_t)h * Tn + t] = acc;
+// delta[h, t] = sum_d dO[t, h, d] * O[t, h, d]: kD / 8 lanes per (t, h) with 16-byte loads, four (t, h) of a lane group in flight (one
+// warp per (t, h) with 4-byte loads: 129 us at 20480 tokens x 32 heads x 128, 2.6 TB/s; now 92)
+template <typename T, int kD>
+__global__ void __launch_bounds__(256) attn_delta_kernel(const T* __restrict__ out, const T* __restrict__ dout, float* __restrict__ delta, int64_t o_ld,
+                                                         int64_t do_ld, int Tn, int nq) {
+  constexpr int kLanes = kD / 8, kGroups = 256 / kLanes, kUnroll = 4;
+  const int sub = threadIdx.x % kLanes, total = Tn * nq;
+  const int w0 = blockIdx.x * kGroups * kUnroll + threadIdx.x / kLanes;
+  float acc[kUnroll];
+  rb::Pack<T, 8> a[kUnroll], g[kUnroll];
+#pragma unroll
+  for (int u = 0; u < kUnroll; ++u) {
+    const int w = w0 + u * kGroups, t = w / nq, h = w - t * nq;
+    if (w < total) {
+      a[u] = *reinterpret_cast<const rb::Pack<T, 8>*>(out + (int64_t)t * o_ld + (int64_t)h * kD + sub * 8);
+      g[u] = *reinterpret_cast<const rb::Pack<T, 8>*>(dout + (int64_t)t * do_ld + (int64_t)h * kD + sub * 8);
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < kUnroll; ++u) {
+    const int w = w0 + u * kGroups, t = w / nq, h = w - t * nq;
+    acc[u] = 0.f;
+    if (w < total) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) acc[u] = fmaf(rb::to_f(a[u].v[i]), rb::to_f(g[u].v[i]), acc[u]);
+    }
+#pragma unroll
+    for (int o = kLanes / 2; o > 0; o >>= 1) acc[u] += __shfl_xor_sync(0xffffffffu, acc[u], o);
+    if (sub == 0 && w < total) delta[(int64_t)h * Tn + t] = acc[u];
+  }
 }
 
 template <int kD, typename T, int kFmt, bool kDKV>
 int launch_bwd(const CUtensorMap& r1, const CUtensorMap& r2, const CUtensorMap& x1, const CUtensorMap& x2, const BwdParams& p,
                int heads, int B, int max_seqlen, cudaStream_t s) {
-  using C = BCfg<kD, kDKV>;
+  using C = BCfg<kD>;
   auto kern = attn_bwd_kernel<kD, T, kFmt, kDKV>;
   static bool attr_set = false;
   if (!attr_set) {
@@ -370,10 +391,9 @@ int run_bwd(const void* q, const void* k, const void* v, const void* out, const 
             int64_t dk_ld, int64_t dv_ld, int Tn, int B, int nq, int nkv, int max_seqlen, float scale, int causal, cudaStream_t s) {
   const int bf = kFmt == 1;
   {
-    const int warps = Tn * nq, threads = 256;
-    attn_delta_kernel<T><<<RB_CEIL_DIV(warps * 32, threads), threads, 0, s>>>(reinterpret_cast<const T*>(out),
-                                                                              reinterpret_cast<const T*>(dout), delta, o_ld, do_ld,
-                                                                              Tn, nq, kD);
+    const int per_cta = 256 / (kD / 8) * 4;
+    attn_delta_kernel<T, kD><<<RB_CEIL_DIV(Tn * nq, per_cta), 256, 0, s>>>(reinterpret_cast<const T*>(out), reinterpret_cast<const T*>(dout), delta, o_ld,
+                                                                           do_ld, Tn, nq);
     if (cudaGetLastError() != cudaSuccess) return -20;
   }
   CUtensorMap q128, do128, k128, v128, q64, do64, k64, v64;
@@ -391,6 +411,13 @@ int run_bwd(const void* q, const void* k, const void* v, const void* out, const 
 
 }  // namespace
 
+extern "C" int rb_attn_bwd_wait_error() {
+  int v = 0, zero = 0;
+  if (cudaMemcpyFromSymbol(&v, g_wait_error, sizeof(int)) != cudaSuccess) return -1;
+  if (v != 0) cudaMemcpyToSymbol(g_wait_error, &zero, sizeof(int));
+  return v;
+}
+
 // All tensors are [T, heads, hd] views with unit stride over hd and packed heads; `delta` is an [nq, T] fp32 scratch tensor.
 // dt: 1 = bf16, 2 = fp16.  Returns 0 or a negative code.
 extern "C" int rb_attn_bwd(const void* q, const void* k, const void* v, const void* out, const void* dout, const float* lse,
@@ -401,7 +428,7 @@ extern "C" int rb_attn_bwd(const void* q, const void* k, const void* v, const vo
   if (dt != 1 && dt != 2) return -2;
   if (nq % nkv != 0 || T <= 0 || B <= 0 || max_seqlen <= 0) return -3;
   if ((q_ld | k_ld | v_ld | o_ld | do_ld | dq_ld | dk_ld | dv_ld) % 8 != 0) return -4;
-  if (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)dout | (uintptr_t)dq | (uintptr_t)dk | (uintptr_t)dv) & 15) return -5;
+  if (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)dout | (uintptr_t)out | (uintptr_t)dq | (uintptr_t)dk | (uintptr_t)dv) & 15) return -5;
 #define RB_RUN(D, TT, F)                                                                                                          \
   return run_bwd<D, TT, F>(q, k, v, out, dout, lse, delta, dq, dk, dv, cu_seqlens, q_ld, k_ld, v_ld, o_ld, do_ld, dq_ld, dk_ld, \
                            dv_ld, T, B, nq, nkv, max_seqlen, scale, causal, s)

@@ -538,6 +538,7 @@ int launch_attn_fwd(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensor
 }  // namespace
 
 extern "C" int rb_attn_bias_wait_error();
+extern "C" int rb_attn_bwd_wait_error();
 extern "C" int rb_attn_fwd_bias(const CUtensorMap* mq, const CUtensorMap* mk, const CUtensorMap* mv, const AttnParams* p, int B, int hd, int max_seqlen,
                                 int kv_shared, int bf, cudaStream_t s);
 
@@ -546,8 +547,8 @@ extern "C" int rb_attn_wait_error() {
   int v = 0, zero = 0;
   if (cudaMemcpyFromSymbol(&v, g_wait_error, sizeof(int)) != cudaSuccess) return -1;
   if (v != 0) cudaMemcpyToSymbol(g_wait_error, &zero, sizeof(int));
-  const int b = rb_attn_bias_wait_error();
-  return b != 0 ? b : v;
+  const int b = rb_attn_bias_wait_error(), c = rb_attn_bwd_wait_error();
+  return b != 0 ? b : c != 0 ? c : v;
 }
 
 // q / k / v: [T, heads, hd] views (unit stride over hd, `heads * hd` contiguous columns, row pitch *_ld elements) -- e.g. the

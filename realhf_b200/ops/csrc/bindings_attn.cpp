@@ -143,10 +143,12 @@ void attn_bwd(const Tensor& dout, const Tensor& q, const Tensor& k, const Tensor
   TORCH_CHECK(cu_seqlens.scalar_type() == at::kInt && cu_seqlens.is_contiguous() && cu_seqlens.is_cuda());
   c10::cuda::CUDAGuard guard(q.device());
   auto delta = at::empty({nq, T}, q.options().dtype(at::kFloat));
+  // the pre-pass reads `out` in 16-byte pieces; a view that starts elsewhere is copied
+  const Tensor o = reinterpret_cast<uintptr_t>(out.data_ptr()) % 16 ? out.clone(at::MemoryFormat::Contiguous) : out;
   const int dt = q.scalar_type() == at::kBFloat16 ? 1 : (q.scalar_type() == at::kHalf ? 2 : -1);
-  int rc = rb_attn_bwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), dout.data_ptr(), lse.data_ptr<float>(),
+  int rc = rb_attn_bwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), dout.data_ptr(), lse.data_ptr<float>(),
                        delta.data_ptr<float>(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), cu_seqlens.data_ptr<int>(), q.stride(0),
-                       k.stride(0), v.stride(0), out.stride(0), dout.stride(0), dq.stride(0), dk.stride(0), dv.stride(0), (int)T,
+                       k.stride(0), v.stride(0), o.stride(0), dout.stride(0), dq.stride(0), dk.stride(0), dv.stride(0), (int)T,
                        (int)cu_seqlens.numel() - 1, (int)nq, (int)nkv, (int)hd, (int)max_seqlen, (float)scale, causal ? 1 : 0, dt,
                        at::cuda::getCurrentCUDAStream().stream());
   TORCH_CHECK(rc == 0, "attn_bwd: unsupported configuration (", rc, ")");
