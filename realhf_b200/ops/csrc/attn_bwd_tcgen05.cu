@@ -23,16 +23,22 @@
 // What bounds it: a step is 1024 (dKV) or 768 (dQ) tensor-pipe cycles at D = 128, and its 8192 elements take the CUDA cores about as long when
 // eight warps share them (a warp has 32 rows and 32 of the 64 columns).  Four warps, P through shared memory, the streamed rows' statistics
 // fetched from global memory inside every step and MMAs issued from a divergent branch kept the tensor pipe 19% busy (32 x 640 tokens x 32
-// heads: dKV 613, dQ 506 us, now 412, 388; 8 x 1500..4096, 32 / 8 heads: 2473, 2109 us, now 1777, 1662).
+// heads: dKV 613, dQ 506 us, now 322, 240; 8 x 1500..4096, 32 / 8 heads: 2473, 2109 us, now 1553, 1152).
+//
+// The grid holds one CTA per (row tile, head) (a bound: the lengths are on the device); a running CTA takes the items of CTAs that have not
+// started (`clusterlaunchcontrol.try_cancel`), so that the next item's tiles load and its first products run while the last accumulators
+// leave.  With a CTA per item 32 x 640 tokens took 17600 cycles an item of which six steps were half.
 //
 // delta[h, t] = sum_d dO[t, h, d] * O[t, h, d] comes from a small pre-pass; LSE is the forward's ([nq, T], natural log).
+#include <type_traits>
+
 #include "attn_common.cuh"
 
 namespace {
 
 constexpr int kR = 128;   // resident rows per CTA (= UMMA M)
 constexpr int kX = 64;    // streamed rows per step (= UMMA N of the S-type products, K of the accumulating ones)
-constexpr int kXStages = 4;
+constexpr int kXStages = 3;
 constexpr int kBwdThreads = 320;   // warp 0: TMA, warp 1: MMA, warps 2-9: elements (two per TMEM quadrant, one per column half)
 
 struct BwdParams {
@@ -42,7 +48,7 @@ struct BwdParams {
   void* out1;          // dKV pass: dV;  dQ pass: dQ      ([T, heads, D] views, row pitch ld1)
   void* out2;          // dKV pass: dK
   int64_t ld1, ld2;
-  int T, nq, nkv;
+  int T, B, nq, nkv, heads;   // heads: of this pass (key heads for dKV, query heads for dQ)
   float scale;
   int causal;
 };
@@ -51,17 +57,19 @@ template <int kD> struct BCfg {
   static constexpr int kDBlocks = kD / 64;
   static constexpr int kRBytes = kR * kD * 2;     // one resident tile
   static constexpr int kXBytes = kX * kD * 2;     // one streamed tile
-  static constexpr int kBars = 2 * kRBytes + kXStages * 2 * kXBytes;
-  static constexpr int kStats = kBars + 256;      // [2 buffers][lse | delta][64]
-  static constexpr int kSmemBytes = kStats + 2 * 2 * kX * 4 + 1024 /*align*/;
+  static constexpr int kOut = 2 * kRBytes + kXStages * 2 * kXBytes;   // 4 KB of output staging per element warp
+  static constexpr int kBars = kOut + 8 * 4096;
+  static constexpr int kStats = kBars + 256;      // [8 element warps][2 buffers][lse | delta][32]
+  static constexpr int kSmemBytes = kStats + 8 * 2 * 2 * 32 * 4 + 1024 /*align*/;
 };
 
-enum BBar { R_FULL = 0, X_FULL = 1, X_EMPTY = X_FULL + kXStages, S_FULL = X_EMPTY + kXStages, P_FULL = S_FULL + 2, ACC_FULL = P_FULL + 2,
-            B_NUM_BARS = ACC_FULL + 1 };
+enum BBar { R_FULL = 0, R_EMPTY = 1, X_FULL = 2, X_EMPTY = X_FULL + kXStages, S_FULL = X_EMPTY + kXStages, P_FULL = S_FULL + 2, ACC_FULL = P_FULL + 2,
+            ACC_EMPTY = ACC_FULL + 1, IT_FULL = ACC_EMPTY + 1, IT_EMPTY = IT_FULL + 2, CLC_FULL = IT_EMPTY + 2, B_NUM_BARS = CLC_FULL + 1 };
+
+// One work item: sequence (first token, length), head and first resident row; L < 0 ends the CTA's loop.
+struct BItem { int tok0, L, head, r0; };
 
 __device__ int g_wait_error = 0;
-
-RB_DEVICE void element_bar_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
 
 // tma_r1 / tma_r2: resident operands (box 64 cols x 128 rows); tma_x1 / tma_x2: streamed operands (box 64 x 64).
 //   kDKV: r1 = K, r2 = V (kv-head columns), x1 = Q, x2 = dO (q-head columns).   !kDKV: r1 = Q, r2 = dO, x1 = K, x2 = V.
@@ -71,19 +79,12 @@ __global__ void __launch_bounds__(kBwdThreads, 1) attn_bwd_kernel(const __grid_c
                                                                   const __grid_constant__ CUtensorMap tma_x1,
                                                                   const __grid_constant__ CUtensorMap tma_x2, const __grid_constant__ BwdParams p) {
   using C = BCfg<kD>;
-  const int seq = blockIdx.z, head = blockIdx.y;  // kDKV: kv head; else q head
-  const int tile = kDKV ? (int)blockIdx.x : (int)(gridDim.x - 1 - blockIdx.x);  // heaviest tiles first in both passes
-  const int tok0 = p.cu_seqlens[seq];
-  const int L = p.cu_seqlens[seq + 1] - tok0;
-  const int r0 = tile * kR;  // first key (dKV) / first query (dQ) of this CTA inside the sequence
-  if (r0 >= L) return;
   const int G = p.nq / p.nkv;
-  const int nblk_all = RB_CEIL_DIV(L, kX);
-  // streamed block range [blk0, blk1): dKV -> query blocks that can see these keys; dQ -> key blocks these queries can see
-  const int blk0 = kDKV ? (p.causal ? r0 / kX : 0) : 0;
-  const int blk1 = kDKV ? nblk_all : (p.causal ? RB_CEIL_DIV(min(L, r0 + kR), kX) : nblk_all);
-  const int nblk = blk1 - blk0;
-  const int n_steps = kDKV ? nblk * G : nblk;  // dKV also walks the q heads of the group (outer loop)
+  // streamed blocks [blk0, blk0 + nblk) of an item: dKV -> query blocks that can see its keys; dQ -> key blocks its queries can see; dKV also walks
+  // the q heads of the group (outer loop)
+  auto first_blk = [&](const BItem& it) { return kDKV && p.causal ? it.r0 / kX : 0; };
+  auto blocks = [&](const BItem& it) { return RB_CEIL_DIV(!kDKV && p.causal ? min(it.L, it.r0 + kR) : it.L, kX) - first_blk(it); };
+  auto steps = [&](const BItem& it) { return blocks(it) * (kDKV ? G : 1); };
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -91,7 +92,9 @@ __global__ void __launch_bounds__(kBwdThreads, 1) attn_bwd_kernel(const __grid_c
   const uint32_t sR2 = sR1 + C::kRBytes;
   const uint32_t sX = sR2 + C::kRBytes;            // stage s: X1 at sX + s * 2 * kXBytes, X2 right after it
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::kBars);
-  uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(bars + B_NUM_BARS);
+  BItem* items = reinterpret_cast<BItem*>(smem + C::kBars + 192);     // two slots of 16 bytes
+  const uint32_t clc = sR1 + C::kBars + 224;                          // 16 bytes
+  uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(smem + C::kBars + 240);
   volatile uint32_t* dead = tmem_ptr + 1;
   float* stats = reinterpret_cast<float*>(smem + C::kStats);
   auto bar = [&](int i) { return ptx::smem_u32(&bars[i]); };
@@ -106,7 +109,8 @@ __global__ void __launch_bounds__(kBwdThreads, 1) attn_bwd_kernel(const __grid_c
     ptx::prefetch_tensormap(&tma_r2);
     ptx::prefetch_tensormap(&tma_x1);
     ptx::prefetch_tensormap(&tma_x2);
-    for (int i = 0; i < B_NUM_BARS; ++i) ptx::mbar_init(bar(i), (i == P_FULL || i == P_FULL + 1) ? 8 : 1);   // one arrival per element warp
+    for (int i = 0; i < B_NUM_BARS; ++i)      // one arrival per element warp; items: the MMA warp too
+      ptx::mbar_init(bar(i), i == P_FULL || i == P_FULL + 1 || i == ACC_EMPTY ? 8 : i == IT_EMPTY || i == IT_EMPTY + 1 ? 9 : 1);
     ptx::fence_barrier_init();
   }
   if (warp == 1) {
@@ -118,47 +122,83 @@ __global__ void __launch_bounds__(kBwdThreads, 1) attn_bwd_kernel(const __grid_c
   ptx::tc_fence_after();
   const uint32_t tmem_base = *tmem_ptr;
 
-  // step t -> (q head, streamed block)
-  auto step_head = [&](int t) { return kDKV ? head * G + t / nblk : head; };
-  auto step_blk = [&](int t) { return blk0 + (kDKV ? t % nblk : t); };
-
   if (warp == 0) {
-    // ===================================================== TMA producer
-    if (lane == 0) {
-      const int x_kv_head = kDKV ? head : head / G;            // dQ pass streams the kv head of this q head
-      ptx::mbar_arrive_expect_tx(bar(R_FULL), 2 * C::kRBytes);
-#pragma unroll
-      for (int kb = 0; kb < C::kDBlocks; ++kb) {
-        ptx::tma_load_2d(sR1 + kb * (kR * 128), &tma_r1, bar(R_FULL), head * kD + kb * 64, tok0 + r0);
-        ptx::tma_load_2d(sR2 + kb * (kR * 128), &tma_r2, bar(R_FULL), head * kD + kb * 64, tok0 + r0);
+    // ===================================================== scheduler + TMA producer
+    auto request = [&] {
+      if (lane == 0) {
+        ptx::mbar_arrive_expect_tx(bar(CLC_FULL), 16);
+        ptx::clc_try_cancel(clc, bar(CLC_FULL));
       }
-      for (int t = 0; t < n_steps; ++t) {
-        const int st = t % kXStages;
-        const int row = tok0 + step_blk(t) * kX;
-        const int col = (kDKV ? step_head(t) : x_kv_head) * kD;
-        wait(X_EMPTY + st, ((uint32_t)(t / kXStages) & 1u) ^ 1u);
-        ptx::mbar_arrive_expect_tx(bar(X_FULL + st), 2 * C::kXBytes);
-        const uint32_t x1 = sX + st * 2 * C::kXBytes, x2 = x1 + C::kXBytes;
+      __syncwarp();
+    };
+    UnitSearch search;
+    int idx = blockIdx.x, n_pub = 0, g = 0;      // g: streamed tiles so far
+    uint32_t n_req = 0;
+    auto publish = [&](const BItem& it) {
+      const int slot = n_pub & 1;
+      wait(IT_EMPTY + slot, ((uint32_t)(n_pub >> 1) & 1u) ^ 1u);
+      if (lane == 0) {
+        items[slot] = it;
+        ptx::mbar_arrive(bar(IT_FULL + slot));
+      }
+      ++n_pub;
+    };
+    request();
+    while (true) {
+      BItem it{0, 0, 0, 0};
+      int r;
+      it.head = idx % p.heads;
+      if (search.find(p.cu_seqlens, p.B, kR, idx / p.heads, it.tok0, it.L, r)) {
+        it.r0 = (kDKV ? r : RB_CEIL_DIV(it.L, kR) - 1 - r) * kR;       // heaviest tiles first in both passes
+        publish(it);
+        if (lane == 0) {
+          wait(R_EMPTY, (uint32_t)n_pub & 1u);      // (n_pub - 1 items before this one)
+          const int nblk = blocks(it), n = steps(it), blk0 = first_blk(it);
+          ptx::mbar_arrive_expect_tx(bar(R_FULL), 2 * C::kRBytes);
 #pragma unroll
-        for (int kb = 0; kb < C::kDBlocks; ++kb) {
-          ptx::tma_load_2d(x1 + kb * (kX * 128), &tma_x1, bar(X_FULL + st), col + kb * 64, row);
-          ptx::tma_load_2d(x2 + kb * (kX * 128), &tma_x2, bar(X_FULL + st), col + kb * 64, row);
+          for (int kb = 0; kb < C::kDBlocks; ++kb) {
+            ptx::tma_load_2d(sR1 + kb * (kR * 128), &tma_r1, bar(R_FULL), it.head * kD + kb * 64, it.tok0 + it.r0);
+            ptx::tma_load_2d(sR2 + kb * (kR * 128), &tma_r2, bar(R_FULL), it.head * kD + kb * 64, it.tok0 + it.r0);
+          }
+          int h = kDKV ? it.head * G : it.head / G, blk = 0;           // dQ streams the kv head of its q head
+          for (int t = 0; t < n; ++t, ++g) {
+            const int st = g % kXStages, row = it.tok0 + (blk0 + blk) * kX;
+            wait(X_EMPTY + st, ((uint32_t)(g / kXStages) & 1u) ^ 1u);
+            ptx::mbar_arrive_expect_tx(bar(X_FULL + st), 2 * C::kXBytes);
+            const uint32_t x1 = sX + st * 2 * C::kXBytes, x2 = x1 + C::kXBytes;
+#pragma unroll
+            for (int kb = 0; kb < C::kDBlocks; ++kb) {
+              ptx::tma_load_2d(x1 + kb * (kX * 128), &tma_x1, bar(X_FULL + st), h * kD + kb * 64, row);
+              ptx::tma_load_2d(x2 + kb * (kX * 128), &tma_x2, bar(X_FULL + st), h * kD + kb * 64, row);
+            }
+            if (++blk == nblk) { blk = 0; ++h; }
+          }
         }
+        __syncwarp();
       }
+      wait(CLC_FULL, n_req & 1u);
+      ++n_req;
+      if (*dead) break;
+      int x;
+      const bool got = ptx::clc_query(clc, x);
+      __syncwarp();
+      if (!got) break;
+      idx = x;
+      ptx::fence_proxy_async();   // the response was read before it is overwritten
+      request();
     }
-    __syncwarp();
+    publish(BItem{0, -1, 0, 0});
   } else if (warp == 1) {
     // ===================================================== MMA issuer: the whole warp runs the loop, one elected lane issues
     constexpr uint32_t idesc_s = ptx::make_idesc_f16(kFmt, kR, kX, 0, 0);   // resident x streamed^T, both K-major
     constexpr uint32_t idesc_a = ptx::make_idesc_f16(kFmt, kR, kD, 0, 1);   // P-type (TMEM) x streamed (MN-major)
     const uint32_t tm = (uint32_t)ptx::uniform((int)tmem_base);
-    const int n = ptx::uniform(n_steps);
     const uint64_t r1 = ptx::make_smem_desc_sw128(sR1, 16, 1024), r2 = ptx::make_smem_desc_sw128(sR2, 16, 1024);
-    auto issue_sdp = [&](int t) {
-      const int st = t % kXStages;
-      wait(X_FULL + st, (uint32_t)(t / kXStages) & 1u);
+    auto issue_sdp = [&](int g, bool last) {      // g: steps of this CTA so far
+      const int st = g % kXStages;
+      wait(X_FULL + st, (uint32_t)(g / kXStages) & 1u);
       ptx::tc_fence_after();
-      const uint32_t d = tm + (t & 1) * 64;
+      const uint32_t d = tm + (g & 1) * 64;
       const uint64_t x1 = ptx::make_smem_desc_sw128(sX + st * 2 * C::kXBytes, 16, 1024);
       const uint64_t x2 = ptx::make_smem_desc_sw128(sX + st * 2 * C::kXBytes + C::kXBytes, 16, 1024);
       if (ptx::elect_one()) {
@@ -170,158 +210,205 @@ __global__ void __launch_bounds__(kBwdThreads, 1) attn_bwd_kernel(const __grid_c
         for (int kk = 0; kk < kD / 16; ++kk)
           ptx::tc_mma_f16(d + kTmDP, r2 + (((kk >> 2) * (kR * 128) + (kk & 3) * 32) >> 4), x2 + (((kk >> 2) * (kX * 128) + (kk & 3) * 32) >> 4), idesc_s,
                           kk != 0 ? 1u : 0u);
-        ptx::tc_commit(bar(S_FULL + (t & 1)));
+        ptx::tc_commit(bar(S_FULL + (g & 1)));
+        if (last) ptx::tc_commit(bar(R_EMPTY));
       }
       __syncwarp();
     };
-    wait(R_FULL, 0);
-    issue_sdp(0);
-    for (int t = 0; t < n; ++t) {
-      if (t + 1 < n) issue_sdp(t + 1);       // its S / dP columns: the products that read P of step t-1 there are ahead in the pipe
-      const int st = t % kXStages;
-      wait(P_FULL + (t & 1), (uint32_t)(t >> 1) & 1u);
-      ptx::tc_fence_after();
-      const uint32_t a = tm + (t & 1) * 64;
-      const uint64_t x1 = ptx::make_smem_desc_sw128(sX + st * 2 * C::kXBytes, kX * 128, 1024);
-      const uint64_t x2 = ptx::make_smem_desc_sw128(sX + st * 2 * C::kXBytes + C::kXBytes, kX * 128, 1024);
-      const uint32_t keep = t != 0 ? 1u : 0u;
-      if (ptx::elect_one()) {
-#pragma unroll
-        for (int kk = 0; kk < kX / 16; ++kk) {
-          // A: 16 streamed rows = 8 columns, the two halves of a row 32 columns apart; B: 16 rows = 2048 B down every 64-wide chunk
-          const uint32_t ao = (kk >> 1) * 32 + (kk & 1) * 8;
-          if constexpr (kDKV) {
-            ptx::tc_mma_f16_ts(tm + kTmAcc1, a + kTmS + ao, x2 + kk * 128, idesc_a, kk != 0 ? 1u : keep);    // dV += P^T dO
-            ptx::tc_mma_f16_ts(tm + kTmAcc2, a + kTmDP + ao, x1 + kk * 128, idesc_a, kk != 0 ? 1u : keep);   // dK += dS^T Q
-          } else {
-            ptx::tc_mma_f16_ts(tm + kTmAcc1, a + kTmDP + ao, x1 + kk * 128, idesc_a, kk != 0 ? 1u : keep);   // dQ += dS K
-          }
-        }
-        ptx::tc_commit(bar(X_EMPTY + st));
-        if (t == n - 1) ptx::tc_commit(bar(ACC_FULL));
-      }
+    int g = 0;
+    for (int n_it = 0;; ++n_it) {
+      const int slot = n_it & 1;
+      wait(IT_FULL + slot, (uint32_t)(n_it >> 1) & 1u);
+      BItem it = items[slot];
+      it.L = ptx::uniform(it.L);
+      it.r0 = ptx::uniform(it.r0);
+      if (lane == 0) ptx::mbar_arrive(bar(IT_EMPTY + slot));
       __syncwarp();
+      if (it.L < 0 || ptx::uniform((int)*dead)) break;
+      const int n = steps(it);
+      wait(R_FULL, (uint32_t)n_it & 1u);
+      issue_sdp(g, n == 1);
+      for (int t = 0; t < n; ++t, ++g) {
+        if (t + 1 < n) issue_sdp(g + 1, t + 2 == n);       // its S / dP columns: the products that read P of step t-1 there are ahead in the pipe
+        const int st = g % kXStages;
+        wait(P_FULL + (g & 1), (uint32_t)(g >> 1) & 1u);
+        if (t == 0) wait(ACC_EMPTY, ((uint32_t)n_it & 1u) ^ 1u);
+        ptx::tc_fence_after();
+        const uint32_t a = tm + (g & 1) * 64;
+        const uint64_t x1 = ptx::make_smem_desc_sw128(sX + st * 2 * C::kXBytes, kX * 128, 1024);
+        const uint64_t x2 = ptx::make_smem_desc_sw128(sX + st * 2 * C::kXBytes + C::kXBytes, kX * 128, 1024);
+        const uint32_t keep = t != 0 ? 1u : 0u;
+        if (ptx::elect_one()) {
+#pragma unroll
+          for (int kk = 0; kk < kX / 16; ++kk) {
+            // A: 16 streamed rows = 8 columns, the two halves of a row 32 columns apart; B: 16 rows = 2048 B down every 64-wide chunk
+            const uint32_t ao = (kk >> 1) * 32 + (kk & 1) * 8;
+            if constexpr (kDKV) {
+              ptx::tc_mma_f16_ts(tm + kTmAcc1, a + kTmS + ao, x2 + kk * 128, idesc_a, kk != 0 ? 1u : keep);    // dV += P^T dO
+              ptx::tc_mma_f16_ts(tm + kTmAcc2, a + kTmDP + ao, x1 + kk * 128, idesc_a, kk != 0 ? 1u : keep);   // dK += dS^T Q
+            } else {
+              ptx::tc_mma_f16_ts(tm + kTmAcc1, a + kTmDP + ao, x1 + kk * 128, idesc_a, kk != 0 ? 1u : keep);   // dQ += dS K
+            }
+          }
+          ptx::tc_commit(bar(X_EMPTY + st));
+          if (t == n - 1) ptx::tc_commit(bar(ACC_FULL));
+        }
+        __syncwarp();
+      }
     }
   } else {
     // ===================================================== element threads (thread = resident row = TMEM lane, and one half of the columns)
     const int quad = warp & 3, half = (warp - 2) >> 2;
-    const int row = quad * 32 + lane, tid = threadIdx.x - 64;
-    const int r_pos = r0 + row;  // key (dKV) / query (dQ) position of this thread inside the sequence
-    const int rw = r0 + quad * 32;
     const uint32_t lane_addr = tmem_base + ((uint32_t)(quad * 32) << 16);
     const float sl2 = p.scale * 1.4426950408889634f;
-    float lse_r = INFINITY, delta_r = 0.f;  // dQ pass: per-row statistics in registers
-    if constexpr (!kDKV) {
-      if (r_pos < L) {
-        lse_r = p.lse[(int64_t)head * p.T + tok0 + r_pos] * 1.4426950408889634f;
-        delta_r = p.delta[(int64_t)head * p.T + tok0 + r_pos];
-      }
-    }
-    // dKV: statistics of a step's 64 streamed queries, [lse * log2e | delta], fetched a step ahead by the first 128 threads; rows past the end of
-    // the sequence get lse = +inf, which zeroes their probabilities
-    auto fetch_stat = [&](int t) {
-      float v = tid < 64 ? INFINITY : 0.f;
-      const int qpos = step_blk(t) * kX + (tid & 63);
-      if (tid < 128 && qpos < L) {
-        const int64_t idx = (int64_t)step_head(t) * p.T + tok0 + qpos;
-        v = tid < 64 ? p.lse[idx] * 1.4426950408889634f : p.delta[idx];
-      }
-      return v;
-    };
-    float stat = kDKV ? fetch_stat(0) : 0.f;
-
-    for (int t = 0; t < n_steps; ++t) {
-      const int b = t & 1;
-      const int x0 = step_blk(t) * kX + half * 32;  // first streamed position of this warp's columns (query for dKV, key for dQ)
-      if constexpr (kDKV) {
-        if (tid < 128) stats[b * 128 + tid] = stat;
-        if (t + 1 < n_steps) stat = fetch_stat(t + 1);
-        element_bar_sync();
-      }
-      wait(S_FULL + b, (uint32_t)(t >> 1) & 1u);
-      ptx::tc_fence_after();
-      const uint32_t tS = lane_addr + kTmS + b * 64 + half * 32, tDP = lane_addr + kTmDP + b * 64 + half * 32;
-      bool need_mask, none;         // some / all elements of the warp's block are hidden (uniform)
-      if constexpr (kDKV) {
-        need_mask = p.causal && rw + 31 > x0;                        // some key > some query
-        none = x0 >= L || (p.causal && rw > x0 + 31);
-      } else {
-        need_mask = x0 + 32 > L || (p.causal && x0 + 31 > rw);        // key past the end / above the diagonal
-        none = x0 >= L || (p.causal && x0 > rw + 31);
-      }
-      uint32_t wp[16], wd[16];
-      if (none) {
-#pragma unroll
-        for (int i = 0; i < 16; ++i) wp[i] = wd[i] = 0u;
-      } else {
-        uint32_t rs[32], rd[32];
-        ptx::tc_ld_32x32(tS, rs);
-        ptx::tc_ld_32x32(tDP, rd);
-        ptx::tc_wait_ld();
-        float lse4[4], del4[4];
-#pragma unroll
-        for (int i = 0; i < 32; i += 2) {
-          if constexpr (kDKV) {
-            if (i % 4 == 0) {
-              *reinterpret_cast<float4*>(lse4) = *reinterpret_cast<const float4*>(stats + b * 128 + half * 32 + i);
-              *reinterpret_cast<float4*>(del4) = *reinterpret_cast<const float4*>(stats + b * 128 + 64 + half * 32 + i);
-            }
-          }
-          float pr[2], ds[2];
-#pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            const float lse_c = kDKV ? lse4[(i + e) & 3] : lse_r, del_c = kDKV ? del4[(i + e) & 3] : delta_r;
-            float pv = exp2f(fmaf(__uint_as_float(rs[i + e]), sl2, -lse_c));
-            if (need_mask) {
-              const int xpos = x0 + i + e;
-              const bool vis = kDKV ? (r_pos <= xpos) : (xpos < L && (!p.causal || xpos <= r_pos));
-              if (!vis) pv = 0.f;
-            }
-            pr[e] = pv;
-            ds[e] = pv * (__uint_as_float(rd[i + e]) - del_c) * p.scale;
-          }
-          wp[i >> 1] = pack2<T>(pr[0], pr[1]);
-          wd[i >> 1] = pack2<T>(ds[0], ds[1]);
+    float* my_stats = stats + (warp - 2) * 128;
+    const uint32_t stage = sR1 + C::kOut + (warp - 2) * 4096;
+    int g = 0;       // steps of this CTA so far
+    for (int n_it = 0;; ++n_it) {
+      const int slot = n_it & 1;
+      wait(IT_FULL + slot, (uint32_t)(n_it >> 1) & 1u);
+      const BItem it = items[slot];
+      __syncwarp();
+      if (lane == 0) ptx::mbar_arrive(bar(IT_EMPTY + slot));
+      if (it.L < 0 || *dead) break;
+      const int L = it.L, tok0 = it.tok0, head = it.head, nblk = blocks(it), blk0 = first_blk(it), n_steps = steps(it);
+      const int rw = it.r0 + quad * 32, r_pos = rw + lane;  // key (dKV) / query (dQ) position of this thread inside the sequence
+      // step t -> (q head, streamed block)
+      auto step_head = [&](int t) { return kDKV ? head * G + t / nblk : head; };
+      auto step_blk = [&](int t) { return blk0 + (kDKV ? t % nblk : t); };
+      float nlse_r = -INFINITY, ndelta_r = 0.f;  // dQ pass: per-row statistics (-lse * log2e, -delta) in registers
+      if constexpr (!kDKV) {
+        if (r_pos < L) {
+          nlse_r = p.lse[(int64_t)head * p.T + tok0 + r_pos] * -1.4426950408889634f;
+          ndelta_r = -p.delta[(int64_t)head * p.T + tok0 + r_pos];
         }
       }
-      if constexpr (kDKV) ptx::tc_st_32x16(tS, wp);
-      ptx::tc_st_32x16(tDP, wd);
-      ptx::tc_wait_st();
-      ptx::tc_fence_before();
-      __syncwarp();
-      if (lane == 0) ptx::mbar_arrive(bar(P_FULL + b));
-    }
+      // dKV: statistics of the warp's 32 streamed queries of a step, -lse * log2e and -delta, one per lane, fetched a step ahead and turned through
+      // shared memory of the warp; rows past the end of the sequence get lse = +inf, which zeroes their probabilities
+      float nlse = -INFINITY, ndelta = 0.f;
+      auto fetch_stats = [&](int t) {
+        const int qpos = step_blk(t) * kX + half * 32 + lane;
+        nlse = -INFINITY;
+        ndelta = 0.f;
+        if (qpos < L) {
+          const int64_t idx = (int64_t)step_head(t) * p.T + tok0 + qpos;
+          nlse = p.lse[idx] * -1.4426950408889634f;
+          ndelta = -p.delta[idx];
+        }
+      };
+      if constexpr (kDKV) fetch_stats(0);
 
-    // ---- accumulators -> global, 64 columns at a time through the warp's staging rows (the streamed ring is done with): dKV: the first four
-    // warps store dV, the others dK; dQ: each half of the warps one 64-column block
-    wait(ACC_FULL, 0);
-    ptx::tc_fence_after();
-    const uint32_t stage = sX + (warp - 2) * 4096;
+      for (int t = 0; t < n_steps; ++t, ++g) {
+        const int b = g & 1;
+        const int x0 = step_blk(t) * kX + half * 32;  // first streamed position of this warp's columns (query for dKV, key for dQ)
+        float* st = my_stats + b * 64;
+        if constexpr (kDKV) {
+          st[lane] = nlse;
+          st[32 + lane] = ndelta;
+          if (t + 1 < n_steps) fetch_stats(t + 1);
+          __syncwarp();
+        }
+        wait(S_FULL + b, (uint32_t)(g >> 1) & 1u);
+        ptx::tc_fence_after();
+        const uint32_t tS = lane_addr + kTmS + b * 64 + half * 32, tDP = lane_addr + kTmDP + b * 64 + half * 32;
+        bool need_mask, none;         // some / all elements of the warp's block are hidden (uniform)
+        if constexpr (kDKV) {
+          need_mask = p.causal && rw + 31 > x0;                        // some key > some query
+          none = x0 >= L || (p.causal && rw > x0 + 31);
+        } else {
+          need_mask = x0 + 32 > L || (p.causal && x0 + 31 > rw);        // key past the end / above the diagonal
+          none = x0 >= L || (p.causal && x0 > rw + 31);
+        }
+        // visible columns of the row: dKV those at or behind its key, dQ those below lim
+        const int lim = kDKV ? r_pos - x0 : (p.causal ? min(L, r_pos + 1) : L) - x0;
+        uint32_t wp[16], wd[16];
+        auto form = [&](auto masked) {
+          uint32_t rs[32], rd[32];
+          ptx::tc_ld_32x32(tS, rs);
+          ptx::tc_ld_32x32(tDP, rd);
+          ptx::tc_wait_ld();
 #pragma unroll
-    for (int blk = 0; blk < C::kDBlocks; ++blk) {
-      if (!kDKV && blk != half) continue;
-      const bool second = kDKV && half == 1;
-      const int64_t ld = second ? p.ld2 : p.ld1;
-      T* dst = reinterpret_cast<T*>(second ? p.out2 : p.out1) + (int64_t)head * kD + blk * 64 + (lane & 7) * 8;
-      uint32_t o[64];
-      ptx::tc_ld_32x32(lane_addr + (second ? kTmAcc2 : kTmAcc1) + blk * 64, o);
-      ptx::tc_ld_32x32(lane_addr + (second ? kTmAcc2 : kTmAcc1) + blk * 64 + 32, o + 32);
-      ptx::tc_wait_ld();
+          for (int i = 0; i < 32; i += 4) {
+            [[maybe_unused]] float l4[4], d4[4];
+            if constexpr (kDKV) {
+              *reinterpret_cast<float4*>(l4) = *reinterpret_cast<const float4*>(st + i);
+              *reinterpret_cast<float4*>(d4) = *reinterpret_cast<const float4*>(st + 32 + i);
+            }
 #pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        uint32_t v[4];
+            for (int e = 0; e < 4; e += 2) {
+              float x0_ = __uint_as_float(rs[i + e]), x1_ = __uint_as_float(rs[i + e + 1]), g0 = __uint_as_float(rd[i + e]), g1 = __uint_as_float(rd[i + e + 1]);
+              if constexpr (kDKV) {
+                fma_pair2(x0_, x1_, sl2, l4[e], l4[e + 1]);
+                add_pair(g0, g1, d4[e], d4[e + 1]);
+              } else {
+                fma_pair(x0_, x1_, sl2, nlse_r);
+                add_pair(g0, g1, ndelta_r, ndelta_r);
+              }
+              float p0 = exp2f(x0_), p1 = exp2f(x1_);
+              if constexpr (decltype(masked)::value) {
+                if (kDKV ? i + e < lim : i + e >= lim) p0 = 0.f;
+                if (kDKV ? i + e + 1 < lim : i + e + 1 >= lim) p1 = 0.f;
+              }
+              if constexpr (kDKV) wp[(i + e) >> 1] = pack2<T>(p0, p1);
+              mul_pair(g0, g1, p0, p1);
+              mul_pair(g0, g1, p.scale, p.scale);
+              wd[(i + e) >> 1] = pack2<T>(g0, g1);
+            }
+          }
+        };
+        if (none) {
 #pragma unroll
-        for (int e = 0; e < 4; ++e) v[e] = pack2<T>(__uint_as_float(o[8 * c + 2 * e]), __uint_as_float(o[8 * c + 2 * e + 1]));
-        st_shared_v4(stage + lane * 128 + ((c ^ (lane & 7)) << 4), v[0], v[1], v[2], v[3]);
+          for (int i = 0; i < 16; ++i) wp[i] = wd[i] = 0u;
+        } else if (need_mask) {
+          form(std::true_type{});
+        } else {
+          form(std::false_type{});
+        }
+        if constexpr (kDKV) ptx::tc_st_32x16(tS, wp);
+        ptx::tc_st_32x16(tDP, wd);
+        ptx::tc_wait_st();
+        ptx::tc_fence_before();
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive(bar(P_FULL + b));
       }
-      __syncwarp();
+
+      // ---- accumulators -> global, 64 columns at a time through the warp's staging rows; dKV: the first four warps store dV, the others dK; dQ:
+      // each half of the warps one 64-column block
+      wait(ACC_FULL, (uint32_t)n_it & 1u);
+      ptx::tc_fence_after();
+      auto release = [&] {
+        ptx::tc_fence_before();
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive(bar(ACC_EMPTY));
+      };
+      if (!kDKV && half >= C::kDBlocks) release();
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int rr = i * 4 + (lane >> 3), pos = rw + rr;
-        const uint4 v = ld_shared_v4(stage + rr * 128 + (((lane & 7) ^ (rr & 7)) << 4));
-        if (pos < L) *reinterpret_cast<uint4*>(dst + (int64_t)(tok0 + pos) * ld) = v;
+      for (int blk = 0; blk < C::kDBlocks; ++blk) {
+        if (!kDKV && blk != half) continue;
+        const bool second = kDKV && half == 1;
+        const int64_t ld = second ? p.ld2 : p.ld1;
+        T* dst = reinterpret_cast<T*>(second ? p.out2 : p.out1) + (int64_t)head * kD + blk * 64 + (lane & 7) * 8;
+        uint32_t o[64];
+        ptx::tc_ld_32x32(lane_addr + (second ? kTmAcc2 : kTmAcc1) + blk * 64, o);
+        ptx::tc_ld_32x32(lane_addr + (second ? kTmAcc2 : kTmAcc1) + blk * 64 + 32, o + 32);
+        ptx::tc_wait_ld();
+        if (!kDKV || blk == C::kDBlocks - 1) release();
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          uint32_t v[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) v[e] = pack2<T>(__uint_as_float(o[8 * c + 2 * e]), __uint_as_float(o[8 * c + 2 * e + 1]));
+          st_shared_v4(stage + lane * 128 + ((c ^ (lane & 7)) << 4), v[0], v[1], v[2], v[3]);
+        }
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int rr = i * 4 + (lane >> 3), pos = rw + rr;
+          const uint4 v = ld_shared_v4(stage + rr * 128 + (((lane & 7) ^ (rr & 7)) << 4));
+          if (pos < L) *reinterpret_cast<uint4*>(dst + (int64_t)(tok0 + pos) * ld) = v;
+        }
+        __syncwarp();
       }
-      __syncwarp();
     }
   }
 
@@ -371,17 +458,20 @@ __global__ void __launch_bounds__(256) attn_delta_kernel(const T* __restrict__ o
 }
 
 template <int kD, typename T, int kFmt, bool kDKV>
-int launch_bwd(const CUtensorMap& r1, const CUtensorMap& r2, const CUtensorMap& x1, const CUtensorMap& x2, const BwdParams& p,
-               int heads, int B, int max_seqlen, cudaStream_t s) {
+int launch_bwd(const CUtensorMap& r1, const CUtensorMap& r2, const CUtensorMap& x1, const CUtensorMap& x2, BwdParams p, cudaStream_t s) {
   using C = BCfg<kD>;
+  static_assert(C::kSmemBytes <= kMaxSmem, "shared memory");
   auto kern = attn_bwd_kernel<kD, T, kFmt, kDKV>;
   static bool attr_set = false;
   if (!attr_set) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes) != cudaSuccess) return -30;
     attr_set = true;
   }
-  dim3 grid(RB_CEIL_DIV(max_seqlen, kR), heads, B);
-  kern<<<grid, kBwdThreads, C::kSmemBytes, s>>>(r1, r2, x1, x2, p);
+  p.heads = kDKV ? p.nkv : p.nq;
+  // the sequences' lengths are on the device: sum of ceil(L / kR) is at most (T + (kR - 1) B) / kR
+  const int64_t n = (p.T + (int64_t)(kR - 1) * p.B) / kR * p.heads;
+  if (n <= 0 || n > 0x7fffffff) return -33;
+  kern<<<dim3((unsigned)n), kBwdThreads, C::kSmemBytes, s>>>(r1, r2, x1, x2, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -31;
 }
 
@@ -402,11 +492,11 @@ int run_bwd(const void* q, const void* k, const void* v, const void* out, const 
       !make_tmap(&q128, q, bf, Tn, (uint64_t)nq * kD, q_ld, 64, kR) || !make_tmap(&do128, dout, bf, Tn, (uint64_t)nq * kD, do_ld, 64, kR) ||
       !make_tmap(&k64, k, bf, Tn, (uint64_t)nkv * kD, k_ld, 64, kX) || !make_tmap(&v64, v, bf, Tn, (uint64_t)nkv * kD, v_ld, 64, kX))
     return -10;
-  BwdParams pkv{cu, lse, delta, dv, dk, dv_ld, dk_ld, Tn, nq, nkv, scale, causal};
-  int rc = launch_bwd<kD, T, kFmt, true>(k128, v128, q64, do64, pkv, nkv, B, max_seqlen, s);
+  BwdParams pkv{cu, lse, delta, dv, dk, dv_ld, dk_ld, Tn, B, nq, nkv, 0, scale, causal};
+  int rc = launch_bwd<kD, T, kFmt, true>(k128, v128, q64, do64, pkv, s);
   if (rc != 0) return rc;
-  BwdParams pq{cu, lse, delta, dq, nullptr, dq_ld, 0, Tn, nq, nkv, scale, causal};
-  return launch_bwd<kD, T, kFmt, false>(q128, do128, k64, v64, pq, nq, B, max_seqlen, s);
+  BwdParams pq{cu, lse, delta, dq, nullptr, dq_ld, 0, Tn, B, nq, nkv, 0, scale, causal};
+  return launch_bwd<kD, T, kFmt, false>(q128, do128, k64, v64, pq, s);
 }
 
 }  // namespace

@@ -64,10 +64,61 @@ template <> RB_DEVICE uint32_t pack2<__half>(float lo, float hi) {
   return *reinterpret_cast<uint32_t*>(&v);
 }
 
+// Which sequence a row unit belongs to, units of `rows` rows numbered sequence by sequence; run by a whole warp.  The numbers asked for mostly
+// grow, so the search goes on from the last block of 32 sequences.
+struct UnitSearch {
+  int base = 0, s0 = 0;      // units in front of sequence s0
+  // true: `tok0`, `L` of the sequence and the unit's number `r` in it; false: beyond the last sequence
+  RB_DEVICE bool find(const int* cu, int B, int rows, int unit, int& tok0, int& L, int& r) {
+    const int lane = threadIdx.x & 31;
+    if (unit < base) { base = 0; s0 = 0; }
+    for (; s0 < B; s0 += 32) {
+      const int s = s0 + lane, a = s < B ? cu[s] : 0, len = s < B ? max(cu[s + 1] - a, 0) : 0, c = (len + rows - 1) / rows;
+      int incl = c;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+      }
+      const unsigned hit = __ballot_sync(0xffffffffu, base + incl > unit);
+      if (hit != 0) {
+        const int w = __ffs(hit) - 1;
+        tok0 = __shfl_sync(0xffffffffu, a, w);
+        L = __shfl_sync(0xffffffffu, len, w);
+        r = unit - base - __shfl_sync(0xffffffffu, incl - c, w);
+        return true;
+      }
+      base += __shfl_sync(0xffffffffu, incl, 31);
+    }
+    base = 0;
+    s0 = 0;
+    return false;
+  }
+};
+
 // cap * tanh(s * scale / cap) + add in the log2 domain, tanh(x) = 1 - 2 / (1 + 2^(2 x log2 e)): c = 2 log2 e * scale / cap,
 // k = cap log2 e, k_add = k + add.  Absolute error a few ulp of k; saturates to +-k.
 RB_DEVICE float soft_cap2(float s, float c, float k, float k_add) {
   return fmaf(-2.f * k, __fdividef(1.f, 1.f + exp2f(fminf(s * c, 80.f))), k_add);
+}
+
+// One instruction for two numbers: (x0, x1) <- (x0, x1) * m + a; (x0, x1) <- (x0, x1) * m + (a0, a1); (s0, s1) <- (s0, s1) + (a0, a1);
+// (x0, x1) <- (x0, x1) * (m0, m1)
+RB_DEVICE void fma_pair(float& x0, float& x1, float m, float a) {
+  asm("{\n\t.reg .b64 x, m, a;\n\tmov.b64 x, {%0, %1};\n\tmov.b64 m, {%2, %2};\n\tmov.b64 a, {%3, %3};\n\tfma.rn.f32x2 x, x, m, a;\n\tmov.b64 {%0, %1}, x;\n\t}"
+      : "+f"(x0), "+f"(x1) : "f"(m), "f"(a));
+}
+RB_DEVICE void add_pair(float& s0, float& s1, float a0, float a1) {
+  asm("{\n\t.reg .b64 s, a;\n\tmov.b64 s, {%0, %1};\n\tmov.b64 a, {%2, %3};\n\tadd.rn.f32x2 s, s, a;\n\tmov.b64 {%0, %1}, s;\n\t}"
+      : "+f"(s0), "+f"(s1) : "f"(a0), "f"(a1));
+}
+RB_DEVICE void fma_pair2(float& x0, float& x1, float m, float a0, float a1) {
+  asm("{\n\t.reg .b64 x, m, a;\n\tmov.b64 x, {%0, %1};\n\tmov.b64 m, {%2, %2};\n\tmov.b64 a, {%3, %4};\n\tfma.rn.f32x2 x, x, m, a;\n\tmov.b64 {%0, %1}, x;\n\t}"
+      : "+f"(x0), "+f"(x1) : "f"(m), "f"(a0), "f"(a1));
+}
+RB_DEVICE void mul_pair(float& x0, float& x1, float m0, float m1) {
+  asm("{\n\t.reg .b64 x, m;\n\tmov.b64 x, {%0, %1};\n\tmov.b64 m, {%2, %3};\n\tmul.rn.f32x2 x, x, m;\n\tmov.b64 {%0, %1}, x;\n\t}"
+      : "+f"(x0), "+f"(x1) : "f"(m0), "f"(m1));
 }
 
 }  // namespace

@@ -62,16 +62,6 @@ enum FBar { Q_FULL = 0, Q_EMPTY = 2, KV_FULL = 4, KV_EMPTY = 8, S_FULL = 12, P_F
 
 __device__ int g_wait_error = 0;
 
-// (x0, x1) <- (x0, x1) * m + a and (s0, s1) <- (s0, s1) + (a0, a1), one instruction each
-RB_DEVICE void fma_pair(float& x0, float& x1, float m, float a) {
-  asm("{\n\t.reg .b64 x, m, a;\n\tmov.b64 x, {%0, %1};\n\tmov.b64 m, {%2, %2};\n\tmov.b64 a, {%3, %3};\n\tfma.rn.f32x2 x, x, m, a;\n\tmov.b64 {%0, %1}, x;\n\t}"
-      : "+f"(x0), "+f"(x1) : "f"(m), "f"(a));
-}
-RB_DEVICE void add_pair(float& s0, float& s1, float a0, float a1) {
-  asm("{\n\t.reg .b64 s, a;\n\tmov.b64 s, {%0, %1};\n\tmov.b64 a, {%2, %3};\n\tadd.rn.f32x2 s, s, a;\n\tmov.b64 {%0, %1}, s;\n\t}"
-      : "+f"(s0), "+f"(s1) : "f"(a0), "f"(a1));
-}
-
 // One work item: sequence (first token, length), heads and query tiles of the two tiles (tile 1 < 0: absent); L < 0 ends the CTA's loop.
 struct Item { int tok0, L, head0, head1, qt0, qt1; };
 
@@ -143,39 +133,17 @@ __global__ void __launch_bounds__(kFwdThreads, 1) attn_fwd_kernel(const __grid_c
         }
         __syncwarp();
       };
-      int unit_base = 0, s0 = 0;    // work units in front of sequence block [s0, s0 + 32): item numbers mostly grow, so the search goes on from here
+      UnitSearch search;
       auto find = [&](int idx, Item& it) {
         const int unit = idx / p.n_head_units, hu = idx - unit * p.n_head_units;
-        if (unit < unit_base) { unit_base = 0; s0 = 0; }
-        for (; s0 < p.B; s0 += 32) {
-          const int s = s0 + lane;
-          const int a = s < p.B ? p.cu_seqlens[s] : 0;
-          const int L = s < p.B ? max(p.cu_seqlens[s + 1] - a, 0) : 0;
-          const int c = p.pair_heads ? RB_CEIL_DIV(L, kTile) : RB_CEIL_DIV(L, 2 * kTile);
-          int incl = c;
-#pragma unroll
-          for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += v;
-          }
-          const unsigned hit = __ballot_sync(0xffffffffu, unit_base + incl > unit);
-          if (hit != 0) {
-            const int w = __ffs(hit) - 1;
-            it.tok0 = __shfl_sync(0xffffffffu, a, w);
-            it.L = __shfl_sync(0xffffffffu, L, w);
-            const int r = unit - unit_base - __shfl_sync(0xffffffffu, incl - c, w);   // r-th unit of the sequence, longest first
-            const int last = RB_CEIL_DIV(it.L, kTile) - 1;
-            it.head0 = p.pair_heads ? 2 * hu : hu;
-            it.head1 = p.pair_heads ? 2 * hu + 1 : hu;
-            it.qt0 = p.pair_heads ? last - r : last - 2 * r;
-            it.qt1 = p.pair_heads ? last - r : last - 2 * r - 1;
-            return true;
-          }
-          unit_base += __shfl_sync(0xffffffffu, incl, 31);
-        }
-        unit_base = 0;
-        s0 = 0;
-        return false;
+        int r;                       // r-th unit of the sequence, longest first
+        if (!search.find(p.cu_seqlens, p.B, p.pair_heads ? kTile : 2 * kTile, unit, it.tok0, it.L, r)) return false;
+        const int last = RB_CEIL_DIV(it.L, kTile) - 1;
+        it.head0 = p.pair_heads ? 2 * hu : hu;
+        it.head1 = p.pair_heads ? 2 * hu + 1 : hu;
+        it.qt0 = p.pair_heads ? last - r : last - 2 * r;
+        it.qt1 = p.pair_heads ? last - r : last - 2 * r - 1;
+        return true;
       };
 
       int idx = blockIdx.x, n_pub = 0;
