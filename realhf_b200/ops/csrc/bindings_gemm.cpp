@@ -202,8 +202,8 @@ Tensor gemm_grouped(const Tensor& a, const Tensor& w, const Tensor& offsets, boo
 extern "C" int rb_gemm_grouped_wgrad(const void* dy, const void* x, void* out, const int* offsets, int G, int Tp, int M, int N,
                                      int64_t ld_dy, int64_t ld_x, int out_dt, int accumulate, int num_sms, cudaStream_t s);
 
-// Grouped wgrad: out[g] (+)= dy[rows of g]^T @ x[rows of g]; rows sorted by group with every group's block padded (zero rows) to a
-// multiple of 64, `offsets` int32 [G+1] on the device holding the PADDED block starts.  out [G, M, N] fp32 or bf16.
+// Grouped wgrad: out[g] (+)= dy[rows of g]^T @ x[rows of g]; rows sorted by group, `offsets` int32 [G+1] on the device holding the groups'
+// row ranges.  out [G, M, N] fp32 or bf16.
 void gemm_grouped_wgrad(const Tensor& dy, const Tensor& x, Tensor out, const Tensor& offsets, bool accumulate, int64_t num_sms) {
   TORCH_CHECK(dy.is_cuda() && dy.dim() == 2 && x.dim() == 2 && out.dim() == 3 && dy.scalar_type() == at::kBFloat16 &&
               x.scalar_type() == at::kBFloat16 && dy.stride(1) == 1 && x.stride(1) == 1 && out.is_contiguous());

@@ -25,7 +25,8 @@ template <int BN> struct Cfg2 {
   static constexpr int kStageBytes = kABytes + kBBytes;
   static constexpr int kStages = BN == 256 ? 6 : 8;
   static constexpr int kTmemCols = 2 * BN;
-  static constexpr int kSmemBytes = kStages * kStageBytes + 1024 /*align*/ + 256 /*barriers*/;
+  static constexpr int kOut = kStages * kStageBytes, kBars = kOut + 4 * 4096;   // 4 KB of output staging per epilogue warp
+  static constexpr int kSmemBytes = kBars + 1024 /*align*/ + 256 /*barriers*/;
 };
 
 RB_DEVICE uint32_t cluster_ctarank() {
@@ -102,7 +103,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_2cta_kernel(const __grid_con
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   uint8_t* smem_a = smem;
   uint8_t* smem_b = smem + C::kStages * C::kABytes;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::kStages * C::kStageBytes);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::kBars);
   uint64_t* full_bar = bars;                      // used on the leader only
   uint64_t* empty_bar = bars + C::kStages;        // one per CTA, armed by the leader's multicast commit
   uint64_t* tmem_full = bars + 2 * C::kStages;    // one per CTA
@@ -181,32 +182,32 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_2cta_kernel(const __grid_con
       }
     }
   } else if (warp == 1) {
-    // ===================================================== MMA issuer (leader CTA only)
-    if (leader && lane == 0) {
+    // ===================================================== MMA issuer (leader CTA only): the warp runs converged, one elected lane issues
+    if (leader) {
       constexpr uint32_t idesc = ptx::make_idesc_f16(kFmt, 2 * BM, BN, kAMN ? 1 : 0, kBMN ? 1 : 0);
+      constexpr uint32_t kAStep = (kAMN ? 2048 : 32) >> 4, kBStep = (kBMN ? 2048 : 32) >> 4;      // 16 K elements further, in descriptor units
+      const uint32_t tm = (uint32_t)ptx::uniform((int)tmem_base);
       int stage = 0, as = 0;
       uint32_t phase = 0, aphase = 0;
       for (int tile = pair; tile < num_tiles; tile += num_pairs) {
         ptx::mbar_wait(ptx::smem_u32(&tmem_empty[as]), aphase ^ 1);
         ptx::tc_fence_after();
-        const uint32_t d_tmem = tmem_base + as * BN;
+        const uint32_t d_tmem = tm + as * BN;
         for (int kb = 0; kb < num_kb; ++kb) {
           ptx::mbar_wait(ptx::smem_u32(&full_bar[stage]), phase);
           ptx::tc_fence_after();
-          const uint32_t sa = ptx::smem_u32(smem_a + stage * C::kABytes);
-          const uint32_t sb = ptx::smem_u32(smem_b + stage * C::kBBytes);
+          const uint64_t da = ptx::make_smem_desc_sw128(ptx::smem_u32(smem_a + stage * C::kABytes), kAMN ? BK * 128 : 16, 1024);
+          const uint64_t db = ptx::make_smem_desc_sw128(ptx::smem_u32(smem_b + stage * C::kBBytes), kBMN ? BK * 128 : 16, 1024);
+          if (ptx::elect_one()) {
 #pragma unroll
-          for (int k = 0; k < BK / 16; ++k) {
-            const uint64_t adesc = kAMN ? ptx::make_smem_desc_sw128(sa + k * 2048, BK * 128, 1024)
-                                        : ptx::make_smem_desc_sw128(sa + k * 32, 16, 1024);
-            const uint64_t bdesc = kBMN ? ptx::make_smem_desc_sw128(sb + k * 2048, BK * 128, 1024)
-                                        : ptx::make_smem_desc_sw128(sb + k * 32, 16, 1024);
-            tc_mma_f16_cg2(d_tmem, adesc, bdesc, idesc, (kb | k) != 0 ? 1u : 0u);
+            for (int k = 0; k < BK / 16; ++k) tc_mma_f16_cg2(d_tmem, da + k * kAStep, db + k * kBStep, idesc, (kb | k) != 0 ? 1u : 0u);
+            tc_commit_cg2(ptx::smem_u32(&empty_bar[stage]), 0b11);  // frees the stage in both CTAs once these MMAs retire
           }
-          tc_commit_cg2(ptx::smem_u32(&empty_bar[stage]), 0b11);  // frees the stage in both CTAs once these MMAs retire
+          __syncwarp();
           if (++stage == C::kStages) { stage = 0; phase ^= 1; }
         }
-        tc_commit_cg2(ptx::smem_u32(&tmem_full[as]), 0b11);  // accumulator complete -> both epilogues
+        if (ptx::elect_one()) tc_commit_cg2(ptx::smem_u32(&tmem_full[as]), 0b11);  // accumulator complete -> both epilogues
+        __syncwarp();
         if (++as == 2) { as = 0; aphase ^= 1; }
       }
     }
@@ -217,13 +218,14 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_2cta_kernel(const __grid_con
     uint32_t aphase = 0;
     OutT* Cp = reinterpret_cast<OutT*>(p.C);
     const OutT* bias = reinterpret_cast<const OutT*>(p.bias);
+    const uint32_t out_stage = ptx::smem_u32(smem + C::kOut + quad * 4096);
     const bool vec_ok = (p.ldc % (16 / sizeof(OutT)) == 0) && ((reinterpret_cast<uintptr_t>(p.C) & 15) == 0);
     for (int tile = pair; tile < num_tiles; tile += num_pairs) {
       int m0, n0;
       tile_coords2(tile, tiles_m, tiles_n, kTileN, p.m_rot, m0, n0);
       ptx::mbar_wait(ptx::smem_u32(&tmem_full[as]), aphase);
       ptx::tc_fence_after();
-      const int row = m0 + (int)rank * BM + quad * 32 + lane;
+      const int row0 = m0 + (int)rank * BM + quad * 32;
       const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + as * BN;
       if constexpr (kGlu) {
         OutT* raw = reinterpret_cast<OutT*>(p.glu_raw);
@@ -236,7 +238,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_2cta_kernel(const __grid_con
           ptx::tc_wait_ld();
           const int col = n0 + c * 32;
           const int n_valid = min(32, p.N - col);
-          if (row < p.M && n_valid > 0) {
+          if (row0 < p.M && n_valid > 0) {
             float g[32], u[32], v[32];
 #pragma unroll
             for (int i = 0; i < 32; ++i) {
@@ -252,10 +254,10 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_2cta_kernel(const __grid_con
                 v[i] = glu_act_fwd(gr, p.glu_act) * ur;
               }
             }
-            store_chunk<OutT>(Cp + (int64_t)row * p.ldc + col, v, n_valid, vec_ok);
+            store_rows32<OutT>(out_stage, v, Cp + (int64_t)row0 * p.ldc + col, p.ldc, p.M - row0, n_valid, vec_ok, false);
             if (raw != nullptr) {
-              store_chunk<OutT>(raw + (int64_t)row * p.ld_raw + col, g, n_valid, raw_vec);
-              store_chunk<OutT>(raw + (int64_t)row * p.ld_raw + p.glu_F + col, u, n_valid, raw_vec);
+              store_rows32<OutT>(out_stage, g, raw + (int64_t)row0 * p.ld_raw + col, p.ld_raw, p.M - row0, n_valid, raw_vec, false);
+              store_rows32<OutT>(out_stage, u, raw + (int64_t)row0 * p.ld_raw + p.glu_F + col, p.ld_raw, p.M - row0, n_valid, raw_vec, false);
             }
           }
         }
@@ -267,7 +269,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_2cta_kernel(const __grid_con
         ptx::tc_wait_ld();
         const int col = n0 + c * 32;
         const int n_valid = min(32, p.N - col);
-        if (row < p.M && n_valid > 0) {
+        if (row0 < p.M && n_valid > 0) {
           float v[32];
 #pragma unroll
           for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
@@ -282,12 +284,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_2cta_kernel(const __grid_con
               if (col + i < p.act_cols) v[i] = a * a;
             }
           }
-          OutT* dst = Cp + (int64_t)row * p.ldc + col;
-          if (p.accumulate) {
-#pragma unroll
-            for (int i = 0; i < 32; ++i) if (i < n_valid) v[i] += rb::to_f(dst[i]);
-          }
-          store_chunk<OutT>(dst, v, n_valid, vec_ok);
+          store_rows32<OutT>(out_stage, v, Cp + (int64_t)row0 * p.ldc + col, p.ldc, p.M - row0, n_valid, vec_ok, p.accumulate);
         }
       }
       }

@@ -65,6 +65,44 @@ template <typename T> RB_DEVICE void store_chunk(T* dst, const float* v, int n_v
   }
 }
 
+// 32 accumulator columns of a warp's 32 rows (lane = row) to memory, through 4 KB of shared memory of the warp at `stage` (1 KB aligned): a lane holds a
+// row, so storing from it writes 32 lines per instruction in 16-byte pieces, and adding to the old value fetched those one element at a time.  Staged as
+// fp32, four lines per instruction leave whole, and the old values of an accumulating GEMM come in the same way; the sum is formed in fp32.
+// dst: first row and column; rows / cols: how many are real.
+template <typename T> RB_DEVICE void store_rows32(uint32_t stage, const float (&v)[32], T* dst, int64_t ldc, int rows, int cols, bool vec_ok, bool accumulate) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int q = 0; q < 8; ++q)
+    asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(stage + lane * 128 + ((q ^ (lane & 7)) << 4)), "f"(v[4 * q]), "f"(v[4 * q + 1]), "f"(v[4 * q + 2]),
+                 "f"(v[4 * q + 3])
+                 : "memory");
+  __syncwarp();
+  const int q = lane & 7, c = q * 4;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int r = i * 4 + (lane >> 3);
+    float x[4];
+    asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(x[0]), "=f"(x[1]), "=f"(x[2]), "=f"(x[3]) : "r"(stage + r * 128 + ((q ^ (r & 7)) << 4)) : "memory");
+    if (r < rows && c < cols) {
+      T* d = dst + (int64_t)r * ldc + c;
+      if (vec_ok && c + 4 <= cols) {
+        rb::Pack<T, 4> o;
+        if (accumulate) {
+          const rb::Pack<T, 4> old = *reinterpret_cast<const rb::Pack<T, 4>*>(d);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) x[k] += rb::to_f(old.v[k]);
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) o.v[k] = rb::from_f<T>(x[k]);
+        *reinterpret_cast<rb::Pack<T, 4>*>(d) = o;
+      } else {
+        for (int k = 0; k < 4 && c + k < cols; ++k) d[k] = rb::from_f<T>(accumulate ? x[k] + rb::to_f(d[k]) : x[k]);
+      }
+    }
+  }
+  __syncwarp();
+}
+
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                   const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);

@@ -1,49 +1,52 @@
 // Grouped weight-gradient GEMM for MoE experts in ONE launch:
 //
-//   dW[g] [M, N] (+)= dY_g^T X_g          dY [Tp, M], X [Tp, N] hold the tokens sorted by expert, expert g owns the row range
-//                                          [off[g], off[g+1]) and every off[g] is a multiple of 64 (the dispatch pads each
-//                                          expert's block with zero rows), so a 64-row K block never straddles two experts.
+//   dW[g] [M, N] (+)= dY_g^T X_g          dY [T, M], X [T, N] hold the tokens sorted by expert, expert g owns the row range [off[g], off[g+1])
 //
 // Reference: grouped_gemm's `gmm(..., trans_a=True)` in the experts' backward (impl/model/modules/moe/experts.py); the first
 // version here ran one GEMM per expert after a host read of the token counts.  This kernel is the wgrad form of the tile GEMM
 // (`gemm_tcgen05.cu`: both operands MN-major, K = tokens) with the K range taken per tile from the device-side offsets:
-// tile -> (expert, m-tile, n-tile), persistent CTAs, TMA producer warp / single-thread tcgen05.mma issuer / four epilogue
-// warps, smem ring + double-buffered TMEM accumulators.  An expert without tokens gets zeros (or is left alone when
-// accumulating).
+// tile -> (expert, m-tile, n-tile), persistent CTAs, TMA producer warp / converged tcgen05.mma issuer / four epilogue warps, smem ring + double-buffered
+// TMEM accumulators.  The last 64-row K block of an expert may reach into the next one's rows: a warp of its own zeroes
+// those rows of both staged operands before the MMAs read them.  (Scattering both operands into buffers padded to 64 rows per expert took
+// 720 us of an 8 x 14336 x 4096 feed-forward's backward on 4096 rows.)  An expert without tokens gets zeros (or is left alone when accumulating).
 //
-// STATUS: compiled for sm_100a, not yet run on hardware: opt-in (`REAL_MOE_GROUPED_WGRAD=1`), GPU test gated by
-// REAL_TEST_EXPERIMENTAL=1; the padding / offset logic around it is tested on CPU.
+// What bounds it: with a few hundred tokens per expert a tile is 4096 tensor-pipe cycles and 64 KB of output, so the epilogue has to
+// leave in whole lines (store_rows32): rows stored lane by lane took as long as the products (2281 us for the two of that backward).
 #include "gemm_common.cuh"
 
 namespace {
 
 struct WgradParams {
   void* C;          // [G, M, N]
-  const int* off;   // [G + 1], multiples of 64
+  const int* off;   // [G + 1]
   int G, M, N;
   int accumulate;
 };
+
+constexpr int kWgradThreads = 224;   // warp 6: tail rows
 
 template <int BN> struct WCfg {
   static constexpr int kStages = BN >= 256 ? 4 : 6;
   static constexpr int kABytes = BM * BK * 2;   // [2 chunks of 64 m][64 k rows][128 B]
   static constexpr int kBBytes = BN * BK * 2;   // [BN/64 chunks][64 k rows][128 B]
   static constexpr int kStageBytes = kABytes + kBBytes;
-  static constexpr int kSmemBytes = kStages * kStageBytes + 1024 + 256;
+  static constexpr int kOut = kStages * kStageBytes, kBars = kOut + 4 * 4096;   // 4 KB of output staging per epilogue warp
+  static constexpr int kSmemBytes = kBars + 1024 + 256;
 };
 
 template <int BN, typename OutT>
-__global__ void __launch_bounds__(kThreads, 1) grouped_wgrad_kernel(const __grid_constant__ CUtensorMap tma_a,
+__global__ void __launch_bounds__(kWgradThreads, 1) grouped_wgrad_kernel(const __grid_constant__ CUtensorMap tma_a,
                                                                     const __grid_constant__ CUtensorMap tma_b, WgradParams p) {
   using C = WCfg<BN>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   uint8_t* smem_a = smem;
   uint8_t* smem_b = smem + C::kStages * C::kABytes;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::kStages * C::kStageBytes);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::kBars);
   uint64_t* full_bar = bars;
   uint64_t* empty_bar = bars + C::kStages;
-  uint64_t* tmem_full = bars + 2 * C::kStages;
+  uint64_t* tail_bar = bars + 2 * C::kStages;     // a stage whose rows behind the expert's last one have been zeroed
+  uint64_t* tmem_full = bars + 3 * C::kStages;
   uint64_t* tmem_empty = tmem_full + 2;
   uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(tmem_empty + 2);
 
@@ -51,14 +54,16 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_wgrad_kernel(const __grid
   const int tiles_m = RB_CEIL_DIV(p.M, BM), tiles_n = RB_CEIL_DIV(p.N, BN);
   const int tpg = tiles_m * tiles_n;
   const int num_tiles = p.G * tpg;
-  // tile -> (expert, m0, n0, first token row, number of 64-row K blocks); m fastest so neighbouring CTAs share the X panel
-  auto coords = [&](int tile, int& g, int& m0, int& n0, int& r0, int& nkb) {
+  // tile -> (expert, m0, n0, first token row, number of 64-row K blocks, real rows of the last one); m fastest so neighbouring CTAs share the X panel
+  auto coords = [&](int tile, int& g, int& m0, int& n0, int& r0, int& nkb, int& tail) {
     g = tile / tpg;
     const int local = tile - g * tpg;
     m0 = (local % tiles_m) * BM;
     n0 = (local / tiles_m) * BN;
     r0 = p.off[g];
-    nkb = (p.off[g + 1] - r0) / BK;
+    const int rows = p.off[g + 1] - r0;
+    nkb = RB_CEIL_DIV(rows, BK);
+    tail = rows - (nkb - 1) * BK;
   };
 
   if (warp == 0 && lane == 0) {
@@ -66,7 +71,8 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_wgrad_kernel(const __grid
     ptx::prefetch_tensormap(&tma_b);
     for (int i = 0; i < C::kStages; ++i) {
       ptx::mbar_init(ptx::smem_u32(&full_bar[i]), 1);
-      ptx::mbar_init(ptx::smem_u32(&empty_bar[i]), 1);
+      ptx::mbar_init(ptx::smem_u32(&empty_bar[i]), 2);      // the MMAs' commit and the tail warp
+      ptx::mbar_init(ptx::smem_u32(&tail_bar[i]), 1);
     }
     for (int i = 0; i < 2; ++i) {
       ptx::mbar_init(ptx::smem_u32(&tmem_full[i]), 1);
@@ -88,8 +94,8 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_wgrad_kernel(const __grid
       int stage = 0;
       uint32_t phase = 0;
       for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
-        int g, m0, n0, r0, nkb;
-        coords(tile, g, m0, n0, r0, nkb);
+        int g, m0, n0, r0, nkb, tail;
+        coords(tile, g, m0, n0, r0, nkb, tail);
         for (int kb = 0; kb < nkb; ++kb) {
           ptx::mbar_wait(ptx::smem_u32(&empty_bar[stage]), phase ^ 1);
           const uint32_t fb = ptx::smem_u32(&full_bar[stage]);
@@ -106,30 +112,62 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_wgrad_kernel(const __grid
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = ptx::make_idesc_f16(1, BM, BN, 1, 1);
-      int stage = 0, as = 0;
-      uint32_t phase = 0, aphase = 0;
-      for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
-        int g, m0, n0, r0, nkb;
-        coords(tile, g, m0, n0, r0, nkb);
-        ptx::mbar_wait(ptx::smem_u32(&tmem_empty[as]), aphase ^ 1);
-        ptx::tc_fence_after();
-        const uint32_t d_tmem = tmem_base + as * BN;
-        for (int kb = 0; kb < nkb; ++kb) {
+    constexpr uint32_t idesc = ptx::make_idesc_f16(1, BM, BN, 1, 1);
+    const uint32_t tm = (uint32_t)ptx::uniform((int)tmem_base);
+    int stage = 0, as = 0;
+    uint32_t phase = 0, aphase = 0, tails = 0;     // tails: bit s = phase of tail_bar[s]
+    for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
+      int g, m0, n0, r0, nkb, tail;
+      coords(tile, g, m0, n0, r0, nkb, tail);
+      nkb = ptx::uniform(nkb);
+      tail = ptx::uniform(tail);
+      ptx::mbar_wait(ptx::smem_u32(&tmem_empty[as]), aphase ^ 1);
+      ptx::tc_fence_after();
+      const uint32_t d_tmem = tm + as * BN;
+      for (int kb = 0; kb < nkb; ++kb) {
+        if (kb == nkb - 1 && tail < BK) {
+          ptx::mbar_wait(ptx::smem_u32(&tail_bar[stage]), (tails >> stage) & 1u);
+          tails ^= 1u << stage;
+        } else {
           ptx::mbar_wait(ptx::smem_u32(&full_bar[stage]), phase);
-          ptx::tc_fence_after();
-          const uint32_t sa = ptx::smem_u32(smem_a + stage * C::kABytes);
-          const uint32_t sb = ptx::smem_u32(smem_b + stage * C::kBBytes);
-#pragma unroll
-          for (int k = 0; k < BK / 16; ++k)
-            ptx::tc_mma_f16(d_tmem, ptx::make_smem_desc_sw128(sa + k * 2048, BK * 128, 1024),
-                            ptx::make_smem_desc_sw128(sb + k * 2048, BK * 128, 1024), idesc, (kb | k) != 0 ? 1u : 0u);
-          ptx::tc_commit(ptx::smem_u32(&empty_bar[stage]));
-          if (++stage == C::kStages) { stage = 0; phase ^= 1; }
         }
-        ptx::tc_commit(ptx::smem_u32(&tmem_full[as]));  // with nkb == 0 nothing is pending: arrives at once
-        if (++as == 2) { as = 0; aphase ^= 1; }
+        ptx::tc_fence_after();
+        const uint64_t da = ptx::make_smem_desc_sw128(ptx::smem_u32(smem_a + stage * C::kABytes), BK * 128, 1024);
+        const uint64_t db = ptx::make_smem_desc_sw128(ptx::smem_u32(smem_b + stage * C::kBBytes), BK * 128, 1024);
+        if (ptx::elect_one()) {
+#pragma unroll
+          for (int k = 0; k < BK / 16; ++k) ptx::tc_mma_f16(d_tmem, da + k * 128, db + k * 128, idesc, (kb | k) != 0 ? 1u : 0u);
+          ptx::tc_commit(ptx::smem_u32(&empty_bar[stage]));
+        }
+        __syncwarp();
+        if (++stage == C::kStages) { stage = 0; phase ^= 1; }
+      }
+      if (ptx::elect_one()) ptx::tc_commit(ptx::smem_u32(&tmem_full[as]));  // with nkb == 0 nothing is pending: arrives at once
+      __syncwarp();
+      if (++as == 2) { as = 0; aphase ^= 1; }
+    }
+  } else if (warp == 6) {
+    // ===================================================== rows of the next expert (or of nobody) in an expert's last K block: zero in both operands.  The
+    // warp follows every stage (and releases it too), so that it is never a turn of the ring ahead or behind.
+    int stage = 0;
+    uint32_t phase = 0;
+    for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
+      int g, m0, n0, r0, nkb, tail;
+      coords(tile, g, m0, n0, r0, nkb, tail);
+      for (int kb = 0; kb < nkb; ++kb) {
+        ptx::mbar_wait(ptx::smem_u32(&full_bar[stage]), phase);
+        if (kb == nkb - 1 && tail < BK) {
+          // chunks of 64 columns: [64 token rows][128 B], rows unswizzled among themselves
+          for (int c = 0; c < (BM + BN) / 64; ++c) {
+            uint8_t* base = c < BM / 64 ? smem_a + stage * C::kABytes + c * (BK * 128) : smem_b + stage * C::kBBytes + (c - BM / 64) * (BK * 128);
+            for (int i = tail * 8 + lane; i < BK * 8; i += 32) reinterpret_cast<uint4*>(base)[i] = make_uint4(0u, 0u, 0u, 0u);
+          }
+          ptx::fence_proxy_async();
+          __syncwarp();
+          if (lane == 0) ptx::mbar_arrive(ptx::smem_u32(&tail_bar[stage]));
+        }
+        if (lane == 0) ptx::mbar_arrive(ptx::smem_u32(&empty_bar[stage]));
+        if (++stage == C::kStages) { stage = 0; phase ^= 1; }
       }
     }
   } else {
@@ -137,13 +175,14 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_wgrad_kernel(const __grid
     int as = 0;
     uint32_t aphase = 0;
     OutT* Cp = reinterpret_cast<OutT*>(p.C);
+    const uint32_t out_stage = ptx::smem_u32(smem + C::kOut + quad * 4096);
     const bool vec_ok = (p.N % (16 / sizeof(OutT)) == 0) && ((reinterpret_cast<uintptr_t>(p.C) & 15) == 0);
     for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
-      int g, m0, n0, r0, nkb;
-      coords(tile, g, m0, n0, r0, nkb);
+      int g, m0, n0, r0, nkb, tail;
+      coords(tile, g, m0, n0, r0, nkb, tail);
       ptx::mbar_wait(ptx::smem_u32(&tmem_full[as]), aphase);
       ptx::tc_fence_after();
-      const int row = m0 + quad * 32 + lane;
+      const int row0 = m0 + quad * 32;
       const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + as * BN;
 #pragma unroll 1
       for (int c = 0; c < BN / 32; ++c) {
@@ -152,16 +191,11 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_wgrad_kernel(const __grid
         ptx::tc_wait_ld();
         const int col = n0 + c * 32;
         const int n_valid = min(32, p.N - col);
-        if (row < p.M && n_valid > 0 && !(nkb == 0 && p.accumulate)) {
+        if (n_valid > 0 && !(nkb == 0 && p.accumulate)) {
           float v[32];
 #pragma unroll
           for (int i = 0; i < 32; ++i) v[i] = nkb == 0 ? 0.f : __uint_as_float(r[i]);  // no tokens: the accumulator is stale
-          OutT* dst = Cp + ((int64_t)g * p.M + row) * p.N + col;
-          if (p.accumulate) {
-#pragma unroll
-            for (int i = 0; i < 32; ++i) if (i < n_valid) v[i] += rb::to_f(dst[i]);
-          }
-          store_chunk<OutT>(dst, v, n_valid, vec_ok);
+          store_rows32<OutT>(out_stage, v, Cp + ((int64_t)g * p.M + row0) * p.N + col, p.N, p.M - row0, n_valid, vec_ok, p.accumulate);
         }
       }
       ptx::tc_fence_before();
@@ -190,18 +224,17 @@ int launch_wgrad(const CUtensorMap& ta, const CUtensorMap& tb, const WgradParams
   }
   const int64_t tiles = (int64_t)p.G * RB_CEIL_DIV(p.M, BM) * RB_CEIL_DIV(p.N, BN);
   const int grid = (int)(tiles < num_sms ? tiles : num_sms);
-  kern<<<grid, kThreads, C::kSmemBytes, s>>>(ta, tb, p);
+  kern<<<grid, kWgradThreads, C::kSmemBytes, s>>>(ta, tb, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -31;
 }
 
 }  // namespace
 
-// dy [Tp, M], x [Tp, N] bf16 (row pitches ld*), offsets: device int32 [G + 1] with every entry a multiple of 64 and
-// offsets[G] <= Tp; out [G, M, N] contiguous, fp32 (out_dt 0) or bf16 (out_dt 1); accumulate: out += result.
+// dy [Tp, M], x [Tp, N] bf16 (row pitches ld*), offsets: device int32 [G + 1], nondecreasing, offsets[G] <= Tp; out [G, M, N] contiguous, fp32 (out_dt 0) or bf16 (out_dt 1); accumulate: out += result.
 extern "C" int rb_gemm_grouped_wgrad(const void* dy, const void* x, void* out, const int* offsets, int G, int Tp, int M, int N,
                                      int64_t ld_dy, int64_t ld_x, int out_dt, int accumulate, int num_sms, cudaStream_t s) {
   if (G <= 0 || M <= 0 || N <= 0) return 0;
-  if (Tp <= 0 || Tp % BK != 0) return -1;
+  if (Tp <= 0) return -1;
   if ((ld_dy % 8) || (ld_x % 8) || (reinterpret_cast<uintptr_t>(dy) & 15) || (reinterpret_cast<uintptr_t>(x) & 15)) return -11;
   if (M % 8 || N % 8) return -12;
   if (num_sms <= 0) num_sms = rb::kNumSMs;

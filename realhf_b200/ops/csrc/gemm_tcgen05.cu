@@ -23,7 +23,8 @@ template <int BN> struct Cfg {
   static constexpr int kBBytes = BN * BK * 2;
   static constexpr int kStageBytes = kABytes + kBBytes;
   static constexpr int kTmemCols = 2 * BN < 32 ? 32 : 2 * BN;
-  static constexpr int kSmemBytes = kStages * kStageBytes + 1024 /*align*/ + 256 /*barriers*/;
+  static constexpr int kOut = kStages * kStageBytes, kBars = kOut + 4 * 4096;   // 4 KB of output staging per epilogue warp
+  static constexpr int kSmemBytes = kBars + 1024 /*align*/ + 256 /*barriers*/;
 };
 
 // Fused tensor-parallel modes (kMode): 0 plain; 1 GEMM -> reduce-scatter: the epilogue stores every output row straight
@@ -76,7 +77,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tcgen05_kernel(const __grid_
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   uint8_t* smem_a = smem;
   uint8_t* smem_b = smem + C::kStages * C::kABytes;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::kStages * C::kStageBytes);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::kBars);
   uint64_t* full_bar = bars;
   uint64_t* empty_bar = bars + C::kStages;
   uint64_t* tmem_full = bars + 2 * C::kStages;
@@ -177,37 +178,36 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tcgen05_kernel(const __grid_
       }
     }
   } else if (warp == 1) {
-    // ===================================================== MMA issuer
-    if (lane == 0) {
-      constexpr uint32_t idesc = ptx::make_idesc_f16(kFmt, BM, BN, kAMN ? 1 : 0, kBMN ? 1 : 0);
-      int stage = 0;
-      uint32_t phase = 0;
-      int as = 0;
-      uint32_t aphase = 0;
-      for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
-        ptx::mbar_wait(ptx::smem_u32(&tmem_empty[as]), aphase ^ 1);
+    // ===================================================== MMA issuer: the warp runs converged, one elected lane issues
+    constexpr uint32_t idesc = ptx::make_idesc_f16(kFmt, BM, BN, kAMN ? 1 : 0, kBMN ? 1 : 0);
+    constexpr uint32_t kAStep = (kAMN ? 2048 : 32) >> 4, kBStep = (kBMN ? 2048 : 32) >> 4;      // 16 K elements further, in descriptor units
+    const uint32_t tm = (uint32_t)ptx::uniform((int)tmem_base);
+    const int n_tiles = ptx::uniform(num_tiles);
+    int stage = 0;
+    uint32_t phase = 0;
+    int as = 0;
+    uint32_t aphase = 0;
+    for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
+      ptx::mbar_wait(ptx::smem_u32(&tmem_empty[as]), aphase ^ 1);
+      ptx::tc_fence_after();
+      const uint32_t d_tmem = tm + as * BN;
+      for (int kb = 0; kb < num_kb; ++kb) {
+        ptx::mbar_wait(ptx::smem_u32(&full_bar[stage]), phase);
         ptx::tc_fence_after();
-        const uint32_t d_tmem = tmem_base + as * BN;
-        for (int kb = 0; kb < num_kb; ++kb) {
-          ptx::mbar_wait(ptx::smem_u32(&full_bar[stage]), phase);
-          ptx::tc_fence_after();
-          const uint32_t sa = ptx::smem_u32(smem_a + stage * C::kABytes);
-          const uint32_t sb = ptx::smem_u32(smem_b + stage * C::kBBytes);
+        const uint64_t da = ptx::make_smem_desc_sw128(ptx::smem_u32(smem_a + stage * C::kABytes), kAMN ? BK * 128 : 16, 1024);
+        const uint64_t db = ptx::make_smem_desc_sw128(ptx::smem_u32(smem_b + stage * C::kBBytes), kBMN ? BK * 128 : 16, 1024);
+        if (ptx::elect_one()) {
 #pragma unroll
-          for (int k = 0; k < BK / 16; ++k) {
-            const uint64_t adesc = kAMN ? ptx::make_smem_desc_sw128(sa + k * 2048, BK * 128, 1024)
-                                        : ptx::make_smem_desc_sw128(sa + k * 32, 16, 1024);
-            const uint64_t bdesc = kBMN ? ptx::make_smem_desc_sw128(sb + k * 2048, BK * 128, 1024)
-                                        : ptx::make_smem_desc_sw128(sb + k * 32, 16, 1024);
-            ptx::tc_mma_f16(d_tmem, adesc, bdesc, idesc, (kb | k) != 0 ? 1u : 0u);
-          }
+          for (int k = 0; k < BK / 16; ++k) ptx::tc_mma_f16(d_tmem, da + k * kAStep, db + k * kBStep, idesc, (kb | k) != 0 ? 1u : 0u);
           if constexpr (kMC > 1) ptx::tc_commit_mcast(ptx::smem_u32(&empty_bar[stage]), kMcMask);
           else ptx::tc_commit(ptx::smem_u32(&empty_bar[stage]));  // smem slot reusable once these MMAs retire
-          if (++stage == C::kStages) { stage = 0; phase ^= 1; }
         }
-        ptx::tc_commit(ptx::smem_u32(&tmem_full[as]));  // accumulator complete -> epilogue
-        if (++as == 2) { as = 0; aphase ^= 1; }
+        __syncwarp();
+        if (++stage == C::kStages) { stage = 0; phase ^= 1; }
       }
+      if (ptx::elect_one()) ptx::tc_commit(ptx::smem_u32(&tmem_full[as]));  // accumulator complete -> epilogue
+      __syncwarp();
+      if (++as == 2) { as = 0; aphase ^= 1; }
     }
   } else {
     // ===================================================== epilogue (4 warps, TMEM lane quadrant = warp % 4)
@@ -216,6 +216,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tcgen05_kernel(const __grid_
     uint32_t aphase = 0;
     OutT* Cp = reinterpret_cast<OutT*>(p.C);
     const OutT* bias = reinterpret_cast<const OutT*>(p.bias);
+    const uint32_t out_stage = ptx::smem_u32(smem + C::kOut + quad * 4096);
     const bool vec_ok = kMode == 1 ? (p.N % (16 / sizeof(OutT)) == 0)
                                    : ((p.ldc % (16 / sizeof(OutT)) == 0) && ((reinterpret_cast<uintptr_t>(p.C) & 15) == 0));
     for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
@@ -224,7 +225,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tcgen05_kernel(const __grid_
       else tile_coords(tile, tiles_m, tiles_n, BN, m0, n0);
       ptx::mbar_wait(ptx::smem_u32(&tmem_full[as]), aphase);
       ptx::tc_fence_after();
-      const int row = m0 + quad * 32 + lane;
+      const int row0 = m0 + quad * 32, row = row0 + lane;
       const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + as * BN;
 #pragma unroll 1
       for (int c = 0; c < BN / 32; ++c) {
@@ -233,7 +234,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tcgen05_kernel(const __grid_
         ptx::tc_wait_ld();
         const int col = n0 + c * 32;
         const int n_valid = min(32, p.N - col);
-        if (row < m_end && n_valid > 0) {
+        if (kMode == 1 ? row < m_end && n_valid > 0 : row0 < m_end && n_valid > 0) {
           float v[32];
 #pragma unroll
           for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
@@ -241,17 +242,13 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tcgen05_kernel(const __grid_
 #pragma unroll
             for (int i = 0; i < 32; ++i) if (i < n_valid) v[i] += rb::to_f(bias[col + i]);
           }
-          OutT* dst = Cp + (int64_t)row * p.ldc + col;
-          if constexpr (kMode == 1) {
+          if constexpr (kMode == 1) {     // rows of several ranks: every lane stores its own
             const int d = row / fp.rows_per_rank;
-            dst = reinterpret_cast<OutT*>(fp.peer_base[d]) + (int64_t)fp.my_rank * fp.slab_elems +
-                  (int64_t)(row - d * fp.rows_per_rank) * p.N + col;
+            OutT* dst = reinterpret_cast<OutT*>(fp.peer_base[d]) + (int64_t)fp.my_rank * fp.slab_elems + (int64_t)(row - d * fp.rows_per_rank) * p.N + col;
+            store_chunk<OutT>(dst, v, n_valid, vec_ok);
+          } else {
+            store_rows32<OutT>(out_stage, v, Cp + (int64_t)row0 * p.ldc + col, p.ldc, m_end - row0, n_valid, vec_ok, p.accumulate);
           }
-          if (p.accumulate) {
-#pragma unroll
-            for (int i = 0; i < 32; ++i) if (i < n_valid) v[i] += rb::to_f(dst[i]);
-          }
-          store_chunk<OutT>(dst, v, n_valid, vec_ok);
         }
       }
       if constexpr (kMode == 1) {

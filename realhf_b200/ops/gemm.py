@@ -179,18 +179,14 @@ def grouped_wgrad_ref(dy, x, offsets, G):
 
 def grouped_wgrad(dy: torch.Tensor, x: torch.Tensor, offsets: torch.Tensor, G: int, out: Optional[torch.Tensor] = None,
                   accumulate: bool = False) -> torch.Tensor:
-    """dW [G, M, N] for group-sorted dy [T, M], x [T, N] in ONE launch (`csrc/gemm_grouped_wgrad.cu`): both tensors are
-    scattered into zero-padded buffers whose group blocks start at multiples of 64 rows, so that no K block of the kernel
-    straddles two experts.  No host synchronisation."""
-    T = dy.shape[0]
-    dest, off_pad, n_pad = pad_groups(offsets, T)
-    # one spare row at the end swallows the rows that belong to no group (see pad_groups)
-    dy_p = torch.zeros(n_pad + 1, dy.shape[1], dtype=dy.dtype, device=dy.device).index_copy_(0, dest, dy)[:n_pad]
-    x_p = torch.zeros(n_pad + 1, x.shape[1], dtype=x.dtype, device=x.device).index_copy_(0, dest, x)[:n_pad]
+    """dW [G, M, N] for group-sorted dy [T, M], x [T, N] in ONE launch (`csrc/gemm_grouped_wgrad.cu`); group g owns the rows
+    [offsets[g], offsets[g + 1]), rows outside every group are not touched.  No host synchronisation."""
     if out is None:
         out = torch.empty(G, dy.shape[1], x.shape[1], dtype=dy.dtype, device=dy.device)
         accumulate = False
-    lib().gemm_grouped_wgrad(dy_p, x_p, out, off_pad, accumulate, _sms(dy.device))
+    if dy.shape[0] == 0:
+        return out if accumulate else out.zero_()
+    lib().gemm_grouped_wgrad(tma_rows(dy), tma_rows(x), out, offsets.int().contiguous(), accumulate, _sms(dy.device))
     return out
 
 

@@ -250,3 +250,48 @@ def test_gated_linear_fused_epilogue_matches_reference(shape, kind):
     with torch.no_grad():
         a2 = OF.gated_linear(x.detach(), w.detach(), kind)
     torch.testing.assert_close(a2, a.detach())
+
+
+def test_grouped_wgrad_tail_rows_of_other_groups():
+    """K blocks that reach into the next group's rows, past the last group and past the tensor, with NaN in one group and in the rows of no group: a
+    group's gradient is that of its own rows.  Products of 16-bit numbers are exact in fp32; 2^-8 for the rounded result, 2^-20 of the summed magnitudes."""
+    from realhf_b200.ops import gemm as G
+    torch.manual_seed(1)
+    counts, lead, M, N = [1, 63, 64, 65, 127, 0, 5, 130, 64], 7, 264, 136
+    off = torch.tensor([lead] + [lead + int(c) for c in torch.tensor(counts).cumsum(0)], dtype=torch.int32, device="cuda")
+    T = int(off[-1]) + 3
+    dy, x = torch.randn(T, M, device="cuda").to(torch.bfloat16), torch.randn(T, N, device="cuda").to(torch.bfloat16)
+    dy[:lead], x[int(off[-1]):] = float("nan"), float("nan")
+    dy[int(off[3]): int(off[4])] = float("nan")
+    for acc in (False, True):
+        out = torch.ones(len(counts), M, N, device="cuda", dtype=torch.bfloat16 if acc else torch.float32)
+        G.grouped_wgrad(dy, x, off, len(counts), out=out, accumulate=acc)
+        for g in range(len(counts)):
+            if g == 3:
+                assert out[g].isnan().all()
+                continue
+            a, b = dy[int(off[g]): int(off[g + 1])].double(), x[int(off[g]): int(off[g + 1])].double()
+            ref, mag = a.T @ b + float(acc), a.abs().T @ b.abs() + float(acc)
+            assert ((out[g].double() - ref).abs() <= (2.0 ** -8 if acc else 0.0) * ref.abs() + 2.0 ** -20 * mag + 1e-6).all(), g
+    assert torch.equal(G.grouped_wgrad(dy[:0], x[:0], torch.zeros(3, dtype=torch.int32, device="cuda"), 2), torch.zeros(2, M, N, device="cuda", dtype=torch.bfloat16))
+
+
+@pytest.mark.parametrize("out_dt", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("M,N,K,shift", [(129, 136, 64, 0), (300, 520, 192, 0), (257, 264, 128, 1), (8, 72, 200, 0), (640, 40, 72, 3)])
+def test_gemm_accumulates_into_ragged_outputs(out_dt, M, N, K, shift):
+    """C += A B through the staged epilogue: ragged rows and columns, an output that starts off every vector boundary, untouched surroundings.  Bound: one
+    rounding of the result and 2^-20 of the summed magnitudes."""
+    from realhf_b200.ops import gemm as G
+    torch.manual_seed(M + N)
+    a, b = torch.randn(K, M, device="cuda").to(torch.bfloat16), torch.randn(K, N, device="cuda").to(torch.bfloat16)
+    if M % 8 or N % 8:
+        a = torch.randn(K, (M + 7) // 8 * 8, device="cuda").to(torch.bfloat16)[:, :M]
+    buf = torch.randn(M + 2, N + 8, device="cuda").to(out_dt)
+    before = buf.clone()
+    out = buf[1:M + 1, shift:shift + N]
+    G.gemm(a, b, out=out, a_mn=True, b_mn=True, accumulate=True)
+    ref = before[1:M + 1, shift:shift + N].double() + a.double().T @ b.double()
+    mag = before[1:M + 1, shift:shift + N].double().abs() + a.double().abs().T @ b.double().abs()
+    assert ((out.double() - ref).abs() <= (2.0 ** -8 if out_dt == torch.bfloat16 else 0.0) * ref.abs() + 2.0 ** -20 * mag).all()
+    buf[1:M + 1, shift:shift + N] = before[1:M + 1, shift:shift + N]
+    assert torch.equal(buf, before)
