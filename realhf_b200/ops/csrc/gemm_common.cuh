@@ -70,14 +70,22 @@ template <typename T> RB_DEVICE void store_chunk(T* dst, const float* v, int n_v
 // fp32, four lines per instruction leave whole, and the old values of an accumulating GEMM come in the same way; the sum is formed in fp32.
 // dst: first row and column; rows / cols: how many are real.
 template <typename T> RB_DEVICE void store_rows32(uint32_t stage, const float (&v)[32], T* dst, int64_t ldc, int rows, int cols, bool vec_ok, bool accumulate) {
-  const int lane = threadIdx.x & 31;
+  const int lane = threadIdx.x & 31, q = lane & 7, c = q * 4;
+  rb::Pack<T, 4> old[8];
+  const bool fetch = accumulate && vec_ok && c + 4 <= cols;
+  if (fetch) {                       // all eight in flight while the new values are staged
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int r = i * 4 + (lane >> 3);
+      if (r < rows) old[i] = *reinterpret_cast<const rb::Pack<T, 4>*>(dst + (int64_t)r * ldc + c);
+    }
+  }
 #pragma unroll
   for (int q = 0; q < 8; ++q)
     asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(stage + lane * 128 + ((q ^ (lane & 7)) << 4)), "f"(v[4 * q]), "f"(v[4 * q + 1]), "f"(v[4 * q + 2]),
                  "f"(v[4 * q + 3])
                  : "memory");
   __syncwarp();
-  const int q = lane & 7, c = q * 4;
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     const int r = i * 4 + (lane >> 3);
@@ -87,10 +95,9 @@ template <typename T> RB_DEVICE void store_rows32(uint32_t stage, const float (&
       T* d = dst + (int64_t)r * ldc + c;
       if (vec_ok && c + 4 <= cols) {
         rb::Pack<T, 4> o;
-        if (accumulate) {
-          const rb::Pack<T, 4> old = *reinterpret_cast<const rb::Pack<T, 4>*>(d);
+        if (fetch) {
 #pragma unroll
-          for (int k = 0; k < 4; ++k) x[k] += rb::to_f(old.v[k]);
+          for (int k = 0; k < 4; ++k) x[k] += rb::to_f(old[i].v[k]);
         }
 #pragma unroll
         for (int k = 0; k < 4; ++k) o.v[k] = rb::from_f<T>(x[k]);

@@ -5,14 +5,16 @@
 // Reference: grouped_gemm's `gmm(..., trans_a=True)` in the experts' backward (impl/model/modules/moe/experts.py); the first
 // version here ran one GEMM per expert after a host read of the token counts.  This kernel is the wgrad form of the tile GEMM
 // (`gemm_tcgen05.cu`: both operands MN-major, K = tokens) with the K range taken per tile from the device-side offsets:
-// tile -> (expert, m-tile, n-tile), persistent CTAs, TMA producer warp / converged tcgen05.mma issuer / four epilogue warps, smem ring + double-buffered
-// TMEM accumulators.  The last 64-row K block of an expert may reach into the next one's rows: a warp of its own zeroes
-// those rows of both staged operands before the MMAs read them.  (Scattering both operands into buffers padded to 64 rows per expert took
+// tile -> (expert, m-tile, n-tile), persistent CTA pairs (cta_group::2, a 256 x BN tile per pair, see gemm_2cta.cu), TMA producer warp / converged
+// tcgen05.mma issuer / four epilogue warps per CTA, smem ring + double-buffered TMEM accumulators.  The last 64-row K block of an expert may reach into
+// the next one's rows: its tiles land on the CTA's own barrier, a warp zeroes the foreign rows of the CTA's share of both operands, and the MMAs
+// wait for both CTAs' word instead of the ring's.  (Scattering both operands into buffers padded to 64 rows per expert took
 // 720 us of an 8 x 14336 x 4096 feed-forward's backward on 4096 rows.)  An expert without tokens gets zeros (or is left alone when accumulating).
 //
-// What bounds it: with a few hundred tokens per expert a tile is 4096 tensor-pipe cycles and 64 KB of output, so the epilogue has to
-// leave in whole lines (store_rows32): rows stored lane by lane took as long as the products (2281 us for the two of that backward).
-#include "gemm_common.cuh"
+// What bounds it: with a few hundred tokens per expert a tile is 4096 tensor-pipe cycles and 64 KB of output per SM, so the output has to leave in
+// whole lines (store_rows32; rows stored lane by lane: 2281 us for the two products of that backward, 1905 us after), and a tile of one SM asks L2 for
+// 96 B per cycle and SM; a pair's for 64.
+#include "cta_pair.cuh"
 
 namespace {
 
@@ -23,42 +25,46 @@ struct WgradParams {
   int accumulate;
 };
 
-constexpr int kWgradThreads = 224;   // warp 6: tail rows
+constexpr int kWgradThreads = 224;   // warps 0 TMA, 1 MMA (leader), 2-5 epilogue, 6 tail rows
 
 template <int BN> struct WCfg {
-  static constexpr int kStages = BN >= 256 ? 4 : 6;
-  static constexpr int kABytes = BM * BK * 2;   // [2 chunks of 64 m][64 k rows][128 B]
-  static constexpr int kBBytes = BN * BK * 2;   // [BN/64 chunks][64 k rows][128 B]
+  static constexpr int kStages = BN >= 256 ? 6 : 8;
+  static constexpr int kABytes = BM * BK * 2;         // [2 chunks of 64 m][64 k rows][128 B]
+  static constexpr int kBBytes = BN / 2 * BK * 2;     // [BN / 128 chunks][64 k rows][128 B]: this CTA's half of the columns
   static constexpr int kStageBytes = kABytes + kBBytes;
   static constexpr int kOut = kStages * kStageBytes, kBars = kOut + 4 * 4096;   // 4 KB of output staging per epilogue warp
-  static constexpr int kSmemBytes = kBars + 1024 + 256;
+  static constexpr int kSmemBytes = kBars + 1024 + 512;
 };
 
 template <int BN, typename OutT>
 __global__ void __launch_bounds__(kWgradThreads, 1) grouped_wgrad_kernel(const __grid_constant__ CUtensorMap tma_a,
-                                                                    const __grid_constant__ CUtensorMap tma_b, WgradParams p) {
+                                                                         const __grid_constant__ CUtensorMap tma_b, WgradParams p) {
   using C = WCfg<BN>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   uint8_t* smem_a = smem;
   uint8_t* smem_b = smem + C::kStages * C::kABytes;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::kBars);
-  uint64_t* full_bar = bars;
-  uint64_t* empty_bar = bars + C::kStages;
-  uint64_t* tail_bar = bars + 2 * C::kStages;     // a stage whose rows behind the expert's last one have been zeroed
-  uint64_t* tmem_full = bars + 3 * C::kStages;
-  uint64_t* tmem_empty = tmem_full + 2;
+  uint64_t* full_bar = bars;                       // leader: both CTAs' bytes of an ordinary stage
+  uint64_t* empty_bar = bars + C::kStages;         // one per CTA, armed by the leader's multicast commit
+  uint64_t* mine_bar = bars + 2 * C::kStages;      // one per CTA: its own bytes of an expert's last, partial stage
+  uint64_t* tail_bar = bars + 3 * C::kStages;      // leader: both CTAs' foreign rows of such a stage are zero
+  uint64_t* tmem_full = bars + 4 * C::kStages;     // one per CTA
+  uint64_t* tmem_empty = tmem_full + 2;            // leader, 8 arrivals
   uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(tmem_empty + 2);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int tiles_m = RB_CEIL_DIV(p.M, BM), tiles_n = RB_CEIL_DIV(p.N, BN);
+  const uint32_t rank = cluster_ctarank();
+  const bool leader = rank == 0;
+  const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
+  const int tiles_m = RB_CEIL_DIV(p.M, 2 * BM), tiles_n = RB_CEIL_DIV(p.N, BN);
   const int tpg = tiles_m * tiles_n;
   const int num_tiles = p.G * tpg;
   // tile -> (expert, m0, n0, first token row, number of 64-row K blocks, real rows of the last one); m fastest so neighbouring CTAs share the X panel
   auto coords = [&](int tile, int& g, int& m0, int& n0, int& r0, int& nkb, int& tail) {
     g = tile / tpg;
     const int local = tile - g * tpg;
-    m0 = (local % tiles_m) * BM;
+    m0 = (local % tiles_m) * (2 * BM);
     n0 = (local / tiles_m) * BN;
     r0 = p.off[g];
     const int rows = p.off[g + 1] - r0;
@@ -71,21 +77,23 @@ __global__ void __launch_bounds__(kWgradThreads, 1) grouped_wgrad_kernel(const _
     ptx::prefetch_tensormap(&tma_b);
     for (int i = 0; i < C::kStages; ++i) {
       ptx::mbar_init(ptx::smem_u32(&full_bar[i]), 1);
-      ptx::mbar_init(ptx::smem_u32(&empty_bar[i]), 2);      // the MMAs' commit and the tail warp
-      ptx::mbar_init(ptx::smem_u32(&tail_bar[i]), 1);
+      ptx::mbar_init(ptx::smem_u32(&empty_bar[i]), 1);
+      ptx::mbar_init(ptx::smem_u32(&mine_bar[i]), 1);
+      ptx::mbar_init(ptx::smem_u32(&tail_bar[i]), 2);
     }
     for (int i = 0; i < 2; ++i) {
       ptx::mbar_init(ptx::smem_u32(&tmem_full[i]), 1);
-      ptx::mbar_init(ptx::smem_u32(&tmem_empty[i]), 4);
+      ptx::mbar_init(ptx::smem_u32(&tmem_empty[i]), 8);
     }
     ptx::fence_barrier_init();
   }
   if (warp == 1) {
-    ptx::tmem_alloc(ptx::smem_u32(tmem_ptr), 2 * BN);
-    ptx::tmem_relinquish();
+    tmem_alloc_cg2(ptx::smem_u32(tmem_ptr), 2 * BN);
+    tmem_relinquish_cg2();
   }
   ptx::tc_fence_before();
   __syncthreads();
+  ptx::cluster_sync();  // the peer's barriers must exist before any remote arrive / multicast commit / cross-CTA TMA completion
   ptx::tc_fence_after();
   const uint32_t tmem_base = *tmem_ptr;
 
@@ -93,82 +101,93 @@ __global__ void __launch_bounds__(kWgradThreads, 1) grouped_wgrad_kernel(const _
     if (lane == 0) {
       int stage = 0;
       uint32_t phase = 0;
-      for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
+      for (int tile = pair; tile < num_tiles; tile += num_pairs) {
         int g, m0, n0, r0, nkb, tail;
         coords(tile, g, m0, n0, r0, nkb, tail);
         for (int kb = 0; kb < nkb; ++kb) {
           ptx::mbar_wait(ptx::smem_u32(&empty_bar[stage]), phase ^ 1);
-          const uint32_t fb = ptx::smem_u32(&full_bar[stage]);
-          ptx::mbar_arrive_expect_tx(fb, C::kStageBytes);
           const uint32_t sa = ptx::smem_u32(smem_a + stage * C::kABytes);
           const uint32_t sb = ptx::smem_u32(smem_b + stage * C::kBBytes);
-          const int k0 = r0 + kb * BK;
+          const int k0 = r0 + kb * BK, ma = m0 + (int)rank * BM, nb = n0 + (int)rank * (BN / 2);
+          if (kb == nkb - 1 && tail < BK) {
+            const uint32_t fb = ptx::smem_u32(&mine_bar[stage]);
+            ptx::mbar_arrive_expect_tx(fb, C::kStageBytes);
 #pragma unroll
-          for (int j = 0; j < BM / 64; ++j) ptx::tma_load_2d(sa + j * (BK * 128), &tma_a, fb, m0 + 64 * j, k0);
+            for (int j = 0; j < BM / 64; ++j) ptx::tma_load_2d(sa + j * (BK * 128), &tma_a, fb, ma + 64 * j, k0);
 #pragma unroll
-          for (int j = 0; j < BN / 64; ++j) ptx::tma_load_2d(sb + j * (BK * 128), &tma_b, fb, n0 + 64 * j, k0);
+            for (int j = 0; j < BN / 128; ++j) ptx::tma_load_2d(sb + j * (BK * 128), &tma_b, fb, nb + 64 * j, k0);
+          } else {
+            const uint32_t fb_local = ptx::smem_u32(&full_bar[stage]);
+            if (leader) ptx::mbar_arrive_expect_tx(fb_local, 2 * C::kStageBytes);  // both CTAs' bytes land on this barrier
+            const uint32_t fb = mapa_u32(fb_local, 0);
+#pragma unroll
+            for (int j = 0; j < BM / 64; ++j) tma_load_2d_cg2(sa + j * (BK * 128), &tma_a, fb, ma + 64 * j, k0);
+#pragma unroll
+            for (int j = 0; j < BN / 128; ++j) tma_load_2d_cg2(sb + j * (BK * 128), &tma_b, fb, nb + 64 * j, k0);
+          }
           if (++stage == C::kStages) { stage = 0; phase ^= 1; }
         }
       }
     }
   } else if (warp == 1) {
-    constexpr uint32_t idesc = ptx::make_idesc_f16(1, BM, BN, 1, 1);
-    const uint32_t tm = (uint32_t)ptx::uniform((int)tmem_base);
-    int stage = 0, as = 0;
-    uint32_t phase = 0, aphase = 0, tails = 0;     // tails: bit s = phase of tail_bar[s]
-    for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
-      int g, m0, n0, r0, nkb, tail;
-      coords(tile, g, m0, n0, r0, nkb, tail);
-      nkb = ptx::uniform(nkb);
-      tail = ptx::uniform(tail);
-      ptx::mbar_wait(ptx::smem_u32(&tmem_empty[as]), aphase ^ 1);
-      ptx::tc_fence_after();
-      const uint32_t d_tmem = tm + as * BN;
-      for (int kb = 0; kb < nkb; ++kb) {
-        if (kb == nkb - 1 && tail < BK) {
-          ptx::mbar_wait(ptx::smem_u32(&tail_bar[stage]), (tails >> stage) & 1u);
-          tails ^= 1u << stage;
-        } else {
-          ptx::mbar_wait(ptx::smem_u32(&full_bar[stage]), phase);
-        }
+    if (leader) {
+      constexpr uint32_t idesc = ptx::make_idesc_f16(1, 2 * BM, BN, 1, 1);
+      const uint32_t tm = (uint32_t)ptx::uniform((int)tmem_base);
+      int stage = 0, as = 0;
+      uint32_t aphase = 0, fulls = 0, tails = 0;     // bit s: phase of full_bar[s] / tail_bar[s] (a stage fills by one of the two)
+      for (int tile = pair; tile < num_tiles; tile += num_pairs) {
+        int g, m0, n0, r0, nkb, tail;
+        coords(tile, g, m0, n0, r0, nkb, tail);
+        nkb = ptx::uniform(nkb);
+        tail = ptx::uniform(tail);
+        ptx::mbar_wait(ptx::smem_u32(&tmem_empty[as]), aphase ^ 1);
         ptx::tc_fence_after();
-        const uint64_t da = ptx::make_smem_desc_sw128(ptx::smem_u32(smem_a + stage * C::kABytes), BK * 128, 1024);
-        const uint64_t db = ptx::make_smem_desc_sw128(ptx::smem_u32(smem_b + stage * C::kBBytes), BK * 128, 1024);
-        if (ptx::elect_one()) {
+        const uint32_t d_tmem = tm + as * BN;
+        for (int kb = 0; kb < nkb; ++kb) {
+          if (kb == nkb - 1 && tail < BK) {
+            mbar_wait_cluster(ptx::smem_u32(&tail_bar[stage]), (tails >> stage) & 1u);
+            tails ^= 1u << stage;
+          } else {
+            ptx::mbar_wait(ptx::smem_u32(&full_bar[stage]), (fulls >> stage) & 1u);
+            fulls ^= 1u << stage;
+          }
+          ptx::tc_fence_after();
+          const uint64_t da = ptx::make_smem_desc_sw128(ptx::smem_u32(smem_a + stage * C::kABytes), BK * 128, 1024);
+          const uint64_t db = ptx::make_smem_desc_sw128(ptx::smem_u32(smem_b + stage * C::kBBytes), BK * 128, 1024);
+          if (ptx::elect_one()) {
 #pragma unroll
-          for (int k = 0; k < BK / 16; ++k) ptx::tc_mma_f16(d_tmem, da + k * 128, db + k * 128, idesc, (kb | k) != 0 ? 1u : 0u);
-          ptx::tc_commit(ptx::smem_u32(&empty_bar[stage]));
+            for (int k = 0; k < BK / 16; ++k) tc_mma_f16_cg2(d_tmem, da + k * 128, db + k * 128, idesc, (kb | k) != 0 ? 1u : 0u);
+            tc_commit_cg2(ptx::smem_u32(&empty_bar[stage]), 0b11);
+          }
+          __syncwarp();
+          if (++stage == C::kStages) stage = 0;
         }
+        if (ptx::elect_one()) tc_commit_cg2(ptx::smem_u32(&tmem_full[as]), 0b11);  // with nkb == 0 nothing is pending: arrives at once
         __syncwarp();
-        if (++stage == C::kStages) { stage = 0; phase ^= 1; }
+        if (++as == 2) { as = 0; aphase ^= 1; }
       }
-      if (ptx::elect_one()) ptx::tc_commit(ptx::smem_u32(&tmem_full[as]));  // with nkb == 0 nothing is pending: arrives at once
-      __syncwarp();
-      if (++as == 2) { as = 0; aphase ^= 1; }
     }
   } else if (warp == 6) {
-    // ===================================================== rows of the next expert (or of nobody) in an expert's last K block: zero in both operands.  The
-    // warp follows every stage (and releases it too), so that it is never a turn of the ring ahead or behind.
+    // ===================================================== rows of the next expert (or of nobody) in an expert's last K block: zero in this CTA's share
     int stage = 0;
-    uint32_t phase = 0;
-    for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
+    uint32_t phases = 0;      // bit s: phase of mine_bar[s], which only such stages use
+    for (int tile = pair; tile < num_tiles; tile += num_pairs) {
       int g, m0, n0, r0, nkb, tail;
       coords(tile, g, m0, n0, r0, nkb, tail);
-      for (int kb = 0; kb < nkb; ++kb) {
-        ptx::mbar_wait(ptx::smem_u32(&full_bar[stage]), phase);
-        if (kb == nkb - 1 && tail < BK) {
-          // chunks of 64 columns: [64 token rows][128 B], rows unswizzled among themselves
-          for (int c = 0; c < (BM + BN) / 64; ++c) {
-            uint8_t* base = c < BM / 64 ? smem_a + stage * C::kABytes + c * (BK * 128) : smem_b + stage * C::kBBytes + (c - BM / 64) * (BK * 128);
-            for (int i = tail * 8 + lane; i < BK * 8; i += 32) reinterpret_cast<uint4*>(base)[i] = make_uint4(0u, 0u, 0u, 0u);
-          }
-          ptx::fence_proxy_async();
-          __syncwarp();
-          if (lane == 0) ptx::mbar_arrive(ptx::smem_u32(&tail_bar[stage]));
+      if (nkb > 0 && tail < BK) {
+        const int st = (stage + nkb - 1) % C::kStages;
+        ptx::mbar_wait(ptx::smem_u32(&mine_bar[st]), (phases >> st) & 1u);
+        phases ^= 1u << st;
+        // chunks of 64 columns: [64 token rows][128 B], rows unswizzled among themselves
+        for (int c = 0; c < BM / 64 + BN / 128; ++c) {
+          uint8_t* base = c < BM / 64 ? smem_a + st * C::kABytes + c * (BK * 128) : smem_b + st * C::kBBytes + (c - BM / 64) * (BK * 128);
+          for (int i = tail * 8 + lane; i < BK * 8; i += 32) reinterpret_cast<uint4*>(base)[i] = make_uint4(0u, 0u, 0u, 0u);
         }
-        if (lane == 0) ptx::mbar_arrive(ptx::smem_u32(&empty_bar[stage]));
-        if (++stage == C::kStages) { stage = 0; phase ^= 1; }
+        asm volatile("fence.proxy.async;" ::: "memory");      // (the leader's MMAs read both CTAs' shared memory)
+        __syncwarp();
+        if (lane == 0) mbar_arrive_remote(ptx::smem_u32(&tail_bar[st]), 0);
       }
+      stage = (stage + nkb) % C::kStages;
     }
   } else {
     const int quad = warp & 3;
@@ -177,12 +196,12 @@ __global__ void __launch_bounds__(kWgradThreads, 1) grouped_wgrad_kernel(const _
     OutT* Cp = reinterpret_cast<OutT*>(p.C);
     const uint32_t out_stage = ptx::smem_u32(smem + C::kOut + quad * 4096);
     const bool vec_ok = (p.N % (16 / sizeof(OutT)) == 0) && ((reinterpret_cast<uintptr_t>(p.C) & 15) == 0);
-    for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
+    for (int tile = pair; tile < num_tiles; tile += num_pairs) {
       int g, m0, n0, r0, nkb, tail;
       coords(tile, g, m0, n0, r0, nkb, tail);
       ptx::mbar_wait(ptx::smem_u32(&tmem_full[as]), aphase);
       ptx::tc_fence_after();
-      const int row0 = m0 + quad * 32;
+      const int row0 = m0 + (int)rank * BM + quad * 32;
       const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + as * BN;
 #pragma unroll 1
       for (int c = 0; c < BN / 32; ++c) {
@@ -191,7 +210,7 @@ __global__ void __launch_bounds__(kWgradThreads, 1) grouped_wgrad_kernel(const _
         ptx::tc_wait_ld();
         const int col = n0 + c * 32;
         const int n_valid = min(32, p.N - col);
-        if (n_valid > 0 && !(nkb == 0 && p.accumulate)) {
+        if (row0 < p.M && n_valid > 0 && !(nkb == 0 && p.accumulate)) {
           float v[32];
 #pragma unroll
           for (int i = 0; i < 32; ++i) v[i] = nkb == 0 ? 0.f : __uint_as_float(r[i]);  // no tokens: the accumulator is stale
@@ -200,16 +219,17 @@ __global__ void __launch_bounds__(kWgradThreads, 1) grouped_wgrad_kernel(const _
       }
       ptx::tc_fence_before();
       __syncwarp();
-      if (lane == 0) ptx::mbar_arrive(ptx::smem_u32(&tmem_empty[as]));
+      if (lane == 0) mbar_arrive_remote(ptx::smem_u32(&tmem_empty[as]), 0);
       if (++as == 2) { as = 0; aphase ^= 1; }
     }
   }
 
   ptx::tc_fence_before();
   __syncthreads();
+  ptx::cluster_sync();  // neither CTA may free TMEM or exit while the pair's MMAs / remote arrivals are in flight
   if (warp == 1) {
     ptx::tc_fence_after();
-    ptx::tmem_dealloc(tmem_base, 2 * BN);
+    tmem_dealloc_cg2(tmem_base, 2 * BN);
   }
 }
 
@@ -222,9 +242,20 @@ int launch_wgrad(const CUtensorMap& ta, const CUtensorMap& tb, const WgradParams
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes) != cudaSuccess) return -30;
     attr_set = true;
   }
-  const int64_t tiles = (int64_t)p.G * RB_CEIL_DIV(p.M, BM) * RB_CEIL_DIV(p.N, BN);
-  const int grid = (int)(tiles < num_sms ? tiles : num_sms);
-  kern<<<grid, kWgradThreads, C::kSmemBytes, s>>>(ta, tb, p);
+  const int64_t tiles = (int64_t)p.G * RB_CEIL_DIV(p.M, 2 * BM) * RB_CEIL_DIV(p.N, BN);
+  const int pairs = num_sms / 2;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)(2 * (tiles < pairs ? tiles : pairs)));
+  cfg.blockDim = dim3(kWgradThreads);
+  cfg.dynamicSmemBytes = C::kSmemBytes;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  if (cudaLaunchKernelEx(&cfg, kern, ta, tb, p) != cudaSuccess) return -31;
   return cudaGetLastError() == cudaSuccess ? 0 : -31;
 }
 
