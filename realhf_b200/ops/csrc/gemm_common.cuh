@@ -110,6 +110,30 @@ template <typename T> RB_DEVICE void store_rows32(uint32_t stage, const float (&
   __syncwarp();
 }
 
+// The same for 64 columns of 16-bit results that are all real, aligned and not added to anything: staged in their own type, eight 16-byte loads and
+// stores a lane.
+template <typename T> RB_DEVICE void store_rows64(uint32_t stage, const uint32_t (&acc)[64], T* dst, int64_t ldc) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    rb::Pack<T, 8> o;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) o.v[e] = rb::from_f<T>(__uint_as_float(acc[q * 8 + e]));
+    const uint4 w = *reinterpret_cast<const uint4*>(&o);
+    asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(stage + lane * 128 + ((q ^ (lane & 7)) << 4)), "r"(w.x), "r"(w.y), "r"(w.z), "r"(w.w) : "memory");
+  }
+  __syncwarp();
+  uint4 y[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int r = i * 4 + (lane >> 3);
+    asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(y[i].x), "=r"(y[i].y), "=r"(y[i].z), "=r"(y[i].w) : "r"(stage + r * 128 + (((lane & 7) ^ (r & 7)) << 4)) : "memory");
+  }
+#pragma unroll
+  for (int i = 0; i < 8; ++i) *reinterpret_cast<uint4*>(dst + (int64_t)(i * 4 + (lane >> 3)) * ldc + (lane & 7) * 8) = y[i];
+  __syncwarp();
+}
+
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                   const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);

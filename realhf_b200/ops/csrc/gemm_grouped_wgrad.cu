@@ -6,14 +6,15 @@
 // version here ran one GEMM per expert after a host read of the token counts.  This kernel is the wgrad form of the tile GEMM
 // (`gemm_tcgen05.cu`: both operands MN-major, K = tokens) with the K range taken per tile from the device-side offsets:
 // tile -> (expert, m-tile, n-tile), persistent CTA pairs (cta_group::2, a 256 x BN tile per pair, see gemm_2cta.cu), TMA producer warp / converged
-// tcgen05.mma issuer / four epilogue warps per CTA, smem ring + double-buffered TMEM accumulators.  The last 64-row K block of an expert may reach into
+// tcgen05.mma issuer / eight epilogue warps per CTA, smem ring + double-buffered TMEM accumulators.  The last 64-row K block of an expert may reach into
 // the next one's rows: its tiles land on the CTA's own barrier, a warp zeroes the foreign rows of the CTA's share of both operands, and the MMAs
 // wait for both CTAs' word instead of the ring's.  (Scattering both operands into buffers padded to 64 rows per expert took
 // 720 us of an 8 x 14336 x 4096 feed-forward's backward on 4096 rows.)  An expert without tokens gets zeros (or is left alone when accumulating).
 //
 // What bounds it: with a few hundred tokens per expert a tile is 4096 tensor-pipe cycles and 64 KB of output per SM, so the output has to leave in
-// whole lines (store_rows32; rows stored lane by lane: 2281 us for the two products of that backward, 1905 us after), and a tile of one SM asks L2 for
-// 96 B per cycle and SM; a pair's for 64.
+// whole lines and as fast as the next tile's MMAs, and a tile of one SM asks L2 for 96 B per cycle and SM; a pair's for 64.  The two products of that
+// backward on 8 x 512 rows: rows stored lane by lane 2281 us, whole lines (store_rows32, four warps) 1905, CTA pairs 1770, eight epilogue warps and 16-bit
+// staging (store_rows64) 1480 (1.3 PFLOP/s); row counts that are no multiple of 64 cost 1010 us instead of 840 on the larger one.
 #include "cta_pair.cuh"
 
 namespace {
@@ -25,14 +26,15 @@ struct WgradParams {
   int accumulate;
 };
 
-constexpr int kWgradThreads = 224;   // warps 0 TMA, 1 MMA (leader), 2-5 epilogue, 6 tail rows
+constexpr int kEpiWarps = 8;         // two per TMEM quadrant, half of the columns each
+constexpr int kWgradThreads = 32 * (3 + kEpiWarps);   // warps 0 TMA, 1 MMA (leader), 2-9 epilogue, 10 tail rows
 
 template <int BN> struct WCfg {
   static constexpr int kStages = BN >= 256 ? 6 : 8;
   static constexpr int kABytes = BM * BK * 2;         // [2 chunks of 64 m][64 k rows][128 B]
   static constexpr int kBBytes = BN / 2 * BK * 2;     // [BN / 128 chunks][64 k rows][128 B]: this CTA's half of the columns
   static constexpr int kStageBytes = kABytes + kBBytes;
-  static constexpr int kOut = kStages * kStageBytes, kBars = kOut + 4 * 4096;   // 4 KB of output staging per epilogue warp
+  static constexpr int kOut = kStages * kStageBytes, kBars = kOut + kEpiWarps * 4096;   // 4 KB of output staging per epilogue warp
   static constexpr int kSmemBytes = kBars + 1024 + 512;
 };
 
@@ -50,7 +52,7 @@ __global__ void __launch_bounds__(kWgradThreads, 1) grouped_wgrad_kernel(const _
   uint64_t* mine_bar = bars + 2 * C::kStages;      // one per CTA: its own bytes of an expert's last, partial stage
   uint64_t* tail_bar = bars + 3 * C::kStages;      // leader: both CTAs' foreign rows of such a stage are zero
   uint64_t* tmem_full = bars + 4 * C::kStages;     // one per CTA
-  uint64_t* tmem_empty = tmem_full + 2;            // leader, 8 arrivals
+  uint64_t* tmem_empty = tmem_full + 2;            // leader, one arrival per epilogue warp of both CTAs
   uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(tmem_empty + 2);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -71,6 +73,8 @@ __global__ void __launch_bounds__(kWgradThreads, 1) grouped_wgrad_kernel(const _
     nkb = RB_CEIL_DIV(rows, BK);
     tail = rows - (nkb - 1) * BK;
   };
+  // A partial block is the first of its tile: it is loaded and cleaned while the MMAs are on the previous tile.
+  auto block = [](int kb, int nkb, int tail) { return tail == BK ? kb : kb == 0 ? nkb - 1 : kb - 1; };
 
   if (warp == 0 && lane == 0) {
     ptx::prefetch_tensormap(&tma_a);
@@ -83,7 +87,7 @@ __global__ void __launch_bounds__(kWgradThreads, 1) grouped_wgrad_kernel(const _
     }
     for (int i = 0; i < 2; ++i) {
       ptx::mbar_init(ptx::smem_u32(&tmem_full[i]), 1);
-      ptx::mbar_init(ptx::smem_u32(&tmem_empty[i]), 8);
+      ptx::mbar_init(ptx::smem_u32(&tmem_empty[i]), 2 * kEpiWarps);
     }
     ptx::fence_barrier_init();
   }
@@ -108,8 +112,8 @@ __global__ void __launch_bounds__(kWgradThreads, 1) grouped_wgrad_kernel(const _
           ptx::mbar_wait(ptx::smem_u32(&empty_bar[stage]), phase ^ 1);
           const uint32_t sa = ptx::smem_u32(smem_a + stage * C::kABytes);
           const uint32_t sb = ptx::smem_u32(smem_b + stage * C::kBBytes);
-          const int k0 = r0 + kb * BK, ma = m0 + (int)rank * BM, nb = n0 + (int)rank * (BN / 2);
-          if (kb == nkb - 1 && tail < BK) {
+          const int k0 = r0 + block(kb, nkb, tail) * BK, ma = m0 + (int)rank * BM, nb = n0 + (int)rank * (BN / 2);
+          if (kb == 0 && tail < BK) {
             const uint32_t fb = ptx::smem_u32(&mine_bar[stage]);
             ptx::mbar_arrive_expect_tx(fb, C::kStageBytes);
 #pragma unroll
@@ -144,7 +148,7 @@ __global__ void __launch_bounds__(kWgradThreads, 1) grouped_wgrad_kernel(const _
         ptx::tc_fence_after();
         const uint32_t d_tmem = tm + as * BN;
         for (int kb = 0; kb < nkb; ++kb) {
-          if (kb == nkb - 1 && tail < BK) {
+          if (kb == 0 && tail < BK) {
             mbar_wait_cluster(ptx::smem_u32(&tail_bar[stage]), (tails >> stage) & 1u);
             tails ^= 1u << stage;
           } else {
@@ -167,7 +171,7 @@ __global__ void __launch_bounds__(kWgradThreads, 1) grouped_wgrad_kernel(const _
         if (++as == 2) { as = 0; aphase ^= 1; }
       }
     }
-  } else if (warp == 6) {
+  } else if (warp == 2 + kEpiWarps) {
     // ===================================================== rows of the next expert (or of nobody) in an expert's last K block: zero in this CTA's share
     int stage = 0;
     uint32_t phases = 0;      // bit s: phase of mine_bar[s], which only such stages use
@@ -175,7 +179,7 @@ __global__ void __launch_bounds__(kWgradThreads, 1) grouped_wgrad_kernel(const _
       int g, m0, n0, r0, nkb, tail;
       coords(tile, g, m0, n0, r0, nkb, tail);
       if (nkb > 0 && tail < BK) {
-        const int st = (stage + nkb - 1) % C::kStages;
+        const int st = stage;
         ptx::mbar_wait(ptx::smem_u32(&mine_bar[st]), (phases >> st) & 1u);
         phases ^= 1u << st;
         // chunks of 64 columns: [64 token rows][128 B], rows unswizzled among themselves
@@ -190,11 +194,11 @@ __global__ void __launch_bounds__(kWgradThreads, 1) grouped_wgrad_kernel(const _
       stage = (stage + nkb) % C::kStages;
     }
   } else {
-    const int quad = warp & 3;
+    const int quad = warp & 3, half = (warp - 2) >> 2;
     int as = 0;
     uint32_t aphase = 0;
     OutT* Cp = reinterpret_cast<OutT*>(p.C);
-    const uint32_t out_stage = ptx::smem_u32(smem + C::kOut + quad * 4096);
+    const uint32_t out_stage = ptx::smem_u32(smem + C::kOut + (warp - 2) * 4096);
     const bool vec_ok = (p.N % (16 / sizeof(OutT)) == 0) && ((reinterpret_cast<uintptr_t>(p.C) & 15) == 0);
     for (int tile = pair; tile < num_tiles; tile += num_pairs) {
       int g, m0, n0, r0, nkb, tail;
@@ -202,19 +206,31 @@ __global__ void __launch_bounds__(kWgradThreads, 1) grouped_wgrad_kernel(const _
       ptx::mbar_wait(ptx::smem_u32(&tmem_full[as]), aphase);
       ptx::tc_fence_after();
       const int row0 = m0 + (int)rank * BM + quad * 32;
-      const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + as * BN;
+      const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + as * BN + half * (BN / 2);
+      n0 += half * (BN / 2);
+      OutT* dst = Cp + ((int64_t)g * p.M + row0) * p.N + n0;
+      if (sizeof(OutT) == 2 && vec_ok && !p.accumulate && nkb > 0 && n0 + BN / 2 <= p.N && row0 + 32 <= p.M) {
 #pragma unroll 1
-      for (int c = 0; c < BN / 32; ++c) {
-        uint32_t r[32];
-        ptx::tc_ld_32x32(taddr + c * 32, r);  // warp-collective: executed by every lane whatever its row
-        ptx::tc_wait_ld();
-        const int col = n0 + c * 32;
-        const int n_valid = min(32, p.N - col);
-        if (row0 < p.M && n_valid > 0 && !(nkb == 0 && p.accumulate)) {
-          float v[32];
+        for (int c = 0; c < BN / 2; c += 64) {
+          uint32_t r[64];
+          ptx::tc_ld_32x32(taddr + c, r);
+          ptx::tc_ld_32x32(taddr + c + 32, r + 32);
+          ptx::tc_wait_ld();
+          store_rows64<OutT>(out_stage, r, dst + c, p.N);
+        }
+      } else {
+#pragma unroll 1
+        for (int c = 0; c < BN / 2; c += 32) {
+          uint32_t r[32];
+          ptx::tc_ld_32x32(taddr + c, r);  // warp-collective: executed by every lane whatever its row
+          ptx::tc_wait_ld();
+          const int n_valid = min(32, p.N - n0 - c);
+          if (row0 < p.M && n_valid > 0 && !(nkb == 0 && p.accumulate)) {
+            float v[32];
 #pragma unroll
-          for (int i = 0; i < 32; ++i) v[i] = nkb == 0 ? 0.f : __uint_as_float(r[i]);  // no tokens: the accumulator is stale
-          store_rows32<OutT>(out_stage, v, Cp + ((int64_t)g * p.M + row0) * p.N + col, p.N, p.M - row0, n_valid, vec_ok, p.accumulate);
+            for (int i = 0; i < 32; ++i) v[i] = nkb == 0 ? 0.f : __uint_as_float(r[i]);  // no tokens: the accumulator is stale
+            store_rows32<OutT>(out_stage, v, dst + c, p.N, p.M - row0, n_valid, vec_ok, p.accumulate);
+          }
         }
       }
       ptx::tc_fence_before();
