@@ -15,7 +15,7 @@
 // Kernels on the decode path are launched with programmatic dependent launch (they signal their successors at once and wait for
 // their predecessor before the first global access), like the framework's other decode kernels.
 //   delta_rule       the recurrence.  A column of S depends only on its own v column, so columns are independent: a thread group of
-//                    LPC lanes owns one column (32 or 64 state rows per lane in registers), a CTA 128 / LPC columns of one
+//                    LPC lanes owns NC columns (16 state rows of each per lane in registers), a CTA 128 / LPC * NC columns of one
 //                    (sequence, head).  q, k, v, beta, g of 8 tokens at a time are staged in shared memory.  Packed form: S starts
 //                    at zero and the final S goes to s_state[slot]; step form: S is loaded from and stored to s_state[slot].
 //   gated_head_norm  o / sqrt(mean(o^2) + eps) * w * silu(gate) or sigmoid(gate) per (token, head) -> model type.
@@ -231,7 +231,7 @@ __global__ void __launch_bounds__(kPThreads) delta_prepare_tiled_kernel(const vo
 }
 
 // ------------------------------------------------------------------------------------------------ recurrence
-constexpr int kScanThreads = 128, kTok = 8;   // kEPL (template): state rows per lane, 32 or 64
+constexpr int kScanThreads = 128, kTok = 8;
 
 struct ScanParams {
   const float* u; float* o;
@@ -241,18 +241,48 @@ struct ScanParams {
   int H, G, d, dv, step;
 };
 
-// Row mapping: lane l of a column's LPC lanes holds the state rows ((e / 4) * LPC + l) * 4 + e % 4, e = 0 .. 31, so that its q / k
-// operands are 8 aligned float4 reads of shared memory per token (the lanes of a column read neighbouring float4s, the columns of
-// a warp the same ones).  Dot products run on four independent accumulators.  kChan: a decay per state row, staged beside q and k.
-template <int LPC, int kEPL, bool kChan>
-__global__ void __launch_bounds__(kScanThreads, kEPL == 32 ? 3 : 2) delta_rule_kernel(ScanParams p) {
-  constexpr int NCOL = kScanThreads / LPC;
+// A group of LPC lanes owns NC neighbouring columns of the state: lane l holds their rows ((e / 4) * LPC + l) * 4 + e % 4, e = 0 .. 15, so that its q / k
+// operands are four aligned float4 reads of shared memory each per token, used for all NC columns.  kChan: a decay per state row, staged beside q and k.
+//
+// What bounds it: a token is one step of a serial chain, so what counts is its latency and, with few sequences, the shared-memory port and the fp32
+// pipe of the SMs that hold two CTAs.  With D the decayed state, the output is S^T q = D^T q + (k . q) u: both products read D, none waits for the
+// update, and k . q is one number per token for all columns.  A scalar decay is not multiplied into the state: S = c Z with c the product of the
+// decays since the last time Z took it in, u enters Z as u / c, and Z takes c in when c falls below 2^-20 (at once for a decay of 0).  That leaves three
+// multiply-adds per state element and token, two elements an instruction.  8 sequences of 700..1024 tokens, 16 heads x 128 x 128: 643 us with the
+// decay, the update and the second product in sequence and one column per lane pair; 595 us with this order (a lane of a column's pair reads 32
+// float4s of q and k a token, and shared memory serves an SM one such read in four cycles); 540 us with four columns to a group of eight lanes.
+RB_DEVICE uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+RB_DEVICE uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+RB_DEVICE uint64_t pair_of(float lo, float hi) {
+  uint64_t d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+  return d;
+}
+RB_DEVICE float2 halves(uint64_t a) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a));
+  return r;
+}
+constexpr float kTakeIn = 1.f / (1 << 20);
+
+template <int LPC, int NC, bool kChan>
+__global__ void __launch_bounds__(kScanThreads, LPC <= 8 ? 3 : 2) delta_rule_kernel(ScanParams p) {
+  constexpr int kRows = 16, NCOL = kScanThreads / LPC * NC;
+  static_assert(2 * NC <= LPC, "a lane ends up with at most one of the group's 2 NC sums");
   extern __shared__ __align__(16) float sm[];
+  __shared__ float4 tok[kTok];                     // per token: beta, c after its decay, 1 / c (0: Z takes c in), k . q
   const int seq = blockIdx.x, h = blockIdx.y, c0 = blockIdx.z * NCOL;
   const int g = h / (p.H / p.G), d = p.d, dv = p.dv;
   const int nqk = p.G * d, C = 2 * nqk + p.H * dv, UW = C + p.H + (kChan ? p.H * d : p.H);
-  const int tid = threadIdx.x, l = tid % LPC, col = c0 + tid / LPC;
-  const bool active = col < dv;
+  const int tid = threadIdx.x, l = tid % LPC, lcol = tid / LPC * NC, col = c0 + lcol, warp = tid >> 5, lane = tid & 31;
   int t0, t1;
   rb::pdl_trigger();
   rb::pdl_wait();
@@ -260,18 +290,21 @@ __global__ void __launch_bounds__(kScanThreads, kEPL == 32 ? 3 : 2) delta_rule_k
   if (t1 <= t0) return;
   const int slot = p.s_state == nullptr ? -1 : (p.slots ? p.slots[seq] : (p.step ? seq : -1));
   float* S_g = slot >= 0 ? p.s_state + (((int64_t)slot * p.H + h) * d) * dv : nullptr;
-  constexpr int dpad = kEPL * LPC;                // rows >= d hold zeros and read zero q / k
+  constexpr int dpad = kRows * LPC;               // rows >= d hold zeros and read zero q / k
   constexpr int kBuf = (kChan ? 3 : 2) * kTok * dpad + kTok * NCOL + 2 * kTok;   // floats of one staging buffer: q, k, v, (beta, g), row decays
   constexpr int NQ = kTok * dpad / kScanThreads, NV = (kTok * NCOL + kScanThreads - 1) / kScanThreads;
   auto row_of = [&](int e) { return ((e >> 2) * LPC + l) * 4 + (e & 3); };
-  float S[kEPL];
+  uint64_t Z[NC][kRows / 2];
 #pragma unroll
-  for (int e = 0; e < kEPL; ++e) {
-    const int row = row_of(e);
-    S[e] = (p.step && S_g && active && row < d) ? S_g[(int64_t)row * dv + col] : 0.f;
-  }
-  // The inputs of the next 8 tokens are fetched into registers while the current 8 are processed out of shared memory (two
-  // staging buffers, one barrier per chunk).
+  for (int j = 0; j < NC; ++j)
+#pragma unroll
+    for (int e = 0; e < kRows; e += 2) {
+      float z[2];
+#pragma unroll
+      for (int i = 0; i < 2; ++i) z[i] = (p.step && S_g && col + j < dv && row_of(e + i) < d) ? S_g[(int64_t)row_of(e + i) * dv + col + j] : 0.f;
+      Z[j][e / 2] = pair_of(z[0], z[1]);
+    }
+  // The inputs of the next 8 tokens are fetched into registers while the current 8 are processed out of shared memory (two staging buffers).
   float rq[NQ], rk[NQ], rg[kChan ? NQ : 1], rv[NV], rb = 0.f;
   auto fetch = [&](int tb) {
     const int nt = min(kTok, t1 - tb);
@@ -303,62 +336,121 @@ __global__ void __launch_bounds__(kScanThreads, kEPL == 32 ? 3 : 2) delta_rule_k
       for (int i = 0; i < NQ; ++i) buf[2 * kTok * dpad + kTok * NCOL + 2 * kTok + tid + i * kScanThreads] = rg[i];
     }
   };
+  // which of the group's sums (k products of its NC columns, then q products) this lane ends up with
+  int mine = 0;
+#pragma unroll
+  for (int n = 2 * NC, o = LPC / 2; n > 1; n >>= 1, o >>= 1) mine += (l & o) ? n / 2 : 0;
+  const int my_col = mine % NC;
+  const bool writes = mine >= NC && (l & (LPC / (2 * NC) - 1)) == 0 && col + my_col < dv;
+
   fetch(t0);
   int which = 0;
+  float c = 1.f;                                   // S = c Z (the same in all threads)
   for (int tb = t0; tb < t1; tb += kTok, which ^= 1) {
     const int nt = min(kTok, t1 - tb);
     float* buf = sm + which * kBuf;
     stage(buf);
-    __syncthreads();
-    if (tb + kTok < t1) fetch(tb + kTok);
+    __syncthreads();                               // (the numbers of the last chunk's tokens have been read, too)
     const float* qs = buf;
     const float* ks = buf + kTok * dpad;
     const float* vs = ks + kTok * dpad;
     const float* bg = vs + kTok * NCOL;
     const float* gs = bg + 2 * kTok;                // kChan: [kTok][dpad]
+    // the chunk's numbers per token: every warp k . q of two tokens, the decays' products in every lane, one token's kept
+    float c1 = 1.f, beta1 = 0.f;
+    bool in1 = false;
+#pragma unroll
+    for (int tt = 0; tt < kTok; ++tt) {
+      if constexpr (!kChan) c *= tt < nt ? bg[tt * 2 + 1] : 1.f;
+      const bool in = !kChan && !(c >= kTakeIn && c <= 1.f / kTakeIn);
+      if (lane == tt) { c1 = c; in1 = in; beta1 = bg[tt * 2]; }
+      if (in) c = 1.f;
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int tt = warp + 4 * i;
+      float a = 0.f;
+#pragma unroll
+      for (int e = 0; e < dpad; e += 32) a = fmaf(ks[tt * dpad + e + lane], qs[tt * dpad + e + lane], a);
+      a = rb::warp_sum(a);
+      if (lane == tt) tok[tt] = make_float4(beta1, c1, in1 ? 0.f : 1.f / c1, a);
+    }
+    __syncthreads();
+    if (tb + kTok < t1) fetch(tb + kTok);
     for (int tt = 0; tt < nt; ++tt) {
-      const float beta = bg[tt * 2], gg = bg[tt * 2 + 1];
-      const float4* kq = reinterpret_cast<const float4*>(ks + tt * dpad) + l;
-      const float4* qq = reinterpret_cast<const float4*>(qs + tt * dpad) + l;
-      const float4* dg = reinterpret_cast<const float4*>(gs + tt * dpad) + l;
-      float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
+      const float4 n = tok[tt];
+      const ulonglong2* kp = reinterpret_cast<const ulonglong2*>(ks + tt * dpad) + l;
+      const ulonglong2* qp = reinterpret_cast<const ulonglong2*>(qs + tt * dpad) + l;
+      const float v = vs[tt * NCOL + lcol + my_col];
+      uint64_t kk[kRows / 2], ak[NC], aq[NC];
 #pragma unroll
-      for (int e4 = 0; e4 < kEPL / 4; ++e4) {
-        const float4 kk = kq[e4 * LPC];
+      for (int j = 0; j < NC; ++j) ak[j] = aq[j] = 0;
+#pragma unroll
+      for (int e4 = 0; e4 < kRows / 4; ++e4) {
+        const ulonglong2 k2 = kp[e4 * LPC], q2 = qp[e4 * LPC];
+        kk[2 * e4] = k2.x;
+        kk[2 * e4 + 1] = k2.y;
         if constexpr (kChan) {
-          const float4 g4 = dg[e4 * LPC];
-          S[e4 * 4] *= g4.x; S[e4 * 4 + 1] *= g4.y; S[e4 * 4 + 2] *= g4.z; S[e4 * 4 + 3] *= g4.w;
-        } else {
-          S[e4 * 4] *= gg; S[e4 * 4 + 1] *= gg; S[e4 * 4 + 2] *= gg; S[e4 * 4 + 3] *= gg;
+          const ulonglong2 g2 = (reinterpret_cast<const ulonglong2*>(gs + tt * dpad) + l)[e4 * LPC];
+#pragma unroll
+          for (int j = 0; j < NC; ++j) {
+            Z[j][2 * e4] = mul2(Z[j][2 * e4], g2.x);
+            Z[j][2 * e4 + 1] = mul2(Z[j][2 * e4 + 1], g2.y);
+          }
         }
-        a0 = fmaf(S[e4 * 4], kk.x, a0); a1 = fmaf(S[e4 * 4 + 1], kk.y, a1);
-        a2 = fmaf(S[e4 * 4 + 2], kk.z, a2); a3 = fmaf(S[e4 * 4 + 3], kk.w, a3);
+#pragma unroll
+        for (int j = 0; j < NC; ++j) { ak[j] = fma2(Z[j][2 * e4], k2.x, ak[j]); aq[j] = fma2(Z[j][2 * e4], q2.x, aq[j]); }
+#pragma unroll
+        for (int j = 0; j < NC; ++j) { ak[j] = fma2(Z[j][2 * e4 + 1], k2.y, ak[j]); aq[j] = fma2(Z[j][2 * e4 + 1], q2.y, aq[j]); }
       }
-      float acc = (a0 + a1) + (a2 + a3);
+      float sum[2 * NC];
 #pragma unroll
-      for (int off = 1; off < LPC; off <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
-      const float w = beta * (vs[tt * NCOL + tid / LPC] - acc);
-      a0 = a1 = a2 = a3 = 0.f;
-#pragma unroll
-      for (int e4 = 0; e4 < kEPL / 4; ++e4) {
-        const float4 kk = kq[e4 * LPC], q4 = qq[e4 * LPC];
-        S[e4 * 4] = fmaf(kk.x, w, S[e4 * 4]); S[e4 * 4 + 1] = fmaf(kk.y, w, S[e4 * 4 + 1]);
-        S[e4 * 4 + 2] = fmaf(kk.z, w, S[e4 * 4 + 2]); S[e4 * 4 + 3] = fmaf(kk.w, w, S[e4 * 4 + 3]);
-        a0 = fmaf(S[e4 * 4], q4.x, a0); a1 = fmaf(S[e4 * 4 + 1], q4.y, a1);
-        a2 = fmaf(S[e4 * 4 + 2], q4.z, a2); a3 = fmaf(S[e4 * 4 + 3], q4.w, a3);
+      for (int j = 0; j < NC; ++j) {
+        const float2 a = halves(ak[j]), b = halves(aq[j]);
+        sum[j] = a.x + a.y;
+        sum[NC + j] = b.x + b.y;
       }
-      float ov = (a0 + a1) + (a2 + a3);
+      // the group's sums over its lanes: every step halves what a lane still carries, then the rest is summed whole
 #pragma unroll
-      for (int off = 1; off < LPC; off <<= 1) ov += __shfl_xor_sync(0xffffffffu, ov, off);
-      if (active && l == 0) p.o[((int64_t)(tb + tt) * p.H + h) * dv + col] = ov;
+      for (int m = 2 * NC, o = LPC / 2; m > 1; m >>= 1, o >>= 1) {
+        const bool hi = (l & o) != 0;
+#pragma unroll
+        for (int i = 0; i < m / 2; ++i) {
+          const float keep = hi ? sum[m / 2 + i] : sum[i], send = hi ? sum[i] : sum[m / 2 + i];
+          sum[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+      }
+#pragma unroll
+      for (int o = LPC / (2 * NC) / 2; o > 0; o >>= 1) sum[0] += __shfl_xor_sync(0xffffffffu, sum[0], o);
+      const float w = n.x * (v - n.y * sum[0]);                                      // (meaningful in the lanes that hold a k product)
+      const float w_mine = __shfl_xor_sync(0xffffffffu, w, LPC / 2);                 // the same column's, in the lanes that hold a q product
+      if (writes) p.o[((int64_t)(tb + tt) * p.H + h) * dv + col + my_col] = fmaf(w_mine, n.w, n.y * sum[0]);
+      const bool take = !kChan && n.z == 0.f;
+      const uint64_t c2 = pair_of(n.y, n.y);
+#pragma unroll
+      for (int j = 0; j < NC; ++j) {
+        float wj = __shfl_sync(0xffffffffu, w, (lane & ~(LPC - 1)) + j * (LPC / (2 * NC)));     // lane that holds sum j
+        if (take) {
+#pragma unroll
+          for (int e = 0; e < kRows / 2; ++e) Z[j][e] = mul2(Z[j][e], c2);
+        } else {
+          wj *= n.z;
+        }
+        const uint64_t w2 = pair_of(wj, wj);
+#pragma unroll
+        for (int e = 0; e < kRows / 2; ++e) Z[j][e] = fma2(kk[e], w2, Z[j][e]);
+      }
     }
   }
-  if (S_g && active) {
+  if (S_g) {
 #pragma unroll
-    for (int e = 0; e < kEPL; ++e) {
-      const int row = row_of(e);
-      if (row < d) S_g[(int64_t)row * dv + col] = S[e];
-    }
+    for (int j = 0; j < NC; ++j)
+#pragma unroll
+      for (int e = 0; e < kRows; e += 2) {
+        const float2 z = halves(Z[j][e / 2]);
+        if (col + j < dv && row_of(e) < d) S_g[(int64_t)row_of(e) * dv + col + j] = c * z.x;
+        if (col + j < dv && row_of(e + 1) < d) S_g[(int64_t)row_of(e + 1) * dv + col + j] = c * z.y;
+      }
   }
 }
 
@@ -422,11 +514,11 @@ extern "C" int rb_delta_prepare(const void* proj, int64_t ld, int dt, const void
   return 0;
 }
 
-template <int LPC, int EPL, bool CHAN>
+template <int LPC, int NC, bool CHAN>
 static int launch_delta_rule(const ScanParams& p, int n_seqs, cudaStream_t s) {
-  constexpr int ncol = kScanThreads / LPC;
-  constexpr size_t smem = 2 * sizeof(float) * ((size_t)(CHAN ? 3 : 2) * kTok * EPL * LPC + (size_t)kTok * ncol + 2 * kTok);   // two staging buffers
-  auto kern = delta_rule_kernel<LPC, EPL, CHAN>;
+  constexpr int ncol = kScanThreads / LPC * NC;
+  constexpr size_t smem = 2 * sizeof(float) * ((size_t)(CHAN ? 3 : 2) * kTok * 16 * LPC + (size_t)kTok * ncol + 2 * kTok);   // two staging buffers
+  auto kern = delta_rule_kernel<LPC, NC, CHAN>;
   if (smem > 48 * 1024 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return -4;
   return rb::launch_pdl(kern, dim3(n_seqs, p.H, RB_CEIL_DIV(p.dv, ncol)), dim3(kScanThreads), smem, s, p) == cudaSuccess ? 0 : -3;
 }
@@ -437,14 +529,13 @@ extern "C" int rb_delta_rule(const float* u, float* o, const int* cu, float* s_s
   if (n_seqs == 0) return 0;
   if (d > 512 || H % G) return -1;
   ScanParams p{u, o, cu, s_state, slots, H, G, d, dv, step};
-  // (lanes per column, state rows per lane): 64 rows per lane from head size 128 up halves the shuffle rounds and the shared
-  // reads per FMA at two CTAs per SM
-#define RB_L(LPC, EPL) return channel ? launch_delta_rule<LPC, EPL, true>(p, n_seqs, s) : launch_delta_rule<LPC, EPL, false>(p, n_seqs, s)
-  if (d <= 32) { RB_L(1, 32); }
-  if (d <= 64) { RB_L(2, 32); }
-  if (d <= 128) { RB_L(2, 64); }
-  if (d <= 256) { RB_L(4, 64); }
-  RB_L(8, 64);
+  // (lanes per group, columns per group): 16 LPC state rows; 64 columns a CTA up to head size 128
+#define RB_L(LPC, NC) return channel ? launch_delta_rule<LPC, NC, true>(p, n_seqs, s) : launch_delta_rule<LPC, NC, false>(p, n_seqs, s)
+  if (d <= 32) { RB_L(2, 1); }
+  if (d <= 64) { RB_L(4, 2); }
+  if (d <= 128) { RB_L(8, 4); }
+  if (d <= 256) { RB_L(16, 4); }
+  RB_L(32, 4);
 #undef RB_L
 }
 

@@ -1,0 +1,50 @@
+"""The delta rule's kernel where its bookkeeping can go wrong: decays whose product leaves the range it is carried in (0, tiny, 1, above 1),
+head sizes at and between the kernel's lane groups, columns that do not fill a group, empty and one-token sequences, both kinds of decay, and
+decode steps that go on from a prompt's state."""
+import pytest
+import torch
+
+from realhf_b200.api.model import DeltaRuleConfig
+from realhf_b200.ops import recurrent as R
+
+pytestmark = pytest.mark.gpu
+LENS = [1, 9, 0, 70, 33]
+
+
+def inputs(d, dv, decays, channel, n, seed):
+    g = torch.Generator().manual_seed(seed)
+    H, G = 4, 2
+    unit = lambda x: torch.nn.functional.normalize(x, dim=-1)
+    q, k, v = unit(torch.randn(n, G, d, generator=g)), unit(torch.randn(n, G, d, generator=g)), torch.randn(n, H, dv, generator=g)
+    r = torch.rand(n, H * d if channel else H, generator=g)
+    decay = {"one": torch.ones_like(r), "mixed": 0.1 + 0.9 * r, "zeros": torch.where(r < 0.2, 0.0, r), "tiny": torch.where(r < 0.3, 1e-30 * r, r),
+             "growing": 0.9 + 0.4 * r}[decays]
+    cfg = DeltaRuleConfig(n_heads=H, n_kv_heads=G, qk_dim=d, v_dim=dv, conv_taps=1, **(dict(decay_rank=8) if channel else {}))
+    return cfg, torch.cat([q.reshape(n, -1), k.reshape(n, -1), v.reshape(n, -1), torch.rand(n, H, generator=g), decay], -1)
+
+
+@pytest.mark.parametrize("d,dv", [(16, 8), (32, 40), (48, 20), (64, 130), (128, 128), (200, 70), (256, 17), (512, 24)])
+@pytest.mark.parametrize("decays,channel", [("one", False), ("mixed", False), ("zeros", False), ("tiny", False), ("growing", False), ("mixed", True),
+                                            ("zeros", True)])
+def test_delta_rule_decays_and_shapes(d, dv, decays, channel):
+    cfg, u = inputs(d, dv, decays, channel, sum(LENS) + 3, d + dv)
+    cu = torch.tensor([0] + LENS).cumsum(0).int()
+    slots = torch.tensor([4, 0, 2, -1, 3], dtype=torch.int32)
+    pick = torch.tensor([0, 4, 3], dtype=torch.int32)            # three decode steps, one on an untouched slot
+    n = sum(LENS)
+
+    def run(u, native):
+        dev = u.device
+        S = torch.full((6, 4, d, dv), 0.25, dtype=u.dtype, device=dev)
+        scan, step = (R.delta_rule_scan, R.delta_rule_step) if native else (R.delta_rule_scan_ref, R.delta_rule_step_ref)
+        args = cu.to(dev), S, slots.to(dev)
+        o = scan(u[:n], cfg, *args)
+        o2 = step(u[n:], cfg, S, pick.to(dev))
+        return torch.cat([o, o2]).double().cpu(), S.double().cpu()
+
+    want = run(u.double(), False)
+    plain, got = run(u, False), run(u.cuda(), True)
+    for w, f, x in zip(want, plain, got):
+        # The yardstick is fp32's own rounding: the plain fp32 recurrence's largest error, four times it for another order of sums and the
+        # decays' product, plus a few ulps of the largest value.
+        assert float((x - w).abs().max()) <= 4 * float((f - w).abs().max()) + 8 * 2.0 ** -23 * float(w.abs().max())
