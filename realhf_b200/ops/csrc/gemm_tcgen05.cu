@@ -407,34 +407,37 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_streamk_kernel(const __grid_
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t idesc = kFmt == 2 ? ptx::make_idesc_f8(0, 0, BM, BN) : ptx::make_idesc_f16(kFmt, BM, BN, 0, 0);
-      int stage = 0, as = 0;
-      uint32_t phase = 0, aphase = 0;
-      int u = u_begin;
-      while (u < u_end) {
-        const int tile = u / num_kb;
-        const int seg_end = min(u_end, (tile + 1) * num_kb);
-        ptx::mbar_wait(ptx::smem_u32(&tmem_empty[as]), aphase ^ 1);
+    // The warp runs converged, one elected lane issues: from a divergent branch every tcgen05.mma cost ~100 cycles, 0.33 us a k-block.
+    const uint32_t idesc = (uint32_t)ptx::uniform((int)(kFmt == 2 ? ptx::make_idesc_f8(0, 0, BM, BN) : ptx::make_idesc_f16(kFmt, BM, BN, 0, 0)));
+    const uint32_t tm = (uint32_t)ptx::uniform((int)tmem_base);
+    const int end = ptx::uniform(u_end), nkb = ptx::uniform(num_kb);
+    int stage = 0, as = 0;
+    uint32_t phase = 0, aphase = 0;
+    int u = ptx::uniform(u_begin);
+    while (u < end) {
+      const int seg_end = min(end, (u / nkb + 1) * nkb);
+      ptx::mbar_wait(ptx::smem_u32(&tmem_empty[as]), aphase ^ 1);
+      ptx::tc_fence_after();
+      const uint32_t d_tmem = tm + as * 256;
+      for (int first = 1; u < seg_end; ++u, first = 0) {
+        ptx::mbar_wait(ptx::smem_u32(&full_bar[stage]), phase);
         ptx::tc_fence_after();
-        const uint32_t d_tmem = tmem_base + as * 256;
-        for (int first = 1; u < seg_end; ++u, first = 0) {
-          ptx::mbar_wait(ptx::smem_u32(&full_bar[stage]), phase);
-          ptx::tc_fence_after();
-          const uint32_t sa = ptx::smem_u32(smem_a + stage * kABytes);
-          const uint32_t sb = ptx::smem_u32(smem_b + stage * b_bytes);
+        const uint64_t da = ptx::make_smem_desc_sw128(ptx::smem_u32(smem_a + stage * kABytes), 16, 1024);
+        const uint64_t db = ptx::make_smem_desc_sw128(ptx::smem_u32(smem_b + stage * b_bytes), 16, 1024);
+        if (ptx::elect_one()) {
 #pragma unroll
           for (int k = 0; k < BK / 16; ++k) {  // 4 instructions of 32 bytes of K each: 16 bf16 or 32 fp8 elements
-            const uint64_t da = ptx::make_smem_desc_sw128(sa + k * 32, 16, 1024), db = ptx::make_smem_desc_sw128(sb + k * 32, 16, 1024);
-            if constexpr (kFmt == 2) ptx::tc_mma_f8(d_tmem, da, db, idesc, (first && k == 0) ? 0u : 1u);
-            else ptx::tc_mma_f16(d_tmem, da, db, idesc, (first && k == 0) ? 0u : 1u);
+            if constexpr (kFmt == 2) ptx::tc_mma_f8(d_tmem, da + k * 2, db + k * 2, idesc, (first && k == 0) ? 0u : 1u);
+            else ptx::tc_mma_f16(d_tmem, da + k * 2, db + k * 2, idesc, (first && k == 0) ? 0u : 1u);
           }
           ptx::tc_commit(ptx::smem_u32(&empty_bar[stage]));
-          if (++stage == n_stages) { stage = 0; phase ^= 1; }
         }
-        ptx::tc_commit(ptx::smem_u32(&tmem_full[as]));
-        if (++as == 2) { as = 0; aphase ^= 1; }
+        __syncwarp();
+        if (++stage == n_stages) { stage = 0; phase ^= 1; }
       }
+      if (ptx::elect_one()) ptx::tc_commit(ptx::smem_u32(&tmem_full[as]));
+      __syncwarp();
+      if (++as == 2) { as = 0; aphase ^= 1; }
     }
   } else {
     const int quad = warp & 3;
