@@ -21,9 +21,9 @@
 //
 // Tensor memory (512 columns): S_t at 128 t, O_t at 256 + 128 t.  P_t (16 bit) overwrites the front of S_t and is the TMEM A operand of
 // P V, so it never travels through shared memory; S_t of the next tile is issued behind that product on the in-order tensor pipe.  O
-// accumulates in TMEM over the whole stream.  The row maximum that weights are taken against only moves when a tile's maximum exceeds it
-// by more than 2^8 (then the warp scales O once the product in flight has retired): weights, sum and output carry the same factor, so the
-// result is the softmax of the same scores, and fp32 / bf16 / fp16 all have room for 2^8.  V_j is the MN-major B operand.
+// accumulates in TMEM over the whole stream; when a row's maximum grows, its warp scales O once the product in flight has retired.  (A maximum
+// that only moves when weights exceed it by 2^8 is 2..3 % faster in training, 10 % with a window, but the largest weight is then no longer exactly
+// 1 when P is rounded to 16 bits: error against 64 bits 0.0028 instead of 0.0025.)  V_j is the MN-major B operand.
 // Issue order: S_0, S_1, then per key tile PV_0, S_0', PV_1, S_1'.  The issuing warp runs converged and elects a lane for the MMAs alone: issued from
 // `if (lane == 0)` with descriptors built there, eight MMAs took 820-960 cycles of one thread, whatever their size (294 -> 242 us converged, 231 us with the
 // descriptors built in front of the elected branch; two scores per instruction in the softmax: 221 us).
@@ -36,7 +36,7 @@
 // maximum is taken over the raw products.  kCap: kSimple with score = softcap * tanh(s * scale / softcap); the cap is monotone, so the
 // raw maximum is capped once.  All three: a per-head sink logit starts the running maximum with denominator 1; the output is
 // multiplied by sigmoid(gate logit of its head, or of the output element); `chunk` > 0 replaces the window: a query sees the keys of its own
-// chunk of positions up to itself.  (32 x 1024 tokens, 16 / 4 heads, window 512 + 64 kept: 1382 us with one tile per CTA, now 259.)
+// chunk of positions up to itself.  (32 x 1024 tokens, 16 / 4 heads, window 512 + 64 kept: 1382 us with one tile per CTA, now 285.)
 // Learned distance biases and shared keys / values run in attn_fwd_bias.cu.
 #include "attn_common.cuh"
 
@@ -46,7 +46,6 @@ constexpr int kTile = 128;          // query rows of a tile (= UMMA M) and keys 
 constexpr int kFwdThreads = 384;    // three warpgroups: 168 registers a thread at launch, 64512 in all
 constexpr int kSoftmaxRegs = 208, kOtherRegs = 80;   // 2 x 128 x 208 + 128 x 80 = 63488: a softmax thread holds a whole score row
 constexpr int kStages = 4;          // K and V tiles share one ring: two key tiles in flight
-constexpr float kLazy = 8.f;        // log2 of how far weights may exceed 1 before the maximum moves
 
 enum Mode { kPlain = 0, kSimple = 1, kCap = 2, kGeneral = 3 };
 
@@ -367,8 +366,8 @@ __global__ void __launch_bounds__(kFwdThreads, 1) attn_fwd_kernel(const __grid_c
           const float m_new = fmaxf(m_run, mx);
           if (m_new != -INFINITY) l_run *= exp2f(m_run - m_new);
           m_run = m_new;
-        } else if (__any_sync(0xffffffffu, mx > m_run + kLazy)) {
-          const float m_new = mx > m_run + kLazy ? mx : m_run;
+        } else if (__any_sync(0xffffffffu, mx > m_run)) {
+          const float m_new = fmaxf(m_run, mx);
           const float a = m_new == m_run ? 1.f : exp2f(m_run - m_new);
           wait(O_FULL + t, (vc - 1) & 1u);          // the product in flight has retired, and the next one waits for this tile's P
           ptx::tc_fence_after();

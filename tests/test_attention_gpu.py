@@ -165,8 +165,8 @@ def _attention_f64(q, k, v, lens, scale, causal, window):
 @pytest.mark.parametrize("form", ["causal", "full", "window", "growing"])
 def test_attn_fwd_tile_pairs(heads, lens, form):
     """Tile pairs over heads (even groups) and over rows (odd groups), left-over tiles, empty sequences, more than 32 sequences, windows, and scores
-    whose maximum grows by far more than the lazy step from tile to tile.  Bound: the weights and the result are rounded to 16 bits once each,
-    2^-9 of the weighted sum of |v| and 2^-9 of the result, doubled for the exponentials and the stale maximum's factor."""
+    whose maximum grows by orders of magnitude from tile to tile.  Bound: the weights and the result are rounded to 16 bits once each,
+    2^-9 of the weighted sum of |v| and 2^-9 of the result, doubled for the exponentials and the scaling of earlier tiles."""
     nq, nkv, hd = heads
     dt = torch.float16 if form == "window" else torch.bfloat16
     torch.manual_seed(len(lens) + nq)
