@@ -10,8 +10,8 @@
 // 48 KB to 32 KB (6 pipeline stages instead of 4), and B is fetched from L2 once per pair.
 //
 // Roles per CTA (6 warps, as in gemm_tcgen05.cu): warp 0 TMA producer (both CTAs load; every transfer completes on the
-// LEADER's full barrier), warp 1 lane 0 of the leader (cluster rank 0) issues all MMAs and multicasts tcgen05.commit
-// onto both CTAs' empty / accumulator-full barriers, warps 2-5 drain the CTA's own 128 accumulator rows from TMEM and
+// LEADER's full barrier), warp 1 of the leader (cluster rank 0; converged, one elected lane) issues all MMAs and multicasts tcgen05.commit
+// onto both CTAs' empty / accumulator-full barriers, warps 2-5 drain the CTA's own 128 accumulator rows from TMEM, store them in whole lines and
 // release the accumulator stage on the leader's barrier (8 arrivals: 4 warps x 2 CTAs).
 // Operand majors as in the tile kernel (K-major or MN-major each), so fwd / dgrad / wgrad all run here.
 #include "cta_pair.cuh"
