@@ -21,7 +21,9 @@
 //
 // Tensor memory (512 columns): S_t at 128 t, O_t at 256 + 128 t.  P_t (16 bit) overwrites the front of S_t and is the TMEM A operand of
 // P V, so it never travels through shared memory; S_t of the next tile is issued behind that product on the in-order tensor pipe.  O
-// accumulates in TMEM over the whole stream; when a row's maximum grows, its warp scales O once the product in flight has retired.  (A maximum
+// accumulates in TMEM over the whole stream; when a row's maximum grows, its warp scales O once the product in flight has retired and
+// the weights are stored: the scores' registers then hold the whole output row at once (before the exponentials, a quarter at a time: 15 us of
+// 305 in a windowed prefill).  (A maximum
 // that only moves when weights exceed it by 2^8 is 2..3 % faster in training, 10 % with a window, but the largest weight is then no longer exactly
 // 1 when P is rounded to 16 bits: error against 64 bits 0.0028 instead of 0.0025.)  V_j is the MN-major B operand.
 // Issue order: S_0, S_1, then per key tile PV_0, S_0', PV_1, S_1'.  The issuing warp runs converged and elects a lane for the MMAs alone: issued from
@@ -36,7 +38,7 @@
 // maximum is taken over the raw products.  kCap: kSimple with score = softcap * tanh(s * scale / softcap); the cap is monotone, so the
 // raw maximum is capped once.  All three: a per-head sink logit starts the running maximum with denominator 1; the output is
 // multiplied by sigmoid(gate logit of its head, or of the output element); `chunk` > 0 replaces the window: a query sees the keys of its own
-// chunk of positions up to itself.  (32 x 1024 tokens, 16 / 4 heads, window 512 + 64 kept: 1382 us with one tile per CTA, now 285.)
+// chunk of positions up to itself.  (32 x 1024 tokens, 16 / 4 heads, window 512 + 64 kept: 1382 us with one tile per CTA, now 263.)
 // Learned distance biases and shared keys / values run in attn_fwd_bias.cu.
 #include "attn_common.cuh"
 
@@ -362,26 +364,18 @@ __global__ void __launch_bounds__(kFwdThreads, 1) attn_fwd_kernel(const __grid_c
           for (int e = 0; e < 4; ++e) mx4[e] = fmaxf(mx4[e], fmaxf(s[i + 2 * e], s[i + 2 * e + 1]));
         float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
         if (kMode != kGeneral && mx != -INFINITY) mx = kMode == kCap ? soft_cap2(mx, cap_c, cap_k, cap_k) : mx * c2;
+        float alpha = 1.f;
+        bool grown = false;                           // the same in the whole warp
         if (first) {
           const float m_new = fmaxf(m_run, mx);
           if (m_new != -INFINITY) l_run *= exp2f(m_run - m_new);
           m_run = m_new;
         } else if (__any_sync(0xffffffffu, mx > m_run)) {
           const float m_new = fmaxf(m_run, mx);
-          const float a = m_new == m_run ? 1.f : exp2f(m_run - m_new);
-          wait(O_FULL + t, (vc - 1) & 1u);          // the product in flight has retired, and the next one waits for this tile's P
-          ptx::tc_fence_after();
-#pragma unroll
-          for (int c = 0; c < kDV / 32; ++c) {
-            uint32_t o[32];
-            ptx::tc_ld_32x32(tO + c * 32, o);
-            ptx::tc_wait_ld();
-#pragma unroll
-            for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * a);
-            ptx::tc_st_32x32(tO + c * 32, o);
-          }
-          l_run *= a;
+          alpha = m_new == m_run ? 1.f : exp2f(m_run - m_new);
+          l_run *= alpha;
           m_run = m_new;
+          grown = true;
         }
         first = false;
         const float neg_m = m_run == -INFINITY ? 0.f : -m_run;      // fully masked so far: keep exp2 arguments finite
@@ -408,6 +402,20 @@ __global__ void __launch_bounds__(kFwdThreads, 1) attn_fwd_kernel(const __grid_c
         }
         ptx::tc_st_32x32(tS + 32, pw + 32);
         l_run += (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
+        if (grown) {                                  // the scores' registers are free: all of the output row is in flight at once
+          wait(O_FULL + t, (vc - 1) & 1u);            // the product in flight has retired, and the next one waits for this tile's P
+          ptx::tc_fence_after();
+          uint32_t o[kDV];
+#pragma unroll
+          for (int c = 0; c < kDV / 32; ++c) ptx::tc_ld_32x32(tO + c * 32, o + c * 32);
+          ptx::tc_wait_ld();
+#pragma unroll
+          for (int c = 0; c < kDV / 32; ++c) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) o[c * 32 + i] = __float_as_uint(__uint_as_float(o[c * 32 + i]) * alpha);
+            ptx::tc_st_32x32(tO + c * 32, o + c * 32);
+          }
+        }
         ptx::tc_wait_st();
         ptx::tc_fence_before();
         __syncwarp();
