@@ -28,7 +28,7 @@
 // 1 when P is rounded to 16 bits: error against 64 bits 0.0028 instead of 0.0025.)  V_j is the MN-major B operand.
 // Issue order: S_0, S_1, then per key tile PV_0, S_0', PV_1, S_1'.  The issuing warp runs converged and elects a lane for the MMAs alone: issued from
 // `if (lane == 0)` with descriptors built there, eight MMAs took 820-960 cycles of one thread, whatever their size (294 -> 242 us converged, 231 us with the
-// descriptors built in front of the elected branch; two scores per instruction in the softmax: 221 us).
+// descriptors built in front of the elected branch; two scores per instruction in the softmax: 221 us; 229 us with the maximum of every tile).
 //
 // Outputs: O [T, nq, DV] through a per-warp staging buffer (whole 128-byte lines), LSE [nq, T] (natural log, scale applied).
 //
@@ -38,7 +38,7 @@
 // maximum is taken over the raw products.  kCap: kSimple with score = softcap * tanh(s * scale / softcap); the cap is monotone, so the
 // raw maximum is capped once.  All three: a per-head sink logit starts the running maximum with denominator 1; the output is
 // multiplied by sigmoid(gate logit of its head, or of the output element); `chunk` > 0 replaces the window: a query sees the keys of its own
-// chunk of positions up to itself.  (32 x 1024 tokens, 16 / 4 heads, window 512 + 64 kept: 1382 us with one tile per CTA, now 263.)
+// chunk of positions up to itself.  (32 x 1024 tokens, 16 / 4 heads, window 512 + 64 kept: 1382 us with one tile per CTA, now 269.)
 // Learned distance biases and shared keys / values run in attn_fwd_bias.cu.
 #include "attn_common.cuh"
 
