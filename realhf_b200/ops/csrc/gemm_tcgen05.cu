@@ -59,17 +59,12 @@ RB_DEVICE void tile_coords(int tile, int tiles_m, int tiles_n, int bn, int& m0, 
   n0 = (within / gsize) * bn;
 }
 
-// kMC > 1: thread-block cluster of kMC CTAs working on kMC adjacent n-tiles of the SAME m-tile (small-M / decode
-// shapes).  Every CTA loads 1/kMC of the shared A tile and TMA-multicasts it to the whole cluster, so A is fetched
-// from L2 once per cluster instead of once per CTA; a smem stage is recycled only after all kMC consumers released it
-// (tcgen05.commit multicast onto every CTA's empty barrier).
-template <int BN, bool kAMN, bool kBMN, typename OutT, int kFmt, int kMC, int kMode = 0>
+template <int BN, bool kAMN, bool kBMN, typename OutT, int kFmt, int kMode = 0>
 __global__ void __launch_bounds__(kThreads, 1) gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tma_a,
                                                                    const __grid_constant__ CUtensorMap tma_b, Params p,
                                                                    const __grid_constant__ FusedParams fp,
                                                                    const __grid_constant__ TmaArray tma_a_peers) {
-  static_assert(kMC == 1 || !kAMN, "A multicast is implemented for K-major A");
-  static_assert(kMode == 0 || (kMC == 1 && !kAMN), "fused TP modes: K-major A, no cluster");
+  static_assert(kMode == 0 || !kAMN, "fused TP modes: K-major A");
   using C = Cfg<BN>;
   // mode 3: tiles of group g are [s_tile_prefix[g], s_tile_prefix[g+1]); inside a group n-tiles are outer, m-tiles inner
   __shared__ int s_tile_prefix[kMode == 3 ? kMaxGroups + 1 : 1];
@@ -97,9 +92,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tcgen05_kernel(const __grid_
     }
     __syncthreads();
   }
-  // with multicast every CTA of a cluster runs the same number of iterations (padded tiles load zeros, store nothing)
-  const int num_tiles = kMode == 3 ? s_tile_prefix[fp.num_groups]
-                                   : (kMC == 1 ? tiles_m * tiles_n : RB_CEIL_DIV(tiles_m * tiles_n, kMC) * kMC);
+  const int num_tiles = kMode == 3 ? s_tile_prefix[fp.num_groups] : tiles_m * tiles_n;
   // grouped tile -> (row start, row end, n0, B row offset)
   auto group_tile = [&](int tile, int& m0, int& m_end, int& n0, int& b_row0) {
     int g = 0;
@@ -113,15 +106,13 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tcgen05_kernel(const __grid_
     b_row0 = g * fp.group_b_rows;
   };
   const int num_kb = RB_CEIL_DIV(p.K, BK);
-  const uint32_t cta_rank = kMC == 1 ? 0u : (blockIdx.x % kMC);
-  constexpr uint16_t kMcMask = (uint16_t)((1u << kMC) - 1u);
 
   if (warp == 0 && lane == 0) {
     ptx::prefetch_tensormap(&tma_a);
     ptx::prefetch_tensormap(&tma_b);
     for (int i = 0; i < C::kStages; ++i) {
       ptx::mbar_init(ptx::smem_u32(&full_bar[i]), 1);
-      ptx::mbar_init(ptx::smem_u32(&empty_bar[i]), kMC);
+      ptx::mbar_init(ptx::smem_u32(&empty_bar[i]), 1);
     }
     for (int i = 0; i < 2; ++i) {
       ptx::mbar_init(ptx::smem_u32(&tmem_full[i]), 1);
@@ -135,7 +126,6 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tcgen05_kernel(const __grid_
   }
   ptx::tc_fence_before();
   __syncthreads();
-  if constexpr (kMC > 1) ptx::cluster_sync();  // peers' barriers must be initialised before any remote arrive / multicast
   ptx::tc_fence_after();
   const uint32_t tmem_base = *tmem_ptr;
 
@@ -158,9 +148,6 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tcgen05_kernel(const __grid_
           if constexpr (kAMN) {
 #pragma unroll
             for (int j = 0; j < BM / 64; ++j) ptx::tma_load_2d(sa + j * (BK * 128), &tma_a, fb, m0 + 64 * j, k0);
-          } else if constexpr (kMC > 1) {
-            constexpr int kRows = BM / kMC;  // my slice of the A tile, delivered to every CTA of the cluster
-            ptx::tma_load_2d_mcast(sa + cta_rank * (kRows * 128), &tma_a, fb, k0, m0 + (int)cta_rank * kRows, kMcMask);
           } else if constexpr (kMode == 2) {
             const int src = m0 / fp.rows_per_rank;  // rows_per_rank % BM == 0 (checked on the host)
             ptx::tma_load_2d(sa, &tma_a_peers.m[src], fb, k0, m0 - src * fp.rows_per_rank);
@@ -199,8 +186,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tcgen05_kernel(const __grid_
         if (ptx::elect_one()) {
 #pragma unroll
           for (int k = 0; k < BK / 16; ++k) ptx::tc_mma_f16(d_tmem, da + k * kAStep, db + k * kBStep, idesc, (kb | k) != 0 ? 1u : 0u);
-          if constexpr (kMC > 1) ptx::tc_commit_mcast(ptx::smem_u32(&empty_bar[stage]), kMcMask);
-          else ptx::tc_commit(ptx::smem_u32(&empty_bar[stage]));  // smem slot reusable once these MMAs retire
+          ptx::tc_commit(ptx::smem_u32(&empty_bar[stage]));  // smem slot reusable once these MMAs retire
         }
         __syncwarp();
         if (++stage == C::kStages) { stage = 0; phase ^= 1; }
@@ -273,7 +259,6 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tcgen05_kernel(const __grid_
 
   ptx::tc_fence_before();
   __syncthreads();
-  if constexpr (kMC > 1) ptx::cluster_sync();  // no CTA may exit while peers still multicast into / arrive on its smem
   if (warp == 1) {
     ptx::tc_fence_after();
     ptx::tmem_dealloc(tmem_base, C::kTmemCols);
@@ -606,37 +591,19 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_streamk_kernel(const __grid_
 static const FusedParams kNoFused{};
 static const TmaArray kNoPeers{};
 
-template <int BN, bool kAMN, bool kBMN, typename OutT, int kFmt, int kMC = 1, int kMode = 0>
+template <int BN, bool kAMN, bool kBMN, typename OutT, int kFmt, int kMode = 0>
 int launch(const CUtensorMap& ta, const CUtensorMap& tb, const Params& p, int num_sms, cudaStream_t s,
            const FusedParams& fp = kNoFused, const TmaArray& peers = kNoPeers) {
-  auto kern = gemm_tcgen05_kernel<BN, kAMN, kBMN, OutT, kFmt, kMC, kMode>;
+  auto kern = gemm_tcgen05_kernel<BN, kAMN, kBMN, OutT, kFmt, kMode>;
   static bool configured = false;
   if (!configured) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<BN>::kSmemBytes) != cudaSuccess) return -2;
     configured = true;
   }
   const int tiles = RB_CEIL_DIV(p.M, BM) * RB_CEIL_DIV(p.N, BN);
-  if constexpr (kMC == 1) {
-    // grouped: every group with rows has its own m-tiles, so the dense count is no bound; the caller passes min(upper bound, #SMs)
-    const int grid = kMode == 3 ? num_sms : (tiles < num_sms ? tiles : num_sms);
-    kern<<<grid, kThreads, Cfg<BN>::kSmemBytes, s>>>(ta, tb, p, fp, peers);
-  } else {
-    const int padded = RB_CEIL_DIV(tiles, kMC) * kMC;
-    const int cap = (num_sms / kMC) * kMC;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(padded < cap ? padded : cap);
-    cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = Cfg<BN>::kSmemBytes;
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = kMC;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    if (cudaLaunchKernelEx(&cfg, kern, ta, tb, p, fp, peers) != cudaSuccess) return -3;
-  }
+  // grouped: every group with rows has its own m-tiles, so the dense count is no bound; the caller passes min(upper bound, #SMs)
+  const int grid = kMode == 3 ? num_sms : (tiles < num_sms ? tiles : num_sms);
+  kern<<<grid, kThreads, Cfg<BN>::kSmemBytes, s>>>(ta, tb, p, fp, peers);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 
@@ -669,12 +636,7 @@ int dispatch_major(bool a_mn, bool b_mn, const CUtensorMap& ta, const CUtensorMa
 }
 
 template <typename OutT, int kFmt>
-int dispatch_bn(int bn, bool a_mn, bool b_mn, int mc, const CUtensorMap& ta, const CUtensorMap& tb, const Params& p, int sms, cudaStream_t s) {
-  if (mc == 4) {  // small-M K-major shapes only (checked by the caller)
-    if (bn == 32) return launch<32, false, false, OutT, kFmt, 4>(ta, tb, p, sms, s);
-    if (bn == 64) return launch<64, false, false, OutT, kFmt, 4>(ta, tb, p, sms, s);
-    return -6;
-  }
+int dispatch_bn(int bn, bool a_mn, bool b_mn, const CUtensorMap& ta, const CUtensorMap& tb, const Params& p, int sms, cudaStream_t s) {
   switch (bn) {
     case 256: return dispatch_major<256, OutT, kFmt>(a_mn, b_mn, ta, tb, p, sms, s);
     case 128: return dispatch_major<128, OutT, kFmt>(a_mn, b_mn, ta, tb, p, sms, s);
@@ -696,22 +658,17 @@ extern "C" {
 // bn = 0 picks the tile width from the problem size.
 int rb_gemm_tcgen05(const void* A, const void* B, void* C, const void* bias, int M, int N, int K, int64_t lda, int64_t ldb,
                     int64_t ldc, int a_mn, int b_mn, int in_dt, int out_dt, int accumulate, int bn, int num_sms, int mc_req, cudaStream_t s) {
-  static const int mc_env = [] { const char* e = getenv("REAL_GEMM_MULTICAST"); return e ? atoi(e) : 0; }();
   static const int cta2_env = [] { const char* e = getenv("REAL_GEMM_2CTA"); return e ? atoi(e) : 1; }();
-  // CTA-pair kernel (gemm_2cta.cu) for everything with at least two m-tiles: mc_req == 2 forces it, -1 follows the env default
+  // CTA-pair kernel (gemm_2cta.cu) for everything with at least two m-tiles: mc_req == 2 forces it, -1 follows the env default, any other value
+  // takes the plain tiles
   if ((mc_req == 2 || (mc_req < 0 && cta2_env != 0)) && M > BM && (bn == 0 || bn == 128 || bn == 256)) {
     const int rc = rb_gemm_2cta(A, B, C, bias, M, N, K, lda, ldb, ldc, a_mn, b_mn, in_dt, out_dt, accumulate, bn, num_sms, s);
     if (rc != -40) return rc;
   }
-  if (mc_req == 2) mc_req = 0;
-  const int mc_mode = mc_req >= 0 ? mc_req : mc_env;  // TMA-multicast clusters for small M: opt-in (measured slower than plain tiles so far)
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if (in_dt != 1 && in_dt != 2) return -10;
   if ((lda % 8) || (ldb % 8) || (reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15)) return -11;
   if (num_sms <= 0) num_sms = rb::kNumSMs;
-  if (bn == 0 && M <= BM && !a_mn && !b_mn && mc_mode != 0 && N >= 256) {
-    bn = 32;  // decode shapes: many small tiles balance the 148 SMs; A traffic is shared by TMA multicast
-  }
   if (bn == 0) {
     const int tm = RB_CEIL_DIV(M, BM);
     const int cands[4] = {256, 128, 64, 32};
@@ -723,18 +680,15 @@ int rb_gemm_tcgen05(const void* A, const void* B, void* C, const void* bias, int
     while (bn > N && bn > (b_mn ? 64 : 32)) bn >>= 1;
   }
   if (b_mn && bn < 64) return -12;
-  // decode-shaped problems (one m-tile, K-major operands): cluster of 4 CTAs shares the A tile by TMA multicast
-  int mc = 1;
-  if (M <= BM && !a_mn && !b_mn && bn <= 64 && RB_CEIL_DIV(N, bn) >= 8 && mc_mode != 0) mc = 4;
   CUtensorMap ta, tb;
   const int bf = in_dt == 1;
   bool ok = a_mn ? make_tmap(&ta, A, bf, (uint64_t)K, (uint64_t)M, (uint64_t)lda, 64, BK)
-                 : make_tmap(&ta, A, bf, (uint64_t)M, (uint64_t)K, (uint64_t)lda, BK, (uint32_t)(BM / mc));
+                 : make_tmap(&ta, A, bf, (uint64_t)M, (uint64_t)K, (uint64_t)lda, BK, (uint32_t)BM);
   ok = ok && (b_mn ? make_tmap(&tb, B, bf, (uint64_t)K, (uint64_t)N, (uint64_t)ldb, 64, BK)
                    : make_tmap(&tb, B, bf, (uint64_t)N, (uint64_t)K, (uint64_t)ldb, BK, (uint32_t)bn));
   if (!ok) return -13;
   Params p{C, bias, ldc, M, N, K, accumulate};
-#define RB_GO(OutT, FMT) return dispatch_bn<OutT, FMT>(bn, a_mn != 0, b_mn != 0, mc, ta, tb, p, num_sms, s)
+#define RB_GO(OutT, FMT) return dispatch_bn<OutT, FMT>(bn, a_mn != 0, b_mn != 0, ta, tb, p, num_sms, s)
   if (in_dt == 1) {
     if (out_dt == 1) RB_GO(__nv_bfloat16, 1);
     if (out_dt == 0) RB_GO(float, 1);
@@ -870,7 +824,7 @@ int rb_gemm_grouped(const void* A, const void* B, void* C, const int* group_offs
   // upper bound of the tile count (the exact number is only known on the device): grid = persistent CTAs
   const int64_t max_tiles = ((int64_t)RB_CEIL_DIV(M, BM) + G) * RB_CEIL_DIV(N, bn);
   const int grid_sms = (int)(max_tiles < num_sms ? max_tiles : num_sms);
-#define RB_G(BNV, BMN) return launch<BNV, false, BMN, __nv_bfloat16, 1, 1, 3>(ta, tb, p, grid_sms, s, fp, kNoPeers)
+#define RB_G(BNV, BMN) return launch<BNV, false, BMN, __nv_bfloat16, 1, 3>(ta, tb, p, grid_sms, s, fp, kNoPeers)
   if (bn == 256) { if (b_mn) RB_G(256, true); else RB_G(256, false); }
   else { if (b_mn) RB_G(128, true); else RB_G(128, false); }
 #undef RB_G
@@ -908,7 +862,7 @@ int rb_gemm_fused_tp(int mode, const void* A, const int64_t* peer_a, const void*
   }
   if (!ok) return -13;
   Params p{C, nullptr, ldc, M, N, K, 0};
-#define RB_F(BNV, BMN, MODE) return launch<BNV, false, BMN, __nv_bfloat16, 1, 1, MODE>(ta, tb, p, num_sms, s, fp, peers)
+#define RB_F(BNV, BMN, MODE) return launch<BNV, false, BMN, __nv_bfloat16, 1, MODE>(ta, tb, p, num_sms, s, fp, peers)
   if (mode == 1) {
     if (bn == 256) { if (b_mn) RB_F(256, true, 1); else RB_F(256, false, 1); }
     else { if (b_mn) RB_F(128, true, 1); else RB_F(128, false, 1); }

@@ -85,15 +85,18 @@ def test_gemm_strided_operand():
 
 @pytest.mark.parametrize("shape", [(128, 4096, 4096), (64, 12288, 4096), (128, 22016, 4096), (1, 4096, 512), (100, 11008, 1024),
                                    (128, 32000, 4096), (7, 264, 136)])
-def test_gemm_small_m_multicast(shape):
-    """M <= 128 takes the cluster / TMA-multicast variant (A tile shared by 4 CTAs)."""
+def test_gemm_small_m(shape):
+    """M <= 128 and K-major operands: the stream-K kernel, and the plain tiles that `mc` other than 2 asks for."""
     M, N, K = shape
     torch.manual_seed(5)
     a = torch.randn(M, K, device=DEV, dtype=torch.bfloat16)
     b = torch.randn(N, K, device=DEV, dtype=torch.bfloat16)
     for _ in range(3):  # repeated launches exercise barrier phase carry-over
         c = G.gemm(a, b)
-    torch.testing.assert_close(c.float(), a.float() @ b.float().t(), atol=K ** 0.5 * 0.05, rtol=2e-2)
+    ref = a.float() @ b.float().t()
+    torch.testing.assert_close(c.float(), ref, atol=K ** 0.5 * 0.05, rtol=2e-2)
+    for mc in (0, 1):
+        torch.testing.assert_close(G.gemm(a, b, mc=mc).float(), ref, atol=K ** 0.5 * 0.05, rtol=2e-2)
 
 
 @pytest.mark.parametrize("shape", [(128, 4096, 4096), (64, 4096, 11008), (17, 12288, 4096), (128, 22016, 4096), (1, 32000, 4096),

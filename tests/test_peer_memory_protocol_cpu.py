@@ -264,3 +264,18 @@ def test_streamk_without_rearm_breaks_the_second_replay():
     with pytest.raises(AssertionError):
         for seed in range(50):
             launch([list(f) for f in flags], seed)
+
+
+def test_no_load_is_sent_to_several_ctas_of_a_cluster():
+    """The kernels here read other GPUs' memory through TMA, and a TMA or bulk load of such memory must not be delivered to several CTAs.  No source
+    therefore has that form of load at all; tcgen05.commit's form, which only arrives on barriers, is allowed."""
+    from pathlib import Path
+
+    import realhf_b200
+    qualifier = ".multi" + "cast::cluster"
+    sources = [f for pat in ("*.cu", "*.cuh", "*.cpp", "*.h") for f in Path(realhf_b200.__file__).parent.rglob(pat)]
+    assert len(sources) > 30
+    for f in sources:
+        statements = f.read_text().split("asm")
+        bad = [s for s in statements if qualifier in s.split(";\n")[0] and "tcgen05.commit" not in s.split(";\n")[0]]
+        assert not bad, f"{f.name}: {bad[0][:200]}"
