@@ -20,6 +20,7 @@ from realhf_b200.api.model import (FinetuneSpec, GenerationHyperparameters, Mode
 from realhf_b200.engine.optim import FlatAdamW, OptimizerConfig
 from realhf_b200.models import generation as gen
 from realhf_b200.models.real_model import ModelOutput, ReaLModel
+from realhf_b200.ops import lib
 
 MAIN_KEY = "packed_input_ids"
 
@@ -58,12 +59,15 @@ class ReaLEngine(PipelinableEngine):
     def config(self):
         return self.module.config
 
-    def _check_ep(self):
-        """The fused expert-parallel exchange sizes its receive buffers for `cap_factor` x the balanced load and reports an
-        overflow through a device flag: read it once per engine call (the only host sync of the MoE path)."""
+    def _check_device_flags(self):
+        """What kernels report beside their outputs, looked at once per engine call.  The fused expert-parallel exchange sizes its receive buffers
+        for `cap_factor` x the balanced load and reports an overflow through a device flag (the only host sync of the MoE path); an attention
+        kernel that gave up a wait says so in host memory (no sync: one still running is seen by the next call)."""
         ep = getattr(self.ctx, "_fused_ep", None)
         if ep is not None:
             ep.raise_if_overflow()
+        if self.module.device.type == "cuda":
+            lib().attn_check()
 
     # ------------------------------------------------------------------ single-stage forward
     def _forward_mb(self, mb: SequenceSample) -> ModelOutput:
@@ -98,7 +102,7 @@ class ReaLEngine(PipelinableEngine):
                     stats[k] = stats[k] + (v.detach() if torch.is_tensor(v) else v) / len(mbs)
         ost = self.optim.step(version_steps)
         self.optim.end_call()
-        self._check_ep()
+        self._check_device_flags()
         stats = dict(stats)
         stats.update(ost)
         return stats
@@ -138,7 +142,7 @@ class ReaLEngine(PipelinableEngine):
             for mb in input_.split(min(n_mbs, input_.bs)):
                 out = self._forward_mb(mb)
                 outs.append(post_hook(out, mb) if post_hook is not None else out.logits)
-            self._check_ep()
+            self._check_device_flags()
             return aggregate_fn(outs) if len(outs) > 1 else outs[0]
         finally:
             if self.optim is not None:
@@ -164,6 +168,7 @@ class ReaLEngine(PipelinableEngine):
             outs.append(o)
         if gconfig.force_cudagraph_recapture:
             self._gen_state = None  # releases the KV cache between calls, like the reference
+        self._check_device_flags()
         return outs
 
 

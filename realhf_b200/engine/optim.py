@@ -388,12 +388,19 @@ class FlatAdamW:
         if self.nvls:
             torch.cuda.current_stream(self.flat_grad.device).wait_stream(self._comm_stream)
 
+    def _count_attention_failure(self):
+        """An attention kernel whose bounded wait ran out has left parts of its gradients unwritten.  Counted like an overflow before the
+        statistics are summed over the ranks, so that every rank skips this update; the host raises at its next attention call."""
+        if self._stats.is_cuda:
+            self._stats[1:2] += lib().attn_status(self._stats.device)
+
     def _step_zero3(self, version_steps: Optional[int]) -> Dict[str, torch.Tensor]:
         cfg, ctx = self.cfg, self.ctx
         z = self.z3
         z.finish_grads()
         self._stats.zero_()
         z.grad_sumsq(self._stats)
+        self._count_attention_failure()
         if ctx.model_group is not None and ctx.topo.world_size() > 1:
             dist.all_reduce(self._stats, group=ctx.model_group)
         inv_ls = 1.0 / self.loss_scale
@@ -427,6 +434,7 @@ class FlatAdamW:
         for (lo, hi), dup in zip(self.ranges, self._dup_idx):
             if dup is not None:
                 self._stats[0] -= self.flat_grad[lo:hi][dup].float().pow(2).sum()
+        self._count_attention_failure()
         if ctx.model_group is not None and ctx.topo.world_size() > 1:
             dist.all_reduce(self._stats, group=ctx.model_group)
         inv_ls = 1.0 / self.loss_scale

@@ -51,6 +51,7 @@ struct BwdParams {
   int T, B, nq, nkv, heads;   // heads: of this pass (key heads for dKV, query heads for dQ)
   float scale;
   int causal;
+  int* status = nullptr;   // set by the launch: rb_attn_status()
 };
 
 template <int kD> struct BCfg {
@@ -68,8 +69,6 @@ enum BBar { R_FULL = 0, R_EMPTY = 1, X_FULL = 2, X_EMPTY = X_FULL + kXStages, S_
 
 // One work item: sequence (first token, length), head and first resident row; L < 0 ends the CTA's loop.
 struct BItem { int tok0, L, head, r0; };
-
-__device__ int g_wait_error = 0;
 
 // tma_r1 / tma_r2: resident operands (box 64 cols x 128 rows); tma_x1 / tma_x2: streamed operands (box 64 x 64).
 //   kDKV: r1 = K, r2 = V (kv-head columns), x1 = Q, x2 = dO (q-head columns).   !kDKV: r1 = Q, r2 = dO, x1 = K, x2 = V.
@@ -414,11 +413,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) attn_bwd_kernel(const __grid_c
 
   ptx::tc_fence_before();
   __syncthreads();
-  if (*dead) {
-    if (threadIdx.x == 0) g_wait_error = 1;
-    for (int i = 0; i < 1000; ++i) __nanosleep(1000);
-    __syncthreads();
-  }
+  rb::report_given_up(dead, p.status);
   if (warp == 1) {
     ptx::tc_fence_after();
     ptx::tmem_dealloc(tmem_base, 512);
@@ -468,6 +463,7 @@ int launch_bwd(const CUtensorMap& r1, const CUtensorMap& r2, const CUtensorMap& 
     attr_set = true;
   }
   p.heads = kDKV ? p.nkv : p.nq;
+  if ((p.status = rb_attn_status()) == nullptr) return -34;
   // the sequences' lengths are on the device: sum of ceil(L / kR) is at most (T + (kR - 1) B) / kR
   const int64_t n = (p.T + (int64_t)(kR - 1) * p.B) / kR * p.heads;
   if (n <= 0 || n > 0x7fffffff) return -33;
@@ -500,13 +496,6 @@ int run_bwd(const void* q, const void* k, const void* v, const void* out, const 
 }
 
 }  // namespace
-
-extern "C" int rb_attn_bwd_wait_error() {
-  int v = 0, zero = 0;
-  if (cudaMemcpyFromSymbol(&v, g_wait_error, sizeof(int)) != cudaSuccess) return -1;
-  if (v != 0) cudaMemcpyToSymbol(g_wait_error, &zero, sizeof(int));
-  return v;
-}
 
 // All tensors are [T, heads, hd] views with unit stride over hd and packed heads; `delta` is an [nq, T] fp32 scratch tensor.
 // dt: 1 = bf16, 2 = fp16.  Returns 0 or a negative code.

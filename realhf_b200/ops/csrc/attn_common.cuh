@@ -27,7 +27,29 @@ struct AttnParams {
   const float* bias = nullptr;   // [nq, bias_ld], the first n_bias columns are used; distances beyond read the last one
   int n_bias = 0, bias_ld = 0;
   int B = 0, pair_heads = 0, n_head_units = 0;   // set by the launch: sequences, tile pairs over heads, work units per row block
+  int* status = nullptr;         // set by the launch: rb_attn_status()
 };
+
+}  // namespace rb
+
+// The process's status word of the attention kernels, in pinned host memory that every device can write (null if it cannot be had): not 0 once a
+// bounded wait has run out, until `rb_attn_wait_error` clears it.  The host reads it without a CUDA call (the bindings do before every launch), the
+// optimizer's kernels read it in stream order.
+extern "C" int* rb_attn_status();
+
+namespace rb {
+
+// At the end of a CTA (all threads): if one of its waits ran out, what it had claimed is missing from the outputs.  Tell the host, and let copies land.
+RB_DEVICE void report_given_up(volatile uint32_t* dead, int* status) {
+  if (*dead) {
+    if (threadIdx.x == 0) {
+      *reinterpret_cast<volatile int*>(status) = 1;
+      __threadfence_system();
+    }
+    for (int i = 0; i < 1000; ++i) __nanosleep(1000);
+    __syncthreads();
+  }
+}
 
 }  // namespace rb
 
@@ -38,7 +60,7 @@ using rb::AttnParams;
 constexpr int kMaxSmem = 227 * 1024;
 
 // Every wait is bounded: a wait that runs out sets the CTA's `dead` flag (all later waits of the CTA then return at once), and the
-// kernel ends normally after a pause that lets its own copies land; `rb_attn_wait_error` tells the host.
+// kernel ends normally after a pause that lets its own copies land; `report_given_up` tells the host.
 constexpr int kWaitPolls = 1 << 20;
 
 RB_DEVICE void bounded_wait(uint32_t bar, uint32_t parity, volatile uint32_t* dead) {

@@ -44,8 +44,6 @@ constexpr int kBiasFront = kBKV - 1, kBiasPad = 2 * kBKV + kBKV;   // table entr
 enum Bar { Q_FULL = 0, K_FULL = 1, K_EMPTY = 3, V_FULL = 5, V_EMPTY = 7, S_FULL = 9, S_EMPTY = 11, P_FULL = 13, P_EMPTY = 14,
            O_FULL = 15, O_EMPTY = 17, NUM_BARS = 19 };
 
-__device__ int g_wait_error = 0;
-
 template <int kD, typename T, int kFmt, bool kShared>
 __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_bias_kernel(const __grid_constant__ CUtensorMap tma_q,
                                                                    const __grid_constant__ CUtensorMap tma_k,
@@ -319,11 +317,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_bias_kernel(const __
 
   ptx::tc_fence_before();
   __syncthreads();
-  if (*dead) {
-    if (threadIdx.x == 0) g_wait_error = 1;
-    for (int i = 0; i < 1000; ++i) __nanosleep(1000);
-    __syncthreads();
-  }
+  rb::report_given_up(dead, p.status);
   if (warp == 1) {
     ptx::tc_fence_after();
     ptx::tmem_dealloc(tmem_base, 512);
@@ -331,10 +325,11 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_bias_kernel(const __
 }
 
 template <int kD, typename T, int kFmt, bool kShared>
-int launch_bias(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const AttnParams& p, int B, int max_seqlen, cudaStream_t s) {
+int launch_bias(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, AttnParams p, int B, int max_seqlen, cudaStream_t s) {
   auto kern = attn_fwd_bias_kernel<kD, T, kFmt, kShared>;
   const int smem = ACfg<kD, kD, kShared>::kSmemBytes + (p.n_bias + kBiasPad) * 4;
   if (smem > kMaxSmem) return -32;
+  if ((p.status = rb_attn_status()) == nullptr) return -34;
   static bool attr_set = false;
   if (!attr_set) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem) != cudaSuccess) return -30;
@@ -346,13 +341,6 @@ int launch_bias(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap&
 }
 
 }  // namespace
-
-extern "C" int rb_attn_bias_wait_error() {
-  int v = 0, zero = 0;
-  if (cudaMemcpyFromSymbol(&v, g_wait_error, sizeof(int)) != cudaSuccess) return -1;
-  if (v != 0) cudaMemcpyToSymbol(g_wait_error, &zero, sizeof(int));
-  return v;
-}
 
 // Called by rb_attn_fwd_sink: tensor maps of boxes 64 columns x 128 rows (mq, mk) and 64 x 64 (mv).
 extern "C" int rb_attn_fwd_bias(const CUtensorMap* mq, const CUtensorMap* mk, const CUtensorMap* mv, const AttnParams* p, int B, int hd, int max_seqlen,

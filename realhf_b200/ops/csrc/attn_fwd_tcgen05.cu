@@ -61,8 +61,6 @@ template <int kD, int kDV> struct FCfg {
 enum FBar { Q_FULL = 0, Q_EMPTY = 2, KV_FULL = 4, KV_EMPTY = 8, S_FULL = 12, P_FULL = 14, O_FULL = 16, O_EMPTY = 18, IT_FULL = 20, IT_EMPTY = 22,
             CLC_FULL = 24, F_NUM_BARS = 25 };
 
-__device__ int g_wait_error = 0;
-
 // One work item: sequence (first token, length), heads and query tiles of the two tiles (tile 1 < 0: absent); L < 0 ends the CTA's loop.
 struct Item { int tok0, L, head0, head1, qt0, qt1; };
 
@@ -478,11 +476,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) attn_fwd_kernel(const __grid_c
 
   ptx::tc_fence_before();
   __syncthreads();
-  if (*dead) {
-    if (threadIdx.x == 0) g_wait_error = 1;
-    for (int i = 0; i < 1000; ++i) __nanosleep(1000);
-    __syncthreads();
-  }
+  rb::report_given_up(dead, p.status);
   if (warp == 8) {
     ptx::tc_fence_after();
     ptx::tmem_dealloc(tmem_base, 512);
@@ -500,6 +494,7 @@ int launch_attn_fwd(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensor
     attr_set = true;
   }
   p.B = B;
+  if ((p.status = rb_attn_status()) == nullptr) return -34;
   p.pair_heads = (p.nq / p.nkv) % 2 == 0;
   p.n_head_units = p.pair_heads ? p.nq / 2 : p.nq;
   // the sequences' lengths are on the device: sum of ceil(L / rows) is at most (T + (rows - 1) B) / rows
@@ -512,18 +507,29 @@ int launch_attn_fwd(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensor
 
 }  // namespace
 
-extern "C" int rb_attn_bias_wait_error();
-extern "C" int rb_attn_bwd_wait_error();
 extern "C" int rb_attn_fwd_bias(const CUtensorMap* mq, const CUtensorMap* mk, const CUtensorMap* mv, const AttnParams* p, int B, int hd, int max_seqlen,
                                 int kv_shared, int bf, cudaStream_t s);
 
-// 1 if a bounded wait of the kernels ran out since the last call (synchronises; for diagnostics)
+extern "C" int* rb_attn_status() {
+  static int* const word = [] {
+    int* w = nullptr;
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;      // the first call may come while a graph is being captured
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (cudaHostAlloc(reinterpret_cast<void**>(&w), sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) w = nullptr;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (w != nullptr) *w = 0;
+    return w;
+  }();
+  return word;
+}
+
+// 1 if a bounded wait of the kernels ran out since the last call (synchronises, and clears the word)
 extern "C" int rb_attn_wait_error() {
-  int v = 0, zero = 0;
-  if (cudaMemcpyFromSymbol(&v, g_wait_error, sizeof(int)) != cudaSuccess) return -1;
-  if (v != 0) cudaMemcpyToSymbol(g_wait_error, &zero, sizeof(int));
-  const int b = rb_attn_bias_wait_error(), c = rb_attn_bwd_wait_error();
-  return b != 0 ? b : c != 0 ? c : v;
+  volatile int* w = rb_attn_status();
+  if (w == nullptr || cudaDeviceSynchronize() != cudaSuccess) return -1;
+  const int v = *w;
+  *w = 0;
+  return v;
 }
 
 // q / k / v: [T, heads, hd] views (unit stride over hd, `heads * hd` contiguous columns, row pitch *_ld elements) -- e.g. the

@@ -87,6 +87,21 @@ std::vector<Tensor> sample(const Tensor& logits, const c10::optional<Tensor>& un
   return {tok, lp, mask};
 }
 
+extern "C" int* rb_attn_status();
+
+// Raises if a bounded wait of an earlier attention kernel ran out (a plain read of host memory): parts of that kernel's outputs were never written.
+void attn_check() {
+  const volatile int* w = rb_attn_status();
+  TORCH_CHECK(w == nullptr || *w == 0, "an earlier attention kernel gave up waiting and left parts of its outputs unwritten (attn_wait_error() clears this)");
+}
+
+// The status word as an int32 [1] tensor on `device` (its kernels read it in stream order); no copy.
+Tensor attn_status(at::Device device) {
+  int* w = rb_attn_status();
+  TORCH_CHECK(w != nullptr && device.is_cuda(), "attn_status: no status word");
+  return at::for_blob(w, {1}).options(at::TensorOptions().dtype(at::kInt).device(device)).target_device(device).make_tensor();
+}
+
 extern "C" int rb_attn_fwd(const void* q, const void* k, const void* v, void* out, float* lse, const int* cu_seqlens, int64_t q_ld,
                            int64_t k_ld, int64_t v_ld, int64_t out_ld, int T, int B, int nq, int nkv, int hd, int max_seqlen,
                            float scale, int causal, int dt, cudaStream_t s);
@@ -112,6 +127,7 @@ std::vector<Tensor> attn_fwd_window(const Tensor& q, const Tensor& k, const Tens
   const int64_t T = q.size(0), nq = q.size(1), hd = q.size(2), nkv = k.size(1);
   for (const Tensor* t : {&q, &k, &v}) TORCH_CHECK(t->stride(2) == 1 && t->stride(1) == hd && t->size(0) == T && t->size(2) == hd);
   TORCH_CHECK(v.size(1) == nkv && k.scalar_type() == q.scalar_type() && v.scalar_type() == q.scalar_type());
+  attn_check();
   TORCH_CHECK(cu_seqlens.scalar_type() == at::kInt && cu_seqlens.is_contiguous() && cu_seqlens.is_cuda());
   c10::cuda::CUDAGuard guard(q.device());
   auto out = at::empty({T, nq, hd}, q.options());
@@ -140,6 +156,7 @@ void attn_bwd(const Tensor& dout, const Tensor& q, const Tensor& k, const Tensor
                 t->scalar_type() == q.scalar_type());
   TORCH_CHECK(out.size(1) == nq && dout.size(1) == nq && dq.size(1) == nq && v.size(1) == nkv && dk.size(1) == nkv && dv.size(1) == nkv);
   TORCH_CHECK(lse.scalar_type() == at::kFloat && lse.is_contiguous() && lse.size(0) == nq && lse.size(1) == T);
+  attn_check();
   TORCH_CHECK(cu_seqlens.scalar_type() == at::kInt && cu_seqlens.is_contiguous() && cu_seqlens.is_cuda());
   c10::cuda::CUDAGuard guard(q.device());
   auto delta = at::empty({nq, T}, q.options().dtype(at::kFloat));
@@ -191,6 +208,8 @@ void sample_graph(const Tensor& logits, Tensor tok_hist, Tensor lp_hist, const c
 
 void register_attn_ops(torch::Library& m) {
   m.def("sample_graph(Tensor logits, Tensor(a!) tok_hist, Tensor(b!) lp_hist, Tensor(c!)? mask_hist, Tensor(d!) unfinished, Tensor(e!) step_rows, Tensor(f!) input_ids, Tensor(g!) cache_lens, Tensor seed, int min_new_tokens, int top_k, float top_p, float inv_temp, int eos_id, bool greedy, int pad_id) -> ()", &sample_graph);
+  m.def("attn_check() -> ()", &attn_check);
+  m.def("attn_status(Device device) -> Tensor", &attn_status);
   m.def("attn_bwd(Tensor dout, Tensor q, Tensor k, Tensor v, Tensor out, Tensor lse, Tensor(a!) dq, Tensor(b!) dk, Tensor(c!) dv, Tensor cu_seqlens, int max_seqlen, float scale, bool causal) -> ()", &attn_bwd);
   m.def("attn_fwd(Tensor q, Tensor k, Tensor v, Tensor cu_seqlens, int max_seqlen, float scale, bool causal) -> Tensor[]", &attn_fwd);
   m.def("attn_fwd_window(Tensor q, Tensor k, Tensor v, Tensor cu_seqlens, int max_seqlen, float scale, bool causal, int window) -> Tensor[]", &attn_fwd_window);

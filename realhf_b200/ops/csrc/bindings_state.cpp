@@ -66,6 +66,8 @@ int rb_branch_norm(void*, int, const void*, int64_t, const void*, int64_t, const
                    const void*, int, float, void*, int, int64_t, int, float, cudaStream_t);
 }
 
+void attn_check();      // bindings_attn.cpp
+
 namespace {
 
 void embed_sinusoid(const Tensor& ids, const Tensor& wte, const Tensor& pos, const OptT& slots, const Tensor& inv_freq, Tensor out) {
@@ -183,6 +185,7 @@ void sink_window_attention_tc(const Tensor& qkvg, const Tensor& vn, Tensor out, 
   TORCH_CHECK(vn.scalar_type() == qkvg.scalar_type() && out.scalar_type() == qkvg.scalar_type() && cu.scalar_type() == at::kInt);
   const Gate ga = gate_arg(gate, element_gate, qkvg, T, H, dv);
   const Bias bi = bias_arg(bias, H);
+  attn_check();
   c10::cuda::CUDAGuard g(qkvg.device());
   const char* base = static_cast<const char*>(qkvg.data_ptr());
   const int es = (int)qkvg.element_size();

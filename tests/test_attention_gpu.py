@@ -186,3 +186,41 @@ def test_attn_fwd_tile_pairs(heads, lens, form):
     eps = 2.0 ** (-8 if dt == torch.bfloat16 else -11)
     assert ((out.double() - ref).abs() <= eps * ref.abs() + eps * mag + 1e-6).all()
     torch.testing.assert_close(lse.double(), rlse, atol=2e-5, rtol=2e-6)
+
+
+def test_a_wait_that_ran_out_is_raised_and_the_update_skipped():
+    """The status word as a kernel leaves it whose bounded wait ran out (set here by a copy): the next attention call of either direction and the
+    engine raise, the optimizer leaves the parameters alone, and clearing the word makes everything run again."""
+    from realhf_b200.api.config import ModelName
+    from realhf_b200.api.model import FinetuneSpec, Model, ReaLModelConfig
+    from realhf_b200.engine.engine import TrainBackend
+    from realhf_b200.models.real_model import ReaLModel
+    dev = torch.device("cuda", 0)
+    cfg = ReaLModelConfig(n_layers=1, n_kv_heads=2, n_q_heads=2, hidden_dim=128, intermediate_dim=256, vocab_size=512, n_positions=64, embd_pdrop=0.0,
+                          resid_pdrop=0.0, attn_pdrop=0.0, activation_function="silu", layer_norm_type="rms", mlp_type="llama", apply_rotary=True)
+    m = ReaLModel(cfg, dtype=torch.bfloat16, device=dev).init_random_fast()
+    engine = TrainBackend(optimizer=dict(lr=1e-2, warmup_steps_proportion=0.0)).initialize(Model(ModelName("actor", 0), m, None, dev),
+                                                                                          FinetuneSpec(1, 10, 10)).module
+    opt = engine.optim
+    q, k, v = (torch.randn(40, 2, 64, device=DEV, dtype=torch.bfloat16) for _ in range(3))
+    cu = torch.tensor([0, 40], dtype=torch.int32, device=DEV)
+    fwd = lambda: lib().attn_fwd(q, k, v, cu, 40, 0.125, True)
+    out, lse = fwd()
+    bwd = lambda: lib().attn_bwd(out, q, k, v, out, lse, torch.empty_like(q), torch.empty_like(k), torch.empty_like(v), cu, 40, 0.125, True)
+
+    def step():
+        opt.zero_grad()
+        opt.flat_grad.fill_(1e-2)
+        return float(opt.step()["skipped"])
+    assert lib().attn_wait_error() == 0
+    word = lib().attn_status(dev)
+    word.fill_(1)
+    before = m.flat_param.detach().clone()
+    assert step() == 1.0 and torch.equal(m.flat_param, before)
+    for call in (fwd, bwd, engine._check_device_flags):
+        with pytest.raises(RuntimeError, match="gave up"):
+            call()
+    assert lib().attn_wait_error() == 1 and lib().attn_wait_error() == 0 and int(word) == 0
+    assert step() == 0.0 and not torch.equal(m.flat_param, before)
+    fwd(), bwd(), engine._check_device_flags()
+    torch.cuda.synchronize()
