@@ -15,8 +15,8 @@
 // Kernels on the decode path are launched with programmatic dependent launch (they signal their successors at once and wait for
 // their predecessor before the first global access), like the framework's other decode kernels.
 //   delta_rule       the recurrence.  A column of S depends only on its own v column, so columns are independent: a thread group of
-//                    LPC lanes owns NC columns (16 state rows of each per lane in registers), a CTA 128 / LPC * NC columns of one
-//                    (sequence, head).  q, k, v, beta, g of 8 tokens at a time are staged in shared memory.  Packed form: S starts
+//                    LPC lanes owns NC columns (16 state rows of each per lane in registers) or one (32 or 64 rows), a CTA all its groups' columns
+//                    of one (sequence, head).  q, k, v, beta, g of 8 tokens at a time are staged in shared memory.  Packed form: S starts
 //                    at zero and the final S goes to s_state[slot]; step form: S is loaded from and stored to s_state[slot].
 //   gated_head_norm  o / sqrt(mean(o^2) + eps) * w * silu(gate) or sigmoid(gate) per (token, head) -> model type.
 #include "anytype.cuh"
@@ -241,7 +241,7 @@ struct ScanParams {
   int H, G, d, dv, step;
 };
 
-// A group of LPC lanes owns NC neighbouring columns of the state: lane l holds their rows ((e / 4) * LPC + l) * 4 + e % 4, e = 0 .. 15, so that its q / k
+// Packed form.  A group of LPC lanes owns NC neighbouring columns of the state: lane l holds their rows ((e / 4) * LPC + l) * 4 + e % 4, e = 0 .. 15, so that its q / k
 // operands are four aligned float4 reads of shared memory each per token, used for all NC columns.  kChan: a decay per state row, staged beside q and k.
 //
 // What bounds it: a token is one step of a serial chain, so what counts is its latency and, with few sequences, the shared-memory port and the fp32
@@ -283,12 +283,11 @@ __global__ void __launch_bounds__(kScanThreads, LPC <= 8 ? 3 : 2) delta_rule_ker
   const int g = h / (p.H / p.G), d = p.d, dv = p.dv;
   const int nqk = p.G * d, C = 2 * nqk + p.H * dv, UW = C + p.H + (kChan ? p.H * d : p.H);
   const int tid = threadIdx.x, l = tid % LPC, lcol = tid / LPC * NC, col = c0 + lcol, warp = tid >> 5, lane = tid & 31;
-  int t0, t1;
   rb::pdl_trigger();
   rb::pdl_wait();
-  if (p.step) { t0 = seq; t1 = seq + 1; } else { t0 = p.cu[seq]; t1 = p.cu[seq + 1]; }
+  const int t0 = p.cu[seq], t1 = p.cu[seq + 1];
   if (t1 <= t0) return;
-  const int slot = p.s_state == nullptr ? -1 : (p.slots ? p.slots[seq] : (p.step ? seq : -1));
+  const int slot = p.s_state == nullptr || p.slots == nullptr ? -1 : p.slots[seq];
   float* S_g = slot >= 0 ? p.s_state + (((int64_t)slot * p.H + h) * d) * dv : nullptr;
   constexpr int dpad = kRows * LPC;               // rows >= d hold zeros and read zero q / k
   constexpr int kBuf = (kChan ? 3 : 2) * kTok * dpad + kTok * NCOL + 2 * kTok;   // floats of one staging buffer: q, k, v, (beta, g), row decays
@@ -298,12 +297,7 @@ __global__ void __launch_bounds__(kScanThreads, LPC <= 8 ? 3 : 2) delta_rule_ker
 #pragma unroll
   for (int j = 0; j < NC; ++j)
 #pragma unroll
-    for (int e = 0; e < kRows; e += 2) {
-      float z[2];
-#pragma unroll
-      for (int i = 0; i < 2; ++i) z[i] = (p.step && S_g && col + j < dv && row_of(e + i) < d) ? S_g[(int64_t)row_of(e + i) * dv + col + j] : 0.f;
-      Z[j][e / 2] = pair_of(z[0], z[1]);
-    }
+    for (int e = 0; e < kRows / 2; ++e) Z[j][e] = 0;
   // The inputs of the next 8 tokens are fetched into registers while the current 8 are processed out of shared memory (two staging buffers).
   float rq[NQ], rk[NQ], rg[kChan ? NQ : 1], rv[NV], rb = 0.f;
   auto fetch = [&](int tb) {
@@ -454,6 +448,130 @@ __global__ void __launch_bounds__(kScanThreads, LPC <= 8 ? 3 : 2) delta_rule_ker
   }
 }
 
+// Step form: one token per row, and reading and writing the state is all the work.  A thread group of LPC lanes owns one column (32 or 64 state rows
+// per lane), so that every access of a warp to the state covers whole 32-byte sectors.  (With the packed form's eight lanes and four columns an access
+// touched 16 sectors for a quarter each: 16 heads x 128 x 128, 1 / 16 / 128 rows 6.1 / 17.9 / 110 us, against 3.8 / 8.9 / 67.6 this way.)
+// Row mapping: lane l of a column's LPC lanes holds the state rows ((e / 4) * LPC + l) * 4 + e % 4, e = 0 .. kEPL - 1, so that its q / k
+// operands are 8 aligned float4 reads of shared memory per token (the lanes of a column read neighbouring float4s, the columns of
+// a warp the same ones).  Dot products run on four independent accumulators.  kChan: a decay per state row, staged beside q and k.
+template <int LPC, int kEPL, bool kChan>
+__global__ void __launch_bounds__(kScanThreads, kEPL == 32 ? 3 : 2) delta_column_kernel(ScanParams p) {
+  constexpr int NCOL = kScanThreads / LPC;
+  extern __shared__ __align__(16) float sm[];
+  const int seq = blockIdx.x, h = blockIdx.y, c0 = blockIdx.z * NCOL;
+  const int g = h / (p.H / p.G), d = p.d, dv = p.dv;
+  const int nqk = p.G * d, C = 2 * nqk + p.H * dv, UW = C + p.H + (kChan ? p.H * d : p.H);
+  const int tid = threadIdx.x, l = tid % LPC, col = c0 + tid / LPC;
+  const bool active = col < dv;
+  int t0, t1;
+  rb::pdl_trigger();
+  rb::pdl_wait();
+  if (p.step) { t0 = seq; t1 = seq + 1; } else { t0 = p.cu[seq]; t1 = p.cu[seq + 1]; }
+  if (t1 <= t0) return;
+  const int slot = p.s_state == nullptr ? -1 : (p.slots ? p.slots[seq] : (p.step ? seq : -1));
+  float* S_g = slot >= 0 ? p.s_state + (((int64_t)slot * p.H + h) * d) * dv : nullptr;
+  constexpr int dpad = kEPL * LPC;                // rows >= d hold zeros and read zero q / k
+  constexpr int kBuf = (kChan ? 3 : 2) * kTok * dpad + kTok * NCOL + 2 * kTok;   // floats of one staging buffer: q, k, v, (beta, g), row decays
+  constexpr int NQ = kTok * dpad / kScanThreads, NV = (kTok * NCOL + kScanThreads - 1) / kScanThreads;
+  auto row_of = [&](int e) { return ((e >> 2) * LPC + l) * 4 + (e & 3); };
+  float S[kEPL];
+#pragma unroll
+  for (int e = 0; e < kEPL; ++e) {
+    const int row = row_of(e);
+    S[e] = (p.step && S_g && active && row < d) ? S_g[(int64_t)row * dv + col] : 0.f;
+  }
+  // The inputs of the next 8 tokens are fetched into registers while the current 8 are processed out of shared memory (two
+  // staging buffers, one barrier per chunk).
+  float rq[NQ], rk[NQ], rg[kChan ? NQ : 1], rv[NV], rb = 0.f;
+  auto fetch = [&](int tb) {
+    const int nt = min(kTok, t1 - tb);
+#pragma unroll
+    for (int i = 0; i < NQ; ++i) {
+      const int idx = tid + i * kScanThreads, tt = idx / dpad, e = idx % dpad;
+      const bool ok = tt < nt && e < d;
+      const float* row = p.u + (int64_t)(tb + tt) * UW;
+      rq[i] = ok ? row[g * d + e] : 0.f;
+      rk[i] = ok ? row[nqk + g * d + e] : 0.f;
+      if constexpr (kChan) rg[i] = ok ? row[C + p.H + h * d + e] : 0.f;
+    }
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      const int idx = tid + i * kScanThreads, tt = idx / NCOL, c = c0 + idx % NCOL;
+      rv[i] = (idx < kTok * NCOL && tt < nt && c < dv) ? p.u[(int64_t)(tb + tt) * UW + 2 * nqk + h * dv + c] : 0.f;
+    }
+    rb = (tid < nt * 2 && !(kChan && (tid & 1))) ? p.u[(int64_t)(tb + tid / 2) * UW + C + (tid & 1) * p.H + h] : 0.f;
+  };
+  auto stage = [&](float* buf) {
+#pragma unroll
+    for (int i = 0; i < NQ; ++i) { buf[tid + i * kScanThreads] = rq[i]; buf[kTok * dpad + tid + i * kScanThreads] = rk[i]; }
+#pragma unroll
+    for (int i = 0; i < NV; ++i)
+      if (tid + i * kScanThreads < kTok * NCOL) buf[2 * kTok * dpad + tid + i * kScanThreads] = rv[i];
+    if (tid < 2 * kTok) buf[2 * kTok * dpad + kTok * NCOL + tid] = rb;
+    if constexpr (kChan) {
+#pragma unroll
+      for (int i = 0; i < NQ; ++i) buf[2 * kTok * dpad + kTok * NCOL + 2 * kTok + tid + i * kScanThreads] = rg[i];
+    }
+  };
+  fetch(t0);
+  int which = 0;
+  for (int tb = t0; tb < t1; tb += kTok, which ^= 1) {
+    const int nt = min(kTok, t1 - tb);
+    float* buf = sm + which * kBuf;
+    stage(buf);
+    __syncthreads();
+    if (tb + kTok < t1) fetch(tb + kTok);
+    const float* qs = buf;
+    const float* ks = buf + kTok * dpad;
+    const float* vs = ks + kTok * dpad;
+    const float* bg = vs + kTok * NCOL;
+    const float* gs = bg + 2 * kTok;                // kChan: [kTok][dpad]
+    for (int tt = 0; tt < nt; ++tt) {
+      const float beta = bg[tt * 2], gg = bg[tt * 2 + 1];
+      const float4* kq = reinterpret_cast<const float4*>(ks + tt * dpad) + l;
+      const float4* qq = reinterpret_cast<const float4*>(qs + tt * dpad) + l;
+      const float4* dg = reinterpret_cast<const float4*>(gs + tt * dpad) + l;
+      float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
+#pragma unroll
+      for (int e4 = 0; e4 < kEPL / 4; ++e4) {
+        const float4 kk = kq[e4 * LPC];
+        if constexpr (kChan) {
+          const float4 g4 = dg[e4 * LPC];
+          S[e4 * 4] *= g4.x; S[e4 * 4 + 1] *= g4.y; S[e4 * 4 + 2] *= g4.z; S[e4 * 4 + 3] *= g4.w;
+        } else {
+          S[e4 * 4] *= gg; S[e4 * 4 + 1] *= gg; S[e4 * 4 + 2] *= gg; S[e4 * 4 + 3] *= gg;
+        }
+        a0 = fmaf(S[e4 * 4], kk.x, a0); a1 = fmaf(S[e4 * 4 + 1], kk.y, a1);
+        a2 = fmaf(S[e4 * 4 + 2], kk.z, a2); a3 = fmaf(S[e4 * 4 + 3], kk.w, a3);
+      }
+      float acc = (a0 + a1) + (a2 + a3);
+#pragma unroll
+      for (int off = 1; off < LPC; off <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
+      const float w = beta * (vs[tt * NCOL + tid / LPC] - acc);
+      a0 = a1 = a2 = a3 = 0.f;
+#pragma unroll
+      for (int e4 = 0; e4 < kEPL / 4; ++e4) {
+        const float4 kk = kq[e4 * LPC], q4 = qq[e4 * LPC];
+        S[e4 * 4] = fmaf(kk.x, w, S[e4 * 4]); S[e4 * 4 + 1] = fmaf(kk.y, w, S[e4 * 4 + 1]);
+        S[e4 * 4 + 2] = fmaf(kk.z, w, S[e4 * 4 + 2]); S[e4 * 4 + 3] = fmaf(kk.w, w, S[e4 * 4 + 3]);
+        a0 = fmaf(S[e4 * 4], q4.x, a0); a1 = fmaf(S[e4 * 4 + 1], q4.y, a1);
+        a2 = fmaf(S[e4 * 4 + 2], q4.z, a2); a3 = fmaf(S[e4 * 4 + 3], q4.w, a3);
+      }
+      float ov = (a0 + a1) + (a2 + a3);
+#pragma unroll
+      for (int off = 1; off < LPC; off <<= 1) ov += __shfl_xor_sync(0xffffffffu, ov, off);
+      if (active && l == 0) p.o[((int64_t)(tb + tt) * p.H + h) * dv + col] = ov;
+    }
+  }
+  if (S_g && active) {
+#pragma unroll
+    for (int e = 0; e < kEPL; ++e) {
+      const int row = row_of(e);
+      if (row < d) S_g[(int64_t)row * dv + col] = S[e];
+    }
+  }
+}
+
 // Head sizes in whole fours up to 128 CH, aligned: a warp takes 4 / CH rows (token, head) and has all their loads in flight before the first sum
 // (8 sequences of 700..1024 tokens, 16 heads x 128: 34 us after the recurrence with a row a warp, o read twice and the gate
 // behind the sum, 26 us this way).
@@ -553,12 +671,30 @@ static int launch_delta_rule(const ScanParams& p, int n_seqs, cudaStream_t s) {
   return rb::launch_pdl(kern, dim3(n_seqs, p.H, RB_CEIL_DIV(p.dv, ncol)), dim3(kScanThreads), smem, s, p) == cudaSuccess ? 0 : -3;
 }
 
+template <int LPC, int EPL, bool CHAN>
+static int launch_delta_column(const ScanParams& p, int n_seqs, cudaStream_t s) {
+  constexpr int ncol = kScanThreads / LPC;
+  constexpr size_t smem = 2 * sizeof(float) * ((size_t)(CHAN ? 3 : 2) * kTok * EPL * LPC + (size_t)kTok * ncol + 2 * kTok);   // two staging buffers
+  auto kern = delta_column_kernel<LPC, EPL, CHAN>;
+  if (smem > 48 * 1024 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return -4;
+  return rb::launch_pdl(kern, dim3(n_seqs, p.H, RB_CEIL_DIV(p.dv, ncol)), dim3(kScanThreads), smem, s, p) == cudaSuccess ? 0 : -3;
+}
+
 // channel: u rows hold a decay per state row (H * d numbers) instead of one per head
 extern "C" int rb_delta_rule(const float* u, float* o, const int* cu, float* s_state, const int* slots, int n_seqs, int H, int G, int d, int dv,
                              int step, int channel, cudaStream_t s) {
   if (n_seqs == 0) return 0;
   if (d > 512 || H % G) return -1;
   ScanParams p{u, o, cu, s_state, slots, H, G, d, dv, step};
+  if (step) {       // (lanes per column, state rows per lane)
+#define RB_L(LPC, EPL) return channel ? launch_delta_column<LPC, EPL, true>(p, n_seqs, s) : launch_delta_column<LPC, EPL, false>(p, n_seqs, s)
+    if (d <= 32) { RB_L(1, 32); }
+    if (d <= 64) { RB_L(2, 32); }
+    if (d <= 128) { RB_L(2, 64); }
+    if (d <= 256) { RB_L(4, 64); }
+    RB_L(8, 64);
+#undef RB_L
+  }
   // (lanes per group, columns per group): 16 LPC state rows; 64 columns a CTA up to head size 128
 #define RB_L(LPC, NC) return channel ? launch_delta_rule<LPC, NC, true>(p, n_seqs, s) : launch_delta_rule<LPC, NC, false>(p, n_seqs, s)
   if (d <= 32) { RB_L(2, 1); }
