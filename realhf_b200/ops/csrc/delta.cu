@@ -239,6 +239,7 @@ struct ScanParams {
   float* s_state;           // [n_slots, H, d, dv] or null
   const int* slots;         // per sequence / row; null = identity (step form) or no state (packed form)
   int H, G, d, dv, step;
+  int vec = 0;              // rows of s_state may be written 16 bytes at a time
 };
 
 // Packed form.  A group of LPC lanes owns NC neighbouring columns of the state: lane l holds their rows ((e / 4) * LPC + l) * 4 + e % 4, e = 0 .. 15, so that its q / k
@@ -436,7 +437,17 @@ __global__ void __launch_bounds__(kScanThreads, LPC <= 8 ? 3 : 2) delta_rule_ker
       }
     }
   }
-  if (S_g) {
+  if (S_g && NC == 4 && p.vec) {
+    if (col < dv) {
+#pragma unroll
+      for (int e = 0; e < kRows; ++e) {
+        float z[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) { const float2 v = halves(Z[j % NC][e / 2]); z[j] = c * (e & 1 ? v.y : v.x); }
+        if (row_of(e) < d) *reinterpret_cast<float4*>(S_g + (int64_t)row_of(e) * dv + col) = make_float4(z[0], z[1], z[2], z[3]);
+      }
+    }
+  } else if (S_g) {
 #pragma unroll
     for (int j = 0; j < NC; ++j)
 #pragma unroll
@@ -449,7 +460,9 @@ __global__ void __launch_bounds__(kScanThreads, LPC <= 8 ? 3 : 2) delta_rule_ker
 }
 
 // Step form: one token per row, and reading and writing the state is all the work.  A thread group of LPC lanes owns one column (32 or 64 state rows
-// per lane), so that every access of a warp to the state covers whole 32-byte sectors.  (With the packed form's eight lanes and four columns an access
+// per lane), so that every access of a warp to the state covers whole 32-byte sectors.  The packed form of head sizes up to 64 also runs here, where
+// sharing q and k between columns saves little: size 64, 8 heads, 2 x 512 / 64 x 100 tokens 142 / 77 us against 166 / 84; size 32 110 / 59 against 122 / 43,
+// so many CTAs of size 32 take the other kernel.  (With the packed form's eight lanes and four columns an access
 // touched 16 sectors for a quarter each: 16 heads x 128 x 128, 1 / 16 / 128 rows 6.1 / 17.9 / 110 us, against 3.8 / 8.9 / 67.6 this way.)
 // Row mapping: lane l of a column's LPC lanes holds the state rows ((e / 4) * LPC + l) * 4 + e % 4, e = 0 .. kEPL - 1, so that its q / k
 // operands are 8 aligned float4 reads of shared memory per token (the lanes of a column read neighbouring float4s, the columns of
@@ -685,8 +698,9 @@ extern "C" int rb_delta_rule(const float* u, float* o, const int* cu, float* s_s
                              int step, int channel, cudaStream_t s) {
   if (n_seqs == 0) return 0;
   if (d > 512 || H % G) return -1;
-  ScanParams p{u, o, cu, s_state, slots, H, G, d, dv, step};
-  if (step) {       // (lanes per column, state rows per lane)
+  ScanParams p{u, o, cu, s_state, slots, H, G, d, dv, step, dv % 4 == 0 && ((uintptr_t)s_state & 15) == 0};
+  const bool many = (int64_t)n_seqs * H * RB_CEIL_DIV(dv, 64) >= rb::kNumSMs;
+  if (step || (d <= 64 && !(d <= 32 && many))) {       // (lanes per column, state rows per lane)
 #define RB_L(LPC, EPL) return channel ? launch_delta_column<LPC, EPL, true>(p, n_seqs, s) : launch_delta_column<LPC, EPL, false>(p, n_seqs, s)
     if (d <= 32) { RB_L(1, 32); }
     if (d <= 64) { RB_L(2, 32); }
@@ -698,7 +712,6 @@ extern "C" int rb_delta_rule(const float* u, float* o, const int* cu, float* s_s
   // (lanes per group, columns per group): 16 LPC state rows; 64 columns a CTA up to head size 128
 #define RB_L(LPC, NC) return channel ? launch_delta_rule<LPC, NC, true>(p, n_seqs, s) : launch_delta_rule<LPC, NC, false>(p, n_seqs, s)
   if (d <= 32) { RB_L(2, 1); }
-  if (d <= 64) { RB_L(4, 2); }
   if (d <= 128) { RB_L(8, 4); }
   if (d <= 256) { RB_L(16, 4); }
   RB_L(32, 4);

@@ -48,3 +48,19 @@ def test_delta_rule_decays_and_shapes(d, dv, decays, channel):
         # The yardstick is fp32's own rounding: the plain fp32 recurrence's largest error, four times it for another order of sums and the
         # decays' product, plus a few ulps of the largest value.
         assert float((x - w).abs().max()) <= 4 * float((f - w).abs().max()) + 8 * 2.0 ** -23 * float(w.abs().max())
+
+
+@pytest.mark.parametrize("d,dv,n_seqs", [(32, 64, 36), (32, 64, 37), (24, 130, 13), (64, 64, 40), (128, 128, 3), (128, 130, 3)])
+def test_delta_rule_on_both_sides_of_the_sequence_count(d, dv, n_seqs):
+    """Head sizes up to 32 change kernels with the number of CTAs (36 and 37 sequences x 4 heads lie on either side), and the final state is written four columns
+    at a time or one by one."""
+    lens = [3 + i % 7 for i in range(n_seqs)]
+    cfg, u = inputs(d, dv, "mixed", False, sum(lens), n_seqs)
+    cu, slots = torch.tensor([0] + lens).cumsum(0).int(), torch.arange(n_seqs, dtype=torch.int32).flip(0)
+
+    def run(u, scan):
+        S = torch.zeros(n_seqs, 4, d, dv, dtype=u.dtype, device=u.device)
+        return scan(u, cfg, cu.to(u.device), S, slots.to(u.device)).double().cpu(), S.double().cpu()
+    want, plain, got = run(u.double(), R.delta_rule_scan_ref), run(u, R.delta_rule_scan_ref), run(u.cuda(), R.delta_rule_scan)
+    for w, f, x in zip(want, plain, got):      # the bound of the test above
+        assert float((x - w).abs().max()) <= 4 * float((f - w).abs().max()) + 8 * 2.0 ** -23 * float(w.abs().max())
