@@ -585,9 +585,8 @@ __global__ void __launch_bounds__(kScanThreads, kEPL == 32 ? 3 : 2) delta_column
   }
 }
 
-// Head sizes in whole fours up to 128 CH, aligned: a warp takes 4 / CH rows (token, head) and has all their loads in flight before the first sum
-// (8 sequences of 700..1024 tokens, 16 heads x 128: 34 us after the recurrence with a row a warp, o read twice and the gate
-// behind the sum, 26 us this way).
+// Many rows of head sizes in whole fours up to 128 CH, aligned: a warp takes 4 / CH rows (token, head) and has all their loads in flight before the first
+// sum (8 sequences of 700..1024 tokens, 16 heads x 128: 34 us after the recurrence with a row a warp, 26 us this way).
 template <int CH>
 __global__ void __launch_bounds__(128) gated_head_norm_vec_kernel(const float* __restrict__ o, const void* __restrict__ w, int dtw,
                                                                   const void* __restrict__ gate, int64_t ldg, int dtg, void* __restrict__ out, int dto,
@@ -626,10 +625,11 @@ __global__ void __launch_bounds__(128) gated_head_norm_vec_kernel(const float* _
   }
 }
 
-// any head size and alignment: one warp per (token, head)
+// one warp per (token, head), `vec`: four elements per access (sizes and alignment allow it).  With few rows, or more than 256 columns, as fast as or
+// faster than rows held in registers (131072 rows x 512: 119 us against 157)
 __global__ void __launch_bounds__(128) gated_head_norm_kernel(const float* __restrict__ o, const void* __restrict__ w, int dtw,
                                                               const void* __restrict__ gate, int64_t ldg, int dtg, void* __restrict__ out, int dto,
-                                                              int64_t rows, int H, int dv, float eps, int sigmoid) {
+                                                              int64_t rows, int H, int dv, float eps, int sigmoid, int vec) {
   const int64_t r = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
   rb::pdl_trigger();
   rb::pdl_wait();
@@ -640,6 +640,17 @@ __global__ void __launch_bounds__(128) gated_head_norm_kernel(const float* __res
   const float* x = o + r * dv;
   auto act = [&](float g) { return (sigmoid ? 1.f : g) / (1.f + expf(-g)); };
   float ss = 0.f;
+  if (vec) {
+    for (int c = lane * 4; c < dv; c += 128) { const float4 v = *reinterpret_cast<const float4*>(x + c); ss += (v.x * v.x + v.y * v.y) + (v.z * v.z + v.w * v.w); }
+    ss = rb::warp_sum(ss);
+    const float rs = 1.f / sqrtf(ss / (float)dv + eps);
+    for (int c = lane * 4; c < dv; c += 128) {
+      const float4 v = *reinterpret_cast<const float4*>(x + c), g = rb::ld4_any(gate, dtg, t * ldg + h * dv + c), ww = rb::ld4_any(w, dtw, c);
+      rb::st4_any(out, dto, r * dv + c, make_float4(v.x * rs * ww.x * act(g.x), v.y * rs * ww.y * act(g.y), v.z * rs * ww.z * act(g.z),
+                                                    v.w * rs * ww.w * act(g.w)));
+    }
+    return;
+  }
   for (int c = lane; c < dv; c += 32) ss += x[c] * x[c];
   ss = rb::warp_sum(ss);
   const float rs = 1.f / sqrtf(ss / (float)dv + eps);
@@ -722,16 +733,15 @@ extern "C" int rb_gated_head_norm(const float* o, const void* w, int dtw, const 
                                   int dv, float eps, int sigmoid, cudaStream_t s) {
   const int64_t rows = T * H;
   if (rows == 0) return 0;
-  if (dv <= 512 && rows < (1ll << 31) && dv % 4 == 0 && ldg % 4 == 0 && (((uintptr_t)o | (uintptr_t)w | (uintptr_t)gate | (uintptr_t)out) & 15) == 0) {
+  const bool vec = dv % 4 == 0 && ldg % 4 == 0 && (((uintptr_t)o | (uintptr_t)w | (uintptr_t)gate | (uintptr_t)out) & 15) == 0;
+  if (vec && dv <= 256 && rows >= rb::kNumSMs * 64 && rows < (1ll << 31)) {      // fewer rows: a row a warp keeps more SMs busy
 #define RB_L(CH)                                                                                                                                  \
   return rb::launch_pdl(gated_head_norm_vec_kernel<CH>, dim3((unsigned)((rows + 16 / CH - 1) / (16 / CH))), dim3(128), 0, s, o, w, dtw, gate, ldg, \
                         dtg, out, dto, rows, H, dv, eps, sigmoid) == cudaSuccess ? 0 : -3
-    const bool many = rows >= rb::kNumSMs * 64;       // fewer (decode): a row a warp
-    if (many && dv <= 128) { RB_L(1); }
-    if (many && dv <= 256) { RB_L(2); }
-    RB_L(4);
+    if (dv <= 128) { RB_L(1); }
+    RB_L(2);
 #undef RB_L
   }
   return rb::launch_pdl(gated_head_norm_kernel, dim3((unsigned)((rows + 3) / 4)), dim3(128), 0, s, o, w, dtw, gate, ldg, dtg, out, dto, rows, H, dv,
-                        eps, sigmoid) == cudaSuccess ? 0 : -3;
+                        eps, sigmoid, (int)vec) == cudaSuccess ? 0 : -3;
 }
