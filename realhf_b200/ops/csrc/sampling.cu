@@ -360,7 +360,7 @@ __global__ void __launch_bounds__(kThreads, 1) sample_kernel(SampleParams p) {
       float before = 0.f, kept = 0.f;
       for (int w = 0; w < kWarps; ++w) { if (w == warp) before = kept; kept += sh.red[w]; }
       const float target = u * kept;
-      if (local > 0.f) {
+      if (local > 0.f || !(kept > 0.f)) {           // (no kept element has a mass: NaN, or infinities alone; the last one is taken)
         const bool here = target >= before && target < before + local;
         float c = before;
         int pick = -1, last = -1;

@@ -138,3 +138,24 @@ def test_sample_thresholds_at_the_edges_of_the_candidate_path(V, top_k, top_p, t
     assert not removed[rows, tok].any()
     ref = torch.log_softmax(xd.masked_fill(removed, float("-inf")), -1)[rows, tok]
     torch.testing.assert_close(lp.double(), ref, atol=2e-5, rtol=1e-5)
+
+
+@pytest.mark.parametrize("V", [500, 2048, 32003])
+@pytest.mark.parametrize("top_k,top_p", [(50, 0.9), (600, 1.0), (None, 1.0), (None, 0.9)])
+def test_sample_without_a_finite_mass_takes_the_last_kept_element(V, top_k, top_p):
+    """Rows whose kept elements have no probability to draw from (all -infinity, all NaN, a +infinity among finite ones): the last element that the mask
+    keeps, as an index inside the row.  Beside them ordinary rows with -infinity in them, which must never draw one."""
+    top_k = min(top_k or V, V)
+    torch.manual_seed(V)
+    x = torch.randn(6, V, device=DEV) * 2
+    x[0] = float("-inf")
+    x[1] = float("nan")
+    x[2, 7] = float("inf")
+    x[3, ::2] = float("-inf")
+    x[4, 3:] = float("-inf")
+    tok, lp, mb = lib().sample(x, None, top_k, top_p, 1.0, -1, False, False, 0, 5, 3, True)
+    kept = ~OF.unpack_mask_bits(mb, V)
+    last = (V - 1 - kept.flip(1).int().argmax(1)).tolist()
+    assert kept.any(1).all() and tok[:3].tolist() == last[:3]
+    rows = torch.arange(3, 6, device=DEV)
+    assert torch.isfinite(x[rows, tok[3:]]).all() and torch.isfinite(lp[3:]).all() and kept[rows, tok[3:]].all()
