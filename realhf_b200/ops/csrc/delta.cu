@@ -585,48 +585,36 @@ __global__ void __launch_bounds__(kScanThreads, kEPL == 32 ? 3 : 2) delta_column
   }
 }
 
-// Many rows of head sizes in whole fours up to 128 CH, aligned: a warp takes 4 / CH rows (token, head) and has all their loads in flight before the first
-// sum (8 sequences of 700..1024 tokens, 16 heads x 128: 34 us after the recurrence with a row a warp, 26 us this way).
-template <int CH>
+// Many rows of head sizes in whole fours up to 128, aligned: a warp takes four rows (token, head) and has all their loads in flight before the first sum
+// (8 sequences of 700..1024 tokens, 16 heads x 128: 34 us after the recurrence with a row a warp, 26 us this way).
 __global__ void __launch_bounds__(128) gated_head_norm_vec_kernel(const float* __restrict__ o, const void* __restrict__ w, int dtw,
                                                                   const void* __restrict__ gate, int64_t ldg, int dtg, void* __restrict__ out, int dto,
                                                                   int64_t rows, int H, int dv, float eps, int sigmoid) {
-  constexpr int U = 4 / CH;
+  constexpr int U = 4;
   const uint32_t r0 = (blockIdx.x * 4 + (threadIdx.x >> 5)) * U;
-  const int lane = threadIdx.x & 31;
+  const int lane = threadIdx.x & 31, c = lane * 4;
   rb::pdl_trigger();
   rb::pdl_wait();
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-  float4 x[U][CH], g[U][CH], ww[CH];
+  float4 x[U], g[U];
 #pragma unroll
-  for (int j = 0; j < CH; ++j) {
-    const int c = j * 128 + lane * 4;
+  for (int i = 0; i < U; ++i) x[i] = r0 + i < rows && c < dv ? *reinterpret_cast<const float4*>(o + (int64_t)(r0 + i) * dv + c) : zero;
 #pragma unroll
-    for (int i = 0; i < U; ++i) x[i][j] = r0 + i < rows && c < dv ? *reinterpret_cast<const float4*>(o + (int64_t)(r0 + i) * dv + c) : zero;
-#pragma unroll
-    for (int i = 0; i < U; ++i) g[i][j] = r0 + i < rows && c < dv ? rb::ld4_any(gate, dtg, (r0 + i) / (uint32_t)H * ldg + (int)((r0 + i) % (uint32_t)H) * dv + c) : zero;
-    ww[j] = c < dv ? rb::ld4_any(w, dtw, c) : zero;
-  }
+  for (int i = 0; i < U; ++i) g[i] = r0 + i < rows && c < dv ? rb::ld4_any(gate, dtg, (r0 + i) / (uint32_t)H * ldg + (int)((r0 + i) % (uint32_t)H) * dv + c) : zero;
+  const float4 ww = c < dv ? rb::ld4_any(w, dtw, c) : zero;
   auto act = [&](float z) { return (sigmoid ? 1.f : z) / (1.f + expf(-z)); };
 #pragma unroll
   for (int i = 0; i < U; ++i) {
-    float ss = 0.f;
-#pragma unroll
-    for (int j = 0; j < CH; ++j) ss += (x[i][j].x * x[i][j].x + x[i][j].y * x[i][j].y) + (x[i][j].z * x[i][j].z + x[i][j].w * x[i][j].w);
-    const float rs = 1.f / sqrtf(rb::warp_sum(ss) / (float)dv + eps);
-#pragma unroll
-    for (int j = 0; j < CH; ++j) {
-      const int c = j * 128 + lane * 4;
-      const float4 v = x[i][j], z = g[i][j], wv = ww[j];
-      if (r0 + i < rows && c < dv)
-        rb::st4_any(out, dto, (int64_t)(r0 + i) * dv + c, make_float4(v.x * rs * wv.x * act(z.x), v.y * rs * wv.y * act(z.y), v.z * rs * wv.z * act(z.z),
-                                                             v.w * rs * wv.w * act(z.w)));
-    }
+    const float4 v = x[i], z = g[i];
+    const float rs = 1.f / sqrtf(rb::warp_sum((v.x * v.x + v.y * v.y) + (v.z * v.z + v.w * v.w)) / (float)dv + eps);
+    if (r0 + i < rows && c < dv)
+      rb::st4_any(out, dto, (int64_t)(r0 + i) * dv + c, make_float4(v.x * rs * ww.x * act(z.x), v.y * rs * ww.y * act(z.y), v.z * rs * ww.z * act(z.z),
+                                                                    v.w * rs * ww.w * act(z.w)));
   }
 }
 
-// one warp per (token, head), `vec`: four elements per access (sizes and alignment allow it).  With few rows, or more than 256 columns, as fast as or
-// faster than rows held in registers (131072 rows x 512: 119 us against 157)
+// one warp per (token, head), `vec`: four elements per access (sizes and alignment allow it).  With few rows, or more than 128 columns, as fast as or
+// faster than rows held in registers (131072 rows x 256 / 512: 74 / 119 us against 76 / 157)
 __global__ void __launch_bounds__(128) gated_head_norm_kernel(const float* __restrict__ o, const void* __restrict__ w, int dtw,
                                                               const void* __restrict__ gate, int64_t ldg, int dtg, void* __restrict__ out, int dto,
                                                               int64_t rows, int H, int dv, float eps, int sigmoid, int vec) {
@@ -734,14 +722,9 @@ extern "C" int rb_gated_head_norm(const float* o, const void* w, int dtw, const 
   const int64_t rows = T * H;
   if (rows == 0) return 0;
   const bool vec = dv % 4 == 0 && ldg % 4 == 0 && (((uintptr_t)o | (uintptr_t)w | (uintptr_t)gate | (uintptr_t)out) & 15) == 0;
-  if (vec && dv <= 256 && rows >= rb::kNumSMs * 64 && rows < (1ll << 31)) {      // fewer rows: a row a warp keeps more SMs busy
-#define RB_L(CH)                                                                                                                                  \
-  return rb::launch_pdl(gated_head_norm_vec_kernel<CH>, dim3((unsigned)((rows + 16 / CH - 1) / (16 / CH))), dim3(128), 0, s, o, w, dtw, gate, ldg, \
-                        dtg, out, dto, rows, H, dv, eps, sigmoid) == cudaSuccess ? 0 : -3
-    if (dv <= 128) { RB_L(1); }
-    RB_L(2);
-#undef RB_L
-  }
+  if (vec && dv <= 128 && rows >= rb::kNumSMs * 64 && rows < (1ll << 31))        // fewer rows: a row a warp keeps more SMs busy
+    return rb::launch_pdl(gated_head_norm_vec_kernel, dim3((unsigned)((rows + 15) / 16)), dim3(128), 0, s, o, w, dtw, gate, ldg, dtg, out, dto, rows, H, dv,
+                          eps, sigmoid) == cudaSuccess ? 0 : -3;
   return rb::launch_pdl(gated_head_norm_kernel, dim3((unsigned)((rows + 3) / 4)), dim3(128), 0, s, o, w, dtw, gate, ldg, dtg, out, dto, rows, H, dv,
                         eps, sigmoid, (int)vec) == cudaSuccess ? 0 : -3;
 }
