@@ -315,15 +315,14 @@ __global__ void __launch_bounds__(kThreads, 1) sample_kernel(SampleParams p) {
         }
         keep_key = prefix;
       }
-      // ---- softmax mass of the top-k set
-      float tot = 0.f;
-      for (int j = tid; j < V; j += kThreads) {
-        const float x = srow[j];
-        if (f2key(x) >= keep_key) tot += __expf(x - mx);
-      }
-      tot = rb::block_reduce<false>(tot, sh.red);
       // ---- top-p: weighted radix descent inside the top-k set
       if (p.top_p < 1.f) {
+        float tot = 0.f;                             // softmax mass of the top-k set
+        for (int j = tid; j < V; j += kThreads) {
+          const float x = srow[j];
+          if (f2key(x) >= keep_key) tot += __expf(x - mx);
+        }
+        tot = rb::block_reduce<false>(tot, sh.red);
         const float P = p.top_p * tot;
         float above = 0.f;
         prefix = 0; maskbits = 0;
@@ -357,37 +356,58 @@ __global__ void __launch_bounds__(kThreads, 1) sample_kernel(SampleParams p) {
       if (lane == 0) sh.red[warp] = local;
       if (tid == 0) { sh.u[2] = 0xffffffffu; sh.u[3] = 0; }
       __syncthreads();
-      float before = 0.f, kept = 0.f;
-      for (int w = 0; w < kWarps; ++w) { if (w == warp) before = kept; kept += sh.red[w]; }
-      const float target = u * kept;
-      if (local > 0.f || !(kept > 0.f)) {           // (no kept element has a mass: NaN, or infinities alone; the last one is taken)
-        const bool here = target >= before && target < before + local;
-        float c = before;
-        int pick = -1, last = -1;
-        for (int j0 = w0; j0 < w1; j0 += 32) {
-          const int j = j0 + lane;
-          const bool in = j < w1 && f2key(srow[j]) >= keep_key;
-          const unsigned b = __ballot_sync(0xffffffffu, in);
-          if (b) last = j0 + 31 - __clz(b);
-          if (here && pick < 0 && b) {
-            float incl = in ? __expf(srow[j] - mx) : 0.f;
+      float upto = sh.red[lane];                     // mass of the ranges up to the lane's
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-              const float x = __shfl_up_sync(0xffffffffu, incl, o);
-              if (lane >= o) incl += x;
-            }
-            const unsigned hit = __ballot_sync(0xffffffffu, in && target < c + incl);
-            if (hit) pick = j0 + __ffs(hit) - 1;
-            c += __shfl_sync(0xffffffffu, incl, 31);
+      for (int o = 1; o < 32; o <<= 1) {
+        const float x = __shfl_up_sync(0xffffffffu, upto, o);
+        if (lane >= o) upto += x;
+      }
+      const float kept = __shfl_sync(0xffffffffu, upto, 31), end = __shfl_sync(0xffffffffu, upto, warp), below = __shfl_sync(0xffffffffu, upto, max(warp - 1, 0));
+      const float before = warp == 0 ? 0.f : below, target = u * kept;
+      if (target >= before && target < end) {        // (the ranges join without gaps)
+        // eight groups of 32 at a time, then inside the one that holds the target
+        float c = before;
+        int group = -1, tail = -1;
+        for (int j0 = w0; j0 < w1 && group < 0; j0 += 256) {
+          float sum[8];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const int j = j0 + i * 32 + lane;
+            sum[i] = rb::warp_sum(j < w1 && f2key(srow[j]) >= keep_key ? __expf(srow[j] - mx) : 0.f);
           }
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+            if (group < 0) {
+              if (target < c + sum[i]) group = j0 + i * 32;
+              else { c += sum[i]; if (sum[i] > 0.f) tail = j0 + i * 32; }
+            }
         }
-        if (lane == 0) {
-          if (here) atomicMin(&sh.u[2], (uint32_t)(pick >= 0 ? pick : last));
-          atomicMax(&sh.u[3], (uint32_t)last);      // rounding at the very end of the CDF: the last kept element
+        if (group < 0) group = tail;                 // rounding: the groups' sums end below the range's; their last element
+        if (group >= 0) {
+          const int j = group + lane;
+          const bool in = j < w1 && f2key(srow[j]) >= keep_key;
+          float incl = in ? __expf(srow[j] - mx) : 0.f;
+          const unsigned all = __ballot_sync(0xffffffffu, incl > 0.f);
+#pragma unroll
+          for (int o = 1; o < 32; o <<= 1) {
+            const float x = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += x;
+          }
+          const unsigned hit = __ballot_sync(0xffffffffu, in && target < c + incl);
+          if (lane == 0) atomicMin(&sh.u[2], (uint32_t)(group + (hit ? __ffs(hit) - 1 : 31 - __clz(all))));
         }
       }
       __syncthreads();
-      chosen = sh.u[2] == 0xffffffffu ? sh.u[3] : sh.u[2];
+      chosen = sh.u[2];
+      if (sh.u[2] == 0xffffffffu) {                  // rounding at the very end of the CDF, or no mass at all (NaN, infinities alone): the last kept element
+        int last = -1;
+        if (local > 0.f || !(kept > 0.f))
+          for (int j = w0 + lane; j < w1; j += 32)
+            if (f2key(srow[j]) >= keep_key) last = j;
+        if (last >= 0) atomicMax(&sh.u[3], (uint32_t)last);
+        __syncthreads();
+        chosen = sh.u[3];
+      }
       chosen_lp = srow[chosen] - mx - __logf(kept);
     }
   }
@@ -407,20 +427,21 @@ __global__ void __launch_bounds__(kThreads, 1) sample_kernel(SampleParams p) {
     }
   }
   if (p.mask_bits != nullptr) {
-    // 32 elements a ballot, 1024 a warp and round: lane i ends up with the i-th word of the round
+    // 32 elements a ballot, up to 1024 a warp and round (the words of a short row spread over all warps): lane i ends up with the i-th word of the round
     uint8_t* mrow = p.mask_bits + (int64_t)row * p.mask_stride;
-    const int nbytes = (V + 7) / 8;
+    const int nbytes = (V + 7) / 8, per_warp = min(32, ((V + 31) / 32 + kWarps - 1) / kWarps);
     const bool words = (reinterpret_cast<uintptr_t>(mrow) & 3) == 0;
-    for (int j0 = warp * 1024; j0 < V; j0 += kThreads * 32) {
+    for (int j0 = warp * per_warp * 32; j0 < V; j0 += kWarps * per_warp * 32) {
       uint32_t word = 0;
 #pragma unroll 8
-      for (int i = 0; i < 32; ++i) {
+      for (int i = 0; i < per_warp; ++i) {
         const int j = j0 + i * 32 + lane;
         const unsigned b = __ballot_sync(0xffffffffu, j < V && f2key(srow[j]) < keep_key);
         if (lane == i) word = b;
       }
       const int byte = j0 / 8 + lane * 4;
-      if (words && byte + 4 <= nbytes) {
+      if (lane >= per_warp) {
+      } else if (words && byte + 4 <= nbytes) {
         *reinterpret_cast<uint32_t*>(mrow + byte) = word;
       } else {
         for (int i = 0; i < 4; ++i)

@@ -1,4 +1,6 @@
 """Fused sampling kernel vs the PyTorch reference filter: same kept set (mask), consistent log-probs, valid samples."""
+import math
+
 import pytest
 import torch
 
@@ -159,3 +161,32 @@ def test_sample_without_a_finite_mass_takes_the_last_kept_element(V, top_k, top_
     assert kept.any(1).all() and tok[:3].tolist() == last[:3]
     rows = torch.arange(3, 6, device=DEV)
     assert torch.isfinite(x[rows, tok[3:]]).all() and torch.isfinite(lp[3:]).all() and kept[rows, tok[3:]].all()
+
+
+@pytest.mark.parametrize("V", [31, 1000, 2048, 4099, 32003, 51200])
+def test_sample_unfiltered_draws_by_inverse_cdf(V):
+    """No filter: the draw over the whole row.  Logits of one element far above the rest, in every group of a row in turn, and a flat row, whose draws
+    over many seeds cover it evenly; the mask removes nothing and ends at the last byte."""
+    at = torch.arange(0, V, max(1, V // 97), device=DEV)
+    x = torch.randn(at.numel(), V, device=DEV)
+    x[torch.arange(at.numel(), device=DEV), at] = 60.0
+    tok, lp, mb = lib().sample(x, None, V, 1.0, 1.0, -1, False, False, 0, 9, 1, True)
+    assert torch.equal(tok, at) and float(lp.abs().max()) < 1e-6 and int(mb.sum()) == 0
+    flat = torch.zeros(4096, V, device=DEV, dtype=torch.bfloat16)
+    tok, lp, _ = lib().sample(flat, None, V, 1.0, 1.0, -1, False, False, 0, 9, 1, False)
+    torch.testing.assert_close(lp, torch.full_like(lp, -math.log(V)), atol=2e-5, rtol=1e-5)
+    # 4096 draws in 16 equal parts of the row (V 31: each part is two elements or one): a part's count is binomial, five standard deviations
+    part = tok * 16 // V
+    share = torch.bincount(torch.arange(V, device=DEV) * 16 // V, minlength=16).double() / V
+    count = torch.bincount(part, minlength=16).double()
+    assert ((count - 4096 * share).abs() <= 5 * (4096 * share * (1 - share)).sqrt()).all()
+
+
+@pytest.mark.parametrize("V,top_k", [(1000, 200), (1003, 126), (264, 60)])
+def test_sample_with_fewer_thread_maxima_than_top_k(V, top_k):
+    """16-byte loads of 16-bit logits leave V / 8 thread maxima: with fewer than top_k of them nothing bounds the candidates."""
+    torch.manual_seed(V)
+    x = (torch.randn(5, V, device=DEV) * 2).to(torch.bfloat16)
+    _, _, mb = lib().sample(x, None, top_k, 1.0, 1.0, -1, False, False, 0, 5, 3, True)
+    kth = torch.topk(x.float(), top_k, -1).values[:, -1:]
+    assert torch.equal(OF.unpack_mask_bits(mb, V), x.float() < kth)
