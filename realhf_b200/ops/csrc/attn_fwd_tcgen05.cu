@@ -35,8 +35,8 @@
 // Modes (`WindowAttentionConfig`, inference only, no LSE): kGeneral: score = s * scale * temp_h - slope_h * (i - j) with slope_h =
 // 2^(-slope_base (h + 1) / nq) (log2 domain, two FMAs per score), a sliding window that also keeps the first `keep` keys (their
 // tiles below the window's first tile are walked first).  kSimple: no distance term, temperature or kept keys and a positive scale: the
-// maximum is taken over the raw products.  kCap: kSimple with score = softcap * tanh(s * scale / softcap); the cap is monotone, so the
-// raw maximum is capped once.  All three: a per-head sink logit starts the running maximum with denominator 1; the output is
+// maximum is taken over the raw products.  kCap: kSimple with score = softcap * tanh(s * scale / softcap), formed before the
+// masks, so that a product that overflowed to -infinity is a visible score of -softcap.  All three: a per-head sink logit starts the running maximum with denominator 1; the output is
 // multiplied by sigmoid(gate logit of its head, or of the output element); `chunk` > 0 replaces the window: a query sees the keys of its own
 // chunk of positions up to itself.  (32 x 1024 tokens, 16 / 4 heads, window 512 + 64 kept: 1382 us with one tile per CTA, now 269.)
 // Learned distance biases and shared keys / values run in attn_fwd_bias.cu.
@@ -339,6 +339,10 @@ __global__ void __launch_bounds__(kFwdThreads, 1) attn_fwd_kernel(const __grid_c
 #pragma unroll
           for (int i = 0; i < 128; ++i) s[i] = fmaf(s[i], c2, fmaf(slope2, (float)i, base));
         }
+        if constexpr (kMode == kCap) {
+#pragma unroll
+          for (int i = 0; i < 128; ++i) s[i] = soft_cap2(s[i], cap_c, cap_k, cap_k);
+        }
         // only the last tile of the sequence, the diagonal tile and the tiles the window's lower edge crosses need per-element masks
         if ((kv0 + kTile > L) || (p.causal && kv0 + kTile - 1 > q0) || (bounded && last_lo > kv0)) {
           const int lim = (p.causal ? min(L, q_pos + 1) : L) - kv0;   // local key columns [lo, lim) are visible to this row
@@ -361,7 +365,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) attn_fwd_kernel(const __grid_c
 #pragma unroll
           for (int e = 0; e < 4; ++e) mx4[e] = fmaxf(mx4[e], fmaxf(s[i + 2 * e], s[i + 2 * e + 1]));
         float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
-        if (kMode != kGeneral && mx != -INFINITY) mx = kMode == kCap ? soft_cap2(mx, cap_c, cap_k, cap_k) : mx * c2;
+        if (kMode != kGeneral && kMode != kCap && mx != -INFINITY) mx *= c2;
         float alpha = 1.f;
         bool grown = false;                           // the same in the whole warp
         if (first) {
@@ -382,10 +386,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) attn_fwd_kernel(const __grid_c
 #pragma unroll
         for (int i = 0; i < 128; i += 2) {
           float e0, e1;
-          if constexpr (kMode == kCap) {
-            e0 = s[i] == -INFINITY ? 0.f : exp2f(soft_cap2(s[i], cap_c, cap_k, cap_k + neg_m));
-            e1 = s[i + 1] == -INFINITY ? 0.f : exp2f(soft_cap2(s[i + 1], cap_c, cap_k, cap_k + neg_m));
-          } else if constexpr (kMode == kGeneral) {
+          if constexpr (kMode == kGeneral || kMode == kCap) {
             e0 = exp2f(s[i] + neg_m);
             e1 = exp2f(s[i + 1] + neg_m);
           } else {

@@ -188,6 +188,41 @@ def test_attn_fwd_tile_pairs(heads, lens, form):
     torch.testing.assert_close(lse.double(), rlse, atol=2e-5, rtol=2e-6)
 
 
+@pytest.mark.parametrize("cap,sink,hd", [(20.0, False, 64), (20.0, True, 64), (3.0, False, 128), (50.0, True, 128)])
+@pytest.mark.parametrize("form", ["ordinary", "overflowing"])
+def test_capped_scores(cap, sink, hd, form):
+    """Capped scores against float64, also where the products overflow fp32: an infinite product is a score of +-cap like any other, hidden keys alone are
+    left out.  Bound as in test_attn_fwd_tile_pairs, and the capped score's own rounding, a few ulps of cap log2 e in the exponent."""
+    H, G, lens = 4, 2, [1, 130, 300]
+    T, dt = sum(lens), torch.bfloat16
+    torch.manual_seed(hd)
+    qkv = torch.randn(T, H * hd + 2 * G * hd, device=DEV)
+    if form == "overflowing":               # one sign a key, so that no sum holds both infinities; the first sequences' keys are all negative
+        sign = torch.where(torch.rand(T, 1, device=DEV) < 0.7, -1.0, 1.0)
+        sign[:131] = -1.0
+        qkv[:, :H * hd] = 1e25
+        qkv[:, H * hd:(H + G) * hd] = sign * 1e25
+    qkv = qkv.to(dt)
+    vn = qkv[:, (H + G) * hd:].contiguous()
+    logit = torch.randn(H, device=DEV).to(dt) if sink else None
+    out = torch.full((T, H * hd), float("nan"), device=DEV, dtype=dt)
+    cu = torch.tensor([0] + list(torch.tensor(lens).cumsum(0)), dtype=torch.int32, device=DEV)
+    scale = hd ** -0.5
+    lib().sink_window_attention_tc(qkv, vn, out, None, logit, cu, max(lens), H, G, hd, scale, 0, 0, -1.0, None, False, 0, cap)
+    eps, a = 2.0 ** -8 + 16 * 2.0 ** -23 * cap * 1.45, 0
+    for n in lens:
+        q, k, v = (t[a:a + n].double().view(n, -1, hd).transpose(0, 1) for t in (qkv[:, :H * hd], qkv[:, H * hd:(H + G) * hd], vn))
+        k, v = k.repeat_interleave(H // G, 0), v.repeat_interleave(H // G, 0)
+        s = cap * torch.tanh(q @ k.transpose(1, 2) * scale / cap)
+        s = s.masked_fill(torch.ones(n, n, dtype=torch.bool, device=DEV).triu(1), float("-inf"))
+        if sink:
+            s = torch.cat([s, logit.double().view(H, 1, 1).expand(H, n, 1)], 2)
+        p = torch.softmax(s, -1)[..., :n]
+        ref, mag = (p @ v).transpose(0, 1), (p @ v.abs()).transpose(0, 1)
+        assert ((out[a:a + n].double().view(n, H, hd) - ref).abs() <= eps * (ref.abs() + mag) + 1e-6).all()
+        a += n
+
+
 def test_a_wait_that_ran_out_is_raised_and_the_update_skipped():
     """The status word as a kernel leaves it whose bounded wait ran out (set here by a copy): the next attention call of either direction and the
     engine raise, the optimizer leaves the parameters alone, and clearing the word makes everything run again."""
