@@ -178,7 +178,7 @@ std::vector<Tensor> rmsnorm_bwd(const Tensor& x, const Tensor& w, const Tensor& 
   int rc = rb_rmsnorm_bwd(x.data_ptr(), w.data_ptr(), dy.data_ptr(), rstd.data_ptr<float>(), dx.data_ptr(),
                           partial.data_ptr<float>(), dw.data_ptr(), rows, H, w_offset, dt_code(x),
                           dres.has_value() ? dres->data_ptr() : nullptr, cur_stream());
-  TORCH_CHECK(rc == 0, "rmsnorm_bwd: unsupported shape/dtype");
+  TORCH_CHECK(rc == 0, "rmsnorm_bwd: unsupported shape / dtype, or the launch failed (", rc, ")");
   return {dx, dw};
 }
 

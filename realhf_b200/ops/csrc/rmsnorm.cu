@@ -5,6 +5,8 @@
 // write-y (+write-residual).  Backward: persistent CTAs walk rows, produce dx and keep the weight
 // gradient in registers; per-CTA partials are reduced by a second tiny kernel (colsum.cuh).
 // Replaces the eager fp32-upcast RMSNorm of the reference (modules/mlp.py:425-467).
+#include <atomic>
+
 #include "colsum.cuh"
 
 namespace {
@@ -71,7 +73,7 @@ __global__ void __launch_bounds__(kThreads) rmsnorm_fwd_kernel(const T* __restri
 // loads, reduces and stores row after row leaves the memory idle for most of each row (20480 x 4096 bf16 with dres: 220 us, 3.0 TB/s; with
 // one row prefetched into registers 192 us).  Every thread therefore keeps the pieces of kStages rows in flight with cp.async, into
 // shared memory only it reads back (no barrier, no wait on another thread), and the reduction takes one barrier (two alternating sets of
-// warp sums).  ~190 KB of rows are in flight per SM at every width.
+// warp sums).  The rings of an SM hold 192 KB (16-bit rows of up to 1024 columns: 96 KB, four CTAs), a third of it for dres.
 template <typename T, int TB, int NV> struct RmsBwd {
   static constexpr int kPieces = 8 * sizeof(T) / 16;                 // 16-byte pieces of a thread's 8 elements
   static constexpr int kStageBytes = 3 * NV * TB * 8 * (int)sizeof(T);
@@ -194,16 +196,19 @@ int launch_rmsnorm_bwd(const void* x, const void* w, const void* dy, const float
                        float w_offset, const void* dres, cudaStream_t s) {
   using C = RmsBwd<T, TB, NV>;
   auto kern = rmsnorm_bwd_kernel<T, TB, NV>;
-  static bool attr_set = false;
-  if (!attr_set) {
+  static std::atomic<uint64_t> opted_in{0};          // the attribute is the kernel's on one device: a bit per device
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return -2;
+  if (dev >= 64 || !(opted_in.load() >> dev & 1)) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmem) != cudaSuccess) return -2;
-    attr_set = true;
+    if (dev < 64) opted_in.fetch_or(1ull << dev);
   }
   const int64_t ctas = (int64_t)rb::kNumSMs * C::kCtas;
   const int grid = (int)(rows < ctas ? rows : ctas);
   kern<<<grid, TB, C::kSmem, s>>>((const T*)x, (const T*)w, (const T*)dy, rstd, (T*)dx, dw_partial, rows, H, w_offset, (const T*)dres);
+  if (cudaGetLastError() != cudaSuccess) return -3;
   rb::launch_colsum<T>(dw_partial, dw, grid, H, s);
-  return 0;
+  return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 
 }  // namespace

@@ -75,6 +75,18 @@ def test_rmsnorm_fwd_bwd(dtype, H):
     torch.testing.assert_close(w.grad.float(), wr.grad, atol=0.3 if dtype != torch.float32 else 1e-3, rtol=3e-2)
 
 
+@pytest.mark.skipif(torch.cuda.device_count() < 2, reason="needs a second GPU")
+@pytest.mark.parametrize("dtype,H", [(torch.bfloat16, 1024), (torch.bfloat16, 4096), (torch.float32, 2048)])
+def test_rmsnorm_bwd_on_every_device_of_a_process(dtype, H):
+    """The kernel's shared-memory opt-in belongs to one device: every further GPU of the process needs its own."""
+    torch.manual_seed(H)
+    x, w, dy = (torch.randn(*s).to(dtype) for s in ((300, H), (H,), (300, H)))
+    rstd = torch.rand(300)
+    got = [[t.cpu() for t in lib().rmsnorm_bwd(x.to(d), w.to(d), dy.to(d), rstd.to(d), 0.0, None)] for d in range(torch.cuda.device_count())]
+    for other in got[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(got[0], other))
+
+
 def test_add_rmsnorm_gemma_offset():
     torch.manual_seed(0)
     x = torch.randn(128, 2048, device=DEV, dtype=torch.bfloat16)
