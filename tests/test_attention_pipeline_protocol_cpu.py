@@ -1,11 +1,13 @@
-"""Model check of the mbarrier protocol of the tcgen05 attention kernels (csrc/attn_fwd_tcgen05.cu, attn_bwd_tcgen05.cu).
+"""Model check of the mbarrier protocols of the tcgen05 attention kernels (csrc/attn_fwd_tcgen05.cu, attn_bwd_tcgen05.cu, attn_fwd_bias.cu).
 
-The three roles of a CTA (TMA producer, MMA issuer, softmax threads) are written as coroutines that perform exactly the waits,
-arrives, expect_tx and commits of the kernels (same barrier names, same parities); TMA completions and tensor-pipe completions
-are asynchronous events.  A randomised scheduler interleaves everything over many seeds and checks
+The roles of a CTA (TMA producer and scheduler, MMA issuer, softmax / element warps) are written as coroutines that perform exactly the waits,
+arrives, expect_tx and commits of the kernels (same barrier names, same parities), over several work items of one CTA where the kernel is
+persistent; TMA completions, answers to requests for further items and tensor-pipe completions are asynchronous events.  A randomised scheduler
+interleaves everything over many seeds and checks
   * no deadlock (every role finishes) and no parity aliasing (a wait never needs a phase that is two completions away),
-  * no buffer hazard: a shared-memory stage / TMEM buffer is never overwritten before its consumer released it and never
-    read before it was produced.
+  * no buffer hazard: a shared-memory stage / TMEM buffer / item slot is never overwritten before its consumers released it and never
+    read before it was produced.  Buffers without a barrier of their own (P over S, which the next products overwrite) rely on the
+    tensor pipe's order, which the model keeps.
 This is the part of the kernels that cannot be unit-tested without hardware and whose failure mode on hardware is a hang."""
 import random
 
@@ -91,7 +93,7 @@ class Sim:
                     del gens[arg]
 
 
-# ------------------------------------------------------------------------------------------------ forward kernel
+# ------------------------------------------------------------------------------------------------ forward kernel with a learned bias
 def fwd_protocol(sim: Sim, n_kv: int):
     B = sim.bars
     KV = 100  # bytes of one K or V stage (any positive number)
@@ -190,113 +192,346 @@ def test_forward_protocol_has_no_deadlock_or_buffer_hazard(n_kv):
         assert all(v in ("free", "full", 0) for v in sim.state.values())
 
 
-# ------------------------------------------------------------------------------------------------ backward kernel (both passes)
-def bwd_protocol(sim: Sim, n_steps: int):
+# ------------------------------------------------------------------------------------------------ persistent kernels: items
+def count_down(sim, key, n):
+    """True for the last of n callers."""
+    sim.state[key] = sim.state.get(key, 0) + 1
+    if sim.state[key] == n:
+        sim.state[key] = 0
+        return True
+    return False
+
+
+class Items:
+    """The two item slots between the scheduler and its readers, and the requests for further items (one outstanding at a time)."""
+
+    def __init__(self, sim, items, readers):
+        self.sim, self.items, self.readers, self.n_pub, self.n_req = sim, items, readers, 0, 0
+        self.slots, self.answer, self.asked = [None, None], None, 0
+
+    def request(self):
+        assert self.answer is None, "an answer is overwritten before it was read"
+        self.sim.bars["CLC_FULL"].expect_tx(16)
+        self.asked += 1
+
+        def land(i=self.asked):
+            self.answer = (i,)
+            self.sim.bars["CLC_FULL"].complete_tx(16)
+        self.sim.tma.append(land)
+
+    def next(self):                                  # -> the next item's number, or None
+        yield ("wait", "CLC_FULL", self.n_req & 1)
+        self.n_req += 1
+        (i,), self.answer = self.answer, None
+        return i if i < len(self.items) else None
+
+    def publish(self, item):
+        slot = self.n_pub & 1
+        yield ("wait", f"IT_EMPTY{slot}", ((self.n_pub >> 1) & 1) ^ 1)
+        self.sim.expect(f"item{slot}", "free", f"item {self.n_pub} published")
+        self.sim.set(f"item{slot}", "full")
+        self.slots[slot] = (self.n_pub, item)
+        self.sim.bars[f"IT_FULL{slot}"].arrive()
+        self.n_pub += 1
+
+    def take(self, n_it):
+        slot = n_it & 1
+        yield ("wait", f"IT_FULL{slot}", (n_it >> 1) & 1)
+        n, item = self.slots[slot]
+        assert n == n_it, f"slot {slot} holds item {n}, read as item {n_it}"
+        if count_down(self.sim, f"item{slot}_readers", self.readers):
+            self.sim.set(f"item{slot}", "free")
+        self.sim.bars[f"IT_EMPTY{slot}"].arrive()
+        return item
+
+
+def load(sim, buf, bar, parts, what):
+    sim.bars[bar].expect_tx(10 * parts)
+    sim.expect(buf, "free", what)
+    sim.set(buf, "loading")
+    done = []
+
+    def part():                                      # the boxes of a tile complete independently
+        done.append(1)
+        if len(done) == parts:
+            sim.set(buf, "full")
+        sim.bars[bar].complete_tx(10)
+    for _ in range(parts):
+        sim.tma.append(part)
+
+
+ITEM_BARS = {"IT_FULL0": 1, "IT_FULL1": 1, "IT_EMPTY0": 9, "IT_EMPTY1": 9, "CLC_FULL": 1}
+
+
+# ------------------------------------------------------------------------------------------------ forward kernel (pairs of query tiles)
+STAGES = 4
+
+
+def fwd_pair_protocol(sim: Sim, items):
+    """An item is the list of its key tiles, each (taken by query tile 0, taken by query tile 1)."""
     B = sim.bars
+    it = Items(sim, items, 9)
 
     def producer():
-        B["R_FULL"].expect_tx(60)
-        sim.set("R", "loading")
-        sim.tma.append(lambda: (sim.set("R", "full"), B["R_FULL"].complete_tx(60)))
-        for t in range(n_steps):
-            b, par = t & 1, (t >> 1) & 1
-            yield ("wait", f"X_EMPTY{b}", par ^ 1)
-            B[f"X_FULL{b}"].expect_tx(40)
-            sim.expect(f"X{b}", "free", f"X load of step {t}"); sim.set(f"X{b}", "loading")
-            done = {"n": 0}
+        kvc, qc, idx = 0, [0, 0], 0
+        it.request()
+        while idx is not None:
+            walk = items[idx]
+            yield from it.publish(walk)
 
-            def part(b=b, done=done):   # four TMA boxes complete independently
-                done["n"] += 1
-                if done["n"] == 4:
-                    sim.set(f"X{b}", "full")
-                B[f"X_FULL{b}"].complete_tx(10)
-            for _ in range(4):
-                sim.tma.append(part)
+            def load_q(t):
+                if any(k[t] for k in walk):
+                    yield ("wait", f"Q_EMPTY{t}", (qc[t] & 1) ^ 1)
+                    qc[t] += 1
+                    load(sim, f"Q{t}", f"Q_FULL{t}", 2, "Q load")
+
+            def load_kv():
+                nonlocal kvc
+                st = kvc % STAGES
+                yield ("wait", f"KV_EMPTY{st}", ((kvc // STAGES) & 1) ^ 1)
+                kvc += 1
+                load(sim, f"KV{st}", f"KV_FULL{st}", 2, "K / V load")
+            yield from load_q(0)
+            yield from load_kv()
+            yield from load_q(1)
+            yield from load_kv()
+            for _ in walk[1:]:
+                yield from load_kv()
+                yield from load_kv()
+            idx = yield from it.next()
+            if idx is not None:
+                it.request()
+        yield from it.publish(None)
 
     def mma():
-        def issue_sdp(t):
-            b, par = t & 1, (t >> 1) & 1
-            yield ("wait", f"X_FULL{b}", par)
-            yield ("wait", f"S_EMPTY{b}", par ^ 1)
+        kvc, qc, pc, oc, n_it = 0, [0, 0], [0, 0], [0, 0], 0
+        while True:
+            walk = yield from it.take(n_it)
+            n_it += 1
+            if walk is None:
+                return
+            s_open, o_open = [False, False], [False, False]
+            last = [max((k for k, x in enumerate(walk) if x[t]), default=-1) for t in range(2)]
 
-            def exec_sdp():
-                sim.expect("R", "full", "S/dP mma"); sim.expect(f"X{b}", "full", f"S/dP mma {t}")
-                sim.expect(f"S{b}", "free", f"S/dP mma {t} overwrites the S/dP buffers"); sim.set(f"S{b}", "full")
-            sim.pipe.append(exec_sdp)
+            def open_kv(c):
+                yield ("wait", f"KV_FULL{c % STAGES}", (c // STAGES) & 1)
+                return c % STAGES
+
+            def free_kv(st):
+                sim.pipe.append(lambda: (sim.set(f"KV{st}", "free"), B[f"KV_EMPTY{st}"].arrive()))
+
+            def issue_s(t, k, st):
+                if not s_open[t]:
+                    yield ("wait", f"Q_FULL{t}", qc[t] & 1)
+                    qc[t] += 1
+                    s_open[t] = True
+
+                def run():
+                    sim.expect(f"Q{t}", "full", "S mma"), sim.expect(f"KV{st}", "full", "S mma"), sim.expect(f"S{t}", "free", "S mma")
+                    sim.set(f"S{t}", "s")
+                sim.pipe.append(run)
+                sim.pipe.append(lambda: B[f"S_FULL{t}"].arrive())
+                if k == last[t]:
+                    sim.pipe.append(lambda: (sim.set(f"Q{t}", "free"), B[f"Q_EMPTY{t}"].arrive()))
+
+            def issue_pv(t, st):
+                yield ("wait", f"P_FULL{t}", pc[t] & 1)
+                pc[t] += 1
+                if not o_open[t]:
+                    yield ("wait", f"O_EMPTY{t}", (oc[t] & 1) ^ 1)
+                    oc[t] += 1
+                was, o_open[t] = "acc" if o_open[t] else "free", True
+                sim.state[f"PV{t}"] = sim.state.get(f"PV{t}", 0) + 1           # issued and not retired
+
+                def run():
+                    sim.expect(f"S{t}", "p", "PV mma"), sim.expect(f"KV{st}", "full", "PV mma"), sim.expect(f"O{t}", was, "PV mma")
+                    sim.set(f"S{t}", "free"), sim.set(f"O{t}", "acc")
+                    sim.state[f"PV{t}"] -= 1
+                sim.pipe.append(run)
+                sim.pipe.append(lambda: B[f"O_FULL{t}"].arrive())
+            st = yield from open_kv(kvc)
+            for t in range(2):
+                if walk[0][t]:
+                    yield from issue_s(t, 0, st)
+            free_kv(st)
+            for k in range(len(walk)):
+                sv, sk = (yield from open_kv(kvc + 2 * k + 1)), None
+                for t in range(2):
+                    if walk[k][t]:
+                        yield from issue_pv(t, sv)
+                    if t == 1:
+                        free_kv(sv)
+                    if k + 1 < len(walk):
+                        if sk is None:
+                            sk = yield from open_kv(kvc + 2 * k + 2)
+                        if walk[k + 1][t]:
+                            yield from issue_s(t, k + 1, sk)
+                if sk is not None:
+                    free_kv(sk)
+            kvc += 2 * len(walk)
+
+    def softmax(w):
+        t, sc, vc, n_it = w >> 2, 0, 0, 0
+        while True:
+            walk = yield from it.take(n_it)
+            n_it += 1
+            if walk is None:
+                return
+            n_tiles = sum(k[t] for k in walk)
+            if n_tiles == 0:
+                continue
+            for k in range(n_tiles):
+                yield ("wait", f"S_FULL{t}", sc & 1)
+                sc += 1
+                sim.expect(f"S{t}", "s", "softmax reads S")
+                if k > 0 and sim.rng.random() < 0.5:               # the row's maximum has grown: O is scaled
+                    yield ("wait", f"O_FULL{t}", (vc - 1) & 1)
+                    sim.expect(f"O{t}", "acc", "O is scaled")
+                    assert sim.state[f"PV{t}"] == 0, "O is scaled with a product in flight"
+                if count_down(sim, f"S{t}_warps", 4):
+                    sim.set(f"S{t}", "p")
+                B[f"P_FULL{t}"].arrive()
+                vc += 1
+            yield ("wait", f"O_FULL{t}", (vc - 1) & 1)
+            sim.expect(f"O{t}", "acc", "output")
+            assert sim.state[f"PV{t}"] == 0, "output with a product in flight"
+            if count_down(sim, f"O{t}_warps", 4):
+                sim.set(f"O{t}", "free")
+            B[f"O_EMPTY{t}"].arrive()
+
+    return {"producer": producer(), "mma": mma(), **{f"softmax{w}": softmax(w) for w in range(8)}}
+
+
+PAIR_BARS = dict(ITEM_BARS)
+for _t in (0, 1):
+    PAIR_BARS.update({f"Q_FULL{_t}": 1, f"Q_EMPTY{_t}": 1, f"S_FULL{_t}": 1, f"P_FULL{_t}": 4, f"O_FULL{_t}": 1, f"O_EMPTY{_t}": 4})
+for _st in range(STAGES):
+    PAIR_BARS.update({f"KV_FULL{_st}": 1, f"KV_EMPTY{_st}": 1})
+
+ONE, BOTH, SECOND = (True, False), (True, True), (False, True)
+
+
+@pytest.mark.parametrize("items", [[[BOTH]], [[ONE]], [[BOTH] * 3 + [ONE]], [[ONE]] * 5, [[BOTH]] * 5, [[BOTH] * 2 + [ONE], [ONE], [BOTH] * 5, [ONE] * 3],
+                                   [[SECOND] * 2 + [BOTH] * 2 + [ONE], [BOTH, SECOND, BOTH, ONE], [ONE]], [[BOTH] * 9, [BOTH] * 2 + [ONE], [BOTH] * 4]],
+                         ids=lambda x: "-".join(str(len(w)) for w in x))
+def test_forward_pair_protocol_has_no_deadlock_or_buffer_hazard(items):
+    for seed in range(100):
+        sim = Sim(seed, PAIR_BARS)
+        sim.run(fwd_pair_protocol(sim, items))
+        assert all(v in ("free", 0) for v in sim.state.values()), sim.state
+
+
+# ------------------------------------------------------------------------------------------------ backward kernel (both passes)
+X_STAGES = 3
+
+
+def bwd_protocol(sim: Sim, items, r_empty_parity=lambda n_pub: n_pub & 1):
+    """An item is its number of steps."""
+    B = sim.bars
+    it = Items(sim, items, 9)
+
+    def producer():
+        g, idx = 0, 0
+        it.request()
+        while idx is not None:
+            yield from it.publish(items[idx])
+            yield ("wait", "R_EMPTY", r_empty_parity(it.n_pub))
+            load(sim, "R", "R_FULL", 4, "resident tiles")
+            for _ in range(items[idx]):
+                st = g % X_STAGES
+                yield ("wait", f"X_EMPTY{st}", ((g // X_STAGES) & 1) ^ 1)
+                load(sim, f"X{st}", f"X_FULL{st}", 4, f"streamed tile {g}")
+                g += 1
+            idx = yield from it.next()
+            if idx is not None:
+                it.request()
+        yield from it.publish(None)
+
+    def mma():
+        def issue_sdp(g, last):
+            st, b = g % X_STAGES, g & 1
+            yield ("wait", f"X_FULL{st}", (g // X_STAGES) & 1)
+
+            def run():
+                sim.expect("R", "full", "S / dP mma"), sim.expect(f"X{st}", "full", "S / dP mma"), sim.expect(f"S{b}", "free", "S / dP mma")
+                sim.set(f"S{b}", "s")
+            sim.pipe.append(run)
             sim.pipe.append(lambda: B[f"S_FULL{b}"].arrive())
-        yield ("wait", "R_FULL", 0)
-        yield from issue_sdp(0)
-        for t in range(n_steps):
-            if t + 1 < n_steps:
-                yield from issue_sdp(t + 1)
-            b, par = t & 1, (t >> 1) & 1
-            yield ("wait", f"P_FULL{b}", par)
+            if last:
+                sim.pipe.append(lambda: (sim.set("R", "free"), B["R_EMPTY"].arrive()))
+        g, n_it = 0, 0
+        while True:
+            n = yield from it.take(n_it)
+            if n is None:
+                return
+            yield ("wait", "R_FULL", n_it & 1)
+            yield from issue_sdp(g, n == 1)
+            for t in range(n):
+                if t + 1 < n:
+                    yield from issue_sdp(g + 1, t + 2 == n)
+                st, b = g % X_STAGES, g & 1
+                yield ("wait", f"P_FULL{b}", (g >> 1) & 1)
+                if t == 0:
+                    yield ("wait", "ACC_EMPTY", (n_it & 1) ^ 1)
 
-            def exec_acc(b=b, t=t):
-                sim.expect(f"P{b}", "full", f"accumulating mma {t}"); sim.expect(f"X{b}", "full", f"accumulating mma {t}")
-            sim.pipe.append(exec_acc)
-            sim.pipe.append(lambda b=b: (sim.set(f"X{b}", "free"), B[f"X_EMPTY{b}"].arrive()))
-            sim.pipe.append(lambda b=b: (sim.set(f"P{b}", "free"), B[f"P_EMPTY{b}"].arrive()))
-        sim.pipe.append(lambda: B["ACC_FULL"].arrive())
+                def run(st=st, b=b, was="acc" if t else "free"):
+                    sim.expect(f"S{b}", "p", "accumulating mma"), sim.expect(f"X{st}", "full", "accumulating mma")
+                    sim.expect("ACC", was, "accumulating mma")
+                    sim.set(f"S{b}", "free"), sim.set("ACC", "acc")
+                sim.pipe.append(run)
+                sim.pipe.append(lambda st=st: (sim.set(f"X{st}", "free"), B[f"X_EMPTY{st}"].arrive()))
+                if t == n - 1:
+                    sim.pipe.append(lambda: (sim.set("ACC", "done"), B["ACC_FULL"].arrive()))
+                g += 1
+            n_it += 1
 
-    def threads(w):
-        for t in range(n_steps):
-            b, par = t & 1, (t >> 1) & 1
-            yield ("wait", f"S_FULL{b}", par)
-            yield ("wait", f"P_EMPTY{b}", par ^ 1)
-            sim.expect(f"S{b}", "full", f"threads read S/dP {t}")
-            sim.expect(f"P{b}", "free", f"threads write P buffers {t}")
-            k = f"cnt{b}"
-            sim.state[k] = sim.state.get(k, 0) + 1
-            if sim.state[k] == 4:
-                sim.state[k] = 0
-                sim.set(f"S{b}", "free")
-                sim.set(f"P{b}", "full")
-            B[f"S_EMPTY{b}"].arrive()
-            B[f"P_FULL{b}"].arrive()
-        yield ("wait", "ACC_FULL", 0)
+    def elements(w):
+        g, n_it = 0, 0
+        while True:
+            n = yield from it.take(n_it)
+            if n is None:
+                return
+            for _ in range(n):
+                b = g & 1
+                yield ("wait", f"S_FULL{b}", (g >> 1) & 1)
+                sim.expect(f"S{b}", "s", f"element warps read S / dP of step {g}")
+                if count_down(sim, f"S{b}_warps", 8):
+                    sim.set(f"S{b}", "p")
+                B[f"P_FULL{b}"].arrive()
+                g += 1
+            yield ("wait", "ACC_FULL", n_it & 1)
+            sim.expect("ACC", "done", "output")
+            if count_down(sim, "ACC_warps", 8):
+                sim.set("ACC", "free")
+            B["ACC_EMPTY"].arrive()
+            n_it += 1
 
-    roles = {"producer": producer(), "mma": mma()}
-    for w in range(4):
-        roles[f"threads{w}"] = threads(w)
-    return roles
+    return {"producer": producer(), "mma": mma(), **{f"elements{w}": elements(w) for w in range(8)}}
 
 
-BWD_BARS = {"R_FULL": 1, "ACC_FULL": 1}
+BWD_BARS = {"R_FULL": 1, "R_EMPTY": 1, "ACC_FULL": 1, "ACC_EMPTY": 8, **ITEM_BARS}
 for _b in (0, 1):
-    BWD_BARS.update({f"X_FULL{_b}": 1, f"X_EMPTY{_b}": 1, f"S_FULL{_b}": 1, f"S_EMPTY{_b}": 4, f"P_FULL{_b}": 4, f"P_EMPTY{_b}": 1})
+    BWD_BARS.update({f"S_FULL{_b}": 1, f"P_FULL{_b}": 8})
+for _st in range(X_STAGES):
+    BWD_BARS.update({f"X_FULL{_st}": 1, f"X_EMPTY{_st}": 1})
 
 
-@pytest.mark.parametrize("n_steps", [1, 2, 3, 4, 7, 12])
-def test_backward_protocol_has_no_deadlock_or_buffer_hazard(n_steps):
-    for seed in range(150):
+@pytest.mark.parametrize("items", [[1], [2], [3], [4], [7], [12], [1, 1, 1, 1, 1], [2, 1, 3, 1], [5, 4, 3], [1, 8, 2, 1]], ids=str)
+def test_backward_protocol_has_no_deadlock_or_buffer_hazard(items):
+    for seed in range(100):
         sim = Sim(seed, BWD_BARS)
-        sim.run(bwd_protocol(sim, n_steps))
+        sim.run(bwd_protocol(sim, items))
+        assert all(v in ("free", 0) for v in sim.state.values()), sim.state
 
 
-def test_the_model_checker_catches_a_wrong_parity():
-    """Sanity of the checker itself: a producer that waits on the wrong phase is reported as a hazard or a deadlock."""
-    def broken(sim, n_steps):
-        roles = bwd_protocol(sim, n_steps)
-
-        def bad_producer():
-            B = sim.bars
-            B["R_FULL"].expect_tx(60)
-            sim.set("R", "loading")
-            sim.tma.append(lambda: (sim.set("R", "full"), B["R_FULL"].complete_tx(60)))
-            for t in range(n_steps):
-                b = t & 1
-                yield ("wait", f"X_EMPTY{b}", 1)   # BUG: constant parity instead of ((t >> 1) & 1) ^ 1
-                B[f"X_FULL{b}"].expect_tx(40)
-                sim.expect(f"X{b}", "free", f"X load of step {t}"); sim.set(f"X{b}", "loading")
-                sim.tma.append(lambda b=b: (sim.set(f"X{b}", "full"), B[f"X_FULL{b}"].complete_tx(40)))
-        roles["producer"] = bad_producer()
-        return roles
+@pytest.mark.parametrize("parity", [lambda n: 1, lambda n: (n & 1) ^ 1], ids=["constant", "inverted"])
+def test_the_model_checker_catches_a_wrong_parity(parity):
+    """Sanity of the checker itself: a producer that waits for the resident tiles on the wrong phase is reported as a hazard or a deadlock."""
     failures = 0
     for seed in range(40):
         sim = Sim(seed, BWD_BARS)
         try:
-            sim.run(broken(sim, 6))
+            sim.run(bwd_protocol(sim, [3, 2, 4, 2], r_empty_parity=parity))
         except AssertionError:
             failures += 1
     assert failures > 0

@@ -1,10 +1,10 @@
 """Tile-level emulation of the tcgen05 attention kernels (csrc/attn_fwd_tcgen05.cu, attn_bwd_tcgen05.cu) in PyTorch.
 
-The kernels could not be run when they were written, so their ALGORITHM -- tile ranges, mask predicates, the deferred fold of
-`T_j = P_j V_j` into the running output, the LSE convention, the transposed dKV pass with per-column statistics, the 64-row
-streamed blocks, the GQA head loop -- is mirrored here statement by statement (same names, same predicates, bf16 rounding of
-P / dS where the kernels round) and checked against the plain fp32 reference and its autograd.  A mistake in any of those
-shows up here; what this cannot check is the hardware protocol (barriers, descriptors, swizzles)."""
+The kernels' ALGORITHM -- which key tiles an item of two query tiles walks and which of the two takes part in each, mask predicates, the output that
+accumulates over the stream and is scaled when a row's maximum grows, the LSE convention, the transposed dKV pass with per-column
+statistics, the 64-row streamed blocks, the GQA head loop -- is mirrored here (same names, same predicates, bf16 rounding of P / dS where the
+kernels round) and checked against the plain fp32 reference and its autograd, or for the walk against the visible keys themselves.  A mistake in
+any of those shows up here; what this cannot check is the hardware protocol (barriers, descriptors, swizzles)."""
 import math
 
 import pytest
@@ -22,7 +22,7 @@ def _bf16(x):
 
 
 def emulate_fwd(q, k, v, cu, scale, causal):
-    """One "CTA" per (sequence, head, 128-row q tile); returns out [T,nq,D] and lse [nq,T]."""
+    """Per (sequence, head, 128-row q tile); scores in the log2 domain; returns out [T,nq,D] and lse [nq,T]."""
     T, nq, D = q.shape
     nkv = k.shape[1]
     out = torch.zeros(T, nq, D)
@@ -44,9 +44,7 @@ def emulate_fwd(q, k, v, cu, scale, causal):
                 Q[:n_in] = q[tok0 + q0: tok0 + q0 + n_in, head]
                 m_run = torch.full((kBQ,), -math.inf)
                 l_run = torch.zeros(kBQ)
-                alpha_prev = torch.zeros(kBQ)
                 O = torch.zeros(kBQ, D)
-                T_tiles = []
                 for j in range(n_kv):
                     kv0 = j * kBKV
                     K = torch.zeros(kBKV, D)
@@ -59,21 +57,20 @@ def emulate_fwd(q, k, v, cu, scale, causal):
                     lim = (torch.minimum(torch.tensor(L), q_pos + 1) if causal else torch.full((kBQ,), L)) - kv0
                     cols = torch.arange(kBKV)
                     masked = need_mask & (cols[None, :] >= lim[:, None])
-                    mx = S.masked_fill(masked, -math.inf).max(dim=1).values
+                    S = S.masked_fill(masked, -math.inf)
+                    mx = S.max(dim=1).values * sl2                     # the scale is positive: the maximum is taken over the raw products
                     m_new = torch.maximum(m_run, mx)
-                    m_eff = torch.where(torch.isinf(m_new) & (m_new < 0), torch.zeros_like(m_new), m_new)
-                    alpha = torch.exp2((m_run - m_eff) * sl2)
-                    P = torch.exp2(S * sl2 - (m_eff * sl2)[:, None]).masked_fill(masked, 0.0)
-                    l_run = l_run * alpha + P.sum(1)
+                    alpha = torch.where(m_new == m_run, torch.ones_like(m_new), torch.exp2(m_run - m_new))
+                    l_run = l_run * alpha
+                    O = O * alpha[:, None]                             # (the kernel skips this while no row of a warp has grown)
                     m_run = m_new
-                    T_tiles.append(_bf16(P) @ V)          # P is rounded to bf16 before the second MMA
-                    if j > 0:                             # fold of T_{j-1} is deferred by one iteration
-                        O = O * alpha_prev[:, None] + T_tiles[j - 1]
-                    alpha_prev = alpha
-                O = O * alpha_prev[:, None] + T_tiles[n_kv - 1]
+                    neg_m = torch.where(torch.isinf(m_run), torch.zeros_like(m_run), -m_run)
+                    P = torch.exp2(S * sl2 + neg_m[:, None])
+                    l_run = l_run + P.sum(1)
+                    O = O + _bf16(P) @ V                               # P is rounded to bf16 before the second product
                 ok = q_pos < L
                 out[tok0 + q_pos[ok], head] = (O / l_run[:, None])[ok]
-                lse[head, tok0 + q_pos[ok]] = (m_run * scale + torch.log(l_run))[ok]
+                lse[head, tok0 + q_pos[ok]] = (m_run * math.log(2) + torch.log(l_run))[ok]
     return out, lse
 
 
@@ -198,3 +195,60 @@ def test_backward_tile_algorithm_matches_autograd(lens, nq, nkv, hd, causal):
         dq, dk, dv = emulate_bwd(q.detach(), k.detach(), v.detach(), out, dout, lse, cu, scale, causal)
     for name, got, want in (("dq", dq, q.grad), ("dk", dk, k.grad), ("dv", dv, v.grad)):
         torch.testing.assert_close(got, want, atol=3e-2, rtol=3e-2, msg=lambda m, n=name: f"{n}: {m}")
+
+
+def _walk(L, qt0, qt1, causal, window, keep, chunk):
+    """The key tiles of an item in order, each with (tile 0 takes part, tile 1 takes part)."""
+    win = window if causal and window > 0 else 0
+    keep_tiles = -(-keep // kBKV) if win > 0 else 0
+
+    def first(qt):
+        q0 = qt * kBQ
+        return q0 // chunk * chunk // kBKV if chunk > 0 else max(0, q0 - win + 1) // kBKV if win > 0 else 0
+
+    def end(qt):
+        return 0 if qt < 0 else -(-(min(L, qt * kBQ + kBQ) if causal else L) // kBKV)
+    firsts, ends = (first(qt0), first(qt0) if qt1 < 0 else first(qt1)), (end(qt0), end(qt1))
+    lo = min(firsts)
+    nk = min(keep_tiles, lo)
+    for k in range(nk + max(ends) - lo):
+        j = k if k < nk else lo + k - nk
+        yield j, tuple(j < ends[t] and (j >= firsts[t] or j < keep_tiles) for t in range(2))
+
+
+def _softmax_tiles(L, qt, causal, window, keep, chunk):
+    """The key tiles that the softmax warps of a query tile go through."""
+    win, q0 = (window if causal and window > 0 else 0), qt * kBQ
+    first_tile = q0 // chunk * chunk // kBKV if chunk > 0 else max(0, q0 - win + 1) // kBKV if win > 0 else 0
+    n_keep = min(-(-keep // kBKV), first_tile) if win > 0 else 0
+    n = n_keep + -(-(min(L, q0 + kBQ) if causal else L) // kBKV) - first_tile
+    return [k if k < n_keep else first_tile + k - n_keep for k in range(n)]
+
+
+@pytest.mark.parametrize("pair_heads", [True, False])
+@pytest.mark.parametrize("causal,window,keep,chunk", [(True, 0, 0, 0), (False, 0, 0, 0), (True, 1, 0, 0), (True, 100, 0, 0), (True, 128, 1, 0), (True, 200, 130, 0),
+                                                      (True, 300, 600, 0), (True, 5000, 64, 0), (True, 0, 0, 1), (True, 0, 0, 90), (True, 0, 0, 256), (True, 0, 0, 300)])
+def test_forward_item_walk_covers_exactly_the_visible_tiles(pair_heads, causal, window, keep, chunk):
+    """Both roles of the kernel agree on the tiles of each query tile and their order; every visible key lies in one of them; every tile walked is taken by
+    somebody; the items of a sequence cover its query tiles once."""
+    for L in (1, 127, 128, 129, 256, 300, 513, 1100):
+        tiles = -(-L // kBQ)
+        last, units = tiles - 1, tiles if pair_heads else -(-tiles // 2)
+        items = [(last - r, last - r) if pair_heads else (last - 2 * r, last - 2 * r - 1) for r in range(units)]
+        covered = sorted(q for it in items for q in (it[:1] if pair_heads else it) if q >= 0)
+        assert covered == list(range(tiles))
+        for qt0, qt1 in items:
+            walk = list(_walk(L, qt0, qt1, causal, window, keep, chunk))
+            assert all(any(t) for _, t in walk)
+            for t, qt in enumerate((qt0, qt1)):
+                taken = [j for j, takes in walk if takes[t]]
+                assert taken == ([] if qt < 0 else _softmax_tiles(L, qt, causal, window, keep, chunk))
+                if qt < 0:
+                    continue
+                i, j = torch.arange(qt * kBQ, min(L, qt * kBQ + kBQ))[:, None], torch.arange(L)[None]
+                ok = (j <= i) if causal else torch.ones(i.numel(), L, dtype=torch.bool)
+                if chunk:
+                    ok = ok & (j // chunk == i // chunk)
+                elif window:
+                    ok = ok & ((j > i - window) | (j < keep))
+                assert set((ok.any(0).nonzero().flatten() // kBKV).tolist()) <= set(taken)
