@@ -223,6 +223,57 @@ def test_capped_scores(cap, sink, hd, form):
         a += n
 
 
+@pytest.mark.parametrize("heads", [(1, 1, 128), (4, 2, 64), (3, 1, 128), (8, 1, 128), (8, 8, 64), (16, 4, 128)])
+@pytest.mark.parametrize("lens", [[1], [127, 128, 129, 255, 256, 257], [0, 5, 0, 640, 1], [33] * 70 + [1100], [1536, 385], [640] * 12],
+                         ids=lambda x: f"{len(x)}x{x[0]}")
+@pytest.mark.parametrize("causal", [True, False])
+def test_attn_bwd_items(heads, lens, causal):
+    """The backward where CTAs take several items (up to 960 of them), one to three query heads and whole groups a key head, left-over rows and blocks,
+    empty sequences and more than 32 of them, in both types; `out` starts off a 16-byte boundary for an odd number of sequences.  Against float64
+    gradients from the same 16-bit inputs.  Bound: P and dS are rounded to 16 bits once (half an ulp, doubled for exp2 and its argument; values under
+    fp16's normal range lose half of its smallest step), dP and delta are fp32 sums whose difference cancels (2^-16 of the sum of magnitudes), and the
+    result is rounded once."""
+    nq, nkv, hd = heads
+    dt = torch.float16 if nq % 4 else torch.bfloat16
+    eps, tiny = (2.0 ** -8, 0.0) if dt == torch.bfloat16 else (2.0 ** -11, 2.0 ** -24)
+    torch.manual_seed(len(lens) + nq)
+    T, scale, rep = sum(lens), hd ** -0.5, nq // nkv
+    cu = torch.tensor([0] + list(torch.tensor(lens).cumsum(0)), dtype=torch.int32, device=DEV)
+    qkv = torch.randn(T, (nq + 2 * nkv) * hd, device=DEV).to(dt)
+    dout = torch.randn(T, nq, hd, device=DEV).to(dt)
+    split = lambda t: [x.view(T, -1, hd) for x in t.split([nq * hd, nkv * hd, nkv * hd], 1)]
+    q, k, v = split(qkv)
+    out = torch.empty(T * nq * hd + 1, device=DEV, dtype=dt)[len(lens) % 2:][:T * nq * hd].view(T, nq, hd)
+    lse = torch.empty(nq, T, device=DEV)
+    want, bound = [torch.zeros(T, n, hd, dtype=torch.float64, device=DEV) for n in (nq, nkv, nkv)], []
+    bound = [torch.zeros_like(t) for t in want]
+    a = 0
+    for n in lens:
+        r = slice(a, a + n)
+        a += n
+        qq, dd = (t[r].double().transpose(0, 1) for t in (q, dout))
+        kk, vv = (t[r].double().transpose(0, 1).repeat_interleave(rep, 0) for t in (k, v))
+        s = qq @ kk.transpose(1, 2) * scale
+        if causal:
+            s = s.masked_fill(torch.ones(n, n, dtype=torch.bool, device=DEV).triu(1), float("-inf"))
+        P = torch.softmax(s, -1)
+        lse[:, r] = torch.logsumexp(s, -1).float()
+        out[r] = (P @ vv).transpose(0, 1).to(dt)
+        oo = out[r].double().transpose(0, 1)                 # delta is defined by the rounded output
+        dP, mag = dd @ vv.transpose(1, 2), dd.abs() @ vv.abs().transpose(1, 2) + (dd * oo).abs().sum(-1, keepdim=True)
+        dS = P * (dP - (dd * oo).sum(-1, keepdim=True)) * scale
+        e_s, e_p = eps * dS.abs() + 2.0 ** -16 * P * mag * scale + tiny * (P > 0), eps * P + tiny * (P > 0)
+        group = lambda t: t.view(nkv, rep, n, hd).sum(1).transpose(0, 1)
+        want[0][r], bound[0][r] = (dS @ kk).transpose(0, 1), (e_s @ kk.abs()).transpose(0, 1)
+        want[1][r], bound[1][r] = group(dS.transpose(1, 2) @ qq), group(e_s.transpose(1, 2) @ qq.abs())
+        want[2][r], bound[2][r] = group(P.transpose(1, 2) @ dd), group(e_p.transpose(1, 2) @ dd.abs())
+    dqkv = torch.full_like(qkv, float("nan"))                # every element must be written
+    lib().attn_bwd(dout, q, k, v, out, lse, *split(dqkv), cu, max(lens), scale, causal)
+    assert lib().attn_wait_error() == 0
+    for got, w, b in zip(split(dqkv), want, bound):
+        assert ((got.double() - w).abs() <= b + eps * w.abs() + 1e-6).all()
+
+
 def test_a_wait_that_ran_out_is_raised_and_the_update_skipped():
     """The status word as a kernel leaves it whose bounded wait ran out (set here by a copy): the next attention call of either direction and the
     engine raise, the optimizer leaves the parameters alone, and clearing the word makes everything run again."""
