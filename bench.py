@@ -397,7 +397,7 @@ def main():
     gen_mbs = 1  # one decode pass over all local sequences: weights are streamed once per token (KV cache 43 GB at N=1)
     inf_mbs = 2 if per_rank * (args.prompt_len + args.new_tokens) > 48 * 1024 else 1
     # On one GPU the 43 GB KV cache must be freed before training, so the decode graph is re-captured every step (~0.15-0.3 s per
-    # generate call: profiles/bench_n1_r2_gen_phases.log); at N=2 keeping the 21.5 GB cache resident costs 7 un-recomputed blocks of
+    # generate call); at N=2 keeping the 21.5 GB cache resident costs 7 un-recomputed blocks of
     # the activation budget and loses more in training than it gains in generation (measured 9.9 k vs 10.1 k tokens/s).  From 4 GPUs
     # on the cache (<= 10.7 GB per GPU) stays resident together with the captured graph, like the reference's default
     # (`force_cudagraph_recapture=False`).

@@ -3,8 +3,7 @@ single-token decode attention over a dense KV cache.
 
 CUDA tensors: decode runs the split-KV sm_100a kernel in `csrc/attn_decode.cu` (with fused RoPE and
 in-place KV append); varlen forward runs `csrc/attn_fwd_tcgen05.cu` and backward `csrc/attn_bwd_tcgen05.cu`
-(TMA + tcgen05 + TMEM; head dim 64 / 128, validated on B200 against the fp32 reference and the library kernel:
-`profiles/attention_validation.log`).  The flash-attn library kernel is only the fallback for what the own
+(TMA + tcgen05 + TMEM; head dim 64 / 128).  The flash-attn library kernel is only the fallback for what the own
 kernels do not cover (attention dropout, other head dims) and the A/B arm: `REAL_ATTN=flash` /
 `REAL_ATTN_BWD=flash` select it explicitly; both produce / consume the same LSE layout.
 CPU tensors: plain PyTorch reference (also the numerics oracle for the tests).
