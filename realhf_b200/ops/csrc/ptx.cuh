@@ -129,14 +129,6 @@ __device__ __forceinline__ void tc_ld_32x32(uint32_t taddr, uint32_t* r) {
       : "memory");
 }
 
-// the same with 16 columns
-__device__ __forceinline__ void tc_ld_32x16(uint32_t taddr, uint32_t* r) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]),
-                 "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-               : "r"(taddr)
-               : "memory");
-}
 __device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 // thread i of the warp writes 32 consecutive 32-bit columns of row (lane_base + i)
 __device__ __forceinline__ void tc_st_32x32(uint32_t taddr, const uint32_t* r) {

@@ -95,8 +95,8 @@ template <typename V> RB_DEVICE V block_inclusive(V v, V* red, V& total) {
   return (warp == 0 ? V(0) : base) + incl;
 }
 
-// The k-th largest of the block's keys, kPer of them per thread (a thread without one passes 0: it is never counted, and k never exceeds
-// the number of real keys).  One counting barrier per bit and key.
+// The k-th largest of the block's keys, kPer of them per thread (a thread without one passes 0, which is never counted), or 0 if there are fewer than k:
+// no bound, and every element is a candidate (thread maxima: with 16-byte loads V elements have V / 4 or V / 8).  One counting barrier per bit and key.
 template <int kPer> RB_DEVICE uint32_t kth_largest(const uint32_t (&key)[kPer], int k) {
   uint32_t prefix = 0;
 #pragma unroll 1

@@ -150,27 +150,6 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None
     return _Linear.apply(x, w, bias)
 
 
-def pad_groups(offsets: torch.Tensor, n_rows: int, block: int = 64):
-    """Row map that pads every group's block of a group-sorted [n_rows, *] tensor to a multiple of `block` rows, computed on
-    the device (no host read of the group sizes).  Returns (dest [n_rows] int64: padded position of every source row,
-    offsets_pad [G + 1] int32: padded block starts, n_pad: static upper bound of padded rows, a multiple of `block`).
-    Rows outside [offsets[0], offsets[G]) belong to no group (an expert-parallel rank that only owns a sub-range of the sorted
-    rows; the unused tail of a receive buffer): their `dest` is n_pad, one row past the padded tensor -- callers allocate
-    n_pad + 1 rows and hand the first n_pad to the kernel, so stale data never lands in a group's zero padding."""
-    G = offsets.numel() - 1
-    off = offsets.long()
-    counts = off[1:] - off[:-1]
-    padded = (counts + block - 1) // block * block
-    off_pad = torch.zeros(G + 1, dtype=torch.long, device=offsets.device)
-    off_pad[1:] = padded.cumsum(0)
-    rows = torch.arange(n_rows, device=offsets.device)
-    g = torch.bucketize(rows, off[1:], right=True).clamp_(max=G - 1)
-    n_pad = (n_rows + G * (block - 1) + block - 1) // block * block
-    dest = rows + (off_pad[:-1] - off[:-1])[g]
-    dest = torch.where((rows >= off[0]) & (rows < off[G]), dest, torch.full_like(dest, n_pad))
-    return dest, off_pad.int(), n_pad
-
-
 def grouped_wgrad_ref(dy, x, offsets, G):
     """fp32 reference: dW[g] = dy[rows of g]^T @ x[rows of g]."""
     off = offsets.tolist()

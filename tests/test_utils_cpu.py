@@ -149,51 +149,36 @@ def test_metric_sinks_jsonl_tensorboard_and_failing_sink(tmp_path, monkeypatch):
     assert [e.step for e in acc.Scalars("actor_train/loss")] == [1, 2, 3]
 
 
-def test_group_padding_for_the_grouped_wgrad_kernel():
-    """The dispatch-side contract of csrc/gemm_grouped_wgrad.cu: blocks start at multiples of 64, padding rows are zero, and
-    the per-expert products over the PADDED blocks equal the products over the original ragged blocks."""
+def test_grouped_wgrad_walks_unpadded_rows():
+    """The walk of csrc/gemm_grouped_wgrad.cu over the rows of an expert: blocks of 64 rows from its first one, a partial last block first, whose rows of the
+    next expert (or of nobody) are zeroed in both operands.  Rows outside every expert's range (an expert-parallel rank's foreign rows, the unused
+    tail of a receive buffer) may hold anything; an expert without rows gets zeros."""
     import torch
-    from realhf_b200.ops.gemm import grouped_wgrad_ref, pad_groups
+    from realhf_b200.ops.gemm import grouped_wgrad_ref
     torch.manual_seed(0)
-    for counts in ([5, 0, 64, 130, 1], [0, 0, 7], [128, 64], [1] * 9, [0, 0]):
-        G, T = len(counts), sum(counts)
-        offsets = torch.tensor([0] + list(torch.tensor(counts).cumsum(0)), dtype=torch.int32)
+    for first, counts, rest in ((0, [5, 0, 64, 130, 1], 0), (0, [0, 0, 7], 3), (0, [128, 64], 0), (37, [70, 0, 5], 188), (3, [1] * 9, 1), (2, [0, 0], 2)):
+        offsets = torch.tensor([first] + counts).cumsum(0).int()
+        T = first + sum(counts) + rest
         dy, x = torch.randn(T, 16), torch.randn(T, 24)
-        dest, off_pad, n_pad = pad_groups(offsets, T)
-        assert n_pad % 64 == 0 and int(off_pad[-1]) <= n_pad and all(int(o) % 64 == 0 for o in off_pad)
-        assert [int(b - a) for a, b in zip(off_pad[:-1], off_pad[1:])] == [(c + 63) // 64 * 64 for c in counts]
-        assert dest.numel() == T and (T == 0 or dest.unique().numel() == T)
-        dy_p = torch.zeros(n_pad, 16).index_copy_(0, dest, dy)
-        x_p = torch.zeros(n_pad, 24).index_copy_(0, dest, x)
-        for g in range(G):   # rows land inside their own block, in order
-            a, b = int(offsets[g]), int(offsets[g + 1])
-            torch.testing.assert_close(dy_p[int(off_pad[g]): int(off_pad[g]) + (b - a)], dy[a:b])
-            assert float(dy_p[int(off_pad[g]) + (b - a): int(off_pad[g + 1])].abs().sum()) == 0.0
-        got = torch.stack([dy_p[int(off_pad[g]): int(off_pad[g + 1])].t() @ x_p[int(off_pad[g]): int(off_pad[g + 1])] for g in range(G)])
-        torch.testing.assert_close(got, grouped_wgrad_ref(dy, x, offsets, G), atol=1e-4, rtol=1e-4)
-
-
-def test_group_padding_drops_rows_that_belong_to_no_group():
-    """An expert-parallel rank hands the grouped wgrad the offsets of ITS experts inside the globally sorted rows (offsets[0] > 0,
-    rows of foreign experts before and after), and a receive buffer has an unused tail: those rows must land in the spare row
-    past the padded tensor, never inside a group's zero padding."""
-    import torch
-    from realhf_b200.ops.gemm import grouped_wgrad_ref, pad_groups
-    torch.manual_seed(1)
-    T = 300
-    offsets = torch.tensor([37, 37 + 70, 37 + 70, 37 + 70 + 5], dtype=torch.int32)   # 3 groups inside rows [37, 112)
-    dy, x = torch.randn(T, 8), torch.randn(T, 12)
-    dest, off_pad, n_pad = pad_groups(offsets, T)
-    outside = torch.cat([torch.arange(0, 37), torch.arange(112, T)])
-    assert (dest[outside] == n_pad).all() and int(dest.min()) >= 0
-    inside = dest[37:112]
-    assert inside.unique().numel() == 75 and int(inside.max()) < int(off_pad[-1])
-    dy_p = torch.zeros(n_pad + 1, 8).index_copy_(0, dest, dy)[:n_pad]
-    x_p = torch.zeros(n_pad + 1, 12).index_copy_(0, dest, x)[:n_pad]
-    got = torch.stack([dy_p[int(off_pad[g]): int(off_pad[g + 1])].t() @ x_p[int(off_pad[g]): int(off_pad[g + 1])] for g in range(3)])
-    off = offsets.tolist()
-    ref = torch.stack([dy[off[g]:off[g + 1]].t() @ x[off[g]:off[g + 1]] for g in range(3)])
-    torch.testing.assert_close(got, ref, atol=1e-4, rtol=1e-4)
+        for t in (dy, x):
+            t[:first] = float("nan")
+            t[T - rest:] = float("nan")
+        got = torch.zeros(len(counts), 16, 24)
+        for g in range(len(counts)):
+            r0, rows = int(offsets[g]), int(offsets[g + 1] - offsets[g])
+            nkb = (rows + 63) // 64
+            tail = rows - (nkb - 1) * 64
+            seen = []
+            for kb in range(nkb):
+                block = kb if tail == 64 else nkb - 1 if kb == 0 else kb - 1
+                k0 = r0 + block * 64
+                a, b = (torch.nn.functional.pad(t[k0:k0 + 64], (0, 0, 0, max(0, k0 + 64 - T))) for t in (dy, x))      # TMA fills past the end with zeros
+                if kb == 0 and tail < 64:
+                    a[tail:], b[tail:] = 0, 0
+                got[g] += a.t() @ b
+                seen.append(block)
+            assert sorted(seen) == list(range(nkb))
+        torch.testing.assert_close(got, grouped_wgrad_ref(dy, x, offsets, len(counts)), atol=1e-4, rtol=1e-4)
 
 
 def test_bench_clock_sampler_queries_one_gpu_per_tick(monkeypatch):
