@@ -298,3 +298,20 @@ def test_gemm_accumulates_into_ragged_outputs(out_dt, M, N, K, shift):
     assert ((out.double() - ref).abs() <= (2.0 ** -8 if out_dt == torch.bfloat16 else 0.0) * ref.abs() + 2.0 ** -20 * mag).all()
     buf[1:M + 1, shift:shift + N] = before[1:M + 1, shift:shift + N]
     assert torch.equal(buf, before)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("M,N,K,shift", [(288, 256, 64, 0), (300, 512, 128, 8), (1000, 776, 72, 0), (257, 264, 512, 0), (512, 256, 64, 4)])
+def test_gemm_cta_pair_output_edges(M, N, K, shift, dtype):
+    """16-bit outputs of the CTA-pair kernel: whole 32 x 64 pieces leave in their own type, the rest through fp32 staging (last rows and columns, rows off a
+    16-byte boundary); what surrounds the output stays as it is.  Bound: fp32 sums of K products (2^-22 of their magnitudes) and one rounding."""
+    torch.manual_seed(M + N)
+    a, b = torch.randn(M, K, device=DEV).to(dtype), torch.randn(N, K, device=DEV).to(dtype)
+    wide = torch.full((M + 2, N + 24), 7.0, device=DEV, dtype=dtype)
+    out = wide[1:M + 1, 8 + shift:8 + shift + N]
+    G.gemm(a, b, out=out, mc=2)
+    ref, mag = a.double() @ b.double().t(), a.double().abs() @ b.double().abs().t()
+    eps = 2.0 ** (-9 if dtype == torch.bfloat16 else -12)
+    assert ((out.double() - ref).abs() <= 2 * eps * ref.abs() + 2.0 ** -22 * mag + 2.0 ** -24).all()
+    out.fill_(7.0)
+    assert (wide == 7.0).all()
