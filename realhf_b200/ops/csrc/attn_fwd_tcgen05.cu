@@ -11,7 +11,7 @@
 // rows (grouped heads, even group: both walk the same tiles), else two neighbouring query tiles of a head (counted from the end of
 // the sequence, so that a left-over single tile is the shortest one).  Sharing the stream also halves the L2 traffic per product: one
 // tile each would ask for 64 B per cycle and SM, more than L2 gives.  With one tile per CTA and four softmax warps the tensor pipe was
-// active 19% of the time: 32 x 640 tokens x 32 heads took 527 us (now 221), 8 x 1500..4096 x 32 / 8 heads 2396 us (now 751).
+// active 19% of the time: 32 x 640 tokens x 32 heads took 518 us (now 228), 8 x 1500..4096 x 32 / 8 heads (26655 tokens) 2365 us (now 818).
 //
 // CTA = 12 warps, one CTA per SM.  Warps 0-3 / 4-7: softmax of tile 0 / 1 (thread = query row = TMEM lane).  Warp 8: MMA issue and TMEM
 // allocation.  Warp 9: TMA producer and scheduler (10, 11: idle, they complete the warpgroup whose registers go to the softmax).  The
@@ -28,7 +28,7 @@
 // 1 when P is rounded to 16 bits: error against 64 bits 0.0028 instead of 0.0025.)  V_j is the MN-major B operand.
 // Issue order: S_0, S_1, then per key tile PV_0, S_0', PV_1, S_1'.  The issuing warp runs converged and elects a lane for the MMAs alone: issued from
 // `if (lane == 0)` with descriptors built there, eight MMAs took 820-960 cycles of one thread, whatever their size (294 -> 242 us converged, 231 us with the
-// descriptors built in front of the elected branch; two scores per instruction in the softmax: 221 us; 229 us with the maximum of every tile).
+// descriptors built in front of the elected branch; two scores per instruction in the softmax: 221 us; 228 us with the maximum of every tile).
 //
 // Outputs: O [T, nq, DV] through a per-warp staging buffer (whole 128-byte lines), LSE [nq, T] (natural log, scale applied).
 //
@@ -38,7 +38,7 @@
 // maximum is taken over the raw products.  kCap: kSimple with score = softcap * tanh(s * scale / softcap), formed before the
 // masks, so that a product that overflowed to -infinity is a visible score of -softcap.  All three: a per-head sink logit starts the running maximum with denominator 1; the output is
 // multiplied by sigmoid(gate logit of its head, or of the output element); `chunk` > 0 replaces the window: a query sees the keys of its own
-// chunk of positions up to itself.  (32 x 1024 tokens, 16 / 4 heads, window 512 + 64 kept: 1382 us with one tile per CTA, now 269.)
+// chunk of positions up to itself.  (32 x 1024 tokens, 16 / 4 heads, window 512 + 64 kept: 1350 us with one tile per CTA, now 278.)
 // Learned distance biases and shared keys / values run in attn_fwd_bias.cu.
 #include "attn_common.cuh"
 

@@ -732,8 +732,8 @@ static int streamk_impl(const void* A, const void* B, void* C, const void* bias,
         double t = cta_bytes / 70e3;                              // us
         const double hbm = (double)N * K * esz / 6.5e6;           // us
         if (t < hbm) t = hbm;
-        // per-k-block term: 0.2 .. 0.25 measured; with 0.33 the layout picked is within 3 % of the best of a sweep over widths and splits
-        // (16 and 64 rows; 12.6 against 11.4 us at 4096 x 4096)
+        // per-k-block term: 0.2 .. 0.25 measured; with 0.33 the layouts picked are within 3 % of the best of a sweep over widths and splits
+        // (16 and 64 rows), but for 4096 x 4096 at 16 rows: 12.6 against 11.4 us
         const double kb_floor = 0.33 * RB_CEIL_DIV(num_kb, sp) * waves;
         if (t < kb_floor) t = kb_floor;
         if (sp > 1) t += 5.0 + 4.5 * (double)M * cand * 4.0 / 60e3;  // partial write + barrier + cooperative reduce (measured)
