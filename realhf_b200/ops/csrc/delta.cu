@@ -294,11 +294,16 @@ __global__ void __launch_bounds__(kScanThreads, LPC <= 8 ? 3 : 2) delta_rule_ker
   constexpr int kBuf = (kChan ? 3 : 2) * kTok * dpad + kTok * NCOL + 2 * kTok;   // floats of one staging buffer: q, k, v, (beta, g), row decays
   constexpr int NQ = kTok * dpad / kScanThreads, NV = (kTok * NCOL + kScanThreads - 1) / kScanThreads;
   auto row_of = [&](int e) { return ((e >> 2) * LPC + l) * 4 + (e & 3); };
+  // Up to 16 lanes the zeros start at an index that the compiler cannot know to be 0 (no head count is negative), so they reach the registers through local
+  // memory, once: with constants in front of it the token loop gets a worse schedule (8 sequences of 700..1024 tokens, 16 heads x 128 x 128: 687 us
+  // against 620, the whole prefill 715 against 669; with registers for four CTAs an SM 612 and 703).  For 32 lanes constants are better (2 x 512 tokens,
+  // 4 heads x 512 x 512: 372 us against 395).
+  const int first = LPC < 32 ? min(p.H, 0) : 0;
   uint64_t Z[NC][kRows / 2];
 #pragma unroll
   for (int j = 0; j < NC; ++j)
 #pragma unroll
-    for (int e = 0; e < kRows / 2; ++e) Z[j][e] = 0;
+    for (int e = first; e < kRows / 2; ++e) Z[j][e] = 0;
   // The inputs of the next 8 tokens are fetched into registers while the current 8 are processed out of shared memory (two staging buffers).
   float rq[NQ], rk[NQ], rg[kChan ? NQ : 1], rv[NV], rb = 0.f;
   auto fetch = [&](int tb) {
