@@ -9,11 +9,11 @@
 
 using at::Tensor;
 
-extern "C" int rb_decode_attention(const void* qkv, void* k_cache, void* v_cache, const int* cache_lens, void* out,
-                                   float* part_acc, float* part_ml, const float* cos, const float* sin, int64_t qkv_stride,
-                                   int64_t kb, int64_t ks, int64_t kh, int64_t vb, int64_t vs, int64_t vh, int B, int nq,
-                                   int nkv, int hd, int S_max, int splits, int rot_dim, int interleaved, float scale, int dt,
-                                   cudaStream_t s);
+extern "C" int rb_decode_attention(const void* qkv, void* k_cache, void* v_cache, const int* cache_lens, void* out, const float* cos,
+                                   const float* sin, int64_t qkv_stride, int64_t kb, int64_t ks, int64_t kh, int64_t vb, int64_t vs, int64_t vh,
+                                   int B, int nq, int nkv, int hd, int S_max, int rot_dim, int interleaved, float scale, int dt, cudaStream_t s);
+
+void attn_check();
 
 // qkv [B, (nq+2nkv)*hd]; caches logical [B, S, nkv, hd] (any b/s/h strides, unit hd stride); cache_lens int32 [B].
 Tensor decode_attention(const Tensor& qkv, Tensor k_cache, Tensor v_cache, const Tensor& cache_lens, int64_t nq, int64_t nkv,
@@ -24,25 +24,11 @@ Tensor decode_attention(const Tensor& qkv, Tensor k_cache, Tensor v_cache, const
   TORCH_CHECK(k_cache.scalar_type() == qkv.scalar_type() && v_cache.scalar_type() == qkv.scalar_type());
   TORCH_CHECK(cache_lens.scalar_type() == at::kInt && cache_lens.is_contiguous());
   TORCH_CHECK(qkv.size(1) == (nq + 2 * nkv) * hd && nq % nkv == 0);
+  attn_check();
   const int B = qkv.size(0);
   const int S = k_cache.size(1);
   c10::cuda::CUDAGuard guard(qkv.device());
   auto out = at::empty({B, nq * hd}, qkv.options());
-  // Split the KV range of a (sequence, kv head) over several CTAs only when there are fewer than two CTAs per SM.  Measured on
-  // B200 at B=16 x 32 heads (512 CTAs, ctx 384): forcing 2-3 splits made the 4-layer decode step 4% SLOWER (565 -> 588 us;
-  // the reduce kernel's launch + the partial round trip cost more than the extra loads in flight buy), so the threshold stays
-  // low; `REAL_DECODE_CTAS_PER_SM` overrides it for experiments.
-  static const int target = [] { const char* e = getenv("REAL_DECODE_CTAS_PER_SM"); return e ? atoi(e) : 2; }();
-  int splits = 1;
-  const int64_t ctas = (int64_t)B * nkv;
-  if (ctas < (int64_t)target * 148 && S >= 512) {
-    splits = (int)std::min<int64_t>(16, ((int64_t)target * 148 + ctas - 1) / ctas);
-  }
-  Tensor pa, pm;
-  if (splits > 1) {
-    pa = at::empty({B, nq, splits, hd}, qkv.options().dtype(at::kFloat));
-    pm = at::empty({B, nq, splits, 2}, qkv.options().dtype(at::kFloat));
-  }
   const float *cp = nullptr, *sp = nullptr;
   if (cos.has_value()) {
     TORCH_CHECK(sin.has_value() && cos->scalar_type() == at::kFloat && cos->is_contiguous() && sin->is_contiguous());
@@ -50,11 +36,10 @@ Tensor decode_attention(const Tensor& qkv, Tensor k_cache, Tensor v_cache, const
     sp = sin->data_ptr<float>();
   }
   const int dt = qkv.scalar_type() == at::kBFloat16 ? 1 : (qkv.scalar_type() == at::kHalf ? 2 : -1);
-  int rc = rb_decode_attention(qkv.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), cache_lens.data_ptr<int>(), out.data_ptr(),
-                               splits > 1 ? pa.data_ptr<float>() : nullptr, splits > 1 ? pm.data_ptr<float>() : nullptr, cp, sp,
-                               qkv.stride(0), k_cache.stride(0), k_cache.stride(1), k_cache.stride(2), v_cache.stride(0),
-                               v_cache.stride(1), v_cache.stride(2), B, (int)nq, (int)nkv, (int)hd, S, splits, (int)rot_dim,
-                               interleaved, (float)scale, dt, at::cuda::getCurrentCUDAStream().stream());
+  int rc = rb_decode_attention(qkv.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), cache_lens.data_ptr<int>(), out.data_ptr(), cp, sp,
+                               qkv.stride(0), k_cache.stride(0), k_cache.stride(1), k_cache.stride(2), v_cache.stride(0), v_cache.stride(1),
+                               v_cache.stride(2), B, (int)nq, (int)nkv, (int)hd, S, (int)rot_dim, interleaved, (float)scale, dt,
+                               at::cuda::getCurrentCUDAStream().stream());
   TORCH_CHECK(rc == 0, "decode_attention: unsupported configuration (", rc, ")");
   return out;
 }

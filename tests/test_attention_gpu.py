@@ -48,6 +48,35 @@ def test_decode_attention(cfg, rope, layout):
     assert torch.equal(vc, vc_ref)
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("nq,nkv,S", [(5, 5, 200), (6, 3, 131), (16, 4, 700), (8, 1, 4096), (256, 256, 70), (4, 2, 9)])
+def test_decode_attention_step_edges(nq, nkv, S, hd, dtype):
+    """Lengths around the 16-row steps of a warp and the 64-row steps of a CTA, few pairs (split over a cluster) and many, and cache rows that
+    nobody has written yet (NaN), against float64.  Bound: the result's rounding (a relative 2^-8 for bf16's 8 significant bits, 2^-11 for fp16's 11), plus what fp32 scores and sums
+    leave: scores of |s| < 64 carry 128 products of relative error 2^-24 each, so weights differ by less than 64 * 128 * 2^-24 / 16 = 3e-5."""
+    edges = [0, 1, 15, 16, 17, 63, 64, 65, 127, 129, 255, 1000, 4095]
+    lens = [n for n in edges if n < S]
+    B = len(lens)
+    g = torch.Generator(device=DEV).manual_seed(nq * 1000 + hd)
+    rnd = lambda *s: torch.randn(*s, device=DEV, generator=g).to(dtype)  # noqa: E731
+    kc, vc = rnd(B, nkv, S, hd).permute(0, 2, 1, 3), rnd(B, S, nkv, hd)
+    for b, n in enumerate(lens):
+        kc[b, n:] = float("nan")
+        vc[b, n:] = float("nan")
+    qkv = rnd(B, (nq + 2 * nkv) * hd)
+    qkv[:, : nq * hd] *= 3
+    q, k, v = (t.reshape(B, -1, hd).double() for t in qkv.split([nq * hd, nkv * hd, nkv * hd], 1))
+    out = A.decode_attention(qkv, kc, vc, torch.tensor(lens, dtype=torch.int32, device=DEV), nq, nkv, hd).view(B, nq, hd)
+    for b, n in enumerate(lens):
+        assert torch.equal(kc[b, n].double(), k[b]) and torch.equal(vc[b, n].double(), v[b])
+        kk, vv = (torch.repeat_interleave(t[b, : n + 1].double(), nq // nkv, 1) for t in (kc, vc))
+        ref = torch.einsum("hn,nhd->hd", torch.softmax(torch.einsum("hd,nhd->hn", q[b], kk) * hd ** -0.5, -1), vv)
+        rounding = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+        bound = rounding * ref.abs() + 3e-5 * vv.abs().amax(0).amax(-1).unsqueeze(-1)
+        assert bool(((out[b].double() - ref).abs() <= bound).all()), (n, float((out[b].double() - ref).abs().max()))
+
+
 @pytest.mark.parametrize("heads", [(8, 8), (8, 2)])
 def test_packed_qkv_attention_forward_backward(heads):
     """Fused-QKV varlen attention (one d(qkv) buffer written by the backward kernel) vs the fp32 reference on sliced q/k/v."""
