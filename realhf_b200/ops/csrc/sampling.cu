@@ -5,12 +5,14 @@
 // Categorical, gather, mask compare: nn/real_llm_generate.py:26-141, utils/logits_warper.py) — about 1 ms per decode
 // step at [128, 32000].  The row is staged once in shared memory as fp32 (V * 4 bytes <= 200 KB).
 //
-// Nothing here is bound by bytes (8 MB at [128, 32000]): a row's time is the chain of block-wide steps.  A radix descent over the whole row
-// (4 digits each for top-k and top-p) spends them on shared atomics that pile up on the few bins logits fall in: 89 us at
-// [128, 32000], top-k 50, top-p 0.9.  For top_k <= 512 the row is therefore cut down first: the k-th largest of the 1024 per-thread maxima is
-// a lower bound of the k-th largest logit (those are k elements at least as large), and only a few hundred elements reach it.  They
-// are compacted in index order; the exact k-th largest among them comes from a bitwise search that counts with the block barrier itself, the
-// top-p threshold from every kept element summing the mass of the strictly larger ones, the draw from one block scan: 25 us.
+// Nothing here is bound by bytes (8 MB at [128, 32000]): a row's time is the chain of block-wide steps, and a barrier of 1024 threads costs as much
+// as 100 .. 200 instructions.  A radix descent over the whole row (4 digits each for top-k and top-p) spends it on shared atomics that pile up on the
+// few bins logits fall in: 89 us at [128, 32000], top-k 50, top-p 0.9.  For top_k <= 512 the row is therefore cut down first: the k-th largest of the
+// per-thread maxima (of groups of threads where k is small) is a lower bound of the k-th largest logit, as that many elements are at least as large,
+// and only k .. 2 k elements reach it.  The threads that hold them append them in any order; one warp finds the exact k-th largest among them bit by
+// bit, over the bits in which they differ; a bitmap of the row brings the kept ones back into index order (and is the complement of the mask that is
+// returned).  Then the top-p threshold from every kept element summing the mass of the strictly larger ones, and the draw by one warp.
+// Counting with block barriers, one a bit, this took 96 of them and 27 us; with one warp in registers it takes 11.7.
 // A larger top_k, and a row with more than 1536 candidates or 1024 kept elements (ties), takes the radix descent:
 //   * top-k threshold = k-th largest key by a 4 x 8-bit descent over a shared histogram;
 //   * top-p threshold = the same descent with probability mass instead of counts (keep x iff the mass of strictly
@@ -19,12 +21,15 @@
 // rule as `logits < kth` in the PyTorch reference).
 #include "common.cuh"
 
+#include <type_traits>
+
 namespace {
 
 constexpr int kThreads = 1024;
 constexpr int kWarps = kThreads / 32;
 constexpr int kFastTopK = 512;      // the thread maxima bound the k-th logit tightly only while k is well below their number
 constexpr int kMaxCand = 1536, kMaxKept = kThreads;   // with 51200 staged logits the block's shared memory is nearly full
+constexpr int kMaxV = 51200;
 
 RB_DEVICE uint32_t f2key(float x) {  // order-preserving float -> uint
   const uint32_t u = __float_as_uint(x);
@@ -65,12 +70,15 @@ struct SampleShared {
   float f[4];
   union {
     struct { uint32_t hist[256]; float histm[256]; };                     // radix descent
-    struct { float cand[kMaxCand]; int cand_idx[kMaxCand]; };             // candidates in index order: value and index
+    uint32_t top[kThreads];                                               // the threads' largest keys
+    struct { uint32_t cand[kMaxCand]; uint16_t cand_idx[kMaxCand]; };     // candidates in any order: key and index
   };
-  float kept[kMaxKept];           // elements of the top-k set: value, index, exp(value - max)
-  int kept_idx[kMaxKept];
+  uint32_t kept[kMaxKept];        // elements of the top-k set in index order: key, index, exp(value - max)
   float kept_e[kMaxKept];
+  uint16_t kept_idx[kMaxKept];
+  uint32_t bitmap[kMaxV / 32];    // a bit an element: kept
 };
+static_assert(sizeof(SampleShared) + kMaxV * 4 <= 227 * 1024, "shared memory");
 
 // Inclusive prefix over the block of `v`, and the block's total; `red` holds one entry per warp.  Two barriers.
 template <typename V> RB_DEVICE V block_inclusive(V v, V* red, V& total) {
@@ -95,19 +103,32 @@ template <typename V> RB_DEVICE V block_inclusive(V v, V* red, V& total) {
   return (warp == 0 ? V(0) : base) + incl;
 }
 
-// The k-th largest of the block's keys, kPer of them per thread (a thread without one passes 0, which is never counted), or 0 if there are fewer than k:
-// no bound, and every element is a candidate (thread maxima: with 16-byte loads V elements have V / 4 or V / 8).  One counting barrier per bit and key.
-template <int kPer> RB_DEVICE uint32_t kth_largest(const uint32_t (&key)[kPer], int k) {
-  uint32_t prefix = 0;
+// The k-th largest of the warp's keys, kPer of them a lane (a lane without one passes 0), or 0 if there are fewer than k: no bound, and every element
+// is a candidate.  Bit by bit from the top over the bits in which the keys differ (sign and most of the exponent are common to what competes, and 16-bit
+// logits have 16 bits that are not), at most `most` of them: with fewer bits than that left undecided, a lower bound.
+template <int kPer> RB_DEVICE uint32_t kth_largest(const uint32_t (&key)[kPer], int k, int most) {
+  uint32_t any = 0, all = 0xffffffffu;
+  int have = 0;
+#pragma unroll
+  for (int i = 0; i < kPer; ++i)
+    if (key[i] != 0) { any |= key[i]; all &= key[i]; ++have; }
+  any = __reduce_or_sync(0xffffffffu, any);
+  all = __reduce_and_sync(0xffffffffu, all);
+  if ((int)__reduce_add_sync(0xffffffffu, have) < k) return 0;
+  uint32_t left = any & ~all, prefix = any & all;       // bits that differ; bits that all keys have
+  uint32_t below = 0;                                   // the bits under the last decided one
 #pragma unroll 1
-  for (int bit = 31; bit >= 0; --bit) {
-    const uint32_t c = prefix | (1u << bit);
+  for (; left != 0 && most > 0; --most) {
+    const uint32_t bit = 0x80000000u >> __clz(left);
+    below = bit - 1;
+    const uint32_t c = (prefix & ~below) | bit;
     int n = 0;
 #pragma unroll
-    for (int i = 0; i < kPer; ++i) n += __syncthreads_count(key[i] >= c);
-    if (n >= k) prefix = c;
+    for (int i = 0; i < kPer; ++i) n += key[i] >= c;
+    if ((int)__reduce_add_sync(0xffffffffu, n) >= k) prefix |= bit;
+    left ^= bit;
   }
-  return prefix;
+  return left == 0 ? prefix : prefix & ~below;
 }
 
 // Largest bin b such that the sum of the bins above it is below `want` and including it reaches it (0 if none does), and that sum above
@@ -169,22 +190,38 @@ __global__ void __launch_bounds__(kThreads, 1) sample_kernel(SampleParams p) {
     return x;
   };
   constexpr int VEC = 16 / sizeof(T);
-  if (p.row_stride % VEC == 0 && (reinterpret_cast<uintptr_t>(p.logits) & 15) == 0) {
+  const bool vec = p.row_stride % VEC == 0 && (reinterpret_cast<uintptr_t>(p.logits) & 15) == 0;
+  if (vec) {
     const int nvec = V / VEC;
-    for (int i = tid; i < nvec; i += kThreads) {
-      const rb::Pack<T, VEC> v = reinterpret_cast<const rb::Pack<T, VEC>*>(src)[i];
+    for (int i0 = tid; i0 < nvec; i0 += 4 * kThreads) {                    // four loads in flight
+      rb::Pack<T, VEC> v[4];
 #pragma unroll
-      for (int q = 0; q < VEC / 4; ++q)
-        reinterpret_cast<float4*>(srow)[i * (VEC / 4) + q] =
-            make_float4(put(i * VEC + 4 * q, rb::to_f(v.v[4 * q])), put(i * VEC + 4 * q + 1, rb::to_f(v.v[4 * q + 1])),
-                        put(i * VEC + 4 * q + 2, rb::to_f(v.v[4 * q + 2])), put(i * VEC + 4 * q + 3, rb::to_f(v.v[4 * q + 3])));
+      for (int n = 0; n < 4; ++n)
+        if (i0 + n * kThreads < nvec) v[n] = reinterpret_cast<const rb::Pack<T, VEC>*>(src)[i0 + n * kThreads];
+#pragma unroll
+      for (int n = 0; n < 4; ++n) {
+        const int i = i0 + n * kThreads;
+        if (i < nvec) {
+#pragma unroll
+          for (int q = 0; q < VEC / 4; ++q)
+            reinterpret_cast<float4*>(srow)[i * (VEC / 4) + q] =
+                make_float4(put(i * VEC + 4 * q, rb::to_f(v[n].v[4 * q])), put(i * VEC + 4 * q + 1, rb::to_f(v[n].v[4 * q + 1])),
+                            put(i * VEC + 4 * q + 2, rb::to_f(v[n].v[4 * q + 2])), put(i * VEC + 4 * q + 3, rb::to_f(v[n].v[4 * q + 3])));
+        }
+      }
     }
     for (int j = nvec * VEC + tid; j < V; j += kThreads) srow[j] = put(j, rb::to_f(src[j]));
   } else {
     for (int j = tid; j < V; j += kThreads) srow[j] = put(j, rb::to_f(src[j]));
   }
-  mx = rb::block_reduce<true>(mx, sh.red);
+  mx = rb::warp_max(mx);
+  if (lane == 0) sh.red[warp] = mx;
+  sh.top[tid] = kmax;
+  if (tid == 0) sh.u[1] = 0;
+  __syncthreads();
+  mx = rb::warp_max(sh.red[lane]);
 
+  bool have_bitmap = false;
   int64_t chosen = 0;
   float chosen_lp = 0.f;
   uint32_t keep_key = 0;  // keep elements with key >= keep_key
@@ -212,82 +249,138 @@ __global__ void __launch_bounds__(kThreads, 1) sample_kernel(SampleParams p) {
     const float u = ((r >> 8) + 0.5f) * (1.0f / 16777216.0f);
     bool done = false;
     if (p.top_k < V && p.top_k <= kFastTopK) {
-      // ---- candidates: elements that reach the k-th largest thread maximum, in index order
-      const uint32_t mine[1] = {kmax};
-      const uint32_t t0 = kth_largest(mine, p.top_k);
-      uint32_t n_w = 0;
-      for (int j = w0 + lane; j - lane < w1; j += 32) n_w += __popc(__ballot_sync(0xffffffffu, j < w1 && f2key(srow[j]) >= t0));
-      __syncthreads();
-      if (lane == 0) sh.redu[warp] = n_w;
-      __syncthreads();
-      uint32_t base = 0, n_cand = 0;
-      for (int w = 0; w < kWarps; ++w) { const uint32_t c = sh.redu[w]; base += w < warp ? c : 0u; n_cand += c; }
-      if (n_cand <= kMaxCand) {
-        for (int j = w0 + lane; j - lane < w1; j += 32) {
-          const float x = j < w1 ? srow[j] : 0.f;
-          const bool in = j < w1 && f2key(x) >= t0;
-          const unsigned b = __ballot_sync(0xffffffffu, in);
-          if (in) {
-            const uint32_t at = base + __popc(b & ((1u << lane) - 1u));
-            sh.cand[at] = x;
-            sh.cand_idx[at] = j;
+      // ---- candidates: elements that reach the k-th largest of 256, 512 or 1024 maxima (at least four times k where there are that many)
+      if (warp == 0) {
+        uint32_t m[32], t0;
+#pragma unroll
+        for (int i = 0; i < 32; ++i) m[i] = sh.top[i * 32 + lane];
+        if (p.top_k > 128) {
+          t0 = kth_largest(m, p.top_k, 14);
+        } else {
+          uint32_t m2[16];
+#pragma unroll
+          for (int i = 0; i < 16; ++i) m2[i] = max(m[i], m[i + 16]);
+          if (p.top_k > 64) {
+            t0 = kth_largest(m2, p.top_k, 14);
+          } else {
+            uint32_t m4[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) m4[i] = max(m2[i], m2[i + 8]);
+            t0 = kth_largest(m4, p.top_k, 14);
           }
-          base += __popc(b);
+        }
+        if (lane == 0) sh.u[0] = t0;
+      }
+      __syncthreads();
+      const uint32_t t0 = sh.u[0];
+      if (kmax >= t0) {                    // the same elements that this thread staged
+        auto offer = [&](int j, float x) {
+          const uint32_t key = f2key(x);
+          if (key >= t0) {
+            const uint32_t at = atomicAdd(&sh.u[1], 1u);
+            if (at < (uint32_t)kMaxCand) { sh.cand[at] = key; sh.cand_idx[at] = (uint16_t)j; }
+          }
+        };
+        if (vec) {
+          const int nvec = V / VEC;
+          for (int i = tid; i < nvec; i += kThreads)
+#pragma unroll
+            for (int q = 0; q < VEC / 4; ++q) {
+              const float4 x = reinterpret_cast<const float4*>(srow)[i * (VEC / 4) + q];
+              const int j = i * VEC + 4 * q;
+              offer(j, x.x); offer(j + 1, x.y); offer(j + 2, x.z); offer(j + 3, x.w);
+            }
+          for (int j = nvec * VEC + tid; j < V; j += kThreads) offer(j, srow[j]);
+        } else {
+          for (int j = tid; j < V; j += kThreads) offer(j, srow[j]);
+        }
+      }
+      const int words = (V + 31) / 32;
+      for (int i = tid; i < words; i += kThreads) sh.bitmap[i] = 0;
+      __syncthreads();
+      const int n_cand = (int)sh.u[1];
+      if (n_cand <= kMaxCand) {
+        // ---- the exact k-th largest
+        if (warp == 0) {
+          auto exact = [&](auto per) {
+            constexpr int kPer = decltype(per)::value;
+            uint32_t key[kPer];
+#pragma unroll
+            for (int i = 0; i < kPer; ++i) key[i] = i * 32 + lane < n_cand ? sh.cand[i * 32 + lane] : 0u;
+            return kth_largest(key, p.top_k, 32);
+          };
+          const uint32_t t = n_cand <= 128 ? exact(std::integral_constant<int, 4>()) : (n_cand <= 512 ? exact(std::integral_constant<int, 16>()) : exact(std::integral_constant<int, 48>()));
+          if (lane == 0) sh.u[0] = t;
         }
         __syncthreads();
-        // ---- the exact k-th largest (two candidates a thread, consecutive ones), then the top-k set in index order
-        const int c0 = 2 * tid;
-        uint32_t key[2];
+        keep_key = sh.u[0];
+        for (int i = tid; i < n_cand; i += kThreads)
+          if (sh.cand[i] >= keep_key) atomicOr(&sh.bitmap[sh.cand_idx[i] >> 5], 1u << (sh.cand_idx[i] & 31));
+        __syncthreads();
+        // ---- the top-k set in index order: a thread lists the elements of two words
+        uint32_t w2[2];
 #pragma unroll
-        for (int i = 0; i < 2; ++i) key[i] = c0 + i < (int)n_cand ? f2key(sh.cand[c0 + i]) : 0u;
-        keep_key = kth_largest(key, p.top_k);
+        for (int i = 0; i < 2; ++i) w2[i] = 2 * tid + i < words ? sh.bitmap[2 * tid + i] : 0u;
         uint32_t n_kept;
-        const bool in0 = c0 < (int)n_cand && key[0] >= keep_key, in1 = c0 + 1 < (int)n_cand && key[1] >= keep_key;
-        uint32_t at = block_inclusive((uint32_t)in0 + (uint32_t)in1, sh.redu, n_kept) - in0 - in1;
+        const uint32_t n_mine = __popc(w2[0]) + __popc(w2[1]);
+        uint32_t at = block_inclusive(n_mine, sh.redu, n_kept) - n_mine;
         if (n_kept <= kMaxKept) {
 #pragma unroll
           for (int i = 0; i < 2; ++i)
-            if (i == 0 ? in0 : in1) {
-              sh.kept[at] = sh.cand[c0 + i];
-              sh.kept_idx[at] = sh.cand_idx[c0 + i];
-              sh.kept_e[at] = __expf(sh.cand[c0 + i] - mx);
-              ++at;
+            for (uint32_t w = w2[i]; w != 0; w &= w - 1, ++at) {
+              const int j = (2 * tid + i) * 32 + __ffs(w) - 1;
+              sh.kept[at] = f2key(srow[j]);
+              sh.kept_idx[at] = (uint16_t)j;
+              sh.kept_e[at] = __expf(srow[j] - mx);
             }
           __syncthreads();
-          const bool have = tid < (int)n_kept;
-          const float x = have ? sh.kept[tid] : 0.f;
-          float e = have ? sh.kept_e[tid] : 0.f;
           if (p.top_p < 1.f) {
-            const float P = p.top_p * rb::block_reduce<false>(e, sh.red);
-            const uint32_t k = f2key(x);
-            float larger = 0.f;
-            if (have)
-              for (int j = 0; j < (int)n_kept; ++j) larger += f2key(sh.kept[j]) > k ? sh.kept_e[j] : 0.f;
-            const bool in = have && larger < P;
-            // the smallest kept key (a key is kept together with all larger ones)
-            uint32_t lowest = in ? k : 0xffffffffu;
-            for (int o = 16; o > 0; o >>= 1) lowest = min(lowest, __shfl_xor_sync(0xffffffffu, lowest, o));
-            __syncthreads();
+            uint32_t lowest = 0xffffffffu;     // the smallest kept key (a key is kept together with all larger ones)
+            if (warp * 32 < (int)n_kept) {
+              float total = 0.f;
+              for (int j = lane; j < (int)n_kept; j += 32) total += sh.kept_e[j];
+              const float P = p.top_p * rb::warp_sum(total);
+              const uint32_t k = tid < (int)n_kept ? sh.kept[tid] : 0xffffffffu;
+              float larger = 0.f;
+#pragma unroll 8
+              for (int j = 0; j < (int)n_kept; ++j) larger += sh.kept[j] > k ? sh.kept_e[j] : 0.f;
+              lowest = __reduce_min_sync(0xffffffffu, tid < (int)n_kept && larger < P ? k : 0xffffffffu);
+            }
             if (lane == 0) sh.redu[warp] = lowest;
             __syncthreads();
-            lowest = sh.redu[lane];
-            for (int o = 16; o > 0; o >>= 1) lowest = min(lowest, __shfl_xor_sync(0xffffffffu, lowest, o));
+            lowest = __reduce_min_sync(0xffffffffu, sh.redu[lane]);
             if (lowest != 0xffffffffu) keep_key = max(keep_key, lowest);
-            if (!(have && k >= keep_key)) e = 0.f;
+            if (tid < (int)n_kept && sh.kept[tid] < keep_key) atomicAnd(&sh.bitmap[sh.kept_idx[tid] >> 5], ~(1u << (sh.kept_idx[tid] & 31)));
           }
+          have_bitmap = done = true;
           // ---- inverse CDF over the kept elements
-          float kept;
-          const float incl = block_inclusive(e, sh.red, kept);
-          const float target = u * kept;
-          if (tid == 0) { sh.u[2] = 0xffffffffu; sh.u[3] = 0; }
-          __syncthreads();
-          if (e > 0.f && target < incl) atomicMin(&sh.u[2], (uint32_t)tid);
-          if (have && f2key(x) >= keep_key) atomicMax(&sh.u[3], (uint32_t)tid);       // rounding at the very end of the CDF: the last kept one
-          __syncthreads();
-          const uint32_t pick = sh.u[2] == 0xffffffffu ? sh.u[3] : sh.u[2];
-          chosen = sh.kept_idx[pick];
-          chosen_lp = sh.kept[pick] - mx - __logf(kept);
-          done = true;
+          if (warp == 0) {
+            auto mass = [&](int j) { return j < (int)n_kept && sh.kept[j] >= keep_key ? sh.kept_e[j] : 0.f; };
+            auto prefix = [&](float e) {
+#pragma unroll
+              for (int o = 1; o < 32; o <<= 1) {
+                const float x = __shfl_up_sync(0xffffffffu, e, o);
+                if (lane >= o) e += x;
+              }
+              return e;
+            };
+            float kept = 0.f;
+            for (int j0 = 0; j0 < (int)n_kept; j0 += 32) kept += __shfl_sync(0xffffffffu, prefix(mass(j0 + lane)), 31);
+            const float target = u * kept;
+            float before = 0.f;
+            int pick = -1, last = 0;           // `last`: rounding at the very end of the CDF
+            for (int j0 = 0; j0 < (int)n_kept && pick < 0; j0 += 32) {
+              const float e = mass(j0 + lane), incl = prefix(e);
+              const unsigned hit = __ballot_sync(0xffffffffu, e > 0.f && target < before + incl);
+              const unsigned in = __ballot_sync(0xffffffffu, j0 + lane < (int)n_kept && sh.kept[j0 + lane] >= keep_key);
+              if (hit != 0) pick = j0 + __ffs(hit) - 1;
+              if (in != 0) last = j0 + 31 - __clz(in);
+              before += __shfl_sync(0xffffffffu, incl, 31);
+            }
+            if (pick < 0) pick = last;
+            chosen = sh.kept_idx[pick];
+            chosen_lp = srow[chosen] - mx - __logf(kept);
+          }
         }
       }
     }
@@ -426,7 +519,20 @@ __global__ void __launch_bounds__(kThreads, 1) sample_kernel(SampleParams p) {
       if (p.eos_id >= 0) p.unfinished_rw[row] = live && tok != (int64_t)p.eos_id;
     }
   }
-  if (p.mask_bits != nullptr) {
+  if (p.mask_bits != nullptr && have_bitmap) {         // (complete since the barrier above)
+    uint8_t* mrow = p.mask_bits + (int64_t)row * p.mask_stride;
+    const int nbytes = (V + 7) / 8;
+    const bool words = (reinterpret_cast<uintptr_t>(mrow) & 3) == 0;
+    for (int i = tid; i * 4 < nbytes; i += kThreads) {
+      const uint32_t word = ~sh.bitmap[i] & (V - i * 32 >= 32 ? 0xffffffffu : (1u << (V - i * 32)) - 1u);
+      if (words && i * 4 + 4 <= nbytes) {
+        *reinterpret_cast<uint32_t*>(mrow + i * 4) = word;
+      } else {
+        for (int e = 0; e < 4; ++e)
+          if (i * 4 + e < nbytes) mrow[i * 4 + e] = (uint8_t)(word >> (8 * e));
+      }
+    }
+  } else if (p.mask_bits != nullptr) {
     // 32 elements a ballot, up to 1024 a warp and round (the words of a short row spread over all warps): lane i ends up with the i-th word of the round
     uint8_t* mrow = p.mask_bits + (int64_t)row * p.mask_stride;
     const int nbytes = (V + 7) / 8, per_warp = min(32, ((V + 31) / 32 + kWarps - 1) / kWarps);
