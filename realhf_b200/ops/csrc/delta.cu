@@ -230,6 +230,86 @@ __global__ void __launch_bounds__(kPThreads) delta_prepare_tiled_kernel(const vo
   }
 }
 
+// The same for head sizes in whole fours up to 128 on aligned rows: a warp owns one unit of channels, four neighbouring ones a lane, and walks kWalk
+// tokens in tiles of 8 whose rows it has in flight together; the per-(token, head) sum of squares stays inside the warp.  The kernel above moves two
+// bytes a lane and load and four a store, and waits for its loads with few of them on their way: 8 sequences of 700 .. 1024 tokens, 16 + 2 x 4 heads x 128
+// (71 MB in, 85 MB out) 121 us; this way 87 (exact exponentials and divisions).  kTaps: the taps that registers are kept for.
+constexpr int kTile = 8;
+
+template <int kTaps, int kWalk>
+__global__ void __launch_bounds__(kPThreads) delta_prepare_warp_kernel(const void* __restrict__ proj, int64_t ld, int dt, const void* __restrict__ conv_w,
+                                                                       GateParams gp, float* __restrict__ u, const int* __restrict__ pos,
+                                                                       float* __restrict__ conv_state, const int* __restrict__ tok_slot,
+                                                                       const int* __restrict__ remain, int64_t T, int H, int G, int d, int dv,
+                                                                       int taps, float unit_eps) {
+  const int nqk = G * d, nv = H * dv, C = 2 * nqk + nv, UW = C + H + gp.N;
+  const int unit = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  constexpr int kPerCta = kPThreads / 32 * kWalk;
+  const int64_t b0 = (int64_t)blockIdx.y * kPerCta;
+  if (unit >= 2 * G + H) {
+    gate_unit(gp, u, dt, unit - 2 * G - H, b0, (int)min((int64_t)kPerCta, T - b0), H, C, UW);
+    return;
+  }
+  const int64_t t0 = b0 + warp * kWalk;
+  const int nt = (int)min((int64_t)kWalk, T - t0);
+  if (nt <= 0) return;
+  const bool is_qk = unit < 2 * G, mine = lane * 4 < (is_qk ? d : dv);
+  const int c = (is_qk ? unit * d : 2 * nqk + (unit - 2 * G) * dv) + lane * 4;
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  float4 w[kTaps], hist[kTaps - 1], x[kTile];             // w[back]: the taps that meet the input `back` tokens ago; hist[back - 1]: that input
+#pragma unroll
+  for (int i = 0; i < kTile; ++i) x[i] = mine && i < nt ? rb::ld4_any(proj, dt, (t0 + i) * ld + c) : zero;
+#pragma unroll
+  for (int back = 1; back < kTaps; ++back) hist[back - 1] = mine && back < taps && t0 - back >= 0 ? rb::ld4_any(proj, dt, (t0 - back) * ld + c) : zero;
+#pragma unroll
+  for (int back = 0; back < kTaps; ++back) {
+    const bool in = mine && back < taps;
+    const int64_t at = (int64_t)c * taps + taps - 1 - back;
+    w[back] = in ? make_float4(ld_any(conv_w, dt, at), ld_any(conv_w, dt, at + taps), ld_any(conv_w, dt, at + 2 * taps), ld_any(conv_w, dt, at + 3 * taps)) : zero;
+  }
+  const float scale = unit < G ? 1.f / sqrtf((float)d) : 1.f;
+  for (int s0 = 0; s0 < nt; s0 += kTile) {
+    const int p0 = lane < kTile && s0 + lane < nt ? pos[t0 + s0 + lane] : 0;
+    float4 nx[kTile];                                     // the next tile's rows
+#pragma unroll
+    for (int i = 0; i < kTile; ++i) nx[i] = mine && s0 + kTile + i < nt ? rb::ld4_any(proj, dt, (t0 + s0 + kTile + i) * ld + c) : zero;
+    if (conv_state != nullptr && taps > 1) {
+#pragma unroll
+      for (int i = 0; i < kTile; ++i)
+        if (s0 + i < nt) {
+          const int slot = tok_slot[t0 + s0 + i], rem = remain[t0 + s0 + i];
+          if (slot >= 0 && rem < taps - 1 && mine) {
+            float* st = conv_state + ((int64_t)slot * (taps - 1) + (taps - 2 - rem)) * C + c;
+            st[0] = x[i].x; st[1] = x[i].y; st[2] = x[i].z; st[3] = x[i].w;
+          }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < kTile; ++i) {
+      const int p = __shfl_sync(0xffffffffu, p0, i);
+      float4 y = zero;
+      auto tap = [&](const float4& a, const float4& b) {
+        y.x = fmaf(a.x, b.x, y.x); y.y = fmaf(a.y, b.y, y.y); y.z = fmaf(a.z, b.z, y.z); y.w = fmaf(a.w, b.w, y.w);
+      };
+#pragma unroll
+      for (int back = kTaps - 1; back >= 1; --back)       // oldest first, the current token last: a fixed order
+        if (back < taps && back <= p) tap(hist[back - 1], w[back]);
+      tap(x[i], w[0]);
+#pragma unroll
+      for (int back = kTaps - 1; back >= 2; --back) hist[back - 1] = hist[back - 2];
+      if constexpr (kTaps > 1) hist[0] = x[i];
+      y.x = y.x / (1.f + expf(-y.x)); y.y = y.y / (1.f + expf(-y.y)); y.z = y.z / (1.f + expf(-y.z)); y.w = y.w / (1.f + expf(-y.w));
+      if (is_qk) {
+        const float r = scale * (1.f / sqrtf(rb::warp_sum((y.x * y.x + y.y * y.y) + (y.z * y.z + y.w * y.w)) + unit_eps));
+        y.x *= r; y.y *= r; y.z *= r; y.w *= r;
+      }
+      if (mine && s0 + i < nt) *reinterpret_cast<float4*>(u + (t0 + s0 + i) * UW + c) = y;
+    }
+#pragma unroll
+    for (int i = 0; i < kTile; ++i) x[i] = nx[i];
+  }
+}
+
 // ------------------------------------------------------------------------------------------------ recurrence
 constexpr int kScanThreads = 128, kTok = 8;
 
@@ -662,6 +742,20 @@ extern "C" int rb_delta_prepare(const void* proj, int64_t ld, int dt, const void
   const GateParams gp{blog, ldb, alog, lda, A_log, dt_bias, N};
   const int units = 2 * G + H + 1 + (N == H ? 0 : H);
   if (pos != nullptr && T >= 64 && d <= 2 * kPThreads && dv <= 2 * kPThreads) {
+    // four channels a lane: whole fours of channels, rows of proj and u on their boundaries
+    if (d <= 128 && dv <= 128 && d % 4 == 0 && dv % 4 == 0 && ld % 4 == 0 && (H + N) % 4 == 0 && T <= 65535ll * kPThreads &&
+        ((reinterpret_cast<uintptr_t>(proj) | reinterpret_cast<uintptr_t>(u)) & 15) == 0) {
+      // 32 tokens a warp share their taps and a halo of taps - 1 rows; with fewer than 16 such warps an SM, one tile a warp (1 sequence of 900 tokens, with the
+      // recurrence and the norm, 351 us against 360; 8 of 20 .. 40 tokens 37 against 52)
+      const int walk = T * units >= (int64_t)rb::kNumSMs * 16 * 32 ? 32 : kTile, per_cta = kPThreads / 32 * walk;
+      const dim3 grid(units, (unsigned)((T + per_cta - 1) / per_cta));
+      auto go = [&](auto kern) { kern<<<grid, kPThreads, 0, s>>>(proj, ld, dt, conv_w, gp, u, pos, conv_state, tok_slot, remain, T, H, G, d, dv, taps, unit_eps); };
+      if (walk == 32 && taps <= 4) go(delta_prepare_warp_kernel<4, 32>);
+      else if (walk == 32) go(delta_prepare_warp_kernel<kMaxTaps, 32>);
+      else if (taps <= 4) go(delta_prepare_warp_kernel<4, kTile>);
+      else go(delta_prepare_warp_kernel<kMaxTaps, kTile>);
+      return 0;
+    }
     dim3 grid((unsigned)((T + kPT - 1) / kPT), units);
     if (d <= kPThreads && dv <= kPThreads)
       delta_prepare_tiled_kernel<1><<<grid, kPThreads, 0, s>>>(proj, ld, dt, conv_w, gp, u, pos, conv_state, tok_slot, remain, T, H, G, d, dv, taps,
