@@ -791,6 +791,8 @@ static int launch_delta_column(const ScanParams& p, int n_seqs, cudaStream_t s) 
   return rb::launch_pdl(kern, dim3(n_seqs, p.H, RB_CEIL_DIV(p.dv, ncol)), dim3(kScanThreads), smem, s, p) == cudaSuccess ? 0 : -3;
 }
 
+extern "C" int rb_delta_chunk(const float* u, float* o, const int* cu, float* s_state, const int* slots, int n_seqs, int H, int G, cudaStream_t s);
+
 // channel: u rows hold a decay per state row (H * d numbers) instead of one per head
 extern "C" int rb_delta_rule(const float* u, float* o, const int* cu, float* s_state, const int* slots, int n_seqs, int H, int G, int d, int dv,
                              int step, int channel, cudaStream_t s) {
@@ -798,6 +800,8 @@ extern "C" int rb_delta_rule(const float* u, float* o, const int* cu, float* s_s
   if (d > 512 || H % G) return -1;
   ScanParams p{u, o, cu, s_state, slots, H, G, d, dv, step, dv % 4 == 0 && ((uintptr_t)s_state & 15) == 0};
   const bool many = (int64_t)n_seqs * H * RB_CEIL_DIV(dv, 64) >= rb::kNumSMs;
+  if (!step && !channel && d == 128 && dv == 128 && H % 2 == 0 && (reinterpret_cast<uintptr_t>(u) & 15) == 0)
+    return rb_delta_chunk(u, o, cu, s_state, slots, n_seqs, H, G, s);
   if (step || (d <= 64 && !(d <= 32 && many))) {       // (lanes per column, state rows per lane)
 #define RB_L(LPC, EPL) return channel ? launch_delta_column<LPC, EPL, true>(p, n_seqs, s) : launch_delta_column<LPC, EPL, false>(p, n_seqs, s)
     if (d <= 32) { RB_L(1, 32); }

@@ -64,3 +64,19 @@ def test_delta_rule_on_both_sides_of_the_sequence_count(d, dv, n_seqs):
     want, plain, got = run(u.double(), R.delta_rule_scan_ref), run(u, R.delta_rule_scan_ref), run(u.cuda(), R.delta_rule_scan)
     for w, f, x in zip(want, plain, got):      # the bound of the test above
         assert float((x - w).abs().max()) <= 4 * float((f - w).abs().max()) + 8 * 2.0 ** -23 * float(w.abs().max())
+
+
+@pytest.mark.parametrize("lens", [[63], [64, 1], [65, 0, 128], [200, 129, 333]])
+@pytest.mark.parametrize("decays", ["one", "mixed", "zeros"])
+@pytest.mark.parametrize("d,dv", [(128, 128), (128, 124)])
+def test_delta_rule_chunks(lens, decays, d, dv):
+    """Head size 128 x 128 runs in chunks of 64 tokens (128 x 124 does not): sequences that end at and around their edges, in one call."""
+    cfg, u = inputs(d, dv, decays, False, sum(lens), len(lens))
+    cu, slots = torch.tensor([0] + lens).cumsum(0).int(), torch.arange(len(lens), dtype=torch.int32)
+
+    def run(u, scan):
+        S = torch.zeros(len(lens), 4, d, dv, dtype=u.dtype, device=u.device)
+        return scan(u, cfg, cu.to(u.device), S, slots.to(u.device)).double().cpu(), S.double().cpu()
+    want, plain, got = run(u.double(), R.delta_rule_scan_ref), run(u, R.delta_rule_scan_ref), run(u.cuda(), R.delta_rule_scan)
+    for w, f, x in zip(want, plain, got):      # the bound of the first test
+        assert float((x - w).abs().max()) <= 4 * float((f - w).abs().max()) + 8 * 2.0 ** -23 * float(w.abs().max())
