@@ -10,12 +10,13 @@
 // 2^-16 of the largest, smallest first, in an fp32 accumulator that starts at zero (the update of S too: adding to S inside the tensor core would cut S off
 // a little 24 times a chunk).  Decays, the inverse and all sums of products are fp32 on CUDA cores.
 //
-// One CTA per (sequence, head).  Warps 0 .. 3, thread = row of S^T (lane of tensor memory): S and its parts, r, parts of U, o.  Warps 4 .. 7: q and k to parts
-// in shared memory, decays, A and its inverse (blocks of 16, then two of 16 and two of 32 at a time), W.  Warp 8 issues.  Loops are rolled: with the
-// chunk's code unrolled a quarter of all stalls were instruction misses.
+// One CTA per (sequence, head).  Warps 0 .. 3, thread = row of S^T (lane of tensor memory): S and its parts, r, parts of U, o.  Warps 4 .. 7: A and its inverse
+// (blocks of 16, then two of 16 and two of 32 at a time), W.  Warps 8 .. 11: q and k to parts in shared memory, decays.  Warp 12 issues; [K; Q] K^T of the next
+// chunk goes ahead of the update of S, so that the inverse is formed while the chain goes on.  Loops are rolled: with the chunk's code unrolled a
+// quarter of all stalls were instruction misses.
 //
-// What bounds it: the chain parts of S -> X, Y -> r -> U -> parts of U -> S of a head, products (about 5400 cycles) and element work in turn, which nothing
-// else on the SM overlaps.  8 sequences of 700..1024 tokens, 16 heads x 128 x 128: 518 us a token at a time on CUDA cores (shared-memory port and
+// What bounds it: the chain parts of S -> X, Y -> r -> U -> parts of U -> S of a head, products and element work in turn, which nothing else on the SM
+// overlaps.  8 sequences of 700..1024 tokens, 16 heads x 128 x 128: 518 us a token at a time on CUDA cores (shared-memory port and
 // latency), 249 this way.
 #include "attn_common.cuh"
 
@@ -24,7 +25,8 @@
 namespace {
 
 constexpr int kL = 64, kD = 128;                   // tokens of a chunk; rows and columns of S
-constexpr int kChunkThreads = 288;
+// four warpgroups; the registers of the launch (128 a thread) moved to where they are needed: 192 + 104 + 144 + 72 = 4 x 128
+constexpr int kChunkThreads = 512, kRegsA = 192, kRegsB = 104, kRegsE = 144, kRegsC = 72;
 
 struct ChunkParams {
   const float* u; float* o;                        // rows of u: q (G x 128) | k (G x 128) | v (H x 128) | beta (H) | g (H)
@@ -104,7 +106,7 @@ __global__ void __launch_bounds__(kChunkThreads, 1) delta_chunk_kernel(const Chu
     for (int i = 0; i < C_NUM_BARS; ++i) ptx::mbar_init(bar(i), i <= O_READ ? 4 : 1);          // (the first ones: an arrival a warp)
     ptx::fence_barrier_init();
   }
-  if (warp == 8) {
+  if (warp == 12) {
     ptx::tmem_alloc(ptx::smem_u32(tmem_ptr), 512);
     ptx::tmem_relinquish();
   }
@@ -121,6 +123,7 @@ __global__ void __launch_bounds__(kChunkThreads, 1) delta_chunk_kernel(const Chu
   };
 
   if (warp < 4) {
+    ptx::reg_inc<kRegsA>();
     // ===================================================== S, r, U, o: thread = row v of S^T
     const uint32_t tm = tmem_base + ((uint32_t)(warp * 32) << 16);
     const int v = warp * 32 + lane;
@@ -145,12 +148,6 @@ __global__ void __launch_bounds__(kChunkThreads, 1) delta_chunk_kernel(const Chu
     float c_last = 1.f;
     for (int c = 0; c < n_chunks; ++c) {
       const float* coef = sCoef + (c & 1) * 4 * kL;
-      float vn[16];                                // v of the next 16 tokens
-      auto load_v = [&](int b) {
-#pragma unroll
-        for (int i = 0; i < 16; ++i) vn[i] = c * kL + b * 16 + i < len ? vp[(int64_t)(c * kL + b * 16 + i) * UW] : 0.f;
-      };
-      load_v(0);
       if (c > 0) { wait(D_DONE, c - 1); ptx::tc_fence_after(); }
 #pragma unroll 1
       for (int b = 7; b >= 0; --b) {
@@ -177,18 +174,20 @@ __global__ void __launch_bounds__(kChunkThreads, 1) delta_chunk_kernel(const Chu
       ptx::tc_fence_before();
       arrive(SP_FULL);
       if (c > 0) write_o(c - 1);
+      float vv[kL];
+#pragma unroll
+      for (int i = 0; i < kL; ++i) vv[i] = c * kL + i < len ? vp[(int64_t)(c * kL + i) * UW] : 0.f;
       wait(COEF_FULL, c);
       c_last = coef[2 * kL + kL - 1];
       wait(X_DONE, c);
       ptx::tc_fence_after();
-#pragma unroll 1
+#pragma unroll
       for (int b = 0; b < 4; ++b) {
         float x[16], r[16];
         ld16(tm + kTX + b * 16, x);
         ptx::tc_wait_ld();
 #pragma unroll
-        for (int i = 0; i < 16; ++i) r[i] = coef[b * 16 + i] * fmaf(-coef[2 * kL + b * 16 + i], x[i], vn[i]);
-        if (b < 3) load_v(b + 1);
+        for (int i = 0; i < 16; ++i) r[i] = coef[b * 16 + i] * fmaf(-coef[2 * kL + b * 16 + i], x[i], vv[b * 16 + i]);
         if (b == 0) { wait(Y_DONE, c); ptx::tc_fence_after(); }                    // the parts of S have been read
         store_parts(tm + kTR + b * 8, 32, r);
       }
@@ -235,70 +234,11 @@ __global__ void __launch_bounds__(kChunkThreads, 1) delta_chunk_kernel(const Chu
       }
     }
   } else if (warp < 8) {
-    // ===================================================== operands from the inputs
-    const int w = warp - 4, tid = threadIdx.x - 128, g = h / (H / G);
+    ptx::reg_dec<kRegsB>();
+    // ===================================================== A, its inverse, W
+    const int w = warp - 4, tid = threadIdx.x - 128;
     const uint32_t tm = tmem_base + ((uint32_t)(w * 32) << 16);
     auto sync = [] { asm volatile("bar.sync 1, 128;" ::: "memory"); };
-    // Rows of the chunk's 64 tokens to parts, 16 a warp in fours, four columns a lane; the next four are on their way.  `row0`: first row of the operand,
-    // `scale` (null: none): a factor a token.
-    auto rows = [&](int c, int col, uint32_t dst, int part_bytes, int row0, const float* scale) {
-      float4 nx[4];
-      auto load = [&](int n) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int tok = c * kL + w * 16 + n * 4 + i;
-          nx[i] = tok < len ? *reinterpret_cast<const float4*>(p.u + (int64_t)(t0 + tok) * UW + col + g * kD + lane * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-      };
-      load(0);
-      const uint32_t to = dst + (lane >> 4) * (part_bytes / 2) + (lane & 1) * 8;
-#pragma unroll 1
-      for (int n = 0; n < 4; ++n) {
-        float4 x[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) x[i] = nx[i];
-        if (n < 3) load(n + 1);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int tok = w * 16 + n * 4 + i, row = row0 + tok;
-          if (scale != nullptr) { const float f = scale[tok]; x[i].x *= f; x[i].y *= f; x[i].z *= f; x[i].w *= f; }
-          uint32_t part[3][2];
-          split3(x[i].x, x[i].y, part[0][0], part[1][0], part[2][0]);
-          split3(x[i].z, x[i].w, part[0][1], part[1][1], part[2][1]);
-          const uint32_t at = to + row * 128 + ((((lane & 15) >> 1) ^ (row & 7)) << 4);
-#pragma unroll
-          for (int f = 0; f < 3; ++f) asm volatile("st.shared.v2.b32 [%0], {%1,%2};" ::"r"(at + f * part_bytes), "r"(part[f][0]), "r"(part[f][1]) : "memory");
-        }
-      }
-      ptx::fence_proxy_async();
-    };
-    // beta, g, C, D_last of chunk c into its buffer: one warp, two tokens a lane
-    auto coefficients = [&](int c) {
-      if (w != 0) return;
-      float* coef = sCoef + (c & 1) * 4 * kL;
-      float beta[2], dec[2];
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const int tok = c * kL + 2 * lane + e;
-        const float* row = p.u + (int64_t)(t0 + tok) * UW + C + h;
-        beta[e] = tok < len ? row[0] : 0.f;
-        dec[e] = tok < len ? row[H] : 1.f;
-      }
-      float up = dec[0] * dec[1], down = up;       // products over the lanes up to this one, from this one on
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const float a = __shfl_up_sync(0xffffffffu, up, o), b = __shfl_down_sync(0xffffffffu, down, o);
-        if (lane >= o) up *= a;
-        if (lane + o < 32) down *= b;
-      }
-      const float prev = __shfl_up_sync(0xffffffffu, up, 1), next = __shfl_down_sync(0xffffffffu, down, 1);
-      const float in = lane == 0 ? 1.f : prev, out = lane == 31 ? 1.f : next;
-      *reinterpret_cast<float2*>(coef + 2 * lane) = make_float2(beta[0], beta[1]);
-      *reinterpret_cast<float2*>(coef + kL + 2 * lane) = make_float2(dec[0], dec[1]);
-      *reinterpret_cast<float2*>(coef + 2 * kL + 2 * lane) = make_float2(in * dec[0], up);
-      *reinterpret_cast<float2*>(coef + 3 * kL + 2 * lane) = make_float2(dec[1] * out, out);
-      arrive(COEF_FULL);
-    };
     // A's block (N rows and columns at `at`, unit lower triangular blocks of N / 2 inverted already on its diagonal): the block below the diagonal becomes
     // -T22 A21 T11.  128 threads, kCols neighbouring outputs each.
     auto join = [&](auto size, int first_of) {
@@ -330,16 +270,10 @@ __global__ void __launch_bounds__(kChunkThreads, 1) delta_chunk_kernel(const Chu
         sync();
       }
     };
-    if (n_chunks > 0) {
-      coefficients(0);
-      rows(0, nqk, sKQ, kPartBytes, 0, nullptr);
-      rows(0, 0, sKQ, kPartBytes, kL, nullptr);
-      arrive(KQ_FULL);
-    }
     for (int c = 0; c < n_chunks; ++c) {
       const float* coef = sCoef + (c & 1) * 4 * kL;
       wait(COEF_FULL, c);
-      wait(P_DONE, c);                             // (and with it everything that was issued for the chunk in front: its W, T and scaled k have been read)
+      wait(P_DONE, c);                             // (T of the chunk in front has been read, too)
       ptx::tc_fence_after();
       // row i of [K; Q] K^T, from the back: lanes 0 .. 63 k_i -> A, 64 .. 127 q_i -> W
       const int i = (w & 1) * 32 + lane;
@@ -357,6 +291,7 @@ __global__ void __launch_bounds__(kChunkThreads, 1) delta_chunk_kernel(const Chu
           x[e] = j <= i ? dec * x[e] : 0.f;
           if (w < 2) x[e] = j < i ? beta * x[e] : 0.f;
         }
+        if (b == 3 && c > 0 && w >= 2) wait(O_DONE, c - 1);    // W of the chunk in front has been read
         if (w < 2) {
 #pragma unroll
           for (int e = 0; e < 16; e += 4) *reinterpret_cast<float4*>(sA + i * kLdA + b * 16 + e) = make_float4(x[e], x[e + 1], x[e + 2], x[e + 3]);
@@ -412,17 +347,103 @@ __global__ void __launch_bounds__(kChunkThreads, 1) delta_chunk_kernel(const Chu
       }
       ptx::fence_proxy_async();
       arrive(T_FULL);
-      rows(c, nqk, sKQ + kSK2, kK2Bytes, 0, coef + 3 * kL);
+    }
+  } else if (warp < 12) {
+    ptx::reg_inc<kRegsE>();
+    // ===================================================== operands from the inputs
+    const int w = warp - 8, g = h / (H / G);
+    // Rows of 64 tokens, 16 a warp, four columns a lane: N of them on their way at once, then fours of them to parts.  `row0`: first row of the operand,
+    // `scale` (null: none): a factor a token.  (The fours move up in the registers, so that the loop's code is that of four rows.)
+    auto load = [&](auto& x, int c, int col, int first) {
+#pragma unroll
+      for (int i = 0; i < (int)(sizeof(x) / sizeof(float4)); ++i) {
+        const int tok = c * kL + w * 16 + first + i;
+        x[i] = tok < len ? *reinterpret_cast<const float4*>(p.u + (int64_t)(t0 + tok) * UW + col + g * kD + lane * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+    };
+    auto rows = [&](auto& x, uint32_t dst, int part_bytes, int row0, int first, const float* scale) {
+      constexpr int N = sizeof(x) / sizeof(float4);
+      const uint32_t to = dst + (lane >> 4) * (part_bytes / 2) + (lane & 1) * 8;
+#pragma unroll 1
+      for (int n = 0; n < N; n += 4) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int tok = w * 16 + first + n + i, row = row0 + tok;
+          const float f = scale != nullptr ? scale[tok] : 1.f;
+          uint32_t part[3][2];
+          split3(x[i].x * f, x[i].y * f, part[0][0], part[1][0], part[2][0]);
+          split3(x[i].z * f, x[i].w * f, part[0][1], part[1][1], part[2][1]);
+          const uint32_t at = to + row * 128 + ((((lane & 15) >> 1) ^ (row & 7)) << 4);
+#pragma unroll
+          for (int q = 0; q < 3; ++q) asm volatile("st.shared.v2.b32 [%0], {%1,%2};" ::"r"(at + q * part_bytes), "r"(part[q][0]), "r"(part[q][1]) : "memory");
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {              // around, so that x is whole again at the end
+          const float4 front = x[i];
+#pragma unroll
+          for (int m = i; m + 4 < N; m += 4) x[m] = x[m + 4];
+          x[N - 4 + i] = front;
+        }
+      }
+    };
+    // beta, g, C, D_last of chunk c into its buffer: one warp, two tokens a lane
+    float beta[2], dec[2];
+    auto load_coefficients = [&](int c) {
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int tok = c * kL + 2 * lane + e;
+        const float* row = p.u + (int64_t)(t0 + tok) * UW + C + h;
+        beta[e] = tok < len ? row[0] : 0.f;
+        dec[e] = tok < len ? row[H] : 1.f;
+      }
+    };
+    auto coefficients = [&](int c) {
+      if (w != 0) return;
+      float* coef = sCoef + (c & 1) * 4 * kL;
+      float up = dec[0] * dec[1], down = up;       // products over the lanes up to this one, from this one on
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const float a = __shfl_up_sync(0xffffffffu, up, o), b = __shfl_down_sync(0xffffffffu, down, o);
+        if (lane >= o) up *= a;
+        if (lane + o < 32) down *= b;
+      }
+      const float prev = __shfl_up_sync(0xffffffffu, up, 1), next = __shfl_down_sync(0xffffffffu, down, 1);
+      const float in = lane == 0 ? 1.f : prev, out = lane == 31 ? 1.f : next;
+      *reinterpret_cast<float2*>(coef + 2 * lane) = make_float2(beta[0], beta[1]);
+      *reinterpret_cast<float2*>(coef + kL + 2 * lane) = make_float2(dec[0], dec[1]);
+      *reinterpret_cast<float2*>(coef + 2 * kL + 2 * lane) = make_float2(in * dec[0], up);
+      *reinterpret_cast<float2*>(coef + 3 * kL + 2 * lane) = make_float2(dec[1] * out, out);
+      arrive(COEF_FULL);
+    };
+    float4 kx[16], qx[8];
+    if (n_chunks > 0) {
+      load_coefficients(0);
+      load(kx, 0, nqk, 0);
+      load(qx, 0, 0, 0);
+    }
+    for (int c = 0; c < n_chunks; ++c) {
+      if (c > 0) wait(Y_DONE, c - 1);              // k and q of the chunk in front have been read
+      rows(qx, sKQ, kPartBytes, kL, 0, nullptr);
+      load(qx, c, 0, 8);
+      rows(kx, sKQ, kPartBytes, 0, 0, nullptr);
+      rows(qx, sKQ, kPartBytes, kL, 8, nullptr);
+      ptx::fence_proxy_async();
+      arrive(KQ_FULL);
+      if (c > 0) wait(UA_DONE, c - 1);             // everybody has seen the coefficients of the chunk in front, and nobody needs those before them
+      coefficients(c);
+      wait(COEF_FULL, c);
+      if (c > 0) wait(D_DONE, c - 1);              // the scaled k of the chunk in front has been read
+      rows(kx, sKQ + kSK2, kK2Bytes, 0, 0, sCoef + (c & 1) * 4 * kL + 3 * kL);
+      ptx::fence_proxy_async();
       arrive(K2_FULL);
       if (c + 1 < n_chunks) {
-        coefficients(c + 1);
-        wait(Y_DONE, c);                           // k and q of this chunk have been read
-        rows(c + 1, nqk, sKQ, kPartBytes, 0, nullptr);
-        rows(c + 1, 0, sKQ, kPartBytes, kL, nullptr);
-        arrive(KQ_FULL);
+        load_coefficients(c + 1);
+        load(kx, c + 1, nqk, 0);
+        load(qx, c + 1, 0, 0);
       }
     }
   } else {
+    ptx::reg_dec<kRegsC>();
     // ===================================================== MMA issue: the whole warp runs the loop, one elected lane issues
     constexpr uint32_t idesc64 = ptx::make_idesc_f16(1, 128, kL, 0, 0), idesc_s = ptx::make_idesc_f16(1, 128, kD, 0, 1);
     const uint32_t tm = (uint32_t)ptx::uniform((int)tmem_base);
@@ -447,7 +468,7 @@ __global__ void __launch_bounds__(kChunkThreads, 1) delta_chunk_kernel(const Chu
           ptx::tc_mma_f16_ts(tm + d, tm + kTParts + part_a(n) * 64 + k * 8,
                              kq + ((part_b(n) * kPartBytes + (k >> 2) * (kPartBytes / 2) + (k & 3) * 32 + row0 * 128) >> 4), idesc64, n != 0 || k != 0);
     };
-    for (int c = 0; c < n_chunks; ++c) {
+    auto products_of = [&](int c) {                // [K; Q] K^T
       wait(KQ_FULL, c);
       ptx::tc_fence_after();
       if (ptx::elect_one()) {
@@ -461,6 +482,9 @@ __global__ void __launch_bounds__(kChunkThreads, 1) delta_chunk_kernel(const Chu
         ptx::tc_commit(bar(P_DONE));
       }
       __syncwarp();
+    };
+    for (int c = 0; warp == 12 && c < n_chunks; ++c) {
+      if (c == 0) products_of(0);
       wait(SP_FULL, c);
       ptx::tc_fence_after();
       if (ptx::elect_one()) {
@@ -482,6 +506,7 @@ __global__ void __launch_bounds__(kChunkThreads, 1) delta_chunk_kernel(const Chu
         ptx::tc_commit(bar(UA_DONE));
       }
       __syncwarp();
+      if (c + 1 < n_chunks) products_of(c + 1);
       wait(U_FULL, c);
       wait(K2_FULL, c);
       ptx::tc_fence_after();
@@ -501,7 +526,7 @@ __global__ void __launch_bounds__(kChunkThreads, 1) delta_chunk_kernel(const Chu
   ptx::tc_fence_before();
   __syncthreads();
   rb::report_given_up(dead, p.status);
-  if (warp == 8) {
+  if (warp == 12) {
     ptx::tc_fence_after();
     ptx::tmem_dealloc(tmem_base, 512);
   }
