@@ -367,7 +367,12 @@ class _LMHeadLogProb(torch.autograd.Function):
         dw = None
         if ctx.needs_input_grad[1]:
             mg = getattr(weight, "main_grad", None)
-            if mg is not None and mg.dtype == torch.float32 and _native_gemm(hidden, weight) is not None:
+            if (mg is None and T <= ctx.chunk and getattr(weight, "_grad_in_flat_buffer", False) and weight.grad is not None
+                    and weight.grad.dtype == weight.dtype and _native_gemm(hidden, weight) is not None and T % 8 == 0):
+                # one chunk and a gradient buffer of the weight's own type: the product's fp32 sums are added to it and rounded once, as for every
+                # other projection (ops.gemm._linear_backward); an fp32 copy of dW, its cast and its sum were four passes over [V, H]
+                dw = weight.grad
+            elif mg is not None and mg.dtype == torch.float32 and _native_gemm(hidden, weight) is not None:
                 dw = mg  # same contract as ops.gemm._Linear: wgrad accumulates into the fp32 main-grad view
             else:
                 dw = torch.zeros(weight.shape, dtype=torch.float32, device=weight.device)
@@ -398,7 +403,7 @@ class _LMHeadLogProb(torch.autograd.Function):
                     G.gemm(dlogits, hidden[s:e], out=dw, a_mn=True, b_mn=True, accumulate=True)  # [t,V]^T x [t,H] += into fp32
                 else:
                     dw += (dlogits.t() @ hidden[s:e]).float()
-        if dw is not None and dw is getattr(weight, "main_grad", None):
+        if dw is not None and (dw is getattr(weight, "main_grad", None) or dw is weight.grad):
             dw = None  # accumulated straight into the flat gradient bucket
         return dh, (dw.to(weight.dtype) if dw is not None else None), None, None, None, None
 
