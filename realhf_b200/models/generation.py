@@ -76,11 +76,9 @@ def genstep(logits: torch.Tensor, g: GenerationHyperparameters, step: int, eos_i
         need_mask = want_mask and not g.force_no_logits_mask and not g.greedy
         seed = int(_SAMPLE_SEED[0])
         _SAMPLE_SEED[0] = (seed * 6364136223846793005 + 1442695040888963407) % (1 << 62)
-        nxt, lp, mb = lib().sample(logits, unfinished, g.top_k, g.top_p, 1.0 / g.temperature, eos_id if eos_id is not None else -1,
-                                   eos_id is not None and step < g.min_new_tokens, g.greedy, pad_id, seed, step, need_mask)
-        if eos_id is not None:
-            unfinished = unfinished & (nxt != eos_id)
-        return nxt, lp, (mb if need_mask else None), unfinished
+        nxt, lp, mb, goes_on = lib().sample_next(logits, unfinished, g.top_k, g.top_p, 1.0 / g.temperature, eos_id if eos_id is not None else -1,
+                                                 eos_id is not None and step < g.min_new_tokens, g.greedy, pad_id, seed, step, need_mask)
+        return nxt, lp, (mb if need_mask else None), (goes_on if eos_id is not None else unfinished)
     x = logits.float()
     if eos_id is not None and step < g.min_new_tokens:
         x[:, eos_id] = torch.finfo(x.dtype).min

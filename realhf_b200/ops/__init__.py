@@ -65,7 +65,7 @@ class _CountingLib:
     def __getattr__(self, name):
         fn = self._cache.get(name)
         if fn is None:
-            op = getattr(self._ns, name)
+            op = getattr(self._ns, name).default      # (the overload itself: no search among overloads a call)
             k = _KERNELS_PER_OP.get(name, 1)
 
             def fn(*a, _op=op, _k=k, _name=name, **kw):

@@ -86,54 +86,57 @@ class _PackedQKVAttention(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, qkv, cu, max_seqlen, nq, nkv, hd, scale, causal, dropout_p):
-        from flash_attn.flash_attn_interface import _wrapped_flash_attn_varlen_forward
-        T = qkv.shape[0]
-        q = qkv[:, : nq * hd].view(T, nq, hd)
-        k = qkv[:, nq * hd:(nq + nkv) * hd].view(T, nkv, hd)
-        v = qkv[:, (nq + nkv) * hd:].view(T, nkv, hd)
+        ctx.meta = (max_seqlen, nq, nkv, hd, scale, causal, dropout_p)
         if _own_fwd_ok(hd, dropout_p):
-            out, lse = lib().attn_fwd(q, k, v, cu, max_seqlen, scale, causal)
-            ctx.save_for_backward(qkv, out, lse, cu, torch.empty(2, dtype=torch.int64, device=qkv.device))
-            ctx.meta = (max_seqlen, nq, nkv, hd, scale, causal, dropout_p)
+            out, lse = lib().attn_fwd_qkv(qkv, cu, max_seqlen, nq, nkv, hd, scale, causal)
+            ctx.save_for_backward(qkv, out, lse, cu)
             return out
+        from flash_attn.flash_attn_interface import _wrapped_flash_attn_varlen_forward
+        q, k, v = _qkv_views(qkv, nq, nkv, hd)
         out, lse, _, rng = _wrapped_flash_attn_varlen_forward(q, k, v, cu, cu, max_seqlen, max_seqlen, dropout_p, scale, causal=causal,
                                                               window_size_left=-1, window_size_right=-1, softcap=0.0, alibi_slopes=None,
                                                               return_softmax=False, block_table=None)
         ctx.save_for_backward(qkv, out, lse, cu, rng)
-        ctx.meta = (max_seqlen, nq, nkv, hd, scale, causal, dropout_p)
         return out
 
     @staticmethod
     def backward(ctx, dout):
-        from flash_attn.flash_attn_interface import _wrapped_flash_attn_varlen_backward
-        qkv, out, lse, cu, rng = ctx.saved_tensors
+        qkv, out, lse, cu = ctx.saved_tensors[:4]
         max_seqlen, nq, nkv, hd, scale, causal, dropout_p = ctx.meta
-        T = qkv.shape[0]
-        q = qkv[:, : nq * hd].view(T, nq, hd)
-        k = qkv[:, nq * hd:(nq + nkv) * hd].view(T, nkv, hd)
-        v = qkv[:, (nq + nkv) * hd:].view(T, nkv, hd)
-        dqkv = torch.empty_like(qkv)
-        dq = dqkv[:, : nq * hd].view(T, nq, hd)
-        dk = dqkv[:, nq * hd:(nq + nkv) * hd].view(T, nkv, hd)
-        dv = dqkv[:, (nq + nkv) * hd:].view(T, nkv, hd)
         if _own_bwd_ok(hd, dropout_p):
-            lib().attn_bwd(dout.contiguous().view(T, nq, hd), q, k, v, out.view(T, nq, hd), lse, dq, dk, dv, cu, max_seqlen, scale, causal)
+            dqkv = lib().attn_bwd_qkv(dout, qkv, out, lse, cu, max_seqlen, nq, nkv, hd, scale, causal)
             return dqkv, None, None, None, None, None, None, None, None
+        from flash_attn.flash_attn_interface import _wrapped_flash_attn_varlen_backward
+        rng = ctx.saved_tensors[4] if len(ctx.saved_tensors) > 4 else torch.empty(2, dtype=torch.int64, device=qkv.device)
+        q, k, v = _qkv_views(qkv, nq, nkv, hd)
+        dqkv = torch.empty_like(qkv)
+        dq, dk, dv = _qkv_views(dqkv, nq, nkv, hd)
         _wrapped_flash_attn_varlen_backward(dout.contiguous(), q, k, v, out, lse, dq, dk, dv, cu, cu, max_seqlen, max_seqlen, dropout_p,
                                             scale, causal, -1, -1, 0.0, None, False, rng_state=rng)
         return dqkv, None, None, None, None, None, None, None, None
+
+
+def _qkv_views(qkv, nq: int, nkv: int, hd: int):
+    """q, k, v [T, heads, hd] as views of the fused [T, (nq + 2 nkv) * hd]."""
+    T = qkv.shape[0]
+    return (qkv[:, : nq * hd].view(T, nq, hd), qkv[:, nq * hd:(nq + nkv) * hd].view(T, nkv, hd), qkv[:, (nq + nkv) * hd:].view(T, nkv, hd))
+
+
+def _transformed() -> bool:
+    """Inside forward-mode differentiation or a function transform, which the autograd function answers for (by refusing)."""
+    return torch.autograd.forward_ad._current_level >= 0 or torch._C._functorch.peek_interpreter_stack() is not None
 
 
 def varlen_attention_qkv(qkv, cu_seqlens, max_seqlen: int, nq: int, nkv: int, hd: int, scale: Optional[float] = None,
                          causal: bool = True, dropout_p: float = 0.0):
     """Packed varlen attention taking the fused [T, (nq + 2 nkv) * hd] projection; returns [T, nq, hd]."""
     scale = scale if scale is not None else 1.0 / math.sqrt(hd)
-    T = qkv.shape[0]
     if use_native(qkv) and qkv.dtype in (torch.bfloat16, torch.float16) and qkv.stride(-1) == 1 and hd % 8 == 0:
+        if not (qkv.requires_grad and torch.is_grad_enabled()) and _own_fwd_ok(hd, dropout_p) and not _transformed():
+            # nothing will ask for a gradient: the autograd function around the kernel is most of a small call (32 us against 14)
+            return lib().attn_fwd_qkv(qkv, cu_seqlens.int(), max_seqlen, nq, nkv, hd, scale, causal)[0]
         return _PackedQKVAttention.apply(qkv, cu_seqlens.int(), max_seqlen, nq, nkv, hd, scale, causal, dropout_p)
-    q = qkv[:, : nq * hd].view(T, nq, hd)
-    k = qkv[:, nq * hd:(nq + nkv) * hd].view(T, nkv, hd)
-    v = qkv[:, (nq + nkv) * hd:].view(T, nkv, hd)
+    q, k, v = _qkv_views(qkv, nq, nkv, hd)
     return varlen_attention(q, k, v, cu_seqlens, max_seqlen, scale, causal, dropout_p)
 
 

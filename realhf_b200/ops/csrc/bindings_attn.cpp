@@ -5,6 +5,7 @@
 #include <torch/library.h>
 #include <torch/types.h>
 
+#include <array>
 #include <vector>
 
 using at::Tensor;
@@ -46,17 +47,18 @@ Tensor decode_attention(const Tensor& qkv, Tensor k_cache, Tensor v_cache, const
 
 extern "C" int rb_sample(const void* logits, int64_t row_stride, int64_t* next_tok, float* logprob, uint8_t* mask_bits,
                          int64_t mask_stride, const bool* unfinished, int B, int V, int top_k, float top_p, float inv_temp,
-                         int eos_id, int suppress_eos, int greedy, int pad_id, uint64_t seed, uint32_t step, int dt,
+                         int eos_id, int suppress_eos, int greedy, int pad_id, uint64_t seed, uint32_t step, bool* unfinished_out, int dt,
                          cudaStream_t s);
 
-// logits [B, V] -> (next token int64 [B], logprob fp32 [B], mask bits uint8 [B, ceil(V/8)] or empty)
-std::vector<Tensor> sample(const Tensor& logits, const c10::optional<Tensor>& unfinished, int64_t top_k, double top_p, double inv_temp,
+// logits [B, V] -> (next token int64 [B], logprob fp32 [B], mask bits uint8 [B, ceil(V/8)] or empty, rows that go on (unfinished and not eos) bool [B])
+std::vector<Tensor> sample_next(const Tensor& logits, const c10::optional<Tensor>& unfinished, int64_t top_k, double top_p, double inv_temp,
                            int64_t eos_id, bool suppress_eos, bool greedy, int64_t pad_id, int64_t seed, int64_t step, bool want_mask) {
   TORCH_CHECK(logits.is_cuda() && logits.dim() == 2 && logits.stride(1) == 1);
   const int B = logits.size(0), V = logits.size(1);
   c10::cuda::CUDAGuard guard(logits.device());
   auto tok = at::empty({B}, logits.options().dtype(at::kLong));
   auto lp = at::empty({B}, logits.options().dtype(at::kFloat));
+  auto goes_on = at::empty({B}, logits.options().dtype(at::kBool));
   Tensor mask = want_mask ? at::empty({B, (V + 7) / 8}, logits.options().dtype(at::kByte)) : at::empty({0}, logits.options().dtype(at::kByte));
   const bool* uf = nullptr;
   if (unfinished.has_value()) {
@@ -66,10 +68,18 @@ std::vector<Tensor> sample(const Tensor& logits, const c10::optional<Tensor>& un
   const int dt = logits.scalar_type() == at::kFloat ? 0 : (logits.scalar_type() == at::kBFloat16 ? 1 : (logits.scalar_type() == at::kHalf ? 2 : -1));
   int rc = rb_sample(logits.data_ptr(), logits.stride(0), tok.data_ptr<int64_t>(), lp.data_ptr<float>(),
                      want_mask ? mask.data_ptr<uint8_t>() : nullptr, want_mask ? mask.stride(0) : 0, uf, B, V, (int)top_k, (float)top_p,
-                     (float)inv_temp, (int)eos_id, suppress_eos, greedy, (int)pad_id, (uint64_t)seed, (uint32_t)step, dt,
+                     (float)inv_temp, (int)eos_id, suppress_eos, greedy, (int)pad_id, (uint64_t)seed, (uint32_t)step, goes_on.data_ptr<bool>(), dt,
                      at::cuda::getCurrentCUDAStream().stream());
   TORCH_CHECK(rc == 0, "sample: unsupported configuration (", rc, ")");
-  return {tok, lp, mask};
+  return {tok, lp, mask, goes_on};
+}
+
+// The same without the last output.
+std::vector<Tensor> sample(const Tensor& logits, const c10::optional<Tensor>& unfinished, int64_t top_k, double top_p, double inv_temp, int64_t eos_id,
+                           bool suppress_eos, bool greedy, int64_t pad_id, int64_t seed, int64_t step, bool want_mask) {
+  auto r = sample_next(logits, unfinished, top_k, top_p, inv_temp, eos_id, suppress_eos, greedy, pad_id, seed, step, want_mask);
+  r.pop_back();
+  return r;
 }
 
 extern "C" int* rb_attn_status();
@@ -156,6 +166,34 @@ void attn_bwd(const Tensor& dout, const Tensor& q, const Tensor& k, const Tensor
   TORCH_CHECK(rc == 0, "attn_bwd: unsupported configuration (", rc, ")");
 }
 
+// The three column ranges (q heads | k heads | v heads) of the fused projection output qkv [T, (nq + 2 nkv) hd] as [T, heads, hd] views.
+static std::array<Tensor, 3> split_qkv(const Tensor& qkv, int64_t nq, int64_t nkv, int64_t hd) {
+  TORCH_CHECK(qkv.dim() == 2 && qkv.stride(1) == 1 && qkv.size(1) == (nq + 2 * nkv) * hd);
+  const int64_t T = qkv.size(0), ld = qkv.stride(0), at0 = qkv.storage_offset();
+  auto part = [&](int64_t first, int64_t n) { return at::as_strided(qkv, {T, n, hd}, {ld, hd, 1}, at0 + first * hd); };
+  return {part(0, nq), part(nq, nkv), part(nq + nkv, nkv)};
+}
+
+// attn_fwd on the fused projection output: (out [T, nq, hd], lse [nq, T] fp32).
+std::vector<Tensor> attn_fwd_qkv(const Tensor& qkv, const Tensor& cu_seqlens, int64_t max_seqlen, int64_t nq, int64_t nkv, int64_t hd, double scale,
+                                 bool causal) {
+  at::NoGradGuard no_grad;
+  const auto [q, k, v] = split_qkv(qkv, nq, nkv, hd);
+  return attn_fwd_window(q, k, v, cu_seqlens, max_seqlen, scale, causal, 0);
+}
+
+// attn_bwd into the three column ranges of one d(qkv) buffer, which is returned.
+Tensor attn_bwd_qkv(const Tensor& dout, const Tensor& qkv, const Tensor& out, const Tensor& lse, const Tensor& cu_seqlens, int64_t max_seqlen, int64_t nq,
+                    int64_t nkv, int64_t hd, double scale, bool causal) {
+  at::NoGradGuard no_grad;
+  const int64_t T = qkv.size(0);
+  Tensor dqkv = at::empty_like(qkv);
+  const auto [q, k, v] = split_qkv(qkv, nq, nkv, hd);
+  const auto [dq, dk, dv] = split_qkv(dqkv, nq, nkv, hd);
+  attn_bwd(dout.contiguous().view({T, nq, hd}), q, k, v, out.view({T, nq, hd}), lse, dq, dk, dv, cu_seqlens, max_seqlen, scale, causal);
+  return dqkv;
+}
+
 extern "C" int rb_sample_graph(const void* logits, int64_t row_stride, int64_t* tok_hist, float* lp_hist, uint8_t* mask_hist,
                                int64_t mask_bytes, bool* unfinished, int* step_rows, int64_t* input_ids, int* cache_lens, int n_gen,
                                int min_new_tokens, int B, int V, int top_k, float top_p, float inv_temp, int eos_id, int greedy,
@@ -196,8 +234,11 @@ void register_attn_ops(torch::Library& m) {
   m.def("attn_check() -> ()", &attn_check);
   m.def("attn_status(Device device) -> Tensor", &attn_status);
   m.def("attn_bwd(Tensor dout, Tensor q, Tensor k, Tensor v, Tensor out, Tensor lse, Tensor(a!) dq, Tensor(b!) dk, Tensor(c!) dv, Tensor cu_seqlens, int max_seqlen, float scale, bool causal) -> ()", &attn_bwd);
+  m.def("attn_fwd_qkv(Tensor qkv, Tensor cu_seqlens, int max_seqlen, int nq, int nkv, int hd, float scale, bool causal) -> Tensor[]", &attn_fwd_qkv);
+  m.def("attn_bwd_qkv(Tensor dout, Tensor qkv, Tensor out, Tensor lse, Tensor cu_seqlens, int max_seqlen, int nq, int nkv, int hd, float scale, bool causal) -> Tensor", &attn_bwd_qkv);
   m.def("attn_fwd(Tensor q, Tensor k, Tensor v, Tensor cu_seqlens, int max_seqlen, float scale, bool causal) -> Tensor[]", &attn_fwd);
   m.def("attn_fwd_window(Tensor q, Tensor k, Tensor v, Tensor cu_seqlens, int max_seqlen, float scale, bool causal, int window) -> Tensor[]", &attn_fwd_window);
+  m.def("sample_next(Tensor logits, Tensor? unfinished, int top_k, float top_p, float inv_temp, int eos_id, bool suppress_eos, bool greedy, int pad_id, int seed, int step, bool want_mask) -> Tensor[]", &sample_next);
   m.def("sample(Tensor logits, Tensor? unfinished, int top_k, float top_p, float inv_temp, int eos_id, bool suppress_eos, bool greedy, int pad_id, int seed, int step, bool want_mask) -> Tensor[]", &sample);
   m.def("decode_attention(Tensor qkv, Tensor(a!) k_cache, Tensor(b!) v_cache, Tensor cache_lens, int nq, int nkv, int hd, float scale, Tensor? cos, Tensor? sin, int rot_dim, bool interleaved) -> Tensor", &decode_attention);
 }

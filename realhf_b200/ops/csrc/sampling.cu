@@ -60,6 +60,7 @@ struct SampleParams {
   int* cache_lens;
   bool* unfinished_rw;
   int n_gen, min_new_tokens;
+  bool* unfinished_out = nullptr;   // eager mode: unfinished and not eos
   const int64_t* seed_ptr;   // device-resident seed (a replayed graph must not repeat the random stream of the previous call)
 };
 
@@ -512,6 +513,7 @@ __global__ void __launch_bounds__(kThreads, 1) sample_kernel(SampleParams p) {
     const int64_t tok = live ? chosen : (int64_t)p.pad_id;
     p.next_tok[row * out_stride] = tok;
     p.logprob[row * out_stride] = live ? chosen_lp : 0.f;
+    if (p.unfinished_out != nullptr) p.unfinished_out[row] = live && tok != (int64_t)p.eos_id;
     if (in_graph) {
       p.input_ids[row] = tok;
       p.cache_lens[row] += 1;
@@ -578,13 +580,13 @@ int launch_sample(const SampleParams& p, int B, int dt, cudaStream_t s) {
 
 extern "C" int rb_sample(const void* logits, int64_t row_stride, int64_t* next_tok, float* logprob, uint8_t* mask_bits,
                          int64_t mask_stride, const bool* unfinished, int B, int V, int top_k, float top_p, float inv_temp,
-                         int eos_id, int suppress_eos, int greedy, int pad_id, uint64_t seed, uint32_t step, int dt,
+                         int eos_id, int suppress_eos, int greedy, int pad_id, uint64_t seed, uint32_t step, bool* unfinished_out, int dt,
                          cudaStream_t s) {
   if (B == 0) return 0;
   const size_t smem = (size_t)V * sizeof(float);
   if (smem > 200 * 1024) return -1;
   SampleParams p{logits, row_stride, next_tok, logprob, mask_bits, mask_stride, unfinished, V, top_k, eos_id, suppress_eos, greedy,
-                 pad_id, inv_temp, top_p, seed, step, nullptr, nullptr, nullptr, nullptr, 1, 0, nullptr};
+                 pad_id, inv_temp, top_p, seed, step, nullptr, nullptr, nullptr, nullptr, 1, 0, unfinished_out, nullptr};
   return launch_sample(p, B, dt, s);
 }
 
@@ -596,7 +598,7 @@ extern "C" int rb_sample_graph(const void* logits, int64_t row_stride, int64_t* 
   if (B == 0) return 0;
   if ((size_t)V * sizeof(float) > 200 * 1024) return -1;
   SampleParams p{logits, row_stride, tok_hist, lp_hist, mask_hist, mask_bytes * n_gen, unfinished, V, top_k, eos_id, 0, greedy,
-                 pad_id, inv_temp, top_p, 0, 0, step_rows, input_ids, cache_lens, unfinished, n_gen, min_new_tokens, seed_ptr};
+                 pad_id, inv_temp, top_p, 0, 0, step_rows, input_ids, cache_lens, unfinished, n_gen, min_new_tokens, nullptr, seed_ptr};
   return launch_sample(p, B, dt, s);
 }
 
