@@ -17,7 +17,7 @@
 //
 // What bounds it: the chain parts of S -> X, Y -> r -> U -> parts of U -> S of a head, products and element work in turn, which nothing else on the SM
 // overlaps.  8 sequences of 700..1024 tokens, 16 heads x 128 x 128: 518 us a token at a time on CUDA cores (shared-memory port and
-// latency), 249 this way.
+// latency), 188 this way (20700 cycles a chunk).
 #include "attn_common.cuh"
 
 #include <atomic>
