@@ -160,6 +160,46 @@ def _scaled_rows(h: torch.Tensor, tok: torch.Tensor, w_sorted: torch.Tensor) -> 
     return (h.index_select(0, tok).float() * w_sorted.float().unsqueeze(-1)).to(h.dtype)
 
 
+class _ToExperts(torch.autograd.Function):
+    """The token rows h [T, H] in the order sorted by expert: row back[t * k + j] is h[t].  Backward: the k rows of a token summed in fp32."""
+
+    @staticmethod
+    def forward(ctx, h, back, idx, E):
+        from realhf_b200.ops import lib
+        ctx.save_for_backward(back, idx)
+        ctx.E = E
+        return lib().moe_gather(h, back, idx.shape[1], None)
+
+    @staticmethod
+    def backward(ctx, dx):
+        from realhf_b200.ops import lib
+        back, idx = ctx.saved_tensors
+        dx = dx.contiguous()
+        dh = torch.empty(idx.shape[0], dx.shape[1], dtype=dx.dtype, device=dx.device)
+        ones = torch.empty(idx.shape, dtype=torch.float32, device=dx.device)       # (not read: every weight is 1)
+        lib().moe_combine(dx, dh, back, ones, idx, None, None, dh, ctx.E, True)
+        return dh, None, None, None
+
+
+class _FromExperts(torch.autograd.Function):
+    """out[t] = sum_j probs[t, j] y[back[t * k + j]], products and sum in fp32."""
+
+    @staticmethod
+    def forward(ctx, y, probs, back, idx, E):
+        from realhf_b200.ops import lib
+        ctx.save_for_backward(y, probs, back)
+        out = torch.empty(idx.shape[0], y.shape[1], dtype=y.dtype, device=y.device)
+        lib().moe_combine(y, out, back, probs, idx, None, None, out, E, False)
+        return out
+
+    @staticmethod
+    def backward(ctx, dout):
+        from realhf_b200.ops import lib
+        y, probs, back = ctx.saved_tensors
+        dy, dp = lib().moe_combine_bwd(dout.contiguous(), y, back, probs)
+        return dy, dp, None, None, None
+
+
 def moe_forward(model, i: int, h: torch.Tensor, mcfg=None, clamp: Optional[Tuple[float, float]] = None) -> torch.Tensor:
     """MoE MLP of block i on normalised hidden states h ([T, H], or [T/t, H] under sequence parallelism).  `mcfg`: the block's own
     MoE config in a heterogeneous stack (default: the model-wide one).  With `fp32_residual` the experts' outputs are combined
@@ -206,6 +246,18 @@ def moe_forward(model, i: int, h: torch.Tensor, mcfg=None, clamp: Optional[Tuple
                           bool(mcfg.scale_input))
         return out
     probs = _apply_capacity(probs, idx, E, mcfg)
+    if (not ep and not fused and not n_id and not mcfg.scale_input and not c.fp32_residual and mcfg.use_grouped_gemm and h.is_contiguous()
+            and _use_grouped_kernel(h, w_gu, w_dn) and 0 < T * k <= 32768 and k <= 8 and E <= 64):
+        # every assignment's place by counting, the rows there and back in one kernel each (forward and backward): the sort, the index arithmetic and two
+        # atomic index_add_ in 16 bits were 450 us of a training pass of 2048 tokens x 4096, this is 100
+        from realhf_b200.ops import gemm as G, lib
+        back, offsets = lib().moe_dispatch(idx, E, E)
+        hid = G.grouped_linear(_ToExperts.apply(h, back, idx, E), w_gu, offsets)
+        y_sorted = G.grouped_linear(_expert_act(hid, act), w_dn, offsets)
+        out = _FromExperts.apply(y_sorted, probs.float().contiguous(), back, idx, E)
+        if ctx.tp_size > 1:  # experts are F-sharded over TP: partial sums
+            out = TP.reduce_scatter_to_sp(out, ctx) if sp else TP.reduce_from_tp(out, ctx)
+        return _add_shared(model, i, h, mcfg, out, act)
     flat_e = idx.reshape(-1)
     order = torch.argsort(flat_e, stable=True)
     tok = torch.arange(T, device=h.device).repeat_interleave(k)[order]

@@ -47,6 +47,7 @@ int rb_softmax_router(const void*, int64_t, int, const void*, int, const void*, 
 int rb_moe_combine(const void*, int, const void*, int64_t, int, const int64_t*, const float*, const int64_t*, const void*, int, const float*, void*, int,
                    int64_t, int, int, int, int, cudaStream_t);
 int rb_moe_dispatch(const int64_t*, int64_t*, int*, int, int, int, cudaStream_t);
+int rb_moe_combine_bwd(const void*, int64_t, const void*, int, const int64_t*, const float*, void*, float*, int64_t, int, int, cudaStream_t);
 int rb_moe_gather(const void*, int64_t, int, const int64_t*, const float*, void*, int64_t, int, int, cudaStream_t);
 int rb_centred_norm(void*, int, const void*, int64_t, const void*, int64_t, int, float, float, const void*, const void*, const void*, int, float, void*,
                     int, int64_t, int, float, int, int, const void*, int64_t, int, cudaStream_t);
@@ -248,15 +249,28 @@ void moe_combine(const Tensor& y, const Tensor& x, const Tensor& row, const Tens
 }
 
 // idx [T, k] int64 (router outputs, E real experts of R) -> (row [T k] int64: place of each assignment in the order sorted by expert,
-// offsets [E + 1] int32: first row of each real expert); T k <= 1024
+// offsets [E + 1] int32: first row of each real expert); T k <= 32768
 std::vector<Tensor> moe_dispatch(const Tensor& idx, int64_t E, int64_t R) {
   CHECK_IN(idx);
   const int64_t N = idx.numel();
-  TORCH_CHECK(idx.scalar_type() == at::kLong && N >= 1 && N <= 1024 && R <= 64 && E <= R, "moe_dispatch: shapes");
+  TORCH_CHECK(idx.scalar_type() == at::kLong && N >= 1 && N <= 32768 && R <= 64 && E <= R, "moe_dispatch: shapes");
   c10::cuda::CUDAGuard g(idx.device());
   Tensor row = at::empty({N}, idx.options()), offsets = at::empty({E + 1}, idx.options().dtype(at::kInt));
   TORCH_CHECK(rb_moe_dispatch(idx.data_ptr<int64_t>(), row.data_ptr<int64_t>(), offsets.data_ptr<int>(), (int)N, (int)E, (int)R, cur_stream()) == 0);
   return {row, offsets};
+}
+
+// (dy [N, H] in y's order, dp [T, k] fp32) of out[t] = sum_j probs[t, j] y[row[t, j]]
+std::vector<Tensor> moe_combine_bwd(const Tensor& dout, const Tensor& y, const Tensor& row, const Tensor& probs) {
+  TORCH_CHECK(dout.is_cuda() && dout.dim() == 2 && dout.stride(1) == 1 && y.dim() == 2 && y.is_contiguous() && y.scalar_type() == dout.scalar_type());
+  TORCH_CHECK(probs.dim() == 2 && probs.is_contiguous() && probs.scalar_type() == at::kFloat && row.is_contiguous() && row.scalar_type() == at::kLong);
+  const int64_t T = dout.size(0), H = dout.size(1), k = probs.size(1);
+  TORCH_CHECK(probs.size(0) == T && row.numel() == T * k && y.size(0) == T * k && y.size(1) == H);
+  c10::cuda::CUDAGuard guard(dout.device());
+  auto dy = at::empty_like(y), dp = at::empty_like(probs);
+  TORCH_CHECK(rb_moe_combine_bwd(dout.data_ptr(), dout.stride(0), y.data_ptr(), dt_code(y), row.data_ptr<int64_t>(), probs.data_ptr<float>(), dy.data_ptr(),
+                                 dp.data_ptr<float>(), T * k, (int)H, (int)k, cur_stream()) == 0);
+  return {dy, dp};
 }
 
 // x [T, H], row [T k] -> xs [T k, H] with xs[row[i]] = x[i / k] (times scale[i], fp32 [T k], when given)
@@ -377,6 +391,7 @@ void register_mix_ops(torch::Library& m) {
   m.def("latent_out(Tensor o, Tensor? gate, bool element, Tensor(a!) out) -> ()", &latent_out);
   m.def("sigmoid_gate_(Tensor(a!) x, Tensor gate) -> ()", &sigmoid_gate_);
   m.def("moe_dispatch(Tensor idx, int E, int R) -> Tensor[]", &moe_dispatch);
+  m.def("moe_combine_bwd(Tensor dout, Tensor y, Tensor row, Tensor probs) -> Tensor[]", &moe_combine_bwd);
   m.def("moe_gather(Tensor x, Tensor row, int k, Tensor? scale=None) -> Tensor", &moe_gather);
   m.def("softmax_router(Tensor x, Tensor w, Tensor? corr, Tensor? u, int k, bool renorm, bool sigmoid=False) -> Tensor[]", &softmax_router);
   m.def("moe_combine(Tensor y, Tensor x, Tensor row, Tensor probs, Tensor idx, Tensor? y_shared, Tensor? gate, Tensor(a!) out, int E, bool unit=False) -> ()", &moe_combine);

@@ -115,3 +115,35 @@ def test_moe_decode_is_cuda_graph_capturable():
         o, _ = gen.generate(m, ids, cu, g, eos_id=2, pad_id=0)
         outs.append(o.tokens)
     assert torch.equal(outs[0], outs[1])
+
+
+@pytest.mark.parametrize("T,k,E", [(1, 2, 8), (512, 2, 8), (513, 2, 8), (1025, 3, 5), (4096, 8, 64)])
+def test_expert_rows_there_and_back(T, k, E):
+    """Places by counting (one tile of 1024 assignments, its edges, many), rows gathered and summed and their gradients, against plain torch in float64 on the
+    same 16-bit rows.  Bounds: a result is rounded once to bf16 (2^-8 of its value) after fp32 sums of k <= 8 products (8 * 2^-24 of the terms, inside the
+    atol); the weights' gradients are fp32 sums of H = 136 products of values below 5 (136 * 2^-24 * 25 = 2e-4)."""
+    from realhf_b200.models.moe import _FromExperts, _ToExperts
+    from realhf_b200.ops import lib
+    g = torch.Generator(device="cuda").manual_seed(T + k)
+    H = 136
+    idx = torch.rand(T, E, device="cuda", generator=g).topk(k, -1).indices
+    back, offsets = lib().moe_dispatch(idx, E, E)
+    order = torch.argsort(idx.reshape(-1), stable=True)
+    assert torch.equal(back[order], torch.arange(T * k, device="cuda"))
+    counts = torch.bincount(idx.reshape(-1), minlength=E).cumsum(0)
+    assert torch.equal(offsets.long(), torch.cat([counts.new_zeros(1), counts]))
+    h = torch.randn(T, H, device="cuda", generator=g).to(torch.bfloat16).requires_grad_(True)
+    y = torch.randn(T * k, H, device="cuda", generator=g).to(torch.bfloat16).requires_grad_(True)
+    p = torch.rand(T, k, device="cuda", generator=g).requires_grad_(True)
+    x = _ToExperts.apply(h, back, idx, E)
+    assert torch.equal(x[back], h.detach().repeat_interleave(k, 0))
+    dx = torch.randn(T * k, H, device="cuda", generator=g).to(torch.bfloat16)
+    (dh,) = torch.autograd.grad(x, h, dx)
+    torch.testing.assert_close(dh.double(), dx[back].double().view(T, k, H).sum(1), rtol=2 ** -8, atol=1e-5)
+    out = _FromExperts.apply(y, p, back, idx, E)
+    yt = y.detach()[back].double().view(T, k, H)
+    torch.testing.assert_close(out.double(), (yt * p.detach().double().unsqueeze(-1)).sum(1), rtol=2 ** -8, atol=1e-5)
+    dout = torch.randn(T, H, device="cuda", generator=g).to(torch.bfloat16)
+    dy, dp = torch.autograd.grad(out, (y, p), dout)
+    torch.testing.assert_close(dy[back].double().view(T, k, H), p.detach().double().unsqueeze(-1) * dout.double().unsqueeze(1), rtol=2 ** -8, atol=1e-5)
+    torch.testing.assert_close(dp.double(), (yt * dout.double().unsqueeze(1)).sum(-1), rtol=1e-5, atol=2e-4)
