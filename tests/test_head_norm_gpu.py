@@ -73,3 +73,50 @@ def test_delta_prepare_taps(d, dv, taps, dtype):
     assert float((got.cpu() - want).abs().max()) <= 2.0 ** -17 * float(want.abs().max())
     if taps > 1:
         assert torch.equal(c_st.cpu(), st)
+
+
+@pytest.mark.parametrize("taps", [2, 4, 7])
+def test_delta_prepare_many_tokens(taps):
+    """Enough tokens that a warp walks 32 of them: sequences that begin and end inside its tiles of 8, a remainder of tokens, the final inputs kept."""
+    from realhf_b200.api.model import DeltaRuleConfig
+    from realhf_b200.models.sharding import delta_sections
+    cfg = DeltaRuleConfig(n_heads=4, n_kv_heads=2, qk_dim=16, v_dim=24, conv_taps=taps)
+    g = torch.Generator().manual_seed(taps)
+    lens = [3000, 1, 2, 33, 31, 7, 5900]
+    T, C = sum(lens), 4 * 16 + 4 * 24
+    rn = lambda *s: torch.randn(*s, generator=g).to(torch.bfloat16)
+    proj, conv, A_log, bias = rn(T, sum(delta_sections(cfg))), rn(C, taps), rn(4), rn(4)
+    pos = torch.cat([torch.arange(n) for n in lens]).int()
+    remain = torch.cat([torch.arange(n - 1, -1, -1) for n in lens]).int()
+    slot = torch.cat([torch.full((n,), s) for n, s in zip(lens, [2, -1, 0, 3, 1, 5, 4])]).int()
+    st = torch.zeros(6, taps - 1, C)
+    c_st = st.clone().cuda()
+    want = R.delta_prepare_ref(proj, conv, A_log, bias, cfg, pos, st, slot, remain)
+    got = R.delta_prepare(proj.cuda(), conv.cuda(), A_log.cuda(), bias.cuda(), cfg, pos.cuda(), c_st, slot.cuda(), remain.cuda())
+    assert float((got.cpu() - want).abs().max()) <= 2.0 ** -17 * float(want.abs().max())      # the bound of the test above
+    assert torch.equal(c_st.cpu(), st)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("G,d,dv,norm", [(3, 128, 128, True), (4, 64, 72, True), (5, 40, 8, False)])
+def test_value_norm_of_many_tokens(G, d, dv, norm, dtype):
+    """Half a warp a (token, head) unit: unit counts that leave the last block partly empty, values narrower and wider than keys, rows of the cache that later
+    tokens overwrite.  Bound: one rounding to the type on each side of the same fp32 value, whose sums differ by a few 2^-24: one unit in the last place."""
+    from realhf_b200.api.model import WindowAttentionConfig
+    from realhf_b200.ops import attention as A
+    a = WindowAttentionConfig(n_heads=G, n_kv_heads=G, qk_dim=d, v_dim=dv, scale=1.0, window=30, keep_first=4, value_norm=norm, out_gate=False)
+    g = torch.Generator().manual_seed(G)
+    lens = [9000 // G, 1000, 1, 77, 1500]
+    T = sum(lens)
+    x = torch.randn(T, G * (2 * d + dv), generator=g).to(dtype)
+    pos = torch.cat([torch.arange(n) for n in lens]).int()
+    remain = torch.cat([torch.arange(n - 1, -1, -1) for n in lens]).int()
+    slot = torch.cat([torch.full((n,), s) for n, s in zip(lens, [2, -1, 0, 3, 1])]).int()
+    kc, vc = torch.zeros(4, G, 40, d, dtype=dtype), torch.zeros(4, G, 40, dv, dtype=dtype)
+    k2, v2 = kc.clone().cuda(), vc.clone().cuda()
+    want = A.value_norm_store(x, a, 1e-5, kc, vc, slot, pos, remain)
+    got = A.value_norm_store(x.cuda(), a, 1e-5, k2, v2, slot.cuda(), pos.cuda(), remain.cuda())
+    rel = 2.0 ** -7 if dtype == torch.bfloat16 else 2.0 ** -10
+    for w, f in ((want, got), (vc, v2)):
+        assert bool(((f.cpu().double() - w.double()).abs() <= rel * w.double().abs()).all())
+    assert torch.equal(k2.cpu(), kc)
