@@ -14,7 +14,7 @@
 //                    come from conv_state[slot], which is shifted by one.
 // Kernels on the decode path are launched with programmatic dependent launch (they signal their successors at once and wait for
 // their predecessor before the first global access), like the framework's other decode kernels.
-//   delta_rule       the recurrence (head size 128 x 128 with a decay per head, packed: delta_chunk.cu).  A column of S depends only on its own v column, so columns are independent: a thread group of
+//   delta_rule       the recurrence.  A column of S depends only on its own v column, so columns are independent: a thread group of
 //                    LPC lanes owns NC columns (16 state rows of each per lane in registers) or one (32 or 64 rows), a CTA all its groups' columns
 //                    of one (sequence, head).  q, k, v, beta, g of 8 tokens at a time are staged in shared memory.  Packed form: S starts
 //                    at zero and the final S goes to s_state[slot]; step form: S is loaded from and stored to s_state[slot].
@@ -791,8 +791,6 @@ static int launch_delta_column(const ScanParams& p, int n_seqs, cudaStream_t s) 
   return rb::launch_pdl(kern, dim3(n_seqs, p.H, RB_CEIL_DIV(p.dv, ncol)), dim3(kScanThreads), smem, s, p) == cudaSuccess ? 0 : -3;
 }
 
-extern "C" int rb_delta_chunk(const float* u, float* o, const int* cu, float* s_state, const int* slots, int n_seqs, int H, int G, cudaStream_t s);
-
 // channel: u rows hold a decay per state row (H * d numbers) instead of one per head
 extern "C" int rb_delta_rule(const float* u, float* o, const int* cu, float* s_state, const int* slots, int n_seqs, int H, int G, int d, int dv,
                              int step, int channel, cudaStream_t s) {
@@ -800,11 +798,6 @@ extern "C" int rb_delta_rule(const float* u, float* o, const int* cu, float* s_s
   if (d > 512 || H % G) return -1;
   ScanParams p{u, o, cu, s_state, slots, H, G, d, dv, step, dv % 4 == 0 && ((uintptr_t)s_state & 15) == 0};
   const bool many = (int64_t)n_seqs * H * RB_CEIL_DIV(dv, 64) >= rb::kNumSMs;
-  // 128 x 128 with a decay per head, rows of u whole float4s: chunks of 64 tokens on the tensor cores, whatever the lengths (the lengths are on the device).
-  // 8 sequences x 16 heads: 700 .. 1024 tokens 518 us a token at a time, 188 in chunks; the whole prefill of one sequence of 900 tokens 351 and 176, of eight of
-  // 20 .. 40 tokens 37.4 and 37.0, of one of 20 tokens 35.5 and 36.1 (the host).
-  if (!step && !channel && d == 128 && dv == 128 && H % 2 == 0 && (reinterpret_cast<uintptr_t>(u) & 15) == 0)
-    return rb_delta_chunk(u, o, cu, s_state, slots, n_seqs, H, G, s);
   if (step || (d <= 64 && !(d <= 32 && many))) {       // (lanes per column, state rows per lane)
 #define RB_L(LPC, EPL) return channel ? launch_delta_column<LPC, EPL, true>(p, n_seqs, s) : launch_delta_column<LPC, EPL, false>(p, n_seqs, s)
     if (d <= 32) { RB_L(1, 32); }
