@@ -15,7 +15,9 @@
 // merge splits): 128 x 32 heads 145 -> 121 us (6.5 TB/s; reading the same rows and doing nothing takes 113), 16 x 32 heads 27.1 -> 20.6 (16.0 of
 // it the kernel), 128 x 8 groups of four heads 95.6 -> 40.6, one group of eight heads a sequence, 20 x 1300 .. 3900, 43.3 -> 17.4.
 // A range that has too few (sequence, kv head) pairs to fill the GPU is split over a cluster of 2 .. 8 CTAs, which merge through
-// distributed shared memory: no partial sums in global memory and no second kernel.
+// distributed shared memory: no partial sums in global memory and no second kernel.  Infinities and NaN among the cached rows mean what they mean in a plain
+// sum (a score of minus infinity: a weight of 0): a warp whose sums are not finite takes its rows again on CUDA cores.  The tensor core's accumulators cut
+// off instead of rounding: 1e-6 of the sum over 4000 rows of values of one sign, a hundredth of what rounding the result to 16 bits does.
 // Replaces flash_attn_with_kvcache (reference: modules/attn.py:238-251).
 #include "attn_common.cuh"
 
@@ -396,30 +398,62 @@ __global__ void __launch_bounds__(kDecThreads, ctas_of(REP)) decode_attn_kernel(
   float* mysum = reinterpret_cast<float*>(ring + warp * NS * kSlotBytes);
   l += __shfl_xor_sync(0xffffffffu, l, 1);
   l += __shfl_xor_sync(0xffffffffu, l, 2);
-  if (g < REP && t == 0) { sm_m[warp][head] = m; sm_l[warp][head] = l; }
+  float finite = l * 0.f;                          // 0, or NaN
 #pragma unroll
-  for (int j = 0; j < HD / 16; ++j) {
-    constexpr float kDown = std::is_same<T, __half>::value ? 1.f / 32768.f : 1.f;
-    float x[4];
+  for (int j = 0; j < HD / 16; ++j)
 #pragma unroll
-    for (int i = 0; i < 4; ++i) x[i] = o[j][i] * kDown;
-    if constexpr (REP == 1) { x[0] += x[1]; x[2] += x[3]; }
-    if constexpr (REP <= 2) {
+    for (int i = 0; i < 4; ++i) finite = fmaf(o[j][i], 0.f, finite);
+  if (__any_sync(0xffffffffu, finite != 0.f)) {
+    // An infinity or a NaN among the keys or values: in a product it meets the zeros beside the parts, and parts of both signs, and what a plain sum
+    // makes of it (a weight of 0, an infinite output) is lost.  The warp goes over its rows again, a row at a time in fp32.
+#pragma unroll 1
+    for (int r = 0; r < REP; ++r) {
+      float mr = -INFINITY, lr = 0.f, acc[HD / 32] = {};
+#pragma unroll 1
+      for (int row0 = lo + warp * kStep; row0 < hi; row0 += kWarps * kStep)
+#pragma unroll 1
+        for (int row = row0; row < min(row0 + kStep, hi); ++row) {
+          float s = 0.f;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) x[i] += __shfl_xor_sync(0xffffffffu, x[i], 1);
+          for (int e = 0; e < HD / 32; ++e) s = fmaf(sq[r][e * 32 + lane], rb::to_f(kc[(int64_t)row * p.ks + e * 32 + lane]), s);
+          s = rb::warp_sum(s);
+          if constexpr (std::is_same<T, __half>::value) s *= s_unit[r];
+          const float mx = fmaxf(mr, s), zero = mx == -INFINITY ? 0.f : mx, corr = exp2f(mr - zero), w = exp2f(s - zero);
+          mr = mx;
+          lr = fmaf(lr, corr, w);
+#pragma unroll
+          for (int e = 0; e < HD / 32; ++e) acc[e] = fmaf(acc[e], corr, w * rb::to_f(vc[(int64_t)row * p.vs + e * 32 + lane]));
+        }
+      if (lane == 0) { sm_m[warp][r] = mr; sm_l[warp][r] = lr; }
+#pragma unroll
+      for (int e = 0; e < HD / 32; ++e) mysum[r * HD + e * 32 + lane] = acc[e];
     }
-    if constexpr (REP <= 4) {
+  } else {
+    if (g < REP && t == 0) { sm_m[warp][head] = m; sm_l[warp][head] = l; }
 #pragma unroll
-      for (int i = 0; i < 4; ++i) x[i] += __shfl_xor_sync(0xffffffffu, x[i], 2);
-    }
-    const int d = 16 * j + g;
-    if constexpr (REP == 1) {
-      if (t == 0) { mysum[d] = x[0]; mysum[d + 8] = x[2]; }
-    } else if (2 * t < REP) {
-      mysum[2 * t * HD + d] = x[0];
-      mysum[(2 * t + 1) * HD + d] = x[1];
-      mysum[2 * t * HD + d + 8] = x[2];
-      mysum[(2 * t + 1) * HD + d + 8] = x[3];
+    for (int j = 0; j < HD / 16; ++j) {
+      constexpr float kDown = std::is_same<T, __half>::value ? 1.f / 32768.f : 1.f;
+      float x[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) x[i] = o[j][i] * kDown;
+      if constexpr (REP == 1) { x[0] += x[1]; x[2] += x[3]; }
+      if constexpr (REP <= 2) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) x[i] += __shfl_xor_sync(0xffffffffu, x[i], 1);
+      }
+      if constexpr (REP <= 4) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) x[i] += __shfl_xor_sync(0xffffffffu, x[i], 2);
+      }
+      const int d = 16 * j + g;
+      if constexpr (REP == 1) {
+        if (t == 0) { mysum[d] = x[0]; mysum[d + 8] = x[2]; }
+      } else if (2 * t < REP) {
+        mysum[2 * t * HD + d] = x[0];
+        mysum[(2 * t + 1) * HD + d] = x[1];
+        mysum[2 * t * HD + d + 8] = x[2];
+        mysum[(2 * t + 1) * HD + d + 8] = x[3];
+      }
     }
   }
   __syncthreads();

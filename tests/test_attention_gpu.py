@@ -77,6 +77,36 @@ def test_decode_attention_step_edges(nq, nkv, S, hd, dtype):
         assert bool(((out[b].double() - ref).abs() <= bound).all()), (n, float((out[b].double() - ref).abs().max()))
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("nq,nkv,S", [(3, 3, 200), (4, 2, 1400), (8, 2, 150), (8, 1, 300)])
+def test_decode_attention_with_infinities_in_the_cache(nq, nkv, S, hd, dtype):
+    """A cached key that scores minus infinity has a weight of 0, an infinite value an infinite output in its column, a NaN a
+    NaN there: as float64 has it, and nothing else is touched.  Bound of the finite outputs: as in the test above."""
+    inf, n, B = float("inf"), S - 1, 5
+    g = torch.Generator(device=DEV).manual_seed(nq * 1000 + hd)
+    rnd = lambda *s: torch.randn(*s, device=DEV, generator=g).to(dtype)  # noqa: E731
+    kc, vc = rnd(B, S, nkv, hd), rnd(B, S, nkv, hd)
+    qkv = rnd(B, (nq + 2 * nkv) * hd)
+    qkv[:, : nq * hd] = qkv[:, : nq * hd].abs() + 0.5          # an element of a key has its sign in every score
+    rows = torch.arange(0, n, 37, device=DEV)
+    kc[0, rows, :, 5] = -inf                                   # sequence 0: weights of 0
+    kc[0, 3, 0, 7], vc[1, 11, 0, 9], vc[1, 60, 0, 10] = -inf, inf, -inf
+    kc[2, n - 1, 0, 0] = -inf
+    vc[3, 0, 0, 3] = float("nan")
+    q, k, v = (t.reshape(B, -1, hd).double() for t in qkv.split([nq * hd, nkv * hd, nkv * hd], 1))
+    out = A.decode_attention(qkv, kc, vc, torch.full((B,), n, dtype=torch.int32, device=DEV), nq, nkv, hd).view(B, nq, hd).double()
+    kk, vv = (torch.repeat_interleave(torch.cat([t[:, :n].double(), x.unsqueeze(1)], 1), nq // nkv, 2) for t, x in ((kc, k), (vc, v)))
+    w = torch.softmax(torch.einsum("bhd,bnhd->bhn", q, kk) * hd ** -0.5, -1)
+    ref = torch.einsum("bhn,bnhd->bhd", w, vv)
+    assert bool(torch.isfinite(ref[0]).all()) and bool(torch.isfinite(ref[4]).all())
+    assert torch.equal(torch.isnan(out), torch.isnan(ref)) and torch.equal(out[torch.isinf(ref)], ref[torch.isinf(ref)])
+    ok = torch.isfinite(ref)
+    most = vv.nan_to_num(0, 0, 0).abs().amax(1).amax(-1, keepdim=True).expand_as(ref)
+    rounding = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    assert bool(((out - ref).abs()[ok] <= (rounding * ref.abs() + 3e-5 * most)[ok]).all())
+
+
 @pytest.mark.parametrize("heads", [(8, 8), (8, 2)])
 def test_packed_qkv_attention_forward_backward(heads):
     """Fused-QKV varlen attention (one d(qkv) buffer written by the backward kernel) vs the fp32 reference on sliced q/k/v."""
