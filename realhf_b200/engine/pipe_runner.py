@@ -314,6 +314,7 @@ class PipelineRunner:
             hnd.wait()
         m.train(was_training)
         m.sequence_parallel = sp_saved
+        gen.raise_if_gave_up(dev)
         if not self.last:
             return None
         outs = []

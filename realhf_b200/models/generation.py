@@ -353,6 +353,15 @@ class StepSession:
         self.state.release([self.slot_of.pop(r) for r in ids])
 
 
+def raise_if_gave_up(dev: torch.device) -> None:
+    """Raises if a kernel of the steps so far gave up a bounded wait and left parts of its outputs unwritten.  Eager calls look at the status word before
+    their launch; a replayed step looks at nothing, so whoever hands its tokens out does, once, behind the last step."""
+    if dev.type == "cuda":
+        from realhf_b200.ops import lib
+        torch.cuda.current_stream(dev).synchronize()
+        lib().attn_check()
+
+
 @torch.no_grad()
 def generate(model: ReaLModel, input_ids: torch.Tensor, cu_seqlens: torch.Tensor, g: GenerationHyperparameters,
              eos_id: Optional[int], pad_id: int, generator: Optional[torch.Generator] = None,
@@ -508,6 +517,7 @@ def generate(model: ReaLModel, input_ids: torch.Tensor, cu_seqlens: torch.Tensor
         state.out = None
     model.train(was_training)
     model.sequence_parallel = sp_saved
+    raise_if_gave_up(dev)
     return GenerationOutput(tokens, logprobs, mask_bits, first.long(), no_eos), state
 
 
@@ -632,4 +642,5 @@ class InflightBatchingGenerator:
                     retire(s)
         m.train(was_training)
         m.sequence_parallel = sp_saved
+        raise_if_gave_up(m.device)
         return results

@@ -369,3 +369,34 @@ def test_a_wait_that_ran_out_is_raised_and_the_update_skipped():
     assert step() == 0.0 and not torch.equal(m.flat_param, before)
     fwd(), bwd(), engine._check_device_flags()
     torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("use_graph", [True, False])
+def test_a_wait_that_ran_out_in_a_generation_step_is_raised(use_graph, monkeypatch):
+    """A replayed step does not look at the status word (set here behind the last step by a copy): generate() does before it hands the tokens out."""
+    from realhf_b200.api.model import GenerationHyperparameters, ReaLModelConfig
+    from realhf_b200.models import generation as gen
+    from realhf_b200.models.real_model import ReaLModel
+    dev = torch.device("cuda", 0)
+    cfg = ReaLModelConfig(n_layers=1, n_kv_heads=2, n_q_heads=2, hidden_dim=128, intermediate_dim=256, vocab_size=512, n_positions=64, embd_pdrop=0.0,
+                          resid_pdrop=0.0, attn_pdrop=0.0, activation_function="silu", layer_norm_type="rms", mlp_type="llama", apply_rotary=True)
+    m = ReaLModel(cfg, dtype=torch.bfloat16, device=dev).init_random_fast()
+    ids, cu = torch.arange(3, 23, device=dev), torch.tensor([0, 8, 20], dtype=torch.int32, device=dev)
+    g = GenerationHyperparameters(max_new_tokens=4, min_new_tokens=4, greedy=True, use_cuda_graph=use_graph)
+    word, steps, final = lib().attn_status(dev), [], gen._final_logits
+
+    def run():
+        with torch.no_grad():
+            return gen.generate(m, ids, cu, g, eos_id=None, pad_id=0)[0].tokens
+
+    want, m.training = run(), True
+    if use_graph:
+        count = gen.launches.count_replay
+        monkeypatch.setattr(gen.launches, "count_replay", lambda n: (count(n), steps.append(1), word.fill_(int(len(steps) == 3))))
+    else:
+        monkeypatch.setattr(gen, "_final_logits", lambda *a: (final(*a), steps.append(1), word.fill_(int(len(steps) == 4)))[0])
+    with pytest.raises(RuntimeError, match="gave up"):
+        run()
+    assert m.training and lib().attn_wait_error() == 1
+    monkeypatch.undo()
+    assert torch.equal(run(), want)
