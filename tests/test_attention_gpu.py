@@ -333,6 +333,49 @@ def test_attn_bwd_items(heads, lens, causal):
         assert ((got.double() - w).abs() <= b + eps * w.abs() + 1e-6).all()
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("nq,nkv,hd", [(4, 4, 64), (8, 2, 128)])
+def test_packed_qkv_attention_on_columns_of_a_wider_buffer(nq, nkv, hd, dtype):
+    """The fused projection as a range of columns of wider rows: outputs and gradients bit for bit those of a copy, with and without a gradient asked for."""
+    lens = [1, 130, 77, 300]
+    T, W = sum(lens), (nq + 2 * nkv) * hd
+    cu = torch.tensor([0] + lens, device=DEV).cumsum(0).int()
+    g = torch.Generator(device=DEV).manual_seed(hd)
+    wide = torch.randn(T, W + 64, device=DEV, generator=g).to(dtype)
+    dout = torch.randn(T, nq, hd, device=DEV, generator=g).to(dtype)
+    a, b = wide[:, 32:32 + W], wide[:, 32:32 + W].contiguous()
+    call = lambda x: A.varlen_attention_qkv(x, cu, max(lens), nq, nkv, hd)
+    want = call(b)
+    assert torch.equal(call(a), want)
+    wide.requires_grad_(True)
+    leaf = b.requires_grad_(True)
+    got, out = call(wide[:, 32:32 + W]), call(leaf)
+    assert torch.equal(got, want) and torch.equal(out, want)
+    got.backward(dout)
+    out.backward(dout)
+    assert torch.equal(wide.grad[:, 32:32 + W], leaf.grad) and not wide.grad[:, :32].any() and not wide.grad[:, 32 + W:].any()
+
+
+def test_packed_qkv_attention_inside_function_transforms():
+    """Without a gradient asked for the kernel is called without its autograd function, which is what refuses forward-mode differentiation and function
+    transforms: they are refused all the same, and a plain tensor inside a forward-mode level is not."""
+    from torch.autograd import forward_ad as fw
+    T, n, hd = 40, 2, 64
+    cu = torch.tensor([0, T], dtype=torch.int32, device=DEV)
+    qkv = torch.randn(T, 3 * n * hd, device=DEV).to(torch.bfloat16)
+    call = lambda x: A.varlen_attention_qkv(x, cu, T, n, n, hd)
+    want = call(qkv)
+    with fw.dual_level():
+        assert torch.equal(call(qkv), want)
+        with pytest.raises((RuntimeError, NotImplementedError)):
+            call(fw.make_dual(qkv, torch.ones_like(qkv)))
+    with pytest.raises((RuntimeError, NotImplementedError)):
+        torch.func.vmap(call)(qkv.unsqueeze(0).expand(2, -1, -1))
+    with pytest.raises((RuntimeError, NotImplementedError)):
+        torch.func.grad(lambda x: call(x).float().sum())(qkv)
+    assert torch.equal(call(qkv), want)
+
+
 def test_a_wait_that_ran_out_is_raised_and_the_update_skipped():
     """The status word as a kernel leaves it whose bounded wait ran out (set here by a copy): the next attention call of either direction and the
     engine raise, the optimizer leaves the parameters alone, and clearing the word makes everything run again."""

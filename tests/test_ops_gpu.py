@@ -202,6 +202,41 @@ def test_lm_head_logprobs_fwd_bwd():
     torch.testing.assert_close(w.grad.float(), wr.grad, atol=5e-2, rtol=5e-2)
 
 
+@pytest.mark.parametrize("T,chunk", [(384, 384), (392, 384), (380, 384), (8, 8192)])
+@pytest.mark.parametrize("buffer", ["weight_type", "fp32", None])
+def test_head_gradient_is_added_to_what_the_buffer_holds(T, chunk, buffer):
+    """One chunk, more than one, a token count that is no multiple of 8; a gradient buffer of the weight's type, an fp32 one, none; twice in a row, the weight
+    also an embedding, against float64.  Bound: logits and their gradients in 16 bits (2^-9 of values up to 4) move the product by less than 2 %, each of at most
+    five sums is rounded to 16 bits; a sum left out or added twice is off by the product itself."""
+    from realhf_b200.ops import gemm as G
+    impl = OF.gemm_impl()
+    OF.set_gemm_impl(G.linear)
+    try:
+        torch.manual_seed(T)
+        H, V = 256, 1000
+        h = (torch.randn(T, H, device=DEV) * 0.5).to(torch.bfloat16)
+        w = torch.nn.Parameter((torch.randn(V, H, device=DEV) * 0.05).to(torch.bfloat16))
+        labels, ids = torch.randint(0, V, (T,), device=DEV), torch.randint(0, V, (T,), device=DEV)
+        d, e = torch.randn(T, device=DEV), torch.randn(T, H, device=DEV).to(torch.bfloat16) * 0.3
+        wr = w.detach().double().requires_grad_(True)
+        lp = torch.log_softmax(h.double() @ wr.t(), -1).gather(1, labels.unsqueeze(1)).squeeze(1)
+        (product,) = torch.autograd.grad((lp * d.double()).sum(), wr)
+        looked_up = torch.zeros_like(product).index_add_(0, ids, e.double())
+        old = torch.randn(V, H, device=DEV) * float(product.std())
+        if buffer == "weight_type":
+            old = old.to(torch.bfloat16)
+            w.grad, w._grad_in_flat_buffer = old.clone(), True
+        elif buffer == "fp32":
+            w.main_grad = old.clone()
+        for _ in range(2):
+            ((OF.lm_head_logprobs(h, w, labels, chunk=chunk) * d).sum() + (torch.nn.functional.embedding(ids, w) * e).sum()).backward()
+        got = sum(t.double() for t in (w.grad, getattr(w, "main_grad", None)) if t is not None)
+        want = 2 * (product + looked_up) + (old.double() if buffer else 0)
+        assert float((got - want).norm()) <= 0.02 * 2 * float(product.norm()) + 5 * 2.0 ** -9 * float(want.norm())
+    finally:
+        OF.set_gemm_impl(impl)
+
+
 @pytest.mark.parametrize("cfg", [("bf16", "bf16", "fp32", True), ("bf16", "bf16", "bf16", False), ("fp32", "fp32", "fp32", False),
                                  ("bf16", "fp32", "fp32", True)])
 def test_adamw_matches_reference(cfg):

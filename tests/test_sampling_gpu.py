@@ -190,3 +190,29 @@ def test_sample_with_fewer_thread_maxima_than_top_k(V, top_k):
     _, _, mb = lib().sample(x, None, top_k, 1.0, 1.0, -1, False, False, 0, 5, 3, True)
     kth = torch.topk(x.float(), top_k, -1).values[:, -1:]
     assert torch.equal(OF.unpack_mask_bits(mb, V), x.float() < kth)
+
+
+@pytest.mark.parametrize("top_k", [63, 64, 65, 127, 128, 129, 512])
+@pytest.mark.parametrize("V,dtype", [(32000, torch.bfloat16), (2051, torch.float32), (8192, torch.float16)])
+def test_sample_at_the_group_sizes_of_the_bound(V, dtype, top_k):
+    """The bound of the candidates comes from 256, 512 or 1024 maxima, by top_k: the kept set on both sides of each change, with ties at the threshold."""
+    torch.manual_seed(V + top_k)
+    x = (torch.randn(7, V, device=DEV) * 2).to(dtype)
+    tok, _, mb = lib().sample(x, None, top_k, 1.0, 1.0, -1, False, False, 0, 5, 3, True)
+    kth = torch.topk(x.float(), top_k, -1).values[:, -1:]
+    removed = OF.unpack_mask_bits(mb, V)
+    assert torch.equal(removed, x.float() < kth) and not removed[torch.arange(7, device=DEV), tok].any()
+
+
+@pytest.mark.parametrize("greedy", [True, False])
+@pytest.mark.parametrize("eos,pad", [(5, 0), (5, 5), (-1, 0)])
+def test_sample_next_says_which_rows_go_on(eos, pad, greedy):
+    """The last output against the expression it stands for: rows that draw eos, rows that draw another token, finished rows, padding that is eos itself, no eos."""
+    B, V = 64, 1000
+    x = torch.zeros(B, V, device=DEV)
+    x[torch.arange(B, device=DEV), torch.tensor([5, 6, 7, 0], device=DEV).repeat(B // 4)] = 60.0
+    live = torch.arange(B, device=DEV) % 3 != 0
+    tok, _, _, goes_on = lib().sample_next(x, live, V if greedy else 50, 1.0, 1.0, eos, False, greedy, pad, 3, 1, False)
+    assert torch.equal(tok, torch.where(live, x.argmax(-1), pad)) and goes_on.dtype == torch.bool
+    assert torch.equal(goes_on, live & (tok != eos))
+    assert torch.equal(lib().sample_next(x, None, 50, 1.0, 1.0, eos, False, greedy, pad, 3, 1, False)[3], x.argmax(-1) != eos)
