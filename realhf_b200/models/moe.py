@@ -247,9 +247,11 @@ def moe_forward(model, i: int, h: torch.Tensor, mcfg=None, clamp: Optional[Tuple
         return out
     probs = _apply_capacity(probs, idx, E, mcfg)
     if (not ep and not fused and not n_id and not mcfg.scale_input and not c.fp32_residual and mcfg.use_grouped_gemm and h.is_contiguous()
-            and _use_grouped_kernel(h, w_gu, w_dn) and 0 < T * k <= 32768 and k <= 8 and E <= 64):
+            and _use_grouped_kernel(h, w_gu, w_dn) and 0 < T * k <= (1 << 20) and k <= 8 and E <= 64):
         # every assignment's place by counting, the rows there and back in one kernel each (forward and backward): the sort, the index arithmetic and two
-        # atomic index_add_ in 16 bits were 450 us of a training pass of 2048 tokens x 4096, this is 100
+        # atomic index_add_ in 16 bits were 450 us of a training pass of 2048 tokens x 4096, this is 100.  Counting is one CTA, 1.4 us a thousand assignments
+        # (2.9 with 64 experts), and stays the smaller part: width 4096, 8 experts 512 wide, two a token, 20480 / 65536 tokens 3059 / 9474 us against 6632 / 20236
+        # with the sort; 64 experts, eight a token, 20480 tokens 10153 against 23140.  The line (a million assignments) lies beyond what was measured.
         from realhf_b200.ops import gemm as G, lib
         back, offsets = lib().moe_dispatch(idx, E, E)
         hid = G.grouped_linear(_ToExperts.apply(h, back, idx, E), w_gu, offsets)

@@ -249,11 +249,11 @@ void moe_combine(const Tensor& y, const Tensor& x, const Tensor& row, const Tens
 }
 
 // idx [T, k] int64 (router outputs, E real experts of R) -> (row [T k] int64: place of each assignment in the order sorted by expert,
-// offsets [E + 1] int32: first row of each real expert); T k <= 32768
+// offsets [E + 1] int32: first row of each real expert); T k <= 2^20
 std::vector<Tensor> moe_dispatch(const Tensor& idx, int64_t E, int64_t R) {
   CHECK_IN(idx);
   const int64_t N = idx.numel();
-  TORCH_CHECK(idx.scalar_type() == at::kLong && N >= 1 && N <= 32768 && R <= 64 && E <= R, "moe_dispatch: shapes");
+  TORCH_CHECK(idx.scalar_type() == at::kLong && N >= 1 && N <= (1 << 20) && R <= 64 && E <= R, "moe_dispatch: shapes");
   c10::cuda::CUDAGuard g(idx.device());
   Tensor row = at::empty({N}, idx.options()), offsets = at::empty({E + 1}, idx.options().dtype(at::kInt));
   TORCH_CHECK(rb_moe_dispatch(idx.data_ptr<int64_t>(), row.data_ptr<int64_t>(), offsets.data_ptr<int>(), (int)N, (int)E, (int)R, cur_stream()) == 0);

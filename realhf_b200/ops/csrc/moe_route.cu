@@ -8,7 +8,7 @@
 //                    order written, in fp32; y holds the expert outputs of the assignments sorted by expert, row[t, j] the place of
 //                    assignment (t, j) in that order; outputs e >= E are identity experts.  `unit`: every p is 1 (the routing weight
 //                    went into the experts' inputs); without g the shared expert's output is added as it is.
-//   moe_dispatch     up to 32768 assignments: their places in the order sorted by expert and the experts' row offsets, one CTA.
+//   moe_dispatch     up to 2^20 assignments: their places in the order sorted by expert and the experts' row offsets, one CTA.
 //   moe_combine_bwd  the gradients of moe_combine's outputs of experts: dy[row[t, j]] = p[t, j] dout[t], dp[t, j] = dout[t] . y[row[t, j]] (fp32).
 //   moe_gather       the token rows copied into that order, optionally times the assignment's routing weight (fp32 product).
 #include "anytype.cuh"
@@ -302,7 +302,7 @@ extern "C" int rb_moe_combine(const void* y, int dty, const void* x, int64_t ldx
 }
 
 extern "C" int rb_moe_dispatch(const int64_t* idx, int64_t* back, int* offsets, int N, int E, int R, cudaStream_t s) {
-  if (N < 1 || N > 32768 || R > kMaxOutputs || E > R) return -1;
+  if (N < 1 || N > (1 << 20) || R > kMaxOutputs || E > R) return -1;
   if (N > 1024)
     return rb::launch_pdl(moe_dispatch_tiles_kernel, dim3(1), dim3(1024), 0, s, idx, back, offsets, N, E, R) == cudaSuccess ? 0 : 2;
   return rb::launch_pdl(moe_dispatch_kernel, dim3(1), dim3(1024), 0, s, idx, back, offsets, N, E, R) == cudaSuccess ? 0 : 2;

@@ -147,3 +147,31 @@ def test_expert_rows_there_and_back(T, k, E):
     dy, dp = torch.autograd.grad(out, (y, p), dout)
     torch.testing.assert_close(dy[back].double().view(T, k, H), p.detach().double().unsqueeze(-1) * dout.double().unsqueeze(1), rtol=2 ** -8, atol=1e-5)
     torch.testing.assert_close(dp.double(), (yt * dout.double().unsqueeze(1)).sum(-1), rtol=1e-5, atol=2e-4)
+
+
+@pytest.mark.parametrize("T", [16392, 20480])
+def test_moe_layer_on_a_whole_minibatch_is_that_of_its_parts(T):
+    """Tokens do not meet in the expert layer: forward and the inputs' gradients of 32784 and 40960 assignments are bit for bit those of the two halves (fp32
+    weights and sums on either side of any limit on the number of assignments), and the sum of a token's rows is rounded once."""
+    from realhf_b200.models.moe import moe_forward
+    impl = OF.gemm_impl()
+    OF.set_gemm_impl(G.linear)
+    try:
+        cfg = hf_io.family("mixtral").make_test_config()
+        cfg.hidden_dim, cfg.intermediate_dim, cfg.n_q_heads, cfg.n_kv_heads, cfg.head_dim, cfg.vocab_size, cfg.n_layers = 256, 512, 4, 4, 64, 1024, 2
+        cfg.moe.num_experts, cfg.moe.top_k, cfg.moe.aux_loss_coeff, cfg.moe.z_loss_coeff = 8, 2, 0.0, 0.0
+        m = ReaLModel(cfg, dtype=torch.bfloat16, device=torch.device("cuda")).instantiate(seed=3, std=0.05)
+        m.train()
+        g = torch.Generator(device="cuda").manual_seed(T)
+        h, d = (torch.randn(T, 256, device="cuda", generator=g).to(torch.bfloat16) for _ in range(2))
+
+        def run(r):
+            x = h[r].clone().requires_grad_(True)
+            out = moe_forward(m, 1, x)
+            out.backward(d[r])
+            return out.detach(), x.grad
+        whole, parts = run(slice(0, T)), [run(slice(a, a + T // 2)) for a in (0, T // 2)]
+        for i in range(2):
+            assert torch.equal(whole[i], torch.cat([p[i] for p in parts]))
+    finally:
+        OF.set_gemm_impl(impl)
