@@ -1,4 +1,4 @@
-"""Best-effort import probe of the UNMODIFIED reference installed under baseline/_ref (see DESIGN.md "Reference arm").
+"""Best-effort import probe of the UNMODIFIED reference installed under baseline/_ref.
 
     python baseline/probe_reference.py
 

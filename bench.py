@@ -32,7 +32,7 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
 METRIC = "PPO tokens/sec (gen+train, device-timed max-over-ranks) LLaMA-7B x4"
-BASELINE_TOKENS_PER_S = 128 * 640 / (574.312 / 39)  # reference quickstart log: 39 steps in 574.312 s on 8 GPUs (BASELINE.md P5)
+BASELINE_TOKENS_PER_S = 128 * 640 / (574.312 / 39)  # reference quickstart log: 39 steps in 574.312 s on 8 GPUs
 
 
 class ClockSampler(threading.Thread):
@@ -123,7 +123,7 @@ class _NoSampler:
 
 
 def run_reference(args):
-    """The unmodified reference cannot run in this image: see DESIGN.md ("Reference arm")."""
+    """The unmodified reference cannot run in this image; the line printed says why."""
     why = ("reference installs into baseline/_ref only with --no-deps --ignore-requires-python; unmodified it cannot be imported on "
            "this image's Python 3.12: realhf/api/core/config.py declares a dataclass instance as a field default, which dataclasses "
            "reject since 3.11 (ValueError: mutable default ... use default_factory) -- every entry point imports that module; beyond "
@@ -282,7 +282,7 @@ def main():
     ap.add_argument("--steps", type=int, default=2)
     ap.add_argument("--warmup", type=int, default=3)
     ap.add_argument("--impl", default="ours", choices=["ours", "reference", "torchlib"],
-                    help="ours; reference (the unmodified reference: unavailable offline, see DESIGN.md); torchlib: an on-box A/B arm that is "
+                    help="ours; reference (the unmodified reference: unavailable offline); torchlib: an on-box A/B arm that is "
                          "NOT the reference -- this repo's executor with library kernels (cuBLAS GEMMs, flash-attn varlen attention, "
                          "F.layer_norm, NCCL reduce-scatter / all-gather / all-reduce) in place of the sm_100a kernels")
     ap.add_argument("--layers", type=int, default=32, help="debug only: fewer layers (result is then NOT the headline config)")

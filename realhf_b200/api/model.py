@@ -783,7 +783,7 @@ class ModelInterface(abc.ABC):
 
     def state_dict(self) -> Dict:
         """Algorithm state that lives outside the model (KL controller, value normaliser, ...): written with the recover
-        states and restored on a recover run.  (The reference loses this state on recovery)"""
+        states and restored on a recover run.  (The reference loses this state on recovery.)"""
         return {}
 
     def load_state_dict(self, sd: Dict):

@@ -247,7 +247,7 @@ class GpuUtilizationMonitor:
     """Samples NVML utilisation / memory / SM clock / power of ONE device on a daemon thread (parity: `gpu_utilization_monitor`,
     monitor.py:255-274, which logs util + memory of GPU `worker_idx % 8` every `interval` seconds for `ttl` seconds).  Differences:
     the samples are kept (bounded ring) and summarised on demand so that they can ride on an MFC reply, and the default
-    interval is seconds, not sub-second — NVML queries take a driver lock that CUDA-graph launches also need (DESIGN.md §3)."""
+    interval is seconds, not sub-second — NVML queries take a driver lock that CUDA-graph launches also need."""
 
     def __init__(self, device_index: int, interval: float = 2.0, ttl: "float | None" = None, max_samples: int = 4096, log: bool = False):
         import threading

@@ -4,7 +4,7 @@ Always: `stats.jsonl` in the run's log directory (one JSON object per MFC reply 
 Optional: TensorBoard event files (`REAL_TENSORBOARD=1` or `tensorboard=True` on the command line; written under
 `<log dir>/tensorboard`) and Weights & Biases (`wandb_mode=online|offline`, i.e. `WANDB_MODE`; offline runs stay on disk under
 the log directory).  The reference carries wandb / tensorboard fields in its configs but never writes to either
-(`api/core/system_api.py:96-104`, SURVEY.md section 5.5).  A sink that fails is switched off with one warning: statistics must
+(`api/core/system_api.py:96-104`).  A sink that fails is switched off with one warning: statistics must
 never stop a training run."""
 
 from __future__ import annotations

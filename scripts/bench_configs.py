@@ -1,4 +1,4 @@
-"""The secondary BASELINE.json configurations through the production runtime (quickstart -> launcher -> master + model workers),
+"""The secondary configurations through the production runtime (quickstart -> launcher -> master + model workers),
 at reduced depth, with random-init weights and synthetic data; prints ONE JSON line per run.
 
     python scripts/bench_configs.py 13b-tp2pp2  --gpus 4    # LLaMA-13B shapes, PPO, every MFC tp2 x pp2, CUDA-graph pipelined decode

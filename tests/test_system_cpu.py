@@ -1,5 +1,5 @@
 """Whole runtime on CPU/gloo: launcher -> master worker + 2 model workers (separate OS processes) -> GPT-2 SFT with
-DP=2 on a synthetic dataset (BASELINE.json config #1), then PPO with parameter reallocation between two layouts."""
+DP=2 on a synthetic dataset, then PPO with parameter reallocation between two layouts."""
 import os
 import sys
 import uuid
