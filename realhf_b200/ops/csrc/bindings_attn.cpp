@@ -74,7 +74,7 @@ std::vector<Tensor> sample_next(const Tensor& logits, const c10::optional<Tensor
   return {tok, lp, mask, goes_on};
 }
 
-// The same without the last output.
+// The same without the last output: the op as callers outside the package know it (the package itself takes sample_next).
 std::vector<Tensor> sample(const Tensor& logits, const c10::optional<Tensor>& unfinished, int64_t top_k, double top_p, double inv_temp, int64_t eos_id,
                            bool suppress_eos, bool greedy, int64_t pad_id, int64_t seed, int64_t step, bool want_mask) {
   auto r = sample_next(logits, unfinished, top_k, top_p, inv_temp, eos_id, suppress_eos, greedy, pad_id, seed, step, want_mask);
@@ -141,7 +141,8 @@ extern "C" int rb_attn_bwd(const void* q, const void* k, const void* v, const vo
                            int64_t o_ld, int64_t do_ld, int64_t dq_ld, int64_t dk_ld, int64_t dv_ld, int T, int B, int nq, int nkv,
                            int hd, int max_seqlen, float scale, int causal, int dt, cudaStream_t s);
 
-// Writes dq / dk / dv (views with the same layout rules as q / k / v, e.g. column ranges of one d(qkv) buffer).
+// Writes dq / dk / dv (views with the same layout rules as q / k / v, e.g. column ranges of one d(qkv) buffer).  attn_bwd_qkv below is what training calls; as an
+// op of its own it stays for callers that hold q, k and v apart.
 void attn_bwd(const Tensor& dout, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& out, const Tensor& lse, Tensor dq,
               Tensor dk, Tensor dv, const Tensor& cu_seqlens, int64_t max_seqlen, double scale, bool causal) {
   TORCH_CHECK(q.is_cuda() && q.dim() == 3);

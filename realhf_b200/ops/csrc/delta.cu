@@ -233,7 +233,9 @@ __global__ void __launch_bounds__(kPThreads) delta_prepare_tiled_kernel(const vo
 // The same for head sizes in whole fours up to 128 on aligned rows: a warp owns one unit of channels, four neighbouring ones a lane, and walks kWalk
 // tokens in tiles of 8 whose rows it has in flight together; the per-(token, head) sum of squares stays inside the warp.  The kernel above moves two
 // bytes a lane and load and four a store, and waits for its loads with few of them on their way: 8 sequences of 700 .. 1024 tokens, 16 + 2 x 4 heads x 128
-// (71 MB in, 85 MB out) 121 us; this way 87 (exact exponentials and divisions).  kTaps: the taps that registers are kept for.
+// (71 MB in, 85 MB out) 121 us; this way 87.  What it waits for is its loads: the tiles take 124 registers, so 14 warps an SM are resident, half of their stalls
+// are on a load, and the issue slots are busy 38 % of the time with 46 instructions a channel and token (24 us of bytes, about 20 of issue).  kTaps: the taps
+// that registers are kept for.
 constexpr int kTile = 8;
 
 template <int kTaps, int kWalk>

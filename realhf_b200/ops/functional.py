@@ -370,7 +370,8 @@ class _LMHeadLogProb(torch.autograd.Function):
             if (mg is None and T <= ctx.chunk and getattr(weight, "_grad_in_flat_buffer", False) and weight.grad is not None
                     and weight.grad.dtype == weight.dtype and _native_gemm(hidden, weight) is not None and T % 8 == 0):
                 # one chunk and a gradient buffer of the weight's own type: the product's fp32 sums are added to it and rounded once, as for every
-                # other projection (ops.gemm._linear_backward); an fp32 copy of dW, its cast and its sum were four passes over [V, H]
+                # other projection (ops.gemm._linear_backward); an fp32 copy of dW, its cast and its sum were four passes over [V, H].  Several chunks keep the
+                # copy: into the buffer each of them would be rounded by itself
                 dw = weight.grad
             elif mg is not None and mg.dtype == torch.float32 and _native_gemm(hidden, weight) is not None:
                 dw = mg  # same contract as ops.gemm._Linear: wgrad accumulates into the fp32 main-grad view
