@@ -118,6 +118,12 @@ struct UnitSearch {
   }
 };
 
+RB_DEVICE float max3(float a, float b, float c) {
+  float d;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
+
 // cap * tanh(s * scale / cap) + add in the log2 domain, tanh(x) = 1 - 2 / (1 + 2^(2 x log2 e)): c = 2 log2 e * scale / cap,
 // k = cap log2 e, k_add = k + add.  Absolute error a few ulp of k; saturates to +-k.
 RB_DEVICE float soft_cap2(float s, float c, float k, float k_add) {

@@ -11,24 +11,29 @@
 // rows (grouped heads, even group: both walk the same tiles), else two neighbouring query tiles of a head (counted from the end of
 // the sequence, so that a left-over single tile is the shortest one).  Sharing the stream also halves the L2 traffic per product: one
 // tile each would ask for 64 B per cycle and SM, more than L2 gives.  With one tile per CTA and four softmax warps the tensor pipe was
-// active 19% of the time: 32 x 640 tokens x 32 heads took 518 us (now 228), 8 x 1500..4096 x 32 / 8 heads (26655 tokens) 2365 us (now 818).
+// active 19% of the time.
 //
-// CTA = 12 warps, one CTA per SM.  Warps 0-3 / 4-7: softmax of tile 0 / 1 (thread = query row = TMEM lane).  Warp 8: MMA issue and TMEM
-// allocation.  Warp 9: TMA producer and scheduler (10, 11: idle, they complete the warpgroup whose registers go to the softmax).  The
-// grid holds one CTA per work item (a bound: sequence lengths are on the device); a running CTA takes the items of CTAs that have
+// CTA = 16 warps, one CTA per SM.  Warps 0-3 / 4-7: softmax of tile 0 / 1 (thread = query row = TMEM lane).  Warp 8: MMA issue and TMEM
+// allocation.  Warp 9: TMA producer and scheduler (10, 11: idle, they complete the warpgroup whose registers go to the softmax).  Warps 12-15 (one per
+// TMEM quadrant, both tiles): they scale O and write it out.  With both left to the softmax warps a key tile cost them 470 of 2370 cycles for the scaling, and the
+// output, 5000 cycles a pair of tiles, lay between two items: 32 x 640 tokens x 32 heads 232 -> 188 us, 8 x 1500..4096 x 32 / 8 heads
+// 839 -> 734 us, 32 x 1024 tokens with window 512 + 64 kept 270 -> 224 us, 300..777 tokens of 12 heads with window 500 114 -> 99 us.  What bounds it
+// now, per key tile and query tile: 580 cycles to the maximum, 1500 for the 128 exponentials of a thread (1090 at 8.5 cycles each if nothing else ran), 1360
+// from the weights to the next scores (two products, 1024); two tiles share the pipe, so it is active 57 % of the time.  Every second pair of
+// exponentials by a polynomial on the multiply-add units was slower (10.9 cycles each).  Long batches run into the power limit (1.7 GHz).
+//
+// The grid holds one CTA per work item (a bound: sequence lengths are on the device); a running CTA takes the items of CTAs that have
 // not started (`clusterlaunchcontrol.try_cancel`), so barriers, TMEM and descriptors are set up once per SM, the next item's Q / K / V
 // load while the last one's softmax and output run, and ragged batches balance themselves.
 //
 // Tensor memory (512 columns): S_t at 128 t, O_t at 256 + 128 t.  P_t (16 bit) overwrites the front of S_t and is the TMEM A operand of
 // P V, so it never travels through shared memory; S_t of the next tile is issued behind that product on the in-order tensor pipe.  O
-// accumulates in TMEM over the whole stream; when a row's maximum grows, its warp scales O once the product in flight has retired and
-// the weights are stored: the scores' registers then hold the whole output row at once (before the exponentials, a quarter at a time: 15 us of
-// 305 in a windowed prefill).  (A maximum
+// accumulates in TMEM over the whole stream; when a row's maximum grows, its factor goes to the output warp of its quadrant, which scales O while the weights
+// are formed: the product before has retired (the scores that showed the growth were issued behind it), and the next one waits for both.  (A maximum
 // that only moves when weights exceed it by 2^8 is 2..3 % faster in training, 10 % with a window, but the largest weight is then no longer exactly
 // 1 when P is rounded to 16 bits: error against 64 bits 0.0028 instead of 0.0025.)  V_j is the MN-major B operand.
-// Issue order: S_0, S_1, then per key tile PV_0, S_0', PV_1, S_1'.  The issuing warp runs converged and elects a lane for the MMAs alone: issued from
-// `if (lane == 0)` with descriptors built there, eight MMAs took 820-960 cycles of one thread, whatever their size (294 -> 242 us converged, 231 us with the
-// descriptors built in front of the elected branch; two scores per instruction in the softmax: 221 us; 228 us with the maximum of every tile).
+// Issue order: S_0, S_1, then per key tile PV_0, S_0', PV_1, S_1'.  The issuing warp runs converged, the MMAs are predicated on an elected lane: issued from
+// `if (lane == 0)` with descriptors built there, eight MMAs took 820-960 cycles of one thread, whatever their size.
 //
 // Outputs: O [T, nq, DV] through a per-warp staging buffer (whole 128-byte lines), LSE [nq, T] (natural log, scale applied).
 //
@@ -38,15 +43,15 @@
 // maximum is taken over the raw products.  kCap: kSimple with score = softcap * tanh(s * scale / softcap), formed before the
 // masks, so that a product that overflowed to -infinity is a visible score of -softcap.  All three: a per-head sink logit starts the running maximum with denominator 1; the output is
 // multiplied by sigmoid(gate logit of its head, or of the output element); `chunk` > 0 replaces the window: a query sees the keys of its own
-// chunk of positions up to itself.  (32 x 1024 tokens, 16 / 4 heads, window 512 + 64 kept: 1350 us with one tile per CTA, now 278.)
+// chunk of positions up to itself.
 // Learned distance biases and shared keys / values run in attn_fwd_bias.cu.
 #include "attn_common.cuh"
 
 namespace {
 
 constexpr int kTile = 128;          // query rows of a tile (= UMMA M) and keys of a tile (= UMMA N of S, K of P V)
-constexpr int kFwdThreads = 384;    // three warpgroups: 168 registers a thread at launch, 64512 in all
-constexpr int kSoftmaxRegs = 208, kOtherRegs = 80;   // 2 x 128 x 208 + 128 x 80 = 63488: a softmax thread holds a whole score row
+constexpr int kFwdThreads = 512;    // four warpgroups: 128 registers a thread at launch
+constexpr int kSoftmaxRegs = 184, kOtherRegs = 64, kOutRegs = 80;   // 128 x (2 x 184 + 64 + 80) = 65536: a softmax thread holds a whole score row
 constexpr int kStages = 4;          // K and V tiles share one ring: two key tiles in flight
 
 enum Mode { kPlain = 0, kSimple = 1, kCap = 2, kGeneral = 3 };
@@ -54,12 +59,13 @@ enum Mode { kPlain = 0, kSimple = 1, kCap = 2, kGeneral = 3 };
 template <int kD, int kDV> struct FCfg {
   static constexpr int kQBytes = kTile * kD * 2, kKBytes = kTile * kD * 2, kVBytes = kTile * kDV * 2;
   static constexpr int kStageBytes = kKBytes > kVBytes ? kKBytes : kVBytes;
-  static constexpr int kKV = 2 * kQBytes, kOut = kKV + kStages * kStageBytes, kBars = kOut + 8 * 4096;
-  static constexpr int kSmemBytes = kBars + 1024 /*align*/ + 512 /*barriers, items*/;
+  static constexpr int kKV = 2 * kQBytes, kOut = kKV + kStages * kStageBytes, kRows = kOut + 4 * 4096, kBars = kRows + 2 * 3 * kTile * 4;
+  static constexpr int kSmemBytes = kBars + 512 /*barriers, items*/;
 };
 
-enum FBar { Q_FULL = 0, Q_EMPTY = 2, KV_FULL = 4, KV_EMPTY = 8, S_FULL = 12, P_FULL = 14, O_FULL = 16, O_EMPTY = 18, IT_FULL = 20, IT_EMPTY = 22,
-            CLC_FULL = 24, F_NUM_BARS = 25 };
+enum FBar { Q_FULL = 0, Q_EMPTY = 2, KV_FULL = 4, KV_EMPTY = 8, S_FULL = 12, P_FULL = 14, O_FULL = 16, A_FULL = 18 /* [tile][quadrant] */, L_FULL = 26, L_EMPTY = 28,
+            IT_FULL = 30, IT_EMPTY = 32, CLC_FULL = 34, F_NUM_BARS = 35 };
+constexpr int kItemReaders = 1 + 8 + 4;      // MMA, softmax and output warps
 
 // One work item: sequence (first token, length), heads and query tiles of the two tiles (tile 1 < 0: absent); L < 0 ends the CTA's loop.
 struct Item { int tok0, L, head0, head1, qt0, qt1; };
@@ -89,17 +95,24 @@ template <int kD, int kDV, typename T, int kFmt, int kMode>
 __global__ void __launch_bounds__(kFwdThreads, 1) attn_fwd_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant__ CUtensorMap tma_k,
                                                                   const __grid_constant__ CUtensorMap tma_v, const __grid_constant__ AttnParams p) {
   using C = FCfg<kD, kDV>;
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  extern __shared__ __align__(1024) uint8_t smem[];      // (addresses are constants then, not registers)
   const uint32_t sQ = ptx::smem_u32(smem), sKV = sQ + C::kKV;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::kBars);
-  Item* items = reinterpret_cast<Item*>(smem + C::kBars + 256);                // two slots of 24 bytes
-  const uint32_t clc = sQ + C::kBars + 256 + 64;                               // 16 bytes
-  uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(smem + C::kBars + 256 + 80);
+  Item* items = reinterpret_cast<Item*>(smem + C::kBars + 288);                // two slots of 24 bytes
+  const uint32_t clc = sQ + C::kBars + 288 + 64;                               // 16 bytes
+  uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(smem + C::kBars + 288 + 80);
+  static_assert(F_NUM_BARS * 8 <= 288, "barriers");
   volatile uint32_t* dead = tmem_ptr + 1;
   auto bar = [&](int i) { return ptx::smem_u32(&bars[i]); };
   auto wait = [&](int i, uint32_t parity) { bounded_wait(bar(i), parity, dead); };
+  if ((sQ & 1023u) != 0u) {                                // (the swizzle wants it; never seen)
+    if (threadIdx.x == 0) *reinterpret_cast<volatile int*>(p.status) = 1;
+    return;
+  }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  float* row_alpha = reinterpret_cast<float*>(smem + C::kRows);      // [tile][row]: factor on the row's O, written with every key tile behind the first
+  float* row_l = row_alpha + 2 * kTile;                              // [tile][row]: denominator and maximum, written behind the last one
+  float* row_m = row_l + 2 * kTile;
 
   if (warp == 9 && lane == 0) {
     *dead = 0;
@@ -107,8 +120,8 @@ __global__ void __launch_bounds__(kFwdThreads, 1) attn_fwd_kernel(const __grid_c
     ptx::prefetch_tensormap(&tma_k);
     ptx::prefetch_tensormap(&tma_v);
     for (int i = 0; i < F_NUM_BARS; ++i) {
-      const bool softmax_side = (i >= P_FULL && i < P_FULL + 2) || (i >= O_EMPTY && i < O_EMPTY + 2);
-      ptx::mbar_init(bar(i), softmax_side ? 4 : (i >= IT_EMPTY && i < IT_EMPTY + 2) ? 9 : 1);   // items: the MMA thread and 8 softmax warps
+      // P_FULL: the four softmax warps of the tile and the four output warps
+      ptx::mbar_init(bar(i), i >= P_FULL && i < P_FULL + 2 ? 8 : i >= L_FULL && i < L_EMPTY + 2 ? 4 : i >= IT_EMPTY && i < IT_EMPTY + 2 ? kItemReaders : 1);
     }
     ptx::fence_barrier_init();
   }
@@ -121,7 +134,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) attn_fwd_kernel(const __grid_c
   ptx::tc_fence_after();
   const uint32_t tmem_base = *tmem_ptr;
 
-  if (warp >= 8) {
+  if (warp >= 8 && warp < 12) {
     ptx::reg_dec<kOtherRegs>();
     if (warp == 9) {
       // ===================================================== scheduler + TMA producer
@@ -207,11 +220,15 @@ __global__ void __launch_bounds__(kFwdThreads, 1) attn_fwd_kernel(const __grid_c
       }
       publish(Item{0, -1, 0, 0, -1, -1});
     } else if (warp == 8) {
-      // ===================================================== MMA issuer: the whole warp runs the loop, one elected lane issues
+      // ===================================================== MMA issuer: the whole warp runs the loop, one elected lane issues.  A wait costs the warp 100 to 200 cycles
+      // even when there is nothing to wait for, and the pipe holds only some 256 cycles of products: what the tiles' barriers say is asked for ahead of the
+      // products in front of them.
       constexpr uint32_t idesc_s = ptx::make_idesc_f16(kFmt, kTile, kTile, 0, 0);   // Q, K both K-major (head-dim contiguous)
       constexpr uint32_t idesc_o = ptx::make_idesc_f16(kFmt, kTile, kDV, 0, 1);     // P (TMEM), V MN-major
-      const uint32_t tm = (uint32_t)ptx::uniform((int)tmem_base);
-      uint32_t kvc = 0, qc[2] = {0, 0}, pc[2] = {0, 0}, oc[2] = {0, 0};
+      constexpr uint32_t kToMN = (uint32_t)((kTile * 128 - 16) >> 4) << 16;         // from the K-major form of a tile to its MN-major one
+      const uint32_t tm = (uint32_t)ptx::uniform((int)tmem_base), el = ptx::elect_one() ? 1u : 0u;
+      const uint32_t q_lo = ptx::desc_lo(sQ, 16), kv_lo = ptx::desc_lo(sKV, 16);
+      uint32_t kvc = 0, qc[2] = {0, 0}, pc[2] = {0, 0};
       for (int n_it = 0;; ++n_it) {
         const int slot = n_it & 1;
         wait(IT_FULL + slot, (uint32_t)(n_it >> 1) & 1u);
@@ -224,44 +241,37 @@ __global__ void __launch_bounds__(kFwdThreads, 1) attn_fwd_kernel(const __grid_c
         if (it.L < 0 || ptx::uniform((int)*dead)) break;
         const Walk w(it, p);
         bool s_open[2] = {false, false}, o_open[2] = {false, false};
-        auto issue_s = [&](int t, int j, int st) {
+        auto last_tile = [&](int t) { return (t ? w.end1 : w.end0) - 1; };
+        auto issue_s = [&](int t, int j, uint32_t st) {
           if (!s_open[t]) { wait(Q_FULL + t, qc[t] & 1u); ++qc[t]; s_open[t] = true; }
           ptx::tc_fence_after();
-          const uint64_t a = ptx::make_smem_desc_sw128(sQ + t * C::kQBytes, 16, 1024), b = ptx::make_smem_desc_sw128(sKV + st * C::kStageBytes, 16, 1024);
-          if (ptx::elect_one()) {
+          const uint32_t a = q_lo + t * (C::kQBytes >> 4), b = kv_lo + st * (C::kStageBytes >> 4);
 #pragma unroll
-            for (int kk = 0; kk < kD / 16; ++kk) {
-              const uint32_t off = (kk >> 2) * (kTile * 128) + (kk & 3) * 32;
-              ptx::tc_mma_f16(tm + t * 128, a + (off >> 4), b + (off >> 4), idesc_s,
-                              kk != 0 ? 1u : 0u);
-            }
-            ptx::tc_commit(bar(S_FULL + t));
-            if (j == (t ? w.end1 : w.end0) - 1) ptx::tc_commit(bar(Q_EMPTY + t));
+          for (int kk = 0; kk < kD / 16; ++kk) {
+            const uint32_t off = ((kk >> 2) * (kTile * 128) + (kk & 3) * 32) >> 4;
+            ptx::tc_mma_f16_if(el, tm + t * 128, a + off, b + off, idesc_s, kk != 0 ? 1u : 0u);
           }
-          __syncwarp();
+          ptx::tc_commit_if(el, bar(S_FULL + t));
+          if (j == last_tile(t)) ptx::tc_commit_if(el, bar(Q_EMPTY + t));
         };
-        auto issue_pv = [&](int t, int st) {
+        auto issue_pv = [&](int t, int j, uint32_t st) {
           wait(P_FULL + t, pc[t] & 1u);
           ++pc[t];
-          if (!o_open[t]) { wait(O_EMPTY + t, (oc[t] & 1u) ^ 1u); ++oc[t]; }
           ptx::tc_fence_after();
-          const uint64_t b = ptx::make_smem_desc_sw128(sKV + st * C::kStageBytes, kTile * 128, 1024);
-          if (ptx::elect_one()) {
+          const uint32_t b = kv_lo + kToMN + st * (C::kStageBytes >> 4), keep = o_open[t] ? 1u : 0u;
 #pragma unroll
-            for (int kk = 0; kk < kTile / 16; ++kk)      // A: 16 keys = 8 TMEM columns; B: 16 key rows = 2048 B down every 64-wide chunk of DV
-              ptx::tc_mma_f16_ts(tm + 256 + t * 128, tm + t * 128 + kk * 8, b + kk * 128, idesc_o,
-                                 (o_open[t] || kk != 0) ? 1u : 0u);
-            ptx::tc_commit(bar(O_FULL + t));
-          }
-          __syncwarp();
+          for (int kk = 0; kk < kTile / 16; ++kk)      // A: 16 keys = 8 TMEM columns; B: 16 key rows = 2048 B down every 64-wide chunk of DV
+            ptx::tc_mma_f16_ts_if(el, tm + 256 + t * 128, tm + t * 128 + kk * 8, b + kk * 128, idesc_o, kk != 0 ? 1u : keep);
+          if (j == last_tile(t)) ptx::tc_commit_if(el, bar(O_FULL + t));
           o_open[t] = true;
         };
-        auto open_kv = [&](uint32_t c) { wait(KV_FULL + (c & (kStages - 1)), (c / kStages) & 1u); return (int)(c & (kStages - 1)); };
-        auto free_kv = [&](int st) {
-          if (ptx::elect_one()) ptx::tc_commit(bar(KV_EMPTY + st));
-          __syncwarp();
+        auto peek_kv = [&](uint32_t c) { return ptx::mbar_try_wait(bar(KV_FULL + (c & (kStages - 1))), (c / kStages) & 1u); };
+        auto pass_kv = [&](uint32_t c, bool ready) {
+          if (!ready) wait(KV_FULL + (c & (kStages - 1)), (c / kStages) & 1u);
+          return c & (kStages - 1);
         };
-        int st = open_kv(kvc);
+        auto free_kv = [&](uint32_t st) { ptx::tc_commit_if(el, bar(KV_EMPTY + st)); };
+        uint32_t st = pass_kv(kvc, false);
 #pragma unroll
         for (int t = 0; t < 2; ++t)
           if (w.takes(t, w.tile(0))) issue_s(t, w.tile(0), st);
@@ -269,34 +279,39 @@ __global__ void __launch_bounds__(kFwdThreads, 1) attn_fwd_kernel(const __grid_c
         for (int k = 0; k < w.n; ++k) {
           const int j = w.tile(k), jn = w.tile(k + 1);
           const bool more = k + 1 < w.n;
-          const int sv = open_kv(kvc + 2 * k + 1);
-          int sk = -1;
+          const uint32_t sv = pass_kv(kvc + 2 * k + 1, peek_kv(kvc + 2 * k + 1));
+          const bool k_ready = more && peek_kv(kvc + 2 * k + 2);
+          uint32_t sk = kStages;
 #pragma unroll
           for (int t = 0; t < 2; ++t) {
-            if (w.takes(t, j)) issue_pv(t, sv);
-            if (t == 1) free_kv(sv);
+            if (w.takes(t, j)) issue_pv(t, j, sv);
             if (more) {
-              if (sk < 0) sk = open_kv(kvc + 2 * k + 2);
+              if (sk == kStages) sk = pass_kv(kvc + 2 * k + 2, k_ready);
               if (w.takes(t, jn)) issue_s(t, jn, sk);
             }
+            if (t == 1) free_kv(sv);
           }
           if (more) free_kv(sk);
         }
         kvc += 2 * w.n;
       }
+      __syncwarp();
     }
-  } else {
+  } else if (warp < 8) {
     ptx::reg_inc<kSoftmaxRegs>();
-    // ===================================================== softmax + output (4 warps per tile; thread = query row = TMEM lane)
+    // ===================================================== softmax (4 warps per tile; thread = query row = TMEM lane)
     const int t = warp >> 2, quad = warp & 3;
     const int row = quad * 32 + lane;
     const uint32_t lane_addr = tmem_base + ((uint32_t)(quad * 32) << 16);
-    const uint32_t tS = lane_addr + t * 128, tO = lane_addr + 256 + t * 128;
-    const uint32_t stage = sQ + C::kOut + warp * 4096;
+    const uint32_t tS = lane_addr + t * 128;
+    auto arrive = [&](int i) {
+      __syncwarp();
+      if (lane == 0) ptx::mbar_arrive(bar(i));
+    };
     const float cap_c = kMode == kCap ? 2.f * 1.4426950408889634f * p.scale / p.softcap : 0.f, cap_k = kMode == kCap ? p.softcap * 1.4426950408889634f : 0.f;
     const int win = (p.causal && p.window > 0) ? p.window : 0;
     const bool bounded = win > 0 || p.chunk > 0;
-    uint32_t sc = 0, vc = 0;      // S tiles / P V products of this tile so far
+    uint32_t sc = 0, n_l = 0;     // S tiles of this tile / items so far
     for (int n_it = 0;; ++n_it) {
       const int slot = n_it & 1;
       wait(IT_FULL + slot, (uint32_t)(n_it >> 1) & 1u);
@@ -306,7 +321,8 @@ __global__ void __launch_bounds__(kFwdThreads, 1) attn_fwd_kernel(const __grid_c
       if (it.L < 0 || *dead) break;
       const int qt = t ? it.qt1 : it.qt0;
       if (qt < 0) continue;
-      const int head = t ? it.head1 : it.head0, L = it.L, q0 = qt * kTile, q_pos = q0 + row;
+      const int L = it.L, q0 = qt * kTile, q_pos = q0 + row;
+      [[maybe_unused]] const int head = t ? it.head1 : it.head0;
       // scores live in the log2 domain: weight = exp2(s * c2 [+ distance term] - m_run)
       float c2 = p.scale * 1.4426950408889634f, slope2 = 0.f, m_run = -INFINITY, l_run = 0.f;
       if constexpr (kMode != kPlain) {
@@ -314,13 +330,13 @@ __global__ void __launch_bounds__(kFwdThreads, 1) attn_fwd_kernel(const __grid_c
         if (kMode == kGeneral && p.slope_base >= 0.f) slope2 = exp2f(-p.slope_base * (float)(head + 1) / (float)p.nq) * 1.4426950408889634f;
         if (p.sink) { m_run = rb::to_f(reinterpret_cast<const T*>(p.sink)[head]) * 1.4426950408889634f; l_run = 1.f; }
       }
-      const int row_lo = p.chunk > 0 ? q_pos / p.chunk * p.chunk : win > 0 ? q_pos - win + 1 : 0;                 // first visible key of the row
+      // first visible key of the row (used where masks are formed; chunks: formed there again would be a division)
+      const int row_lo = p.chunk > 0 ? q_pos / p.chunk * p.chunk : win > 0 ? q_pos - win + 1 : 0;
       const int last_lo = p.chunk > 0 ? (q0 + kTile - 1) / p.chunk * p.chunk : q0 + kTile - win;                  // of the tile's last row
       // this tile's key tiles, in the order of the item's walk
       const int first_tile = p.chunk > 0 ? (q0 / p.chunk * p.chunk) / kTile : win > 0 ? max(0, q0 - win + 1) / kTile : 0;
       const int n_keep = win > 0 ? min(RB_CEIL_DIV(p.keep, kTile), first_tile) : 0;
       const int n_tiles = n_keep + RB_CEIL_DIV(p.causal ? min(L, q0 + kTile) : L, kTile) - first_tile;
-      bool first = true;
 
       for (int k = 0; k < n_tiles; ++k) {
         const int kv0 = (k < n_keep ? k : first_tile + k - n_keep) * kTile;
@@ -337,7 +353,11 @@ __global__ void __launch_bounds__(kFwdThreads, 1) attn_fwd_kernel(const __grid_c
         if constexpr (kMode == kGeneral) {
           const float base = slope2 * (float)(kv0 - q_pos);
 #pragma unroll
-          for (int i = 0; i < 128; ++i) s[i] = fmaf(s[i], c2, fmaf(slope2, (float)i, base));
+          for (int i = 0; i < 128; i += 2) {
+            float b0 = (float)i, b1 = (float)(i + 1);
+            fma_pair(b0, b1, slope2, base);
+            fma_pair2(s[i], s[i + 1], c2, b0, b1);
+          }
         }
         if constexpr (kMode == kCap) {
 #pragma unroll
@@ -347,130 +367,180 @@ __global__ void __launch_bounds__(kFwdThreads, 1) attn_fwd_kernel(const __grid_c
         if ((kv0 + kTile > L) || (p.causal && kv0 + kTile - 1 > q0) || (bounded && last_lo > kv0)) {
           const int lim = (p.causal ? min(L, q_pos + 1) : L) - kv0;   // local key columns [lo, lim) are visible to this row
           const int lo = bounded ? row_lo - kv0 : 0;
-          if constexpr (kMode == kGeneral) {
-            const int kept = p.keep - kv0;                            // columns below `kept` stay visible under `lo`
+          const int kept = kMode == kGeneral ? p.keep - kv0 : 0;      // columns below `kept` stay visible under `lo`
 #pragma unroll
-            for (int i = 0; i < 128; ++i)
-              if (i >= lim || (i < lo && i >= kept)) s[i] = -INFINITY;
-          } else {
-            const uint32_t n_vis = (uint32_t)max(lim - lo, 0);
+          for (int c = 0; c < 4; ++c) {                               // bit i: column 32 c + i is visible
+            auto below = [&](int n) { n -= 32 * c; return n <= 0 ? 0u : n >= 32 ? 0xffffffffu : (1u << n) - 1u; };
+            const uint32_t vis = below(lim) & (~below(lo) | below(kept));
 #pragma unroll
-            for (int i = 0; i < 128; ++i)
-              if ((uint32_t)(i - lo) >= n_vis) s[i] = -INFINITY;
+            for (int i = 0; i < 32; ++i)
+              if ((vis & (1u << i)) == 0u) s[32 * c + i] = -INFINITY;
           }
         }
         float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
         for (int i = 0; i < 128; i += 8)
 #pragma unroll
-          for (int e = 0; e < 4; ++e) mx4[e] = fmaxf(mx4[e], fmaxf(s[i + 2 * e], s[i + 2 * e + 1]));
+          for (int e = 0; e < 4; ++e) mx4[e] = max3(mx4[e], s[i + 2 * e], s[i + 2 * e + 1]);
         float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
         if (kMode != kGeneral && kMode != kCap && mx != -INFINITY) mx *= c2;
-        float alpha = 1.f;
-        bool grown = false;                           // the same in the whole warp
-        if (first) {
-          const float m_new = fmaxf(m_run, mx);
-          if (m_new != -INFINITY) l_run *= exp2f(m_run - m_new);
-          m_run = m_new;
-        } else if (__any_sync(0xffffffffu, mx > m_run)) {
-          const float m_new = fmaxf(m_run, mx);
-          alpha = m_new == m_run ? 1.f : exp2f(m_run - m_new);
-          l_run *= alpha;
-          m_run = m_new;
-          grown = true;
+        const float m_new = fmaxf(m_run, mx);
+        const float alpha = m_new == m_run ? 1.f : exp2f(m_run - m_new);
+        l_run *= alpha;
+        m_run = m_new;
+        if (k > 0) {                                  // the output warps scale the row while its weights are formed
+          row_alpha[t * kTile + row] = alpha;
+          arrive(A_FULL + t * 4 + quad);
         }
-        first = false;
         const float neg_m = m_run == -INFINITY ? 0.f : -m_run;      // fully masked so far: keep exp2 arguments finite
         float sum4[4] = {0.f, 0.f, 0.f, 0.f};
-        uint32_t pw[64];
 #pragma unroll
-        for (int i = 0; i < 128; i += 2) {
-          float e0, e1;
-          if constexpr (kMode == kGeneral || kMode == kCap) {
-            e0 = exp2f(s[i] + neg_m);
-            e1 = exp2f(s[i + 1] + neg_m);
-          } else {
-            float x0 = s[i], x1 = s[i + 1];
-            fma_pair(x0, x1, c2, neg_m);
-            e0 = exp2f(x0);
-            e1 = exp2f(x1);
+        for (int c = 0; c < 4; ++c) {                 // 32 keys at a time: 16 columns of weights (registers: stored 32 at a time the scores spill)
+          uint32_t pw[16];
+#pragma unroll
+          for (int i = 0; i < 32; i += 2) {
+            float e0 = s[32 * c + i], e1 = s[32 * c + i + 1];
+            if constexpr (kMode == kGeneral || kMode == kCap) add_pair(e0, e1, neg_m, neg_m);
+            else fma_pair(e0, e1, c2, neg_m);
+            e0 = exp2f(e0);
+            e1 = exp2f(e1);
+            add_pair(sum4[i & 2], sum4[(i & 2) + 1], e0, e1);
+            pw[i >> 1] = pack2<T>(e0, e1);
           }
-          add_pair(sum4[i & 2], sum4[(i & 2) + 1], e0, e1);
-          pw[i >> 1] = pack2<T>(e0, e1);
-          if (i == 62) ptx::tc_st_32x32(tS, pw);
+          ptx::tc_st_32x16(tS + 16 * c, pw);
         }
-        ptx::tc_st_32x32(tS + 32, pw + 32);
         l_run += (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
-        if (grown) {                                  // the scores' registers are free: all of the output row is in flight at once
-          wait(O_FULL + t, (vc - 1) & 1u);            // the product in flight has retired, and the next one waits for this tile's P
-          ptx::tc_fence_after();
-          uint32_t o[kDV];
-#pragma unroll
-          for (int c = 0; c < kDV / 32; ++c) ptx::tc_ld_32x32(tO + c * 32, o + c * 32);
-          ptx::tc_wait_ld();
-#pragma unroll
-          for (int c = 0; c < kDV / 32; ++c) {
-#pragma unroll
-            for (int i = 0; i < 32; ++i) o[c * 32 + i] = __float_as_uint(__uint_as_float(o[c * 32 + i]) * alpha);
-            ptx::tc_st_32x32(tO + c * 32, o + c * 32);
-          }
-        }
         ptx::tc_wait_st();
         ptx::tc_fence_before();
-        __syncwarp();
-        if (lane == 0) ptx::mbar_arrive(bar(P_FULL + t));
-        ++vc;
+        arrive(P_FULL + t);
       }
-
-      // ---- output: O / l (times the gate), 64 columns at a time through the warp's staging rows
-      float inv = 1.f / l_run;
-      if constexpr (kMode != kPlain) {
-        if (p.gate && p.gate_mode == 1 && q_pos < L)
-          inv *= 1.f / (1.f + __expf(-rb::to_f(reinterpret_cast<const T*>(p.gate)[(int64_t)(it.tok0 + q_pos) * p.gate_ld + head])));
-      }
-      wait(O_FULL + t, (vc - 1) & 1u);
-      ptx::tc_fence_after();
+      wait(L_EMPTY + t, (n_l & 1u) ^ 1u);            // (items of one key tile: the output warps may be two behind)
+      ++n_l;
+      row_l[t * kTile + row] = l_run;
+      row_m[t * kTile + row] = m_run;
+      arrive(L_FULL + t);
+    }
+  } else {
+    ptx::reg_dec<kOutRegs>();
+    // ===================================================== output (warp = TMEM quadrant, thread = row of both tiles): O of a tile is scaled where a row's maximum has grown (its
+    // product in front of the scores that showed it has retired, and the next one waits for these warps too), and leaves when its last product has
+    const int quad = warp & 3, row = quad * 32 + lane;
+    const uint32_t lane_addr = tmem_base + ((uint32_t)(quad * 32) << 16);
+    const uint32_t stage = sQ + C::kOut + quad * 4096;
+    uint32_t a_par = 0, o_par = 0;                    // parities of A_FULL / O_FULL, a bit a tile
+    if (lane == 0) {                                  // O is free for a first product: said again when it has been read out
+      ptx::mbar_arrive(bar(P_FULL));
+      ptx::mbar_arrive(bar(P_FULL + 1));
+    }
+    for (int n_it = 0;; ++n_it) {
+      const int slot = n_it & 1;
+      wait(IT_FULL + slot, (uint32_t)(n_it >> 1) & 1u);
+      const Item it = items[slot];
+      __syncwarp();
+      if (lane == 0) ptx::mbar_arrive(bar(IT_EMPTY + slot));
+      if (it.L < 0 || *dead) break;
+      {
+        const Walk w(it, p);
+        uint32_t open = 0;
+#pragma unroll 1
+        for (int k = 0; k < w.n; ++k) {
+          const int j = w.tile(k);
+#pragma unroll 1
+          for (int t = 0; t < 2; ++t) {
+            if (!w.takes(t, j)) continue;
+            if ((open >> t & 1u) == 0u) {
+              open |= 1u << t;
+            } else {
+              wait(A_FULL + t * 4 + quad, a_par >> t & 1u);
+              a_par ^= 1u << t;
+              ptx::tc_fence_after();
+              const float alpha = row_alpha[t * kTile + row];
+              if (__any_sync(0xffffffffu, alpha != 1.f)) {
+#pragma unroll 1
+                for (uint32_t tO = lane_addr + 256 + t * 128, end = tO + kDV; tO != end; tO += 32) {
+                  uint32_t o[32];
+                  ptx::tc_ld_32x32(tO, o);
+                  ptx::tc_wait_ld();
 #pragma unroll
-      for (int half = 0; half < kDV / 64; ++half) {
-        uint32_t o[64];
-        ptx::tc_ld_32x32(tO + half * 64, o);
-        ptx::tc_ld_32x32(tO + half * 64 + 32, o + 32);
-        ptx::tc_wait_ld();
-        if (half == kDV / 64 - 1) {
-          ptx::tc_fence_before();
-          __syncwarp();
-          if (lane == 0) ptx::mbar_arrive(bar(O_EMPTY + t));
-        }
-        float of[64];
-#pragma unroll
-        for (int i = 0; i < 64; ++i) of[i] = __uint_as_float(o[i]);
-        if constexpr (kMode != kPlain) {
-          if (p.gate && p.gate_mode == 2 && q_pos < L) {          // (rows of the gate are 16-byte aligned: checked by the host)
-            const T* gr = reinterpret_cast<const T*>(p.gate) + (int64_t)(it.tok0 + q_pos) * p.gate_ld + (int64_t)head * kDV + half * 64;
-#pragma unroll
-            for (int i = 0; i < 64; i += 8) {
-              const rb::Pack<T, 8> gv = *reinterpret_cast<const rb::Pack<T, 8>*>(gr + i);
-#pragma unroll
-              for (int e = 0; e < 8; ++e) of[i + e] *= __fdividef(1.f, 1.f + __expf(-rb::to_f(gv.v[e])));
+                  for (int i = 0; i < 32; i += 2) {
+                    float x0 = __uint_as_float(o[i]), x1 = __uint_as_float(o[i + 1]);
+                    mul_pair(x0, x1, alpha, alpha);
+                    o[i] = __float_as_uint(x0);
+                    o[i + 1] = __float_as_uint(x1);
+                  }
+                  ptx::tc_st_32x32(tO, o);
+                }
+                ptx::tc_wait_st();
+                ptx::tc_fence_before();
+              }
+              __syncwarp();
+              if (lane == 0) ptx::mbar_arrive(bar(P_FULL + t));
             }
           }
         }
-#pragma unroll
-        for (int c = 0; c < 8; ++c)
-          st_shared_v4(stage + lane * 128 + ((c ^ (lane & 7)) << 4), pack2<T>(of[8 * c] * inv, of[8 * c + 1] * inv), pack2<T>(of[8 * c + 2] * inv, of[8 * c + 3] * inv),
-                       pack2<T>(of[8 * c + 4] * inv, of[8 * c + 5] * inv), pack2<T>(of[8 * c + 6] * inv, of[8 * c + 7] * inv));
-        __syncwarp();
-        T* dst = reinterpret_cast<T*>(p.out) + (int64_t)head * kDV + half * 64 + (lane & 7) * 8;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const int rr = i * 4 + (lane >> 3), pos = q0 + quad * 32 + rr;
-          const uint4 v = ld_shared_v4(stage + rr * 128 + (((lane & 7) ^ (rr & 7)) << 4));
-          if (pos < L) *reinterpret_cast<uint4*>(dst + (int64_t)(it.tok0 + pos) * p.out_ld) = v;
+      }
+      // ---- O / l (times the gate), 64 columns at a time through the warp's staging rows
+#pragma unroll 1
+      for (int t = 0; t < 2; ++t) {
+        const int qt = t ? it.qt1 : it.qt0, head = t ? it.head1 : it.head0;
+        if (qt < 0) continue;
+        const int q_pos = qt * kTile + row;
+        float inv = 1.f;
+        if constexpr (kMode != kPlain) {
+          if (p.gate && p.gate_mode == 1 && q_pos < it.L)
+            inv = 1.f / (1.f + __expf(-rb::to_f(reinterpret_cast<const T*>(p.gate)[(int64_t)(it.tok0 + q_pos) * p.gate_ld + head])));
+        }
+        wait(L_FULL + t, o_par >> t & 1u);
+        const float l_run = row_l[t * kTile + row];
+        inv *= 1.f / l_run;
+        if constexpr (kMode == kPlain) {
+          if (q_pos < it.L) p.lse[(int64_t)head * p.T + it.tok0 + q_pos] = row_m[t * kTile + row] * 0.6931471805599453f + __logf(l_run);
         }
         __syncwarp();
-      }
-      if constexpr (kMode == kPlain) {
-        if (q_pos < L) p.lse[(int64_t)head * p.T + it.tok0 + q_pos] = m_run * 0.6931471805599453f + __logf(l_run);
+        if (lane == 0) ptx::mbar_arrive(bar(L_EMPTY + t));
+        wait(O_FULL + t, o_par >> t & 1u);
+        o_par ^= 1u << t;
+        ptx::tc_fence_after();
+#pragma unroll 1
+        for (int half = 0; half < kDV / 64; ++half) {
+#pragma unroll 1
+          for (int c2 = 0; c2 < 2; ++c2) {
+            uint32_t o[32];
+            ptx::tc_ld_32x32(lane_addr + 256 + t * 128 + half * 64 + c2 * 32, o);
+            ptx::tc_wait_ld();
+            if constexpr (kMode != kPlain) {
+              if (p.gate && p.gate_mode == 2 && q_pos < it.L) {          // (rows of the gate are 16-byte aligned: checked by the host)
+                const T* gr = reinterpret_cast<const T*>(p.gate) + (int64_t)(it.tok0 + q_pos) * p.gate_ld + (int64_t)head * kDV + half * 64 + c2 * 32;
+#pragma unroll
+                for (int i = 0; i < 32; i += 8) {
+                  asm volatile("" ::: "memory");                      // one load after the other: registers
+                  const rb::Pack<T, 8> gv = *reinterpret_cast<const rb::Pack<T, 8>*>(gr + i);
+#pragma unroll
+                  for (int e = 0; e < 8; ++e)
+                    o[i + e] = __float_as_uint(__uint_as_float(o[i + e]) * __fdividef(1.f, 1.f + __expf(-rb::to_f(gv.v[e]))));
+                }
+              }
+            }
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+              uint32_t v[4];
+#pragma unroll
+              for (int e = 0; e < 4; ++e) v[e] = pack2<T>(__uint_as_float(o[8 * c + 2 * e]) * inv, __uint_as_float(o[8 * c + 2 * e + 1]) * inv);
+              st_shared_v4(stage + lane * 128 + (((c2 * 4 + c) ^ (lane & 7)) << 4), v[0], v[1], v[2], v[3]);
+            }
+          }
+          ptx::tc_fence_before();
+          __syncwarp();
+          if (half == kDV / 64 - 1 && lane == 0) ptx::mbar_arrive(bar(P_FULL + t));
+          T* dst = reinterpret_cast<T*>(p.out) + (int64_t)head * kDV + half * 64 + (lane & 7) * 8;
+#pragma unroll 4
+          for (int i = 0; i < 8; ++i) {
+            const int rr = i * 4 + (lane >> 3), pos = qt * kTile + quad * 32 + rr;
+            const uint4 v = ld_shared_v4(stage + rr * 128 + (((lane & 7) ^ (rr & 7)) << 4));
+            if (pos < it.L) *reinterpret_cast<uint4*>(dst + (int64_t)(it.tok0 + pos) * p.out_ld) = v;
+          }
+          __syncwarp();
+        }
       }
     }
   }

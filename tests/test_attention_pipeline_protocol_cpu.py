@@ -264,6 +264,7 @@ ITEM_BARS = {"IT_FULL0": 1, "IT_FULL1": 1, "IT_EMPTY0": 9, "IT_EMPTY1": 9, "CLC_
 
 
 # ------------------------------------------------------------------------------------------------ forward kernel (pairs of query tiles)
+# (with the output left to the softmax warps; test_attention_forward_protocol_cpu.py has the kernel with output warps of its own)
 STAGES = 4
 
 
