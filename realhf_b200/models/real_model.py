@@ -360,7 +360,7 @@ class ReaLModel(nn.Module):
             return OF.embed_sinusoid(input_ids, self.p["0.wte.weight"], position_ids, c.sinusoid_base, slots)
         x = TP.vocab_parallel_embedding(input_ids, self.p["0.wte.weight"], self.ctx, sp=self.sequence_parallel)
         if not c.apply_rotary and c.n_positions:
-            pe = F.embedding(position_ids.long() + c.abs_position_embedding_offset, self.p["0.wpe.weight"])
+            pe = OF.embedding(position_ids.long() + c.abs_position_embedding_offset, self.p["0.wpe.weight"])
             if self.sequence_parallel:
                 pe = TP._split_first_dim(pe, self.ctx)
             x = x + pe

@@ -303,6 +303,24 @@ void logprob_bwd_(Tensor logits, const Tensor& labels, const c10::optional<Tenso
   TORCH_CHECK(rc == 0);
 }
 
+extern "C" int rb_embedding_grad(const void* dy, const void* ids, int ids_64, void* dst, int* scratch, int64_t T, int64_t V, int64_t H, int g_dt, int d_dt,
+                                 cudaStream_t s);
+
+// dst [V, H] += the rows of dy [T, H] summed by id (ids outside [0, V) are passed over): the gradient of a table lookup, into a gradient buffer of dy's
+// type or fp32.
+void embedding_grad_(const Tensor& dy, const Tensor& ids, Tensor dst) {
+  CHECK_IN(dy); CHECK_IN(ids); CHECK_IN(dst);
+  TORCH_CHECK(dy.dim() == 2 && dst.dim() == 2 && ids.numel() == dy.size(0) && dy.size(1) == dst.size(1), "embedding_grad_: shapes");
+  TORCH_CHECK(ids.scalar_type() == at::kLong || ids.scalar_type() == at::kInt, "embedding_grad_: ids are int64 or int32");
+  TORCH_CHECK(dst.scalar_type() == dy.scalar_type() || dst.scalar_type() == at::kFloat, "embedding_grad_: buffer type");
+  c10::cuda::CUDAGuard guard(dy.device());
+  const int64_t T = dy.size(0), V = dst.size(0);
+  auto scratch = at::empty({2 * V + 1 + T / 32 + T}, dy.options().dtype(at::kInt));
+  const int rc = rb_embedding_grad(dy.data_ptr(), ids.data_ptr(), ids.scalar_type() == at::kLong, dst.data_ptr(), scratch.data_ptr<int>(), T, V, dy.size(1),
+                                   dt_code(dy), dt_code(dst), cur_stream());
+  TORCH_CHECK(rc == 0, "embedding_grad_: unsupported configuration (", rc, ")");
+}
+
 void register_gemm_ops(torch::Library& m);     // bindings_gemm.cpp
 void register_attn_ops(torch::Library& m);     // bindings_attn.cpp
 void register_comm_ops(torch::Library& m);
@@ -329,6 +347,7 @@ TORCH_LIBRARY(realhf_b200, m) {
   m.def("gated_act_bwd(Tensor gu, Tensor dout, int kind) -> Tensor", &gated_act_bwd);
   m.def("logprob_fwd(Tensor logits, Tensor labels, Tensor? mask, float inv_temp, int vocab_start, bool partials) -> Tensor[]", &logprob_fwd);
   m.def("logprob_bwd_(Tensor(a!) logits, Tensor labels, Tensor? mask, Tensor lse, Tensor dlogp, float inv_temp, int vocab_start) -> ()", &logprob_bwd_);
+  m.def("embedding_grad_(Tensor dy, Tensor ids, Tensor(a!) dst) -> ()", &embedding_grad_);
   register_gemm_ops(m);
   register_attn_ops(m);
   register_comm_ops(m);

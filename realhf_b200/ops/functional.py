@@ -814,6 +814,49 @@ def embed_sinusoid_ref(ids, wte, pos, inv_freq):
     return x
 
 
+class _Embedding(torch.autograd.Function):
+    """A table lookup whose gradient is added to the table's gradient buffer row by row (`csrc/embed_grad.cu`): no sort, no dense [V, H] beside the buffer."""
+
+    @staticmethod
+    def forward(ctx, ids, weight):
+        ctx.save_for_backward(ids)
+        ctx.weight = weight          # a leaf with a buffer; not saved, as a plain lookup does not need its values either
+        return F.embedding(ids, weight)
+
+    @staticmethod
+    def backward(ctx, dy):
+        (ids,), weight = ctx.saved_tensors, ctx.weight
+        if not ctx.needs_input_grad[1]:
+            return None, None
+        dy = dy.reshape(-1, weight.shape[1]).contiguous()
+        g = _row_grad_buffer(weight)
+        if g is None or (g.dtype != dy.dtype and g.dtype != torch.float32) or dy.data_ptr() % 16:
+            return None, torch.ops.aten.embedding_dense_backward(dy, ids.reshape(-1), weight.shape[0], -1, False)
+        lib().embedding_grad_(dy, ids.reshape(-1).contiguous(), g)
+        return None, None
+
+
+def _row_grad_buffer(weight):
+    """The gradient buffer of a [V, H] parameter that rows can be added to in place (`ReaLModel.attach_grad_buffer`), or None."""
+    g = getattr(weight, "main_grad", None)
+    if g is None and getattr(weight, "_grad_in_flat_buffer", False):
+        g = weight.grad
+    if g is None or g.dtype not in (torch.float32, torch.bfloat16, torch.float16) or g.numel() != weight.numel():
+        return None
+    g = g.view(weight.shape)
+    return g if g.is_contiguous() and weight.shape[1] % 8 == 0 and g.data_ptr() % 16 == 0 else None
+
+
+def embedding(ids, weight):
+    """weight[ids].  With a gradient asked for and a gradient buffer on the GPU the rows' gradients go straight into the buffer; elsewhere (and inside
+    function transforms and forward-mode differentiation, which the autograd function does not answer for) the plain lookup."""
+    if (use_native(weight) and weight.requires_grad and weight.is_leaf and weight.dim() == 2 and torch.is_grad_enabled() and ids.dtype in (torch.int64, torch.int32)
+            and not (torch.autograd.forward_ad._current_level >= 0 or torch._C._functorch.peek_interpreter_stack() is not None)
+            and _row_grad_buffer(weight) is not None):
+        return _Embedding.apply(ids, weight)
+    return F.embedding(ids, weight)
+
+
 def embed_sinusoid(ids, wte, pos, base: float = 10000.0, slots=None):
     """fp32 x [T, W] = wte[ids] + pe(p): pe[2i] = sin(p f_i), pe[2i + 1] = cos(p f_i), f_i = base^(-2i / W); positions and angles in
     fp32 with exact sinf / cosf.  p = pos[t], or pos[slots[t]] with `slots` (decode: `pos` is the per-slot length table)."""

@@ -234,11 +234,11 @@ def vocab_range(vocab_size: int, ctx: Optional[ParallelContext]) -> Tuple[int, i
 def vocab_parallel_embedding(ids, weight, ctx: Optional[ParallelContext], sp: bool = False):
     """weight is the local [V/t, H] shard. Out-of-shard ids contribute zeros, then reduce over TP."""
     if _tp(ctx) == 1:
-        return torch.nn.functional.embedding(ids, weight)
+        return OF.embedding(ids, weight)
     lo, hi = ctx.tp_rank * weight.shape[0], (ctx.tp_rank + 1) * weight.shape[0]
     mask = (ids < lo) | (ids >= hi)
     local = (ids - lo).masked_fill(mask, 0)
-    out = torch.nn.functional.embedding(local, weight)
+    out = OF.embedding(local, weight)
     out = out.masked_fill(mask.unsqueeze(-1), 0.0)
     return reduce_scatter_to_sp(out, ctx) if sp else reduce_from_tp(out, ctx)
 

@@ -349,3 +349,40 @@ def test_rmsnorm_bwd_row_rings(dtype, rows, H, with_dres):
     mag = r * (g.abs() + xh.abs() * (g * xh).abs().mean(-1, keepdim=True)) + (dres.double().abs() if with_dres else 0.0)
     assert ((dx.double() - rdx).abs() <= eps * rdx.abs() + 2.0 ** -20 * mag + 1e-7).all()
     assert ((dw.double() - rdw).abs() <= eps * rdw.abs() + 2.0 ** -20 * (dy.double() * xh).abs().sum(0) + 1e-7).all()
+
+
+@pytest.mark.parametrize("dtype,buffer", [(torch.bfloat16, torch.bfloat16), (torch.bfloat16, torch.float32), (torch.float16, torch.float16), (torch.float32, torch.float32)])
+@pytest.mark.parametrize("T,V,H", [(1, 3, 8), (33, 1, 64), (300, 7, 72), (1000, 50, 264), (5000, 4000, 2048), (2000, 2, 1032)])
+def test_embedding_gradient_goes_into_the_buffer(T, V, H, dtype, buffer):
+    """Against the sums in float64: an fp32 sum of c rows errs by at most c ulps of the sum of their magnitudes, and the result is rounded once to the buffer's type.
+    Chains of one token, of up to 32, and longer ones; ids that do not occur; the same every time."""
+    from realhf_b200.ops import functional as OF
+    g = torch.Generator(device="cuda").manual_seed(T + H)
+    ids = torch.randint(0, V, (T,), device="cuda", generator=g)
+    ids[: T // 3] = V // 2
+    if V > 4:
+        ids[ids == V - 1] = 0
+    w = torch.nn.Parameter(torch.randn(V, H, device="cuda", generator=g).to(dtype))
+    dy = torch.randn(T, H, device="cuda", generator=g).to(dtype)
+    start = torch.randn(V, H, device="cuda", generator=g).to(buffer)
+    got = []
+    for _ in range(2):
+        buf = start.clone()
+        if buffer == dtype:
+            w.grad, w._grad_in_flat_buffer = buf, True
+        else:
+            w.main_grad = buf
+        y = OF.embedding(ids.view(1, -1), w)
+        assert torch.equal(y[0], w.detach()[ids])
+        y.backward(dy.view(1, T, H))
+        got.append(buf)
+    assert torch.equal(got[0], got[1])
+    want = start.double().index_add(0, ids, dy.double())
+    size = start.double().abs().index_add(0, ids, dy.double().abs())
+    n = torch.bincount(ids, minlength=V).max().item() + 1
+    bound = size * n * 2.0 ** -24 + want.abs() * torch.finfo(buffer).eps / 2 * 1.01 + 1e-12
+    if buffer == torch.float16:
+        bound = bound + 2.0 ** -25
+    assert ((got[0].double() - want).abs() <= bound).all()
+    if V > 4:
+        assert torch.equal(got[0][V - 1], start[V - 1])
