@@ -306,6 +306,22 @@ void logprob_bwd_(Tensor logits, const Tensor& labels, const c10::optional<Tenso
 extern "C" int rb_embedding_grad(const void* dy, const void* ids, int ids_64, void* dst, int* scratch, int64_t T, int64_t V, int64_t H, int g_dt, int d_dt,
                                  cudaStream_t s);
 
+extern "C" int rb_embedding_rows(const void* table, const void* ids, int ids_64, void* out, int64_t T, int64_t V, int64_t row_bytes, cudaStream_t s);
+
+// table[ids] for a packed table whose rows are whole 16-byte pieces.
+Tensor embedding_rows(const Tensor& table, const Tensor& ids) {
+  CHECK_IN(table); CHECK_IN(ids);
+  TORCH_CHECK(table.dim() == 2 && (ids.scalar_type() == at::kLong || ids.scalar_type() == at::kInt), "embedding_rows: a table and integer ids");
+  c10::cuda::CUDAGuard guard(table.device());
+  auto sizes = ids.sizes().vec();
+  sizes.push_back(table.size(1));
+  auto out = at::empty(sizes, table.options());
+  const int rc = rb_embedding_rows(table.data_ptr(), ids.data_ptr(), ids.scalar_type() == at::kLong, out.data_ptr(), ids.numel(), table.size(0),
+                                   table.size(1) * table.element_size(), cur_stream());
+  TORCH_CHECK(rc == 0, "embedding_rows: unsupported configuration (", rc, ")");
+  return out;
+}
+
 // dst [V, H] += the rows of dy [T, H] summed by id (ids outside [0, V) are passed over): the gradient of a table lookup, into a gradient buffer of dy's
 // type or fp32.
 void embedding_grad_(const Tensor& dy, const Tensor& ids, Tensor dst) {
@@ -347,6 +363,7 @@ TORCH_LIBRARY(realhf_b200, m) {
   m.def("gated_act_bwd(Tensor gu, Tensor dout, int kind) -> Tensor", &gated_act_bwd);
   m.def("logprob_fwd(Tensor logits, Tensor labels, Tensor? mask, float inv_temp, int vocab_start, bool partials) -> Tensor[]", &logprob_fwd);
   m.def("logprob_bwd_(Tensor(a!) logits, Tensor labels, Tensor? mask, Tensor lse, Tensor dlogp, float inv_temp, int vocab_start) -> ()", &logprob_bwd_);
+  m.def("embedding_rows(Tensor table, Tensor ids) -> Tensor", &embedding_rows);
   m.def("embedding_grad_(Tensor dy, Tensor ids, Tensor(a!) dst) -> ()", &embedding_grad_);
   register_gemm_ops(m);
   register_attn_ops(m);

@@ -821,7 +821,7 @@ class _Embedding(torch.autograd.Function):
     def forward(ctx, ids, weight):
         ctx.save_for_backward(ids)
         ctx.weight = weight          # a leaf with a buffer; not saved, as a plain lookup does not need its values either
-        return F.embedding(ids, weight)
+        return _rows(ids, weight)
 
     @staticmethod
     def backward(ctx, dy):
@@ -847,13 +847,23 @@ def _row_grad_buffer(weight):
     return g if g.is_contiguous() and weight.shape[1] % 8 == 0 and g.data_ptr() % 16 == 0 else None
 
 
+def _rows(ids, weight):
+    if (weight.dim() == 2 and weight.is_contiguous() and weight.shape[1] * weight.element_size() % 16 == 0 and weight.data_ptr() % 16 == 0
+            and ids.device == weight.device):
+        return lib().embedding_rows(weight, ids.contiguous())
+    return F.embedding(ids, weight)
+
+
 def embedding(ids, weight):
-    """weight[ids].  With a gradient asked for and a gradient buffer on the GPU the rows' gradients go straight into the buffer; elsewhere (and inside
-    function transforms and forward-mode differentiation, which the autograd function does not answer for) the plain lookup."""
-    if (use_native(weight) and weight.requires_grad and weight.is_leaf and weight.dim() == 2 and torch.is_grad_enabled() and ids.dtype in (torch.int64, torch.int32)
-            and not (torch.autograd.forward_ad._current_level >= 0 or torch._C._functorch.peek_interpreter_stack() is not None)
-            and _row_grad_buffer(weight) is not None):
-        return _Embedding.apply(ids, weight)
+    """weight[ids].  With a gradient asked for and a gradient buffer on the GPU the rows' gradients go straight into the buffer; without a gradient the lookup is
+    a kernel of its own; elsewhere (and inside function transforms and forward-mode differentiation, which the autograd function does not answer for) the
+    plain lookup."""
+    if (use_native(weight) and ids.dtype in (torch.int64, torch.int32)
+            and not (torch.autograd.forward_ad._current_level >= 0 or torch._C._functorch.peek_interpreter_stack() is not None)):
+        if not (weight.requires_grad and torch.is_grad_enabled()):
+            return _rows(ids, weight)
+        if weight.is_leaf and weight.dim() == 2 and _row_grad_buffer(weight) is not None:
+            return _Embedding.apply(ids, weight)
     return F.embedding(ids, weight)
 
 

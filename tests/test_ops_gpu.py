@@ -386,3 +386,18 @@ def test_embedding_gradient_goes_into_the_buffer(T, V, H, dtype, buffer):
     assert ((got[0].double() - want).abs() <= bound).all()
     if V > 4:
         assert torch.equal(got[0][V - 1], start[V - 1])
+
+
+@pytest.mark.parametrize("dtype,ids_dtype", [(torch.bfloat16, torch.int64), (torch.float16, torch.int32), (torch.float32, torch.int64)])
+@pytest.mark.parametrize("shape,V,H", [((1,), 1, 8), ((16,), 50, 4096), ((3, 5), 7, 1032), ((0,), 3, 64), ((700,), 300, 72), ((300,), 64, 4104), ((9,), 5, 12)])
+def test_embedding_rows_are_copied(shape, V, H, dtype, ids_dtype):
+    """A lookup without a gradient: few and many rows, rows that end within a block's share of pieces and that are no whole 16-byte pieces, ids in any shape and stride."""
+    from realhf_b200.ops import functional as OF
+    g = torch.Generator(device="cuda").manual_seed(V + H)
+    w = torch.randn(V, H, device="cuda", generator=g).to(dtype)
+    ids = torch.randint(0, V, shape, device="cuda", generator=g).to(ids_dtype)
+    for i in (ids, ids.flip(0).transpose(0, -1), ids[..., ::2]):
+        got = OF.embedding(i, w)
+        assert got.dtype == dtype and torch.equal(got, w[i.long()])
+    with torch.no_grad():
+        assert torch.equal(OF.embedding(ids, torch.nn.Parameter(w)), w[ids.long()])
