@@ -13,6 +13,8 @@
 // smem full/empty ring (TMA <-> MMA), TMEM full/empty double buffer (MMA <-> epilogue), and a static
 // persistent tile loop (one CTA per SM).  The epilogue stages 32 rows in shared memory and stores whole
 // lines, with optional bias and accumulate-into-C.
+#include <atomic>
+
 #include "gemm_common.cuh"
 
 namespace {
@@ -279,6 +281,11 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tcgen05_kernel(const __grid_
 // ever waits on tiles at or before its own, so with all CTAs resident (grid <= #SMs, 1 CTA/SM) the scheme cannot
 // deadlock.  The last reader re-arms the tile counters, so no per-call memset is needed and CUDA graphs can replay it.  A is loaded with a box of only round_up(M, 8) rows; the remaining rows
 // of the 128-row UMMA tile hold stale shared memory and only ever influence accumulator rows that are never stored.
+//
+// Where a tile is cut into 2 or 4 parts of K (kCluster), its CTAs are a cluster and the partials never leave the chip: each CTA leaves
+// its accumulator in its own shared memory (the ring is empty by then), and behind one cluster barrier sums 1/S of the tile's columns out of the S CTAs'
+// shared memory, in the same order.  Through the workspace a part waits for its stores, the counter, the last CTA and a round trip to L2 (figures at the choice of
+// the layout below).
 struct StreamKParams {
   float* ws;         // [2 * gridDim.x][BM][BN] fp32 partials: slot 2g for CTA g's first segment, 2g+1 for its last
   uint32_t* flags;   // [2 * tiles_n]: (arrived, done) per tile, zero at entry and exit
@@ -289,6 +296,7 @@ struct StreamKParams {
   // scale); nullptr for 16-bit operands
   const float* scale_a;
   const float* scale_b;
+  int parts;         // kCluster: CTAs of a tile
 };
 
 RB_DEVICE uint32_t ld_acquire_gpu(const uint32_t* p) {
@@ -301,7 +309,7 @@ RB_DEVICE void epi_bar_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 
 // kFmt: 0 fp16, 1 bf16, 2 fp8 e4m3 (W8A8 generation path: same byte geometry -- a k-block is one 128-byte swizzle row, i.e.
 // 128 fp8 elements instead of 64 bf16 -- `tcgen05.mma.kind::f8f6f4`, per-row x per-column scales in the epilogue)
-template <typename OutT, int kFmt>
+template <typename OutT, int kFmt, bool kCluster>
 __global__ void __launch_bounds__(kThreads, 1) gemm_streamk_kernel(const __grid_constant__ CUtensorMap tma_a,
                                                                    const __grid_constant__ CUtensorMap tma_b, Params p,
                                                                    StreamKParams sk) {
@@ -325,7 +333,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_streamk_kernel(const __grid_
   uint64_t* tmem_empty = tmem_full + 2;
   uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(tmem_empty + 2);
 
-  __shared__ int slot_of[160];
+  __shared__ int slot_of[kCluster ? 1 : 160];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   constexpr int KBE = kFmt == 2 ? 2 * BK : BK;  // elements per k-block (128 bytes either way)
   const int num_kb = RB_CEIL_DIV(p.K, KBE);
@@ -429,6 +437,28 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_streamk_kernel(const __grid_
     const int row = quad * 32 + lane;
     const bool row_ok = row < p.M;
     const int et = threadIdx.x - 64;  // 0..127 over the epilogue warps
+    if constexpr (kCluster) {          // the CTA's part of its tile -> its shared memory, [column / 4][row] in float4 units
+      if (u_begin < u_end) {
+        ptx::mbar_wait(ptx::smem_u32(&tmem_full[0]), 0);
+        ptx::tc_fence_after();
+        const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16);
+        float4* part = reinterpret_cast<float4*>(smem);
+#pragma unroll 1
+        for (int c = 0; c < (BN + 31) / 32; ++c) {
+          uint32_t r[32];
+          ptx::tc_ld_32x32(taddr + c * 32, r);
+          ptx::tc_wait_ld();
+          const int n4 = min(8, BN / 4 - c * 8);
+          if (row_ok) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+              if (i < n4)
+                part[(c * 8 + i) * sk.a_box_rows + row] = make_float4(__uint_as_float(r[4 * i]), __uint_as_float(r[4 * i + 1]), __uint_as_float(r[4 * i + 2]),
+                                                                      __uint_as_float(r[4 * i + 3]));
+          }
+        }
+      }
+    } else {
     rb::pdl_wait();  // output buffer, bias and the stream-K workspace may still be in use by the predecessor
     int as = 0;
     uint32_t aphase = 0;
@@ -577,8 +607,53 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_streamk_kernel(const __grid_
         if (old == (uint32_t)S - 1u) { arrived[1] = 0u; __threadfence(); arrived[0] = 0u; }  // last reader re-arms the tile
       }
     }
+    }
   }
 
+  if constexpr (kCluster) {
+    __syncwarp();
+    ptx::cluster_sync();               // every part of the tile is in its CTA's shared memory
+    if (warp >= 2) {
+      rb::pdl_wait();                  // the output may still be in use by the predecessor
+      const int S = sk.parts, j = g % S, n0 = g / S * BN, kC4 = BN / 4, c_lo = kC4 * j / S, c_hi = kC4 * (j + 1) / S;
+      const int n_rb = RB_CEIL_DIV(p.M, 8), n_blocks = n_rb * RB_CEIL_DIV(c_hi - c_lo, 4);
+      OutT* Cp = reinterpret_cast<OutT*>(p.C);
+      const OutT* bias = reinterpret_cast<const OutT*>(p.bias);
+      const bool vec4 = (p.ldc % 4 == 0) && ((reinterpret_cast<uintptr_t>(p.C) & 7) == 0);
+      for (int blk = warp - 2; blk < n_blocks; blk += 4) {       // a warp takes 8 rows x 4 float4 columns, as the fix-up above
+        const int rr = (blk % n_rb) * 8 + (lane & 7), c4 = c_lo + (blk / n_rb) * 4 + (lane >> 3), col = n0 + c4 * 4;
+        if (rr >= p.M || c4 >= c_hi || col >= p.N) continue;
+        const uint32_t at = ptx::smem_u32(smem) + (uint32_t)(c4 * sk.a_box_rows + rr) * 16u;
+        float4 t[4];
+#pragma unroll
+        for (int m = 0; m < 4; ++m)
+          if (m < S) t[m] = ptx::ld_cluster_f4(at, (uint32_t)m);
+        float v[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int m = 0; m < 4; ++m)
+          if (m < S) { v[0] += t[m].x; v[1] += t[m].y; v[2] += t[m].z; v[3] += t[m].w; }
+        const int nv = min(4, p.N - col);
+        if constexpr (kFmt == 2) {
+          const float sa = sk.scale_a[rr];
+          for (int i = 0; i < nv; ++i) v[i] *= sa * sk.scale_b[col + i];
+        }
+        if (bias != nullptr) {
+          for (int i = 0; i < nv; ++i) v[i] += rb::to_f(bias[col + i]);
+        }
+        OutT* dst = Cp + (int64_t)rr * p.ldc + col;
+        if (nv == 4 && vec4) {
+          rb::Pack<OutT, 4> pk;
+#pragma unroll
+          for (int i = 0; i < 4; ++i) pk.v[i] = rb::from_f<OutT>(v[i]);
+          *reinterpret_cast<rb::Pack<OutT, 4>*>(dst) = pk;
+        } else {
+          for (int i = 0; i < nv; ++i) dst[i] = rb::from_f<OutT>(v[i]);
+        }
+      }
+    }
+    __syncwarp();
+    ptx::cluster_sync();               // nobody leaves while its shared memory is read
+  }
   ptx::tc_fence_before();
   __syncthreads();
   if (warp == 1) {
@@ -608,17 +683,41 @@ int launch(const CUtensorMap& ta, const CUtensorMap& tb, const Params& p, int nu
 }
 
 
+constexpr int kStreamkSmem = 227 * 1024 - 1024;
+
+template <typename OutT, int kFmt, bool kCluster> int configure_streamk() {
+  static std::atomic<uint64_t> opted_in{0};          // the attribute is the kernel's on one device: a bit per device
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return -2;
+  if (dev >= 64 || !(opted_in.load(std::memory_order_relaxed) >> dev & 1)) {
+    if (cudaFuncSetAttribute(gemm_streamk_kernel<OutT, kFmt, kCluster>, cudaFuncAttributeMaxDynamicSharedMemorySize, kStreamkSmem) != cudaSuccess) return -2;
+    if (dev < 64) opted_in.fetch_or(uint64_t(1) << dev, std::memory_order_relaxed);
+  }
+  return 0;
+}
+
 template <typename OutT, int kFmt>
 int launch_streamk(const CUtensorMap& ta, const CUtensorMap& tb, const Params& p, const StreamKParams& sk, int grid, cudaStream_t s) {
-  auto kern = gemm_streamk_kernel<OutT, kFmt>;
-  constexpr int kMaxSmem = 227 * 1024 - 1024;
-  static bool configured = false;
-  if (!configured) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem) != cudaSuccess) return -2;
-    configured = true;
-  }
   const int smem = sk.stages * (sk.a_box_rows * 128 + sk.bn * BK * 2) + 1024 + 512;
-  if (rb::launch_pdl(kern, dim3(grid), dim3(kThreads), (size_t)smem, s, ta, tb, p, sk) != cudaSuccess) return -3;
+  if (sk.parts > 1) {
+    if (configure_streamk<OutT, kFmt, true>() != 0) return -2;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = sk.parts;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = rb::pdl_enabled() ? 2 : 1;
+    return cudaLaunchKernelEx(&cfg, gemm_streamk_kernel<OutT, kFmt, true>, ta, tb, p, sk) == cudaSuccess ? 0 : -3;
+  }
+  if (configure_streamk<OutT, kFmt, false>() != 0) return -2;
+  if (rb::launch_pdl(gemm_streamk_kernel<OutT, kFmt, false>, dim3(grid), dim3(kThreads), (size_t)smem, s, ta, tb, p, sk) != cudaSuccess) return -3;
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 
@@ -703,7 +802,7 @@ int rb_gemm_tcgen05(const void* A, const void* B, void* C, const void* bias, int
 // Small-M GEMM (decode shapes): M <= 128, K-major operands, no accumulate.  `ws` holds 2 * num_sms * 128 * 256 floats,
 // `flags` 8192 zero-initialised words (persistent per device; calls sharing them must be stream-ordered).
 // bn = 0 / split = 0: pick the tile width (multiple of 16) and the K split from a byte-ingest cost model:
-//   t = max(weight bytes / HBM, bytes per CTA / ~70 GB/s per-SM TMA ingest) + fix-up(split > 1),
+//   t = max(weight bytes / HBM, bytes per CTA / ~85 GB/s per-SM TMA ingest) + fix-up(split > 1),
 // over the layouts with tiles_n * split <= #SMs (tile-aligned split: one fix-up round per CTA).
 // in_dt: 1 bf16, 2 fp16, 3 fp8 e4m3 (then scale_a [M] / scale_b [N] fp32 are required; lda / ldb count bytes = elements)
 static int streamk_impl(const void* A, const void* B, void* C, const void* bias, int M, int N, int K, int64_t lda, int64_t ldb,
@@ -719,6 +818,7 @@ static int streamk_impl(const void* A, const void* B, void* C, const void* bias,
   const int kbe = 128 / esz;  // elements per 128-byte k-block
   const int num_kb = RB_CEIL_DIV(K, kbe);
   const int box_rows = ((M + 7) / 8) * 8;
+  int parts = 1;
   if (bn == 0) {
     double best = 1e30;
     for (int cand = 32; cand <= 256; cand += 16) {
@@ -729,15 +829,21 @@ static int streamk_impl(const void* A, const void* B, void* C, const void* bias,
       for (int sp = 1; sp <= smax; ++sp) {
         const double waves = (double)RB_CEIL_DIV(tiles * sp, num_sms);
         const double cta_bytes = (double)(box_rows + cand) * 128.0 * RB_CEIL_DIV(num_kb, sp) * waves;
-        double t = cta_bytes / 70e3;                              // us
+        double t = cta_bytes / 85e3;                              // us
         const double hbm = (double)N * K * esz / 6.5e6;           // us
         if (t < hbm) t = hbm;
-        // per-k-block term: 0.2 .. 0.25 measured; with 0.33 the layouts picked are within 3 % of the best of a sweep over widths and splits
-        // (16 and 64 rows), but for 4096 x 4096 at 16 rows: 12.6 against 11.4 us
-        const double kb_floor = 0.33 * RB_CEIL_DIV(num_kb, sp) * waves;
+        // per-k-block term: 0.2 .. 0.25 measured; with 0.33 (whole tiles: 0.30) the layouts picked are within 3 % of the best of a sweep over widths and splits
+        const double kb_floor = (sp > 1 ? 0.33 : 0.30) * RB_CEIL_DIV(num_kb, sp) * waves;
         if (t < kb_floor) t = kb_floor;
-        if (sp > 1) t += 5.0 + 4.5 * (double)M * cand * 4.0 / 60e3;  // partial write + barrier + cooperative reduce (measured)
-        if (t < best) { best = t; bn = cand; split = sp; }
+        // The parts of a tile in a cluster of 2 or 4: what the merge takes is nearly constant.  Cold weights at 16, 64 and 128 rows, through the workspace / so:
+        // 4096 x 4096 12.4 / 9.8, 12.3 / 10.5, 14.2 / 11.7 us; 4096 x 11008 20.3 / 17.6, 21.8 / 19.2, 25.5 / 21.4; 2048 x 2048 7.7 / 6.1, 8.2 / 6.7, 9.0 / 7.4;
+        // 6144 x 4096 13.9 / 11.7, 15.4 / 13.4, 18.1 / 15.6; 768 x 3072 8.7 / 5.7, 8.1 / 6.6, 7.2 / 7.4 us.
+        // Of 4 as long as all are there at once (32 of 37 SMs; 148 CTAs take two rounds: 15.0 us for the first); clusters of 8 wait for 8 free SMs of one GPC
+        // (16.1).  Taken when it is clearly ahead: 12288 x 4096 in two parts takes 19.4 / 22.5 / 27.0, whole 19.1 / 20.7 / 22.8.
+        const double in_cluster = t + 3.3 + 0.2e-3 * M * cand;
+        if ((sp == 2 || (sp == 4 && tiles * 4 <= num_sms * 32 / 37)) && in_cluster < 0.96 * best) { best = in_cluster / 0.96; bn = cand; split = parts = sp; }
+        if (sp > 1) t += 5.0 + 0.12 * sp + 4.5 * (double)M * cand * 4.0 / 60e3;  // partial write + barrier + cooperative reduce of sp parts (measured)
+        if (t < best) { best = t; bn = cand; split = sp; parts = 1; }
       }
     }
   }
@@ -770,7 +876,7 @@ static int streamk_impl(const void* A, const void* B, void* C, const void* bias,
   if (!ok) return -13;
   Params p{C, bias, ldc, M, N, K, 0};
   StreamKParams sk{reinterpret_cast<float*>(ws), reinterpret_cast<uint32_t*>(flags), box_rows, bn, stages,
-                   reinterpret_cast<long long*>(dbg), scale_a, scale_b};
+                   reinterpret_cast<long long*>(dbg), scale_a, scale_b, parts};
   if (in_dt == 3) {
     if (out_dt == 1) return launch_streamk<__nv_bfloat16, 2>(ta, tb, p, sk, grid, s);
     if (out_dt == 0) return launch_streamk<float, 2>(ta, tb, p, sk, grid, s);

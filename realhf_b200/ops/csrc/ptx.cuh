@@ -115,6 +115,13 @@ __device__ __forceinline__ void tc_mma_f8(uint32_t tmem_d, uint64_t adesc, uint6
 __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// four floats at the same shared-memory address in CTA `cta` of the cluster
+__device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr, uint32_t cta) {
+  float4 v;
+  asm volatile("{\n\t.reg .b32 r;\n\tmapa.shared::cluster.u32 r, %4, %5;\n\tld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [r];\n\t}"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr), "r"(cta) : "memory");
+  return v;
+}
 __device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 // 32 lanes x 32 consecutive fp32 columns: thread i of the warp receives row (lane_base + i)
 __device__ __forceinline__ void tc_ld_32x32(uint32_t taddr, uint32_t* r) {

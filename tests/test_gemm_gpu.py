@@ -279,6 +279,23 @@ def test_grouped_wgrad_tail_rows_of_other_groups():
     assert torch.equal(G.grouped_wgrad(dy[:0], x[:0], torch.zeros(3, dtype=torch.int32, device="cuda"), 2), torch.zeros(2, M, N, device="cuda", dtype=torch.bfloat16))
 
 
+@pytest.mark.parametrize("M,N,K", [(1, 4096, 4096), (7, 2040, 2048), (16, 6144, 4096), (33, 4104, 4168), (64, 8184, 2048), (128, 4096, 11008), (128, 2040, 136)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_small_products_with_parts_of_k(M, N, K, dtype):
+    """Few rows, narrow outputs: K cut into parts that are merged in a cluster or through the workspace; ragged rows, columns and parts.  Products of 16-bit numbers are
+    exact in fp32: 2^-20 of the summed magnitudes for the sums, 2^-8 (bf16; fp16 2^-11) of the value for a rounded result; the same every time."""
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    a, b = (torch.randn(n, K, device="cuda", generator=g).to(dtype) for n in (M, N))
+    bias = torch.randn(N, device="cuda", generator=g).to(dtype)
+    ref, mag = a.double() @ b.double().T, a.double().abs() @ b.double().abs().T
+    y = G.gemm_streamk(a, b, out_dtype=torch.float32)
+    assert ((y.double() - ref).abs() <= 2.0 ** -20 * mag).all()
+    assert all(torch.equal(G.gemm_streamk(a, b, out_dtype=torch.float32), y) for _ in range(3))
+    z = G.gemm_streamk(a, b, bias=bias)
+    want = ref + bias.double()
+    assert ((z.double() - want).abs() <= 2.0 ** -20 * mag + want.abs() * (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11)).all()
+
+
 @pytest.mark.parametrize("out_dt", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("M,N,K,shift", [(129, 136, 64, 0), (300, 520, 192, 0), (257, 264, 128, 1), (8, 72, 200, 0), (640, 40, 72, 3)])
 def test_gemm_accumulates_into_ragged_outputs(out_dt, M, N, K, shift):
