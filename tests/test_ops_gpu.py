@@ -401,3 +401,23 @@ def test_embedding_rows_are_copied(shape, V, H, dtype, ids_dtype):
         assert got.dtype == dtype and torch.equal(got, w[i.long()])
     with torch.no_grad():
         assert torch.equal(OF.embedding(ids, torch.nn.Parameter(w)), w[ids.long()])
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("rows,H", [(1, 8), (1, 4096), (3, 264), (16, 8192), (148, 4104), (296, 1000), (297, 1000)])
+def test_rms_norm_of_few_rows(rows, H, dtype):
+    """A piece a thread up to two rows an SM, several beyond.  The sum of squares takes at most 8 + 5 + 5 roundings on a path, the square root and the products a few:
+    2^-19 of the value, and half an ulp of the type for the result; the residual sum is rounded once."""
+    from realhf_b200.ops import lib
+    g = torch.Generator(device="cuda").manual_seed(rows + H)
+    x, r, w = (torch.randn(n, device="cuda", generator=g).to(dtype) for n in ((rows, H), (rows, H), (H,)))
+    for res, off in ((None, 0.0), (r, 1.0)):
+        out = lib().rmsnorm_fwd(x, res, w, 1e-5, off)
+        h = x if res is None else (x.float() + res.float()).to(dtype)
+        if res is not None:
+            assert torch.equal(out[2], h)
+        rstd = (h.double().square().mean(-1) + 1e-5).rsqrt()
+        want = h.double() * rstd[:, None] * (w.double() + off)
+        bound = want.abs() * (2.0 ** -19 + torch.finfo(dtype).eps / 2) + (2.0 ** -24 if dtype == torch.float16 else 0)
+        assert ((out[0].double() - want).abs() <= bound).all()
+        assert ((out[1].double().flatten() - rstd).abs() <= rstd * 2.0 ** -19).all()
