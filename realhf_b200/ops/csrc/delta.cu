@@ -19,6 +19,8 @@
 //                    of one (sequence, head).  q, k, v, beta, g of 8 tokens at a time are staged in shared memory.  Packed form: S starts
 //                    at zero and the final S goes to s_state[slot]; step form: S is loaded from and stored to s_state[slot].
 //   gated_head_norm  o / sqrt(mean(o^2) + eps) * w * silu(gate) or sigmoid(gate) per (token, head) -> model type.
+#include <type_traits>
+
 #include "anytype.cuh"
 
 namespace {
@@ -233,13 +235,13 @@ __global__ void __launch_bounds__(kPThreads) delta_prepare_tiled_kernel(const vo
 // The same for head sizes in whole fours up to 128 on aligned rows: a warp owns one unit of channels, four neighbouring ones a lane, and walks kWalk
 // tokens in tiles of 8 whose rows it has in flight together; the per-(token, head) sum of squares stays inside the warp.  The kernel above moves two
 // bytes a lane and load and four a store, and waits for its loads with few of them on their way: 8 sequences of 700 .. 1024 tokens, 16 + 2 x 4 heads x 128
-// (71 MB in, 85 MB out) 121 us; this way 87.  What it waits for is its loads: the tiles take 124 registers, so 14 warps an SM are resident, half of their stalls
-// are on a load, and the issue slots are busy 38 % of the time with 46 instructions a channel and token (24 us of bytes, about 20 of issue).  kTaps: the taps
-// that registers are kept for.
+// (71 MB in, 85 MB out) 121 us; this way 49.  What it waits for is its loads and the issue of some 45 instructions a channel and token (24 us of bytes, about 20
+// of issue), so rows on their way stay as they are in memory: 96 registers and five CTAs an SM for 16-bit rows (widened on arrival, the type told apart at
+// run time, 124 registers: 87 us; four CTAs 57, six, with spills, 53; bf16 widened by the pair conversions instead of shifts 59).  kTaps: the taps that registers are kept for.
 constexpr int kTile = 8;
 
-template <int kTaps, int kWalk>
-__global__ void __launch_bounds__(kPThreads) delta_prepare_warp_kernel(const void* __restrict__ proj, int64_t ld, int dt, const void* __restrict__ conv_w,
+template <typename T4, int kTaps, int kWalk>
+__global__ void __launch_bounds__(kPThreads, kTaps > 4 ? 3 : (sizeof(T4) == 2 ? 5 : 4)) delta_prepare_warp_kernel(const void* __restrict__ proj, int64_t ld, int dt, const void* __restrict__ conv_w,
                                                                        GateParams gp, float* __restrict__ u, const int* __restrict__ pos,
                                                                        float* __restrict__ conv_state, const int* __restrict__ tok_slot,
                                                                        const int* __restrict__ remain, int64_t T, int H, int G, int d, int dv,
@@ -258,11 +260,21 @@ __global__ void __launch_bounds__(kPThreads) delta_prepare_warp_kernel(const voi
   const bool is_qk = unit < 2 * G, mine = lane * 4 < (is_qk ? d : dv);
   const int c = (is_qk ? unit * d : 2 * nqk + (unit - 2 * G) * dv) + lane * 4;
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-  float4 w[kTaps], hist[kTaps - 1], x[kTile];             // w[back]: the taps that meet the input `back` tokens ago; hist[back - 1]: that input
+  using Raw = std::conditional_t<sizeof(T4) == 2, uint2, float4>;   // rows on their way stay as they are in memory
+  const T4* rows = static_cast<const T4*>(proj) + t0 * ld + c;
+  auto load = [&](int i) { return mine && i < nt ? *reinterpret_cast<const Raw*>(rows + i * ld) : Raw{}; };
+  auto wide = [](const Raw& r) {
+    if constexpr (std::is_same_v<T4, __nv_bfloat16>)
+      return make_float4(__uint_as_float(r.x << 16), __uint_as_float(r.x & 0xffff0000u), __uint_as_float(r.y << 16), __uint_as_float(r.y & 0xffff0000u));
+    else
+      return rb::ld4_any(&r, sizeof(T4) == 4 ? 0 : 2, 0);
+  };
+  float4 w[kTaps], hist[kTaps - 1];                       // w[back]: the taps that meet the input `back` tokens ago; hist[back - 1]: that input
+  Raw xr[kTile];
 #pragma unroll
-  for (int i = 0; i < kTile; ++i) x[i] = mine && i < nt ? rb::ld4_any(proj, dt, (t0 + i) * ld + c) : zero;
+  for (int i = 0; i < kTile; ++i) xr[i] = load(i);
 #pragma unroll
-  for (int back = 1; back < kTaps; ++back) hist[back - 1] = mine && back < taps && t0 - back >= 0 ? rb::ld4_any(proj, dt, (t0 - back) * ld + c) : zero;
+  for (int back = 1; back < kTaps; ++back) hist[back - 1] = mine && back < taps && t0 - back >= 0 ? wide(*reinterpret_cast<const Raw*>(rows - back * ld)) : zero;
 #pragma unroll
   for (int back = 0; back < kTaps; ++back) {
     const bool in = mine && back < taps;
@@ -272,9 +284,9 @@ __global__ void __launch_bounds__(kPThreads) delta_prepare_warp_kernel(const voi
   const float scale = unit < G ? 1.f / sqrtf((float)d) : 1.f;
   for (int s0 = 0; s0 < nt; s0 += kTile) {
     const int p0 = lane < kTile && s0 + lane < nt ? pos[t0 + s0 + lane] : 0;
-    float4 nx[kTile];                                     // the next tile's rows
+    Raw nx[kTile];                                        // the next tile's rows
 #pragma unroll
-    for (int i = 0; i < kTile; ++i) nx[i] = mine && s0 + kTile + i < nt ? rb::ld4_any(proj, dt, (t0 + s0 + kTile + i) * ld + c) : zero;
+    for (int i = 0; i < kTile; ++i) nx[i] = load(s0 + kTile + i);
     if (conv_state != nullptr && taps > 1) {
 #pragma unroll
       for (int i = 0; i < kTile; ++i)
@@ -282,7 +294,8 @@ __global__ void __launch_bounds__(kPThreads) delta_prepare_warp_kernel(const voi
           const int slot = tok_slot[t0 + s0 + i], rem = remain[t0 + s0 + i];
           if (slot >= 0 && rem < taps - 1 && mine) {
             float* st = conv_state + ((int64_t)slot * (taps - 1) + (taps - 2 - rem)) * C + c;
-            st[0] = x[i].x; st[1] = x[i].y; st[2] = x[i].z; st[3] = x[i].w;
+            const float4 x = wide(xr[i]);
+            st[0] = x.x; st[1] = x.y; st[2] = x.z; st[3] = x.w;
           }
         }
     }
@@ -290,16 +303,17 @@ __global__ void __launch_bounds__(kPThreads) delta_prepare_warp_kernel(const voi
     for (int i = 0; i < kTile; ++i) {
       const int p = __shfl_sync(0xffffffffu, p0, i);
       float4 y = zero;
+      const float4 x = wide(xr[i]);
       auto tap = [&](const float4& a, const float4& b) {
         y.x = fmaf(a.x, b.x, y.x); y.y = fmaf(a.y, b.y, y.y); y.z = fmaf(a.z, b.z, y.z); y.w = fmaf(a.w, b.w, y.w);
       };
 #pragma unroll
       for (int back = kTaps - 1; back >= 1; --back)       // oldest first, the current token last: a fixed order
         if (back < taps && back <= p) tap(hist[back - 1], w[back]);
-      tap(x[i], w[0]);
+      tap(x, w[0]);
 #pragma unroll
       for (int back = kTaps - 1; back >= 2; --back) hist[back - 1] = hist[back - 2];
-      if constexpr (kTaps > 1) hist[0] = x[i];
+      if constexpr (kTaps > 1) hist[0] = x;
       y.x = y.x / (1.f + expf(-y.x)); y.y = y.y / (1.f + expf(-y.y)); y.z = y.z / (1.f + expf(-y.z)); y.w = y.w / (1.f + expf(-y.w));
       if (is_qk) {
         const float r = scale * (1.f / sqrtf(rb::warp_sum((y.x * y.x + y.y * y.y) + (y.z * y.z + y.w * y.w)) + unit_eps));
@@ -308,7 +322,7 @@ __global__ void __launch_bounds__(kPThreads) delta_prepare_warp_kernel(const voi
       if (mine && s0 + i < nt) *reinterpret_cast<float4*>(u + (t0 + s0 + i) * UW + c) = y;
     }
 #pragma unroll
-    for (int i = 0; i < kTile; ++i) x[i] = nx[i];
+    for (int i = 0; i < kTile; ++i) xr[i] = nx[i];
   }
 }
 
@@ -752,10 +766,13 @@ extern "C" int rb_delta_prepare(const void* proj, int64_t ld, int dt, const void
       const int walk = T * units >= (int64_t)rb::kNumSMs * 16 * 32 ? 32 : kTile, per_cta = kPThreads / 32 * walk;
       const dim3 grid(units, (unsigned)((T + per_cta - 1) / per_cta));
       auto go = [&](auto kern) { kern<<<grid, kPThreads, 0, s>>>(proj, ld, dt, conv_w, gp, u, pos, conv_state, tok_slot, remain, T, H, G, d, dv, taps, unit_eps); };
-      if (walk == 32 && taps <= 4) go(delta_prepare_warp_kernel<4, 32>);
-      else if (walk == 32) go(delta_prepare_warp_kernel<kMaxTaps, 32>);
-      else if (taps <= 4) go(delta_prepare_warp_kernel<4, kTile>);
-      else go(delta_prepare_warp_kernel<kMaxTaps, kTile>);
+#define RB_GO(T4)                                                                \
+  if (walk == 32 && taps <= 4) go(delta_prepare_warp_kernel<T4, 4, 32>);         \
+  else if (walk == 32) go(delta_prepare_warp_kernel<T4, kMaxTaps, 32>);          \
+  else if (taps <= 4) go(delta_prepare_warp_kernel<T4, 4, kTile>);               \
+  else go(delta_prepare_warp_kernel<T4, kMaxTaps, kTile>)
+      if (dt == 0) { RB_GO(float); } else if (dt == 1) { RB_GO(__nv_bfloat16); } else { RB_GO(__half); }
+#undef RB_GO
       return 0;
     }
     dim3 grid((unsigned)((T + kPT - 1) / kPT), units);

@@ -75,6 +75,21 @@ def test_delta_prepare_taps(d, dv, taps, dtype):
         assert torch.equal(c_st.cpu(), st)
 
 
+@pytest.mark.parametrize("T", [100, 9000])
+@pytest.mark.parametrize("taps", [3, 8])
+def test_delta_prepare_is_the_same_for_every_type(taps, T):
+    """Inputs that all three types hold exactly: everything behind the loads is fp32, so the results are the same bits."""
+    from realhf_b200.api.model import DeltaRuleConfig
+    from realhf_b200.models.sharding import delta_sections
+    cfg = DeltaRuleConfig(n_heads=4, n_kv_heads=2, qk_dim=16, v_dim=24, conv_taps=taps)
+    g = torch.Generator().manual_seed(taps)
+    rn = lambda *s: (torch.randint(-63, 64, s, generator=g) / 32).cuda()
+    args = [rn(T, sum(delta_sections(cfg))), rn(4 * 16 + 4 * 24, taps), rn(4), rn(4)]
+    pos = torch.cat([torch.arange(41), torch.arange(T - 41)]).int().cuda()
+    got = [R.delta_prepare(*(a.to(dt) for a in args), cfg, pos, None, None, None) for dt in (torch.float32, torch.bfloat16, torch.float16)]
+    assert torch.equal(got[0], got[1]) and torch.equal(got[0], got[2])
+
+
 @pytest.mark.parametrize("taps", [2, 4, 7])
 def test_delta_prepare_many_tokens(taps):
     """Enough tokens that a warp walks 32 of them: sequences that begin and end inside its tiles of 8, a remainder of tokens, the final inputs kept."""
