@@ -236,7 +236,7 @@ __global__ void __launch_bounds__(kPThreads) delta_prepare_tiled_kernel(const vo
 // tokens in tiles of 8 whose rows it has in flight together; the per-(token, head) sum of squares stays inside the warp.  The kernel above moves two
 // bytes a lane and load and four a store, and waits for its loads with few of them on their way: 8 sequences of 700 .. 1024 tokens, 16 + 2 x 4 heads x 128
 // (71 MB in, 85 MB out) 121 us; this way 49.  What it waits for is its loads and the issue of some 45 instructions a channel and token (24 us of bytes, about 20
-// of issue), so rows on their way stay as they are in memory: 96 registers and five CTAs an SM for 16-bit rows (widened on arrival, the type told apart at
+// of issue), so rows on their way stay as they are in memory: 94 registers and five CTAs an SM for 16-bit rows (widened on arrival, the type told apart at
 // run time, 124 registers: 87 us; four CTAs 57, six, with spills, 53; bf16 widened by the pair conversions instead of shifts 59).  kTaps: the taps that registers are kept for.
 constexpr int kTile = 8;
 
