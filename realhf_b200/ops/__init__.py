@@ -19,8 +19,8 @@ _lib = None
 _host = None
 
 
-# kernels launched per op call (for the `gpu_launches` accounting of bench.py)
-_KERNELS_PER_OP = {"rmsnorm_bwd": 2, "embedding_grad_": 3, "adamw_step": 1, "decode_attention": 1, "attn_check": 0, "attn_status": 0, "attn_wait_error": 0}
+# kernels launched per op call (for the `gpu_launches` accounting of bench.py); embedding_into: with its gradient
+_KERNELS_PER_OP = {"rmsnorm_bwd": 2, "embedding_grad_": 3, "embedding_into": 4, "adamw_step": 1, "decode_attention": 1, "attn_check": 0, "attn_status": 0, "attn_wait_error": 0}
 
 
 class _LaunchCounter:

@@ -815,7 +815,8 @@ def embed_sinusoid_ref(ids, wte, pos, inv_freq):
 
 
 class _Embedding(torch.autograd.Function):
-    """A table lookup whose gradient is added to the table's gradient buffer row by row (`csrc/embed_grad.cu`): no sort, no dense [V, H] beside the buffer."""
+    """A table lookup whose gradient is added to the table's gradient buffer row by row (`csrc/embed_grad.cu`): no sort, no dense [V, H] beside the buffer.
+    For a buffer beside `.grad` (`main_grad`); with the buffer in `.grad` the native `embedding_into` does the same."""
 
     @staticmethod
     def forward(ctx, ids, weight):
@@ -847,9 +848,13 @@ def _row_grad_buffer(weight):
     return g if g.is_contiguous() and weight.shape[1] % 8 == 0 and g.data_ptr() % 16 == 0 else None
 
 
+def _packed_rows(ids, weight):
+    return (weight.dim() == 2 and weight.is_contiguous() and weight.shape[1] * weight.element_size() % 16 == 0 and weight.data_ptr() % 16 == 0
+            and ids.device == weight.device)
+
+
 def _rows(ids, weight):
-    if (weight.dim() == 2 and weight.is_contiguous() and weight.shape[1] * weight.element_size() % 16 == 0 and weight.data_ptr() % 16 == 0
-            and ids.device == weight.device):
+    if _packed_rows(ids, weight):
         return lib().embedding_rows(weight, ids.contiguous())
     return F.embedding(ids, weight)
 
@@ -863,6 +868,8 @@ def embedding(ids, weight):
         if not (weight.requires_grad and torch.is_grad_enabled()):
             return _rows(ids, weight)
         if weight.is_leaf and weight.dim() == 2 and _row_grad_buffer(weight) is not None:
+            if getattr(weight, "main_grad", None) is None and _packed_rows(ids, weight):
+                return lib().embedding_into(weight, ids.contiguous())
             return _Embedding.apply(ids, weight)
     return F.embedding(ids, weight)
 

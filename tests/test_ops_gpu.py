@@ -421,3 +421,29 @@ def test_rms_norm_of_few_rows(rows, H, dtype):
         bound = want.abs() * (2.0 ** -19 + torch.finfo(dtype).eps / 2) + (2.0 ** -24 if dtype == torch.float16 else 0)
         assert ((out[0].double() - want).abs() <= bound).all()
         assert ((out[1].double().flatten() - rstd).abs() <= rstd * 2.0 ** -19).all()
+
+
+def test_embedding_gradient_finds_the_buffer_when_it_comes():
+    """The buffer of the backward pass counts, not that of the forward pass; without one the gradient is the library's; ids of two forms; twice through one table."""
+    from realhf_b200.ops import functional as OF
+    g = torch.Generator(device="cuda").manual_seed(2)
+    w = torch.nn.Parameter(torch.randn(40, 64, device="cuda", generator=g).bfloat16())
+    ids = torch.randint(0, 40, (2, 30), device="cuda", generator=g)
+    dy = torch.randint(-4, 5, (2, 30, 64), device="cuda", generator=g).bfloat16()      # sums are exact
+    want = torch.zeros(40, 64, device="cuda").index_add_(0, ids.view(-1), dy.view(-1, 64).float()).bfloat16()
+    first, second = torch.zeros_like(w), torch.ones_like(w)
+    w.grad, w._grad_in_flat_buffer = first, True
+    y = OF.embedding(ids, w)
+    w.grad = second
+    y.backward(dy)
+    assert not first.any() and w.grad is second and torch.equal(second, want + 1)
+    w.grad = first
+    y = OF.embedding(ids, w)
+    w.grad = None
+    y.backward(dy)
+    assert torch.equal(w.grad, want)
+    w.grad = first
+    (OF.embedding(ids, w) + OF.embedding(ids.t().int(), w).transpose(0, 1)).backward(dy)
+    assert w.grad is first and torch.equal(first, 2 * want)
+    with torch.no_grad():
+        assert torch.equal(OF.embedding(ids, w), w[ids])
