@@ -36,12 +36,13 @@ template <typename T> RB_DEVICE void store8(T* p, const float* acc) {
   }
 }
 
-// A block copies kVec x 128 pieces of one row.  Launched so that the next kernel may become resident meanwhile, as the others of a generation step.
+// A block copies kVec x 128 pieces of one row.  It heads a forward pass, so it lets the next kernels start only behind its own wait: a small-row product two kernels
+// on asks for weight tiles in front of ITS wait, and what wrote the weights may be the kernel in front of this one, whose stores nothing but a wait makes visible.
 constexpr int kRowThreads = 128;
 template <typename I, int kVec>
 __global__ void __launch_bounds__(kRowThreads) rows_kernel(const I* __restrict__ ids, const uint4* __restrict__ table, uint4* __restrict__ out, int64_t V, int n) {
-  rb::pdl_trigger();
   rb::pdl_wait();
+  rb::pdl_trigger();
   const int64_t t = blockIdx.x, v = (int64_t)ids[t];
   assert(v >= 0 && v < V);                                // as the library's lookup does
   const int first = blockIdx.y * (kVec * kRowThreads) + threadIdx.x;

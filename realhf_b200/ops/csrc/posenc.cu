@@ -12,8 +12,8 @@ namespace {
 __global__ void embed_sinusoid_kernel(const int64_t* __restrict__ ids, const void* __restrict__ wte, int dtw, const int* __restrict__ pos,
                                       const int* __restrict__ slots, const float* __restrict__ inv_freq, float* __restrict__ out, int W, int vocab) {
   const int64_t t = blockIdx.x;
+  rb::pdl_wait();                      // it heads a forward pass: the next kernels start behind this wait only (as the row copy in embed_grad.cu)
   rb::pdl_trigger();
-  rb::pdl_wait();
   int64_t id = ids[t];
   id = id < 0 ? 0 : (id >= vocab ? vocab - 1 : id);
   const float p = (float)(slots ? pos[slots[t]] : pos[t]);
