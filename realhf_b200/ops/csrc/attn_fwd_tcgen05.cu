@@ -386,7 +386,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) attn_fwd_kernel(const __grid_c
         if (kMode != kGeneral && kMode != kCap && mx != -INFINITY) mx *= c2;
         const float m_new = fmaxf(m_run, mx);
         const float alpha = m_new == m_run ? 1.f : exp2f(m_run - m_new);
-        l_run *= alpha;
+        l_run = __fmul_rn(l_run, alpha);              // (rounded by itself: contracted with the sum below, the statistics' last bits would depend on the compiler)
         m_run = m_new;
         if (k > 0) {                                  // the output warps scale the row while its weights are formed
           row_alpha[t * kTile + row] = alpha;
@@ -494,7 +494,9 @@ __global__ void __launch_bounds__(kFwdThreads, 1) attn_fwd_kernel(const __grid_c
         const float l_run = row_l[t * kTile + row];
         inv *= 1.f / l_run;
         if constexpr (kMode == kPlain) {
-          if (q_pos < it.L) p.lse[(int64_t)head * p.T + it.tok0 + q_pos] = row_m[t * kTile + row] * 0.6931471805599453f + __logf(l_run);
+          // (the larger product rounded by itself, spelled out: the statistics do not depend on what the compiler contracts)
+          if (q_pos < it.L)
+            p.lse[(int64_t)head * p.T + it.tok0 + q_pos] = __fmaf_rn(__log2f(l_run), 0.6931471805599453f, __fmul_rn(row_m[t * kTile + row], 0.6931471805599453f));
         }
         __syncwarp();
         if (lane == 0) ptx::mbar_arrive(bar(L_EMPTY + t));

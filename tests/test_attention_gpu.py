@@ -443,3 +443,54 @@ def test_a_wait_that_ran_out_in_a_generation_step_is_raised(use_graph, monkeypat
     assert m.training and lib().attn_wait_error() == 1
     monkeypatch.undo()
     assert torch.equal(run(), want)
+
+
+def _scores(cols):
+    """Sequences [S, n keys, 128] of scores -> q, k, v of one head whose query r has the scores of column r % 128, one sequence after the other."""
+    S, n, _ = cols.shape
+    q = torch.eye(128, device=DEV, dtype=torch.bfloat16)[torch.arange(n, device=DEV) % 128].repeat(S, 1).view(S * n, 1, 128)
+    k = cols.reshape(S * n, 1, 128).bfloat16()
+    assert torch.equal(k.float(), cols.reshape(S * n, 1, 128))
+    return q, k, torch.zeros_like(k), torch.arange(S + 1, device=DEV, dtype=torch.int32) * n
+
+
+def _bits(x, ones, n=128):
+    """Scores [..., n]: weights 2^score whose sum is x (< 4, 24 bits): `ones` keys of weight one first."""
+    i = torch.arange(n, device=DEV)
+    frac = (x - x.floor()).double().unsqueeze(-1)
+    bit = (frac * 2.0 ** i.clamp(max=24)).floor() % 2
+    s = torch.where((i >= 1) & (i <= 23) & (bit == 1), -i.double(), -256.0)
+    return torch.where((i == 0) | ((i > 23) & (i < 23 + ones.unsqueeze(-1))), 0.0, s).float()
+
+
+LN2 = 0.6931471805599453            # as the scale: a weight is 2^score exactly
+
+
+def test_attention_statistics_are_rounded_tile_by_tile():
+    """The denominator of two key tiles is round(round(l * factor) + sum of the second tile): scores chosen so that the weights are powers of two and their sums exact leave these two
+    roundings alone, and a sequence of one tile with that very denominator gives the same statistics bit for bit."""
+    g = torch.Generator(device=DEV).manual_seed(3)
+    draw = lambda: 1 + torch.randint(0, 2 ** 23, (16, 128), device=DEV, generator=g).float() * 2.0 ** -23  # noqa: E731
+    l1, s2 = draw(), draw()
+    one = torch.ones_like(l1)
+    first = _bits(l1, one)
+    cols = torch.cat([torch.where(first > -100, first - 0.5, first), _bits(s2, one)], -1).transpose(1, 2).contiguous()
+    factor = torch.exp2(torch.tensor(-0.5, device=DEV))
+    total = l1 * factor + s2
+    assert (total.double() != (l1.double() * factor.double() + s2.double()).float().double()).sum() > 100       # a contracted sum would show
+    q, k, v, cu = _scores(cols)
+    lse = lib().attn_fwd(q, k, v, cu, 256, LN2, False)[1].view(16, 2, 128)
+    q, k, v, cu = _scores(_bits(total, total.floor()).transpose(1, 2).contiguous())
+    want = lib().attn_fwd(q, k, v, cu, 128, LN2, False)[1].view(16, 1, 128)
+    assert torch.equal(lse, want.expand_as(lse))
+
+
+def test_attention_statistics_end_in_one_rounding():
+    """log2 of a power of two is exact: the statistics are the maximum's product rounded once, the logarithm's added with one rounding."""
+    j = torch.arange(8, device=DEV).repeat(16)
+    m = (torch.arange(128, device=DEV) - 64) * 0.5 - 3.5
+    i = torch.arange(128, device=DEV)[:, None]
+    q, k, v, cu = _scores(torch.where(i < 2 ** j, m, -256.0)[None].float())
+    lse = lib().attn_fwd(q, k, v, cu, 128, LN2, False)[1][0]
+    ln2 = torch.tensor(LN2, dtype=torch.float32, device=DEV)
+    assert torch.equal(lse, (j.double() * ln2.double() + (m.float() * ln2).double()).float())
