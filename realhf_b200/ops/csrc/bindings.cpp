@@ -307,6 +307,8 @@ void logprob_bwd_(Tensor logits, const Tensor& labels, const c10::optional<Tenso
 extern "C" int rb_embedding_grad(const void* dy, const void* ids, int ids_64, void* dst, int* scratch, int64_t T, int64_t V, int64_t H, int g_dt, int d_dt,
                                  cudaStream_t s);
 
+extern "C" int64_t rb_embedding_grad_tokens();
+
 extern "C" int rb_embedding_rows(const void* table, const void* ids, int ids_64, void* out, int64_t T, int64_t V, int64_t row_bytes, cudaStream_t s);
 
 // table[ids] for a packed table whose rows are whole 16-byte pieces.
@@ -332,7 +334,7 @@ void embedding_grad_(const Tensor& dy, const Tensor& ids, Tensor dst) {
   TORCH_CHECK(dst.scalar_type() == dy.scalar_type() || dst.scalar_type() == at::kFloat, "embedding_grad_: buffer type");
   c10::cuda::CUDAGuard guard(dy.device());
   const int64_t T = dy.size(0), V = dst.size(0);
-  auto scratch = at::empty({2 * V + 1 + T / 32 + T}, dy.options().dtype(at::kInt));
+  auto scratch = at::empty({2 * V + 2 + 2 * T + 3 * (T / 33)}, dy.options().dtype(at::kInt));
   const int rc = rb_embedding_grad(dy.data_ptr(), ids.data_ptr(), ids.scalar_type() == at::kLong, dst.data_ptr(), scratch.data_ptr<int>(), T, V, dy.size(1),
                                    dt_code(dy), dt_code(dst), cur_stream());
   TORCH_CHECK(rc == 0, "embedding_grad_: unsupported configuration (", rc, ")");
@@ -351,7 +353,7 @@ class EmbeddingInto : public torch::autograd::Function<EmbeddingInto> {
     if (!grads[0].defined() || !ctx->needs_input_grad(1)) return {Tensor(), Tensor()};
     const Tensor ids = ctx->get_saved_variables()[0].reshape({-1}).contiguous(), table = ctx->saved_data["table"].toTensor();
     const Tensor dy = grads[0].reshape({-1, table.size(1)}).contiguous(), g = table.grad();
-    const bool fits = g.defined() && g.is_cuda() && g.sizes() == table.sizes() && g.is_contiguous() && table.size(1) % 8 == 0 &&
+    const bool fits = dy.size(0) <= rb_embedding_grad_tokens() && g.defined() && g.is_cuda() && g.sizes() == table.sizes() && g.is_contiguous() && table.size(1) % 8 == 0 &&
                       (g.scalar_type() == at::kFloat || (g.scalar_type() == dy.scalar_type() && (dy.scalar_type() == at::kBFloat16 || dy.scalar_type() == at::kHalf))) &&
                       ((reinterpret_cast<uintptr_t>(g.data_ptr()) | reinterpret_cast<uintptr_t>(dy.data_ptr())) & 15) == 0;
     if (!fits) return {Tensor(), at::embedding_dense_backward(dy, ids, table.size(0), -1, false)};
@@ -390,6 +392,7 @@ TORCH_LIBRARY(realhf_b200, m) {
   m.def("logprob_bwd_(Tensor(a!) logits, Tensor labels, Tensor? mask, Tensor lse, Tensor dlogp, float inv_temp, int vocab_start) -> ()", &logprob_bwd_);
   m.def("embedding_rows(Tensor table, Tensor ids) -> Tensor", &embedding_rows);
   m.def("embedding_into(Tensor table, Tensor ids) -> Tensor", &embedding_into);
+  m.def("embedding_grad_tokens() -> int", &rb_embedding_grad_tokens);
   m.def("embedding_grad_(Tensor dy, Tensor ids, Tensor(a!) dst) -> ()", &embedding_grad_);
   register_gemm_ops(m);
   register_attn_ops(m);

@@ -831,7 +831,7 @@ class _Embedding(torch.autograd.Function):
             return None, None
         dy = dy.reshape(-1, weight.shape[1]).contiguous()
         g = _row_grad_buffer(weight)
-        if g is None or (g.dtype != dy.dtype and g.dtype != torch.float32) or dy.data_ptr() % 16:
+        if g is None or dy.shape[0] > lib().embedding_grad_tokens() or (g.dtype != dy.dtype and g.dtype != torch.float32) or dy.data_ptr() % 16:
             return None, torch.ops.aten.embedding_dense_backward(dy, ids.reshape(-1), weight.shape[0], -1, False)
         lib().embedding_grad_(dy, ids.reshape(-1).contiguous(), g)
         return None, None

@@ -388,6 +388,52 @@ def test_embedding_gradient_goes_into_the_buffer(T, V, H, dtype, buffer):
         assert torch.equal(got[0][V - 1], start[V - 1])
 
 
+def _positions(B, n):
+    return torch.arange(n, device="cuda").repeat(B)
+
+
+@pytest.mark.parametrize("B,n,H,ids_dtype", [(33, 50, 264, torch.int64), (40, 700, 1032, torch.int32), (512, 30, 72, torch.int64), (513, 30, 72, torch.int32),
+                                             (1030, 68, 136, torch.int64), (33, 1, 8, torch.int64)])
+def test_embedding_gradient_of_many_long_chains(B, n, H, ids_dtype):
+    """Positions of B sequences: every id has B tokens, ranked up to 512 and through a bitmap beyond, over more than one window of 65536 tokens too; some ids outside the
+    table, which are passed over.  Small whole numbers, so that the sums are exact; the tokens in any order, and the same for fp32 rows."""
+    from realhf_b200.ops import lib
+    g = torch.Generator(device="cuda").manual_seed(B + n)
+    ids = _positions(B, n)[torch.randperm(B * n, device="cuda", generator=g)]
+    ids[ids == n // 2] = torch.where(torch.rand(B, device="cuda", generator=g) < 0.5, -1, n + 3) if n > 1 else 0
+    keep = (ids >= 0) & (ids < n)
+    dy = torch.randint(-3, 4, (B * n, H), device="cuda", generator=g).float()
+    want = torch.ones(n, H, device="cuda").index_add_(0, ids[keep], dy[keep])
+    for dtype, buffer in ((torch.float32, torch.float32), (torch.bfloat16, torch.float32), (torch.float16, torch.float16)):
+        buf = torch.ones(n, H, device="cuda", dtype=buffer)
+        lib().embedding_grad_(dy.to(dtype), ids.to(ids_dtype), buf)
+        assert torch.equal(buf, want.to(buffer))
+
+
+@pytest.mark.parametrize("ids,V,H", [(lambda: _positions(64, 1024), 1024, 1024), (lambda: _positions(128, 512), 1024, 768),
+                                     (lambda: torch.arange(32768, device="cuda") * 7919 % 256, 256, 1024), (lambda: torch.zeros(100000, device="cuda", dtype=torch.long), 8, 256)],
+                         ids=["64x1024 positions", "128x512 positions", "256 ids", "one id"])
+def test_embedding_gradient_is_no_slower_than_the_library(ids, V, H):
+    """Where every id is frequent: against the library's dense gradient and its sum into the buffer, best of a few (2 .. 8 times as fast when written)."""
+    from realhf_b200.ops import lib
+    ids, L = ids(), lib()
+    dy, buf = torch.randn(ids.numel(), H, device="cuda").bfloat16(), torch.zeros(V, H, device="cuda", dtype=torch.bfloat16)
+
+    def best(f):
+        times = []
+        for _ in range(6):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            for _ in range(5):
+                f()
+            b.record()
+            b.synchronize()
+            times.append(a.elapsed_time(b))
+        return min(times)
+    ours = best(lambda: L.embedding_grad_(dy, ids, buf))
+    assert ours <= best(lambda: buf.add_(torch.ops.aten.embedding_dense_backward(dy, ids, V, -1, False)))
+
+
 @pytest.mark.parametrize("dtype,ids_dtype", [(torch.bfloat16, torch.int64), (torch.float16, torch.int32), (torch.float32, torch.int64)])
 @pytest.mark.parametrize("shape,V,H", [((1,), 1, 8), ((16,), 50, 4096), ((3, 5), 7, 1032), ((0,), 3, 64), ((700,), 300, 72), ((300,), 64, 4104), ((9,), 5, 12)])
 def test_embedding_rows_are_copied(shape, V, H, dtype, ids_dtype):
