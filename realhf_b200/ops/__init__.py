@@ -20,7 +20,7 @@ _host = None
 
 
 # kernels launched per op call (for the `gpu_launches` accounting of bench.py); embedding_into: with its gradient
-_KERNELS_PER_OP = {"rmsnorm_bwd": 2, "embedding_grad_": 4, "embedding_into": 5, "embedding_grad_tokens": 0, "adamw_step": 1, "decode_attention": 1, "attn_check": 0, "attn_status": 0, "attn_wait_error": 0}
+_KERNELS_PER_OP = {"rmsnorm_bwd": 2, "embedding_grad_": 4, "embedding_into": 5, "embedding_grad_tokens": 0, "gradient_goes_past": 0, "adamw_step": 1, "decode_attention": 1, "attn_check": 0, "attn_status": 0, "attn_wait_error": 0}
 
 
 class _LaunchCounter:

@@ -3,6 +3,9 @@
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/csrc/autograd/custom_function.h>
+#include <torch/csrc/autograd/function.h>
+#include <torch/csrc/autograd/graph_task.h>
+#include <torch/csrc/autograd/variable.h>
 #include <torch/library.h>
 #include <torch/types.h>
 
@@ -340,6 +343,20 @@ void embedding_grad_(const Tensor& dy, const Tensor& ids, Tensor dst) {
   TORCH_CHECK(rc == 0, "embedding_grad_: unsupported configuration (", rc, ")");
 }
 
+// In a backward pass: whether the gradient of a leaf may be added to its buffer here, past autograd's own accumulation.  Not when somebody is to get the gradient
+// itself: `torch.autograd.grad` with respect to the leaf, hooks of the tensor or of its accumulation (own_hook: there is one after the accumulation that the buffer
+// brought with it), a gradient that is to be differentiated again.
+bool gradient_goes_past(const Tensor& leaf, bool own_hook) {
+  if (at::GradMode::is_enabled()) return false;
+  const auto acc = torch::autograd::impl::try_get_grad_accumulator(leaf);
+  if (acc == nullptr || !acc->tensor_pre_hooks().empty() || !acc->pre_hooks().empty() || !acc->post_hooks().empty()) return false;
+  if (!own_hook && acc->tensor_post_acc_grad_hooks() != nullptr) return false;
+  const auto* info = torch::autograd::get_current_graph_task_exec_info();      // empty: every leaf accumulates
+  if (info == nullptr || info->empty()) return true;
+  const auto it = info->find(acc.get());
+  return it != info->end() && it->second.needed_ && !it->second.captures_;
+}
+
 // table[ids] whose gradient is added to the table's .grad (a leaf's, looked up when the gradient comes; a gradient buffer keeps it there).  Native, as a training step
 // of few tokens waits for the host: as a Python function, forward and backward cost 20 us more than the library's lookup, which a step of 1200 us showed.
 class EmbeddingInto : public torch::autograd::Function<EmbeddingInto> {
@@ -353,7 +370,7 @@ class EmbeddingInto : public torch::autograd::Function<EmbeddingInto> {
     if (!grads[0].defined() || !ctx->needs_input_grad(1)) return {Tensor(), Tensor()};
     const Tensor ids = ctx->get_saved_variables()[0].reshape({-1}).contiguous(), table = ctx->saved_data["table"].toTensor();
     const Tensor dy = grads[0].reshape({-1, table.size(1)}).contiguous(), g = table.grad();
-    const bool fits = dy.size(0) <= rb_embedding_grad_tokens() && g.defined() && g.is_cuda() && g.sizes() == table.sizes() && g.is_contiguous() && table.size(1) % 8 == 0 &&
+    const bool fits = gradient_goes_past(table, false) && dy.size(0) <= rb_embedding_grad_tokens() && g.defined() && g.is_cuda() && g.sizes() == table.sizes() && g.is_contiguous() && table.size(1) % 8 == 0 &&
                       (g.scalar_type() == at::kFloat || (g.scalar_type() == dy.scalar_type() && (dy.scalar_type() == at::kBFloat16 || dy.scalar_type() == at::kHalf))) &&
                       ((reinterpret_cast<uintptr_t>(g.data_ptr()) | reinterpret_cast<uintptr_t>(dy.data_ptr())) & 15) == 0;
     if (!fits) return {Tensor(), at::embedding_dense_backward(dy, ids, table.size(0), -1, false)};
@@ -392,6 +409,7 @@ TORCH_LIBRARY(realhf_b200, m) {
   m.def("logprob_bwd_(Tensor(a!) logits, Tensor labels, Tensor? mask, Tensor lse, Tensor dlogp, float inv_temp, int vocab_start) -> ()", &logprob_bwd_);
   m.def("embedding_rows(Tensor table, Tensor ids) -> Tensor", &embedding_rows);
   m.def("embedding_into(Tensor table, Tensor ids) -> Tensor", &embedding_into);
+  m.def("gradient_goes_past(Tensor leaf, bool own_hook) -> bool", &gradient_goes_past);
   m.def("embedding_grad_tokens() -> int", &rb_embedding_grad_tokens);
   m.def("embedding_grad_(Tensor dy, Tensor ids, Tensor(a!) dst) -> ()", &embedding_grad_);
   register_gemm_ops(m);

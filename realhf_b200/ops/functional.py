@@ -830,7 +830,8 @@ class _Embedding(torch.autograd.Function):
         if not ctx.needs_input_grad[1]:
             return None, None
         dy = dy.reshape(-1, weight.shape[1]).contiguous()
-        g = _row_grad_buffer(weight)
+        own = bool(getattr(weight, "_main_grad_hooked", False)) and len(weight._post_accumulate_grad_hooks or ()) == 1
+        g = _row_grad_buffer(weight) if lib().gradient_goes_past(weight, own) else None
         if g is None or dy.shape[0] > lib().embedding_grad_tokens() or (g.dtype != dy.dtype and g.dtype != torch.float32) or dy.data_ptr() % 16:
             return None, torch.ops.aten.embedding_dense_backward(dy, ids.reshape(-1), weight.shape[0], -1, False)
         lib().embedding_grad_(dy, ids.reshape(-1).contiguous(), g)
@@ -860,9 +861,10 @@ def _rows(ids, weight):
 
 
 def embedding(ids, weight):
-    """weight[ids].  With a gradient asked for and a gradient buffer on the GPU the rows' gradients go straight into the buffer; without a gradient the lookup is
-    a kernel of its own; elsewhere (and inside function transforms and forward-mode differentiation, which the autograd function does not answer for) the
-    plain lookup."""
+    """weight[ids].  With a gradient asked for and a gradient buffer on the GPU the rows' gradients go straight into the buffer, unless somebody is to get the gradient
+    itself (`torch.autograd.grad` with respect to the table, hooks on it, a gradient that is differentiated again: autograd accumulates then, as for a plain
+    lookup); without a gradient the lookup is a kernel of its own; elsewhere (and inside function transforms and forward-mode differentiation, which the autograd
+    function does not answer for) the plain lookup."""
     if (use_native(weight) and ids.dtype in (torch.int64, torch.int32)
             and not (torch.autograd.forward_ad._current_level >= 0 or torch._C._functorch.peek_interpreter_stack() is not None)):
         if not (weight.requires_grad and torch.is_grad_enabled()):

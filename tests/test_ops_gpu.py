@@ -493,3 +493,83 @@ def test_embedding_gradient_finds_the_buffer_when_it_comes():
     assert w.grad is first and torch.equal(first, 2 * want)
     with torch.no_grad():
         assert torch.equal(OF.embedding(ids, w), w[ids])
+
+
+def _table(form):
+    """A table with its gradient buffer as `ReaLModel.attach_grad_buffer` leaves it: in .grad, or in fp32 beside it with the hook that folds .grad into it."""
+    g = torch.Generator(device="cuda").manual_seed(5)
+    w = torch.nn.Parameter(torch.randn(40, 64, device="cuda", generator=g).bfloat16())
+    ids = torch.randint(0, 40, (2, 30), device="cuda", generator=g)
+    dy = torch.randint(-4, 5, (2, 30, 64), device="cuda", generator=g).bfloat16()
+    want = torch.zeros(40, 64, device="cuda").index_add_(0, ids.view(-1), dy.view(-1, 64).float())
+    if form == "grad":
+        w.grad, w._grad_in_flat_buffer = torch.ones_like(w), True
+        return w, ids, dy, want, w.grad
+    w.main_grad = torch.ones(40, 64, device="cuda")
+
+    def fold(p):
+        if p.grad is not None:
+            p.main_grad.add_(p.grad)
+            p.grad = None
+    w.register_post_accumulate_grad_hook(fold)
+    w._main_grad_hooked = True
+    return w, ids, dy, want, w.main_grad
+
+
+@pytest.mark.parametrize("form", ["grad", "main_grad"])
+def test_embedding_gradient_is_given_to_who_asks_for_it(form):
+    """With a buffer attached: `torch.autograd.grad` returns the table's gradient and leaves the buffer alone, also twice differentiated and over a batch of gradients; hooks get
+    it; a plain backward pass and one restricted to the table go into the buffer without a dense gradient."""
+    from realhf_b200.ops import functional as OF
+    w, ids, dy, want, buf = _table(form)
+    one = buf.clone()
+    got, = torch.autograd.grad(OF.embedding(ids, w), w, dy)
+    assert torch.equal(got.float(), want) and torch.equal(buf, one)
+    got, = torch.autograd.grad(OF.embedding(ids, w), w, torch.stack([dy, 2 * dy]), is_grads_batched=True)
+    assert torch.equal(got.float(), torch.stack([want, 2 * want])) and torch.equal(buf, one)
+    c = torch.ones((), device="cuda", requires_grad=True)
+    first, = torch.autograd.grad(OF.embedding(ids, w), w, dy * c.bfloat16(), create_graph=True)
+    second, = torch.autograd.grad(first.float().sum(), c)
+    assert torch.equal(first.float(), want) and second.item() == dy.float().sum().item() and torch.equal(buf, one)
+
+    OF.embedding(ids, w).backward(dy)
+    assert torch.equal(buf.float(), want + 1)
+    OF.embedding(ids, w).backward(dy, inputs=[w])
+    assert torch.equal(buf.float(), 2 * want + 1)
+
+    seen = []
+    handle = w.register_hook(lambda g: seen.append(g.clone()))
+    OF.embedding(ids, w).backward(dy)
+    handle.remove()
+    assert len(seen) == 1 and torch.equal(seen[0].float(), want) and torch.equal(buf.float(), 3 * want + 1)
+    after = []
+    handle = w.register_post_accumulate_grad_hook(lambda p: after.append(1))
+    OF.embedding(ids, w).backward(dy)
+    handle.remove()
+    assert after == [1] and torch.equal(buf.float(), 4 * want + 1)
+    node = w.view_as(w).grad_fn.next_functions[0][0]
+    calls = []
+    handle = node.register_hook(lambda *a: calls.append(a[1][0].clone()))
+    OF.embedding(ids, w).backward(dy)
+    handle.remove()
+    assert len(calls) == 1 and torch.equal(calls[0].float(), want) and torch.equal(buf.float(), 5 * want + 1)
+
+
+@pytest.mark.parametrize("form", ["grad", "main_grad"])
+def test_embedding_gradient_of_a_plain_pass_is_not_dense(form):
+    """A plain backward pass adds to the buffer by the kernels: nothing of the table's size is allocated."""
+    from realhf_b200.ops import functional as OF
+    w, ids, dy, want, buf = _table(form)
+    big = torch.nn.Parameter(torch.zeros(200000, 64, device="cuda", dtype=torch.bfloat16))
+    if form == "grad":
+        big.grad, big._grad_in_flat_buffer = torch.zeros_like(big), True
+    else:
+        big.main_grad, big._main_grad_hooked = torch.zeros(200000, 64, device="cuda"), True
+        big.register_post_accumulate_grad_hook(lambda p: None)
+    y = OF.embedding(ids, big)
+    torch.cuda.synchronize()
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    y.backward(dy)
+    assert torch.cuda.max_memory_allocated() - before < big.numel()
+    assert torch.equal((big.grad if form == "grad" else big.main_grad)[:40].float(), want)
