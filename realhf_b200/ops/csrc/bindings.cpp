@@ -345,11 +345,14 @@ void embedding_grad_(const Tensor& dy, const Tensor& ids, Tensor dst) {
 
 // In a backward pass: whether the gradient of a leaf may be added to its buffer here, past autograd's own accumulation.  Not when somebody is to get the gradient
 // itself: `torch.autograd.grad` with respect to the leaf, hooks of the tensor or of its accumulation (own_hook: there is one after the accumulation that the buffer
-// brought with it), a gradient that is to be differentiated again.
+// brought with it), a gradient that is to be differentiated again.  Nor on another stream than the one the leaf's gradients are accumulated on, which alone orders
+// two uses of one leaf.
 bool gradient_goes_past(const Tensor& leaf, bool own_hook) {
   if (at::GradMode::is_enabled()) return false;
   const auto acc = torch::autograd::impl::try_get_grad_accumulator(leaf);
   if (acc == nullptr || !acc->tensor_pre_hooks().empty() || !acc->pre_hooks().empty() || !acc->post_hooks().empty()) return false;
+  const auto stream = acc->stream();
+  if (!stream.has_value() || *stream != at::cuda::getCurrentCUDAStream(leaf.get_device()).unwrap()) return false;
   if (!own_hook && acc->tensor_post_acc_grad_hooks() != nullptr) return false;
   const auto* info = torch::autograd::get_current_graph_task_exec_info();      // empty: every leaf accumulates
   if (info == nullptr || info->empty()) return true;

@@ -573,3 +573,61 @@ def test_embedding_gradient_of_a_plain_pass_is_not_dense(form):
     y.backward(dy)
     assert torch.cuda.max_memory_allocated() - before < big.numel()
     assert torch.equal((big.grad if form == "grad" else big.main_grad)[:40].float(), want)
+
+
+@pytest.mark.parametrize("form", ["grad", "main_grad"])
+def test_embedding_gradient_of_two_streams(form):
+    """Two lookups of one table on two streams: their gradients are added one after the other, as autograd orders its accumulation.  The second stream is kept behind the first by
+    long work of its own on some passes and ahead of it on others; ids and gradients are such that both change the same rows."""
+    from realhf_b200.ops import functional as OF
+    g = torch.Generator(device="cuda").manual_seed(6)
+    w = torch.nn.Parameter(torch.zeros(500, 512, device="cuda", dtype=torch.bfloat16))
+    buf = torch.zeros(500, 512, device="cuda", dtype=torch.bfloat16 if form == "grad" else torch.float32)
+    if form == "grad":
+        w.grad, w._grad_in_flat_buffer = buf, True
+    else:
+        w.main_grad = buf
+    ids = torch.randint(0, 500, (4000,), device="cuda", generator=g)
+    dy = torch.randint(-1, 2, (4000, 512), device="cuda", generator=g).bfloat16()
+    want = torch.zeros(500, 512, device="cuda").index_add_(0, ids, dy.float())
+    side, load = torch.cuda.Stream(), torch.randn(2048, 2048, device="cuda")
+    for k in range(6):
+        buf.zero_()
+        w.grad = buf if form == "grad" else None
+        side.wait_stream(torch.cuda.current_stream())
+        a = OF.embedding(ids, w)
+        with torch.cuda.stream(side):
+            b = OF.embedding(ids, w)
+            for _ in range(k % 3):
+                load = load @ load * 1e-3
+        torch.autograd.backward([a, b], [dy, dy])
+        torch.cuda.current_stream().wait_stream(side)
+        total = buf.float() + (w.grad.float() if form == "main_grad" and w.grad is not None else 0)
+        assert torch.equal(total, 2 * want)
+
+
+def test_gradients_go_past_autograd_on_the_accumulating_stream_only():
+    """Asked from backward passes on the stream that the leaf's accumulation belongs to (that of its first use) and on another one."""
+    from realhf_b200.ops import lib
+    w, said = torch.nn.Parameter(torch.zeros(4, 8, device="cuda")), []
+
+    class Ask(torch.autograd.Function):
+        @staticmethod
+        def forward(ctx, w):
+            ctx.w = w
+            return w * 1
+
+        @staticmethod
+        def backward(ctx, dy):
+            said.append(lib().gradient_goes_past(ctx.w, False))
+            return dy
+
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    a = Ask.apply(w)
+    with torch.cuda.stream(side):
+        b = Ask.apply(w)
+        b.sum().backward()
+    torch.cuda.current_stream().wait_stream(side)
+    a.sum().backward()
+    assert said == [False, True] and torch.equal(w.grad, torch.full_like(w, 2.0))
