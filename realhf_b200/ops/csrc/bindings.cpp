@@ -364,25 +364,30 @@ bool gradient_goes_past(const Tensor& leaf, bool own_hook) {
 // of few tokens waits for the host: as a Python function, forward and backward cost 20 us more than the library's lookup, which a step of 1200 us showed.
 class EmbeddingInto : public torch::autograd::Function<EmbeddingInto> {
  public:
-  static Tensor forward(torch::autograd::AutogradContext* ctx, const Tensor& ids, const Tensor& table) {
-    ctx->save_for_backward({ids});
+  static Tensor forward(torch::autograd::AutogradContext* ctx, const Tensor& ids, const Tensor& table, const c10::optional<Tensor>& grad_ids) {
+    ctx->save_for_backward({ids, grad_ids.has_value() ? *grad_ids : ids});
     ctx->saved_data["table"] = table;       // not saved as a value: a plain lookup does not need its values either
     return embedding_rows(table, ids);
   }
   static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::variable_list grads) {
-    if (!grads[0].defined() || !ctx->needs_input_grad(1)) return {Tensor(), Tensor()};
-    const Tensor ids = ctx->get_saved_variables()[0].reshape({-1}).contiguous(), table = ctx->saved_data["table"].toTensor();
+    if (!grads[0].defined() || !ctx->needs_input_grad(1)) return {Tensor(), Tensor(), Tensor()};
+    const auto saved = ctx->get_saved_variables();
+    const Tensor table = ctx->saved_data["table"].toTensor();
     const Tensor dy = grads[0].reshape({-1, table.size(1)}).contiguous(), g = table.grad();
     const bool fits = gradient_goes_past(table, false) && dy.size(0) <= rb_embedding_grad_tokens() && g.defined() && g.is_cuda() && g.sizes() == table.sizes() && g.is_contiguous() && table.size(1) % 8 == 0 &&
                       (g.scalar_type() == at::kFloat || (g.scalar_type() == dy.scalar_type() && (dy.scalar_type() == at::kBFloat16 || dy.scalar_type() == at::kHalf))) &&
                       ((reinterpret_cast<uintptr_t>(g.data_ptr()) | reinterpret_cast<uintptr_t>(dy.data_ptr())) & 15) == 0;
-    if (!fits) return {Tensor(), at::embedding_dense_backward(dy, ids, table.size(0), -1, false)};
-    embedding_grad_(dy, ids, g);
-    return {Tensor(), Tensor()};
+    if (!fits) return {Tensor(), at::embedding_dense_backward(dy, saved[0].reshape({-1}), table.size(0), -1, false), Tensor()};
+    embedding_grad_(dy, saved[1].reshape({-1}).contiguous(), g);
+    return {Tensor(), Tensor(), Tensor()};
   }
 };
 
-Tensor embedding_into(const Tensor& table, const Tensor& ids) { return EmbeddingInto::apply(ids, table); }
+// grad_ids: the ids that the gradient goes to (outside the table: nowhere), where they differ from the ids that are looked up
+Tensor embedding_into(const Tensor& table, const Tensor& ids, const c10::optional<Tensor>& grad_ids) {
+  TORCH_CHECK(!grad_ids.has_value() || grad_ids->sizes() == ids.sizes(), "embedding_into: ids and grad_ids");
+  return EmbeddingInto::apply(ids, table, grad_ids);
+}
 
 void register_gemm_ops(torch::Library& m);     // bindings_gemm.cpp
 void register_attn_ops(torch::Library& m);     // bindings_attn.cpp
@@ -411,7 +416,7 @@ TORCH_LIBRARY(realhf_b200, m) {
   m.def("logprob_fwd(Tensor logits, Tensor labels, Tensor? mask, float inv_temp, int vocab_start, bool partials) -> Tensor[]", &logprob_fwd);
   m.def("logprob_bwd_(Tensor(a!) logits, Tensor labels, Tensor? mask, Tensor lse, Tensor dlogp, float inv_temp, int vocab_start) -> ()", &logprob_bwd_);
   m.def("embedding_rows(Tensor table, Tensor ids) -> Tensor", &embedding_rows);
-  m.def("embedding_into(Tensor table, Tensor ids) -> Tensor", &embedding_into);
+  m.def("embedding_into(Tensor table, Tensor ids, Tensor? grad_ids=None) -> Tensor", &embedding_into);
   m.def("gradient_goes_past(Tensor leaf, bool own_hook) -> bool", &gradient_goes_past);
   m.def("embedding_grad_tokens() -> int", &rb_embedding_grad_tokens);
   m.def("embedding_grad_(Tensor dy, Tensor ids, Tensor(a!) dst) -> ()", &embedding_grad_);

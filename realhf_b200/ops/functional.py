@@ -819,23 +819,23 @@ class _Embedding(torch.autograd.Function):
     For a buffer beside `.grad` (`main_grad`); with the buffer in `.grad` the native `embedding_into` does the same."""
 
     @staticmethod
-    def forward(ctx, ids, weight):
-        ctx.save_for_backward(ids)
+    def forward(ctx, ids, weight, grad_ids):
+        ctx.save_for_backward(ids, ids if grad_ids is None else grad_ids)
         ctx.weight = weight          # a leaf with a buffer; not saved, as a plain lookup does not need its values either
         return _rows(ids, weight)
 
     @staticmethod
     def backward(ctx, dy):
-        (ids,), weight = ctx.saved_tensors, ctx.weight
+        (ids, grad_ids), weight = ctx.saved_tensors, ctx.weight
         if not ctx.needs_input_grad[1]:
-            return None, None
+            return None, None, None
         dy = dy.reshape(-1, weight.shape[1]).contiguous()
         own = bool(getattr(weight, "_main_grad_hooked", False)) and len(weight._post_accumulate_grad_hooks or ()) == 1
         g = _row_grad_buffer(weight) if lib().gradient_goes_past(weight, own) else None
         if g is None or dy.shape[0] > lib().embedding_grad_tokens() or (g.dtype != dy.dtype and g.dtype != torch.float32) or dy.data_ptr() % 16:
-            return None, torch.ops.aten.embedding_dense_backward(dy, ids.reshape(-1), weight.shape[0], -1, False)
-        lib().embedding_grad_(dy, ids.reshape(-1).contiguous(), g)
-        return None, None
+            return None, torch.ops.aten.embedding_dense_backward(dy, ids.reshape(-1), weight.shape[0], -1, False), None
+        lib().embedding_grad_(dy, grad_ids.reshape(-1).contiguous(), g)
+        return None, None, None
 
 
 def _row_grad_buffer(weight):
@@ -860,19 +860,20 @@ def _rows(ids, weight):
     return F.embedding(ids, weight)
 
 
-def embedding(ids, weight):
+def embedding(ids, weight, grad_ids=None):
     """weight[ids].  With a gradient asked for and a gradient buffer on the GPU the rows' gradients go straight into the buffer, unless somebody is to get the gradient
     itself (`torch.autograd.grad` with respect to the table, hooks on it, a gradient that is differentiated again: autograd accumulates then, as for a plain
     lookup); without a gradient the lookup is a kernel of its own; elsewhere (and inside function transforms and forward-mode differentiation, which the autograd
-    function does not answer for) the plain lookup."""
+    function does not answer for) the plain lookup.  `grad_ids` (a shard of a table): the ids that the gradient goes to where some of `ids` stand for rows that are
+    not here; outside the table it goes nowhere.  The caller sees to it that these rows' gradients are zero, so that a plain lookup's gradient is the same."""
     if (use_native(weight) and ids.dtype in (torch.int64, torch.int32)
             and not (torch.autograd.forward_ad._current_level >= 0 or torch._C._functorch.peek_interpreter_stack() is not None)):
         if not (weight.requires_grad and torch.is_grad_enabled()):
             return _rows(ids, weight)
         if weight.is_leaf and weight.dim() == 2 and _row_grad_buffer(weight) is not None:
             if getattr(weight, "main_grad", None) is None and _packed_rows(ids, weight):
-                return lib().embedding_into(weight, ids.contiguous())
-            return _Embedding.apply(ids, weight)
+                return lib().embedding_into(weight, ids.contiguous(), grad_ids)
+            return _Embedding.apply(ids, weight, grad_ids)
     return F.embedding(ids, weight)
 
 

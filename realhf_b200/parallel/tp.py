@@ -237,8 +237,8 @@ def vocab_parallel_embedding(ids, weight, ctx: Optional[ParallelContext], sp: bo
         return OF.embedding(ids, weight)
     lo, hi = ctx.tp_rank * weight.shape[0], (ctx.tp_rank + 1) * weight.shape[0]
     mask = (ids < lo) | (ids >= hi)
-    local = (ids - lo).masked_fill(mask, 0)
-    out = OF.embedding(local, weight)
+    local = ids - lo
+    out = OF.embedding(local.masked_fill(mask, 0), weight, local)       # (the other shards' tokens are not all row 0's: their gradients are zero)
     out = out.masked_fill(mask.unsqueeze(-1), 0.0)
     return reduce_scatter_to_sp(out, ctx) if sp else reduce_from_tp(out, ctx)
 

@@ -631,3 +631,34 @@ def test_gradients_go_past_autograd_on_the_accumulating_stream_only():
     torch.cuda.current_stream().wait_stream(side)
     a.sum().backward()
     assert said == [False, True] and torch.equal(w.grad, torch.full_like(w, 2.0))
+
+
+@pytest.mark.parametrize("ids_dtype", [torch.int64, torch.int32])
+@pytest.mark.parametrize("form", ["grad", "main_grad", "none"])
+@pytest.mark.parametrize("rank", [0, 1])
+def test_embedding_shard_leaves_rows_alone_that_no_token_reads(rank, form, ids_dtype, monkeypatch):
+    """A shard of a table: tokens of the other shard are looked up as row 0 and blanked; they add nothing to row 0's gradient, not even zeros (a row of -0.0 stays)."""
+    import types
+
+    from realhf_b200.parallel import tp as TP
+    monkeypatch.setattr(TP, "reduce_from_tp", lambda x, ctx: x)
+    g = torch.Generator(device="cuda").manual_seed(rank)
+    V, H, lo = 50, 72, 50 * rank
+    ids = torch.randint(1, 100, (3, 400), device="cuda", generator=g)
+    ids[ids == 50] = 51
+    ids = ids.to(ids_dtype)
+    here = (ids >= lo) & (ids < lo + V)
+    w = torch.nn.Parameter(torch.randn(V, H, device="cuda", generator=g).bfloat16())
+    buf = torch.full((V, H), -0.0, device="cuda", dtype=torch.float32 if form == "main_grad" else torch.bfloat16)
+    if form == "grad":
+        w.grad, w._grad_in_flat_buffer = buf, True
+    elif form == "main_grad":
+        w.main_grad = buf
+    dy = torch.randint(-2, 3, (3, 400, H), device="cuda", generator=g).bfloat16()
+    out = TP.vocab_parallel_embedding(ids, w, types.SimpleNamespace(tp_size=2, tp_rank=rank))
+    assert torch.equal(out, torch.where(here.unsqueeze(-1), w[(ids - lo).clamp(0, V - 1).long()], torch.zeros((), device="cuda", dtype=torch.bfloat16)))
+    out.backward(dy)
+    got = w.grad if form == "none" else buf
+    want = torch.zeros(V, H, device="cuda").index_add_(0, (ids - lo)[here].long(), dy[here].float())
+    assert torch.equal(got.float(), want)
+    assert form == "none" or bool(torch.signbit(buf[0]).all())
