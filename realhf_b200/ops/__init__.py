@@ -19,8 +19,10 @@ _lib = None
 _host = None
 
 
-# kernels launched per op call (for the `gpu_launches` accounting of bench.py); embedding_into: with its gradient
-_KERNELS_PER_OP = {"rmsnorm_bwd": 2, "embedding_grad_": 4, "embedding_into": 5, "embedding_grad_tokens": 0, "gradient_goes_past": 0, "adamw_step": 1, "decode_attention": 1, "attn_check": 0, "attn_status": 0, "attn_wait_error": 0}
+# kernels launched per op call (for the `gpu_launches` accounting of bench.py); the embedding's gradient, which a native backward pass launches without a call from
+# here, is counted by the library (`native_launches`)
+_KERNELS_PER_OP = {"rmsnorm_bwd": 2, "embedding_grad_": 0, "embedding_grad_tokens": 0, "gradient_goes_past": 0, "adamw_step": 1, "decode_attention": 1, "attn_check": 0,
+                   "attn_status": 0, "attn_wait_error": 0}
 
 
 class _LaunchCounter:
@@ -28,30 +30,49 @@ class _LaunchCounter:
     to that graph (`begin_capture` / `end_capture`) and re-counted on every replay (`count_replay`)."""
 
     def __init__(self):
-        self.total = 0
-        self.by_op = {}
+        self._total = 0
+        self._by_op = {}
         self._capturing = None
 
     def add(self, op: str, n: int = 1):
-        self.total += n
-        self.by_op[op] = self.by_op.get(op, 0) + n
+        self._total += n
+        self._by_op[op] = self._by_op.get(op, 0) + n
         if self._capturing is not None:
             self._capturing[0] += n
 
+    def _collect(self):
+        """Adds what the library has launched by itself since the last question."""
+        n = torch.ops.realhf_b200.native_launches() if _lib is not None else 0
+        if n:
+            self.add("embedding_grad_", n)
+
+    @property
+    def total(self) -> int:
+        self._collect()
+        return self._total
+
+    @property
+    def by_op(self) -> dict:
+        self._collect()
+        return self._by_op
+
     def begin_capture(self):
+        self._collect()
         self._capturing = [0]
 
     def end_capture(self) -> int:
+        self._collect()
         n, self._capturing = self._capturing[0], None
-        self.total -= n  # a capture does not execute the kernels
+        self._total -= n  # a capture does not execute the kernels
         return n
 
     def count_replay(self, n: int):
-        self.total += n
-        self.by_op["<graph replay>"] = self.by_op.get("<graph replay>", 0) + n
+        self._total += n
+        self._by_op["<graph replay>"] = self._by_op.get("<graph replay>", 0) + n
 
     def reset(self):
-        self.total, self.by_op = 0, {}
+        self._collect()
+        self._total, self._by_op = 0, {}
 
 
 launches = _LaunchCounter()

@@ -1,5 +1,7 @@
 // torch.ops.realhf_b200.* registrations.  Compiled with g++ (no nvcc): every kernel lives in a .cu file
 // behind an `extern "C"` launcher taking raw pointers and the *current* torch CUDA stream.
+#include <atomic>
+
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/csrc/autograd/custom_function.h>
@@ -328,6 +330,10 @@ Tensor embedding_rows(const Tensor& table, const Tensor& ids) {
   return out;
 }
 
+// Kernels launched where Python does not see the call (in a native backward pass), since the last question.
+std::atomic<int64_t> unseen_launches{0};
+int64_t native_launches() { return unseen_launches.exchange(0); }
+
 // dst [V, H] += the rows of dy [T, H] summed by id (ids outside [0, V) are passed over): the gradient of a table lookup, into a gradient buffer of dy's
 // type or fp32.
 void embedding_grad_(const Tensor& dy, const Tensor& ids, Tensor dst) {
@@ -340,7 +346,8 @@ void embedding_grad_(const Tensor& dy, const Tensor& ids, Tensor dst) {
   auto scratch = at::empty({2 * V + 2 + 2 * T + 3 * (T / 33)}, dy.options().dtype(at::kInt));
   const int rc = rb_embedding_grad(dy.data_ptr(), ids.data_ptr(), ids.scalar_type() == at::kLong, dst.data_ptr(), scratch.data_ptr<int>(), T, V, dy.size(1),
                                    dt_code(dy), dt_code(dst), cur_stream());
-  TORCH_CHECK(rc == 0, "embedding_grad_: unsupported configuration (", rc, ")");
+  TORCH_CHECK(rc >= 0, "embedding_grad_: unsupported configuration (", rc, ")");
+  unseen_launches += rc;
 }
 
 // In a backward pass: whether the gradient of a leaf may be added to its buffer here, past autograd's own accumulation.  Not when somebody is to get the gradient
@@ -418,6 +425,7 @@ TORCH_LIBRARY(realhf_b200, m) {
   m.def("embedding_rows(Tensor table, Tensor ids) -> Tensor", &embedding_rows);
   m.def("embedding_into(Tensor table, Tensor ids, Tensor? grad_ids=None) -> Tensor", &embedding_into);
   m.def("gradient_goes_past(Tensor leaf, bool own_hook) -> bool", &gradient_goes_past);
+  m.def("native_launches() -> int", &native_launches);
   m.def("embedding_grad_tokens() -> int", &rb_embedding_grad_tokens);
   m.def("embedding_grad_(Tensor dy, Tensor ids, Tensor(a!) dst) -> ()", &embedding_grad_);
   register_gemm_ops(m);

@@ -262,13 +262,14 @@ int run(const void* dy_, const void* ids_, void* dst_, int* scratch, int T, int 
     const int64_t most = (int64_t)(T / (kChain + 1)) * RB_CEIL_DIV(H, kSlice);
     heavy_kernel<G, D><<<(int)(most < 4 * rb::kNumSMs ? most : 4 * rb::kNumSMs), kThreads, 0, s>>>(totals, heavy, next, dy, dst, T, H);
   }
-  return cudaGetLastError() == cudaSuccess ? 0 : -3;
+  return cudaGetLastError() != cudaSuccess ? -3 : T > kChain ? 4 : 2;
 }
 
 }  // namespace
 
 // dy [T, H], dst [V, H] (packed, 16-byte aligned, H a multiple of 8); g_dt / d_dt: 0 fp32, 1 bf16, 2 fp16, d_dt = g_dt or 0; ids int64 or int32, those outside
-// [0, V) are passed over; scratch: 2 V + 2 + 2 T + 3 (T / 33) words.
+// [0, V) are passed over; scratch: 2 V + 2 + 2 T + 3 (T / 33) words.  Returns the
+// number of kernels launched, or a negative code.
 extern "C" int rb_embedding_grad(const void* dy, const void* ids, int ids_64, void* dst, int* scratch, int64_t T, int64_t V, int64_t H, int g_dt, int d_dt,
                                  cudaStream_t s) {
   if (T <= 0 || V <= 0 || H <= 0) return 0;

@@ -662,3 +662,24 @@ def test_embedding_shard_leaves_rows_alone_that_no_token_reads(rank, form, ids_d
     want = torch.zeros(V, H, device="cuda").index_add_(0, (ids - lo)[here].long(), dy[here].float())
     assert torch.equal(got.float(), want)
     assert form == "none" or bool(torch.signbit(buf[0]).all())
+
+
+@pytest.mark.parametrize("form", ["grad", "main_grad"])
+def test_launches_of_the_embedding_gradient_are_counted_when_they_come(form):
+    """The lookup counts as one kernel, its gradient as those that the backward pass launched: none without one, none of ours when the library forms the gradient."""
+    from realhf_b200.ops import functional as OF, launches
+    w, ids, dy, _, _ = _table(form)
+    launches.reset()
+    y = OF.embedding(ids, w)
+    assert launches.total == 1
+    y.backward(dy)
+    assert launches.total == 1 + 4 and launches.by_op["embedding_grad_"] == 4
+    OF.embedding(ids[:, :5], w).backward(dy[:, :5])
+    assert launches.total == 5 + 1 + 2                      # (up to 32 tokens: no long chains)
+    torch.autograd.grad(OF.embedding(ids, w), w, dy)
+    assert launches.total == 8 + 1
+    launches.reset()
+    launches.begin_capture()
+    OF.embedding(ids, w).backward(dy)
+    assert launches.end_capture() == 5 and launches.total == 0
+    launches.reset()
