@@ -33,17 +33,19 @@ struct AttnParams {
 }  // namespace rb
 
 // The process's status word of the attention kernels, in pinned host memory that every device can write (null if it cannot be had): not 0 once a
-// bounded wait has run out, until `rb_attn_wait_error` clears it.  The host reads it without a CUDA call (the bindings do before every launch), the
+// bounded wait has run out (kStatusGaveUp) or a kernel found its shared memory where it cannot work (kStatusUnaligned), until `rb_attn_wait_error` clears it.  The host reads it without a CUDA call (the bindings do before every launch), the
 // optimizer's kernels read it in stream order.
 extern "C" int* rb_attn_status();
 
 namespace rb {
 
+constexpr int kStatusGaveUp = 1, kStatusUnaligned = 2;
+
 // At the end of a CTA (all threads): if one of its waits ran out, what it had claimed is missing from the outputs.  Tell the host, and let copies land.
 RB_DEVICE void report_given_up(volatile uint32_t* dead, int* status) {
   if (*dead) {
     if (threadIdx.x == 0) {
-      *reinterpret_cast<volatile int*>(status) = 1;
+      *reinterpret_cast<volatile int*>(status) = kStatusGaveUp;
       __threadfence_system();
     }
     for (int i = 0; i < 1000; ++i) __nanosleep(1000);

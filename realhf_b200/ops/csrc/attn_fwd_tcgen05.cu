@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) attn_fwd_kernel(const __grid_c
   auto bar = [&](int i) { return ptx::smem_u32(&bars[i]); };
   auto wait = [&](int i, uint32_t parity) { bounded_wait(bar(i), parity, dead); };
   if ((sQ & 1023u) != 0u) {                                // (the swizzle wants it; never seen)
-    if (threadIdx.x == 0) *reinterpret_cast<volatile int*>(p.status) = 1;
+    if (threadIdx.x == 0) *reinterpret_cast<volatile int*>(p.status) = rb::kStatusUnaligned;
     return;
   }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -596,7 +596,7 @@ extern "C" int* rb_attn_status() {
   return word;
 }
 
-// 1 if a bounded wait of the kernels ran out since the last call (synchronises, and clears the word)
+// The status word since the last call: not 0 if a kernel left outputs unwritten (synchronises, and clears the word)
 extern "C" int rb_attn_wait_error() {
   volatile int* w = rb_attn_status();
   if (w == nullptr || cudaDeviceSynchronize() != cudaSuccess) return -1;

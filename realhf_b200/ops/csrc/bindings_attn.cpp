@@ -84,9 +84,12 @@ std::vector<Tensor> sample(const Tensor& logits, const c10::optional<Tensor>& un
 
 extern "C" int* rb_attn_status();
 
-// Raises if a bounded wait of an earlier attention kernel ran out (a plain read of host memory): parts of that kernel's outputs were never written.
+// Raises if an earlier attention kernel left parts of its outputs unwritten (a plain read of host memory): a bounded wait ran out, or (2) its shared memory did not
+// begin on 1024 bytes.
 void attn_check() {
   const volatile int* w = rb_attn_status();
+  TORCH_CHECK(w == nullptr || *w != 2, "an earlier attention kernel did not run, its outputs are unwritten: its shared memory did not begin on a multiple of 1024 bytes "
+                                       "(attn_wait_error() clears this)");
   TORCH_CHECK(w == nullptr || *w == 0, "an earlier attention kernel gave up waiting and left parts of its outputs unwritten (attn_wait_error() clears this)");
 }
 

@@ -445,6 +445,20 @@ def test_a_wait_that_ran_out_in_a_generation_step_is_raised(use_graph, monkeypat
     assert torch.equal(run(), want)
 
 
+def test_attention_status_says_what_went_wrong():
+    """Shared memory that a kernel cannot work in is not reported as a wait that ran out."""
+    q = torch.randn(40, 2, 64, device=DEV, dtype=torch.bfloat16)
+    cu = torch.tensor([0, 40], dtype=torch.int32, device=DEV)
+    word = lib().attn_status(torch.device("cuda", 0))
+    assert lib().attn_wait_error() == 0
+    for code, text in ((2, "1024 bytes"), (1, "gave up waiting")):
+        word.fill_(code)
+        torch.cuda.synchronize()
+        with pytest.raises(RuntimeError, match=text):
+            lib().attn_fwd(q, q, q, cu, 40, 0.125, True)
+        assert lib().attn_wait_error() == code and lib().attn_wait_error() == 0
+
+
 def _scores(cols):
     """Sequences [S, n keys, 128] of scores -> q, k, v of one head whose query r has the scores of column r % 128, one sequence after the other."""
     S, n, _ = cols.shape
