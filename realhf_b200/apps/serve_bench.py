@@ -342,7 +342,7 @@ def tizodra_kernel_numbers(name: str, s: dict, batch: int, prompt_len: int, ctx:
     wte = torch.randn(s["vocab"], W, device=dev).to(bf)
     ids = torch.randint(0, s["vocab"], (T,), device=dev)
     add("embed_sinusoid (prefill)", False, _time(lambda: OF.embed_sinusoid(ids, wte, meta.pos), 10, flush=flush), T * W * 6, 0)
-    add("embedding lookup (llama, prefill)", True, _time(lambda: torch.nn.functional.embedding(ids, wte), 10, flush=flush), T * W * 4, 0)
+    add("embedding lookup (llama, prefill)", True, _time(lambda: OF.embedding(ids, wte), 10, flush=flush), T * W * 4, 0)
     add("sublayer_input (RMSNorm of the fp32 stream, prefill)", False, _time(lambda: OF.sublayer_input(x32, w, 1, 1e-5, None, None, bf), 10, flush=flush),
         T * W * 6, 0)
     add("residual_add_norm_ (fp32 stream += branch, prefill)", False, _time(lambda: OF.residual_add_norm_(x32, xb, None, 1, 1e-5), 10, flush=flush),
