@@ -802,7 +802,7 @@ int rb_gemm_tcgen05(const void* A, const void* B, void* C, const void* bias, int
 // Small-M GEMM (decode shapes): M <= 128, K-major operands, no accumulate.  `ws` holds 2 * num_sms * 128 * 256 floats,
 // `flags` 8192 zero-initialised words (persistent per device; calls sharing them must be stream-ordered).
 // bn = 0 / split = 0: pick the tile width (multiple of 16) and the K split from a byte-ingest cost model:
-//   t = max(weight bytes / HBM, bytes per CTA / ~85 GB/s per-SM TMA ingest) + fix-up(split > 1),
+//   t = max(weight bytes / HBM, bytes per CTA / ~70 GB/s per-SM TMA ingest) + fix-up(split > 1),
 // over the layouts with tiles_n * split <= #SMs (tile-aligned split: one fix-up round per CTA).
 // in_dt: 1 bf16, 2 fp16, 3 fp8 e4m3 (then scale_a [M] / scale_b [N] fp32 are required; lda / ldb count bytes = elements)
 static int streamk_impl(const void* A, const void* B, void* C, const void* bias, int M, int N, int K, int64_t lda, int64_t ldb,
@@ -829,20 +829,23 @@ static int streamk_impl(const void* A, const void* B, void* C, const void* bias,
       for (int sp = 1; sp <= smax; ++sp) {
         const double waves = (double)RB_CEIL_DIV(tiles * sp, num_sms);
         const double cta_bytes = (double)(box_rows + cand) * 128.0 * RB_CEIL_DIV(num_kb, sp) * waves;
-        double t = cta_bytes / 85e3;                              // us
+        double t = cta_bytes / 70e3;                              // us
         const double hbm = (double)N * K * esz / 6.5e6;           // us
         if (t < hbm) t = hbm;
-        // per-k-block term: 0.2 .. 0.25 measured; with 0.33 (whole tiles: 0.30) the layouts picked are within 3 % of the best of a sweep over widths and splits
+        // per-k-block term: 0.2 .. 0.25 measured, 0.33 (whole tiles: 0.30) stands for what lies around it
         const double kb_floor = (sp > 1 ? 0.33 : 0.30) * RB_CEIL_DIV(num_kb, sp) * waves;
         if (t < kb_floor) t = kb_floor;
         // The parts of a tile in a cluster of 2 or 4: what the merge takes is nearly constant.  Cold weights at 16, 64 and 128 rows, through the workspace / so:
-        // 4096 x 4096 12.4 / 9.8, 12.3 / 10.5, 14.2 / 11.7 us; 4096 x 11008 20.3 / 17.6, 21.8 / 19.2, 25.5 / 21.4; 2048 x 2048 7.7 / 6.1, 8.2 / 6.7, 9.0 / 7.4;
-        // 6144 x 4096 13.9 / 11.7, 15.4 / 13.4, 18.1 / 15.6; 768 x 3072 8.7 / 5.7, 8.1 / 6.6, 7.2 / 7.4 us.
+        // 4096 x 4096 12.2 / 9.7, 12.2 / 10.6, 14.0 / 11.9 us; 4096 x 11008 19.7 / 17.6, 21.6 / 19.2, 25.4 / 21.4; 2048 x 2048 7.6 / 6.1, 8.1 / 6.7, 8.9 / 7.4;
+        // 6144 x 4096 13.4 / 11.6, 15.0 / 13.3, 17.6 / 15.3; 768 x 3072 8.7 / 5.7, 8.2 / 6.7, 8.3 / 7.3 us.
         // Of 4 as long as all are there at once (32 of 37 SMs; 148 CTAs take two rounds: 15.0 us for the first); clusters of 8 wait for 8 free SMs of one GPC
-        // (16.1).  Taken when it is clearly ahead: 12288 x 4096 in two parts takes 19.4 / 22.5 / 27.0, whole 19.1 / 20.7 / 22.8.
+        // (16.1).  Taken when it is clearly ahead: 12288 x 4096 in two parts takes 19.4 / 22.5 / 27.0, whole 18.9 / 20.7 / 23.0.
         const double in_cluster = t + 3.3 + 0.2e-3 * M * cand;
         if ((sp == 2 || (sp == 4 && tiles * 4 <= num_sms * 32 / 37)) && in_cluster < 0.96 * best) { best = in_cluster / 0.96; bn = cand; split = parts = sp; }
-        if (sp > 1) t += 5.0 + 0.12 * sp + 4.5 * (double)M * cand * 4.0 / 60e3;  // partial write + barrier + cooperative reduce of sp parts (measured)
+        // Through the workspace: partial write, barrier, and a reduction that takes eight parts a round trip to L2, so 16 parts cost no more than 13 (with a cost for every
+        // single part 512 x 8192 at 80 rows took 9.9 us in 13 parts, in 16 9.3).  Over 760 shapes of 1 .. 128 rows against layouts chosen without clusters and at a constant
+        // cost of the merge: 1.09 times as fast in the geometric mean, the slowest 0.96, four below 0.985 (1536 x 8192 from 112 rows, 2048 x 14336 up to 48).
+        if (sp > 1) t += 5.4 + 0.02 * sp + 0.8 * RB_CEIL_DIV(sp, 8) + 4.5 * (double)M * cand * 4.0 / 60e3;
         if (t < best) { best = t; bn = cand; split = sp; parts = 1; }
       }
     }
