@@ -1,4 +1,5 @@
-"""Model check of the mbarrier protocols of the tcgen05 attention kernels (csrc/attn_fwd_tcgen05.cu, attn_bwd_tcgen05.cu, attn_fwd_bias.cu).
+"""Model check of the mbarrier protocols of the tcgen05 attention kernels (csrc/attn_bwd_tcgen05.cu, attn_fwd_bias.cu; with the simulator for
+csrc/attn_fwd_tcgen05.cu, whose roles are in test_attention_forward_protocol_cpu.py).
 
 The roles of a CTA (TMA producer and scheduler, MMA issuer, softmax / element warps) are written as coroutines that perform exactly the waits,
 arrives, expect_tx and commits of the kernels (same barrier names, same parities), over several work items of one CTA where the kernel is
@@ -263,163 +264,9 @@ def load(sim, buf, bar, parts, what):
 ITEM_BARS = {"IT_FULL0": 1, "IT_FULL1": 1, "IT_EMPTY0": 9, "IT_EMPTY1": 9, "CLC_FULL": 1}
 
 
-# ------------------------------------------------------------------------------------------------ forward kernel (pairs of query tiles)
-# (with the output left to the softmax warps; test_attention_forward_protocol_cpu.py has the kernel with output warps of its own)
+# The forward kernel's walk (its roles: test_attention_forward_protocol_cpu.py): stages of its K / V ring, which of a pair's query tiles takes a key tile
 STAGES = 4
-
-
-def fwd_pair_protocol(sim: Sim, items):
-    """An item is the list of its key tiles, each (taken by query tile 0, taken by query tile 1)."""
-    B = sim.bars
-    it = Items(sim, items, 9)
-
-    def producer():
-        kvc, qc, idx = 0, [0, 0], 0
-        it.request()
-        while idx is not None:
-            walk = items[idx]
-            yield from it.publish(walk)
-
-            def load_q(t):
-                if any(k[t] for k in walk):
-                    yield ("wait", f"Q_EMPTY{t}", (qc[t] & 1) ^ 1)
-                    qc[t] += 1
-                    load(sim, f"Q{t}", f"Q_FULL{t}", 2, "Q load")
-
-            def load_kv():
-                nonlocal kvc
-                st = kvc % STAGES
-                yield ("wait", f"KV_EMPTY{st}", ((kvc // STAGES) & 1) ^ 1)
-                kvc += 1
-                load(sim, f"KV{st}", f"KV_FULL{st}", 2, "K / V load")
-            yield from load_q(0)
-            yield from load_kv()
-            yield from load_q(1)
-            yield from load_kv()
-            for _ in walk[1:]:
-                yield from load_kv()
-                yield from load_kv()
-            idx = yield from it.next()
-            if idx is not None:
-                it.request()
-        yield from it.publish(None)
-
-    def mma():
-        kvc, qc, pc, oc, n_it = 0, [0, 0], [0, 0], [0, 0], 0
-        while True:
-            walk = yield from it.take(n_it)
-            n_it += 1
-            if walk is None:
-                return
-            s_open, o_open = [False, False], [False, False]
-            last = [max((k for k, x in enumerate(walk) if x[t]), default=-1) for t in range(2)]
-
-            def open_kv(c):
-                yield ("wait", f"KV_FULL{c % STAGES}", (c // STAGES) & 1)
-                return c % STAGES
-
-            def free_kv(st):
-                sim.pipe.append(lambda: (sim.set(f"KV{st}", "free"), B[f"KV_EMPTY{st}"].arrive()))
-
-            def issue_s(t, k, st):
-                if not s_open[t]:
-                    yield ("wait", f"Q_FULL{t}", qc[t] & 1)
-                    qc[t] += 1
-                    s_open[t] = True
-
-                def run():
-                    sim.expect(f"Q{t}", "full", "S mma"), sim.expect(f"KV{st}", "full", "S mma"), sim.expect(f"S{t}", "free", "S mma")
-                    sim.set(f"S{t}", "s")
-                sim.pipe.append(run)
-                sim.pipe.append(lambda: B[f"S_FULL{t}"].arrive())
-                if k == last[t]:
-                    sim.pipe.append(lambda: (sim.set(f"Q{t}", "free"), B[f"Q_EMPTY{t}"].arrive()))
-
-            def issue_pv(t, st):
-                yield ("wait", f"P_FULL{t}", pc[t] & 1)
-                pc[t] += 1
-                if not o_open[t]:
-                    yield ("wait", f"O_EMPTY{t}", (oc[t] & 1) ^ 1)
-                    oc[t] += 1
-                was, o_open[t] = "acc" if o_open[t] else "free", True
-                sim.state[f"PV{t}"] = sim.state.get(f"PV{t}", 0) + 1           # issued and not retired
-
-                def run():
-                    sim.expect(f"S{t}", "p", "PV mma"), sim.expect(f"KV{st}", "full", "PV mma"), sim.expect(f"O{t}", was, "PV mma")
-                    sim.set(f"S{t}", "free"), sim.set(f"O{t}", "acc")
-                    sim.state[f"PV{t}"] -= 1
-                sim.pipe.append(run)
-                sim.pipe.append(lambda: B[f"O_FULL{t}"].arrive())
-            st = yield from open_kv(kvc)
-            for t in range(2):
-                if walk[0][t]:
-                    yield from issue_s(t, 0, st)
-            free_kv(st)
-            for k in range(len(walk)):
-                sv, sk = (yield from open_kv(kvc + 2 * k + 1)), None
-                for t in range(2):
-                    if walk[k][t]:
-                        yield from issue_pv(t, sv)
-                    if t == 1:
-                        free_kv(sv)
-                    if k + 1 < len(walk):
-                        if sk is None:
-                            sk = yield from open_kv(kvc + 2 * k + 2)
-                        if walk[k + 1][t]:
-                            yield from issue_s(t, k + 1, sk)
-                if sk is not None:
-                    free_kv(sk)
-            kvc += 2 * len(walk)
-
-    def softmax(w):
-        t, sc, vc, n_it = w >> 2, 0, 0, 0
-        while True:
-            walk = yield from it.take(n_it)
-            n_it += 1
-            if walk is None:
-                return
-            n_tiles = sum(k[t] for k in walk)
-            if n_tiles == 0:
-                continue
-            for k in range(n_tiles):
-                yield ("wait", f"S_FULL{t}", sc & 1)
-                sc += 1
-                sim.expect(f"S{t}", "s", "softmax reads S")
-                if k > 0 and sim.rng.random() < 0.5:               # the row's maximum has grown: O is scaled
-                    yield ("wait", f"O_FULL{t}", (vc - 1) & 1)
-                    sim.expect(f"O{t}", "acc", "O is scaled")
-                    assert sim.state[f"PV{t}"] == 0, "O is scaled with a product in flight"
-                if count_down(sim, f"S{t}_warps", 4):
-                    sim.set(f"S{t}", "p")
-                B[f"P_FULL{t}"].arrive()
-                vc += 1
-            yield ("wait", f"O_FULL{t}", (vc - 1) & 1)
-            sim.expect(f"O{t}", "acc", "output")
-            assert sim.state[f"PV{t}"] == 0, "output with a product in flight"
-            if count_down(sim, f"O{t}_warps", 4):
-                sim.set(f"O{t}", "free")
-            B[f"O_EMPTY{t}"].arrive()
-
-    return {"producer": producer(), "mma": mma(), **{f"softmax{w}": softmax(w) for w in range(8)}}
-
-
-PAIR_BARS = dict(ITEM_BARS)
-for _t in (0, 1):
-    PAIR_BARS.update({f"Q_FULL{_t}": 1, f"Q_EMPTY{_t}": 1, f"S_FULL{_t}": 1, f"P_FULL{_t}": 4, f"O_FULL{_t}": 1, f"O_EMPTY{_t}": 4})
-for _st in range(STAGES):
-    PAIR_BARS.update({f"KV_FULL{_st}": 1, f"KV_EMPTY{_st}": 1})
-
 ONE, BOTH, SECOND = (True, False), (True, True), (False, True)
-
-
-@pytest.mark.parametrize("items", [[[BOTH]], [[ONE]], [[BOTH] * 3 + [ONE]], [[ONE]] * 5, [[BOTH]] * 5, [[BOTH] * 2 + [ONE], [ONE], [BOTH] * 5, [ONE] * 3],
-                                   [[SECOND] * 2 + [BOTH] * 2 + [ONE], [BOTH, SECOND, BOTH, ONE], [ONE]], [[BOTH] * 9, [BOTH] * 2 + [ONE], [BOTH] * 4]],
-                         ids=lambda x: "-".join(str(len(w)) for w in x))
-def test_forward_pair_protocol_has_no_deadlock_or_buffer_hazard(items):
-    for seed in range(100):
-        sim = Sim(seed, PAIR_BARS)
-        sim.run(fwd_pair_protocol(sim, items))
-        assert all(v in ("free", 0) for v in sim.state.values()), sim.state
 
 
 # ------------------------------------------------------------------------------------------------ backward kernel (both passes)
