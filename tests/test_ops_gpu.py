@@ -683,3 +683,16 @@ def test_launches_of_the_embedding_gradient_are_counted_when_they_come(form):
     OF.embedding(ids, w).backward(dy)
     assert launches.end_capture() == 5 and launches.total == 0
     launches.reset()
+
+
+@pytest.mark.parametrize("dtype,buffer", [(torch.float32, torch.float32), (torch.bfloat16, torch.float32), (torch.bfloat16, torch.bfloat16)])
+def test_embedding_gradient_keeps_numbers_below_the_normal_ones(dtype, buffer):
+    """Sums of subnormal numbers are exact, in short chains and in long ones, as in the sums of a plain lookup's gradient."""
+    from realhf_b200.ops import lib
+    tiny = 2.0 ** -130                                       # a multiple of bf16's smallest number too
+    ids = torch.tensor([0] + [1] * 3 + [2] * 40 + [3] * 600, device="cuda")
+    dy = torch.full((ids.numel(), 16), tiny, device="cuda").to(dtype)
+    buf = torch.full((5, 16), tiny, device="cuda").to(buffer)
+    lib().embedding_grad_(dy, ids, buf)
+    want = torch.tensor([2.0, 4.0, 41.0, 601.0, 1.0], dtype=torch.float64, device="cuda") * tiny
+    assert torch.equal(buf, want.to(buffer)[:, None].expand(5, 16))
