@@ -336,25 +336,27 @@ def test_gemm_cta_pair_output_edges(M, N, K, shift, dtype):
 
 @pytest.mark.parametrize("M,N,K,bn,split", [(80, 512, 8192, 64, 16), (128, 384, 8192, 48, 16), (112, 512, 8192, 64, 16)])
 def test_few_row_layout_fills_its_round_trips(M, N, K, bn, split):
-    """The reduction of a tile's parts takes eight of them at a time: the layout that is chosen must not be behind one whose parts fill those eights (cold weights, a captured loop,
-    medians; it was 5 .. 6 % behind while every part had a cost of its own)."""
+    """The reduction of a tile's parts takes eight of them at a time: the layout that is chosen must not be behind one whose parts fill those eights (cold weights, captured loops
+    in turn, the best of each; it was 5 .. 6 % behind while every part had a cost of its own)."""
     x = torch.randn(M, K, device="cuda").bfloat16()
     ws = [torch.randn(N, K, device="cuda").bfloat16() * 0.02 for _ in range(30)]
 
-    def median(**layout):
+    def loop(**layout):
         graph = torch.cuda.CUDAGraph()
         G.gemm_streamk(x, ws[0], **layout)
         torch.cuda.synchronize()
         with torch.cuda.graph(graph):
             for w in ws:
                 G.gemm_streamk(x, w, **layout)
-        times = []
-        for _ in range(15):
-            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-            a.record()
-            graph.replay()
-            b.record()
-            b.synchronize()
-            times.append(a.elapsed_time(b))
-        return sorted(times)[7]
-    assert median() <= 1.03 * median(bn=bn, split=split)
+        return graph
+
+    def time(graph):
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        a.record()
+        graph.replay()
+        b.record()
+        b.synchronize()
+        return a.elapsed_time(b)
+    chosen, full = loop(), loop(bn=bn, split=split)
+    pairs = [(time(chosen), time(full)) for _ in range(25)]
+    assert min(t for t, _ in pairs) <= 1.03 * min(t for _, t in pairs)
