@@ -67,6 +67,29 @@ __global__ void __launch_bounds__(kRowThreads) rows_kernel(const I* __restrict__
     if (first + i * kRowThreads < n) out[t * n + first + i * kRowThreads] = x[i];
 }
 
+// The same for many rows: a warp a row, four pieces a lane in flight.  A block a row is launched as often as there are rows, whatever is in them.
+template <typename I>
+__global__ void __launch_bounds__(kThreads) rows_warp_kernel(const I* __restrict__ ids, const uint4* __restrict__ table, uint4* __restrict__ out, int64_t V, int n, int64_t T) {
+  constexpr int kAhead = 4;
+  rb::pdl_wait();
+  rb::pdl_trigger();
+  const int64_t t = (int64_t)blockIdx.x * kWarps + (threadIdx.x >> 5);
+  if (t >= T) return;
+  const int64_t v = (int64_t)ids[t];
+  assert(v >= 0 && v < V);
+  const uint4* from = table + v * n;
+  uint4* to = out + t * n;
+  for (int c = threadIdx.x & 31; c < n; c += 32 * kAhead) {
+    uint4 x[kAhead];
+#pragma unroll
+    for (int i = 0; i < kAhead; ++i)
+      if (c + 32 * i < n) x[i] = from[c + 32 * i];
+#pragma unroll
+    for (int i = 0; i < kAhead; ++i)
+      if (c + 32 * i < n) to[c + 32 * i] = x[i];
+  }
+}
+
 // head[v]: last token of the chain plus one (0: none), next[t]: the one before it, in the same form; rank[t]: how many of its id were counted before it
 template <typename I>
 __global__ void __launch_bounds__(kThreads) chain_kernel(const I* __restrict__ ids, int* __restrict__ head, int* __restrict__ count, int* __restrict__ next,
@@ -284,16 +307,29 @@ extern "C" int rb_embedding_grad(const void* dy, const void* ids, int ids_64, vo
   return -4;
 }
 
-// out [T, row_bytes], table [V, row_bytes] (packed, 16-byte aligned, row_bytes a multiple of 16); ids int64 or int32 below V.  A piece a thread while that leaves
-// SMs without a block, two otherwise (four: 3.3 us for 1024 rows of 8 KB, two 2.9).
+// out [T, row_bytes], table [V, row_bytes] (packed, 16-byte aligned, row_bytes a multiple of 16); ids int64 or int32 below V.  A block a row: a piece a thread while that
+// leaves SMs without a block, two otherwise (four: 3.3 us for 1024 rows of 8 KB, two 2.9), four for some thousand rows from 16 KB (1800 of 16 KB two 7.5, four 6.3; 20480 of
+// them two 94, four 98).  A warp a row for many rows where blocks would idle for more than a tenth or all stays in L2 (us, the library's lookup / a block / a warp a row:
+// 4000 rows of 1.5 KB 3.8 / 4.8 / 3.1, 20480 of them 12.2 / 22.0 / 7.1, 20480 of 6400 bytes 36.1 / 43.3 / 22.6, 4000 of 8 KB 8.4 / 9.1 / 8.2; but 1000 of 1.5 KB
+// 2.2 / 1.8 / 2.2, 1300 of 10 KB 4.5 / 4.9 / 5.2, 20480 of 8 KB 61 / 48 / 52).
 extern "C" int rb_embedding_rows(const void* table, const void* ids, int ids_64, void* out, int64_t T, int64_t V, int64_t row_bytes, cudaStream_t s) {
   if (T <= 0 || row_bytes <= 0) return 0;
   if (row_bytes % 16 != 0 || T > 0x7fffffff || row_bytes > (1 << 24) || (((uintptr_t)table | (uintptr_t)out) & 15)) return -1;
   const int n = (int)(row_bytes / 16);
+  const int64_t slots = (int64_t)RB_CEIL_DIV(n, 2 * kRowThreads) * (2 * kRowThreads);
+  if (10 * (slots - n) > slots ? T >= 1536 : n < 1024 && T >= 2048 && T * row_bytes <= (48 << 20)) {
+    const dim3 warps((unsigned)RB_CEIL_DIV(T, kWarps));
+#define RB_GO(I) rb::launch_pdl(rows_warp_kernel<I>, warps, dim3(kThreads), 0, s, (const I*)ids, (const uint4*)table, (uint4*)out, V, n, T) == cudaSuccess ? 0 : -3
+    if (ids_64) return RB_GO(int64_t);
+    return RB_GO(int32_t);
+#undef RB_GO
+  }
   const bool many = T * RB_CEIL_DIV(n, 2 * kRowThreads) >= rb::kNumSMs;
-  const dim3 grid((unsigned)T, RB_CEIL_DIV(n, (many ? 2 : 1) * kRowThreads));
+  const int per = many ? (n >= 1024 && T > 1000 && T <= 8192 ? 4 : 2) : 1;
+  const dim3 grid((unsigned)T, RB_CEIL_DIV(n, per * kRowThreads));
 #define RB_GO(I, N) \
   rb::launch_pdl(rows_kernel<I, N>, grid, dim3(kRowThreads), 0, s, (const I*)ids, (const uint4*)table, (uint4*)out, V, n) == cudaSuccess ? 0 : -3
+  if (per == 4) return ids_64 ? RB_GO(int64_t, 4) : RB_GO(int32_t, 4);
   if (ids_64) return many ? RB_GO(int64_t, 2) : RB_GO(int64_t, 1);
   return many ? RB_GO(int32_t, 2) : RB_GO(int32_t, 1);
 #undef RB_GO

@@ -22,7 +22,7 @@ def body(file: str, kernel: str) -> str:
             return text[at:end]
 
 
-@pytest.mark.parametrize("file,kernel", [("embed_grad.cu", "rows_kernel"), ("posenc.cu", "embed_sinusoid_kernel")])
+@pytest.mark.parametrize("file,kernel", [("embed_grad.cu", "rows_kernel"), ("embed_grad.cu", "rows_warp_kernel"), ("posenc.cu", "embed_sinusoid_kernel")])
 def test_the_first_kernel_of_a_pass_triggers_behind_its_wait(file, kernel):
     text = body(file, kernel)
     assert text.count("pdl_wait()") == 1 and text.count("pdl_trigger()") == 1
