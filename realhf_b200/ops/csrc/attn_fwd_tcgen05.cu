@@ -34,9 +34,9 @@
 // are formed: the product before has retired (the scores that showed the growth were issued behind it), and the next one waits for both.  (A maximum
 // that only moves when weights exceed it by 2^8 is 2..3 % faster in training, 10 % with a window, but the largest weight is then no longer exactly
 // 1 when P is rounded to 16 bits: error against 64 bits 0.0028 instead of 0.0025.)  V_j is the MN-major B operand.
-// Issue order: S_0, S_1, then per key tile PV_0, S_0', PV_1, S_1'.  The issuing warp runs converged and one elected lane issues: from a branch of one lane with
-// descriptors built there, eight MMAs took 820-960 cycles, whatever their size.  (Behind a predicate instead of a branch they took as long on 640 tokens and on
-// long batches, and a windowed prefill took 247 against 240 us.)
+// Issue order: S_0, S_1, then per key tile PV_0, S_0', PV_1, S_1'.  The issuing warp runs converged, the MMAs are predicated on an elected lane: issued from
+// `if (lane == 0)` with descriptors built there, eight MMAs took 820-960 cycles of one thread, whatever their size.  (Behind one branch of the elected lane, S alone or all,
+// windowed prefill is 3 % faster and 39 of 282 forms by 2 .. 5 %, but items of one key tile without grouped heads are 4 % slower; both in one kernel: most forms slower, up to 14 %.)
 //
 // Outputs: O [T, nq, DV] through a per-warp staging buffer (whole 128-byte lines), LSE [nq, T] (natural log, scale applied).
 //
@@ -229,8 +229,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) attn_fwd_kernel(const __grid_c
       constexpr uint32_t idesc_s = ptx::make_idesc_f16(kFmt, kTile, kTile, 0, 0);   // Q, K both K-major (head-dim contiguous)
       constexpr uint32_t idesc_o = ptx::make_idesc_f16(kFmt, kTile, kDV, 0, 1);     // P (TMEM), V MN-major
       constexpr uint32_t kToMN = (uint32_t)((kTile * 128 - 16) >> 4) << 16;         // from the K-major form of a tile to its MN-major one
-      const uint32_t tm = (uint32_t)ptx::uniform((int)tmem_base);
-      const bool el = ptx::elect_one();
+      const uint32_t tm = (uint32_t)ptx::uniform((int)tmem_base), el = ptx::elect_one() ? 1u : 0u;
       const uint32_t q_lo = ptx::desc_lo(sQ, 16), kv_lo = ptx::desc_lo(sKV, 16);
       uint32_t kvc = 0, qc[2] = {0, 0}, pc[2] = {0, 0};
       for (int n_it = 0;; ++n_it) {
@@ -250,29 +249,23 @@ __global__ void __launch_bounds__(kFwdThreads, 1) attn_fwd_kernel(const __grid_c
           if (!s_open[t]) { wait(Q_FULL + t, qc[t] & 1u); ++qc[t]; s_open[t] = true; }
           ptx::tc_fence_after();
           const uint32_t a = q_lo + t * (C::kQBytes >> 4), b = kv_lo + st * (C::kStageBytes >> 4);
-          if (el) {
 #pragma unroll
-            for (int kk = 0; kk < kD / 16; ++kk) {
-              const uint32_t off = ((kk >> 2) * (kTile * 128) + (kk & 3) * 32) >> 4;
-              ptx::tc_mma_f16(tm + t * 128, ptx::desc1024(a + off), ptx::desc1024(b + off), idesc_s, kk != 0 ? 1u : 0u);
-            }
-            ptx::tc_commit(bar(S_FULL + t));
-            if (j == last_tile(t)) ptx::tc_commit(bar(Q_EMPTY + t));
+          for (int kk = 0; kk < kD / 16; ++kk) {
+            const uint32_t off = ((kk >> 2) * (kTile * 128) + (kk & 3) * 32) >> 4;
+            ptx::tc_mma_f16_if(el, tm + t * 128, a + off, b + off, idesc_s, kk != 0 ? 1u : 0u);
           }
-          __syncwarp();
+          ptx::tc_commit_if(el, bar(S_FULL + t));
+          if (j == last_tile(t)) ptx::tc_commit_if(el, bar(Q_EMPTY + t));
         };
         auto issue_pv = [&](int t, int j, uint32_t st) {
           wait(P_FULL + t, pc[t] & 1u);
           ++pc[t];
           ptx::tc_fence_after();
           const uint32_t b = kv_lo + kToMN + st * (C::kStageBytes >> 4), keep = o_open[t] ? 1u : 0u;
-          if (el) {
 #pragma unroll
-            for (int kk = 0; kk < kTile / 16; ++kk)      // A: 16 keys = 8 TMEM columns; B: 16 key rows = 2048 B down every 64-wide chunk of DV
-              ptx::tc_mma_f16_ts(tm + 256 + t * 128, tm + t * 128 + kk * 8, ptx::desc1024(b + kk * 128), idesc_o, kk != 0 ? 1u : keep);
-            if (j == last_tile(t)) ptx::tc_commit(bar(O_FULL + t));
-          }
-          __syncwarp();
+          for (int kk = 0; kk < kTile / 16; ++kk)      // A: 16 keys = 8 TMEM columns; B: 16 key rows = 2048 B down every 64-wide chunk of DV
+            ptx::tc_mma_f16_ts_if(el, tm + 256 + t * 128, tm + t * 128 + kk * 8, b + kk * 128, idesc_o, kk != 0 ? 1u : keep);
+          if (j == last_tile(t)) ptx::tc_commit_if(el, bar(O_FULL + t));
           o_open[t] = true;
         };
         auto peek_kv = [&](uint32_t c) { return ptx::mbar_try_wait(bar(KV_FULL + (c & (kStages - 1))), (c / kStages) & 1u); };
@@ -280,10 +273,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) attn_fwd_kernel(const __grid_c
           if (!ready) wait(KV_FULL + (c & (kStages - 1)), (c / kStages) & 1u);
           return c & (kStages - 1);
         };
-        auto free_kv = [&](uint32_t st) {
-          if (el) ptx::tc_commit(bar(KV_EMPTY + st));
-          __syncwarp();
-        };
+        auto free_kv = [&](uint32_t st) { ptx::tc_commit_if(el, bar(KV_EMPTY + st)); };
         uint32_t st = pass_kv(kvc, false);
 #pragma unroll
         for (int t = 0; t < 2; ++t)

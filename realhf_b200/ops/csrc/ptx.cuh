@@ -136,6 +136,29 @@ __device__ __forceinline__ void tc_ld_32x32(uint32_t taddr, uint32_t* r) {
       : "memory");
 }
 
+// Predicated forms for code that all 32 lanes run: `el` is 1 in the lane that issues (elect_one() once) and 0 in the others.  Without a branch around them the
+// warp stays converged and their operands are formed on the uniform datapath: 40 cycles an MMA against 48 behind a branch (N = 32, descriptors in
+// registers).  Descriptors come as their varying lower halves; the upper half of an sw128 descriptor with 1024 bytes between row groups is a constant.
+constexpr uint32_t kDescHi1024 = (1024u >> 4) | (1u << 14) | (2u << 29);
+__device__ __forceinline__ void tc_mma_f16_if(uint32_t el, uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, e;\n\t.reg .b64 a, b;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 e, %5, 0;\n\tmov.b64 a, {%1, %6};\n\tmov.b64 b, {%2, %6};\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p;\n\t}" ::"r"(tmem_d),
+      "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(el), "r"(kDescHi1024)
+      : "memory");
+}
+__device__ __forceinline__ void tc_mma_f16_ts_if(uint32_t el, uint32_t tmem_d, uint32_t tmem_a, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, e;\n\t.reg .b64 b;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 e, %5, 0;\n\tmov.b64 b, {%2, %6};\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %3, p;\n\t}" ::"r"(tmem_d),
+      "r"(tmem_a), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(el), "r"(kDescHi1024)
+      : "memory");
+}
+__device__ __forceinline__ void tc_commit_if(uint32_t el, uint32_t bar) {
+  asm volatile("{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %1, 0;\n\t@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar), "r"(el)
+               : "memory");
+}
+
 __device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 // thread i of the warp writes 32 consecutive 32-bit columns of row (lane_base + i)
 __device__ __forceinline__ void tc_st_32x32(uint32_t taddr, const uint32_t* r) {
@@ -190,9 +213,8 @@ __device__ __forceinline__ uint64_t make_smem_desc_sw128(uint32_t smem_addr, uin
   d |= (uint64_t)2 << 61;  // SWIZZLE_128B
   return d;
 }
-// Its lower half, which holds the address, and the whole with 1024 bytes between row groups, whose upper half is a constant.
+// Its lower half, which holds the address (the upper one: kDescHi1024 with 1024 bytes between row groups).
 __device__ __forceinline__ uint32_t desc_lo(uint32_t smem_addr, uint32_t lbo_bytes) { return ((smem_addr >> 4) & 0x3fffu) | (lbo_bytes >> 4) << 16; }
-__device__ __forceinline__ uint64_t desc1024(uint32_t lo) { return (uint64_t)((1024u >> 4) | (1u << 14) | (2u << 29)) << 32 | lo; }
 // Instruction descriptor for kind::f16 with fp32 accumulation. fmt: 0 = fp16, 1 = bf16. major: 0 = K, 1 = MN.
 __host__ __device__ constexpr uint32_t make_idesc_f16(int fmt, int M, int N, int a_major, int b_major) {
   return (1u << 4) | ((uint32_t)fmt << 7) | ((uint32_t)fmt << 10) | ((uint32_t)a_major << 15) | ((uint32_t)b_major << 16) |
